@@ -397,6 +397,11 @@ int ntcb_texture_set_sample(NtcbTextureSet* textureSet, const float* deviceQueri
 /* Waits for everything queued on the texture set's stream. */
 int ntcb_texture_set_synchronize(NtcbTextureSet* textureSet);
 
+/* Orders the texture set's stream after what is queued on `stream` (a cudaStream_t) at the time of the call: work the
+   set queues from here on - blocks, pixels or answers written into a buffer of the caller's - starts when that has
+   finished.  The host does not wait. */
+int ntcb_texture_set_wait_for_stream(NtcbTextureSet* textureSet, void* stream);
+
 /* One decoded mip (fp16, device memory, `layout`, `channels` channels per texel) converted into
    pixel-interleaved client data in device memory with the given strides: the kernel behind
    ntcb_texture_set_read_channels, for callers that hold the decoded texels themselves.  Replaces

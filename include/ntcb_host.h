@@ -89,6 +89,8 @@ public:
     // pixel-major copy is made then too; the call waits for the answers.
     virtual Status Sample(float const* deviceQueries, uint64_t numQueries, void* deviceOut, bool useInt8Weights) = 0;
     virtual Status Synchronize() = 0;
+    // Orders the set's stream after what is queued on `stream` (a cudaStream_t) now; the host does not wait.
+    virtual Status WaitForStream(void* stream) = 0;
     virtual ~ITextureSet() = default;
 };
 

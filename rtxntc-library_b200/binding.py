@@ -233,6 +233,7 @@ def lib():
         handle.ntcb_texture_set_device_mip.argtypes = [
             ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_size_t)]
         handle.ntcb_texture_set_synchronize.argtypes = [ctypes.c_void_p]
+        handle.ntcb_texture_set_wait_for_stream.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
         handle.ntcb_read_channels_to_host_noalloc.argtypes = [
             ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
             ctypes.c_void_p, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_void_p]
@@ -243,6 +244,22 @@ def lib():
 def check(code: int) -> None:
     if code != 0:
         raise NtcbError(code, lib().ntcb_last_error().decode())
+
+
+def _queue(device, entry_point, *arguments) -> None:
+    """Calls a C entry point whose last argument is a stream with torch's current stream of `device` (a torch.device
+    with an index), on that device.  The small launches are bound by what Python does per call, so the stream is looked
+    up as a plain handle (torch.cuda.current_stream() builds an object: 3.3 us) and the device is only switched when
+    another one is current (the context manager: 1.5 us)."""
+    import torch
+
+    index = device.index
+    stream = torch._C._cuda_getCurrentRawStream(index)
+    if torch.cuda.current_device() == index:
+        check(entry_point(*arguments, stream))
+    else:
+        with torch.cuda.device(index):
+            check(entry_point(*arguments, stream))
 
 
 def stage_network(blob: bytes, weight_mode: int, numerics: int = NUMERICS_REFERENCE) -> np.ndarray:
@@ -345,7 +362,7 @@ def convert_channels(texels, conversion: OutputConversion, layout: int = LAYOUT_
     dtype = {CHANNEL_FORMAT_UNORM8: torch.uint8, CHANNEL_FORMAT_UNORM16: torch.int16, CHANNEL_FORMAT_FLOAT16: torch.float16,
              CHANNEL_FORMAT_FLOAT32: torch.float32, CHANNEL_FORMAT_UINT32: torch.int32}[conversion.channelFormat]
     out_width, out_height = (width, height) if size is None else size  # another size: bilinear resize
-    out = torch.zeros((out_height, out_width, conversion.components), dtype=dtype, device=texels.device)
+    out = torch.empty((out_height, out_width, conversion.components), dtype=dtype, device=texels.device)  # every component is written
     params = ConvertParams()
     params.deviceMip = texels.data_ptr()
     params.layout, params.width, params.height, params.channels = layout, width, height, channels
@@ -355,9 +372,7 @@ def convert_channels(texels, conversion: OutputConversion, layout: int = LAYOUT_
     params.conversion = conversion
     if size is not None:
         params.dstWidth, params.dstHeight = size
-    with torch.cuda.device(texels.device):
-        stream = torch.cuda.current_stream(texels.device).cuda_stream
-        check(lib().ntcb_convert_channels(ctypes.byref(params), ctypes.c_void_p(stream)))
+    _queue(texels.device, lib().ntcb_convert_channels, ctypes.byref(params))
     return out
 
 
@@ -382,10 +397,7 @@ def pack_latents(latents, width: int, height: int, num_layers: int, latent_strid
     if latents.dtype != torch.float16 or latents.numel() < needed:
         raise ValueError(f"latents must be float16 with at least {needed} elements")
     out = torch.empty((num_layers, height, width), dtype=torch.int16, device=latents.device)
-    with torch.cuda.device(latents.device):
-        stream = torch.cuda.current_stream(latents.device).cuda_stream
-        check(lib().ntcb_pack_latents(ctypes.c_void_p(latents.data_ptr()), width, height, num_layers, latent_stride,
-                                      ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(stream)))
+    _queue(latents.device, lib().ntcb_pack_latents, latents.data_ptr(), width, height, num_layers, latent_stride, out.data_ptr())
     return out
 
 
@@ -401,7 +413,7 @@ def quantize_network(weights, biases, weight_mode: int, output_scale=None, outpu
     if biases.dtype != torch.float16 or biases.numel() != NETWORK_COLUMN_COUNT:
         raise ValueError("biases must be float16 with NETWORK_COLUMN_COUNT elements")
     blob_bytes = INT8_BLOB_BYTES if weight_mode == WEIGHTS_INT8 else FP8_BLOB_BYTES
-    blob = torch.zeros(blob_bytes, dtype=torch.uint8, device=weights.device)
+    blob = torch.empty(blob_bytes, dtype=torch.uint8, device=weights.device)  # the sections fill it without gaps
     rounded = torch.empty_like(weights) if want_rounded else None
     params = QuantizeNetworkParams()
     params.weights, params.biases = weights.data_ptr(), biases.data_ptr()
@@ -414,9 +426,7 @@ def quantize_network(weights, biases, weight_mode: int, output_scale=None, outpu
     params.weightMode = weight_mode
     params.blob = blob.data_ptr()
     params.roundedWeights = rounded.data_ptr() if want_rounded else None
-    with torch.cuda.device(weights.device):
-        stream = torch.cuda.current_stream(weights.device).cuda_stream
-        check(lib().ntcb_quantize_network(ctypes.byref(params), ctypes.c_void_p(stream)))
+    _queue(weights.device, lib().ntcb_quantize_network, ctypes.byref(params))
     return (blob, rounded) if want_rounded else blob
 
 
@@ -469,7 +479,7 @@ def block_compress(texels, block_format: int, first_channel: int = 0, layout: in
     bw = (width - src_left + 3) // 4 if width_in_blocks is None else width_in_blocks
     bh = (height - src_top + 3) // 4 if height_in_blocks is None else height_in_blocks
     block_bytes = 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
-    out = torch.zeros((bh, bw, block_bytes), dtype=torch.uint8, device=texels.device)
+    out = torch.empty((bh, bw, block_bytes), dtype=torch.uint8, device=texels.device)  # every block is written
     params = BlockCompressParams()
     params.deviceMip = texels.data_ptr()
     params.layout, params.width, params.height, params.channels = layout, width, height, channels
@@ -483,9 +493,7 @@ def block_compress(texels, block_format: int, first_channel: int = 0, layout: in
         params.modeBufferByteOffset = mode_buffer_byte_offset
         params.modeMapWidthInBlocks, params.modeMapHeightInBlocks = mode_map_size if mode_map_size is not None else (bw, bh)
         params.modeMapOffsetX, params.modeMapOffsetY = mode_map_offset
-    with torch.cuda.device(texels.device):
-        stream = torch.cuda.current_stream(texels.device).cuda_stream
-        check(lib().ntcb_block_compress(ctypes.byref(params), ctypes.c_void_p(stream)))
+    _queue(texels.device, lib().ntcb_block_compress, ctypes.byref(params))
     return out
 
 
@@ -511,6 +519,8 @@ class ResidentTextureSet:
         }
         self.status = torch.zeros(STATUS_WORDS, dtype=torch.int32, device=self.device)
         self.out = torch.empty(out_elements(geo), dtype=torch.float16, device=self.device) if allocate_output else None
+        self._decode_plans: dict = {}  # weight mode -> (what the parameters were filled from, parameters of a whole-set decode)
+        self._sample_plans: dict = {}  # (weight mode, interleaved) -> the same for sample()
 
     @classmethod
     def from_synthetic(cls, synthetic_set, **kwargs) -> "ResidentTextureSet":
@@ -532,19 +542,33 @@ class ResidentTextureSet:
         torch = self.torch
         dtype = {CHANNEL_FORMAT_UNORM8: torch.uint8, CHANNEL_FORMAT_UNORM16: torch.int16, CHANNEL_FORMAT_FLOAT16: torch.float16,
                  CHANNEL_FORMAT_FLOAT32: torch.float32, CHANNEL_FORMAT_UINT32: torch.int32}[conversion.channelFormat]
-        out = torch.zeros(self.geometry.total_texels * conversion.components, dtype=dtype, device=self.device)
-        with torch.cuda.device(self.device):
-            self.launch(self.params(use_int8, out=out, mips=mips, row_ranges=row_ranges, conversion=conversion))
+        # a decode of some mips or rows leaves the rest at zero; a whole one writes every pixel
+        allocate = torch.empty if mips is None and not row_ranges else torch.zeros
+        out = allocate(self.geometry.total_texels * conversion.components, dtype=dtype, device=self.device)
+        self.launch(self.params(use_int8, out=out, mips=mips, row_ranges=row_ranges, conversion=conversion))
         return out
 
     def launch(self, params: DecodeParams) -> None:
         """Queues one decode on torch's current stream of this device."""
-        stream = self.torch.cuda.current_stream(self.device).cuda_stream
-        check(lib().ntcb_decode(ctypes.byref(params), ctypes.c_void_p(stream)))
+        _queue(self.latents.device, lib().ntcb_decode, ctypes.byref(params))
+
+    def _pointers(self, mode: int) -> tuple:
+        """What the parameters of a launch depend on besides the geometry: they are filled again when one of these changes."""
+        return (self.latents.data_ptr(), self.networks[mode].data_ptr(), self.status.data_ptr(),
+                None if self.out is None else self.out.data_ptr(), self.layout, self.numerics)
 
     def decode(self, use_int8: bool, mips=None, row_ranges=None) -> None:
-        with self.torch.cuda.device(self.device):
+        if mips is not None or row_ranges:
             self.launch(self.params(use_int8, mips=mips, row_ranges=row_ranges))
+            return
+        # Filling the parameters takes as long as launching them (6.5 us for six mips), so those of the whole set are kept;
+        # nothing writes to them afterwards, which makes them safe to launch from several threads.
+        mode = WEIGHTS_INT8 if use_int8 else WEIGHTS_FP8
+        key = self._pointers(mode)
+        plan = self._decode_plans.get(mode)
+        if plan is None or plan[0] != key:
+            plan = self._decode_plans[mode] = (key, self.params(use_int8))
+        self.launch(plan[1])
 
     def interleave_latents(self):
         """ntcb_interleave_latents: the pixel-major copy of the latents (a slot of 1, 2 or 4 elements per latent
@@ -559,37 +583,36 @@ class ResidentTextureSet:
             # (only the mip descriptions of these parameters are used)
             decode = fill_params(self.geometry, self.latents.data_ptr(), self.networks[WEIGHTS_INT8].data_ptr(),
                                  self.status.data_ptr(), self.status.data_ptr(), WEIGHTS_INT8)
-            with torch.cuda.device(self.device):
-                stream = torch.cuda.current_stream(self.device).cuda_stream
-                check(lib().ntcb_interleave_latents(ctypes.c_void_p(self.latents.data_ptr()),
-                                                    ctypes.c_void_p(self.interleaved_latents.data_ptr()), decode.mips,
-                                                    decode.numMips, decode.numFeatures, ctypes.c_void_p(stream)))
+            _queue(self.latents.device, lib().ntcb_interleave_latents, self.latents.data_ptr(),
+                   self.interleaved_latents.data_ptr(), decode.mips, decode.numMips, decode.numFeatures)
         return self.interleaved_latents
 
     def sample(self, queries, use_int8: bool, interleaved: bool = False):
         """Inference on sample: `queries` is a float32 CUDA tensor [n][3] of (u, v, lod); returns a
         float16 CUDA tensor [n][channels].  Queued on torch's current stream.  `interleaved`: read the
         latents from the copy `interleave_latents()` makes (same answers, fewer memory requests)."""
-        torch = self.torch
         mode = WEIGHTS_INT8 if use_int8 else WEIGHTS_FP8
         queries = queries.contiguous()
-        out = torch.empty((queries.shape[0], self.geometry.channels), dtype=torch.float16, device=self.device)
-        network = self.networks[mode]
+        out = self.torch.empty((queries.shape[0], self.geometry.channels), dtype=self.torch.float16, device=self.device)
         latents = self.interleave_latents() if interleaved else self.latents
-        decode = fill_params(self.geometry, latents.data_ptr(), network.data_ptr(), out.data_ptr(),
-                             self.status.data_ptr(), mode)
-        params = SampleParams()
-        params.latentLayout = LATENTS_INTERLEAVED if interleaved else LATENTS_PLANAR
-        params.latents, params.network, params.queries = decode.latents, decode.network, queries.data_ptr()
-        params.out, params.status, params.numQueries = out.data_ptr(), decode.status, queries.shape[0]
-        params.numMips, params.numFeatures, params.channels = decode.numMips, decode.numFeatures, decode.channels
-        params.weightMode = mode
-        params.numerics = self.numerics
-        for i in range(decode.numMips):
-            params.mips[i] = decode.mips[i]
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream(self.device).cuda_stream
-            check(lib().ntcb_sample(ctypes.byref(params), ctypes.c_void_p(stream)))
+        key = self._pointers(mode) + (latents.data_ptr(),)
+        plan = self._sample_plans.get((mode, interleaved))
+        if plan is None or plan[0] != key:
+            decode = fill_params(self.geometry, latents.data_ptr(), self.networks[mode].data_ptr(), out.data_ptr(),
+                                 self.status.data_ptr(), mode)
+            params = SampleParams()
+            params.latentLayout = LATENTS_INTERLEAVED if interleaved else LATENTS_PLANAR
+            params.latents, params.network, params.status = decode.latents, decode.network, decode.status
+            params.numMips, params.numFeatures, params.channels = decode.numMips, decode.numFeatures, decode.channels
+            params.weightMode = mode
+            params.numerics = self.numerics
+            for i in range(decode.numMips):
+                params.mips[i] = decode.mips[i]
+            plan = self._sample_plans[(mode, interleaved)] = (key, params)
+        # a copy of its own for every call: another thread may be sampling too
+        params = SampleParams.from_buffer_copy(plan[1])
+        params.queries, params.out, params.numQueries = queries.data_ptr(), out.data_ptr(), queries.shape[0]
+        _queue(self.latents.device, lib().ntcb_sample, ctypes.byref(params))
         return out
 
     def check_status(self) -> None:
@@ -653,6 +676,20 @@ class TextureSet:
                                                         ctypes.byref(features), ctypes.byref(self.handle)))
         self.desc = TextureSetDesc()
         check(lib().ntcb_texture_set_get_desc(self.handle, ctypes.byref(self.desc)))
+        self._block_formats: dict = {}  # texture index -> the block format its header names
+
+    def _empty_blocks(self, mip: int, block_format: int):
+        """(uninitialised CUDA uint8 tensor for the blocks of one mip, its row pitch).  The set's stream is made to wait for
+        torch's current one, whose queued work may still be using the memory the tensor was given; the encoders write
+        every block, so nothing has to be cleared and the host waits for nothing here."""
+        import torch
+
+        width, height = self.mip_size(mip)
+        bw, bh = (width + 3) // 4, (height + 3) // 4
+        block_bytes = 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
+        out = torch.empty((bh, bw, block_bytes), dtype=torch.uint8, device="cuda")
+        check(lib().ntcb_texture_set_wait_for_stream(self.handle, torch._C._cuda_getCurrentRawStream(out.device.index)))
+        return out, bw * block_bytes
 
     def mip_size(self, mip: int) -> Tuple[int, int]:
         return max(1, self.desc.width >> mip), max(1, self.desc.height >> mip)
@@ -733,20 +770,15 @@ class TextureSet:
                        alpha_threshold: float = 1.0 / 255.0):
         """One decoded mip as BC1 - BC5 blocks: a CUDA uint8 tensor [blocks_y][blocks_x][8 or 16]
         (waits for the texture set's stream)."""
-        import torch
-
-        width, height = self.mip_size(mip)
-        bw, bh = (width + 3) // 4, (height + 3) // 4
-        block_bytes = 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
-        out = torch.zeros((bh, bw, block_bytes), dtype=torch.uint8, device="cuda")
-        torch.cuda.synchronize()
+        out, row_pitch = self._empty_blocks(mip, block_format)
         check(lib().ntcb_texture_set_block_compress(self.handle, mip, first_channel, num_channels, block_format,
-                                                    alpha_threshold, ctypes.c_void_p(out.data_ptr()), bw * block_bytes))
+                                                    alpha_threshold, out.data_ptr(), row_pitch))
         self.synchronize()
         return out
 
     def load_from_memory(self, container: bytes) -> None:
         """Another compressed set of the same shape into this one's buffers (ITextureSet::LoadFromMemory)."""
+        self._block_formats = {}
         check(lib().ntcb_texture_set_load_from_memory(self.handle, container, len(container)))
 
     def bc7_mode_buffer(self, texture_index: int, mip_level: int) -> Optional[np.ndarray]:
@@ -767,16 +799,12 @@ class TextureSet:
     def block_compress_texture(self, texture_index: int, mip_level: int, alpha_threshold: float = 1.0 / 255.0):
         """One mip of one texture in the block format its header names (BC7: from its stored mode bitmap when it
         has one): a CUDA uint8 tensor [blocks_y][blocks_x][8 or 16] (waits for the texture set's stream)."""
-        import torch
-
-        block_format = self.textures()[texture_index]["blockCompressedFormat"]
-        width, height = self.mip_size(mip_level)
-        bw, bh = (width + 3) // 4, (height + 3) // 4
-        block_bytes = 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
-        out = torch.zeros((bh, bw, block_bytes), dtype=torch.uint8, device="cuda")
-        torch.cuda.synchronize()
+        block_format = self._block_formats.get(texture_index)
+        if block_format is None:
+            block_format = self._block_formats[texture_index] = self.textures()[texture_index]["blockCompressedFormat"]
+        out, row_pitch = self._empty_blocks(mip_level, block_format)
         check(lib().ntcb_texture_set_block_compress_texture(self.handle, texture_index, mip_level, alpha_threshold,
-                                                            ctypes.c_void_p(out.data_ptr()), bw * block_bytes))
+                                                            out.data_ptr(), row_pitch))
         self.synchronize()
         return out
 
@@ -805,8 +833,7 @@ class TextureSet:
 
         queries = queries.contiguous()
         out = torch.empty((queries.shape[0], self.desc.channels), dtype=torch.float16, device=queries.device)
-        check(lib().ntcb_texture_set_sample(self.handle, ctypes.c_void_p(queries.data_ptr()), queries.shape[0],
-                                            ctypes.c_void_p(out.data_ptr()), 1 if use_int8 else 0))
+        check(lib().ntcb_texture_set_sample(self.handle, queries.data_ptr(), queries.shape[0], out.data_ptr(), 1 if use_int8 else 0))
         return out
 
     def synchronize(self) -> None:

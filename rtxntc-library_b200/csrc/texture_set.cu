@@ -94,6 +94,7 @@ public:
     Status LoadFromMemory(void const* pData, size_t size) override;
     Status Sample(float const* deviceQueries, uint64_t numQueries, void* deviceOut, bool useInt8Weights) override;
     Status Synchronize() override;
+    Status WaitForStream(void* stream) override;
 
     const SetGeometry& Geometry() const { return m_geometry; }
 
@@ -135,6 +136,7 @@ private:
     bool m_deviceCurrent = false, m_pixelMajorCurrent = false;
     uint16_t* m_pixelMajor = nullptr;
     cudaEvent_t m_eventStart = nullptr, m_eventStop = nullptr;
+    cudaEvent_t m_eventClient = nullptr; // see WaitForStream
     bool m_decoded = false;
 
     // A whole-set decode of a large set is issued as kBands launches over row bands of mip 0 plus one
@@ -330,6 +332,8 @@ Status TextureSet::Initialize(LoadedSet&& loaded, const TextureSetFeatures& feat
     err = cudaEventCreate(&m_eventStart);
     if (err == cudaSuccess)
         err = cudaEventCreate(&m_eventStop);
+    if (err == cudaSuccess)
+        err = cudaEventCreateWithFlags(&m_eventClient, cudaEventDisableTiming);
     for (int b = 0; b <= kBands && err == cudaSuccess; ++b)
         err = cudaEventCreateWithFlags(&m_bandEvents[b], cudaEventDisableTiming);
     if (err != cudaSuccess)
@@ -426,6 +430,7 @@ void TextureSet::Release()
     }
     if (m_eventStart) cudaEventDestroy(m_eventStart);
     if (m_eventStop) cudaEventDestroy(m_eventStop);
+    if (m_eventClient) cudaEventDestroy(m_eventClient);
     for (std::vector<void*>& perMip : m_deviceModeBuffers)
         for (void*& copy : perMip)
         {
@@ -441,7 +446,7 @@ void TextureSet::Release()
     if (m_texels) cudaFree(m_texels);
     if (m_deviceUpload) cudaFree(m_deviceUpload);
     if (m_hostUpload) cudaFreeHost(m_hostUpload);
-    m_eventStart = m_eventStop = nullptr;
+    m_eventStart = m_eventStop = m_eventClient = nullptr;
     m_staging = nullptr;
     m_status = nullptr;
     m_hostStatus = nullptr;
@@ -1225,6 +1230,26 @@ Status TextureSet::Synchronize()
     return NTCB_OK;
 }
 
+Status TextureSet::WaitForStream(void* stream)
+{
+    DeviceGuard guard(m_device);
+    if (!guard.Success())
+        return NTCB_ERR_CUDA;
+    const cudaStream_t client = static_cast<cudaStream_t>(stream);
+    cudaError_t err = cudaStreamQuery(client);
+    if (err == cudaErrorNotReady) // an idle stream has nothing to wait for
+    {
+        (void)cudaGetLastError(); // the query's answer is not a failure of a later launch
+        err = cudaEventRecord(m_eventClient, client);
+        if (err == cudaSuccess)
+            err = cudaStreamWaitEvent(m_stream, m_eventClient, 0);
+    }
+    if (err != cudaSuccess)
+        return CudaFailure("cudaStreamWaitEvent", err);
+    ClearError();
+    return NTCB_OK;
+}
+
 } // namespace
 
 Status CreateContext(IContext** pOutContext, ContextParameters const& params)
@@ -1586,6 +1611,16 @@ int ntcb_texture_set_synchronize(NtcbTextureSet* textureSet)
         return NTCB_ERR_INVALID_ARGUMENT;
     }
     return ntcb::Guarded(__func__, [&]() { return textureSet->impl->Synchronize(); });
+}
+
+int ntcb_texture_set_wait_for_stream(NtcbTextureSet* textureSet, void* stream)
+{
+    if (!textureSet)
+    {
+        ntcb::SetError("textureSet is NULL.");
+        return NTCB_ERR_INVALID_ARGUMENT;
+    }
+    return ntcb::Guarded(__func__, [&]() { return textureSet->impl->WaitForStream(stream); });
 }
 
 } // extern "C"
