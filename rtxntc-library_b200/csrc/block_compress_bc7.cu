@@ -7,7 +7,7 @@
 //    compressed offline (ntc::MakeBC7ModeBuffer, src/PublicFunctions.cpp:488-556); the encoder only
 //    fits endpoints and indices for that one configuration.  The threads of a CTA are re-ordered by
 //    mode through shared memory so that a warp runs one mode (CompressBC7.hlsl:1446-1493);
-//  * without: every mode is tried - 64 partitions of modes 0 / 2, 1 / 3 and 7 by estimated error, the
+//  * without (the offline path): every mode is tried - 64 partitions of modes 0 / 2, 1 / 3 and 7 by estimated error, the
 //    best one of each encoded, modes 4 / 5 under the four channel rotations, mode 6 - and the block
 //    with the smallest squared error of its reconstruction kept (ties: the later mode).
 //
@@ -41,13 +41,18 @@ constexpr uint32_t kAllPixels = 0xffffu;
 // rest; pixel 0 is always in subset 0).  Three subsets: subset 1 in the low half, subset 2 in the high
 // half.  Anchors: bits 0-3 the anchor of subset 1 of a two-subset partition, bits 4-7 and 8-11 those of
 // subsets 1 and 2 of a three-subset partition.
-__constant__ uint16_t kPartition2[64] = {
+struct PartitionTables
+{
+    uint16_t two[64];
+    uint32_t three[64];
+    uint16_t anchors[64];
+};
+constexpr PartitionTables kHostPartitions = {{
     0xcccc, 0x8888, 0xeeee, 0xecc8, 0xc880, 0xfeec, 0xfec8, 0xec80, 0xc800, 0xffec, 0xfe80, 0xe800, 0xffe8, 0xff00, 0xfff0, 0xf000,
     0xf710, 0x008e, 0x7100, 0x08ce, 0x008c, 0x7310, 0x3100, 0x8cce, 0x088c, 0x3110, 0x6666, 0x366c, 0x17e8, 0x0ff0, 0x718e, 0x399c,
     0xaaaa, 0xf0f0, 0x5a5a, 0x33cc, 0x3c3c, 0x55aa, 0x9696, 0xa55a, 0x73ce, 0x13c8, 0x324c, 0x3bdc, 0x6996, 0xc33c, 0x9966, 0x0660,
     0x0272, 0x04e4, 0x4e40, 0x2720, 0xc936, 0x936c, 0x39c6, 0x639c, 0x9336, 0x9cc6, 0x817e, 0xe718, 0xccf0, 0x0fcc, 0x7744, 0xee22,
-};
-__constant__ uint32_t kPartition3[64] = {
+}, {
     0xf60008ccu, 0x73008cc8u, 0x3310cc80u, 0x00ceec00u, 0xcc003300u, 0xcc0000ccu, 0x00ccff00u, 0x3300ccccu,
     0xf0000f00u, 0xf0000ff0u, 0xff0000f0u, 0x88884444u, 0x88886666u, 0xcccc2222u, 0xec80136cu, 0x7310008cu,
     0xc80036c8u, 0x310008ceu, 0xccc03330u, 0x0cccf000u, 0xee0000eeu, 0x77008888u, 0xcc0022c0u, 0x33004430u,
@@ -56,13 +61,44 @@ __constant__ uint32_t kPartition3[64] = {
     0x03c0c03cu, 0xff0000aau, 0x5500aa00u, 0xcccc3030u, 0x0c0cc0c0u, 0x66669090u, 0x0ff0a00au, 0x5550aaa0u,
     0xf0000aaau, 0x0e0ee0e0u, 0x88887070u, 0x99906660u, 0xe00e0ee0u, 0x88880770u, 0xf0000666u, 0x99006600u,
     0xff000066u, 0xc00c0cc0u, 0xcccc0330u, 0x90006000u, 0x08088080u, 0xeeee1010u, 0xfff0000au, 0x731008ceu,
-};
-__constant__ uint16_t kAnchors[64] = {
+}, {
     0xf3f, 0x83f, 0x8ff, 0x3ff, 0xf8f, 0xf3f, 0x3ff, 0x8ff, 0xf8f, 0xf8f, 0xf6f, 0xf6f, 0xf6f, 0xf5f, 0xf3f, 0x83f,
     0xf3f, 0x832, 0xf88, 0x3f2, 0xf32, 0x838, 0xf68, 0x8af, 0x352, 0xf88, 0x682, 0xa62, 0xf88, 0xf58, 0xaf2, 0x8f2,
     0xf8f, 0x3ff, 0xf36, 0xa58, 0xa62, 0x8a8, 0x98f, 0xaff, 0x6f2, 0xf38, 0x8f2, 0xf52, 0x3f2, 0x6ff, 0x6ff, 0x8f6,
     0xf36, 0x3f2, 0xf56, 0xf58, 0xf5f, 0xf8f, 0xf52, 0xfa2, 0xf5f, 0xfaf, 0xf8f, 0xfdf, 0x3ff, 0xfc2, 0xf32, 0x83f,
+}};
+__constant__ PartitionTables kPartitions = kHostPartitions;
+
+// The pixels of a partition subset by subset, each subset's in ascending order: four bits per pixel in `order`, and where
+// the subsets end (bytes 0 to 2 of `ends`).  The partition search walks these lists, so it never visits a pixel for a
+// subset that does not hold it.
+struct PixelLists
+{
+    uint64_t order[64];
+    uint32_t ends[64];
 };
+
+constexpr PixelLists MakePixelLists(bool three)
+{
+    PixelLists lists{};
+    for (int partition = 0; partition < 64; ++partition)
+    {
+        const uint32_t second = three ? kHostPartitions.three[partition] & kAllPixels : uint32_t(kHostPartitions.two[partition]);
+        const uint32_t third = three ? kHostPartitions.three[partition] >> 16 : 0u;
+        const uint32_t masks[3] = {~(second | third) & kAllPixels, second, third};
+        int position = 0;
+        for (int subset = 0; subset < 3; ++subset)
+        {
+            for (int pixel = 0; pixel < 16; ++pixel)
+                if ((masks[subset] >> pixel) & 1u)
+                    lists.order[partition] |= uint64_t(pixel) << (4 * position++);
+            lists.ends[partition] |= uint32_t(position) << (8 * subset);
+        }
+    }
+    return lists;
+}
+__constant__ PixelLists kPixelLists2 = MakePixelLists(false);
+__constant__ PixelLists kPixelLists3 = MakePixelLists(true);
 
 // The subsets of a partition: pixel masks and anchor pixels (the pixel whose index loses its top bit).
 struct Subsets
@@ -73,15 +109,15 @@ struct Subsets
 
 __device__ __forceinline__ Subsets TwoSubsets(int partition)
 {
-    const uint32_t second = kPartition2[partition];
-    return {{~second & kAllPixels, second, 0u}, {0, int(kAnchors[partition] & 15), 0}};
+    const uint32_t second = kPartitions.two[partition];
+    return {{~second & kAllPixels, second, 0u}, {0, int(kPartitions.anchors[partition] & 15), 0}};
 }
 
 __device__ __forceinline__ Subsets ThreeSubsets(int partition)
 {
-    const uint32_t packed = kPartition3[partition];
+    const uint32_t packed = kPartitions.three[partition];
     const uint32_t second = packed & kAllPixels, third = packed >> 16;
-    const uint32_t anchors = kAnchors[partition];
+    const uint32_t anchors = kPartitions.anchors[partition];
     return {{~(second | third) & kAllPixels, second, third}, {0, int((anchors >> 4) & 15), int((anchors >> 8) & 15)}};
 }
 
@@ -142,19 +178,48 @@ __device__ __forceinline__ float Saturate(float v)
     return fminf(fmaxf(v, 0.f), 1.f); // NaN -> 0
 }
 
+// Saturate(a * b)
+__device__ __forceinline__ float MultiplySaturate(float a, float b)
+{
+    float r;
+    asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // ---- the texels of a block ------------------------------------------------------------------------------
 // rotation: which channel is the scalar one of a dual-plane mode (0: alpha, 1: red, 2: green, 3: blue, the
 // other one of the pair taking alpha's place); the vector part is the first three components.
 struct Pixels
 {
-    const uint2* base; // texel i at base[i * kThreads]
+    const uint2* base; // texel i at base[i * stride]
     int rotation;
+    int stride;
 };
+
+// Calls body(i) for the pixels of a subset in ascending order.  A mask is walked bit by bit: the lanes of a warp hold
+// different partitions in the searching kernel, and looping over all sixteen pixels for every subset would leave half to
+// two thirds of them idle.
+template <bool kAll, typename Body>
+__device__ __forceinline__ void ForEachPixel(uint32_t mask, Body&& body)
+{
+    if (kAll)
+    {
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i)
+            body(i);
+    }
+    else
+    {
+#pragma unroll 1
+        for (uint32_t rest = mask; rest; rest &= rest - 1u)
+            body(__ffs(rest) - 1);
+    }
+}
 
 template <int C>
 __device__ __forceinline__ Vec<C> Pixel(const Pixels& pixels, int i)
 {
-    const uint2 raw = pixels.base[i * kThreads];
+    const uint2 raw = pixels.base[i * pixels.stride];
     const float2 rg = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
     const float2 ba = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
     float r = rg.x, g = rg.y, b = ba.x, a = ba.y;
@@ -191,10 +256,25 @@ __device__ __forceinline__ Vec<C> Pixel(const Pixels& pixels, int i)
 }
 
 // ---- the encoder's building blocks (CompressBC7.hlsl:144-527) ----------------------------------------
+// rintf for |x| < 2^22 (and NaN): adding 1.5 * 2^23 leaves no room for a fraction, so the sum is x rounded half to even.
+__device__ __forceinline__ float RoundSmall(float x)
+{
+    return (x + 12582912.f) - 12582912.f;
+}
+
+// v / 255 for an integer v of 0 to 255, rounded as the division rounds it: one correction of the product with the
+// reciprocal (Markstein, IBM J. Res. Dev. 34, 1990; all 256 quotients compared with the division's).
+__device__ __forceinline__ float Over255(float v)
+{
+    constexpr float reciprocal = 1.f / 255.f;
+    const float quotient = v * reciprocal;
+    return __fmaf_rn(__fmaf_rn(-quotient, 255.f, v), reciprocal, quotient);
+}
+
 __device__ __forceinline__ int Quantize(float value, int bits)
 {
     const float scale = float((1u << bits) - 1u);
-    return int(rintf(Saturate(value) * scale));
+    return int(RoundSmall(Saturate(value) * scale));
 }
 
 __device__ __forceinline__ int ExpandTo8Bits(int q, int bits)
@@ -202,24 +282,21 @@ __device__ __forceinline__ int ExpandTo8Bits(int q, int bits)
     return (q << (8 - bits)) | (q >> (2 * bits - 8));
 }
 
-template <int C>
+template <int C, bool kAll>
 __device__ __forceinline__ void MinMax(const Pixels& pixels, uint32_t mask, Vec<C>& mins, Vec<C>& maxs)
 {
     mins = Splat<C>(FLT_MAX);
     maxs = Splat<C>(-FLT_MAX);
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        if ((mask >> i) & 1u)
-        {
-            const Vec<C> p = Pixel<C>(pixels, i);
-            mins = Min(mins, p);
-            maxs = Max(maxs, p);
-        }
+    ForEachPixel<kAll>(mask, [&](int i) {
+        const Vec<C> p = Pixel<C>(pixels, i);
+        mins = Min(mins, p);
+        maxs = Max(maxs, p);
+    });
 }
 
 // Two rounds of least squares on the endpoints for the indices the current endpoints give
 // (BC7_OptimizeEndpoints, :188-244); endpoint components at exactly 0 or 1 stay.
-template <int C>
+template <int C, bool kAll>
 __device__ void OptimizeEndpoints(const Pixels& pixels, uint32_t mask, Vec<C>& ep0, Vec<C>& ep1, int indexBits)
 {
 #pragma unroll 1
@@ -233,20 +310,17 @@ __device__ void OptimizeEndpoints(const Pixels& pixels, uint32_t mask, Vec<C>& e
         const float inverseScale = 1.0f / scale;
         float alpha2 = 0.f, beta2 = 0.f, alphaBeta = 0.f;
         Vec<C> alphaX = Splat<C>(0.f), betaX = Splat<C>(0.f);
-#pragma unroll 1
-        for (int i = 0; i < 16; ++i)
-            if ((mask >> i) & 1u)
-            {
-                const Vec<C> color = Pixel<C>(pixels, i);
-                const float index = Saturate(Dot(color - ep0, axis) * mul);
-                const float beta = rintf(index * scale) * inverseScale;
-                const float alpha = 1.0f - beta;
-                alpha2 += alpha * alpha;
-                beta2 += beta * beta;
-                alphaBeta += alpha * beta;
-                alphaX = alphaX + color * alpha;
-                betaX = betaX + color * beta;
-            }
+        ForEachPixel<kAll>(mask, [&](int i) {
+            const Vec<C> color = Pixel<C>(pixels, i);
+            const float index = MultiplySaturate(Dot(color - ep0, axis), mul);
+            const float beta = RoundSmall(index * scale) * inverseScale;
+            const float alpha = 1.0f - beta;
+            alpha2 += alpha * alpha;
+            beta2 += beta * beta;
+            alphaBeta += alpha * beta;
+            alphaX = alphaX + color * alpha;
+            betaX = betaX + color * beta;
+        });
         const float denominator = alpha2 * beta2 - alphaBeta * alphaBeta;
         if (!(fabsf(denominator) > 0.0001f))
             break;
@@ -254,8 +328,8 @@ __device__ void OptimizeEndpoints(const Pixels& pixels, uint32_t mask, Vec<C>& e
 #pragma unroll
         for (int c = 0; c < C; ++c)
         {
-            const float a = Saturate((alphaX.v[c] * beta2 - betaX.v[c] * alphaBeta) * factor);
-            const float b = Saturate((betaX.v[c] * alpha2 - alphaX.v[c] * alphaBeta) * factor);
+            const float a = MultiplySaturate(alphaX.v[c] * beta2 - betaX.v[c] * alphaBeta, factor);
+            const float b = MultiplySaturate(betaX.v[c] * alpha2 - alphaX.v[c] * alphaBeta, factor);
             if (!(ep0.v[c] == 0.0f || ep0.v[c] == 1.0f))
                 ep0.v[c] = a;
             if (!(ep1.v[c] == 0.0f || ep1.v[c] == 1.0f))
@@ -267,14 +341,11 @@ __device__ void OptimizeEndpoints(const Pixels& pixels, uint32_t mask, Vec<C>& e
 // Min / max endpoints put every component's low value in ep0; where two components run against each
 // other over the subset, one of them is swapped (BC7_SwapEndpointComponents_RGB / _RGBA, :248-345): the
 // first component with an extent is the reference, the later ones follow the sign of their covariance with it.
-template <int C>
+template <int C, bool kAll>
 __device__ void SwapEndpointComponents(const Pixels& pixels, uint32_t mask, Vec<C>& ep0, Vec<C>& ep1)
 {
     Vec<C> sum = Splat<C>(0.f);
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        if ((mask >> i) & 1u)
-            sum = sum + Pixel<C>(pixels, i);
+    ForEachPixel<kAll>(mask, [&](int i) { sum = sum + Pixel<C>(pixels, i); });
     const float count = float(__popc(mask));
     Vec<C> center;
 #pragma unroll
@@ -286,17 +357,14 @@ __device__ void SwapEndpointComponents(const Pixels& pixels, uint32_t mask, Vec<
 #pragma unroll
         for (int b = 0; b < C; ++b)
             covariance[a][b] = 0.f;
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        if ((mask >> i) & 1u)
-        {
-            const Vec<C> p = Pixel<C>(pixels, i) - center;
+    ForEachPixel<kAll>(mask, [&](int i) {
+        const Vec<C> p = Pixel<C>(pixels, i) - center;
 #pragma unroll
-            for (int a = 0; a < C; ++a)
+        for (int a = 0; a < C; ++a)
 #pragma unroll
-                for (int b = a + 1; b < C; ++b)
-                    covariance[a][b] += p.v[a] * p.v[b];
-        }
+            for (int b = a + 1; b < C; ++b)
+                covariance[a][b] += p.v[a] * p.v[b];
+    });
     bool done = false;
 #pragma unroll
     for (int a = 0; a + 1 < C; ++a)
@@ -314,92 +382,62 @@ __device__ void SwapEndpointComponents(const Pixels& pixels, uint32_t mask, Vec<
         }
 }
 
-// Squared error of the subset against the line between two unquantised endpoints, with the indices
-// rounded to `indexBits` but not clamped (BC7_EstimateError, :347-377).
-template <int C>
-__device__ float EstimateError(const Pixels& pixels, uint32_t mask, const Vec<C>& ep0, const Vec<C>& ep1, int indexBits)
-{
-    const Vec<C> axis = ep1 - ep0;
-    float mul = Dot(axis, axis);
-    if (mul > 0.0f)
-        mul = 1.0f / mul;
-    const float maxIndex = float((1u << indexBits) - 1u);
-    const float indexScale = 1.f / maxIndex;
-    float error = 0.f;
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        if ((mask >> i) & 1u)
-        {
-            const Vec<C> p = Pixel<C>(pixels, i) - ep0;
-            float index = Dot(p, axis) * mul;
-            index = rintf(index * maxIndex) * indexScale;
-            const Vec<C> difference = axis * index - p;
-            error += Dot(difference, difference);
-        }
-    return error;
-}
-
 // Indices of a subset's pixels, 4 bits per pixel in `indices`; true when the anchor's top bit was set and
 // all of the subset's indices were therefore inverted - the caller then swaps the endpoints
 // (BC7_CalculateIndices, :441-489; the anchor-0 form :493-527 gives the same indices).
-template <int C>
+// kError: `error` receives the squared error of the subset as a decoder reconstructs it (BC7_ComputeError, :379-412).
+// Inverting the indices and swapping the endpoints leaves that error as it is - the interpolation weights of index i and of
+// its inverse add up to 64 - so it is summed in the same walk over the pixels, before it is known whether they flip.
+template <int C, bool kAll, bool kError>
 __device__ bool CalculateIndices(const Pixels& pixels, uint32_t mask, int anchor, int indexBits, int endpointBits,
-    const int (&q0)[C], const int (&q1)[C], uint64_t& indices)
+    const int (&q0)[C], const int (&q1)[C], uint64_t& indices, float& error)
 {
     Vec<C> ep0, axis;
+    float base[C], extent[C]; // 64 * endpoint 0 + 32 and the 8-bit extent: the decoder's interpolation is floor((base + weight * extent) / 64)
 #pragma unroll
     for (int c = 0; c < C; ++c)
     {
-        ep0.v[c] = float(ExpandTo8Bits(q0[c], endpointBits)) / 255.0f;
-        axis.v[c] = float(ExpandTo8Bits(q1[c], endpointBits)) / 255.0f - ep0.v[c];
+        const float low = float(ExpandTo8Bits(q0[c], endpointBits)), high = float(ExpandTo8Bits(q1[c], endpointBits));
+        ep0.v[c] = Over255(low);
+        axis.v[c] = Over255(high) - ep0.v[c];
+        base[c] = low * 64.f + 32.f;
+        extent[c] = high - low;
     }
     float mul = Dot(axis, axis);
     if (mul > 0.0f)
         mul = 1.0f / mul;
+    const float maxIndex = float((1u << indexBits) - 1u);
+    const float weightScale = 64.f / maxIndex;
     uint64_t subsetIndices = 0, subsetMask = 0;
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        if ((mask >> i) & 1u)
-        {
-            const float index = Dot(Pixel<C>(pixels, i) - ep0, axis) * mul;
-            subsetIndices |= uint64_t(Quantize(index, indexBits)) << (4 * i);
+    float sum = 0.f;
+    ForEachPixel<kAll>(mask, [&](int i) {
+        const Vec<C> p = Pixel<C>(pixels, i);
+        const float index = RoundSmall(MultiplySaturate(Dot(p - ep0, axis), mul) * maxIndex);
+        subsetIndices |= uint64_t(uint32_t(int(index))) << (4 * i);
+        if (!kAll)
             subsetMask |= uint64_t((1u << indexBits) - 1u) << (4 * i);
+        if (kError)
+        {
+            const float weight = RoundSmall(index * weightScale); // 0..64
+            Vec<C> difference;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+            {
+                // floor(x / 64), x < 2^14: rounding x / 64 + 2^23 down drops the fraction
+                const float value = __fmaf_rd(__fmaf_rn(weight, extent[c], base[c]), 0.015625f, 8388608.f) - 8388608.f;
+                difference.v[c] = Over255(value) - p.v[c];
+            }
+            sum += Dot(difference, difference);
         }
+    });
+    if (kAll)
+        subsetMask = uint64_t((1u << indexBits) - 1u) * 0x1111111111111111ull;
     const bool flip = ((subsetIndices >> (4 * anchor)) >> (indexBits - 1)) & 1u;
     if (flip)
         subsetIndices ^= subsetMask;
     indices = (indices & ~subsetMask) | subsetIndices;
+    error = sum;
     return flip;
-}
-
-// Squared error of the subset as a decoder reconstructs it (BC7_ComputeError, :379-412).
-template <int C>
-__device__ float ComputeError(const Pixels& pixels, uint64_t indices, uint32_t mask, const int (&q0)[C], const int (&q1)[C],
-    int indexBits, int endpointBits)
-{
-    int e0[C], e1[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-    {
-        e0[c] = ExpandTo8Bits(q0[c], endpointBits);
-        e1[c] = ExpandTo8Bits(q1[c], endpointBits);
-    }
-    const float maxIndex = float((1u << indexBits) - 1u);
-    const float indexScale = 64.f / maxIndex;
-    float error = 0.f;
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        if ((mask >> i) & 1u)
-        {
-            const int weight = int(rintf(float(int(indices >> (4 * i)) & 15) * indexScale)); // 0..64
-            const Vec<C> p = Pixel<C>(pixels, i);
-            Vec<C> difference;
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                difference.v[c] = float((e0[c] * (64 - weight) + e1[c] * weight + 32) >> 6) / 255.0f - p.v[c];
-            error += Dot(difference, difference);
-        }
-    return error;
 }
 
 // ---- the 128 bits of a block ------------------------------------------------------------------------------
@@ -408,9 +446,9 @@ struct BlockBits
     uint64_t low = 0, high = 0;
     int offset = 0;
 
-    __device__ __forceinline__ void Put(int length, uint32_t value)
+    // `length` bits (the others of `bits` are zero)
+    __device__ __forceinline__ void Append(int length, uint64_t bits)
     {
-        const uint64_t bits = value & ((1u << length) - 1u);
         if (offset < 64)
         {
             low |= bits << offset;
@@ -421,11 +459,39 @@ struct BlockBits
             high |= bits << (offset - 64);
         offset += length;
     }
+    __device__ __forceinline__ void Put(int length, uint32_t value) { Append(length, value & ((1u << length) - 1u)); }
     __device__ __forceinline__ uint4 Words() const
     {
         return make_uint4(uint32_t(low), uint32_t(low >> 32), uint32_t(high), uint32_t(high >> 32));
     }
 };
+
+// Sixteen indices of kBits bits, one per nibble, moved together (a loop over the pixels with a 64-bit shift each cost more
+// than finding the indices).
+template <int kBits>
+__device__ __forceinline__ uint64_t JoinIndices(uint64_t x)
+{
+    if (kBits == 4)
+        return x;
+    constexpr int kGap = 4 - kBits; // every step joins two fields, whose gap doubles
+    constexpr uint64_t kField = (1u << kBits) - 1u;
+    constexpr uint64_t kNibbles = kField * 0x0101010101010101ull;
+    x = (x & kNibbles) | ((x >> kGap) & (kNibbles << kBits));
+    constexpr uint64_t kBytes = ((1u << (2 * kBits)) - 1u) * 0x0001000100010001ull;
+    x = (x & kBytes) | ((x >> (2 * kGap)) & (kBytes << (2 * kBits)));
+    constexpr uint64_t kShorts = ((1u << (4 * kBits)) - 1u) * 0x0000000100000001ull;
+    x = (x & kShorts) | ((x >> (4 * kGap)) & (kShorts << (4 * kBits)));
+    constexpr uint64_t kWord = (1ull << (8 * kBits)) - 1ull;
+    return (x & kWord) | ((x >> (8 * kGap)) & (kWord << (8 * kBits)));
+}
+
+// The index of an anchor pixel is stored without its top bit, which is zero: that bit is taken out.
+template <int kBits>
+__device__ __forceinline__ uint64_t DropAnchorBit(uint64_t joined, int pixel)
+{
+    const uint64_t below = (1ull << (kBits * pixel + kBits - 1)) - 1ull;
+    return (joined & below) | ((joined >> 1) & ~below);
+}
 
 // ---- modes 0-3, 6, 7: one colour plane, one to three subsets ------------------------------------------
 template <int kMode>
@@ -446,6 +512,55 @@ NTCB_BC7_MODE(6, 1, 4, 4, 8, 1, 0)
 NTCB_BC7_MODE(7, 2, 4, 2, 6, 1, 6)
 #undef NTCB_BC7_MODE
 
+// The p-bit of an endpoint with alpha: what most components end in, but 0 stays 0 and 1 stays 1
+// (BC7_RGBA_QuantizeEndpoint, :439-455).
+template <int C>
+__device__ __forceinline__ void ShareLowBit(int (&q)[C], float alpha)
+{
+    const bool majorityOdd = (q[0] & 1) + (q[1] & 1) + (q[2] & 1) + (q[C - 1] & 1) >= 2;
+    const int bit = ((majorityOdd && q[C - 1] != 0) || alpha == 1.0f) ? 1 : 0;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+        q[c] = (q[c] & 0xFE) | bit;
+}
+
+template <int kMode>
+__device__ __forceinline__ uint4 PackSinglePlane(int partition, const int (&anchor)[3],
+    const int (&q)[2 * ModeTraits<kMode>::kSubsets][ModeTraits<kMode>::kComponents], uint64_t indices)
+{
+    using Traits = ModeTraits<kMode>;
+    constexpr int C = Traits::kComponents, kSubsets = Traits::kSubsets, kIndexBits = Traits::kIndexBits, kEndpointBits = Traits::kEndpointBits;
+    BlockBits bits;
+    bits.Put(kMode + 1, 1u << kMode);
+    if (Traits::kPartitionBits)
+        bits.Put(Traits::kPartitionBits, uint32_t(partition));
+    constexpr int kStoredBits = Traits::kPBits ? kEndpointBits - 1 : kEndpointBits;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int i = 0; i < 2 * kSubsets; ++i)
+            bits.Put(kStoredBits, uint32_t(q[i][c]) >> (Traits::kPBits ? 1 : 0));
+    if (Traits::kPBits == 1)
+    {
+#pragma unroll
+        for (int i = 0; i < 2 * kSubsets; ++i)
+            bits.Put(1, uint32_t(q[i][0]));
+    }
+    else if (Traits::kPBits == 2)
+    {
+#pragma unroll
+        for (int s = 0; s < kSubsets; ++s)
+            bits.Put(1, uint32_t(q[2 * s][0]));
+    }
+    uint64_t joined = JoinIndices<kIndexBits>(indices);
+    if (kSubsets > 2) // the later pixel first: taking a bit out moves what is above it
+        joined = DropAnchorBit<kIndexBits>(joined, max(anchor[1], anchor[2]));
+    if (kSubsets > 1)
+        joined = DropAnchorBit<kIndexBits>(joined, kSubsets > 2 ? min(anchor[1], anchor[2]) : anchor[1]);
+    bits.Append(16 * kIndexBits - kSubsets, DropAnchorBit<kIndexBits>(joined, 0));
+    return bits.Words();
+}
+
 // Refines the endpoints found for a partition, quantises them, assigns indices and, when the block is no
 // worse than the best one so far, encodes it (BC7_Mode0_Finalize ... BC7_Mode3_Finalize, BC7_Mode6_Compress,
 // the second half of BC7_Mode7_Compress).  With a mode buffer there is nothing to compare: the error stays 0.
@@ -462,7 +577,7 @@ __device__ void FinalizeMode(const Pixels& pixels, int partition, const Subsets&
         ep[i] = endpoints[i];
 #pragma unroll
     for (int s = 0; s < kSubsets; ++s)
-        OptimizeEndpoints<C>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1], kIndexBits);
+        OptimizeEndpoints<C, kSubsets == 1>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1], kIndexBits);
 
     int q[2 * kSubsets][C];
 #pragma unroll
@@ -484,18 +599,9 @@ __device__ void FinalizeMode(const Pixels& pixels, int partition, const Subsets&
     }
     else if (Traits::kPBits == 1)
     {
-        // with alpha: 0 stays 0 and 1 stays 1 (BC7_RGBA_QuantizeEndpoint, :439-455)
 #pragma unroll
         for (int i = 0; i < 2 * kSubsets; ++i)
-        {
-            const bool majorityOdd = (q[i][0] & 1) + (q[i][1] & 1) + (q[i][2] & 1) + (q[i][C - 1] & 1) >= 2;
-            const bool alphaZero = q[i][C - 1] == 0;
-            const bool alphaOne = ep[i].v[C - 1] == 1.0f;
-            const int bit = ((majorityOdd && !alphaZero) || alphaOne) ? 1 : 0;
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                q[i][c] = (q[i][c] & 0xFE) | bit;
-        }
+            ShareLowBit<C>(q[i], ep[i].v[C - 1]);
     }
     else if (Traits::kPBits == 2)
     {
@@ -522,7 +628,9 @@ __device__ void FinalizeMode(const Pixels& pixels, int partition, const Subsets&
 #pragma unroll
     for (int s = 0; s < kSubsets; ++s)
     {
-        if (CalculateIndices<C>(pixels, subsets.mask[s], subsets.anchor[s], kIndexBits, kEndpointBits, q[2 * s], q[2 * s + 1], indices))
+        float subsetError;
+        if (CalculateIndices<C, kSubsets == 1, !kSingleMode>(pixels, subsets.mask[s], subsets.anchor[s], kIndexBits, kEndpointBits, q[2 * s],
+                q[2 * s + 1], indices, subsetError))
         {
 #pragma unroll
             for (int c = 0; c < C; ++c)
@@ -533,44 +641,13 @@ __device__ void FinalizeMode(const Pixels& pixels, int partition, const Subsets&
             }
         }
         if (!kSingleMode)
-        {
-            const float subsetError = ComputeError<C>(pixels, indices, subsets.mask[s], q[2 * s], q[2 * s + 1], kIndexBits, kEndpointBits);
             error = s == 0 ? subsetError : error + subsetError;
-        }
     }
     if (error > currentError)
         return;
 
-    BlockBits bits;
-    bits.Put(kMode + 1, 1u << kMode);
-    if (Traits::kPartitionBits)
-        bits.Put(Traits::kPartitionBits, uint32_t(partition));
-    constexpr int kStoredBits = Traits::kPBits ? kEndpointBits - 1 : kEndpointBits;
-#pragma unroll
-    for (int c = 0; c < C; ++c)
-#pragma unroll
-        for (int i = 0; i < 2 * kSubsets; ++i)
-            bits.Put(kStoredBits, uint32_t(q[i][c]) >> (Traits::kPBits ? 1 : 0));
-    if (Traits::kPBits == 1)
-    {
-#pragma unroll
-        for (int i = 0; i < 2 * kSubsets; ++i)
-            bits.Put(1, uint32_t(q[i][0]));
-    }
-    else if (Traits::kPBits == 2)
-    {
-#pragma unroll
-        for (int s = 0; s < kSubsets; ++s)
-            bits.Put(1, uint32_t(q[2 * s][0]));
-    }
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-    {
-        const bool anchor = i == 0 || (kSubsets > 1 && i == subsets.anchor[1]) || (kSubsets > 2 && i == subsets.anchor[2]);
-        bits.Put(anchor ? kIndexBits - 1 : kIndexBits, uint32_t(indices >> (4 * i)) & 15u);
-    }
     currentError = error;
-    currentBlock = bits.Words();
+    currentBlock = PackSinglePlane<kMode>(partition, subsets.anchor, q, indices);
 }
 
 // The endpoints a partition starts from: per subset the extremes of each component, components swapped
@@ -581,77 +658,81 @@ __device__ __forceinline__ void StartingEndpoints(const Pixels& pixels, const Su
 #pragma unroll
     for (int s = 0; s < kSubsets; ++s)
     {
-        MinMax<C>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1]);
+        MinMax<C, kSubsets == 1>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1]);
         if (kSwap)
-            SwapEndpointComponents<C>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1]);
+            SwapEndpointComponents<C, kSubsets == 1>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1]);
     }
-}
-
-// The partition of `kSubsets` subsets with the smallest estimated error (the first one on ties) and its
-// starting endpoints (the loops of BC7_Mode0_2_Compress :724-775, BC7_Mode1_3_Compress :930-979,
-// BC7_Mode7_Compress :1296-1335).
-template <int C, int kSubsets, bool kSwap>
-__device__ int SearchPartitions(const Pixels& pixels, int searchIndexBits, Vec<C>* bestEndpoints)
-{
-    int best = 0;
-    float bestError = FLT_MAX;
-#pragma unroll 1
-    for (int partition = 0; partition < 64; ++partition)
-    {
-        const Subsets subsets = kSubsets == 3 ? ThreeSubsets(partition) : TwoSubsets(partition);
-        Vec<C> ep[2 * kSubsets];
-        StartingEndpoints<C, kSubsets, kSwap>(pixels, subsets, ep);
-        float error = 0.f;
-#pragma unroll
-        for (int s = 0; s < kSubsets; ++s)
-        {
-            const float subsetError = EstimateError<C>(pixels, subsets.mask[s], ep[2 * s], ep[2 * s + 1], searchIndexBits);
-            error = s == 0 ? subsetError : error + subsetError;
-        }
-        if (error < bestError)
-        {
-            best = partition;
-            bestError = error;
-#pragma unroll
-            for (int i = 0; i < 2 * kSubsets; ++i)
-                bestEndpoints[i] = ep[i];
-        }
-    }
-    return best;
 }
 
 // ---- modes 4 and 5: a colour plane and a scalar plane with indices of their own ----------------------
 // mode 4: 5-bit colours, 6-bit scalar, 2- and 3-bit indices (kSelector: the colours get the 3-bit ones);
 // mode 5: 7-bit colours, 8-bit scalar, 2-bit indices for both.  (BC7_Mode4_Compress_Internal :982-1069,
 // BC7_Mode5_Compress_Internal :1071-1147.)
-template <int kMode, bool kSelector, bool kSingleMode>
-__device__ void EncodeDualPlane(const Pixels& pixels, float& currentError, uint4& currentBlock)
+template <int kMode, bool kSelector>
+struct DualPlaneTraits
 {
-    constexpr int kColorIndexBits = kMode == 5 ? 2 : kSelector ? 3 : 2;
-    constexpr int kScalarIndexBits = kMode == 5 ? 2 : kSelector ? 2 : 3;
-    constexpr int kColorBits = kMode == 5 ? 7 : 5, kScalarBits = kMode == 5 ? 8 : 6;
+    static constexpr int kColorIndexBits = kMode == 5 ? 2 : kSelector ? 3 : 2, kScalarIndexBits = kMode == 5 ? 2 : kSelector ? 2 : 3,
+                         kColorBits = kMode == 5 ? 7 : 5, kScalarBits = kMode == 5 ? 8 : 6;
+};
 
+template <int kMode, bool kSelector>
+__device__ uint4 PackDualPlane(int rotation, const int (&q0)[3], const int (&q1)[3], int a0, int a1, uint64_t colorIndices, uint64_t scalarIndices)
+{
+    using Traits = DualPlaneTraits<kMode, kSelector>;
+    BlockBits bits;
+    bits.Put(kMode + 1, 1u << kMode);
+    bits.Put(2, uint32_t(rotation));
+    if (kMode == 4)
+        bits.Put(1, kSelector ? 1u : 0u);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+        bits.Put(Traits::kColorBits, uint32_t(q0[c]));
+        bits.Put(Traits::kColorBits, uint32_t(q1[c]));
+    }
+    bits.Put(Traits::kScalarBits, uint32_t(a0));
+    bits.Put(Traits::kScalarBits, uint32_t(a1));
+    const uint64_t colors = DropAnchorBit<Traits::kColorIndexBits>(JoinIndices<Traits::kColorIndexBits>(colorIndices), 0);
+    const uint64_t scalars = DropAnchorBit<Traits::kScalarIndexBits>(JoinIndices<Traits::kScalarIndexBits>(scalarIndices), 0);
+    // mode 4 stores its 2-bit indices first, whichever plane they belong to; mode 5 colours, then scalar
+    if (kMode == 4 && kSelector)
+    {
+        bits.Append(16 * Traits::kScalarIndexBits - 1, scalars);
+        bits.Append(16 * Traits::kColorIndexBits - 1, colors);
+    }
+    else
+    {
+        bits.Append(16 * Traits::kColorIndexBits - 1, colors);
+        bits.Append(16 * Traits::kScalarIndexBits - 1, scalars);
+    }
+    return bits.Words();
+}
+
+// The one dual-plane configuration a mode buffer names.
+template <int kMode, bool kSelector>
+__device__ uint4 EncodeDualPlane(const Pixels& pixels)
+{
+    using Traits = DualPlaneTraits<kMode, kSelector>;
     Vec<1> s0, s1;
-    MinMax<1>(pixels, kAllPixels, s0, s1);
-    OptimizeEndpoints<1>(pixels, kAllPixels, s0, s1, kScalarIndexBits);
+    MinMax<1, true>(pixels, kAllPixels, s0, s1);
+    OptimizeEndpoints<1, true>(pixels, kAllPixels, s0, s1, Traits::kScalarIndexBits);
     Vec<3> c0, c1;
-    MinMax<3>(pixels, kAllPixels, c0, c1);
-    SwapEndpointComponents<3>(pixels, kAllPixels, c0, c1);
-    OptimizeEndpoints<3>(pixels, kAllPixels, c0, c1, kColorIndexBits);
-
+    MinMax<3, true>(pixels, kAllPixels, c0, c1);
+    SwapEndpointComponents<3, true>(pixels, kAllPixels, c0, c1);
+    OptimizeEndpoints<3, true>(pixels, kAllPixels, c0, c1, Traits::kColorIndexBits);
     int q0[3], q1[3], a0[1], a1[1];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
     {
-        q0[c] = Quantize(c0.v[c], kColorBits);
-        q1[c] = Quantize(c1.v[c], kColorBits);
+        q0[c] = Quantize(c0.v[c], Traits::kColorBits);
+        q1[c] = Quantize(c1.v[c], Traits::kColorBits);
     }
-    a0[0] = Quantize(s0.v[0], kScalarBits);
-    a1[0] = Quantize(s1.v[0], kScalarBits);
+    a0[0] = Quantize(s0.v[0], Traits::kScalarBits);
+    a1[0] = Quantize(s1.v[0], Traits::kScalarBits);
 
     uint64_t colorIndices = 0, scalarIndices = 0;
-    float error = 0.f;
-    if (CalculateIndices<3>(pixels, kAllPixels, 0, kColorIndexBits, kColorBits, q0, q1, colorIndices))
+    float ignored;
+    if (CalculateIndices<3, true, false>(pixels, kAllPixels, 0, Traits::kColorIndexBits, Traits::kColorBits, q0, q1, colorIndices, ignored))
     {
 #pragma unroll
         for (int c = 0; c < 3; ++c)
@@ -661,44 +742,13 @@ __device__ void EncodeDualPlane(const Pixels& pixels, float& currentError, uint4
             q1[c] = t;
         }
     }
-    if (!kSingleMode)
-        error = ComputeError<3>(pixels, colorIndices, kAllPixels, q0, q1, kColorIndexBits, kColorBits);
-    if (CalculateIndices<1>(pixels, kAllPixels, 0, kScalarIndexBits, kScalarBits, a0, a1, scalarIndices))
+    if (CalculateIndices<1, true, false>(pixels, kAllPixels, 0, Traits::kScalarIndexBits, Traits::kScalarBits, a0, a1, scalarIndices, ignored))
     {
         const int t = a0[0];
         a0[0] = a1[0];
         a1[0] = t;
     }
-    if (!kSingleMode)
-        error += ComputeError<1>(pixels, scalarIndices, kAllPixels, a0, a1, kScalarIndexBits, kScalarBits);
-    if (error > currentError)
-        return;
-
-    BlockBits bits;
-    bits.Put(kMode + 1, 1u << kMode);
-    bits.Put(2, uint32_t(pixels.rotation));
-    if (kMode == 4)
-        bits.Put(1, kSelector ? 1u : 0u);
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-        bits.Put(kColorBits, uint32_t(q0[c]));
-        bits.Put(kColorBits, uint32_t(q1[c]));
-    }
-    bits.Put(kScalarBits, uint32_t(a0[0]));
-    bits.Put(kScalarBits, uint32_t(a1[0]));
-    // mode 4 stores its 2-bit indices first, whichever plane they belong to; mode 5 colours, then scalar
-    const bool scalarFirst = kMode == 4 && kSelector;
-    const uint64_t first = scalarFirst ? scalarIndices : colorIndices, second = scalarFirst ? colorIndices : scalarIndices;
-    const int firstBits = scalarFirst ? kScalarIndexBits : kColorIndexBits, secondBits = scalarFirst ? kColorIndexBits : kScalarIndexBits;
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        bits.Put(i == 0 ? firstBits - 1 : firstBits, uint32_t(first >> (4 * i)) & 15u);
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i)
-        bits.Put(i == 0 ? secondBits - 1 : secondBits, uint32_t(second >> (4 * i)) & 15u);
-    currentError = error;
-    currentBlock = bits.Words();
+    return PackDualPlane<kMode, kSelector>(pixels.rotation, q0, q1, a0[0], a1[0], colorIndices, scalarIndices);
 }
 
 // ---- the kernel -----------------------------------------------------------------------------------------
@@ -742,126 +792,98 @@ __device__ __forceinline__ bool LoadModeAndPartition(const Bc7Arguments& args, i
     return true;
 }
 
-// One block: with a mode buffer the one configuration it names, otherwise the best of all
-// (CompressBC7.hlsl main(), :1548-1587).  texels: the block's texel i at texels[i * kThreads].
-template <bool kSingleMode>
-__device__ uint4 EncodeBlock(const uint2* texels, uint32_t mode, uint32_t partition)
+// One block in the one configuration its mode-buffer entry names (CompressBC7.hlsl main(), :1548-1587).
+// texels: the block's texel i at texels[i * kThreads].
+__device__ uint4 EncodeInMode(const uint2* texels, uint32_t mode, uint32_t partition)
 {
     Pixels pixels;
     pixels.base = texels;
     pixels.rotation = 0;
+    pixels.stride = kThreads;
     float error = FLT_MAX;
     uint4 block = make_uint4(0u, 0u, 0u, 0u);
 
-    if (kSingleMode)
+    switch (mode)
     {
-        switch (mode)
-        {
-        case 0:
-        case 2:
-        {
-            const Subsets subsets = ThreeSubsets(int(partition));
-            Vec<3> ep[6];
-            StartingEndpoints<3, 3, true>(pixels, subsets, ep);
-            if (mode == 0)
-                FinalizeMode<0, true>(pixels, int(partition), subsets, ep, error, block);
-            else
-                FinalizeMode<2, true>(pixels, int(partition), subsets, ep, error, block);
-            break;
-        }
-        case 1:
-        case 3:
-        {
-            const Subsets subsets = TwoSubsets(int(partition));
-            Vec<3> ep[4];
-            StartingEndpoints<3, 2, true>(pixels, subsets, ep);
-            if (mode == 1)
-                FinalizeMode<1, true>(pixels, int(partition), subsets, ep, error, block);
-            else
-                FinalizeMode<3, true>(pixels, int(partition), subsets, ep, error, block);
-            break;
-        }
-        case 4:
-        case 5:
-            // the partition field of these modes: rotation in bits 0-1, mode 4's index selector in bit 2
-            pixels.rotation = int(partition & 3u);
-            if (mode == 5)
-                EncodeDualPlane<5, false, true>(pixels, error, block);
-            else if (partition & 4u)
-                EncodeDualPlane<4, true, true>(pixels, error, block);
-            else
-                EncodeDualPlane<4, false, true>(pixels, error, block);
-            break;
-        case 6:
-        {
-            const Subsets subsets = {{kAllPixels, 0u, 0u}, {0, 0, 0}};
-            Vec<4> ep[2];
-            StartingEndpoints<4, 1, true>(pixels, subsets, ep);
-            FinalizeMode<6, true>(pixels, 0, subsets, ep, error, block);
-            break;
-        }
-        default:
-        {
-            const Subsets subsets = TwoSubsets(int(partition));
-            Vec<4> ep[4];
-            StartingEndpoints<4, 2, false>(pixels, subsets, ep);
-            FinalizeMode<7, true>(pixels, int(partition), subsets, ep, error, block);
-            break;
-        }
-        }
+    case 0:
+    case 2:
+    {
+        const Subsets subsets = ThreeSubsets(int(partition));
+        Vec<3> ep[6];
+        StartingEndpoints<3, 3, true>(pixels, subsets, ep);
+        if (mode == 0)
+            FinalizeMode<0, true>(pixels, int(partition), subsets, ep, error, block);
+        else
+            FinalizeMode<2, true>(pixels, int(partition), subsets, ep, error, block);
+        break;
     }
-    else
+    case 1:
+    case 3:
     {
-        // the three-component modes cannot hold alpha: only for blocks without a texel of alpha < 1
-        bool opaque = true;
-#pragma unroll 1
-        for (int i = 0; i < 16; ++i)
-            if (Pixel<4>(pixels, i).v[3] < 1.0f)
-                opaque = false;
-        if (opaque)
-        {
-            {
-                Vec<3> ep[6];
-                const int best = SearchPartitions<3, 3, true>(pixels, 3, ep);
-                const Subsets subsets = ThreeSubsets(best);
-                if (best < 16)
-                    FinalizeMode<0, false>(pixels, best, subsets, ep, error, block);
-                FinalizeMode<2, false>(pixels, best, subsets, ep, error, block);
-            }
-            {
-                Vec<3> ep[4];
-                const int best = SearchPartitions<3, 2, true>(pixels, 3, ep);
-                const Subsets subsets = TwoSubsets(best);
-                FinalizeMode<1, false>(pixels, best, subsets, ep, error, block);
-                FinalizeMode<3, false>(pixels, best, subsets, ep, error, block);
-            }
-        }
-#pragma unroll 1
-        for (int rotation = 0; rotation < 4; ++rotation)
-        {
-            pixels.rotation = rotation;
-            EncodeDualPlane<4, false, false>(pixels, error, block);
-            EncodeDualPlane<4, true, false>(pixels, error, block);
-            EncodeDualPlane<5, false, false>(pixels, error, block);
-        }
-        pixels.rotation = 0;
-        {
-            const Subsets subsets = {{kAllPixels, 0u, 0u}, {0, 0, 0}};
-            Vec<4> ep[2];
-            StartingEndpoints<4, 1, true>(pixels, subsets, ep);
-            FinalizeMode<6, false>(pixels, 0, subsets, ep, error, block);
-        }
-        {
-            Vec<4> ep[4];
-            const int best = SearchPartitions<4, 2, false>(pixels, 2, ep);
-            FinalizeMode<7, false>(pixels, best, TwoSubsets(best), ep, error, block);
-        }
+        const Subsets subsets = TwoSubsets(int(partition));
+        Vec<3> ep[4];
+        StartingEndpoints<3, 2, true>(pixels, subsets, ep);
+        if (mode == 1)
+            FinalizeMode<1, true>(pixels, int(partition), subsets, ep, error, block);
+        else
+            FinalizeMode<3, true>(pixels, int(partition), subsets, ep, error, block);
+        break;
+    }
+    case 4:
+    case 5:
+        // the partition field of these modes: rotation in bits 0-1, mode 4's index selector in bit 2
+        pixels.rotation = int(partition & 3u);
+        if (mode == 5)
+            block = EncodeDualPlane<5, false>(pixels);
+        else if (partition & 4u)
+            block = EncodeDualPlane<4, true>(pixels);
+        else
+            block = EncodeDualPlane<4, false>(pixels);
+        break;
+    case 6:
+    {
+        const Subsets subsets = {{kAllPixels, 0u, 0u}, {0, 0, 0}};
+        Vec<4> ep[2];
+        StartingEndpoints<4, 1, true>(pixels, subsets, ep);
+        FinalizeMode<6, true>(pixels, 0, subsets, ep, error, block);
+        break;
+    }
+    default:
+    {
+        const Subsets subsets = TwoSubsets(int(partition));
+        Vec<4> ep[4];
+        StartingEndpoints<4, 2, false>(pixels, subsets, ep);
+        FinalizeMode<7, true>(pixels, int(partition), subsets, ep, error, block);
+        break;
+    }
     }
     return block;
 }
 
-template <bool kSingleMode>
-__global__ void __launch_bounds__(kThreads) Bc7Kernel(const Bc7Arguments args)
+// One texel as two words of halves, red-green and blue-alpha; missing channels read 0, alpha 1, and outside the mip
+// every component reads 0.
+__device__ __forceinline__ uint2 LoadTexel(const Bc7Arguments& args, int x, int y)
+{
+    if (x >= args.base.width || y >= args.base.height)
+        return make_uint2(0u, 0u);
+    const int first = args.base.firstChannel, count = args.numChannels;
+    if (!(first & 1) && !(args.base.channels & 1)) // channel pairs are aligned words in both layouts
+    {
+        const uint32_t redGreen = count >= 2 ? LoadPair(args.base, x, y, first) : uint32_t(__half_as_ushort(LoadHalf(args.base, x, y, first)));
+        const uint32_t blueAlpha = count == 4 ? LoadPair(args.base, x, y, first + 2)
+                                 : (count == 3 ? uint32_t(__half_as_ushort(LoadHalf(args.base, x, y, first + 2))) : 0u) | 0x3c000000u;
+        return make_uint2(redGreen, blueAlpha);
+    }
+    uint32_t c[4] = {0u, 0u, 0u, 0x3c00u};
+#pragma unroll
+    for (int channel = 0; channel < 4; ++channel)
+        if (channel < count)
+            c[channel] = __half_as_ushort(LoadHalf(args.base, x, y, first + channel));
+    return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
+}
+
+// With a mode buffer: one thread per block, 32 x 8 blocks per CTA.
+__global__ void __launch_bounds__(kThreads) Bc7ModeKernel(const Bc7Arguments args)
 {
     __shared__ uint2 staged[16 * kThreads];
     __shared__ uint32_t binCount[2 * kThreads + 1]; // blocks per (mode, partition) pair, then where each pair's blocks start
@@ -869,45 +891,20 @@ __global__ void __launch_bounds__(kThreads) Bc7Kernel(const Bc7Arguments args)
     __shared__ uint32_t order[kThreads];
 
     const int tid = threadIdx.x;
-    if (kSingleMode)
-    {
-        binCount[tid] = 0;
-        binCount[tid + kThreads] = 0;
-        if (tid == 0)
-            binCount[2 * kThreads] = 0;
-    }
+    binCount[tid] = 0;
+    binCount[tid + kThreads] = 0;
+    if (tid == 0)
+        binCount[2 * kThreads] = 0;
     // The CTA's 128 x 32 texels, neighbouring threads on neighbouring texels of a row, handed to the slot of
     // their block through shared memory; red-green and blue-alpha as two 32-bit words.
-    const bool pairs = !(args.base.firstChannel & 1) && !(args.base.channels & 1);
 #pragma unroll 1
     for (int k = 0; k < 16; ++k)
     {
         const int p = k * kThreads + tid;
         const int localX = p & (4 * kGroupWidth - 1), localY = p / (4 * kGroupWidth);
-        const int x = args.base.srcLeft + blockIdx.x * (4 * kGroupWidth) + localX, y = args.base.srcTop + blockIdx.y * (4 * kGroupHeight) + localY;
-        uint32_t redGreen = 0u, blueAlpha = 0u; // outside the mip every component reads 0
-        if (x < args.base.width && y < args.base.height)
-        {
-            const int first = args.base.firstChannel, count = args.numChannels;
-            if (pairs)
-            {
-                redGreen = count >= 2 ? LoadPair(args.base, x, y, first) : uint32_t(__half_as_ushort(LoadHalf(args.base, x, y, first)));
-                blueAlpha = count == 4 ? LoadPair(args.base, x, y, first + 2)
-                          : (count == 3 ? uint32_t(__half_as_ushort(LoadHalf(args.base, x, y, first + 2))) : 0u) | 0x3c000000u;
-            }
-            else
-            {
-                uint32_t c[4] = {0u, 0u, 0u, 0x3c00u};
-#pragma unroll
-                for (int channel = 0; channel < 4; ++channel)
-                    if (channel < count)
-                        c[channel] = __half_as_ushort(LoadHalf(args.base, x, y, first + channel));
-                redGreen = c[0] | (c[1] << 16);
-                blueAlpha = c[2] | (c[3] << 16);
-            }
-        }
         const int owner = (localY >> 2) * kGroupWidth + (localX >> 2), texel = (localY & 3) * 4 + (localX & 3);
-        staged[texel * kThreads + owner] = make_uint2(redGreen, blueAlpha);
+        staged[texel * kThreads + owner] = LoadTexel(args, args.base.srcLeft + blockIdx.x * (4 * kGroupWidth) + localX,
+            args.base.srcTop + blockIdx.y * (4 * kGroupHeight) + localY);
     }
 
     int slot = tid;
@@ -917,61 +914,953 @@ __global__ void __launch_bounds__(kThreads) Bc7Kernel(const Bc7Arguments args)
         const int blockX = blockIdx.x * kGroupWidth + (tid & (kGroupWidth - 1));
         const int blockY = blockIdx.y * kGroupHeight + tid / kGroupWidth;
         active = blockX < args.base.widthInBlocks && blockY < args.base.heightInBlocks;
-        if (kSingleMode)
+        if (active && !LoadModeAndPartition(args, blockX, blockY, mode, partition))
         {
-            if (active && !LoadModeAndPartition(args, blockX, blockY, mode, partition))
-            {
-                reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = MissingModeBlock();
-                active = false;
-            }
-            // Threads trade blocks so that those of one mode AND partition sit next to each other: a warp then
-            // runs one encoder, and its lanes loop over the same subsets (sorted by mode alone, as the shader
-            // does, half of the lanes idle in the pixel loops: 16 active lanes per instruction).  A counting
-            // sort over the 512 (mode, partition) pairs, blocks without work last.
-            __syncthreads();
-            const uint32_t key = active ? (mode << 6 | partition) : 512u;
-            const uint32_t rank = atomicAdd(&binCount[key], 1u);
-            __syncthreads();
-            {
-                // exclusive prefix sum of the bins: two per thread, scanned within the warp, then over the warps
-                const uint32_t first = binCount[2 * tid], second = binCount[2 * tid + 1], pair = first + second;
-                uint32_t inclusive = pair;
-#pragma unroll
-                for (int delta = 1; delta < 32; delta *= 2)
-                {
-                    const uint32_t below = __shfl_up_sync(0xFFFFFFFFu, inclusive, delta);
-                    if ((tid & 31) >= delta)
-                        inclusive += below;
-                }
-                if ((tid & 31) == 31)
-                    warpTotal[tid >> 5] = inclusive;
-                __syncthreads();
-                uint32_t start = inclusive - pair;
-                for (int w = 0; w < (tid >> 5); ++w)
-                    start += warpTotal[w];
-                binCount[2 * tid] = start;
-                binCount[2 * tid + 1] = start + first;
-                if (tid == kThreads - 1)
-                    binCount[512] = start + pair;
-            }
-            __syncthreads();
-            order[binCount[key] + rank] = uint32_t(tid) | (partition << 16) | ((active ? mode : 8u) << 24);
-            __syncthreads();
-            const uint32_t task = order[tid];
-            slot = int(task & 0xffffu);
-            partition = (task >> 16) & 0x3fu;
-            mode = task >> 24;
-            active = mode < 8u;
+            reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = MissingModeBlock();
+            active = false;
         }
-        else
+        // Threads trade blocks so that those of one mode AND partition sit next to each other: a warp then
+        // runs one encoder, and its lanes loop over the same subsets (sorted by mode alone, as the shader
+        // does, half of the lanes idle in the pixel loops: 16 active lanes per instruction).  A counting
+        // sort over the 512 (mode, partition) pairs, blocks without work last.
+        __syncthreads();
+        const uint32_t key = active ? (mode << 6 | partition) : 512u;
+        const uint32_t rank = atomicAdd(&binCount[key], 1u);
+        __syncthreads();
+        {
+            // exclusive prefix sum of the bins: two per thread, scanned within the warp, then over the warps
+            const uint32_t first = binCount[2 * tid], second = binCount[2 * tid + 1], pair = first + second;
+            uint32_t inclusive = pair;
+#pragma unroll
+            for (int delta = 1; delta < 32; delta *= 2)
+            {
+                const uint32_t below = __shfl_up_sync(0xFFFFFFFFu, inclusive, delta);
+                if ((tid & 31) >= delta)
+                    inclusive += below;
+            }
+            if ((tid & 31) == 31)
+                warpTotal[tid >> 5] = inclusive;
             __syncthreads();
+            uint32_t start = inclusive - pair;
+            for (int w = 0; w < (tid >> 5); ++w)
+                start += warpTotal[w];
+            binCount[2 * tid] = start;
+            binCount[2 * tid + 1] = start + first;
+            if (tid == kThreads - 1)
+                binCount[512] = start + pair;
+        }
+        __syncthreads();
+        order[binCount[key] + rank] = uint32_t(tid) | (partition << 16) | ((active ? mode : 8u) << 24);
+        __syncthreads();
+        const uint32_t task = order[tid];
+        slot = int(task & 0xffffu);
+        partition = (task >> 16) & 0x3fu;
+        mode = task >> 24;
+        active = mode < 8u;
     }
     if (!active)
         return;
 
-    const uint4 block = EncodeBlock<kSingleMode>(staged + slot, mode, partition);
+    const uint4 block = EncodeInMode(staged + slot, mode, partition);
     const int blockX = blockIdx.x * kGroupWidth + (slot & (kGroupWidth - 1));
     const int blockY = blockIdx.y * kGroupHeight + slot / kGroupWidth;
+    reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = block;
+}
+
+// ---- full search ------------------------------------------------------------------------------------------
+//
+// A CTA of eight warps searches 64 blocks.  The partition searches - 64 partitions of modes 0 / 2, 1 / 3 and 7 each, five
+// sixths of the arithmetic - go over all blocks at once: every warp tries every eighth partition on all 64 blocks, a thread
+// on two of them, block `lane` and block `lane + 32`, in the two halves of packed binary32 instructions (add / mul / fma
+// .f32x2: the same IEEE operations, two per issue slot).  The partition is the same for the whole warp, so its pixel lists
+// are too.  What follows - refining and encoding the best partition of each kind, the dual-plane modes under four
+// rotations, mode 6 - is eight independent tasks per block, a warp each per 32 blocks; the block with the smallest error is
+// picked at the end, in the shader's order.
+//
+// With one thread per block for everything a 1024 x 1024 image was 2048 warps of 800 k instructions, 14 resident per SM:
+// 1.81 ms.  Eight warps per 64 blocks and packed arithmetic fill the machine from a few thousand blocks up: 0.52 ms, bound by
+// the FMA pipe (61 % of its cycles) and instruction issue (67 %), three CTAs of 80 registers per SM (four of 64 spill in the
+// tasks: 3 % slower).
+constexpr int kSearchWarps = 8;
+constexpr int kSearchThreads = 32 * kSearchWarps;
+constexpr int kSearchWidth = 16, kSearchHeight = 4; // blocks per CTA
+constexpr int kSearchBlocks = kSearchWidth * kSearchHeight;
+constexpr int kSearchTasks = 8;
+
+// Two binary32 values: of blocks `lane` and `lane + 32`.
+struct Pair
+{
+    unsigned long long bits;
+};
+
+__device__ __forceinline__ Pair MakePair(float first, float second)
+{
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.bits) : "f"(first), "f"(second));
+    return r;
+}
+__device__ __forceinline__ Pair Both(float v) { return MakePair(v, v); }
+__device__ __forceinline__ void Split(Pair p, float& first, float& second)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(first), "=f"(second) : "l"(p.bits));
+}
+__device__ __forceinline__ Pair operator*(Pair a, Pair b)
+{
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.bits) : "l"(a.bits), "l"(b.bits));
+    return r;
+}
+__device__ __forceinline__ Pair MultiplyAdd(Pair a, Pair b, Pair c)
+{
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.bits) : "l"(a.bits), "l"(b.bits), "l"(c.bits));
+    return r;
+}
+__device__ __forceinline__ Pair Negate(Pair a)
+{
+    float x, y;
+    Split(a, x, y);
+    return MakePair(-x, -y);
+}
+// Sums are multiply-adds with factors of 1 and -1 (an exact product: one rounding, the sum's).  The factors come from
+// constant memory, so that they are not known at compile time: written as add.rn.f32x2, a sum is fused with the packed
+// multiplication before it, whatever --fmad says, and the candidates' errors come out with other roundings.
+__constant__ float2 kOne = {1.f, 1.f};
+__constant__ float2 kMinusOne = {-1.f, -1.f};
+__device__ __forceinline__ Pair operator+(Pair a, Pair b) { return MultiplyAdd(a, MakePair(kOne.x, kOne.y), b); }
+// a + b where neither is a product
+__device__ __forceinline__ Pair PlainAdd(Pair a, Pair b)
+{
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.bits) : "l"(a.bits), "l"(b.bits));
+    return r;
+}
+__device__ __forceinline__ Pair operator-(Pair a, Pair b) { return MultiplyAdd(b, MakePair(kMinusOne.x, kMinusOne.y), a); }
+__device__ __forceinline__ Pair RoundSmall(Pair x) { return PlainAdd(x + Both(12582912.f), Both(-12582912.f)); }
+
+// ---- the searches' whole-block parts on two blocks at once ------------------------------------------------
+// Modes 4, 5 and 6 have one subset, the whole block, so both blocks of a thread walk the same pixels and the packed
+// instructions serve here too.
+
+// Component planes of the staged texels, in the order the rotation gives them.
+struct PairPixels
+{
+    const float2* plane[4]; // texel i of a lane's two blocks at plane[c][i * 32]
+};
+
+template <int C>
+struct PairVec
+{
+    Pair v[C];
+};
+
+// C = 1: the scalar plane, otherwise the first C components.
+template <int C>
+__device__ __forceinline__ PairVec<C> PairPixel(const PairPixels& pixels, int i)
+{
+    PairVec<C> r;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        const float2 value = pixels.plane[C == 1 ? 3 : c][i * 32];
+        r.v[c] = MakePair(value.x, value.y);
+    }
+    return r;
+}
+
+template <int C>
+__device__ __forceinline__ Pair Dot(const PairVec<C>& a, const PairVec<C>& b)
+{
+    Pair sum = a.v[0] * b.v[0];
+#pragma unroll
+    for (int c = 1; c < C; ++c)
+        sum = sum + a.v[c] * b.v[c];
+    return sum;
+}
+template <int C>
+__device__ __forceinline__ PairVec<C> operator-(const PairVec<C>& a, const PairVec<C>& b)
+{
+    PairVec<C> r;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+        r.v[c] = a.v[c] - b.v[c];
+    return r;
+}
+
+// Applies f(first, second, ...) to both halves of its arguments.
+template <typename F>
+__device__ __forceinline__ Pair PerBlock(Pair a, F&& f)
+{
+    float x, y;
+    Split(a, x, y);
+    return MakePair(f(x), f(y));
+}
+template <typename F>
+__device__ __forceinline__ Pair PerBlock(Pair a, Pair b, F&& f)
+{
+    float ax, ay, bx, by;
+    Split(a, ax, ay);
+    Split(b, bx, by);
+    return MakePair(f(ax, bx), f(ay, by));
+}
+__device__ __forceinline__ Pair Min(Pair a, Pair b)
+{
+    return PerBlock(a, b, [](float x, float y) { return fminf(x, y); });
+}
+__device__ __forceinline__ Pair Max(Pair a, Pair b)
+{
+    return PerBlock(a, b, [](float x, float y) { return fmaxf(x, y); });
+}
+__device__ __forceinline__ Pair MultiplySaturate(Pair a, Pair b)
+{
+    return PerBlock(a, b, [](float x, float y) { return MultiplySaturate(x, y); });
+}
+
+// SwapEndpointComponents of the whole block, given the sums of its components.
+template <int C>
+__device__ __forceinline__ void OrientEndpoints(const PairPixels& pixels, const PairVec<C>& sum, PairVec<C>& ep0, PairVec<C>& ep1)
+{
+    PairVec<C> center;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+        center.v[c] = sum.v[c] * Both(0.0625f); // the sixteenth is exact
+    Pair covariance[C][C];
+#pragma unroll
+    for (int a = 0; a < C; ++a)
+#pragma unroll
+        for (int b = 0; b < C; ++b)
+            covariance[a][b] = Both(0.f);
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+    {
+        const PairVec<C> p = PairPixel<C>(pixels, i) - center;
+#pragma unroll
+        for (int a = 0; a < C; ++a)
+#pragma unroll
+            for (int b = a + 1; b < C; ++b)
+                covariance[a][b] = covariance[a][b] + p.v[a] * p.v[b];
+    }
+    float low[C][2], high[C][2];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        Split(ep0.v[c], low[c][0], low[c][1]);
+        Split(ep1.v[c], high[c][0], high[c][1]);
+    }
+    bool done[2] = {false, false};
+#pragma unroll
+    for (int a = 0; a + 1 < C; ++a)
+    {
+        bool reference[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+        {
+            reference[k] = !done[k] && low[a][k] != high[a][k];
+            done[k] = done[k] || reference[k];
+        }
+#pragma unroll
+        for (int b = a + 1; b < C; ++b)
+        {
+            float sign[2];
+            Split(covariance[a][b], sign[0], sign[1]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+            {
+                const bool swap = reference[k] && sign[k] < 0.f;
+                const float t = low[b][k];
+                low[b][k] = swap ? high[b][k] : t;
+                high[b][k] = swap ? t : high[b][k];
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        ep0.v[c] = MakePair(low[c][0], low[c][1]);
+        ep1.v[c] = MakePair(high[c][0], high[c][1]);
+    }
+}
+
+// MinMax and SwapEndpointComponents (C > 1) of the whole block.
+template <int C>
+__device__ __forceinline__ void StartingEndpoints(const PairPixels& pixels, PairVec<C>& ep0, PairVec<C>& ep1)
+{
+    PairVec<C> sum;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        ep0.v[c] = Both(FLT_MAX);
+        ep1.v[c] = Both(-FLT_MAX);
+        sum.v[c] = Both(0.f);
+    }
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+    {
+        const PairVec<C> p = PairPixel<C>(pixels, i);
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+        {
+            ep0.v[c] = Min(ep0.v[c], p.v[c]);
+            ep1.v[c] = Max(ep1.v[c], p.v[c]);
+            if (C > 1)
+                sum.v[c] = sum.v[c] + p.v[c];
+        }
+    }
+    if constexpr (C > 1)
+        OrientEndpoints<C>(pixels, sum, ep0, ep1);
+}
+__device__ __forceinline__ float ReciprocalOrZero(float v)
+{
+    return v > 0.0f ? 1.0f / v : v;
+}
+
+// OptimizeEndpoints of the whole block.
+template <int C>
+__device__ __forceinline__ void OptimizeEndpoints(const PairPixels& pixels, PairVec<C>& ep0, PairVec<C>& ep1, int indexBits)
+{
+    bool stopped[2] = {false, false};
+    const float scale = float((1u << indexBits) - 1u);
+    const Pair indexMax = Both(scale), indexScale = Both(1.0f / scale);
+#pragma unroll 1
+    for (int iteration = 0; iteration < 2; ++iteration)
+    {
+        const PairVec<C> axis = ep1 - ep0;
+        const Pair mul = PerBlock(Dot(axis, axis), ReciprocalOrZero);
+        Pair alpha2 = Both(0.f), beta2 = Both(0.f), alphaBeta = Both(0.f);
+        PairVec<C> alphaX, betaX;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            alphaX.v[c] = betaX.v[c] = Both(0.f);
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i)
+        {
+            const PairVec<C> color = PairPixel<C>(pixels, i);
+            const Pair index = MultiplySaturate(Dot(color - ep0, axis), mul);
+            const Pair beta = RoundSmall(index * indexMax) * indexScale;
+            const Pair alpha = Both(1.0f) - beta;
+            alpha2 = alpha2 + alpha * alpha;
+            beta2 = beta2 + beta * beta;
+            alphaBeta = alphaBeta + alpha * beta;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+            {
+                alphaX.v[c] = alphaX.v[c] + color.v[c] * alpha;
+                betaX.v[c] = betaX.v[c] + color.v[c] * beta;
+            }
+        }
+        const Pair denominators = alpha2 * beta2 - alphaBeta * alphaBeta;
+        float denominator[2];
+        Split(denominators, denominator[0], denominator[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            stopped[k] = stopped[k] || !(fabsf(denominator[k]) > 0.0001f);
+        const Pair factor = PerBlock(denominators, [](float v) { return 1.0f / v; });
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+        {
+            float a[2], b[2], e0[2], e1[2];
+            Split(MultiplySaturate(alphaX.v[c] * beta2 - betaX.v[c] * alphaBeta, factor), a[0], a[1]);
+            Split(MultiplySaturate(betaX.v[c] * alpha2 - alphaX.v[c] * alphaBeta, factor), b[0], b[1]);
+            Split(ep0.v[c], e0[0], e0[1]);
+            Split(ep1.v[c], e1[0], e1[1]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+            {
+                if (!stopped[k] && !(e0[k] == 0.0f || e0[k] == 1.0f))
+                    e0[k] = a[k];
+                if (!stopped[k] && !(e1[k] == 0.0f || e1[k] == 1.0f))
+                    e1[k] = b[k];
+            }
+            ep0.v[c] = MakePair(e0[0], e0[1]);
+            ep1.v[c] = MakePair(e1[0], e1[1]);
+        }
+    }
+}
+
+template <int C>
+__device__ __forceinline__ void QuantizeEndpoints(const PairVec<C>& ep0, const PairVec<C>& ep1, int bits, int (&q0)[2][C], int (&q1)[2][C])
+{
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        float a[2], b[2];
+        Split(ep0.v[c], a[0], a[1]);
+        Split(ep1.v[c], b[0], b[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+        {
+            q0[k][c] = Quantize(a[k], bits);
+            q1[k][c] = Quantize(b[k], bits);
+        }
+    }
+}
+
+__device__ __forceinline__ Pair Over255(Pair v)
+{
+    constexpr float reciprocal = 1.f / 255.f;
+    const Pair quotient = v * Both(reciprocal);
+    return MultiplyAdd(MultiplyAdd(quotient, Both(-255.f), v), Both(reciprocal), quotient);
+}
+
+// CalculateIndices of the whole block: indices (inverted, endpoints swapped, where the anchor's top bit was set) and error.
+template <int C>
+__device__ __forceinline__ void CalculateIndices(const PairPixels& pixels, int indexBits, int endpointBits, int (&q0)[2][C], int (&q1)[2][C],
+    uint64_t (&indices)[2], Pair& error)
+{
+    PairVec<C> ep0, axis, base, extent;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        const Pair low = MakePair(float(ExpandTo8Bits(q0[0][c], endpointBits)), float(ExpandTo8Bits(q0[1][c], endpointBits)));
+        const Pair high = MakePair(float(ExpandTo8Bits(q1[0][c], endpointBits)), float(ExpandTo8Bits(q1[1][c], endpointBits)));
+        ep0.v[c] = Over255(low);
+        axis.v[c] = Over255(high) - ep0.v[c];
+        base.v[c] = MultiplyAdd(low, Both(64.f), Both(32.f));
+        extent.v[c] = high - low;
+    }
+    const Pair mul = PerBlock(Dot(axis, axis), ReciprocalOrZero);
+    const float maxIndex = float((1u << indexBits) - 1u);
+    const Pair indexMax = Both(maxIndex), weightScale = Both(64.f / maxIndex);
+    uint32_t low[2] = {0u, 0u}, high[2] = {0u, 0u}; // sixteen nibbles; every pixel enters at the top and moves down
+    error = Both(0.f);
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i)
+    {
+        const PairVec<C> p = PairPixel<C>(pixels, i);
+        // the sum with 1.5 * 2^23 holds the rounded index in its low bits
+        const Pair shifted = MultiplySaturate(Dot(p - ep0, axis), mul) * indexMax + Both(12582912.f);
+        float bits[2];
+        Split(shifted, bits[0], bits[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+        {
+            low[k] = __funnelshift_r(low[k], high[k], 4);
+            high[k] = (high[k] >> 4) | (__float_as_uint(bits[k]) << 28);
+        }
+        const Pair weight = RoundSmall((shifted + Both(-12582912.f)) * weightScale); // 0..64
+        PairVec<C> difference;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+        {
+            Pair value;
+            asm("fma.rm.f32x2 %0, %1, %2, %3;"
+                : "=l"(value.bits)
+                : "l"(MultiplyAdd(weight, extent.v[c], base.v[c]).bits), "l"(Both(0.015625f).bits), "l"(Both(8388608.f).bits));
+            difference.v[c] = Over255(value + Both(-8388608.f)) - p.v[c];
+        }
+        error = error + Dot(difference, difference);
+    }
+    const uint64_t all = uint64_t((1u << indexBits) - 1u) * 0x1111111111111111ull;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        indices[k] = uint64_t(high[k]) << 32 | low[k];
+        if ((indices[k] >> (indexBits - 1)) & 1u)
+        {
+            indices[k] ^= all;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+            {
+                const int t = q0[k][c];
+                q0[k][c] = q1[k][c];
+                q1[k][c] = t;
+            }
+        }
+    }
+}
+
+struct PairBest
+{
+    float error[2];
+    uint4 block[2];
+};
+
+template <int kMode, bool kSelector>
+__device__ void FinalizeDualPlane(const PairPixels& pixels, int rotation, const PairVec<1>& s0, const PairVec<1>& s1, const PairVec<3>& c0,
+    const PairVec<3>& c1, PairBest& best)
+{
+    using Traits = DualPlaneTraits<kMode, kSelector>;
+    int q0[2][3], q1[2][3], a0[2][1], a1[2][1];
+    QuantizeEndpoints<3>(c0, c1, Traits::kColorBits, q0, q1);
+    QuantizeEndpoints<1>(s0, s1, Traits::kScalarBits, a0, a1);
+    uint64_t colorIndices[2], scalarIndices[2];
+    Pair colorError, scalarError;
+    CalculateIndices<3>(pixels, Traits::kColorIndexBits, Traits::kColorBits, q0, q1, colorIndices, colorError);
+    CalculateIndices<1>(pixels, Traits::kScalarIndexBits, Traits::kScalarBits, a0, a1, scalarIndices, scalarError);
+    float error[2];
+    Split(colorError + scalarError, error[0], error[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (!(error[k] > best.error[k]))
+        {
+            best.error[k] = error[k];
+            best.block[k] = PackDualPlane<kMode, kSelector>(rotation, q0[k], q1[k], a0[k][0], a1[k][0], colorIndices[k], scalarIndices[k]);
+        }
+}
+
+// The three dual-plane configurations of one rotation.  They start from the same endpoints, and each plane is refined for
+// 2-bit and for 3-bit indices only: four refinements instead of six.
+__device__ void EncodeRotation(const PairPixels& pixels, int rotation, PairBest& best)
+{
+    PairVec<1> low, high, s0[2], s1[2]; // refined for 2-bit and for 3-bit indices
+    StartingEndpoints<1>(pixels, low, high);
+    PairVec<3> darkest, brightest, c0[2], c1[2];
+    StartingEndpoints<3>(pixels, darkest, brightest);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        s0[k] = low;
+        s1[k] = high;
+        OptimizeEndpoints<1>(pixels, s0[k], s1[k], 2 + k);
+        c0[k] = darkest;
+        c1[k] = brightest;
+        OptimizeEndpoints<3>(pixels, c0[k], c1[k], 2 + k);
+    }
+    FinalizeDualPlane<4, false>(pixels, rotation, s0[1], s1[1], c0[0], c1[0], best);
+    FinalizeDualPlane<4, true>(pixels, rotation, s0[0], s1[0], c0[1], c1[1], best);
+    FinalizeDualPlane<5, false>(pixels, rotation, s0[0], s1[0], c0[0], c1[0], best);
+}
+
+// Mode 6 (FinalizeMode<6> on two blocks).
+__device__ void EncodeMode6(const PairPixels& pixels, PairBest& best)
+{
+    PairVec<4> ep0, ep1;
+    StartingEndpoints<4>(pixels, ep0, ep1);
+    OptimizeEndpoints<4>(pixels, ep0, ep1, 4);
+    int q0[2][4], q1[2][4];
+    QuantizeEndpoints<4>(ep0, ep1, 8, q0, q1);
+    float alpha0[2], alpha1[2];
+    Split(ep0.v[3], alpha0[0], alpha0[1]);
+    Split(ep1.v[3], alpha1[0], alpha1[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        ShareLowBit<4>(q0[k], alpha0[k]);
+        ShareLowBit<4>(q1[k], alpha1[k]);
+    }
+    uint64_t indices[2];
+    Pair errors;
+    CalculateIndices<4>(pixels, 4, 8, q0, q1, indices, errors);
+    Split(errors, best.error[0], best.error[1]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        int q[2][4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+        {
+            q[0][c] = q0[k][c];
+            q[1][c] = q1[k][c];
+        }
+        if (!(best.error[k] > FLT_MAX))
+            best.block[k] = PackSinglePlane<6>(0, {0, 0, 0}, q, indices[k]);
+        else
+            best.error[k] = FLT_MAX;
+    }
+}
+
+struct SearchStorage
+{
+    uint2 texels[16 * kSearchBlocks];  // texel i of block b at i * 64 + b: red-green, blue-alpha
+    float2 planes[4][16 * 32];         // component c of texel i of blocks (lane, lane + 32) at [c][i * 32 + lane]
+    union
+    {
+        uint4 halves[16 * 32];         // while the partitions are searched: the same as halves, the two reds, greens, blues, alphas
+        struct                         // afterwards the tasks' results
+        {
+            uint4 block[kSearchTasks][kSearchBlocks];
+            float error[kSearchTasks][kSearchBlocks];
+        } results;
+    };
+    float partitionError[3][kSearchWarps][kSearchBlocks]; // best partition of each warp: three subsets, two, two with alpha
+    uint8_t partition[3][kSearchWarps][kSearchBlocks];
+};
+
+// The staged texels of a lane's two blocks, alpha in the place of the rotation's channel and that channel in alpha's.
+__device__ __forceinline__ PairPixels StagedPixels(const SearchStorage& shared, int lane, int rotation)
+{
+    PairPixels pixels;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        pixels.plane[c] = shared.planes[c < 3 ? (rotation == c + 1 ? 3 : c) : (rotation ? rotation - 1 : 3)] + lane;
+    return pixels;
+}
+
+// Correctly rounded n-ths of the packed values, n = 1 .. 16: one correction of the product with the rounded reciprocal
+// (Markstein, IBM J. Res. Dev. 34, 1990; compared with the division for every 24-bit significand and every n).
+__device__ __forceinline__ Pair DivideByCount(Pair a, float count, float reciprocal)
+{
+    const Pair quotient = a * Both(reciprocal);
+    return MultiplyAdd(MultiplyAdd(quotient, Both(-count), a), Both(reciprocal), quotient);
+}
+
+// BC7_EstimateError (:347-377) of one subset of both blocks: squared error against the line between the starting
+// endpoints, with the indices rounded but not clamped.  The subset's pixels are the nibbles [begin, end) of `order`.
+// C = 3: endpoint components swapped as SwapEndpointComponents does; C = 4: as they are.
+template <int C>
+__device__ __forceinline__ Pair EstimateSubset(const SearchStorage& shared, int lane, uint64_t order, int begin, int end, float maxIndex)
+{
+    const PairPixels pixels = StagedPixels(shared, lane, 0);
+    const uint64_t list = order >> (4 * begin);
+    const int count = end - begin;
+    // extremes of the halves (exact, so the order does not matter), sums in binary32
+    __half2 low[C], high[C];
+    Pair sum[3];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        low[c] = __halves2half2(__ushort_as_half(0x7c00), __ushort_as_half(0x7c00));
+        high[c] = __halves2half2(__ushort_as_half(0xfc00), __ushort_as_half(0xfc00));
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        sum[c] = Both(0.f);
+    {
+        uint64_t rest = list;
+#pragma unroll 1
+        for (int k = 0; k < count; ++k, rest >>= 4)
+        {
+            const uint4 raw = shared.halves[(uint32_t(rest) & 15u) * 32 + lane];
+            const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+            const PairVec<3> texel = C == 3 ? PairPixel<3>(pixels, int(uint32_t(rest) & 15u)) : PairVec<3>();
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+            {
+                const __half2 h = *reinterpret_cast<const __half2*>(&words[c]);
+                low[c] = __hmin2(low[c], h);
+                high[c] = __hmax2(high[c], h);
+                if (C == 3)
+                    sum[c] = PlainAdd(sum[c], texel.v[c]);
+            }
+        }
+    }
+    float2 e0[C], e1[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        e0[c] = __half22float2(low[c]);
+        e1[c] = __half22float2(high[c]);
+    }
+    if (C == 3)
+    {
+        const float countValue = float(count), reciprocal = 1.0f / countValue;
+        Pair center[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            center[c] = Negate(DivideByCount(sum[c], countValue, reciprocal));
+        Pair redGreen = Both(0.f), redBlue = Both(0.f), greenBlue = Both(0.f);
+        uint64_t rest = list;
+#pragma unroll 1
+        for (int k = 0; k < count; ++k, rest >>= 4)
+        {
+            PairVec<3> p = PairPixel<3>(pixels, int(uint32_t(rest) & 15u));
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                p.v[c] = PlainAdd(p.v[c], center[c]);
+            redGreen = redGreen + p.v[0] * p.v[1];
+            redBlue = redBlue + p.v[0] * p.v[2];
+            greenBlue = greenBlue + p.v[1] * p.v[2];
+        }
+        float2 rgCov, rbCov, gbCov;
+        Split(redGreen, rgCov.x, rgCov.y);
+        Split(redBlue, rbCov.x, rbCov.y);
+        Split(greenBlue, gbCov.x, gbCov.y);
+        // the first component with an extent is the reference, the later ones follow the sign of their covariance with it
+        auto orient = [](float& r0, float& r1, float& g0, float& g1, float& b0, float& b1, float rg, float rb, float gb) {
+            const bool redExtent = r0 != r1;
+            const bool swapGreen = redExtent && rg < 0.f;
+            const bool swapBlue = redExtent ? rb < 0.f : (g0 != g1 && gb < 0.f);
+            const float lowGreen = g0, lowBlue = b0;
+            g0 = swapGreen ? g1 : g0;
+            g1 = swapGreen ? lowGreen : g1;
+            b0 = swapBlue ? b1 : b0;
+            b1 = swapBlue ? lowBlue : b1;
+        };
+        orient(e0[0].x, e1[0].x, e0[1].x, e1[1].x, e0[C - 1].x, e1[C - 1].x, rgCov.x, rbCov.x, gbCov.x);
+        orient(e0[0].y, e1[0].y, e0[1].y, e1[1].y, e0[C - 1].y, e1[C - 1].y, rgCov.y, rbCov.y, gbCov.y);
+    }
+    Pair ep0[C], axis[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+    {
+        ep0[c] = MakePair(e0[c].x, e0[c].y);
+        axis[c] = MakePair(e1[c].x, e1[c].y) - ep0[c];
+        ep0[c] = Negate(ep0[c]);
+    }
+    Pair squared = axis[0] * axis[0];
+#pragma unroll
+    for (int c = 1; c < C; ++c)
+        squared = squared + axis[c] * axis[c];
+    float mul0, mul1;
+    Split(squared, mul0, mul1);
+    if (mul0 > 0.0f)
+        mul0 = 1.0f / mul0;
+    if (mul1 > 0.0f)
+        mul1 = 1.0f / mul1;
+    const Pair mul = MakePair(mul0, mul1), indexMax = Both(maxIndex), indexScale = Both(1.f / maxIndex);
+    Pair error = Both(0.f);
+    uint64_t rest = list;
+#pragma unroll 1
+    for (int k = 0; k < count; ++k, rest >>= 4)
+    {
+        const PairVec<C> texel = PairPixel<C>(pixels, int(uint32_t(rest) & 15u));
+        Pair p[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            p[c] = PlainAdd(texel.v[c], ep0[c]);
+        Pair dot = p[0] * axis[0];
+#pragma unroll
+        for (int c = 1; c < C; ++c)
+            dot = dot + p[c] * axis[c];
+        const Pair index = RoundSmall(dot * mul * indexMax) * indexScale;
+        Pair distance;
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+        {
+            const Pair difference = axis[c] * index - p[c];
+            const Pair square = difference * difference;
+            distance = c == 0 ? square : distance + square;
+        }
+        error = error + distance;
+    }
+    return error;
+}
+
+// One warp's share of a partition search: every eighth partition, on 64 blocks; the warp's best goes to shared memory.
+// (The loops of BC7_Mode0_2_Compress :724-775, BC7_Mode1_3_Compress :930-979, BC7_Mode7_Compress :1296-1335.)
+template <int C, int kSubsets>
+__device__ void SearchPartitions(SearchStorage& shared, int kind, int warp, int lane, float maxIndex)
+{
+    float best0 = FLT_MAX, best1 = FLT_MAX;
+    int partition0 = 0, partition1 = 0;
+#pragma unroll 1
+    for (int partition = warp; partition < 64; partition += kSearchWarps)
+    {
+        const uint64_t order = kSubsets == 3 ? kPixelLists3.order[partition] : kPixelLists2.order[partition];
+        const uint32_t ends = kSubsets == 3 ? kPixelLists3.ends[partition] : kPixelLists2.ends[partition];
+        Pair error = Both(0.f);
+        float error0 = 0.f, error1 = 0.f;
+        int begin = 0;
+#pragma unroll 1
+        for (int s = 0; s < kSubsets; ++s)
+        {
+            const int end = int(ends >> (8 * s)) & 255;
+            const Pair subsetError = EstimateSubset<C>(shared, lane, order, begin, end, maxIndex);
+            // (Tried: leaving a partition once it is no better than the best one for any of the 64 blocks, the best of this
+            // warp or of all eight - the vote costs more than it saves, 1 to 3 %.)
+            error = s == 0 ? subsetError : PlainAdd(error, subsetError);
+            begin = end;
+        }
+        Split(error, error0, error1);
+        if (error0 < best0)
+        {
+            best0 = error0;
+            partition0 = partition;
+        }
+        if (error1 < best1)
+        {
+            best1 = error1;
+            partition1 = partition;
+        }
+    }
+    shared.partitionError[kind][warp][lane] = best0;
+    shared.partitionError[kind][warp][lane + 32] = best1;
+    shared.partition[kind][warp][lane] = uint8_t(partition0);
+    shared.partition[kind][warp][lane + 32] = uint8_t(partition1);
+}
+
+// The partition with the smallest error of all warps', the first one on ties.
+__device__ __forceinline__ int BestPartition(const SearchStorage& shared, int kind, int block)
+{
+    float bestError = FLT_MAX;
+    int best = 0;
+#pragma unroll
+    for (int w = 0; w < kSearchWarps; ++w)
+    {
+        const float error = shared.partitionError[kind][w][block];
+        const int partition = shared.partition[kind][w][block];
+        if (error < bestError || (error == bestError && partition < best))
+        {
+            bestError = error;
+            best = partition;
+        }
+    }
+    return best;
+}
+
+// The independent parts of a block's search after the partitions are known, cheapest schedule over eight warps: the
+// rotations are the long ones.
+enum SearchTask
+{
+    kTaskRotation0 = 0, // .. 3
+    kTaskModes02 = 4,
+    kTaskModes13 = 5,
+    kTaskMode6 = 6,
+    kTaskMode7 = 7
+};
+
+// Tasks whose blocks differ in their partitions: one block per thread.
+__device__ void RunPartitionTask(SearchStorage& shared, int task, int block)
+{
+    Pixels pixels;
+    pixels.base = shared.texels + block;
+    pixels.rotation = 0;
+    pixels.stride = kSearchBlocks;
+    float error = FLT_MAX;
+    uint4 bits = make_uint4(0u, 0u, 0u, 0u);
+    switch (task)
+    {
+    case kTaskModes02:
+    {
+        const int best = BestPartition(shared, 0, block);
+        const Subsets subsets = ThreeSubsets(best);
+        Vec<3> ep[6];
+        StartingEndpoints<3, 3, true>(pixels, subsets, ep);
+        if (best < 16)
+            FinalizeMode<0, false>(pixels, best, subsets, ep, error, bits);
+        FinalizeMode<2, false>(pixels, best, subsets, ep, error, bits);
+        break;
+    }
+    case kTaskModes13:
+    {
+        const int best = BestPartition(shared, 1, block);
+        const Subsets subsets = TwoSubsets(best);
+        Vec<3> ep[4];
+        StartingEndpoints<3, 2, true>(pixels, subsets, ep);
+        FinalizeMode<1, false>(pixels, best, subsets, ep, error, bits);
+        FinalizeMode<3, false>(pixels, best, subsets, ep, error, bits);
+        break;
+    }
+    case kTaskMode7:
+    {
+        const int best = BestPartition(shared, 2, block);
+        const Subsets subsets = TwoSubsets(best);
+        Vec<4> ep[4];
+        StartingEndpoints<4, 2, false>(pixels, subsets, ep);
+        FinalizeMode<7, false>(pixels, best, subsets, ep, error, bits);
+        break;
+    }
+    default:
+        break;
+    }
+    shared.results.block[task][block] = bits;
+    shared.results.error[task][block] = error;
+}
+
+// Tasks over whole blocks: two per thread.
+__device__ void RunWholeBlockTask(SearchStorage& shared, int task, int lane)
+{
+    PairBest best;
+    best.error[0] = best.error[1] = FLT_MAX;
+    best.block[0] = best.block[1] = make_uint4(0u, 0u, 0u, 0u);
+    if (task == kTaskMode6)
+        EncodeMode6(StagedPixels(shared, lane, 0), best);
+    else
+        EncodeRotation(StagedPixels(shared, lane, task), task, best);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+    {
+        shared.results.block[task][lane + 32 * k] = best.block[k];
+        shared.results.error[task][lane + 32 * k] = best.error[k];
+    }
+}
+
+__global__ void __launch_bounds__(kSearchThreads, 3) Bc7SearchKernel(const Bc7Arguments args)
+{
+    __shared__ SearchStorage shared;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0); // visibly the same in every lane
+
+    // the CTA's 64 x 16 texels, neighbouring threads on neighbouring texels of a row
+#pragma unroll
+    for (int k = 0; k < 16 * kSearchBlocks / kSearchThreads; ++k)
+    {
+        const int p = k * kSearchThreads + tid;
+        const int localX = p & (4 * kSearchWidth - 1), localY = p / (4 * kSearchWidth);
+        const int owner = (localY >> 2) * kSearchWidth + (localX >> 2), texel = (localY & 3) * 4 + (localX & 3);
+        shared.texels[texel * kSearchBlocks + owner] = LoadTexel(args, args.base.srcLeft + blockIdx.x * (4 * kSearchWidth) + localX,
+            args.base.srcTop + blockIdx.y * (4 * kSearchHeight) + localY);
+    }
+    __syncthreads();
+    // blocks `lane` and `lane + 32` side by side, as halves and as binary32
+    bool transparent0 = false, transparent1 = false;
+#pragma unroll
+    for (int k = 0; k < 16 / kSearchWarps; ++k)
+    {
+        const int i = k * kSearchWarps + warp;
+        const uint2 first = shared.texels[i * kSearchBlocks + lane], second = shared.texels[i * kSearchBlocks + lane + 32];
+        shared.halves[i * 32 + lane] = make_uint4(__byte_perm(first.x, second.x, 0x5410), __byte_perm(first.x, second.x, 0x7632),
+            __byte_perm(first.y, second.y, 0x5410), __byte_perm(first.y, second.y, 0x7632));
+        const float2 rg0 = __half22float2(*reinterpret_cast<const __half2*>(&first.x)), ba0 = __half22float2(*reinterpret_cast<const __half2*>(&first.y));
+        const float2 rg1 = __half22float2(*reinterpret_cast<const __half2*>(&second.x)), ba1 = __half22float2(*reinterpret_cast<const __half2*>(&second.y));
+        shared.planes[0][i * 32 + lane] = make_float2(rg0.x, rg1.x);
+        shared.planes[1][i * 32 + lane] = make_float2(rg0.y, rg1.y);
+        shared.planes[2][i * 32 + lane] = make_float2(ba0.x, ba1.x);
+        shared.planes[3][i * 32 + lane] = make_float2(ba0.y, ba1.y);
+    }
+    __syncthreads();
+    // The three-component modes cannot hold alpha: only for blocks without a texel of alpha < 1.
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+    {
+        const float2 a = shared.planes[3][i * 32 + lane];
+        transparent0 |= a.x < 1.0f;
+        transparent1 |= a.y < 1.0f;
+    }
+    const uint32_t opaqueLow = __ballot_sync(0xFFFFFFFFu, !transparent0), opaqueHigh = __ballot_sync(0xFFFFFFFFu, !transparent1);
+    if (opaqueLow | opaqueHigh)
+    {
+        SearchPartitions<3, 3>(shared, 0, warp, lane, 7.f);
+        SearchPartitions<3, 2>(shared, 1, warp, lane, 7.f);
+    }
+    SearchPartitions<4, 2>(shared, 2, warp, lane, 3.f);
+    __syncthreads(); // the halves give way to the results
+    // A rotation is about as long as two of the other tasks.  Warps 0 - 3: a rotation each; 4: mode 6 and the first half's
+    // modes 0 / 2; 5: the second half's and mode 7 of the first; 6, 7: modes 1 / 3 of a half each, and mode 7 of the second.
+    if (warp < 4)
+        RunWholeBlockTask(shared, kTaskRotation0 + warp, lane);
+    else
+    {
+        if (warp == 4)
+            RunWholeBlockTask(shared, kTaskMode6, lane);
+        const int schedule = warp == 4 ? 0x0004 : warp == 5 ? 0x070c : warp == 6 ? 0x0005 : 0x0f0d; // task | half << 3, a byte each
+#pragma unroll 1
+        for (int rest = schedule; rest; rest >>= 8)
+        {
+            const int task = rest & 7, half = (rest >> 3) & 1;
+            const bool opaque = ((half ? opaqueHigh : opaqueLow) >> lane) & 1u;
+            if (opaque || task == kTaskMode7)
+                RunPartitionTask(shared, task, half * 32 + lane);
+        }
+    }
+    __syncthreads();
+    if (tid >= kSearchBlocks)
+        return;
+    const int blockX = blockIdx.x * kSearchWidth + (tid & (kSearchWidth - 1)), blockY = blockIdx.y * kSearchHeight + tid / kSearchWidth;
+    if (blockX >= args.base.widthInBlocks || blockY >= args.base.heightInBlocks)
+        return;
+    // the smallest error wins, ties to the later candidate, in the shader's order (a NaN is taken and then replaced)
+    const bool opaque = ((tid < 32 ? opaqueLow : opaqueHigh) >> lane) & 1u;
+    float error = FLT_MAX;
+    uint4 block = make_uint4(0u, 0u, 0u, 0u);
+    auto consider = [&](int task) {
+        const float candidate = shared.results.error[task][tid];
+        if (!(candidate > error))
+        {
+            error = candidate;
+            block = shared.results.block[task][tid];
+        }
+    };
+    if (opaque)
+    {
+        consider(kTaskModes02);
+        consider(kTaskModes13);
+    }
+#pragma unroll
+    for (int rotation = 0; rotation < 4; ++rotation)
+        consider(kTaskRotation0 + rotation);
+    consider(kTaskMode6);
+    consider(kTaskMode7);
     reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = block;
 }
 
@@ -1001,15 +1890,17 @@ int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCom
             return NTCB_ERR_INVALID_ARGUMENT;
         }
     }
-    const dim3 grid(unsigned(base.widthInBlocks + kGroupWidth - 1) / kGroupWidth, unsigned(base.heightInBlocks + kGroupHeight - 1) / kGroupHeight);
-    if (args.modeBuffer)
-        Bc7Kernel<true><<<grid, kThreads, 0, stream>>>(args);
+    const bool search = !args.modeBuffer;
+    const int groupWidth = search ? kSearchWidth : kGroupWidth, groupHeight = search ? kSearchHeight : kGroupHeight;
+    const dim3 grid(unsigned(base.widthInBlocks + groupWidth - 1) / groupWidth, unsigned(base.heightInBlocks + groupHeight - 1) / groupHeight);
+    if (search)
+        Bc7SearchKernel<<<grid, kSearchThreads, 0, stream>>>(args);
     else
-        Bc7Kernel<false><<<grid, kThreads, 0, stream>>>(args);
+        Bc7ModeKernel<<<grid, kThreads, 0, stream>>>(args);
     CountLaunch();
     const cudaError_t error = cudaGetLastError();
     if (error != cudaSuccess)
-        return CudaFailure("Bc7Kernel", error);
+        return CudaFailure("Bc7 kernel", error);
     ClearError();
     return NTCB_OK;
 }

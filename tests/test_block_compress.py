@@ -417,6 +417,32 @@ def test_bc7_kernels_reproduce_the_reference_shader_source(pinned, name):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rows,columns", [(1, 1), (1, 17), (4, 16), (5, 33), (9, 64), (32, 40)])
+def test_rearranged_pinned_blocks_keep_their_encoding(pinned, rows, columns):
+    """Blocks are encoded one by one, so the pinned images' blocks laid out in any other way must come out as the same
+    bytes: grids around the sizes the kernels group blocks by (16 x 4 and 64 for the BC7 search, 16 x 8, 32 x 8), opaque
+    blocks beside transparent ones, blocks of one image beside another's."""
+    import torch
+
+    rng = np.random.default_rng(rows * 100 + columns)
+    keys = {1: "bc1_", 2: "bc2_", 3: "bc3_", 4: "bc4_", 5: "bc5_", 7: "bc7_", -7: "bc7_opaque_"}
+    texels, encoded = [], {key: [] for key in keys}
+    for name in PIN_IMAGES:
+        image = pinned["image_" + name]
+        for y in range(image.shape[0] // 4):
+            for x in range(image.shape[1] // 4):
+                texels.append(image[4 * y:4 * y + 4, 4 * x:4 * x + 4])
+                for key, prefix in keys.items():
+                    encoded[key].append(pinned[prefix + name][y, x])
+    picked = rng.integers(0, len(texels), size=(rows, columns))
+    image = np.stack(texels)[picked].transpose(0, 2, 1, 3, 4).reshape(4 * rows, 4 * columns, -1)
+    device = torch.from_numpy(np.ascontiguousarray(image)).cuda()
+    for key in keys:
+        got = binding.block_compress(device, abs(key), num_channels=3 if key < 0 else 0).cpu().numpy()
+        assert np.array_equal(got, np.stack(encoded[key])[picked]), keys[key]
+
+
+@pytest.mark.gpu
 def test_bc7_kernels_against_the_live_shader_source_on_larger_images(oracle):
     """Images of several CTAs (a CTA covers 32 x 8 blocks), both layouts, channels taken from the middle of a
     wider mip, against the reference's shader source run on the CPU on the same texels."""
