@@ -49,6 +49,25 @@ __device__ __forceinline__ uint32_t LoadPair(const BlockCompressArguments& args,
     return *reinterpret_cast<const uint32_t*>(args.texels + index);
 }
 
+// Sixteen indices of kBits bits, one per nibble, moved together (a loop over the pixels with a 64-bit shift each cost more
+// than finding the indices).
+template <int kBits>
+__device__ __forceinline__ uint64_t JoinIndices(uint64_t x)
+{
+    if (kBits == 4)
+        return x;
+    constexpr int kGap = 4 - kBits; // every step joins two fields, whose gap doubles
+    constexpr uint64_t kField = (1u << kBits) - 1u;
+    constexpr uint64_t kNibbles = kField * 0x0101010101010101ull;
+    x = (x & kNibbles) | ((x >> kGap) & (kNibbles << kBits));
+    constexpr uint64_t kBytes = ((1u << (2 * kBits)) - 1u) * 0x0001000100010001ull;
+    x = (x & kBytes) | ((x >> (2 * kGap)) & (kBytes << (2 * kBits)));
+    constexpr uint64_t kShorts = ((1u << (4 * kBits)) - 1u) * 0x0000000100000001ull;
+    x = (x & kShorts) | ((x >> (4 * kGap)) & (kShorts << (4 * kBits)));
+    constexpr uint64_t kWord = (1ull << (8 * kBits)) - 1ull;
+    return (x & kWord) | ((x >> (8 * kGap)) & (kWord << (8 * kBits)));
+}
+
 // The BC7 half of ntcb_block_compress (block_compress_bc7.cu); `params` has passed the checks common to all formats.
 int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCompressArguments& args, cudaStream_t stream);
 

@@ -25,6 +25,7 @@
 #include "block_compress.h"
 #include "error.h"
 #include "ntcb.h"
+#include "packed_float.cuh"
 
 namespace ntcb
 {
@@ -465,25 +466,6 @@ struct BlockBits
         return make_uint4(uint32_t(low), uint32_t(low >> 32), uint32_t(high), uint32_t(high >> 32));
     }
 };
-
-// Sixteen indices of kBits bits, one per nibble, moved together (a loop over the pixels with a 64-bit shift each cost more
-// than finding the indices).
-template <int kBits>
-__device__ __forceinline__ uint64_t JoinIndices(uint64_t x)
-{
-    if (kBits == 4)
-        return x;
-    constexpr int kGap = 4 - kBits; // every step joins two fields, whose gap doubles
-    constexpr uint64_t kField = (1u << kBits) - 1u;
-    constexpr uint64_t kNibbles = kField * 0x0101010101010101ull;
-    x = (x & kNibbles) | ((x >> kGap) & (kNibbles << kBits));
-    constexpr uint64_t kBytes = ((1u << (2 * kBits)) - 1u) * 0x0001000100010001ull;
-    x = (x & kBytes) | ((x >> (2 * kGap)) & (kBytes << (2 * kBits)));
-    constexpr uint64_t kShorts = ((1u << (4 * kBits)) - 1u) * 0x0000000100000001ull;
-    x = (x & kShorts) | ((x >> (4 * kGap)) & (kShorts << (4 * kBits)));
-    constexpr uint64_t kWord = (1ull << (8 * kBits)) - 1ull;
-    return (x & kWord) | ((x >> (8 * kGap)) & (kWord << (8 * kBits)));
-}
 
 // The index of an anchor pixel is stored without its top bit, which is zero: that bit is taken out.
 template <int kBits>
@@ -987,55 +969,6 @@ constexpr int kSearchWidth = 16, kSearchHeight = 4; // blocks per CTA
 constexpr int kSearchBlocks = kSearchWidth * kSearchHeight;
 constexpr int kSearchTasks = 8;
 
-// Two binary32 values: of blocks `lane` and `lane + 32`.
-struct Pair
-{
-    unsigned long long bits;
-};
-
-__device__ __forceinline__ Pair MakePair(float first, float second)
-{
-    Pair r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.bits) : "f"(first), "f"(second));
-    return r;
-}
-__device__ __forceinline__ Pair Both(float v) { return MakePair(v, v); }
-__device__ __forceinline__ void Split(Pair p, float& first, float& second)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(first), "=f"(second) : "l"(p.bits));
-}
-__device__ __forceinline__ Pair operator*(Pair a, Pair b)
-{
-    Pair r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.bits) : "l"(a.bits), "l"(b.bits));
-    return r;
-}
-__device__ __forceinline__ Pair MultiplyAdd(Pair a, Pair b, Pair c)
-{
-    Pair r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.bits) : "l"(a.bits), "l"(b.bits), "l"(c.bits));
-    return r;
-}
-__device__ __forceinline__ Pair Negate(Pair a)
-{
-    float x, y;
-    Split(a, x, y);
-    return MakePair(-x, -y);
-}
-// Sums are multiply-adds with factors of 1 and -1 (an exact product: one rounding, the sum's).  The factors come from
-// constant memory, so that they are not known at compile time: written as add.rn.f32x2, a sum is fused with the packed
-// multiplication before it, whatever --fmad says, and the candidates' errors come out with other roundings.
-__constant__ float2 kOne = {1.f, 1.f};
-__constant__ float2 kMinusOne = {-1.f, -1.f};
-__device__ __forceinline__ Pair operator+(Pair a, Pair b) { return MultiplyAdd(a, MakePair(kOne.x, kOne.y), b); }
-// a + b where neither is a product
-__device__ __forceinline__ Pair PlainAdd(Pair a, Pair b)
-{
-    Pair r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.bits) : "l"(a.bits), "l"(b.bits));
-    return r;
-}
-__device__ __forceinline__ Pair operator-(Pair a, Pair b) { return MultiplyAdd(b, MakePair(kMinusOne.x, kMinusOne.y), a); }
 __device__ __forceinline__ Pair RoundSmall(Pair x) { return PlainAdd(x + Both(12582912.f), Both(-12582912.f)); }
 
 // ---- the searches' whole-block parts on two blocks at once ------------------------------------------------
@@ -1342,11 +1275,8 @@ __device__ __forceinline__ void CalculateIndices(const PairPixels& pixels, int i
 #pragma unroll
         for (int c = 0; c < C; ++c)
         {
-            Pair value;
-            asm("fma.rm.f32x2 %0, %1, %2, %3;"
-                : "=l"(value.bits)
-                : "l"(MultiplyAdd(weight, extent.v[c], base.v[c]).bits), "l"(Both(0.015625f).bits), "l"(Both(8388608.f).bits));
-            difference.v[c] = Over255(value + Both(-8388608.f)) - p.v[c];
+            const Pair value = MultiplyAddDown(MultiplyAdd(weight, extent.v[c], base.v[c]), Both(0.015625f), Both(8388608.f));
+            difference.v[c] = Over255(PlainAdd(value, Both(-8388608.f))) - p.v[c];
         }
         error = error + Dot(difference, difference);
     }
