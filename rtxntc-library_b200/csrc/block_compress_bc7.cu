@@ -15,7 +15,7 @@
 // of operations with nothing fused, divisions and `round` (half to even) IEEE; min / max / saturate
 // return the other operand when one is a NaN, as the HLSL intrinsics do.  The input is the decode
 // kernel's fp16 output (either layout), staged per CTA in shared memory as four halves per texel,
-// texel i of block slot t at word i * 256 + t, so the loops over the texels stay rolled.
+// texel i of block slot t at word i * (blocks per CTA) + t, so the loops over the texels stay rolled.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <float.h>
@@ -32,9 +32,7 @@ namespace ntcb
 namespace
 {
 
-constexpr int kGroupWidth = 32;  // blocks per CTA, x
-constexpr int kGroupHeight = 8;  // and y
-constexpr int kThreads = kGroupWidth * kGroupHeight;
+constexpr int kThreads = 256; // of the mode-buffer kernel
 constexpr uint32_t kAllPixels = 0xffffu;
 
 // The partition tables of the BC7 format (Khronos data format specification, BPTC: tables P2, P3 and
@@ -741,6 +739,7 @@ struct Bc7Arguments
     const uint32_t* modeBuffer; // null: full search
     uint32_t modeBufferByteOffset, modeMapWidthInBlocks, modeMapHeightInBlocks;
     int modeMapOffsetX, modeMapOffsetY;
+    int groupWidthLog2, groupHeight; // mode-buffer kernel: blocks per CTA, at most 256
 };
 
 // The block a wrong or missing mode-buffer entry produces: four 2x2 squares, black, red, green, blue
@@ -775,13 +774,13 @@ __device__ __forceinline__ bool LoadModeAndPartition(const Bc7Arguments& args, i
 }
 
 // One block in the one configuration its mode-buffer entry names (CompressBC7.hlsl main(), :1548-1587).
-// texels: the block's texel i at texels[i * kThreads].
-__device__ uint4 EncodeInMode(const uint2* texels, uint32_t mode, uint32_t partition)
+// texels: the block's texel i at texels[i * stride].
+__device__ uint4 EncodeInMode(const uint2* texels, int stride, uint32_t mode, uint32_t partition)
 {
     Pixels pixels;
     pixels.base = texels;
     pixels.rotation = 0;
-    pixels.stride = kThreads;
+    pixels.stride = stride;
     float error = FLT_MAX;
     uint4 block = make_uint4(0u, 0u, 0u, 0u);
 
@@ -864,89 +863,122 @@ __device__ __forceinline__ uint2 LoadTexel(const Bc7Arguments& args, int x, int 
     return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
 }
 
-// With a mode buffer: one thread per block, 32 x 8 blocks per CTA.
+// With a mode buffer.  A CTA takes a rectangle of up to 256 blocks, sorts them by what the mode buffer names - encoder
+// first (eight modes, mode 4 with either index selector), partition second - and its warps work through the encoders' runs
+// of blocks, 32 at a time: a warp runs one encoder, its lanes loop over the same or similar subsets, and different encoders
+// run side by side.  (With one thread per block in sorted order, warps at the border of two runs, and every warp of a small
+// image, ran several encoders one after the other: a 32 x 32 mip took 66 us.)
+constexpr int kEncoders = 9;
+
 __global__ void __launch_bounds__(kThreads) Bc7ModeKernel(const Bc7Arguments args)
 {
     __shared__ uint2 staged[16 * kThreads];
-    __shared__ uint32_t binCount[2 * kThreads + 1]; // blocks per (mode, partition) pair, then where each pair's blocks start
+    __shared__ uint32_t binCount[2 * kThreads + 1]; // blocks per sort key, then where each key's blocks start
     __shared__ uint32_t warpTotal[kThreads / 32];
     __shared__ uint32_t order[kThreads];
+    __shared__ uint32_t nextRun;
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int widthLog2 = args.groupWidthLog2, blocks = args.groupHeight << widthLog2;
     binCount[tid] = 0;
     binCount[tid + kThreads] = 0;
     if (tid == 0)
+    {
         binCount[2 * kThreads] = 0;
-    // The CTA's 128 x 32 texels, neighbouring threads on neighbouring texels of a row, handed to the slot of
+        nextRun = 0;
+    }
+    // The CTA's texels, neighbouring threads on neighbouring texels of a row, handed to the slot of
     // their block through shared memory; red-green and blue-alpha as two 32-bit words.
-#pragma unroll 1
-    for (int k = 0; k < 16; ++k)
+#pragma unroll 4
+    for (int p = tid; p < 16 * blocks; p += kThreads)
     {
-        const int p = k * kThreads + tid;
-        const int localX = p & (4 * kGroupWidth - 1), localY = p / (4 * kGroupWidth);
-        const int owner = (localY >> 2) * kGroupWidth + (localX >> 2), texel = (localY & 3) * 4 + (localX & 3);
-        staged[texel * kThreads + owner] = LoadTexel(args, args.base.srcLeft + blockIdx.x * (4 * kGroupWidth) + localX,
-            args.base.srcTop + blockIdx.y * (4 * kGroupHeight) + localY);
+        const int localX = p & ((4 << widthLog2) - 1), localY = p >> (widthLog2 + 2);
+        const int owner = ((localY >> 2) << widthLog2) + (localX >> 2), texel = (localY & 3) * 4 + (localX & 3);
+        staged[texel * blocks + owner] = LoadTexel(args, args.base.srcLeft + ((blockIdx.x * 4) << widthLog2) + localX,
+            args.base.srcTop + blockIdx.y * (4 * args.groupHeight) + localY);
     }
-
-    int slot = tid;
-    uint32_t mode = 0, partition = 0;
-    bool active;
+    auto place = [&](int slot, int& blockX, int& blockY) {
+        blockX = (blockIdx.x << widthLog2) + (slot & ((1 << widthLog2) - 1));
+        blockY = blockIdx.y * args.groupHeight + (slot >> widthLog2);
+    };
+    uint32_t key = 512u; // blocks without work come last
+    uint32_t partition = 0;
+    if (tid < blocks)
     {
-        const int blockX = blockIdx.x * kGroupWidth + (tid & (kGroupWidth - 1));
-        const int blockY = blockIdx.y * kGroupHeight + tid / kGroupWidth;
-        active = blockX < args.base.widthInBlocks && blockY < args.base.heightInBlocks;
-        if (active && !LoadModeAndPartition(args, blockX, blockY, mode, partition))
+        int blockX, blockY;
+        place(tid, blockX, blockY);
+        uint32_t mode;
+        if (blockX < args.base.widthInBlocks && blockY < args.base.heightInBlocks)
         {
-            reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = MissingModeBlock();
-            active = false;
+            if (LoadModeAndPartition(args, blockX, blockY, mode, partition))
+                // (the index selector of mode 4, bit 2 of its field, above the other bits)
+                key = mode << 6 | (mode == 4u ? (partition & 4u) << 3 | (partition & 3u) : partition);
+            else
+                reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = MissingModeBlock();
         }
-        // Threads trade blocks so that those of one mode AND partition sit next to each other: a warp then
-        // runs one encoder, and its lanes loop over the same subsets (sorted by mode alone, as the shader
-        // does, half of the lanes idle in the pixel loops: 16 active lanes per instruction).  A counting
-        // sort over the 512 (mode, partition) pairs, blocks without work last.
-        __syncthreads();
-        const uint32_t key = active ? (mode << 6 | partition) : 512u;
-        const uint32_t rank = atomicAdd(&binCount[key], 1u);
-        __syncthreads();
-        {
-            // exclusive prefix sum of the bins: two per thread, scanned within the warp, then over the warps
-            const uint32_t first = binCount[2 * tid], second = binCount[2 * tid + 1], pair = first + second;
-            uint32_t inclusive = pair;
+    }
+    __syncthreads();
+    const uint32_t rank = atomicAdd(&binCount[key], 1u);
+    __syncthreads();
+    {
+        // exclusive prefix sum of the bins: two per thread, scanned within the warp, then over the warps
+        const uint32_t first = binCount[2 * tid], second = binCount[2 * tid + 1], pair = first + second;
+        uint32_t inclusive = pair;
 #pragma unroll
-            for (int delta = 1; delta < 32; delta *= 2)
-            {
-                const uint32_t below = __shfl_up_sync(0xFFFFFFFFu, inclusive, delta);
-                if ((tid & 31) >= delta)
-                    inclusive += below;
-            }
-            if ((tid & 31) == 31)
-                warpTotal[tid >> 5] = inclusive;
-            __syncthreads();
-            uint32_t start = inclusive - pair;
-            for (int w = 0; w < (tid >> 5); ++w)
-                start += warpTotal[w];
-            binCount[2 * tid] = start;
-            binCount[2 * tid + 1] = start + first;
-            if (tid == kThreads - 1)
-                binCount[512] = start + pair;
+        for (int delta = 1; delta < 32; delta *= 2)
+        {
+            const uint32_t below = __shfl_up_sync(0xFFFFFFFFu, inclusive, delta);
+            if (lane >= delta)
+                inclusive += below;
         }
+        if (lane == 31)
+            warpTotal[tid >> 5] = inclusive;
         __syncthreads();
-        order[binCount[key] + rank] = uint32_t(tid) | (partition << 16) | ((active ? mode : 8u) << 24);
-        __syncthreads();
-        const uint32_t task = order[tid];
-        slot = int(task & 0xffffu);
-        partition = (task >> 16) & 0x3fu;
-        mode = task >> 24;
-        active = mode < 8u;
+        uint32_t start = inclusive - pair;
+        for (int w = 0; w < (tid >> 5); ++w)
+            start += warpTotal[w];
+        binCount[2 * tid] = start;
+        binCount[2 * tid + 1] = start + first;
+        if (tid == kThreads - 1)
+            binCount[512] = start + pair;
     }
-    if (!active)
-        return;
-
-    const uint4 block = EncodeInMode(staged + slot, mode, partition);
-    const int blockX = blockIdx.x * kGroupWidth + (slot & (kGroupWidth - 1));
-    const int blockY = blockIdx.y * kGroupHeight + slot / kGroupWidth;
-    reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = block;
+    __syncthreads();
+    order[binCount[key] + rank] = uint32_t(tid) | (partition << 16);
+    __syncthreads();
+    for (;;)
+    {
+        int run = 0;
+        if (lane == 0)
+            run = int(atomicAdd(&nextRun, 1u));
+        run = __shfl_sync(0xFFFFFFFFu, run, 0);
+        // run number `run` over all encoders: 32 blocks of one of them, or what is left of it
+        int encoder = 0, begin = 0, end = 0;
+        for (; encoder < kEncoders; ++encoder)
+        {
+            // encoders 0 - 3: modes 0 - 3, 4 and 5: mode 4 with either selector, 6 - 8: modes 5 - 7
+            const int firstKey = encoder < 5 ? encoder * 64 : encoder == 5 ? 288 : (encoder - 1) * 64;
+            const int lastKey = encoder == 4 ? 288 : encoder == 5 ? 320 : firstKey + 64;
+            begin = int(binCount[firstKey]);
+            end = int(binCount[lastKey]);
+            const int runs = (end - begin + 31) >> 5;
+            if (run < runs)
+                break;
+            run -= runs;
+        }
+        if (encoder == kEncoders)
+            break;
+        const int position = begin + 32 * run + lane;
+        if (position < end)
+        {
+            const uint32_t task = order[position];
+            const int slot = int(task & 0xffffu);
+            const uint4 block = EncodeInMode(staged + slot, blocks, uint32_t(encoder < 5 ? encoder : encoder - 1), task >> 16);
+            int blockX, blockY;
+            place(slot, blockX, blockY);
+            reinterpret_cast<uint4*>(args.base.blocks + size_t(blockY) * args.base.rowPitch)[blockX] = block;
+        }
+        __syncwarp();
+    }
 }
 
 // ---- full search ------------------------------------------------------------------------------------------
@@ -1821,14 +1853,25 @@ int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCom
         }
     }
     const bool search = !args.modeBuffer;
-    const int groupWidth = search ? kSearchWidth : kGroupWidth, groupHeight = search ? kSearchHeight : kGroupHeight;
+    // Mode-buffer kernel: 256 blocks per CTA keep the encoders' runs long; images that would then leave SMs without a CTA are
+    // cut finer, down to 64 blocks.
+    int device = 0, sms = 0;
+    cudaError_t error = cudaGetDevice(&device);
+    if (error == cudaSuccess)
+        error = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (error != cudaSuccess)
+        return CudaFailure("cudaDeviceGetAttribute", error);
+    const long long blocks = (long long)base.widthInBlocks * base.heightInBlocks;
+    args.groupWidthLog2 = blocks >= 256ll * sms ? 5 : 4;
+    args.groupHeight = blocks >= 128ll * sms ? 8 : 4;
+    const int groupWidth = search ? kSearchWidth : 1 << args.groupWidthLog2, groupHeight = search ? kSearchHeight : args.groupHeight;
     const dim3 grid(unsigned(base.widthInBlocks + groupWidth - 1) / groupWidth, unsigned(base.heightInBlocks + groupHeight - 1) / groupHeight);
     if (search)
         Bc7SearchKernel<<<grid, kSearchThreads, 0, stream>>>(args);
     else
         Bc7ModeKernel<<<grid, kThreads, 0, stream>>>(args);
     CountLaunch();
-    const cudaError_t error = cudaGetLastError();
+    error = cudaGetLastError();
     if (error != cudaSuccess)
         return CudaFailure("Bc7 kernel", error);
     ClearError();
