@@ -336,9 +336,9 @@ int ntcb_texture_set_get_desc(const NtcbTextureSet* textureSet, NtcbTextureSetDe
 
 /* Uploads the compressed data (as the reference does on every call for a set loaded from a file,
    src/TextureSet.cpp:1691-1757) and decodes every mip into the internal texel buffer: one kernel
-   launch, or - when mip 0 has 512 rows or more - four launches for row bands of mip 0 and one for
-   the other mips, so that a host read can copy a band while the next is decoded.  With `stats` the call waits for the GPU and reports the device time; without it
-   the work is only queued.  Replaces ITextureSet::Decompress (include/libntc/ntc.h:933,
+   launch, or - when mip 0 has 512 rows or more - one for the first rows of mip 0 and one for the rest,
+   so that a host read can copy the first band while the rest is decoded.  With `stats` the call waits for the GPU
+   and reports the device time; without it the work is only queued.  Replaces ITextureSet::Decompress (include/libntc/ntc.h:933,
    src/TextureSet.cpp:1664-1897). */
 int ntcb_texture_set_decompress(NtcbTextureSet* textureSet, NtcbDecompressionStats* stats, int useInt8Weights);
 

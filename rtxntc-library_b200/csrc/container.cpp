@@ -173,6 +173,16 @@ struct Reader
     // A view must exist, be uncompressed and hold at least `bytes`.
     int Fetch(uint64_t index, size_t bytes, void* dst, const char* what)
     {
+        const uint8_t* source = nullptr;
+        const int rc = Locate(index, bytes, source, what);
+        if (rc == NTCB_OK)
+            memcpy(dst, source, bytes);
+        return rc;
+    }
+
+    // ... its place inside the container.
+    int Locate(uint64_t index, size_t bytes, const uint8_t*& source, const char* what)
+    {
         if (index >= views.size())
         {
             SetError("%s refers to buffer view %llu, but the file has only %zu views.", what, (unsigned long long)index,
@@ -191,7 +201,7 @@ struct Reader
                 (unsigned long long)view.storedSize, bytes);
             return NTCB_ERR_FILE_UNRECOGNIZED;
         }
-        memcpy(dst, binary + view.offset, bytes);
+        source = binary + view.offset;
         return NTCB_OK;
     }
 
@@ -689,16 +699,16 @@ int LoadContainer(const void* data, size_t size, LoadedSet& out)
     }
 
     // latent planes -> device order
-    out.latents.resize(size_t(geo.TotalLatentPixels()) * geo.numLayers);
     for (int m = 0; m < geo.numNeuralMips; ++m)
     {
         const size_t plane = size_t(geo.latentWidth[m]) * geo.latentHeight[m];
         for (int layer = 0; layer < geo.numLayers; ++layer)
         {
-            uint16_t* dst = out.latents.data() + size_t(geo.latentPixelOffset[m]) * geo.numLayers + plane * layer;
-            rc = reader.Fetch(images[m].layerViews[layer], plane * 2, dst, "Latent image view");
+            LatentPlane view{nullptr, plane * 2};
+            rc = reader.Locate(images[m].layerViews[layer], plane * 2, view.pixels, "Latent image view");
             if (rc != NTCB_OK)
                 return rc;
+            out.latents.push_back(view);
         }
     }
 

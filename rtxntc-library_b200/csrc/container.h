@@ -58,11 +58,18 @@ struct LoadedTexture
     std::vector<uint64_t> modeBufferOffset, modeBufferStoredSize; // per mip: where the file keeps it (0, 0: nowhere)
 };
 
+// One layer of one latent image: rows of BGRA4 pixels, `bytes` bytes inside the container the set was loaded from (valid as
+// long as that is), in the order in which the device holds them - for each neural mip, for each layer.
+struct LatentPlane
+{
+    const uint8_t* pixels;
+    size_t bytes;
+};
+
 struct LoadedSet
 {
     SetGeometry geometry;
-    // BGRA4 latent pixels in device order: for each neural mip, for each layer, rows of pixels
-    std::vector<uint16_t> latents;
+    std::vector<LatentPlane> latents; // (views: a copy of them cost more than parsing the rest of the container)
     std::vector<uint8_t> int8Blob; // GenericInt8, empty when the file has no Int8 network
     std::vector<uint8_t> fp8Blob;  // GenericFP8, empty when the file has no FloatE4M3 network
     int channelColorSpaces[kMaxChannels] = {}; // ntc::ColorSpace each channel is stored in (0 Linear, 1 sRGB, 2 HLG)

@@ -100,12 +100,13 @@ public:
 
 private:
     Status CheckKernelStatus();
+    Status ClearKernelStatus();
     Status CheckTextureAndMip(int textureIndex, int mipLevel) const;
     Status FillUpload(const LoadedSet& loaded);
     Status GrowStaging(size_t bytes);
     Status CopyBands(const uint8_t* deviceMip0, uint8_t* host, size_t rowBytes);
     Status DecodeInto(const int32_t* rowRanges, DecompressionStats* pOutStats, bool useInt8Weights,
-        const NtcbOutputConversion* conversion, void* deviceOut);
+        const NtcbOutputConversion* conversion, void* deviceOut, bool forHost);
 
     const Context* m_context;
     int m_device;
@@ -124,8 +125,10 @@ private:
     size_t m_uploadBytes = 0, m_latentBytes = 0;
     __half* m_texels = nullptr;
     size_t m_texelBytes = 0;
-    uint32_t* m_status = nullptr;
-    uint32_t* m_hostStatus = nullptr; // pinned
+    // The kernels' status words, in mapped pinned memory: a kernel writes them only when a wait expires, so nothing has to be
+    // cleared or copied back around a launch (a memset and a copy of 16 bytes cost 4 us of a 20 us call).
+    uint32_t* m_hostStatus = nullptr;
+    uint32_t* m_status = nullptr; // the device's address of the same words
     int m_channelColorSpaces[kMaxChannels] = {}; // ntc::ColorSpace each channel is stored in (from the container)
     std::vector<LoadedTexture> m_textures;
     std::vector<std::vector<void*>> m_deviceModeBuffers; // [texture][mip]: device copies of the BC7 mode bitmaps, made on first use
@@ -139,13 +142,14 @@ private:
     cudaEvent_t m_eventClient = nullptr; // see WaitForStream
     bool m_decoded = false;
 
-    // A whole-set decode of a large set is issued as kBands launches over row bands of mip 0 plus one
-    // for the other mips, so that a host read of mip 0 can start copying the first band while the
-    // rest is still being decoded (the read-back, not the decode, bounds Decompress + ReadChannels).
-    static constexpr int kBands = 4;
+    // A whole-set decode of a large set that a host read may follow is issued as two launches, the first rows of mip 0 and
+    // everything else, so that a host read of mip 0 can start copying the first band while the rest is still being
+    // decoded (the read-back, not the decode, bounds Decompress + ReadChannels).  See FirstBandRows.
+    static constexpr int kBands = 2;
     static constexpr int kBandMinRows = 512;
+    int FirstBandRows(size_t texelBytes) const;
     cudaStream_t m_copyStream = nullptr;
-    cudaEvent_t m_bandEvents[kBands + 1] = {}; // [b]: band b of mip 0 decoded; [kBands]: everything decoded
+    cudaEvent_t m_bandEvents[kBands] = {};     // [b]: band b of mip 0 decoded
     int m_bandEnd[kBands] = {};                // last row + 1 of each band
     int m_bandCount = 0;                       // 0: the last decode was a single launch
 };
@@ -296,7 +300,7 @@ Status TextureSet::Initialize(LoadedSet&& loaded, const TextureSetFeatures& feat
     m_networkBytes = m_numerics == NTCB_NUMERICS_REFERENCE ? size_t(kRefNetworkBytes) : size_t(kStagedNetworkBytes);
 
     // upload image: latents (padded to 16 bytes), then the Int8 and the FP8 network images
-    m_latentBytes = (loaded.latents.size() * 2 + 15) & ~size_t(15);
+    m_latentBytes = (size_t(m_geometry.TotalLatentPixels()) * m_geometry.numLayers * 2 + 15) & ~size_t(15);
     m_uploadBytes = m_latentBytes + 2 * m_networkBytes;
     cudaError_t err = cudaHostAlloc(reinterpret_cast<void**>(&m_hostUpload), m_uploadBytes, cudaHostAllocDefault);
     if (err != cudaSuccess)
@@ -321,9 +325,12 @@ Status TextureSet::Initialize(LoadedSet&& loaded, const TextureSetFeatures& feat
         SetError("Failed to allocate %zu bytes of device memory for the decoded texture data.", m_texelBytes);
         return NTCB_ERR_OUT_OF_MEMORY;
     }
-    err = cudaMalloc(reinterpret_cast<void**>(&m_status), NTCB_STATUS_WORDS * sizeof(uint32_t));
+    err = cudaHostAlloc(reinterpret_cast<void**>(&m_hostStatus), NTCB_STATUS_WORDS * sizeof(uint32_t), cudaHostAllocMapped);
     if (err == cudaSuccess)
-        err = cudaHostAlloc(reinterpret_cast<void**>(&m_hostStatus), NTCB_STATUS_WORDS * sizeof(uint32_t), cudaHostAllocDefault);
+    {
+        memset(m_hostStatus, 0, NTCB_STATUS_WORDS * sizeof(uint32_t));
+        err = cudaHostGetDevicePointer(reinterpret_cast<void**>(&m_status), m_hostStatus, 0);
+    }
     if (err != cudaSuccess)
     {
         SetError("Failed to allocate the status words.");
@@ -334,7 +341,7 @@ Status TextureSet::Initialize(LoadedSet&& loaded, const TextureSetFeatures& feat
         err = cudaEventCreate(&m_eventStop);
     if (err == cudaSuccess)
         err = cudaEventCreateWithFlags(&m_eventClient, cudaEventDisableTiming);
-    for (int b = 0; b <= kBands && err == cudaSuccess; ++b)
+    for (int b = 0; b < kBands && err == cudaSuccess; ++b)
         err = cudaEventCreateWithFlags(&m_bandEvents[b], cudaEventDisableTiming);
     if (err != cudaSuccess)
         return CudaFailure("cudaEventCreate", err);
@@ -360,8 +367,14 @@ Status TextureSet::FillUpload(const LoadedSet& loaded)
     m_deviceModeBuffers.assign(m_textures.size(), std::vector<void*>(size_t(m_geometry.mips), nullptr));
     m_hasInt8 = !loaded.int8Blob.empty();
     m_hasFp8 = !loaded.fp8Blob.empty();
-    memset(m_hostUpload, 0, m_uploadBytes);
-    memcpy(m_hostUpload, loaded.latents.data(), loaded.latents.size() * 2);
+    uint8_t* target = m_hostUpload;
+    for (const LatentPlane& plane : loaded.latents)
+    {
+        memcpy(target, plane.pixels, plane.bytes);
+        target += plane.bytes;
+    }
+    memset(target, 0, size_t(m_hostUpload + m_latentBytes - target)); // the padding before the networks
+    // (a network that the file does not hold is never read)
     auto stage = m_numerics == NTCB_NUMERICS_REFERENCE ? ntcb_stage_network_reference : ntcb_stage_network;
     if (m_hasInt8)
     {
@@ -441,7 +454,6 @@ void TextureSet::Release()
     if (m_pixelMajor) cudaFree(m_pixelMajor);
     m_pixelMajor = nullptr;
     m_deviceCurrent = m_pixelMajorCurrent = false;
-    if (m_status) cudaFree(m_status);
     if (m_hostStatus) cudaFreeHost(m_hostStatus);
     if (m_texels) cudaFree(m_texels);
     if (m_deviceUpload) cudaFree(m_deviceUpload);
@@ -455,20 +467,33 @@ void TextureSet::Release()
     m_hostUpload = nullptr;
 }
 
+// For a caller that has synchronized with the launch.
 Status TextureSet::CheckKernelStatus()
 {
-    if (m_hostStatus[0] != 0)
+    const volatile uint32_t* status = m_hostStatus;
+    if (status[0] != 0)
     {
-        SetError("A bounded wait inside the decode kernel expired (code %u, tile %u, layer %u).", m_hostStatus[0],
-            m_hostStatus[1], m_hostStatus[2]);
+        SetError("A bounded wait inside the decode kernel expired (code %u, tile %u, layer %u).", status[0], status[1], status[2]);
         return NTCB_ERR_DEVICE_TIMEOUT;
     }
     return NTCB_OK;
 }
 
+// Before a launch: an expired wait of an earlier one is forgotten (after everything queued has finished).
+Status TextureSet::ClearKernelStatus()
+{
+    if (*const_cast<const volatile uint32_t*>(m_hostStatus) == 0)
+        return NTCB_OK;
+    const cudaError_t err = cudaStreamSynchronize(m_stream);
+    if (err != cudaSuccess)
+        return CudaFailure("cudaStreamSynchronize", err);
+    memset(m_hostStatus, 0, NTCB_STATUS_WORDS * sizeof(uint32_t));
+    return NTCB_OK;
+}
+
 Status TextureSet::DecompressRows(const int32_t* rowRanges, DecompressionStats* pOutStats, bool useInt8Weights)
 {
-    Status status = DecodeInto(rowRanges, pOutStats, useInt8Weights, nullptr, m_texels);
+    Status status = DecodeInto(rowRanges, pOutStats, useInt8Weights, nullptr, m_texels, true);
     if (status == NTCB_OK)
         m_decoded = true;
     return status;
@@ -522,7 +547,7 @@ Status TextureSet::DecompressConverted(DecompressionStats* pOutStats, bool useIn
             return status;
         target = m_staging;
     }
-    status = DecodeInto(nullptr, pOutStats, useInt8Weights, &conversion, target);
+    status = DecodeInto(nullptr, pOutStats, useInt8Weights, &conversion, target, toHost);
     if (status != NTCB_OK)
         return status;
     cudaError_t err;
@@ -602,10 +627,22 @@ Status TextureSet::GrowStaging(size_t bytes)
     return NTCB_OK;
 }
 
+// Rows of the first band: copying it should take as long as decoding everything else does, so that the copies never wait
+// again.  The kernels decode about 20 Gtexel/s, the host link takes about 57 GB/s: copying a texel of n bytes takes 0.35 n
+// times as long as decoding it, and the band's share of the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips
+// apart took five launches, each with a ramp at both ends: 326 us for a 2048 x 2048 set that decodes in 250.)
+int TextureSet::FirstBandRows(size_t texelBytes) const
+{
+    const int height = m_geometry.mipHeight[0];
+    const int rows = int(float(height) / (1.f + 0.35f * float(texelBytes)));
+    return std::min(height, (rows + 15) & ~15);
+}
+
 // One decode launch of all mips (or of a row range per mip) into `deviceOut`: fp16 texels in the
-// set's layout, or converted pixels (mip after mip, rows without padding) when `conversion` is set.
+// set's layout, or converted pixels (mip after mip, rows without padding) when `conversion` is set.  forHost: a host read
+// may follow (see kBands).
 Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOutStats, bool useInt8Weights,
-    const NtcbOutputConversion* conversion, void* deviceOut)
+    const NtcbOutputConversion* conversion, void* deviceOut, bool forHost)
 {
     if (useInt8Weights ? !m_hasInt8 : !m_hasFp8)
     {
@@ -625,9 +662,9 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
     if (err != cudaSuccess)
         return CudaFailure("cudaMemcpyAsync (compressed data)", err);
     m_deviceCurrent = true;
-    err = cudaMemsetAsync(m_status, 0, NTCB_STATUS_WORDS * sizeof(uint32_t), m_stream);
-    if (err != cudaSuccess)
-        return CudaFailure("cudaMemsetAsync (status)", err);
+    Status status = ClearKernelStatus();
+    if (status != NTCB_OK)
+        return status;
 
     NtcbDecodeParams params{};
     params.latents = reinterpret_cast<const uint16_t*>(m_deviceUpload);
@@ -674,31 +711,20 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
         if (err != cudaSuccess)
             return CudaFailure("cudaEventRecord (1)", err);
     }
-    Status status = NTCB_OK;
     m_bandCount = 0;
     const int height0 = m_geometry.mipHeight[0];
-    if (!rowRanges && height0 >= kBandMinRows)
+    if (!rowRanges && forHost && height0 >= kBandMinRows)
     {
-        // row bands of mip 0 (whole tile rows), then the other mips
-        const int bandRows = ((height0 + kBands - 1) / kBands + 15) & ~15;
-        NtcbDecodeParams part = params;
-        for (int mip = 1; mip < m_geometry.mips; ++mip)
-            part.mips[mip].rowBegin = part.mips[mip].rowEnd = 0;
+        const size_t texelBytes = conversion ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat)
+                                             : size_t(m_geometry.channels) * sizeof(__half);
+        NtcbDecodeParams first = params;
+        first.numMips = 1;
+        first.mips[0].rowEnd = params.mips[0].rowBegin = m_bandEnd[0] = FirstBandRows(texelBytes);
+        m_bandEnd[1] = height0;
         for (int b = 0; b < kBands && status == NTCB_OK; ++b)
         {
-            part.mips[0].rowBegin = std::min(height0, b * bandRows);
-            part.mips[0].rowEnd = std::min(height0, (b + 1) * bandRows);
-            m_bandEnd[b] = part.mips[0].rowEnd;
-            status = ntcb_decode(&part, m_stream);
+            status = ntcb_decode(b == 0 ? &first : &params, m_stream);
             if (status == NTCB_OK && cudaEventRecord(m_bandEvents[b], m_stream) != cudaSuccess)
-                status = CudaFailure("cudaEventRecord (band)", cudaGetLastError());
-        }
-        if (status == NTCB_OK)
-        {
-            part = params;
-            part.mips[0].rowBegin = part.mips[0].rowEnd = 0;
-            status = ntcb_decode(&part, m_stream);
-            if (status == NTCB_OK && cudaEventRecord(m_bandEvents[kBands], m_stream) != cudaSuccess)
                 status = CudaFailure("cudaEventRecord (band)", cudaGetLastError());
         }
         if (status == NTCB_OK)
@@ -714,9 +740,6 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
         if (err != cudaSuccess)
             return CudaFailure("cudaEventRecord (2)", err);
     }
-    err = cudaMemcpyAsync(m_hostStatus, m_status, NTCB_STATUS_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, m_stream);
-    if (err != cudaSuccess)
-        return CudaFailure("cudaMemcpyAsync (status)", err);
     if (pOutStats)
     {
         err = cudaStreamSynchronize(m_stream);
@@ -804,9 +827,9 @@ Status TextureSet::Sample(float const* deviceQueries, uint64_t numQueries, void*
             return status;
         m_pixelMajorCurrent = true;
     }
-    err = cudaMemsetAsync(m_status, 0, NTCB_STATUS_WORDS * sizeof(uint32_t), m_stream);
-    if (err != cudaSuccess)
-        return CudaFailure("cudaMemsetAsync (status)", err);
+    Status status = ClearKernelStatus();
+    if (status != NTCB_OK)
+        return status;
     params.latents = m_pixelMajor;
     params.latentLayout = NTCB_LATENTS_INTERLEAVED;
     params.network = m_deviceUpload + m_latentBytes + (useInt8Weights ? 0 : m_networkBytes);
@@ -817,12 +840,9 @@ Status TextureSet::Sample(float const* deviceQueries, uint64_t numQueries, void*
     params.channels = m_geometry.channels;
     params.weightMode = useInt8Weights ? NTCB_WEIGHTS_INT8 : NTCB_WEIGHTS_FP8;
     params.numerics = m_numerics;
-    Status status = ntcb_sample(&params, m_stream);
+    status = ntcb_sample(&params, m_stream);
     if (status != NTCB_OK)
         return status;
-    err = cudaMemcpyAsync(m_hostStatus, m_status, NTCB_STATUS_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, m_stream);
-    if (err != cudaSuccess)
-        return CudaFailure("cudaMemcpyAsync (status)", err);
     err = cudaStreamSynchronize(m_stream);
     if (err != cudaSuccess)
         return CudaFailure("cudaStreamSynchronize", err);
