@@ -58,45 +58,27 @@ __device__ __forceinline__ void StorePixel(unsigned char* pixel, const uint32_t 
     }
 }
 
-// max(0, min(limit, roundf(x))) for limit < 2^22: RoundToCode with the floor taken by an addition of 2^23 that rounds down
-// instead of a conversion; the code is in the low bits of the result.
-__device__ __forceinline__ uint32_t RoundToLowBits(float x, float limit)
+// max(0, min(limit, roundf(x))) for an integer limit below 2^16, as RoundToCode, from a sum that rounds down: of x + 2^15 + 0.5
+// bits 8 to 15 are the integer part (8-bit codes), of x + 2^16 + 0.5 bits 7 to 22 (16-bit codes).
+__device__ __forceinline__ uint32_t RoundToByte1(float x)
 {
-    float shifted = AddFtz(x, 0.5f);
-    if (x == 0.49999997f)
-        shifted = 0.f;
-    return __float_as_uint(__fadd_rd(fmaxf(fminf(shifted, limit + 0.5f), 0.f), 8388608.f));
+    return __float_as_uint(__fadd_rd(fmaxf(fminf(x, 255.f), 0.f), 32768.5f));
+}
+__device__ __forceinline__ uint32_t RoundTo16Bits(float x)
+{
+    return (__float_as_uint(__fadd_rd(fmaxf(fminf(x, 65535.f), 0.f), 65536.5f)) >> 7) & 0xFFFFu;
 }
 
-// A linear, undithered channel pair in the channel format; codes of 8 and 16 bits in the low bits, with anything above.
-template <int kFormat>
-__device__ __forceinline__ void LinearPair(uint32_t pair, uint32_t& lo, uint32_t& hi)
+// SrgbEncode clamped to [0, 1].  (The value is finite, so no NaN reaches the clamp.)
+__device__ __forceinline__ float SrgbEncodeSaturated(float linear)
 {
-    const __half2 texels = AsHalf2(pair);
-    if (kFormat == kFormatUnorm8)
-    {
-        // round(clamp(v) * 255).  The product of a binary16 value and 255 is
-        // exact in binary32 and its only tie inside [0, 255] is 127.5 (v = 0.5), which rounds to 128
-        // both to nearest-even and away from zero, so adding 1.5 * 2^23 leaves the reference's
-        // roundf() result in the low byte.  (Decoded texels are finite: the epilogue scrubs Inf / NaN.)
-        const float2 v = __half22float2(__hmul2_sat(texels, __float2half2_rn(1.f)));
-        lo = __float_as_uint(__fmaf_rn(v.x, 255.f, 12582912.f));
-        hi = __float_as_uint(__fmaf_rn(v.y, 255.f, 12582912.f));
-    }
-    else if (kFormat == kFormatFloat16)
-    {
-        lo = pair & 0xFFFFu; // finite binary16 values as they are
-        hi = pair >> 16;
-    }
-    else
-    {
-        const float2 v = __half22float2(texels);
-        lo = kFormat == kFormatUnorm16 ? RoundToLowBits(MulFtz(v.x, 65535.f), 65535.f) : QuantizeComponent(kFormat, v.x, 0.f);
-        hi = kFormat == kFormatUnorm16 ? RoundToLowBits(MulFtz(v.y, 65535.f), 65535.f) : QuantizeComponent(kFormat, v.y, 0.f);
-    }
+    float low, high;
+    asm("mul.ftz.sat.f32 %0, %1, %2;" : "=f"(low) : "f"(linear), "f"(12.92f));
+    asm("fma.rn.ftz.sat.f32 %0, %1, %2, %3;" : "=f"(high) : "f"(1.055f), "f"(ApproxPow(linear, 1.0f / 2.4f)), "f"(-0.055f));
+    return linear <= 0.0031308f ? low : high;
 }
 
-// Any other undithered component: a channel in colour spaces, or a default (0; component 3: 1).
+// An undithered component that is a channel in colour spaces, or a default (0; component 3: 1).
 template <int kFormat>
 __device__ __forceinline__ uint32_t UnditheredComponent(const OutputConversion& conversion, int numChannels, int c, uint32_t half)
 {
@@ -106,17 +88,31 @@ __device__ __forceinline__ uint32_t UnditheredComponent(const OutputConversion& 
                                     : kFormat == kFormatFloat32 ? 0x3f800000u : 1u;
         return c == 3 ? kOneCode : 0u;
     }
-    const int srcSpace = (conversion.srcSpaces >> (2 * c)) & 3, dstSpace = (conversion.dstSpaces >> (2 * c)) & 3;
+    const uint32_t kind = (conversion.componentKinds >> (2 * c)) & 3u;
+    if (kFormat == kFormatFloat16 && kind == kKindLinear)
+        return half; // finite binary16 values as they are
     float value = __half2float(__ushort_as_half((unsigned short)half));
-    if (srcSpace)
-        value = DecodeColorSpace(srcSpace, value);
-    if (dstSpace)
-        value = EncodeColorSpace(dstSpace, value);
+    if (kFormat == kFormatUnorm8 && kind == kKindSrgbEncode)
+        return __byte_perm(RoundToByte1(MulFtz(SrgbEncodeSaturated(value), 255.f)), 0u, 0x4441);
+    if (kind != kKindLinear)
+    {
+        const int srcSpace = (conversion.srcSpaces >> (2 * c)) & 3, dstSpace = (conversion.dstSpaces >> (2 * c)) & 3;
+        value = EncodeColorSpace(dstSpace, DecodeColorSpace(srcSpace, value));
+    }
     if (kFormat == kFormatUnorm8)
-        return RoundToLowBits(MulFtz(value, 255.f), 255.f);
+        return __byte_perm(RoundToByte1(MulFtz(value, 255.f)), 0u, 0x4441);
     if (kFormat == kFormatUnorm16)
-        return RoundToLowBits(MulFtz(value, 65535.f), 65535.f);
+        return RoundTo16Bits(MulFtz(value, 65535.f));
     return QuantizeComponent(kFormat, value, 0.f);
+}
+
+// Two linear channels as 8-bit codes in bytes 0 and 2: round(clamp(v) * 255).  In binary16 the sum v * 255 + 1024 lies in
+// [1024, 1279], where the spacing is 1, and the fused multiply-add rounds it once; the only tie, v = 0.5, goes to 1152 - to
+// even and away from zero - so the low byte is the reference's roundf() result.  (Decoded texels are finite.)
+__device__ __forceinline__ uint32_t LinearCodes(uint32_t pair)
+{
+    const __half2 clamped = __hmul2_sat(AsHalf2(pair), __float2half2_rn(1.f));
+    return AsU32(__hfma2(clamped, __float2half2_rn(255.f), __float2half2_rn(1024.f)));
 }
 
 // Converting epilogue for one channel format: pairs[j] holds the requested channels 2j and 2j + 1
@@ -135,37 +131,55 @@ __device__ __forceinline__ void ConvertPixel(const OutputConversion& conversion,
     for (int w = 0; w < kMaxWords; ++w)
         words[w] = 0;
 
-    if (!conversion.dither)
+    if (!conversion.dither && kFormat == kFormatUnorm8)
     {
-        // Channel pair by channel pair: which of them keep their colour space is the same for every pixel, so a pair of
-        // linear channels takes the short way whatever the others need (with one sRGB texture in a 12-channel set all twelve
-        // went through the general quantiser: 500 us more on a 4096 x 4096 chain).
-        const uint32_t spaces = conversion.srcSpaces | conversion.dstSpaces;
+        // Word by word.  What the four components of a word take is the same for every pixel; four linear channels, the
+        // usual case, cost five instructions.  (With one sRGB texture in a 12-channel set all channels went through the general
+        // quantiser: 500 us more on a 4096 x 4096 chain than fp16 texels; now 165.)
+#pragma unroll
+        for (int w = 0; w < kMaxWords; ++w)
+        {
+            if (4 * w < components)
+            {
+                const uint32_t kinds = (conversion.componentKinds >> (8 * w)) & 0xFFu;
+                if (kinds == kKindLinear * 0x55u)
+                    words[w] = __byte_perm(LinearCodes(pairs[2 * w]), LinearCodes(pairs[2 * w + 1]), 0x6420);
+                else
+                {
+                    uint32_t word = 0;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                    {
+                        const uint32_t half = (k & 1) ? pairs[2 * w + (k >> 1)] >> 16 : pairs[2 * w + (k >> 1)] & 0xFFFFu;
+                        word |= UnditheredComponent<kFormat>(conversion, numChannels, 4 * w + k, half) << (8 * k);
+                    }
+                    words[w] = word;
+                }
+            }
+        }
+    }
+    else if (!conversion.dither)
+    {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
         {
             if (2 * j < components)
             {
                 uint32_t lo, hi;
-                if (2 * j + 1 < numChannels && !((spaces >> (4 * j)) & 15u))
-                    LinearPair<kFormat>(pairs[j], lo, hi);
-                else
+                if (kFormat == kFormatFloat16 && ((conversion.componentKinds >> (4 * j)) & 15u) == kKindLinear * 5u)
                 {
-                    lo = UnditheredComponent<kFormat>(conversion, numChannels, 2 * j, pairs[j] & 0xFFFFu);
-                    hi = 2 * j + 1 < components ? UnditheredComponent<kFormat>(conversion, numChannels, 2 * j + 1, pairs[j] >> 16) : 0u;
+                    words[j % kMaxWords] = pairs[j];
+                    continue;
                 }
+                lo = UnditheredComponent<kFormat>(conversion, numChannels, 2 * j, pairs[j] & 0xFFFFu);
+                hi = 2 * j + 1 < components ? UnditheredComponent<kFormat>(conversion, numChannels, 2 * j + 1, pairs[j] >> 16) : 0u;
                 if (kBytes == 4)
                 {
                     words[(2 * j) % kMaxWords] = lo;
                     words[(2 * j + 1) % kMaxWords] = hi;
                 }
-                else if (kBytes == 2)
-                    words[j % kMaxWords] = __byte_perm(lo, hi, 0x5410);
                 else
-                {
-                    const uint32_t both = __byte_perm(lo, hi, 0x0040);
-                    words[(j >> 1) % kMaxWords] = (j & 1) ? __byte_perm(words[(j >> 1) % kMaxWords], both, 0x5410) : both & 0xFFFFu;
-                }
+                    words[j % kMaxWords] = __byte_perm(lo, hi, 0x5410);
             }
         }
     }

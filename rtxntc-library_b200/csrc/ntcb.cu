@@ -187,6 +187,9 @@ int MakeOutputConversion(const NtcbOutputConversion& request, int channels, Outp
         }
         out.srcSpaces |= uint32_t(request.srcColorSpaces[c]) << (2 * c);
         out.dstSpaces |= uint32_t(request.dstColorSpaces[c]) << (2 * c);
+        const bool toSrgb = request.srcColorSpaces[c] == NTCB_COLOR_SPACE_LINEAR && request.dstColorSpaces[c] == NTCB_COLOR_SPACE_SRGB;
+        const bool linear = request.srcColorSpaces[c] == NTCB_COLOR_SPACE_LINEAR && request.dstColorSpaces[c] == NTCB_COLOR_SPACE_LINEAR;
+        out.componentKinds |= (linear ? kKindLinear : toSrgb ? kKindSrgbEncode : kKindOther) << (2 * c);
     }
     return NTCB_OK;
 }

@@ -36,7 +36,14 @@ struct OutputConversion
     int dstChannels;  // components written per pixel; those past the requested channels get 0 (component 3: 1)
     int dither;       // nonzero: add a hash-based offset in [-0.5, 0.5) code units before rounding
     uint32_t srcSpaces, dstSpaces;
+    uint32_t componentKinds; // kKind* of component c in bits 2 c and 2 c + 1 (MakeOutputConversion)
 };
+
+// What an undithered component takes.
+constexpr uint32_t kKindDefault = 0;    // no channel: 0, component 3: 1
+constexpr uint32_t kKindLinear = 1;     // the channel as it is
+constexpr uint32_t kKindSrgbEncode = 2; // a linear channel encoded to sRGB
+constexpr uint32_t kKindOther = 3;      // any other pair of colour spaces
 
 __host__ __device__ inline int BytesPerComponent(int format)
 {
