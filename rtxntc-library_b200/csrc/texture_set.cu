@@ -142,12 +142,18 @@ private:
     cudaEvent_t m_eventClient = nullptr; // see WaitForStream
     bool m_decoded = false;
 
-    // A whole-set decode of a large set that a host read may follow is issued as two launches, the first rows of mip 0 and
-    // everything else, so that a host read of mip 0 can start copying the first band while the rest is still being
-    // decoded (the read-back, not the decode, bounds Decompress + ReadChannels).  See FirstBandRows.
+    // A whole-set decode of a large set is issued as two launches, the first rows of mip 0 and everything else, when a host
+    // read may follow, so that it can start copying the first band while the rest is still being decoded (the
+    // read-back, not the decode, bounds Decompress + ReadChannels), or when the upload is large.  See FirstBandRows.
     static constexpr int kBands = 2;
     static constexpr int kBandMinRows = 512;
-    int FirstBandRows(size_t texelBytes) const;
+    // An upload of this size (73 us) is worth the second launch even when the texels stay on the device.
+    static constexpr size_t kStreamedUploadBytes = size_t(4) << 20;
+    int FirstBandRows(size_t hostTexelBytes) const;
+    int LatentRows(int firstRows) const;
+    cudaError_t UploadFirst(int firstRows);
+    cudaStream_t m_uploadStream = nullptr;
+    cudaEvent_t m_eventUploaded = nullptr;
     cudaStream_t m_copyStream = nullptr;
     cudaEvent_t m_bandEvents[kBands] = {};     // [b]: band b of mip 0 decoded
     int m_bandEnd[kBands] = {};                // last row + 1 of each band
@@ -346,6 +352,12 @@ Status TextureSet::Initialize(LoadedSet&& loaded, const TextureSetFeatures& feat
     if (err != cudaSuccess)
         return CudaFailure("cudaEventCreate", err);
     err = cudaStreamCreateWithFlags(&m_copyStream, cudaStreamNonBlocking);
+    if (err == cudaSuccess && m_latentBytes >= kStreamedUploadBytes)
+    {
+        err = cudaStreamCreateWithFlags(&m_uploadStream, cudaStreamNonBlocking);
+        if (err == cudaSuccess)
+            err = cudaEventCreateWithFlags(&m_eventUploaded, cudaEventDisableTiming);
+    }
     if (err != cudaSuccess)
         return CudaFailure("cudaStreamCreateWithFlags", err);
     return NTCB_OK;
@@ -436,6 +448,14 @@ void TextureSet::Release()
         cudaStreamDestroy(m_copyStream);
         m_copyStream = nullptr;
     }
+    if (m_uploadStream)
+    {
+        cudaStreamSynchronize(m_uploadStream);
+        cudaStreamDestroy(m_uploadStream);
+        m_uploadStream = nullptr;
+    }
+    if (m_eventUploaded) cudaEventDestroy(m_eventUploaded);
+    m_eventUploaded = nullptr;
     for (cudaEvent_t& event : m_bandEvents)
     {
         if (event) cudaEventDestroy(event);
@@ -627,15 +647,65 @@ Status TextureSet::GrowStaging(size_t bytes)
     return NTCB_OK;
 }
 
-// Rows of the first band: copying it should take as long as decoding everything else does, so that the copies never wait
-// again.  The kernels decode about 20 Gtexel/s, the host link takes about 57 GB/s: copying a texel of n bytes takes 0.35 n
-// times as long as decoding it, and the band's share of the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips
-// apart took five launches, each with a ramp at both ends: 326 us for a 2048 x 2048 set that decodes in 250.)
-int TextureSet::FirstBandRows(size_t texelBytes) const
+// Rows of mip 0 that are decoded in a launch of their own, 0: none.
+//
+// For a host read of texels of `hostTexelBytes` bytes (0: the texels stay on the device): copying the first band should take
+// as long as decoding everything else does, so that the copies never wait again.  The kernels decode about 20 Gtexel/s, the
+// host link takes about 57 GB/s: copying a texel of n bytes takes 0.35 n times as long as decoding it, and the band's share of
+// the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips apart took five launches, each with a ramp at both
+// ends: 326 us for a 2048 x 2048 set that decodes in 250.)
+//
+// For a streamed upload: decoding the first band should take as long as the rest of the upload does.
+int TextureSet::FirstBandRows(size_t hostTexelBytes) const
 {
     const int height = m_geometry.mipHeight[0];
-    const int rows = int(float(height) / (1.f + 0.35f * float(texelBytes)));
-    return std::min(height, (rows + 15) & ~15);
+    if (height < kBandMinRows)
+        return 0;
+    float share = hostTexelBytes ? 1.f / (1.f + 0.35f * float(hostTexelBytes)) : 0.f;
+    if (m_latentBytes >= kStreamedUploadBytes)
+    {
+        const float latentBytes = float(m_geometry.latentPixelOffset[1]) * float(m_geometry.numLayers) * 2.f;
+        const float upload = latentBytes / 57.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 20.f; // nanoseconds
+        share = std::max(share, upload / (upload + decode));
+    }
+    return std::min(height, (int(float(height) * share) + 15) & ~15);
+}
+
+// Rows of neural mip 0 that texel rows [0, firstRows) of mip 0 read, apart from the last one (row -1 wraps around to it).
+int TextureSet::LatentRows(int firstRows) const
+{
+    return int((int64_t(firstRows) * m_geometry.latentHeight[0] + m_geometry.mipHeight[0] - 1) / m_geometry.mipHeight[0]) + 2;
+}
+
+// The compressed data to the device on the upload stream, what the first rows of mip 0 read before the rest; m_stream waits
+// for the former here, the caller makes it wait for m_eventUploaded before it reads the rest.
+cudaError_t TextureSet::UploadFirst(int firstRows)
+{
+    const size_t rowBytes = size_t(m_geometry.latentWidth[0]) * 2, planeBytes = rowBytes * m_geometry.latentHeight[0];
+    const size_t otherMips = planeBytes * m_geometry.numLayers; // the networks follow the latents
+    const int needed = LatentRows(firstRows), last = m_geometry.latentHeight[0] - 1;
+    auto copyRows = [&](int begin, int end) { // rows of every layer of neural mip 0
+        return cudaMemcpy2DAsync(m_deviceUpload + begin * rowBytes, planeBytes, m_hostUpload + begin * rowBytes, planeBytes,
+            (end - begin) * rowBytes, m_geometry.numLayers, cudaMemcpyHostToDevice, m_uploadStream);
+    };
+    cudaError_t err = cudaEventRecord(m_eventUploaded, m_stream); // what is queued reads the data of an earlier upload
+    if (err == cudaSuccess)
+        err = cudaStreamWaitEvent(m_uploadStream, m_eventUploaded, 0);
+    if (err == cudaSuccess)
+        err = cudaMemcpyAsync(m_deviceUpload + otherMips, m_hostUpload + otherMips, m_uploadBytes - otherMips, cudaMemcpyHostToDevice, m_uploadStream);
+    if (err == cudaSuccess)
+        err = copyRows(0, needed);
+    if (err == cudaSuccess)
+        err = copyRows(last, last + 1);
+    if (err == cudaSuccess)
+        err = cudaEventRecord(m_eventUploaded, m_uploadStream);
+    if (err == cudaSuccess)
+        err = cudaStreamWaitEvent(m_stream, m_eventUploaded, 0);
+    if (err == cudaSuccess)
+        err = copyRows(needed, last);
+    if (err == cudaSuccess)
+        err = cudaEventRecord(m_eventUploaded, m_uploadStream);
+    return err;
 }
 
 // One decode launch of all mips (or of a row range per mip) into `deviceOut`: fp16 texels in the
@@ -656,9 +726,14 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
     if (!guard.Success())
         return NTCB_ERR_CUDA;
 
-    // upload the encoded latents and the network weights, as the reference does on every
-    // Decompress of a loaded set (src/TextureSet.cpp:1691-1757)
-    cudaError_t err = cudaMemcpyAsync(m_deviceUpload, m_hostUpload, m_uploadBytes, cudaMemcpyHostToDevice, m_stream);
+    // Upload the encoded latents and the network weights, as the reference does on every
+    // Decompress of a loaded set (src/TextureSet.cpp:1691-1757).  A large upload runs beside the decode: the first rows of mip 0
+    // start when what they read has arrived.
+    const int firstRows = rowRanges ? 0 : FirstBandRows(forHost ? conversion
+        ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat) : size_t(m_geometry.channels) * sizeof(__half) : 0);
+    const bool streamed = firstRows > 0 && m_latentBytes >= kStreamedUploadBytes && LatentRows(firstRows) < m_geometry.latentHeight[0] - 1;
+    cudaError_t err = streamed ? UploadFirst(firstRows)
+                               : cudaMemcpyAsync(m_deviceUpload, m_hostUpload, m_uploadBytes, cudaMemcpyHostToDevice, m_stream);
     if (err != cudaSuccess)
         return CudaFailure("cudaMemcpyAsync (compressed data)", err);
     m_deviceCurrent = true;
@@ -712,22 +787,25 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
             return CudaFailure("cudaEventRecord (1)", err);
     }
     m_bandCount = 0;
-    const int height0 = m_geometry.mipHeight[0];
-    if (!rowRanges && forHost && height0 >= kBandMinRows)
+    if (firstRows > 0)
     {
-        const size_t texelBytes = conversion ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat)
-                                             : size_t(m_geometry.channels) * sizeof(__half);
         NtcbDecodeParams first = params;
         first.numMips = 1;
-        first.mips[0].rowEnd = params.mips[0].rowBegin = m_bandEnd[0] = FirstBandRows(texelBytes);
-        m_bandEnd[1] = height0;
+        first.mips[0].rowEnd = params.mips[0].rowBegin = m_bandEnd[0] = firstRows;
+        m_bandEnd[1] = m_geometry.mipHeight[0];
         for (int b = 0; b < kBands && status == NTCB_OK; ++b)
         {
+            if (b == 1 && streamed)
+            {
+                err = cudaStreamWaitEvent(m_stream, m_eventUploaded, 0);
+                if (err != cudaSuccess)
+                    return CudaFailure("cudaStreamWaitEvent (compressed data)", err);
+            }
             status = ntcb_decode(b == 0 ? &first : &params, m_stream);
-            if (status == NTCB_OK && cudaEventRecord(m_bandEvents[b], m_stream) != cudaSuccess)
+            if (status == NTCB_OK && forHost && cudaEventRecord(m_bandEvents[b], m_stream) != cudaSuccess)
                 status = CudaFailure("cudaEventRecord (band)", cudaGetLastError());
         }
-        if (status == NTCB_OK)
+        if (status == NTCB_OK && forHost)
             m_bandCount = kBands;
     }
     else

@@ -329,6 +329,36 @@ def test_large_sets_decode_in_row_bands_with_pipelined_readback():
             texture_set.close()
 
 
+@pytest.mark.parametrize("width,height,mips,scale,features", [(1024, 1024, 0, 1, 8), (1000, 1531, 1, 1, 12), (2048, 512, 3, 1, 16)])
+def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, mips, scale, features):
+    """Latents of 4 MiB and more are uploaded in parts while the first rows of mip 0 are already being decoded: the same bits
+    as a decode of resident latents, for texels read by the host, converted pixels on the device, and again after another
+    set of the same shape was loaded."""
+    import torch
+
+    first, second = (synthetic.make_texture_set(synthetic.TextureSetSpec(width, height, 4, mips, scale, features, seed=seed, network="unit"))
+                     for seed in (3, 4))
+    assert first.geometry.encoded_latent_bytes >= 4 << 20
+    conversion = binding.make_conversion(binding.CHANNEL_FORMAT_UNORM8, 4)
+    with binding.Context(0) as context:
+        texture_set = context.create_texture_set(first.container)
+        for data in (first, second, first):
+            texture_set.load_from_memory(data.container)
+            resident = binding.ResidentTextureSet.from_synthetic(data)
+            resident.decode(True)
+            expected_pixels = resident.decode_converted(True, conversion)
+            _sync()
+            pixels = torch.zeros_like(expected_pixels)
+            _sync()
+            texture_set.decompress_converted(conversion, True, device_address=pixels.data_ptr())
+            assert torch.equal(pixels, expected_pixels)
+            texture_set.decompress(True)
+            texture_set.decompress(True)  # the second upload waits for the first decode
+            for mip in range(data.geometry.mips):
+                assert np.array_equal(texture_set.read_mip(mip).view(np.uint16), resident.mip_numpy(mip).view(np.uint16)), mip
+        texture_set.close()
+
+
 def test_live_reference_comparison(oracle):
     """Runs the unmodified reference decoder (oracle/_ref) on this GPU next to ours on a set the
     fixtures do not contain."""
