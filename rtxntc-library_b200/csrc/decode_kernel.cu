@@ -418,6 +418,7 @@ __device__ __forceinline__ int RunLayer(const Params& params, const SharedStorag
 // bounded wait for the copy done, tensor memory released): the caller returns at once.
 __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
+    GridDependencyLaunch();
     // src/Quantizer.cu:490-495: value = float(nibble) * (1.f / 15.f), stored as binary16
     for (int i = tid; i < 256; i += kThreadsPerCta)
     {
@@ -438,11 +439,15 @@ __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* ne
         MbarrierInit(SharedAddress(&shared.barrier), 1);
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
-        MbarrierArriveExpectTx(loadBarrier, kStagedNetworkBytes);
-        BulkCopyToShared(SharedAddress(shared.network), network, kStagedNetworkBytes, loadBarrier);
     }
     if (warp == 0)
         TmemAlloc(SharedAddress(&shared.tmemBase), kTmemColumns);
+    GridDependencyWait();
+    if (tid == 0)
+    {
+        MbarrierArriveExpectTx(loadBarrier, kStagedNetworkBytes);
+        BulkCopyToShared(SharedAddress(shared.network), network, kStagedNetworkBytes, loadBarrier);
+    }
     FenceProxyAsyncShared(); // the bias region is read by the tensor core (async proxy)
     TcgenFenceBeforeSync();
     __syncthreads();         // also publishes the barriers' initialisation
@@ -737,8 +742,7 @@ cudaError_t LaunchWithSharedStorage(Kernel kernel, std::atomic<unsigned long lon
     cudaError_t err = AllowSharedStorage(kernel, doneMask);
     if (err != cudaSuccess)
         return err;
-    kernel<<<ctas, kThreadsPerCta, bytes, stream>>>(params);
-    return cudaGetLastError();
+    return LaunchOverlapped(kernel, ctas, kThreadsPerCta, bytes, stream, params);
 }
 
 } // namespace

@@ -577,6 +577,7 @@ __device__ __forceinline__ int RunLayerRef(const Params& params, const RefTileCo
 // thread that gave up waiting for the image (status words written).
 __device__ __forceinline__ int SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
+    GridDependencyLaunch();
     // src/Quantizer.cu:490-495: value = float(nibble) * (1.f / 15.f), stored as binary16
     for (int i = tid; i < 256; i += kRefThreadsPerCta)
     {
@@ -599,11 +600,15 @@ __device__ __forceinline__ int SetupCtaRef(RefSharedStorage& shared, const uint8
             MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
-        MbarrierArriveExpectTx(loadBarrier, kRefInt8NetworkBytes);
-        BulkCopyToShared(SharedAddress(shared.network), network, kRefInt8NetworkBytes, loadBarrier);
     }
     if (warp == 0)
         TmemAlloc(SharedAddress(&shared.tmemBase), kRefTmemColumns);
+    GridDependencyWait();
+    if (tid == 0)
+    {
+        MbarrierArriveExpectTx(loadBarrier, kRefInt8NetworkBytes);
+        BulkCopyToShared(SharedAddress(shared.network), network, kRefInt8NetworkBytes, loadBarrier);
+    }
     FenceProxyAsyncShared(); // the bias region is read by the tensor core (async proxy)
     TcgenFenceBeforeSync();
     __syncthreads();
@@ -1265,6 +1270,7 @@ __device__ __forceinline__ int RunLayerRefFp8(const Params& params, const RefTil
 // Setup and teardown as for the binary16 kernel, on the FP8 kernel's shared-memory structure.
 __device__ __forceinline__ int SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
+    GridDependencyLaunch();
     for (int i = tid; i < 256; i += kThreadsPerCta)
     {
         __half lo = __float2half_rn(__fmul_rn(float(i & 15), 1.f / 15.f));
@@ -1280,11 +1286,15 @@ __device__ __forceinline__ int SetupCtaRefFp8(RefFp8SharedStorage& shared, const
             MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
-        MbarrierArriveExpectTx(loadBarrier, kRefNetworkBytes);
-        BulkCopyToShared(SharedAddress(shared.network), network, kRefNetworkBytes, loadBarrier);
     }
     if (warp == 0)
         TmemAlloc(SharedAddress(&shared.tmemBase), kTmemColumns);
+    GridDependencyWait();
+    if (tid == 0)
+    {
+        MbarrierArriveExpectTx(loadBarrier, kRefNetworkBytes);
+        BulkCopyToShared(SharedAddress(shared.network), network, kRefNetworkBytes, loadBarrier);
+    }
     FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
     __syncthreads();
@@ -1555,8 +1565,7 @@ cudaError_t LaunchRefKernel(Kernel kernel, std::atomic<unsigned long long>& done
             return err;
         done.fetch_or(bit, std::memory_order_release);
     }
-    kernel<<<ctas, threads, sharedBytes, stream>>>(params);
-    return cudaGetLastError();
+    return LaunchOverlapped(kernel, ctas, threads, sharedBytes, stream, params);
 }
 
 cudaError_t LaunchDecodeRef(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream)
@@ -1622,8 +1631,7 @@ cudaError_t LaunchSampleRef(const SampleParams& params, bool fp8, int ctas, cuda
                 return err;
             doneMask.fetch_or(bit, std::memory_order_release);
         }
-        kernel<<<ctas, kRefThreadsPerCta, offsetof(RefSharedStorage, tables), stream>>>(params);
-        return cudaGetLastError();
+        return LaunchOverlapped(kernel, ctas, kRefThreadsPerCta, offsetof(RefSharedStorage, tables), stream, params);
     };
     if (fp8)
     {
@@ -1639,8 +1647,7 @@ cudaError_t LaunchSampleRef(const SampleParams& params, bool fp8, int ctas, cuda
                 return err;
             done[1].fetch_or(bit, std::memory_order_release);
         }
-        SampleKernelRefFp8<<<ctas, kThreadsPerCta, offsetof(RefFp8SharedStorage, tables), stream>>>(params);
-        return cudaGetLastError();
+        return LaunchOverlapped(SampleKernelRefFp8, ctas, kThreadsPerCta, offsetof(RefFp8SharedStorage, tables), stream, params);
     }
     return launch(SampleKernelRef<false>, done[0]);
 }
