@@ -8,8 +8,7 @@
 //
 // Per tile:
 //   1. every thread samples the two latent grids for its texel (packed BGRA4 pixels, nibble ->
-//      binary16 through a 256-entry shared-memory table, bilinear blend in binary16), appends the
-//      positional encoding and quantises the 48 inputs to int8 codes or e4m3, and writes its 64-byte
+//      binary16, bilinear blend in binary16), appends the positional encoding and quantises the 48 inputs to int8 codes or e4m3, and writes its 64-byte
 //      row of the A operand straight into the tensor core's K-major core-matrix order (a 16-byte
 //      chunk per store, consecutive threads hit consecutive chunks: conflict-free);
 //   2. one thread issues tcgen05.mma (kind::i8 or kind::f8f6f4, M=128, N=64/48/32/16, K=32 per
@@ -166,16 +165,18 @@ struct __align__(128) SharedStorage
     // the tensor core reads operands as 128-byte core matrices: keep them on 128-byte lines
     alignas(128) uint8_t operandA[2 * kOperandBytes];  // A operands of the current layer (top half, bottom half), core-matrix order
     alignas(128) uint8_t biasRegion[kBiasRegionBytes]; // constant A operand of the bias K step of the int8 layers
-    uint32_t latentTable[256];            // byte (two nibbles) -> two binary16 latent values
     uint64_t barrier;                     // MMA completion
     uint64_t loadBarrier;                 // arrival of the network image (bulk copy)
     uint32_t tmemBase;
-    // What inference on sample does not use comes last: its launches ask for the bytes before `tables` only.
+    // What inference on sample does not use comes last: its launches ask for the bytes before `stage` only.
     // (With the whole structure, a sample kernel's own static shared memory - its table of mips - puts four CTAs
     // above an SM's 228 KB: three were resident and the fourth quarter of the grid ran alone afterwards.)
-    alignas(128) TileTables tables;
-    uint8_t footprintHi[kFootprintHiBytes]; // unpacked latents of the tile's footprint in the high-res grid
-    uint8_t footprintLo[kFootprintLoBytes]; // ... and in the low-res grid
+    struct alignas(128)
+    {
+        TileTables<WideTile> tables;
+        uint8_t footprintHi[kFootprintHiBytes]; // unpacked latents of the tile's footprint in the high-res grid
+        uint8_t footprintLo[kFootprintLoBytes]; // ... and in the low-res grid
+    } stage;
 };
 
 
@@ -194,6 +195,7 @@ struct TileContext
                             // converting epilogue: the address of the thread's pixel in the client's format
     uint32_t outStepWords;  // 32-bit words between consecutive channel pairs; with a converting epilogue:
                             // the pixel's linear index in its mip (the dither seed)
+    int storeBytes;         // widest store the texel may go out with (KernelMip::storeBytes)
 };
 
 // First half of a layer of the MLP for the CTA's current tile: barrier and MMA issue (both halves
@@ -380,12 +382,7 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Sha
                 StoreConverted(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
         }
         else if (ctx.out)
-        {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j < channelPairs)
-                    ctx.out[j * ctx.outStepWords] = bits[j];
-        }
+            StoreTexel(ctx.out, ctx.outStepWords, ctx.storeBytes, bits, channelPairs);
     }
 }
 
@@ -419,13 +416,6 @@ __device__ __forceinline__ int RunLayer(const Params& params, const SharedStorag
 __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
     GridDependencyLaunch();
-    // src/Quantizer.cu:490-495: value = float(nibble) * (1.f / 15.f), stored as binary16
-    for (int i = tid; i < 256; i += kThreadsPerCta)
-    {
-        __half lo = __float2half_rn(__fmul_rn(float(i & 15), 1.f / 15.f));
-        __half hi = __float2half_rn(__fmul_rn(float(i >> 4), 1.f / 15.f));
-        shared.latentTable[i] = AsU32(__halves2half2(lo, hi));
-    }
     // constant inputs of the bias K step: 31 slots of kBiasSlotValue and a last slot of 1 per row
     for (int i = tid; i < kBiasRegionBytes / 16; i += kThreadsPerCta)
     {
@@ -515,7 +505,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConvertin
         const KernelMip& mip = params.mips[place.mipIndex];
         const int local = tile - mip.firstTile;
         // local / tilesX through a precomputed reciprocal (exact while local * tilesX < 2^32)
-        const int tileY = mip.tilesX == 1 ? local : int(__umulhi(uint32_t(local), mip.tilesXMagic));
+        const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
         place.tileX0 = (local - tileY * mip.tilesX) * kTileWidth;
         place.tileY0 = mip.rowBegin + tileY * kTileHeight;
         return place;
@@ -528,8 +518,8 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConvertin
     {
         // ---- tables and latent footprints of the first tile -----------------------------------
         place = locate(tile, 0);
-        PrepareTile<kFp8, false>(params, params.mips[place.mipIndex], shared, place.tileX0, place.tileY0, lane, warp, false);
-        tablesMip = TileKeepsTables(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
+        PrepareTile<WideTile, kFp8, false, 0>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, lane, warp, false);
+        tablesMip = TileKeepsTables<WideTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
         __syncthreads();
     }
     while (tile < params.totalTiles)
@@ -557,12 +547,13 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConvertin
             {
                 ctx.out = inside ? reinterpret_cast<uint32_t*>(params.out + mip.outOffset + first) : nullptr;
                 ctx.outStepWords = planar ? uint32_t(mip.width) : 1u; // channel pairs are 2 * width or 2 elements apart
+                ctx.storeBytes = mip.storeBytes;
             }
         }
 
         // ---- 1. this tile's network inputs -> A operand (the last MMA that read the A operand has
         //         completed: every thread waited for it) -------------------------------------------
-        BuildInputs<kFp8, false>(params, mip, shared, ctx, lane, warp);
+        BuildInputs<kFp8, false>(params, mip, shared.stage, ctx, lane, warp);
 
         // ---- 2. layer 0; while the tensor core works on it, prepare the NEXT tile: its tables and
         //         footprints replace this tile's, which nobody reads after the barrier inside
@@ -575,8 +566,8 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConvertin
         {
             place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = TileKeepsTables(params.mips[place.mipIndex], place.tileX0, place.tileY0);
-            PrepareTile<kFp8, false>(params, params.mips[place.mipIndex], shared, place.tileX0, place.tileY0, lane, warp, keepsTables && place.mipIndex == tablesMip);
+            const bool keepsTables = TileKeepsTables<WideTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
+            PrepareTile<WideTile, kFp8, false, 0>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, lane, warp, keepsTables && place.mipIndex == tablesMip);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayer<kFp8, 0, false>(params, shared, ctx, phase, failed);
@@ -636,6 +627,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPe
     ctx.networkBase = SharedAddress(shared.network);
     ctx.biasRegion = SharedAddress(shared.biasRegion);
     ctx.outStepWords = 1;
+    ctx.storeBytes = params.storeBytes;
 
     const unsigned long long tiles = (params.numQueries + kThreadsPerCta - 1) / kThreadsPerCta;
     // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
@@ -676,7 +668,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPe
             const uint32_t slotFill = kFp8 ? 0u : kBiasSlotValue * 0x01010101u;
             words[12] = words[13] = words[14] = slotFill;
             words[15] = kFp8 ? 0u : ((slotFill & 0x00FFFFFFu) | 0x01000000u);
-            SampleGridsDirect<kFp8, false>(params.latents, params.numLayers, mip, x, y, shared.latentTable, words, params.interleaved != 0);
+            SampleGridsDirect<kFp8, false>(params.latents, params.numLayers, mip, x, y, words, params.interleaved != 0);
             // src/RegressionKernels.h:59-85
             float xf = __fmul_rn(float(x), mip.positionScale);
             float yf = __fmul_rn(float(y), mip.positionScale);
@@ -750,7 +742,7 @@ cudaError_t LaunchWithSharedStorage(Kernel kernel, std::atomic<unsigned long lon
 cudaError_t LaunchSample(const SampleParams& params, bool fp8, int ctas, cudaStream_t stream)
 {
     static std::atomic<unsigned long long> done[2];
-    const size_t bytes = offsetof(SharedStorage, tables); // the tables and footprints are not used
+    const size_t bytes = offsetof(SharedStorage, stage); // the tables and footprints are not used
     return fp8 ? LaunchWithSharedStorage(SampleKernel<true>, done[1], params, ctas, stream, bytes)
                : LaunchWithSharedStorage(SampleKernel<false>, done[0], params, ctas, stream, bytes);
 }

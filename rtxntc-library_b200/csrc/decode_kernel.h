@@ -81,27 +81,26 @@ constexpr int kRefInt8NetworkBytes = 17408; // ... what the Int8 kernels copy to
 // has 48 inputs; of layer 1's 64 the first 32 are here, the other 32 in tensor memory, like all of
 // layers 2 and 3.
 constexpr int kRefOperandBytes = 128 * 96;
-// Tile of the reference-numerics kernel: kRefChains 128-row chains (32 x 4 texels each) per CTA.
-// Two chains (32x8 texels, 256 threads) at three CTAs per SM measured faster than four chains
-// (32x16, 512 threads) at two.
+// Reference-numerics kernels: a CTA is two chains of 128 threads that share the network in shared memory and nothing else.
+// Each walks tiles of its own, 16 x 8 texels, with its own tables and footprints, and meets only its own threads in barriers.
+constexpr int kChainTileWidth = 16;
+constexpr int kChainTileHeight = 8;
 constexpr int kRefChains = 2;
-constexpr int kRefTileHeight = 4 * kRefChains;
 constexpr int kRefThreadsPerCta = 128 * kRefChains;
 constexpr int kRefTmemColumns = kRefChains * kTmemColumnsPerHalf;
-constexpr int kRefFootprintHiBytes = 8192;  // the binary16 operands leave less room for the high-res footprint
-constexpr int kRefFootprintLoBytes = 4096;
-// The Int8 kernels, whose binary16 operands take more room, have less for the low-res footprint: enough for
-// what fits into the high-res one (the low-res grid has half the resolution: at a grid-to-mip ratio of 1/2
-// a tile's footprint is 18 x 6 pixels of 24 bytes).
-constexpr int kRefInt8FootprintLoBytes = 2816;
-// The warp that issues the matrix products of both chains of a tile after a CTA-wide barrier, chain 0 first:
-// the first warp of chain 1.  It then waits for chain 1, whose products finish last anyway; a warp of chain 0
-// would start on its own chain's results late by the time it takes to issue chain 1's (2 %).  (After a
-// chain-local barrier each chain's first warp issues its own.)
-constexpr int kIssuingWarp = 4;
+// Footprints of a chain: what a tile covers at a grid-to-mip ratio of 1 (high-res: 18 x 10 pixels of 24 bytes) and 1/2
+// (low-res: 10 x 6).
+constexpr int kRefFootprintHiBytes = 4352;
+constexpr int kRefFootprintLoBytes = 1536;
+constexpr int kRefInt8FootprintHiBytes = kRefFootprintHiBytes;
+constexpr int kRefInt8FootprintLoBytes = 1440;
 constexpr int kCtasPerSmRef = 4;       // Int8 networks: 56 KB of shared memory and 64 registers, like the FP8 kernels
 constexpr int kCtasPerSmRefFp8 = 4; // FP8 networks: 8-bit operands halve the A buffers
 constexpr int kCtasPerSmRefSample = 4; // inference on sample, Int8 networks (its launches leave the footprints out)
+
+// Dynamic shared memory a CTA may have for `ctas` of them to be resident: an SM has 228 KB, 1 KB per CTA is the system's.
+template <int ctas>
+constexpr size_t kMaxSharedBytes = 228 * 1024 / ctas / 128 * 128 - 1024;
 
 constexpr uint32_t kStatusBarrierTimeout = 1;
 
@@ -118,7 +117,7 @@ struct KernelMip
     float invWidth, invHeight;
     float positionScale, positionLod;
     int firstTile, tilesX;
-    unsigned tilesXMagic; // ceil(2^32 / tilesX) for tilesX > 1: local / tilesX == umulhi(local, magic) while local * tilesX < 2^32
+    unsigned tilesXMagic; // ceil(2^32 / tilesX): local / tilesX == umulhi(local, magic) for every tile of the mip; 0: divide
     int staged;      // the tile footprints of both grids fit into shared memory
     int strideBytes; // bytes per staged latent pixel: 8 per layer, padded to an odd multiple of 8 (8, 24, 24, 40) so that
                      // the 8-byte reads of neighbouring pixels fall into different shared-memory banks
@@ -164,6 +163,7 @@ struct SampleParams
     // by side in a slot of 1, 2 or 4 elements (three layers are padded to four) - and hiOffset / loOffset of the
     // mips are element offsets into THAT buffer.
     int interleaved;
+    int storeBytes; // widest store (4, 8 or 16 bytes) an answer may go out with
     KernelMip mips[16];
 };
 

@@ -58,7 +58,7 @@
 // gather and blend (constants are stored instead); 64: the tap tables are rebuilt for every tile; 4: the activation arithmetic of layers 0-2 (the
 // raw accumulator words are stored); 8: the global stores of the epilogue; 16: the tensor-core work
 // (no MMA issue, no wait for it); 32: the tensor-memory loads; 128: the proxy fence before each layer's
-// barrier; 256: a plain barrier instead of the one that also agrees on giving up.
+// barrier.
 #ifndef NTCB_ABLATE
 #define NTCB_ABLATE 0
 #endif
@@ -176,14 +176,24 @@ __device__ __forceinline__ uint32_t ActivateRef(uint32_t bits)
 // quantised binary16 pairs.
 struct __align__(16) RefTileTables
 {
-    TapTables taps;
+    TapTables<ChainTile> taps;
     // positional encoding: word w = (wave w phase 0, wave w phase 0.25)
-    uint4 colEnc[kTileWidth];
-    uint4 rowEnc[kRefTileHeight];
+    uint4 colEnc[ChainTile::kWidth];
+    uint4 rowEnc[ChainTile::kHeight];
     uint32_t lodPair;   // (lod, lod)
     uint32_t zeroPair;  // (quantised 0, quantised 0)
     uint32_t pad[2];
 };
+
+// What a chain prepares per tile.
+template <typename Tables, int kHiBytes, int kLoBytes>
+struct __align__(16) ChainStage
+{
+    Tables tables;
+    uint8_t footprintHi[kHiBytes];
+    uint8_t footprintLo[kLoBytes];
+};
+using RefStage = ChainStage<RefTileTables, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes>;
 
 struct __align__(128) RefSharedStorage
 {
@@ -193,22 +203,21 @@ struct __align__(128) RefSharedStorage
     // vectors e_0 .. e_3, and one of zeros (the second 8-wide half of every step).  A stride offset of 0 in
     // the descriptor makes all sixteen 8-row groups of the 128-row operand read the same core matrix.
     alignas(128) uint8_t onesRegion[5 * 128];
-    uint32_t latentTable[256];
     uint64_t barrier[kRefChains]; // MMA completion, per chain: a chain's threads go on as soon as their accumulators are ready
     uint64_t loadBarrier;  // arrival of the network image
+    alignas(8) uint32_t giveUp[kRefChains][2]; // see LayerBarrier
     uint32_t tmemBase;
-    // what inference on sample does not use comes last: its launches ask for the bytes before `tables` only
-    alignas(128) RefTileTables tables;
-    uint8_t footprintHi[kRefFootprintHiBytes];
-    uint8_t footprintLo[kRefInt8FootprintLoBytes];
+    // what inference on sample does not use comes last: its launches ask for the bytes before `stage` only
+    alignas(128) RefStage stage[kRefChains];
 };
+static_assert(sizeof(RefSharedStorage) <= kMaxSharedBytes<kCtasPerSmRef>, "resident CTAs must fit into shared memory");
 
 struct RefTileContext
 {
     int tid;
-    uint32_t tmemBase, tmemLane, operandA, networkBase, biasRegion;
-    uint32_t barrierBase; // shared address of the chains' MMA-completion mbarriers
-    uint32_t barrier;     // ... of this thread's chain
+    uint32_t tmemLane;    // the chain's first tensor-memory column at this thread's lane (its warp's first lane, to be precise)
+    uint32_t barrier;     // shared address of the chain's MMA-completion mbarrier
+    uint32_t giveUp;      // shared address of the chain's give-up word for the current tile (LayerBarrier)
     uint4* rowChunk; // this thread's 16-byte slot in chunk 0 of its half's A operand
     int tile, x, y;
     uint32_t* out;
@@ -221,18 +230,18 @@ struct RefTileContext
 // ---------------------------------------------------------------------------------------------
 
 // Builds the tile's lookup tables and stages the latent footprint of both grids in shared memory
-// (`tablesValid`: the tables already hold this tile's values, see PrepareTaps).
+// (`tablesValid`: the tables already hold this tile's values, see PrepareTaps).  `warp`: of the chain's four.
 template <bool kFp8, int kLayers = 0>
-__device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const KernelMip& mip, RefSharedStorage& shared,
+__device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
     int tileX0, int tileY0, int lane, int warp, bool tablesValid)
 {
-    static_assert(kRefTileHeight == kTileHeight && kRefThreadsPerCta == kThreadsPerCta, "the tap tables assume the common tile");
     if (!tablesValid && warp >= 2 && warp < 4)
     {
         // positional encoding (src/RegressionKernels.h:59-85): warp 2 the x part per column, warp 3
         // the y part per row, quantised exactly as the per-texel inputs would be
         const bool rows = warp == 3;
-        const int coordinate = rows ? min(tileY0 + (lane & (kRefTileHeight - 1)), mip.rowEnd - 1) : min(tileX0 + lane, mip.width - 1);
+        const int coordinate = rows ? min(tileY0 + (lane & (ChainTile::kHeight - 1)), mip.rowEnd - 1)
+                                    : min(tileX0 + (lane & (ChainTile::kWidth - 1)), mip.width - 1);
         float f = __fmul_rn(float(coordinate), mip.positionScale);
         uint32_t q[3];
 #pragma unroll
@@ -243,17 +252,17 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
             q[wave] = AsU32(QuantizeInputRef<kFp8>(__floats2half2_rn(e0, e1)));
             f = __fmul_rn(f, 2.f);
         }
-        if (!rows)
-            shared.tables.colEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
-        else if (lane < kRefTileHeight)
-            shared.tables.rowEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
-        if (rows && lane == kRefTileHeight)
+        if (!rows && lane < ChainTile::kWidth)
+            stage.tables.colEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
+        if (rows && lane < ChainTile::kHeight)
+            stage.tables.rowEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
+        if (rows && lane == ChainTile::kHeight)
         {
-            shared.tables.lodPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(mip.positionLod)));
-            shared.tables.zeroPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(0.f)));
+            stage.tables.lodPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(mip.positionLod)));
+            stage.tables.zeroPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(0.f)));
         }
     }
-    PrepareTaps<true, kLayers>(params, mip, shared.tables.taps, shared.footprintHi, shared.footprintLo, shared.latentTable, tileX0,
+    PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, tileX0,
         tileY0, lane, warp, tablesValid);
 }
 
@@ -280,11 +289,11 @@ __device__ __forceinline__ void BlendLayerRef(uint2 l00, uint2 l01, uint2 l10, u
 
 // Inputs 0..15 or 16..31 of one texel (eight binary16 pairs) from the staged footprint of one grid.
 template <bool kFp8, int kLayers = 0>
-__device__ __forceinline__ void GatherGridRef(const KernelParams& params, const KernelMip& mip, const RefSharedStorage& shared,
-    int grid, int lane, int tileRow, uint32_t* words)
+__device__ __forceinline__ void GatherGridRef(const KernelParams& params, const KernelMip& mip, const RefStage& stage,
+    int grid, int tileColumn, int tileRow, uint32_t* words)
 {
-    const int4 col = shared.tables.taps.colTap[grid][lane];
-    const int4 row = shared.tables.taps.rowTap[grid][tileRow];
+    const int4 col = stage.tables.taps.colTap[grid][tileColumn];
+    const int4 row = stage.tables.taps.rowTap[grid][tileRow];
     const float dx = __int_as_float(col.y), dxn = __int_as_float(col.z);
     const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
     // src/FeatureGridDevice.h:46-49
@@ -293,7 +302,7 @@ __device__ __forceinline__ void GatherGridRef(const KernelParams& params, const 
     const __half2 w10 = __floats2half2_rn(f10, f10), w11 = __floats2half2_rn(f11, f11);
 
     const int stride = StrideBytes<kLayers>(mip);
-    const uint8_t* tap00 = (grid ? shared.footprintLo : shared.footprintHi) + (col.x + row.x);
+    const uint8_t* tap00 = (grid ? stage.footprintLo : stage.footprintHi) + (col.x + row.x);
     const uint8_t* tap10 = tap00 + row.w;
 #pragma unroll
     for (int layer = 0; layer < 4; ++layer)
@@ -311,48 +320,53 @@ __device__ __forceinline__ void GatherGridRef(const KernelParams& params, const 
 
 // One latent layer of one grid (the low 16 bits of each p are the tap's four features) -> two pairs of inputs.
 template <bool kFp8>
-__device__ __forceinline__ void BlendPixelsRef(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps,
-    const uint32_t* __restrict__ lut, uint32_t* words)
+__device__ __forceinline__ void BlendPixelsRef(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, uint32_t* words)
 {
+    __half2 inputs[2];
+    BlendPixels(p00, p01, p10, p11, taps, inputs);
+    words[0] = AsU32(QuantizeInputRef<kFp8>(inputs[0]));
+    words[1] = AsU32(QuantizeInputRef<kFp8>(inputs[1]));
+}
+
+// Two latent layers of one grid (a word of each tap) -> two pairs of inputs each.
+template <bool kFp8>
+__device__ __forceinline__ void BlendLayersRef(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, uint32_t* words)
+{
+    __half2 inputs[4];
+    BlendTwoLayers(p00, p01, p10, p11, taps, inputs);
 #pragma unroll
     for (int j = 0; j < 2; ++j)
     {
-        const __half2 l00 = AsHalf2(lut[(p00 >> (8 * j)) & 0xFF]), l01 = AsHalf2(lut[(p01 >> (8 * j)) & 0xFF]);
-        const __half2 l10 = AsHalf2(lut[(p10 >> (8 * j)) & 0xFF]), l11 = AsHalf2(lut[(p11 >> (8 * j)) & 0xFF]);
-        __half2 d = __hmul2_rn(l01, taps.w01);
-        d = __hfma2(l00, taps.w00, d);
-        d = __hfma2(l10, taps.w10, d);
-        d = __hfma2(l11, taps.w11, d);
-        d = __hfma2(d, __float2half2_rn(2.f), __float2half2_rn(-1.f));
-        words[j] = AsU32(QuantizeInputRef<kFp8>(d));
+        const uint32_t even = AsU32(QuantizeInputRef<kFp8>(inputs[2 * j])), odd = AsU32(QuantizeInputRef<kFp8>(inputs[2 * j + 1]));
+        words[j] = __byte_perm(even, odd, 0x5410);
+        words[2 + j] = __byte_perm(even, odd, 0x7632);
     }
 }
 
 // ... with the taps read straight from the layer's plane in global memory.
 template <bool kFp8>
-__device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plane, const GridTaps& taps,
-    const uint32_t* __restrict__ lut, uint32_t* words)
+__device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plane, const GridTaps& taps, uint32_t* words)
 {
     const uint32_t p00 = __ldg(plane + taps.o00), p01 = __ldg(plane + taps.o01);
     const uint32_t p10 = __ldg(plane + taps.o10), p11 = __ldg(plane + taps.o11);
-    BlendPixelsRef<kFp8>(p00, p01, p10, p11, taps, lut, words);
+    BlendPixelsRef<kFp8>(p00, p01, p10, p11, taps, words);
 }
 
 // The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.
 template <bool kFp8, int kLayers = 0>
-__device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, const RefSharedStorage& shared,
-    const RefTileContext& ctx, int lane, int tileRow)
+__device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, const RefStage& stage,
+    const RefTileContext& ctx, int tileColumn, int tileRow)
 {
     uint32_t words[24];
-    const uint32_t zeroPair = shared.tables.zeroPair;
+    const uint32_t zeroPair = stage.tables.zeroPair;
 #pragma unroll
     for (int i = 0; i < 16; ++i)
         words[i] = zeroPair; // unused feature slots hold quantised zeros (src/Inference.cu:49)
 
     if (mip.staged)
     {
-        GatherGridRef<kFp8, kLayers>(params, mip, shared, 0, lane, tileRow, words);
-        GatherGridRef<kFp8, kLayers>(params, mip, shared, 1, lane, tileRow, words + 8);
+        GatherGridRef<kFp8, kLayers>(params, mip, stage, 0, tileColumn, tileRow, words);
+        GatherGridRef<kFp8, kLayers>(params, mip, stage, 1, tileColumn, tileRow, words + 8);
     }
     else
     {
@@ -367,25 +381,25 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
             if (layer < NumLayers<kLayers>(params))
-                SampleLayerRef<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, shared.latentTable, words + 2 * layer);
+                SampleLayerRef<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
         SetupTaps(u, v, mip.loWidth, mip.loHeight, taps);
         const uint16_t* lo = params.latents + mip.loOffset;
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
             if (layer < NumLayers<kLayers>(params))
-                SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, shared.latentTable, words + 8 + 2 * layer);
+                SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
     }
 
     // positional encoding: per wave the inputs (x phase 0, y phase 0, x phase 0.25, y phase 0.25)
-    const uint4 cx = shared.tables.colEnc[lane];
-    const uint4 ry = shared.tables.rowEnc[tileRow];
+    const uint4 cx = stage.tables.colEnc[tileColumn];
+    const uint4 ry = stage.tables.rowEnc[tileRow];
     words[16] = __byte_perm(cx.x, ry.x, 0x5410);
     words[17] = __byte_perm(cx.x, ry.x, 0x7632);
     words[18] = __byte_perm(cx.y, ry.y, 0x5410);
     words[19] = __byte_perm(cx.y, ry.y, 0x7632);
     words[20] = __byte_perm(cx.z, ry.z, 0x5410);
     words[21] = __byte_perm(cx.z, ry.z, 0x7632);
-    words[22] = shared.tables.lodPair;
+    words[22] = stage.tables.lodPair;
     words[23] = zeroPair;
 
 #pragma unroll
@@ -424,11 +438,10 @@ __device__ __forceinline__ void UmmaF16FromTmem(uint32_t tmemD, uint32_t tmemA, 
         : "memory");
 }
 
-// First half of a layer for the current tile: barrier (LayerBarrier) and MMA issue - of both chains by warp 4
-// after a CTA-wide barrier, of its own chain by the chain's first warp after a chain-local one.  Returns
-// nonzero (uniformly over the threads that met in the barrier) when some thread gave up on a wait.
-template <int kLayer, int kChainLocal = TileLayerBarrier<kLayer>()>
-__device__ __forceinline__ int IssueLayerRef(const RefTileContext& ctx, int failed)
+// First half of a layer for the chain's current tile: the chain's barrier (LayerBarrier), and MMA issue by its first
+// warp.  Returns nonzero (uniformly over the chain) when some thread gave up on a wait.
+template <int kLayer>
+__device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
     constexpr int kK = kLayer == 0 ? 48 : kLayer == 1 ? 64 : kLayer == 2 ? 48 : 32;
@@ -443,52 +456,45 @@ __device__ __forceinline__ int IssueLayerRef(const RefTileContext& ctx, int fail
     if (kRefOperandInShared<kLayer>)
         FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
-    if (LayerBarrier<kChainLocal>(ctx.tid, failed))
+    if (LayerBarrier<kLayer>(ctx.tid, ctx.giveUp))
         return 1;
 
     // The whole issuing warp runs the descriptor arithmetic on values that are visibly the same in every
     // lane; one elected lane hands the work to the tensor core (see IssueLayerRefFp8).
     const int warpIndex = ctx.tid >> 5;
-    if (kChainLocal ? (warpIndex & 3) == 0 : warpIndex == kIssuingWarp)
+    if ((warpIndex & 3) == 0)
     {
         TcgenFenceAfterSync();
         constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
-        const uint32_t networkBase = __shfl_sync(0xFFFFFFFFu, ctx.networkBase, 0);
-        const uint32_t tmemBase = __shfl_sync(0xFFFFFFFFu, ctx.tmemBase, 0);
-        const uint32_t barrierBase = __shfl_sync(0xFFFFFFFFu, ctx.barrierBase, 0);
+        const uint32_t base = DynamicSharedBase(), networkBase = base + uint32_t(offsetof(RefSharedStorage, network));
         // the four base descriptors are built once, every operand is then a constant offset (in 16-byte
         // units) added to the address field
-        const uint64_t operandBase = MakeSmemDescriptor(__shfl_sync(0xFFFFFFFFu, ctx.operandA, 0), 2048, 128);
+        const uint64_t operandBase = MakeSmemDescriptor(base + uint32_t(offsetof(RefSharedStorage, operandA)), 2048, 128);
         // rows e_kLayer (every 8-row group reads the same core matrix: stride 0), then the core matrix of zeros
-        const uint64_t onesBase = MakeSmemDescriptor(__shfl_sync(0xFFFFFFFFu, ctx.biasRegion, 0) + kLayer * 128, (4 - kLayer) * 128, 0);
+        const uint64_t onesBase = MakeSmemDescriptor(base + uint32_t(offsetof(RefSharedStorage, onesRegion)) + kLayer * 128, (4 - kLayer) * 128, 0);
         const uint64_t weightBase = MakeSmemDescriptor(networkBase + kWeightOffset, kN * 16, 128);
         // the matrix of biases, read twice (leading offset 0): its second copy meets the zeros
         const uint64_t biasBase = MakeSmemDescriptor(networkBase + kRefInt8BiasOffset, 0, 128);
         const uint32_t elected = ElectOne();
-        const int ownChain = __shfl_sync(0xFFFFFFFFu, warpIndex >> 2, 0);
+        const int chain = __shfl_sync(0xFFFFFFFFu, warpIndex >> 2, 0);
+        const uint32_t accumulators = __shfl_sync(0xFFFFFFFFu, ctx.tmemLane, 0); // the chain's first warp has its lane 0
+        const uint64_t chainOperand = operandBase + uint64_t(uint32_t(chain) * uint32_t(kRefOperandBytes >> 4));
+        // accumulators := bias (rows e_l times the matrix whose column l is the layer's bias: exact)
+        UmmaF16(accumulators, onesBase, biasBase, instr, 0, elected);
 #pragma unroll
-        for (int half = 0; half < kRefChains; ++half)
+        for (int kStep = 0; kStep < kK / 16; ++kStep)
         {
-            if (kChainLocal && half != ownChain)
-                continue;
-            const uint32_t accumulators = tmemBase + half * kTmemColumnsPerHalf;
-            // accumulators := bias (rows e_l times the matrix whose column l is the layer's bias: exact)
-            UmmaF16(accumulators, onesBase, biasBase, instr, 0, elected);
-#pragma unroll
-            for (int kStep = 0; kStep < kK / 16; ++kStep)
-            {
-                // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
-                const uint64_t descA = operandBase + uint64_t((half * kRefOperandBytes + kStep * 2 * 2048) >> 4);
-                const uint64_t descB = weightBase + uint64_t((kStep * 2 * kN * 16) >> 4);
-                if (kStep >= kRefFirstTmemStep<kLayer>)
-                    UmmaF16FromTmem(accumulators, accumulators + kRefOperandColumn + uint32_t(kStep) * 8u, descB, instr, 1, elected);
-                else
-                    UmmaF16(accumulators, descA, descB, instr, 1, elected);
-            }
-            // arrives once everything issued so far has completed: this chain's accumulators are ready
-            if (elected)
-                UmmaCommit(barrierBase + half * 8);
+            // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
+            const uint64_t descA = chainOperand + uint64_t((kStep * 2 * 2048) >> 4);
+            const uint64_t descB = weightBase + uint64_t((kStep * 2 * kN * 16) >> 4);
+            if (kStep >= kRefFirstTmemStep<kLayer>)
+                UmmaF16FromTmem(accumulators, accumulators + kRefOperandColumn + uint32_t(kStep) * 8u, descB, instr, 1, elected);
+            else
+                UmmaF16(accumulators, descA, descB, instr, 1, elected);
         }
+        // arrives once everything issued so far has completed: the chain's accumulators are ready
+        if (elected)
+            UmmaCommit(base + uint32_t(offsetof(RefSharedStorage, barrier)) + chain * 8);
     }
     return 0;
 }
@@ -496,13 +502,13 @@ __device__ __forceinline__ int IssueLayerRef(const RefTileContext& ctx, int fail
 // Second half of a layer: waits for the MMA, then applies the activation and writes the next
 // layer's A operand (layers 0-2) or stores the texel (layer 3).
 template <bool kFp8, int kLayer, bool kConvert, typename Params>
-__device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefTileContext& ctx, uint32_t& phase, int& failed)
+__device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefTileContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
 
     if (!MbarrierWaitBounded(ctx.barrier, phase))
     {
-        failed = 1;
+        SetGiveUp(ctx.giveUp);
         ReportTimeout(params.status, uint32_t(ctx.tile), uint32_t(kLayer));
     }
     phase ^= 1;
@@ -563,28 +569,21 @@ __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefT
     }
 }
 
-template <bool kFp8, int kLayer, bool kConvert, int kChainLocal = TileLayerBarrier<kLayer>(), typename Params>
-__device__ __forceinline__ int RunLayerRef(const Params& params, const RefTileContext& ctx, uint32_t& phase, int& failed)
+template <bool kFp8, int kLayer, bool kConvert, typename Params>
+__device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext& ctx, uint32_t& phase)
 {
-    if (IssueLayerRef<kLayer, kChainLocal>(ctx, failed))
+    if (IssueLayerRef<kLayer>(ctx))
         return 1;
-    ConsumeLayerRef<kFp8, kLayer, kConvert>(params, ctx, phase, failed);
+    ConsumeLayerRef<kFp8, kLayer, kConvert>(params, ctx, phase);
     return 0;
 }
 
 // One-time setup of a CTA: the network image arrives by one TMA bulk copy while the threads fill
 // the constant tables, set up the barriers and allocate tensor memory.  Returns nonzero in every
 // thread that gave up waiting for the image (status words written).
-__device__ __forceinline__ int SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
+__device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
     GridDependencyLaunch();
-    // src/Quantizer.cu:490-495: value = float(nibble) * (1.f / 15.f), stored as binary16
-    for (int i = tid; i < 256; i += kRefThreadsPerCta)
-    {
-        __half lo = __float2half_rn(__fmul_rn(float(i & 15), 1.f / 15.f));
-        __half hi = __float2half_rn(__fmul_rn(float(i >> 4), 1.f / 15.f));
-        shared.latentTable[i] = AsU32(__halves2half2(lo, hi));
-    }
     // constant A operands of the bias steps: core matrix l (8 rows of 16 bytes) has 1.0 as half l of every row,
     // core matrix 4 is zero
     for (int i = tid; i < 5 * 8; i += kRefThreadsPerCta)
@@ -597,7 +596,10 @@ __device__ __forceinline__ int SetupCtaRef(RefSharedStorage& shared, const uint8
     if (tid == 0)
     {
         for (int chain = 0; chain < kRefChains; ++chain)
+        {
             MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
+            shared.giveUp[chain][0] = shared.giveUp[chain][1] = 0;
+        }
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
     }
@@ -613,31 +615,30 @@ __device__ __forceinline__ int SetupCtaRef(RefSharedStorage& shared, const uint8
     TcgenFenceBeforeSync();
     __syncthreads();
     TcgenFenceAfterSync();
-    int failed = 0;
     if (!MbarrierWaitBounded(loadBarrier, 0, loadWaitPolls))
     {
-        failed = 1;
+        SetGiveUp(SharedAddress(&shared.giveUp[tid >> 7][0]));
         ReportTimeout(status, 0xFFFFFFFFu, 0xFFFFFFFFu); // no tile: the network image did not arrive
     }
-    return failed;
 }
 
 // End of a CTA: agrees on whether anything went wrong, gives work in flight one more bounded chance
 // to drain, and releases the tensor memory.
-__device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const RefTileContext& ctx, uint32_t phase, int failed,
+__device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const RefTileContext& ctx, uint32_t phase,
     int tid, int warp)
 {
     TcgenFenceBeforeSync();
-    const int aborted = __syncthreads_or(failed);
-    if (aborted && tid == 0)
+    __syncthreads();
+    const volatile uint32_t* gaveUp = &shared.giveUp[0][0];
+    if (tid == 0 && (gaveUp[0] | gaveUp[1] | gaveUp[2] | gaveUp[3]))
     {
         for (int chain = 0; chain < kRefChains; ++chain)
-            (void)MbarrierWaitBounded(ctx.barrierBase + chain * 8, phase ^ 1);
+            (void)MbarrierWaitBounded(SharedAddress(&shared.barrier[chain]), phase ^ 1);
         (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
     }
     __syncthreads();
     if (warp == 0)
-        TmemFree(ctx.tmemBase, kRefTmemColumns);
+        TmemFree(shared.tmemBase, kRefTmemColumns);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -652,26 +653,23 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int warp = tid >> 5;      // = the thread's row of the tile
-    const int half = warp >> 2;     // the 128-row chain of this thread: rows 4 * half .. + 3 of the tile
+    const int warp = tid >> 5;
+    const int chain = warp >> 2, chainWarp = warp & 3;
+    const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
-    int failed = SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp); // this thread gave up on a wait
-    const uint32_t tmemBase = shared.tmemBase;
+    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
     uint32_t phase = 0;
-    int aborted = 0;  // some thread of the CTA gave up (uniform: comes out of a barrier)
+    int aborted = 0;  // some thread of the chain gave up (uniform over the chain)
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemBase = tmemBase;
     // a warp may only touch the TMEM lanes 32 * (warp % 4) .. + 31
-    ctx.tmemLane = tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrierBase = SharedAddress(&shared.barrier[0]);
-    ctx.barrier = ctx.barrierBase + half * 8;
-    ctx.operandA = SharedAddress(shared.operandA);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kRefOperandBytes) + (tid & 127);
-    ctx.networkBase = SharedAddress(shared.network);
-    ctx.biasRegion = SharedAddress(shared.onesRegion);
+    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
 
+    RefStage& stage = shared.stage[chain];
     struct TilePlace
     {
         int mipIndex, tileX0, tileY0;
@@ -683,50 +681,49 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
             ++place.mipIndex;
         const KernelMip& mip = params.mips[place.mipIndex];
         const int local = tile - mip.firstTile;
-        const int tileY = mip.tilesX == 1 ? local : int(__umulhi(uint32_t(local), mip.tilesXMagic));
-        place.tileX0 = (local - tileY * mip.tilesX) * kTileWidth;
-        place.tileY0 = mip.rowBegin + tileY * kRefTileHeight;
+        const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
+        place.tileX0 = (local - tileY * mip.tilesX) * kChainTileWidth;
+        place.tileY0 = mip.rowBegin + tileY * kChainTileHeight;
         return place;
     };
 
-    int tile = blockIdx.x;
+    // the first chains of all CTAs take the first tiles, so that a launch of few tiles spreads over the SMs
+    int tile = int(blockIdx.x) + chain * int(gridDim.x);
     TilePlace place{0, 0, 0};
     int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
     if (tile < params.totalTiles)
     {
         place = locate(tile, 0);
-        PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], shared, place.tileX0, place.tileY0, lane, warp, false);
-        tablesMip = TileKeepsTables(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
-        __syncthreads();
+        PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, false);
+        tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
+        ChainBarrier(chain);
     }
     while (tile < params.totalTiles)
     {
         const KernelMip& mip = params.mips[place.mipIndex];
         ctx.tile = tile;
-        ctx.x = place.tileX0 + lane;
-        ctx.y = place.tileY0 + warp;
-        BuildInputsRef<kFp8, kLayers>(params, mip, shared, ctx, lane, warp);
+        ctx.x = place.tileX0 + tileColumn;
+        ctx.y = place.tileY0 + tileRow;
+        BuildInputsRef<kFp8, kLayers>(params, mip, stage, ctx, tileColumn, tileRow);
 
-        // layer 0; while the tensor core works on it, prepare the NEXT tile (its tables and
+        // layer 0; while the tensor core works on it, prepare the chain's NEXT tile (its tables and
         // footprints replace this tile's, which nobody reads after the barrier inside IssueLayerRef)
-        aborted = IssueLayerRef<0>(ctx, failed);
+        aborted = IssueLayerRef<0>(ctx);
         if (aborted)
             break;
-        const int nextTile = tile + int(gridDim.x);
+        const int nextTile = tile + kRefChains * int(gridDim.x);
         if (nextTile < params.totalTiles)
         {
             place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = TileKeepsTables(params.mips[place.mipIndex], place.tileX0, place.tileY0);
-            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], shared, place.tileX0, place.tileY0, lane, warp, keepsTables && place.mipIndex == tablesMip);
+            const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
+            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, keepsTables && place.mipIndex == tablesMip);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
-        ConsumeLayerRef<kFp8, 0, false>(params, ctx, phase, failed);
+        ConsumeLayerRef<kFp8, 0, false>(params, ctx, phase);
 
-        aborted = RunLayerRef<kFp8, 1, false>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRef<kFp8, 2, false>(params, ctx, phase, failed);
-        if (aborted)
-            break;
+        RunLayerRef<kFp8, 1, false>(params, ctx, phase);
+        RunLayerRef<kFp8, 2, false>(params, ctx, phase);
         {
             // where the texel goes (worked out only now: nothing of it has to stay in registers through the
             // layers); the element index inside a mip fits 32 bits (checked on the host)
@@ -750,13 +747,11 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
                 ctx.storeBytes = mip.storeBytes;
             }
         }
-        aborted = RunLayerRef<kFp8, 3, kConvert>(params, ctx, phase, failed);
-        if (aborted)
-            break;
+        RunLayerRef<kFp8, 3, kConvert>(params, ctx, phase);
         tile = nextTile;
     }
 
-    TeardownCtaRef(shared, ctx, phase, failed, tid, warp);
+    TeardownCtaRef(shared, ctx, phase, tid, warp);
 }
 
 // Inference on sample with the reference's numerics: one thread per query (u, v, lod) -> the texel
@@ -776,22 +771,18 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
     // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCtaRef)
     if (tid < params.numMips)
         mipTable[tid] = params.mips[tid];
-    int failed = SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
     int aborted = 0;
     uint32_t phase = 0;
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemBase = shared.tmemBase;
-    ctx.tmemLane = ctx.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrierBase = SharedAddress(&shared.barrier[0]);
-    ctx.barrier = ctx.barrierBase + half * 8;
-    ctx.operandA = SharedAddress(shared.operandA);
+    ctx.tmemLane = shared.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[half]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[half][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kRefOperandBytes) + (tid & 127);
-    ctx.networkBase = SharedAddress(shared.network);
-    ctx.biasRegion = SharedAddress(shared.onesRegion);
     ctx.outStepWords = 1;
-    ctx.storeBytes = 4;
+    ctx.storeBytes = params.storeBytes;
 
     const uint32_t zeroPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(0.f)));
     const unsigned long long tiles = (params.numQueries + kRefThreadsPerCta - 1) / kRefThreadsPerCta;
@@ -840,7 +831,10 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
                 SetupTaps(su, sv, mip.loWidth, mip.loHeight, lowTaps);
                 SampleInterleaved(hi, lo, params.numLayers, taps, lowTaps,
                     [&](int grid, int layer, uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11) {
-                        BlendPixelsRef<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, shared.latentTable, words + 8 * grid + 2 * layer);
+                        BlendLayersRef<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, words + 8 * grid + 2 * layer);
+                    },
+                    [&](int grid, int layer, uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11) {
+                        BlendPixelsRef<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, words + 8 * grid + 2 * layer);
                     });
             }
             else
@@ -848,12 +842,12 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
 #pragma unroll
                 for (int layer = 0; layer < 4; ++layer)
                     if (layer < params.numLayers)
-                        SampleLayerRef<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, shared.latentTable, words + 2 * layer);
+                        SampleLayerRef<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
                 SetupTaps(su, sv, mip.loWidth, mip.loHeight, taps);
 #pragma unroll
                 for (int layer = 0; layer < 4; ++layer)
                     if (layer < params.numLayers)
-                        SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, shared.latentTable, words + 8 + 2 * layer);
+                        SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
             }
             // src/RegressionKernels.h:59-85: per wave the inputs (x phase 0, y phase 0, x phase 0.25, y phase 0.25)
             float xf = __fmul_rn(float(x), mip.positionScale);
@@ -877,14 +871,14 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
         }
 
         // nothing is shared between the chains of a query tile: each runs at its own pace
-        aborted = RunLayerRef<kFp8, 0, false, 2>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRef<kFp8, 1, false, 2>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRef<kFp8, 2, false, 2>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRef<kFp8, 3, false, 2>(params, ctx, phase, failed);
+        aborted = RunLayerRef<kFp8, 0, false>(params, ctx, phase);
         if (aborted)
             break;
+        RunLayerRef<kFp8, 1, false>(params, ctx, phase);
+        RunLayerRef<kFp8, 2, false>(params, ctx, phase);
+        RunLayerRef<kFp8, 3, false>(params, ctx, phase);
     }
-    TeardownCtaRef(shared, ctx, phase, failed, tid, warp);
+    TeardownCtaRef(shared, ctx, phase, tid, warp);
 }
 
 // =============================================================================================
@@ -903,21 +897,22 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
 // activations, weights rebuilt from int8) stays on the binary16 path; its 32 inputs fit the same
 // 64-byte rows.
 
+using RefFp8Stage = ChainStage<TileTables<ChainTile>, kRefFootprintHiBytes, kRefFootprintLoBytes>;
+
 struct __align__(128) RefFp8SharedStorage
 {
     uint8_t network[kRefNetworkBytes];                  // layers 0-2: split e4m3 weight copies; layer 3 and bias steps: binary16
     alignas(128) uint8_t operandA[2 * kOperandBytes];   // A operands (top half, bottom half): 128 rows x 64 bytes each
     alignas(128) uint8_t biasRegion[128 * 32];          // constant binary16 A operand of the bias step: rows (1, 0 x 15)
-    uint32_t latentTable[256];
     uint64_t barrier[kRefChains]; // MMA completion, per chain
     uint64_t loadBarrier;         // arrival of the network image
+    alignas(8) uint32_t giveUp[kRefChains][2]; // see LayerBarrier
     uint32_t tmemBase;
-    // what inference on sample does not use comes last: its launches ask for the bytes before `tables` only
+    // what inference on sample does not use comes last: its launches ask for the bytes before `stage` only
     // (with the whole structure a sample kernel's static table of mips would cost it the fourth CTA per SM)
-    alignas(128) TileTables tables;
-    uint8_t footprintHi[kRefFootprintHiBytes];
-    uint8_t footprintLo[kRefFootprintLoBytes];
+    alignas(128) RefFp8Stage stage[kRefChains];
 };
+static_assert(sizeof(RefFp8SharedStorage) <= kMaxSharedBytes<kCtasPerSmRefFp8>, "resident CTAs must fit into shared memory");
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 e4m3 operands, binary16 accumulators.
 __device__ __forceinline__ void UmmaE4m3F16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
@@ -949,46 +944,29 @@ __device__ __forceinline__ void UmmaE4m3F16FromTmem(uint32_t tmemD, uint32_t tme
         : "memory");
 }
 
-// What the matrix products of a layer address, the same for every tile: descriptors of the operand regions
-// (those of chain 1 lie kOperandBytes further) and the accumulator columns.
-struct ChainBases
-{
-    uint64_t operand, ones, weight, bias;
-    uint32_t accumulators, barrierBase;
-};
-
+// The matrix products of one layer of a chain's tile, issued by the thread with `enabled` set.  `accumulators`: the chain's
+// first tensor-memory column.
 template <int kLayer>
-__device__ __forceinline__ ChainBases MakeChainBases(const RefTileContext& ctx)
+__device__ __forceinline__ void IssueChainRefFp8(int chain, uint32_t accumulators, uint32_t enabled)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
+    constexpr int kK = kLayer == 0 ? 48 : kLayer == 1 ? 64 : kLayer == 2 ? 48 : 32;
     constexpr int kWeightOffset =
         kLayer == 0 ? kRefWeightOffset0 : kLayer == 1 ? kRefWeightOffset1 : kLayer == 2 ? kRefWeightOffset2 : kRefWeightOffset3;
     constexpr int kBiasOffset =
         kLayer == 0 ? kRefBiasOffset0 : kLayer == 1 ? kRefBiasOffset1 : kLayer == 2 ? kRefBiasOffset2 : kRefBiasOffset3;
-    ChainBases bases;
-    // The issuing thread is the critical path of the layer: the four base descriptors are built
-    // once, every operand is then a constant offset (in 16-byte units) added to the address field.
-    bases.operand = MakeSmemDescriptor(ctx.operandA, 2048, 128);
-    bases.ones = MakeSmemDescriptor(ctx.biasRegion, 2048, 128);
-    bases.weight = MakeSmemDescriptor(ctx.networkBase + kWeightOffset, kN * 16, 128);
-    bases.bias = MakeSmemDescriptor(ctx.networkBase + kBiasOffset, kN * 16, 128);
-    bases.accumulators = ctx.tmemBase;
-    bases.barrierBase = ctx.barrierBase;
-    return bases;
-}
-
-// The matrix products of one layer for one chain of the tile, issued by the calling thread.
-template <int kLayer>
-__device__ __forceinline__ void IssueChainRefFp8(const ChainBases& bases, int half, uint32_t enabled)
-{
-    constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
-    constexpr int kK = kLayer == 0 ? 48 : kLayer == 1 ? 64 : kLayer == 2 ? 48 : 32;
     // both descriptors: binary16 accumulators, operand formats 0 (binary16 for kind::f16, e4m3 for kind::f8f6f4)
     constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
-    const uint64_t operandBase = bases.operand + uint64_t(uint32_t(half) * uint32_t(kOperandBytes >> 4));
-    const uint32_t accumulators = bases.accumulators + half * kTmemColumnsPerHalf;
+    // The issuing thread is the critical path of the layer: the four base descriptors are built
+    // once, every operand is then a constant offset (in 16-byte units) added to the address field.
+    const uint32_t base = DynamicSharedBase(), networkBase = base + uint32_t(offsetof(RefFp8SharedStorage, network));
+    const uint64_t operandBase =
+        MakeSmemDescriptor(base + uint32_t(offsetof(RefFp8SharedStorage, operandA)) + uint32_t(chain) * uint32_t(kOperandBytes), 2048, 128);
+    const uint64_t onesBase = MakeSmemDescriptor(base + uint32_t(offsetof(RefFp8SharedStorage, biasRegion)), 2048, 128);
+    const uint64_t weightBase = MakeSmemDescriptor(networkBase + kWeightOffset, kN * 16, 128);
+    const uint64_t biasBase = MakeSmemDescriptor(networkBase + kBiasOffset, kN * 16, 128);
     // accumulators := bias (binary16 step: rows (1, 0, ...) times the bias column: exact)
-    UmmaF16(accumulators, bases.ones, bases.bias, instr, 0, enabled);
+    UmmaF16(accumulators, onesBase, biasBase, instr, 0, enabled);
 #pragma unroll
     for (int step = 0; step < kK / 16; ++step)
     {
@@ -996,7 +974,7 @@ __device__ __forceinline__ void IssueChainRefFp8(const ChainBases& bases, int ha
         {
             // 16 products of the 32-wide chunk step / 2: weight copy `step` has the other 16 columns zeroed
             const uint64_t descA = operandBase + uint64_t(((step / 2) * 2 * 2048) >> 4);
-            const uint64_t descB = bases.weight + uint64_t((step * kN * 32) >> 4);
+            const uint64_t descB = weightBase + uint64_t((step * kN * 32) >> 4);
             if (kTmemOperand && kLayer > 0)
                 UmmaE4m3F16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step / 2) * 8u, descB, instr, 1, enabled);
             else
@@ -1006,7 +984,7 @@ __device__ __forceinline__ void IssueChainRefFp8(const ChainBases& bases, int ha
         {
             // binary16 operands: one K step = two core matrices of 8 halves
             const uint64_t descA = operandBase + uint64_t((step * 2 * 2048) >> 4);
-            const uint64_t descB = bases.weight + uint64_t((step * 2 * kN * 16) >> 4);
+            const uint64_t descB = weightBase + uint64_t((step * 2 * kN * 16) >> 4);
             if (kTmemOperand)
                 UmmaF16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step) * 8u, descB, instr, 1, enabled);
             else
@@ -1015,34 +993,13 @@ __device__ __forceinline__ void IssueChainRefFp8(const ChainBases& bases, int ha
     }
     // arrives once everything issued so far has completed: this chain's accumulators are ready
     if (enabled)
-        UmmaCommit(bases.barrierBase + half * 8);
-}
-
-template <int kLayer>
-__device__ __forceinline__ void IssueChainRefFp8(const RefTileContext& ctx, int half, uint32_t enabled)
-{
-    IssueChainRefFp8<kLayer>(MakeChainBases<kLayer>(ctx), half, enabled);
-}
-
-// The issuing warp's view of the context: values the compiler can see are the same in every lane.
-__device__ __forceinline__ RefTileContext UniformContext(const RefTileContext& ctx)
-{
-    RefTileContext uniform = ctx;
-    uniform.operandA = __shfl_sync(0xFFFFFFFFu, ctx.operandA, 0);
-    uniform.biasRegion = __shfl_sync(0xFFFFFFFFu, ctx.biasRegion, 0);
-    uniform.networkBase = __shfl_sync(0xFFFFFFFFu, ctx.networkBase, 0);
-    uniform.tmemBase = __shfl_sync(0xFFFFFFFFu, ctx.tmemBase, 0);
-    uniform.barrierBase = __shfl_sync(0xFFFFFFFFu, ctx.barrierBase, 0);
-    return uniform;
+        UmmaCommit(base + uint32_t(offsetof(RefFp8SharedStorage, barrier)) + chain * 8);
 }
 
 // First half of a layer: hands the A operand written before this call to the tensor core.  Returns
-// nonzero (uniformly over the CTA) when some thread gave up on a wait.
-// (Tried and dropped: letting the two chains run apart between tiles - each chain with its own
-// issuing thread waiting on an mbarrier its 128 threads arrive on - was 4 % slower than this
-// CTA-wide barrier with one issuing thread.)
-template <int kLayer, int kChainLocal = TileLayerBarrier<kLayer>()>
-__device__ __forceinline__ int IssueLayerRefFp8(const RefTileContext& ctx, int failed)
+// nonzero (uniformly over the chain) when some thread gave up on a wait.
+template <int kLayer>
+__device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
 {
     // Makes the A operand visible to the tensor core (async proxy), orders this thread's reads of the
     // previous layer's accumulators before they are overwritten, and agrees on giving up.
@@ -1055,32 +1012,19 @@ __device__ __forceinline__ int IssueLayerRefFp8(const RefTileContext& ctx, int f
     else if (!(kAblate & 128))
         FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
-    if (kAblate & 1024)
-        ;
-    else if (kAblate & 256)
-        __syncthreads();
-    else if (LayerBarrier<kChainLocal>(ctx.tid, failed))
+    if (!(kAblate & 1024) && LayerBarrier<kLayer>(ctx.tid, ctx.giveUp))
         return 1;
     // The whole issuing warp runs the descriptor arithmetic, on values the compiler can see are the same
-    // in every lane (hence the shuffles), and one elected lane hands the work to the tensor core: issued
+    // in every lane (hence the shuffles, and addresses counted from the start of dynamic shared memory instead of taken from
+    // the context: five shuffles per layer less were 2 %), and one elected lane hands the work to the tensor core: issued
     // from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
     // (Tried: building the descriptors before the barrier - 3 % slower.)
     const int warpIndex = ctx.tid >> 5;
-    // (after a CTA-wide barrier one warp issues both chains: each chain's first warp issuing its own was 1 % slower)
-    constexpr bool kOwnChainOnly = kChainLocal != 0;
-    if ((kOwnChainOnly ? (warpIndex & 3) == 0 : warpIndex == kIssuingWarp) && !(kAblate & 16))
+    if ((warpIndex & 3) == 0 && !(kAblate & 16))
     {
         TcgenFenceAfterSync();
-        const ChainBases bases = MakeChainBases<kLayer>(UniformContext(ctx));
         const uint32_t elected = ElectOne();
-        if (kOwnChainOnly)
-            IssueChainRefFp8<kLayer>(bases, __shfl_sync(0xFFFFFFFFu, warpIndex >> 2, 0), elected);
-        else
-        {
-#pragma unroll
-            for (int half = 0; half < kRefChains; ++half)
-                IssueChainRefFp8<kLayer>(bases, half, elected);
-        }
+        IssueChainRefFp8<kLayer>(__shfl_sync(0xFFFFFFFFu, warpIndex >> 2, 0), __shfl_sync(0xFFFFFFFFu, ctx.tmemLane, 0), elected);
     }
     return 0;
 }
@@ -1097,7 +1041,7 @@ __device__ __forceinline__ uint32_t ActivateToE4m3(uint32_t bits)
 }
 
 template <int kLayer, bool kConvert, typename Params>
-__device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const RefTileContext& ctx, uint32_t& phase, int& failed)
+__device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const RefTileContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
 
@@ -1107,7 +1051,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     // hint, the same speed.)
     if (!(kAblate & 16) && !MbarrierWaitBounded(ctx.barrier, phase))
     {
-        failed = 1;
+        SetGiveUp(ctx.giveUp);
         ReportTimeout(params.status, uint32_t(ctx.tile), uint32_t(kLayer));
     }
     phase ^= 1;
@@ -1258,32 +1202,29 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     }
 }
 
-template <int kLayer, bool kConvert, int kChainLocal = TileLayerBarrier<kLayer>(), typename Params>
-__device__ __forceinline__ int RunLayerRefFp8(const Params& params, const RefTileContext& ctx, uint32_t& phase, int& failed)
+template <int kLayer, bool kConvert, typename Params>
+__device__ __forceinline__ int RunLayerRefFp8(const Params& params, RefTileContext& ctx, uint32_t& phase)
 {
-    if (IssueLayerRefFp8<kLayer, kChainLocal>(ctx, failed))
+    if (IssueLayerRefFp8<kLayer>(ctx))
         return 1;
-    ConsumeLayerRefFp8<kLayer, kConvert>(params, ctx, phase, failed);
+    ConsumeLayerRefFp8<kLayer, kConvert>(params, ctx, phase);
     return 0;
 }
 
 // Setup and teardown as for the binary16 kernel, on the FP8 kernel's shared-memory structure.
-__device__ __forceinline__ int SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
+__device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
     GridDependencyLaunch();
-    for (int i = tid; i < 256; i += kThreadsPerCta)
-    {
-        __half lo = __float2half_rn(__fmul_rn(float(i & 15), 1.f / 15.f));
-        __half hi = __float2half_rn(__fmul_rn(float(i >> 4), 1.f / 15.f));
-        shared.latentTable[i] = AsU32(__halves2half2(lo, hi));
-    }
     for (int i = tid; i < 128 * 32 / 16; i += kThreadsPerCta)
         reinterpret_cast<uint4*>(shared.biasRegion)[i] = make_uint4(i < 128 ? 0x00003C00u : 0u, 0u, 0u, 0u);
     const uint32_t loadBarrier = SharedAddress(&shared.loadBarrier);
     if (tid == 0)
     {
         for (int chain = 0; chain < kRefChains; ++chain)
+        {
             MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
+            shared.giveUp[chain][0] = shared.giveUp[chain][1] = 0;
+        }
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
     }
@@ -1299,29 +1240,28 @@ __device__ __forceinline__ int SetupCtaRefFp8(RefFp8SharedStorage& shared, const
     TcgenFenceBeforeSync();
     __syncthreads();
     TcgenFenceAfterSync();
-    int failed = 0;
     if (!MbarrierWaitBounded(loadBarrier, 0, loadWaitPolls))
     {
-        failed = 1;
+        SetGiveUp(SharedAddress(&shared.giveUp[tid >> 7][0]));
         ReportTimeout(status, 0xFFFFFFFFu, 0xFFFFFFFFu); // no tile: the network image did not arrive
     }
-    return failed;
 }
 
-__device__ __forceinline__ void TeardownCtaRefFp8(RefFp8SharedStorage& shared, const RefTileContext& ctx, uint32_t phase, int failed,
+__device__ __forceinline__ void TeardownCtaRefFp8(RefFp8SharedStorage& shared, const RefTileContext& ctx, uint32_t phase,
     int tid, int warp)
 {
     TcgenFenceBeforeSync();
-    const int aborted = __syncthreads_or(failed);
-    if (aborted && tid == 0)
+    __syncthreads();
+    const volatile uint32_t* gaveUp = &shared.giveUp[0][0];
+    if (tid == 0 && (gaveUp[0] | gaveUp[1] | gaveUp[2] | gaveUp[3]))
     {
         for (int chain = 0; chain < kRefChains; ++chain)
-            (void)MbarrierWaitBounded(ctx.barrierBase + chain * 8, phase ^ 1);
+            (void)MbarrierWaitBounded(SharedAddress(&shared.barrier[chain]), phase ^ 1);
         (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
     }
     __syncthreads();
     if (warp == 0)
-        TmemFree(ctx.tmemBase, kTmemColumns);
+        TmemFree(shared.tmemBase, kTmemColumns);
 }
 
 template <bool kConvert, int kLayers>
@@ -1332,24 +1272,22 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int warp = tid >> 5;      // = the thread's row of the tile
-    const int half = warp >> 2;     // the 128-row chain of this thread
+    const int warp = tid >> 5;
+    const int chain = warp >> 2, chainWarp = warp & 3;
+    const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
-    int failed = SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
     uint32_t phase = 0;
     int aborted = 0;
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemBase = shared.tmemBase;
-    ctx.tmemLane = ctx.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrierBase = SharedAddress(&shared.barrier[0]);
-    ctx.barrier = ctx.barrierBase + half * 8;
-    ctx.operandA = SharedAddress(shared.operandA);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kOperandBytes) + (tid & 127);
-    ctx.networkBase = SharedAddress(shared.network);
-    ctx.biasRegion = SharedAddress(shared.biasRegion);
+    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kOperandBytes) + (tid & 127);
 
+    RefFp8Stage& stage = shared.stage[chain];
     struct TilePlace
     {
         int mipIndex, tileX0, tileY0;
@@ -1361,28 +1299,29 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
             ++place.mipIndex;
         const KernelMip& mip = params.mips[place.mipIndex];
         const int local = tile - mip.firstTile;
-        const int tileY = mip.tilesX == 1 ? local : int(__umulhi(uint32_t(local), mip.tilesXMagic));
-        place.tileX0 = (local - tileY * mip.tilesX) * kTileWidth;
-        place.tileY0 = mip.rowBegin + tileY * kTileHeight;
+        const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
+        place.tileX0 = (local - tileY * mip.tilesX) * kChainTileWidth;
+        place.tileY0 = mip.rowBegin + tileY * kChainTileHeight;
         return place;
     };
 
-    int tile = blockIdx.x;
+    // the first chains of all CTAs take the first tiles, so that a launch of few tiles spreads over the SMs
+    int tile = int(blockIdx.x) + chain * int(gridDim.x);
     TilePlace place{0, 0, 0};
     int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
     if (tile < params.totalTiles)
     {
         place = locate(tile, 0);
-        PrepareTile<true, true, kLayers>(params, params.mips[place.mipIndex], shared, place.tileX0, place.tileY0, lane, warp, false);
-        tablesMip = TileKeepsTables(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
-        __syncthreads();
+        PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, false);
+        tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
+        ChainBarrier(chain);
     }
     while (tile < params.totalTiles)
     {
         const KernelMip& mip = params.mips[place.mipIndex];
         ctx.tile = tile;
-        ctx.x = place.tileX0 + lane;
-        ctx.y = place.tileY0 + warp;
+        ctx.x = place.tileX0 + tileColumn;
+        ctx.y = place.tileY0 + tileRow;
         // the e4m3 input stage is the one of the exact-accumulation kernel (64-byte rows of codes)
         if (kAblate & 2)
         {
@@ -1392,29 +1331,27 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
                 ctx.rowChunk[chunk * 128] = make_uint4(filler, filler + chunk, filler, filler);
         }
         else
-            BuildInputs<true, true, kLayers>(params, mip, shared, ctx, lane, warp);
+            BuildInputs<true, true, kLayers>(params, mip, stage, ctx, tileColumn, tileRow);
 
-        aborted = IssueLayerRefFp8<0>(ctx, failed);
+        aborted = IssueLayerRefFp8<0>(ctx);
         if (aborted)
             break;
-        const int nextTile = tile + int(gridDim.x);
+        const int nextTile = tile + kRefChains * int(gridDim.x);
         if (nextTile < params.totalTiles)
         {
             if (!(kAblate & 512))
                 place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = (kAblate & 512) ? true : TileKeepsTables(params.mips[place.mipIndex], place.tileX0, place.tileY0);
+            const bool keepsTables = (kAblate & 512) ? true : TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
             if (!(kAblate & 1))
-                PrepareTile<true, true, kLayers>(params, params.mips[place.mipIndex], shared, place.tileX0, place.tileY0, lane, warp,
+                PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp,
                     keepsTables && place.mipIndex == tablesMip && !(kAblate & 64));
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
-        ConsumeLayerRefFp8<0, false>(params, ctx, phase, failed);
+        ConsumeLayerRefFp8<0, false>(params, ctx, phase);
 
-        aborted = RunLayerRefFp8<1, false>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRefFp8<2, false>(params, ctx, phase, failed);
-        if (aborted)
-            break;
+        RunLayerRefFp8<1, false>(params, ctx, phase);
+        RunLayerRefFp8<2, false>(params, ctx, phase);
         {
             // where the texel goes (worked out only now: nothing of it has to stay in registers through the layers)
             const bool planar = params.outputLayout == kLayoutPlanarPairs;
@@ -1436,12 +1373,10 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
                 ctx.storeBytes = mip.storeBytes;
             }
         }
-        aborted = RunLayerRefFp8<3, kConvert>(params, ctx, phase, failed);
-        if (aborted)
-            break;
+        RunLayerRefFp8<3, kConvert>(params, ctx, phase);
         tile = nextTile;
     }
-    TeardownCtaRefFp8(shared, ctx, phase, failed, tid, warp);
+    TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
 }
 
 // Inference on sample for FP8 networks (8-bit operands): one thread per query, taps read straight
@@ -1458,22 +1393,18 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
 
     if (tid < params.numMips)
         mipTable[tid] = params.mips[tid];
-    int failed = SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
     int aborted = 0;
     uint32_t phase = 0;
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemBase = shared.tmemBase;
-    ctx.tmemLane = ctx.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrierBase = SharedAddress(&shared.barrier[0]);
-    ctx.barrier = ctx.barrierBase + half * 8;
-    ctx.operandA = SharedAddress(shared.operandA);
+    ctx.tmemLane = shared.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[half]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[half][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kOperandBytes) + (tid & 127);
-    ctx.networkBase = SharedAddress(shared.network);
-    ctx.biasRegion = SharedAddress(shared.biasRegion);
     ctx.outStepWords = 1;
-    ctx.storeBytes = 4;
+    ctx.storeBytes = params.storeBytes;
 
     const unsigned long long tiles = (params.numQueries + kThreadsPerCta - 1) / kThreadsPerCta;
     // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
@@ -1513,7 +1444,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
 #pragma unroll
             for (int i = 12; i < 16; ++i)
                 words[i] = 0;        // K padding
-            SampleGridsDirect<true, true>(params.latents, params.numLayers, mip, x, y, shared.latentTable, words, params.interleaved != 0);
+            SampleGridsDirect<true, true>(params.latents, params.numLayers, mip, x, y, words, params.interleaved != 0);
             // src/RegressionKernels.h:59-85
             float xf = __fmul_rn(float(x), mip.positionScale);
             float yf = __fmul_rn(float(y), mip.positionScale);
@@ -1536,14 +1467,14 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
         }
 
         // nothing is shared between the chains of a query tile: each runs at its own pace
-        aborted = RunLayerRefFp8<0, false, 2>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRefFp8<1, false, 2>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRefFp8<2, false, 2>(params, ctx, phase, failed);
-        if (!aborted) aborted = RunLayerRefFp8<3, false, 2>(params, ctx, phase, failed);
+        aborted = RunLayerRefFp8<0, false>(params, ctx, phase);
         if (aborted)
             break;
+        RunLayerRefFp8<1, false>(params, ctx, phase);
+        RunLayerRefFp8<2, false>(params, ctx, phase);
+        RunLayerRefFp8<3, false>(params, ctx, phase);
     }
-    TeardownCtaRefFp8(shared, ctx, phase, failed, tid, warp);
+    TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
 }
 
 } // namespace
@@ -1626,12 +1557,12 @@ cudaError_t LaunchSampleRef(const SampleParams& params, bool fp8, int ctas, cuda
         const unsigned long long bit = 1ull << (device & 63);
         if (!(doneMask.load(std::memory_order_acquire) & bit))
         {
-            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(offsetof(RefSharedStorage, tables)));
+            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(offsetof(RefSharedStorage, stage)));
             if (err != cudaSuccess)
                 return err;
             doneMask.fetch_or(bit, std::memory_order_release);
         }
-        return LaunchOverlapped(kernel, ctas, kRefThreadsPerCta, offsetof(RefSharedStorage, tables), stream, params);
+        return LaunchOverlapped(kernel, ctas, kRefThreadsPerCta, offsetof(RefSharedStorage, stage), stream, params);
     };
     if (fp8)
     {
@@ -1642,12 +1573,12 @@ cudaError_t LaunchSampleRef(const SampleParams& params, bool fp8, int ctas, cuda
         const unsigned long long bit = 1ull << (device & 63);
         if (!(done[1].load(std::memory_order_acquire) & bit))
         {
-            err = cudaFuncSetAttribute(SampleKernelRefFp8, cudaFuncAttributeMaxDynamicSharedMemorySize, int(offsetof(RefFp8SharedStorage, tables)));
+            err = cudaFuncSetAttribute(SampleKernelRefFp8, cudaFuncAttributeMaxDynamicSharedMemorySize, int(offsetof(RefFp8SharedStorage, stage)));
             if (err != cudaSuccess)
                 return err;
             done[1].fetch_or(bit, std::memory_order_release);
         }
-        return LaunchOverlapped(SampleKernelRefFp8, ctas, kThreadsPerCta, offsetof(RefFp8SharedStorage, tables), stream, params);
+        return LaunchOverlapped(SampleKernelRefFp8, ctas, kThreadsPerCta, offsetof(RefFp8SharedStorage, stage), stream, params);
     }
     return launch(SampleKernelRef<false>, done[0]);
 }

@@ -1,7 +1,7 @@
 // Input stage of the decode kernels whose A operand holds 8-bit codes (int8 or e4m3): per-tile
 // lookup tables, staging of the latent footprint, the bilinear gather, and the thread's 64-byte row
 // of the A operand.  `Shared` is the kernel's shared-memory structure (members tables,
-// footprintHi, footprintLo, latentTable), `Context` its per-thread tile context (members x, y,
+// footprintHi, footprintLo), `Context` its per-thread tile context (members x, y,
 // rowChunk).
 #pragma once
 
@@ -68,47 +68,88 @@ __device__ __forceinline__ uint32_t PackCodes(uint32_t pair0, uint32_t pair1)
     return __byte_perm(pair0, pair1, 0x6420);
 }
 
-// One latent pixel layer (four 4-bit features, the low 16 bits of each p) of one grid -> four quantised inputs.
+// The bilinear blend of four taps and its mapping to [-1, 1].
 // Blend order as the reference build evaluates it: fma(l11,w3, fma(l10,w2, fma(l00,w0, l01*w1))).
-template <bool kFp8>
-__device__ __forceinline__ uint32_t BlendLayer(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps,
-    const uint32_t* __restrict__ lut)
+__device__ __forceinline__ __half2 BlendTaps(__half2 l00, __half2 l01, __half2 l10, __half2 l11, __half2 w00, __half2 w01, __half2 w10,
+    __half2 w11)
 {
-    uint32_t pairs[2];
+    __half2 d = __hmul2_rn(l01, w01);
+    d = __hfma2(l00, w00, d);
+    d = __hfma2(l10, w10, d);
+    d = __hfma2(l11, w11, d);
+    return __hfma2(d, __float2half2_rn(2.f), __float2half2_rn(-1.f));
+}
+
+// One layer of one grid (the low 16 bits of each p are the tap's four features) -> the inputs (0, 1) and (2, 3), not yet quantised.
+__device__ __forceinline__ void BlendPixels(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, __half2 (&inputs)[2])
+{
+    __half2 l00[2], l01[2], l10[2], l11[2];
+    UnpackPixel(p00, l00[0], l00[1]);
+    UnpackPixel(p01, l01[0], l01[1]);
+    UnpackPixel(p10, l10[0], l10[1]);
+    UnpackPixel(p11, l11[0], l11[1]);
 #pragma unroll
     for (int j = 0; j < 2; ++j)
-    {
-        __half2 l00 = AsHalf2(lut[(p00 >> (8 * j)) & 0xFF]), l01 = AsHalf2(lut[(p01 >> (8 * j)) & 0xFF]);
-        __half2 l10 = AsHalf2(lut[(p10 >> (8 * j)) & 0xFF]), l11 = AsHalf2(lut[(p11 >> (8 * j)) & 0xFF]);
-        __half2 d = __hmul2_rn(l01, taps.w01);
-        d = __hfma2(l00, taps.w00, d);
-        d = __hfma2(l10, taps.w10, d);
-        d = __hfma2(l11, taps.w11, d);
-        d = __hfma2(d, __float2half2_rn(2.f), __float2half2_rn(-1.f));
-        pairs[j] = QuantizeInputPair<kFp8>(d);
-    }
-    return PackCodes<kFp8>(pairs[0], pairs[1]);
+        inputs[j] = BlendTaps(l00[j], l01[j], l10[j], l11[j], taps.w00, taps.w01, taps.w10, taps.w11);
+}
+
+// Two layers (a word of each tap) -> per feature the inputs of (first layer, second layer).
+__device__ __forceinline__ void BlendTwoLayers(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, __half2 (&inputs)[4])
+{
+    __half2 l00[4], l01[4], l10[4], l11[4];
+    UnpackTwoLayers(p00, l00);
+    UnpackTwoLayers(p01, l01);
+    UnpackTwoLayers(p10, l10);
+    UnpackTwoLayers(p11, l11);
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+        inputs[f] = BlendTaps(l00[f], l01[f], l10[f], l11[f], taps.w00, taps.w01, taps.w10, taps.w11);
+}
+
+// One layer of one grid -> four quantised inputs.
+template <bool kFp8>
+__device__ __forceinline__ uint32_t BlendLayer(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps)
+{
+    __half2 inputs[2];
+    BlendPixels(p00, p01, p10, p11, taps, inputs);
+    return PackCodes<kFp8>(QuantizeInputPair<kFp8>(inputs[0]), QuantizeInputPair<kFp8>(inputs[1]));
+}
+
+// Two layers of one grid -> four quantised inputs each.
+template <bool kFp8>
+__device__ __forceinline__ void BlendLayers(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, uint32_t* words)
+{
+    __half2 inputs[4];
+    BlendTwoLayers(p00, p01, p10, p11, taps, inputs);
+    uint32_t codes[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+        codes[f] = QuantizeInputPair<kFp8>(inputs[f]);
+    // the first layer's codes of two features, then the second layer's (e4m3: bytes 0 and 1; int8: bytes 0 and 2)
+    constexpr uint32_t kInterleave = kFp8 ? 0x5140u : 0x6240u;
+    const uint32_t low = __byte_perm(codes[0], codes[1], kInterleave), high = __byte_perm(codes[2], codes[3], kInterleave);
+    words[0] = __byte_perm(low, high, 0x5410);
+    words[1] = __byte_perm(low, high, 0x7632);
 }
 
 // ... with the taps read from one layer's plane in global memory.
 template <bool kFp8>
-__device__ __forceinline__ uint32_t SampleLayer(const uint16_t* __restrict__ plane, const GridTaps& taps,
-    const uint32_t* __restrict__ lut)
+__device__ __forceinline__ uint32_t SampleLayer(const uint16_t* __restrict__ plane, const GridTaps& taps)
 {
     uint32_t p00 = __ldg(plane + taps.o00), p01 = __ldg(plane + taps.o01);
     uint32_t p10 = __ldg(plane + taps.o10), p11 = __ldg(plane + taps.o11);
-    return BlendLayer<kFp8>(p00, p01, p10, p11, taps, lut);
+    return BlendLayer<kFp8>(p00, p01, p10, p11, taps);
 }
 
 // Both grids of a texel from the pixel-major copy of the latents (ntcb_interleave_latents): latent pixel p of a
 // grid is ONE aligned word at grid + p * slot holding its layers side by side - 8 bytes for three or four layers,
-// 4 for two, 2 for one.  `blend(grid, layer, p00, p01, p10, p11)` receives layer l of the four taps in the low 16
-// bits of its arguments.  Inference on sample, whose taps are scattered, is bound by the rate at which the L1
+// 4 for two, 2 for one.  `two(grid, layer, p00, p01, p10, p11)` receives layers l and l + 1 of the four taps, `one(...)` layer l in
+// the low 16 bits of its arguments.  Inference on sample, whose taps are scattered, is bound by the rate at which the L1
 // serves scattered words: a tap costs it one request instead of one per layer, and the eight requests of a query
 // are all in flight before the first is needed.
-template <typename Blend>
+template <typename Two, typename One>
 __device__ __forceinline__ void SampleInterleaved(const uint16_t* __restrict__ hi, const uint16_t* __restrict__ lo, int numLayers,
-    const GridTaps& hiTaps, const GridTaps& loTaps, Blend&& blend)
+    const GridTaps& hiTaps, const GridTaps& loTaps, Two&& two, One&& one)
 {
     if (numLayers >= 3)
     {
@@ -118,16 +159,16 @@ __device__ __forceinline__ void SampleInterleaved(const uint16_t* __restrict__ h
         const uint2 h10 = __ldg(wideHi + hiTaps.o10), h11 = __ldg(wideHi + hiTaps.o11);
         const uint2 l00 = __ldg(wideLo + loTaps.o00), l01 = __ldg(wideLo + loTaps.o01);
         const uint2 l10 = __ldg(wideLo + loTaps.o10), l11 = __ldg(wideLo + loTaps.o11);
-        blend(0, 0, h00.x, h01.x, h10.x, h11.x);
-        blend(0, 1, h00.x >> 16, h01.x >> 16, h10.x >> 16, h11.x >> 16);
-        blend(0, 2, h00.y, h01.y, h10.y, h11.y);
+        two(0, 0, h00.x, h01.x, h10.x, h11.x);
         if (numLayers == 4)
-            blend(0, 3, h00.y >> 16, h01.y >> 16, h10.y >> 16, h11.y >> 16);
-        blend(1, 0, l00.x, l01.x, l10.x, l11.x);
-        blend(1, 1, l00.x >> 16, l01.x >> 16, l10.x >> 16, l11.x >> 16);
-        blend(1, 2, l00.y, l01.y, l10.y, l11.y);
+            two(0, 2, h00.y, h01.y, h10.y, h11.y);
+        else
+            one(0, 2, h00.y, h01.y, h10.y, h11.y);
+        two(1, 0, l00.x, l01.x, l10.x, l11.x);
         if (numLayers == 4)
-            blend(1, 3, l00.y >> 16, l01.y >> 16, l10.y >> 16, l11.y >> 16);
+            two(1, 2, l00.y, l01.y, l10.y, l11.y);
+        else
+            one(1, 2, l00.y, l01.y, l10.y, l11.y);
     }
     else if (numLayers == 2)
     {
@@ -137,27 +178,41 @@ __device__ __forceinline__ void SampleInterleaved(const uint16_t* __restrict__ h
         const uint32_t h10 = __ldg(wideHi + hiTaps.o10), h11 = __ldg(wideHi + hiTaps.o11);
         const uint32_t l00 = __ldg(wideLo + loTaps.o00), l01 = __ldg(wideLo + loTaps.o01);
         const uint32_t l10 = __ldg(wideLo + loTaps.o10), l11 = __ldg(wideLo + loTaps.o11);
-        blend(0, 0, h00, h01, h10, h11);
-        blend(0, 1, h00 >> 16, h01 >> 16, h10 >> 16, h11 >> 16);
-        blend(1, 0, l00, l01, l10, l11);
-        blend(1, 1, l00 >> 16, l01 >> 16, l10 >> 16, l11 >> 16);
+        two(0, 0, h00, h01, h10, h11);
+        two(1, 0, l00, l01, l10, l11);
     }
     else
     {
-        blend(0, 0, __ldg(hi + hiTaps.o00), __ldg(hi + hiTaps.o01), __ldg(hi + hiTaps.o10), __ldg(hi + hiTaps.o11));
-        blend(1, 0, __ldg(lo + loTaps.o00), __ldg(lo + loTaps.o01), __ldg(lo + loTaps.o10), __ldg(lo + loTaps.o11));
+        one(0, 0, __ldg(hi + hiTaps.o00), __ldg(hi + hiTaps.o01), __ldg(hi + hiTaps.o10), __ldg(hi + hiTaps.o11));
+        one(1, 0, __ldg(lo + loTaps.o00), __ldg(lo + loTaps.o01), __ldg(lo + loTaps.o10), __ldg(lo + loTaps.o11));
     }
 }
+
+// The unit of texels whose tables and footprints are prepared together, and the warps that do it: all eight of a CTA on a
+// 32 x 8 tile (exact accumulation), or the four of a chain on a 16 x 8 tile of its own (reference numerics).
+struct WideTile
+{
+    static constexpr int kWidth = kTileWidth, kHeight = kTileHeight, kWarps = 8, kWidthLog2 = 5, kHeightLog2 = 3;
+};
+struct ChainTile
+{
+    static constexpr int kWidth = kChainTileWidth, kHeight = kChainTileHeight, kWarps = 4, kWidthLog2 = 4, kHeightLog2 = 3;
+};
+static_assert(WideTile::kWidth == 1 << WideTile::kWidthLog2 && WideTile::kHeight == 1 << WideTile::kHeightLog2 &&
+                  ChainTile::kWidth == 1 << ChainTile::kWidthLog2 && ChainTile::kHeight == 1 << ChainTile::kHeightLog2 &&
+                  WideTile::kWidth * WideTile::kHeight == 32 * WideTile::kWarps && ChainTile::kWidth * ChainTile::kHeight == 32 * ChainTile::kWarps,
+    "one thread per texel");
 
 // Per-tile lookup tables of the bilinear taps: tap position and weights are separable in x and y, so
 // they are computed once per tile column / row instead of once per texel.  Shared by every decode
 // kernel.
+template <typename Tile>
 struct __align__(16) TapTables
 {
     // per grid (0 = high-res, 1 = low-res) and tile column: byte offset of the left tap inside a footprint row, dx, 1 - dx
-    int4 colTap[2][kTileWidth];
+    int4 colTap[2][Tile::kWidth];
     // per grid and tile row: byte offset of the upper tap's footprint row, dy, 1 - dy, bytes per footprint row
-    int4 rowTap[2][kTileHeight];
+    int4 rowTap[2][Tile::kHeight];
     // per grid: footprint width and height in latent pixels, pixel count, and the multiplier that divides a
     // pixel index by the width (p / width == (p * magic) >> 20 for p < 2048)
     int4 footprint[2];
@@ -166,20 +221,20 @@ struct __align__(16) TapTables
 };
 
 // Tap tables plus the positional encoding as operand bytes (kernels whose A operand holds 8-bit codes).
+template <typename Tile>
 struct __align__(16) TileTables
 {
-    TapTables taps;
+    TapTables<Tile> taps;
     // positional-encoding operand bytes: x = {X0 w0, X1 w0, X0 w1, X1 w1}, y = {X0 w2, X1 w2, 0, 0}
-    uint2 colEnc[kTileWidth];
-    uint2 rowEnc[kTileHeight];
+    uint2 colEnc[Tile::kWidth];
+    uint2 rowEnc[Tile::kHeight];
     uint32_t lodWord;  // operand bytes of inputs 44..47: lod, lod, 0, 0
     uint32_t pad[3];
 };
 
 // Builds the tile's tap tables and stages the latent footprint of both grids in shared memory
 // (nibbles unpacked to binary16 once per latent pixel instead of once per texel and tap).
-// Even warps work on the high-res grid, odd warps on the low-res grid; the 128 threads of a grid
-// share its footprint pixels.
+// Even warps work on the high-res grid, odd warps on the low-res grid; the threads of a grid share its footprint pixels.
 // (Tried and dropped, both slower although they execute fewer instructions: two warps staging the
 // footprints while the others go on - the tile then waits for those two; and requesting the latents
 // before the wait for layer 0 and unpacking them after it.)
@@ -188,9 +243,9 @@ struct __align__(16) TileTables
 // are powers of two (KernelMip::invariant) every tile that lies wholly inside the mip has the same
 // tap offsets and fractions relative to its own footprint - all the arithmetic is exact - so the
 // tables are built for the first such tile and only the footprint is staged for the others.
-template <bool kReferenceDivision, int kLayers = 0>
-__device__ __forceinline__ void PrepareTaps(const KernelParams& params, const KernelMip& mip, TapTables& taps,
-    uint8_t* footprintHi, uint8_t* footprintLo, const uint32_t* latentTable, int tileX0, int tileY0, int lane, int warp,
+template <typename Tile, bool kReferenceDivision, int kLayers>
+__device__ __forceinline__ void PrepareTaps(const KernelParams& params, const KernelMip& mip, TapTables<Tile>& taps,
+    uint8_t* footprintHi, uint8_t* footprintLo, int tileX0, int tileY0, int lane, int warp,
     bool tablesValid)
 {
     const int grid = warp & 1;
@@ -209,8 +264,8 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
         if (32 * (warp >> 1) >= footprint.z)
             return;
         const int4 origin = taps.origin[grid];
-        fx0 = origin.x + ((tileX0 - origin.z) >> 5) * (grid ? mip.loStepX : mip.hiStepX);
-        fy0 = origin.y + ((tileY0 - origin.w) >> 3) * (grid ? mip.loStepY : mip.hiStepY);
+        fx0 = origin.x + ((tileX0 - origin.z) >> Tile::kWidthLog2) * (grid ? mip.loStepX : mip.hiStepX);
+        fy0 = origin.y + ((tileY0 - origin.w) >> Tile::kHeightLog2) * (grid ? mip.loStepY : mip.hiStepY);
         footW = footprint.x;
         count = footprint.z;
         magic = uint32_t(footprint.w);
@@ -219,19 +274,20 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
     {
         int xb, yb;
         float dx, dy;
-        AxisTap<kReferenceDivision>(min(tileX0 + lane, mip.width - 1), mip.width, mip.invWidth, gw, xb, dx);
-        AxisTap<kReferenceDivision>(min(tileY0 + (lane & (kTileHeight - 1)), mip.rowEnd - 1), mip.height, mip.invHeight, gh, yb, dy);
+        AxisTap<kReferenceDivision>(min(tileX0 + (lane & (Tile::kWidth - 1)), mip.width - 1), mip.width, mip.invWidth, gw, xb, dx);
+        AxisTap<kReferenceDivision>(min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1), mip.height, mip.invHeight, gh, yb, dy);
         fx0 = __shfl_sync(0xFFFFFFFFu, xb, 0);
         fy0 = __shfl_sync(0xFFFFFFFFu, yb, 0);
-        footW = __shfl_sync(0xFFFFFFFFu, xb, 31) - fx0 + 2;
-        const int footH = __shfl_sync(0xFFFFFFFFu, yb, kTileHeight - 1) - fy0 + 2;
+        footW = __shfl_sync(0xFFFFFFFFu, xb, Tile::kWidth - 1) - fx0 + 2;
+        const int footH = __shfl_sync(0xFFFFFFFFu, yb, Tile::kHeight - 1) - fy0 + 2;
         count = footW * footH;
         // the IEEE quotient of 2^20 / footW floors exactly
         magic = uint32_t(__float2int_rd(__fdiv_rn(1048576.f, float(footW)))) + 1;
         if (warp < 2)
         {
-            taps.colTap[grid][lane] = make_int4((xb - fx0) * stride, __float_as_int(dx), __float_as_int(__fsub_rn(1.f, dx)), 0);
-            if (lane < kTileHeight)
+            if (lane < Tile::kWidth)
+                taps.colTap[grid][lane] = make_int4((xb - fx0) * stride, __float_as_int(dx), __float_as_int(__fsub_rn(1.f, dx)), 0);
+            if (lane < Tile::kHeight)
                 taps.rowTap[grid][lane] =
                     make_int4((yb - fy0) * footW * stride, __float_as_int(dy), __float_as_int(__fsub_rn(1.f, dy)), footW * stride);
             if (lane == 0)
@@ -244,13 +300,13 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
 
     if (mip.staged)
     {
-        // footprint pixel p = fy * footW + fx, handed out over the 128 threads that share this grid
+        // footprint pixel p = fy * footW + fx, handed out over the threads that share this grid
         // (tried: one footprint row per warp - no division, but more warps with a few active lanes each:
         // 5 % more instructions and 6 % slower; prefetching the next tile's latents into L1 a tile ahead: 5 % slower)
         const uint16_t* plane0 = params.latents + (grid ? mip.loOffset : mip.hiOffset);
         const uint32_t planePixels = uint32_t(grid ? mip.loPlane : mip.hiPlane);
         uint8_t* foot = grid ? footprintLo : footprintHi;
-        for (int p = lane + 32 * (warp >> 1); p < count; p += kThreadsPerCta / 2)
+        for (int p = lane + 32 * (warp >> 1); p < count; p += 16 * Tile::kWarps)
         {
             const int fy = int((uint32_t(p) * magic) >> 20);
             const int fx = p - fy * footW;
@@ -268,7 +324,9 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
                 if (layer < NumLayers<kLayers>(params))
                 {
                     const uint32_t pixel = __ldg(plane0 + (first + uint32_t(layer) * planePixels));
-                    dst[layer] = make_uint2(latentTable[pixel & 0xFF], latentTable[pixel >> 8]);
+                    __half2 first, second;
+                    UnpackPixel(pixel, first, second);
+                    dst[layer] = make_uint2(AsU32(first), AsU32(second));
                 }
             }
         }
@@ -276,8 +334,8 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
 }
 
 // The tile's tables (taps and positional encoding as operand bytes) and its staged footprints.
-template <bool kFp8, bool kReferenceDivision, int kLayers = 0, typename Shared>
-__device__ __forceinline__ void PrepareTile(const KernelParams& params, const KernelMip& mip, Shared& shared,
+template <typename Tile, bool kFp8, bool kReferenceDivision, int kLayers, typename Stage>
+__device__ __forceinline__ void PrepareTile(const KernelParams& params, const KernelMip& mip, Stage& stage,
     int tileX0, int tileY0, int lane, int warp, bool tablesValid)
 {
     if (!tablesValid && warp >= 2 && warp < 4)
@@ -285,7 +343,8 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
         // positional encoding (src/RegressionKernels.h:59-85): warp 2 the x part per column, warp 3
         // the y part per row, quantised exactly as the per-texel inputs would be
         const bool rows = warp == 3;
-        const int coordinate = rows ? min(tileY0 + (lane & (kTileHeight - 1)), mip.rowEnd - 1) : min(tileX0 + lane, mip.width - 1);
+        const int coordinate = rows ? min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1)
+                                    : min(tileX0 + (lane & (Tile::kWidth - 1)), mip.width - 1);
         float f = __fmul_rn(float(coordinate), mip.positionScale);
         uint32_t q[3];
 #pragma unroll
@@ -297,24 +356,25 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
             f = __fmul_rn(f, 2.f);
         }
         const uint2 enc = make_uint2(PackCodes<kFp8>(q[0], q[1]), PackCodes<kFp8>(q[2], 0));
-        if (!rows)
-            shared.tables.colEnc[lane] = enc;
-        else if (lane < kTileHeight)
-            shared.tables.rowEnc[lane] = enc;
-        if (rows && lane == kTileHeight)
-            shared.tables.lodWord = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(mip.positionLod)),
+        if (!rows && lane < Tile::kWidth)
+            stage.tables.colEnc[lane] = enc;
+        if (rows && lane < Tile::kHeight)
+            stage.tables.rowEnc[lane] = enc;
+        if (rows && lane == Tile::kHeight)
+            stage.tables.lodWord = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(mip.positionLod)),
                                                    QuantizeInputPair<kFp8>(__float2half2_rn(0.f)));
     }
-    PrepareTaps<kReferenceDivision, kLayers>(params, mip, shared.tables.taps, shared.footprintHi, shared.footprintLo, shared.latentTable,
+    PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo,
         tileX0, tileY0, lane, warp, tablesValid);
 }
 
 // Whether the tables built for one tile of `mip` serve the tile at (tileX0, tileY0) too, and whether
 // tables built for that tile may be kept for later ones: the tile lies wholly inside the decoded rows
 // of a mip with invariant tables.
+template <typename Tile>
 __device__ __forceinline__ bool TileKeepsTables(const KernelMip& mip, int tileX0, int tileY0)
 {
-    return mip.invariant && tileX0 + kTileWidth <= mip.width && tileY0 + kTileHeight <= mip.rowEnd;
+    return mip.invariant && tileX0 + Tile::kWidth <= mip.width && tileY0 + Tile::kHeight <= mip.rowEnd;
 }
 
 // Four quantised inputs of one latent layer from the four staged taps.
@@ -338,12 +398,12 @@ __device__ __forceinline__ uint32_t BlendLayer(uint2 l00, uint2 l01, uint2 l10, 
 }
 
 // Inputs 0..15 or 16..31 of one texel from the staged footprint of one grid.
-template <bool kFp8, int kLayers = 0, typename Shared>
-__device__ __forceinline__ void GatherGrid(const KernelParams& params, const KernelMip& mip, const Shared& shared,
-    int grid, int lane, int tileRow, uint32_t* words)
+template <bool kFp8, int kLayers = 0, typename Stage>
+__device__ __forceinline__ void GatherGrid(const KernelParams& params, const KernelMip& mip, const Stage& stage,
+    int grid, int tileColumn, int tileRow, uint32_t* words)
 {
-    const int4 col = shared.tables.taps.colTap[grid][lane];
-    const int4 row = shared.tables.taps.rowTap[grid][tileRow];
+    const int4 col = stage.tables.taps.colTap[grid][tileColumn];
+    const int4 row = stage.tables.taps.rowTap[grid][tileRow];
     const float dx = __int_as_float(col.y), dxn = __int_as_float(col.z);
     const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
     // src/FeatureGridDevice.h:46-49
@@ -352,7 +412,7 @@ __device__ __forceinline__ void GatherGrid(const KernelParams& params, const Ker
     const __half2 w10 = __floats2half2_rn(f10, f10), w11 = __floats2half2_rn(f11, f11);
 
     const int stride = StrideBytes<kLayers>(mip);
-    const uint8_t* tap00 = (grid ? shared.footprintLo : shared.footprintHi) + (col.x + row.x);
+    const uint8_t* tap00 = (grid ? stage.footprintLo : stage.footprintHi) + (col.x + row.x);
     const uint8_t* tap10 = tap00 + row.w;
 #pragma unroll
     for (int layer = 0; layer < 4; ++layer)
@@ -372,7 +432,7 @@ __device__ __forceinline__ void GatherGrid(const KernelParams& params, const Ker
 // copy ntcb_interleave_latents makes instead of the file's planes; the mip's offsets then refer to that copy).
 template <bool kFp8, bool kReferenceDivision>
 __device__ __forceinline__ void SampleGridsDirect(const uint16_t* __restrict__ latents, int numLayers, const KernelMip& mip,
-    int x, int y, const uint32_t* __restrict__ latentTable, uint32_t* words, bool interleaved = false)
+    int x, int y, uint32_t* words, bool interleaved = false)
 {
     // src/Inference.cu:52-53
     const float u = TexelCoordinate<kReferenceDivision>(x, mip.width, mip.invWidth);
@@ -386,27 +446,30 @@ __device__ __forceinline__ void SampleGridsDirect(const uint16_t* __restrict__ l
         SetupTaps(u, v, mip.loWidth, mip.loHeight, lowTaps);
         SampleInterleaved(hi, latents + mip.loOffset, numLayers, taps, lowTaps,
             [&](int grid, int layer, uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11) {
-                words[4 * grid + layer] = BlendLayer<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, latentTable);
+                BlendLayers<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, words + 4 * grid + layer);
+            },
+            [&](int grid, int layer, uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11) {
+                words[4 * grid + layer] = BlendLayer<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps);
             });
         return;
     }
 #pragma unroll
     for (int layer = 0; layer < 4; ++layer)
         if (layer < numLayers)
-            words[layer] = SampleLayer<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, latentTable);
+            words[layer] = SampleLayer<kFp8>(hi + size_t(layer) * mip.hiPlane, taps);
     SetupTaps(u, v, mip.loWidth, mip.loHeight, taps);
     const uint16_t* lo = latents + mip.loOffset;
 #pragma unroll
     for (int layer = 0; layer < 4; ++layer)
         if (layer < numLayers)
-            words[4 + layer] = SampleLayer<kFp8>(lo + size_t(layer) * mip.loPlane, taps, latentTable);
+            words[4 + layer] = SampleLayer<kFp8>(lo + size_t(layer) * mip.loPlane, taps);
 }
 
 // The 48 network inputs of one texel -> its 64-byte row of the A operand (K-major core matrices:
 // 16-byte chunk j of row r lives at j * 2048 + r * 16).
-template <bool kFp8, bool kReferenceDivision, int kLayers = 0, typename Shared, typename Context>
-__device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, const Shared& shared,
-    const Context& ctx, int lane, int tileRow)
+template <bool kFp8, bool kReferenceDivision, int kLayers = 0, typename Stage, typename Context>
+__device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, const Stage& stage,
+    const Context& ctx, int tileColumn, int tileRow)
 {
     uint32_t words[16];
     const uint32_t zeroWord = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(0.f)),
@@ -421,24 +484,24 @@ __device__ __forceinline__ void BuildInputs(const KernelParams& params, const Ke
 
     if (mip.staged)
     {
-        GatherGrid<kFp8, kLayers>(params, mip, shared, 0, lane, tileRow, words);
-        GatherGrid<kFp8, kLayers>(params, mip, shared, 1, lane, tileRow, words + 4);
+        GatherGrid<kFp8, kLayers>(params, mip, stage, 0, tileColumn, tileRow, words);
+        GatherGrid<kFp8, kLayers>(params, mip, stage, 1, tileColumn, tileRow, words + 4);
     }
     else
     {
         // footprint too large to stage (strong minification): read the taps from global memory;
         // threads past the right / bottom edge compute a clamped texel and store nothing
         SampleGridsDirect<kFp8, kReferenceDivision>(params.latents, NumLayers<kLayers>(params), mip, min(ctx.x, mip.width - 1), min(ctx.y, mip.rowEnd - 1),
-            shared.latentTable, words);
+            words);
     }
 
     // positional encoding: interleave the column's x bytes with the row's y bytes
-    const uint2 cx = shared.tables.colEnc[lane];
-    const uint2 ry = shared.tables.rowEnc[tileRow];
+    const uint2 cx = stage.tables.colEnc[tileColumn];
+    const uint2 ry = stage.tables.rowEnc[tileRow];
     words[8] = __byte_perm(cx.x, ry.x, 0x5140);
     words[9] = __byte_perm(cx.x, ry.x, 0x7362);
     words[10] = __byte_perm(cx.y, ry.y, 0x5140);
-    words[11] = shared.tables.lodWord;
+    words[11] = stage.tables.lodWord;
 
 #pragma unroll
     for (int chunk = 0; chunk < 4; ++chunk)

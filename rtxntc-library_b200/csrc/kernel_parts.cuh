@@ -19,6 +19,13 @@ __device__ __forceinline__ uint32_t SharedAddress(const void* p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Start of the kernel's dynamic shared memory: a constant, so what is computed from it is visibly the same in every thread.
+__device__ __forceinline__ uint32_t DynamicSharedBase()
+{
+    extern __shared__ __align__(128) unsigned char dynamicShared[];
+    return SharedAddress(dynamicShared);
+}
+
 __device__ __forceinline__ void MbarrierInit(uint32_t bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -241,6 +248,36 @@ __device__ __forceinline__ void StoreTexel(uint32_t* out, uint32_t stepWords, in
     }
 }
 
+// Latent codes to binary16 without a table.  A code n (0 .. 15) in bits 4-7 of a binary16 is the subnormal number n * 2^-20;
+// times 2^20 / 15, in two terms because the factor is beyond the format, it becomes the value the reference's
+// fp16(float(n) * (1.f / 15.f)) has (src/Quantizer.cu:490-495): the first product is rounded, the sum too, and for all sixteen codes
+// the result is the same number (compared). Two
+// operations on two codes at a time.  (Looked up in a table of all bytes in shared memory, the 32 unrelated bytes of a warp
+// fell on 3.5 deep banks on average, 48 times per query of inference on sample, whose bound was the L1's data pipe: 16.7 M
+// queries 0.97 -> 0.84 ms without.)
+__device__ __forceinline__ __half2 CodesToHalves(uint32_t codes)
+{
+    const __half2 z = AsHalf2(codes & 0x00F000F0u);
+    return __hfma2(z, __float2half2_rn(17680.f), __hmul2_rn(z, __float2half2_rn(52224.f)));
+}
+
+// A latent pixel of one layer (four 4-bit features in the low 16 bits) -> features (0, 1) and (2, 3).
+__device__ __forceinline__ void UnpackPixel(uint32_t pixel, __half2& first, __half2& second)
+{
+    // a byte's low code to bits 4-7, its high code to bits 20-23
+    first = CodesToHalves((pixel & 0xFFu) * 0x10010u);
+    second = CodesToHalves(__byte_perm(pixel, 0u, 0x4441) * 0x10010u);
+}
+
+// Two layers of a latent pixel side by side in one word -> per feature the values of (first layer, second layer).
+__device__ __forceinline__ void UnpackTwoLayers(uint32_t word, __half2 (&features)[4])
+{
+    features[0] = CodesToHalves(word << 4);
+    features[1] = CodesToHalves(word);
+    features[2] = CodesToHalves(word >> 4);
+    features[3] = CodesToHalves(word >> 8);
+}
+
 struct GridTaps
 {
     int o00, o01, o10, o11;
@@ -322,59 +359,39 @@ __device__ __forceinline__ uint32_t ElectOne()
     return elected;
 }
 
-// The barrier before a layer's matrix products.  The operand rows of a chain are written by the chain's
-// own 128 threads, and only they read the chain's accumulators, so between two layers of the same tile a
-// chain needs nobody else: kChainLocal = 1 makes its threads meet in a named barrier of their own (1 or 2)
-// and go on without the other chain - 3.3 % faster on the benchmark workload than the CTA-wide barrier for
-// every layer.  Giving up is then agreed on at the CTA-wide barriers that remain (kChainLocal = 0: layers 0
-// and 3 of the decode kernels, where all eight warps share the tile's tables), or, with kChainLocal = 2,
-// among the chain's threads (inference on sample, where nothing is shared).  Returns nonzero when the
-// caller is to give up.
-template <int kChainLocal>
-__device__ __forceinline__ int LayerBarrier(int tid, int failed)
+// All 128 threads of a chain.
+__device__ __forceinline__ void ChainBarrier(int chain)
 {
-    if (kChainLocal == 0)
-        return __syncthreads_or(failed);
-    const int half = tid >> 7;
-    if (kChainLocal == 1)
-    {
-        if (half)
-            asm volatile("bar.sync 2, 128;" ::: "memory");
-        else
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-        return 0;
-    }
-    uint32_t any;
-    if (half)
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p, q;\n\t"
-            "setp.ne.b32 q, %1, 0;\n\t"
-            "bar.red.or.pred p, 2, 128, q;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t"
-            "}"
-            : "=r"(any)
-            : "r"(failed)
-            : "memory");
+    if (chain)
+        asm volatile("bar.sync 2, 128;" ::: "memory");
     else
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p, q;\n\t"
-            "setp.ne.b32 q, %1, 0;\n\t"
-            "bar.red.or.pred p, 1, 128, q;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t"
-            "}"
-            : "=r"(any)
-            : "r"(failed)
-            : "memory");
-    return int(any);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
-// Which barrier a layer of the tile decoders takes: see LayerBarrier.
-template <int kLayer>
-constexpr int TileLayerBarrier()
+// The barrier before a layer's matrix products (reference-numerics kernels).  The operand rows, tables and footprints of a
+// chain are written by the chain's own 128 threads, and only they read its accumulators, so a chain meets in a named barrier of
+// its own and the two chains of a CTA drift apart instead of waiting for each other.
+//
+// Giving up: a thread whose wait expired sets the chain's give-up word for the tile, of which there are two in turn, and goes on; in
+// the next tile's layer 0, after the barrier, all threads read it.  The words alternate, so a word that some thread may still
+// be reading is not written before that thread has met the others again, and all take the same decision.  (A barrier that
+// reduces a predicate, bar.red, says the same at once but costs more than the barrier alone: inference on sample became
+// 6 % faster with half as many of them.)  Returns nonzero when the chain is to leave.
+__device__ __forceinline__ void SetGiveUp(uint32_t word)
 {
-    return (kLayer == 1 || kLayer == 2) ? 1 : 0;
+    asm volatile("st.volatile.shared.u32 [%0], 1;" ::"r"(word) : "memory");
+}
+
+template <int kLayer>
+__device__ __forceinline__ uint32_t LayerBarrier(int tid, uint32_t& giveUp)
+{
+    ChainBarrier(tid >> 7);
+    if (kLayer != 0)
+        return 0;
+    uint32_t word;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(word) : "r"(giveUp) : "memory");
+    giveUp ^= 4u; // the two words share an aligned pair
+    return word;
 }
 
 // Launches a kernel that calls GridDependencyWait before it touches global memory, so that its start overlaps the end of

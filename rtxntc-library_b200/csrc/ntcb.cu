@@ -92,7 +92,7 @@ bool ValidMip(const NtcbMipDesc& m, bool pairedOutput)
 
 // The kernel's view of one mip (everything but its place in the tile list).
 void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprintHiBytes = kFootprintHiBytes,
-    int footprintLoBytes = kFootprintLoBytes, int tileHeight = kTileHeight)
+    int footprintLoBytes = kFootprintLoBytes, int tileWidth = kTileWidth, int tileHeight = kTileHeight)
 {
     km.width = m.width;
     km.height = m.height;
@@ -112,37 +112,41 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprin
     km.positionScale = m.positionScale;
     km.positionLod = m.positionLod;
     // Largest footprint a tile can have in each grid: the tap index of the last column (row) minus
-    // that of the first is at most floor(31 (7) * grid / mip) + 1, plus the second tap.
+    // that of the first is at most floor((size - 1) * grid / mip) + 1, plus the second tap.
     km.strideBytes = layers == 1 ? 8 : layers <= 3 ? 24 : 40;
     const long long hiCapacity = footprintHiBytes / km.strideBytes, loCapacity = footprintLoBytes / km.strideBytes;
     auto footprint = [](int grid, int mip, int span) { return (long long)((long long)span * grid / mip) + 3; };
-    const long long hiPixels = footprint(m.hiWidth, m.width, kTileWidth - 1) * footprint(m.hiHeight, m.height, tileHeight - 1);
-    const long long loPixels = footprint(m.loWidth, m.width, kTileWidth - 1) * footprint(m.loHeight, m.height, tileHeight - 1);
+    const long long hiPixels = footprint(m.hiWidth, m.width, tileWidth - 1) * footprint(m.hiHeight, m.height, tileHeight - 1);
+    const long long loPixels = footprint(m.loWidth, m.width, tileWidth - 1) * footprint(m.loHeight, m.height, tileHeight - 1);
     km.staged = (hiPixels <= hiCapacity && loPixels <= loCapacity) ? 1 : 0;
     // Tables that do not depend on the tile: with power-of-two sizes all the tap arithmetic is exact in
     // binary32, and when a tile's width and height map to whole latent pixels of both grids (and to whole
     // periods of the positional encoding) moving from tile to tile shifts every tap by an integer.
     auto powerOfTwo = [](long long v) { return v > 0 && (v & (v - 1)) == 0; };
-    const float scaledColumns = m.positionScale * float(kTileWidth), scaledRows = m.positionScale * float(tileHeight);
+    const float scaledColumns = m.positionScale * float(tileWidth), scaledRows = m.positionScale * float(tileHeight);
     int exponent = 0;
     const bool scaleIsPowerOfTwo = m.positionScale > 0.f && frexpf(m.positionScale, &exponent) == 0.5f && exponent > -20 && exponent < 20;
     km.invariant = powerOfTwo(m.width) && powerOfTwo(m.height) && powerOfTwo(m.hiWidth) && powerOfTwo(m.hiHeight) &&
-                   powerOfTwo(m.loWidth) && powerOfTwo(m.loHeight) && m.width >= kTileWidth && m.height >= tileHeight &&
+                   powerOfTwo(m.loWidth) && powerOfTwo(m.loHeight) && m.width >= tileWidth && m.height >= tileHeight &&
                    (m.rowBegin % tileHeight) == 0 &&
-                   ((long long)kTileWidth * m.hiWidth) % m.width == 0 && ((long long)kTileWidth * m.loWidth) % m.width == 0 &&
+                   ((long long)tileWidth * m.hiWidth) % m.width == 0 && ((long long)tileWidth * m.loWidth) % m.width == 0 &&
                    ((long long)tileHeight * m.hiHeight) % m.height == 0 && ((long long)tileHeight * m.loHeight) % m.height == 0 &&
                    scaledColumns == floorf(scaledColumns) && scaledRows == floorf(scaledRows) && scaleIsPowerOfTwo
         ? 1 : 0;
     km.hiStepX = km.hiStepY = km.loStepX = km.loStepY = 0;
     if (km.invariant)
     {
-        km.hiStepX = int((long long)kTileWidth * m.hiWidth / m.width);
-        km.loStepX = int((long long)kTileWidth * m.loWidth / m.width);
+        km.hiStepX = int((long long)tileWidth * m.hiWidth / m.width);
+        km.loStepX = int((long long)tileWidth * m.loWidth / m.width);
         km.hiStepY = int((long long)tileHeight * m.hiHeight / m.height);
         km.loStepY = int((long long)tileHeight * m.loHeight / m.height);
     }
-    km.tilesX = (m.width + kTileWidth - 1) / kTileWidth;
-    km.tilesXMagic = km.tilesX == 1 ? 0u : unsigned((0x100000000ull + km.tilesX - 1) / km.tilesX);
+    km.tilesX = (m.width + tileWidth - 1) / tileWidth;
+    // ceil(2^32 / tilesX) divides every local < n when local * (magic * tilesX - 2^32) stays below 2^32
+    const unsigned long long tilesX = (unsigned long long)km.tilesX, magic = (0x100000000ull + tilesX - 1) / tilesX;
+    const unsigned long long tilesY = (unsigned long long)((m.rowEnd - m.rowBegin + tileHeight - 1) / tileHeight);
+    const bool exact = tilesX > 1 && (tilesX * tilesY) * (magic * tilesX - 0x100000000ull) < 0x100000000ull;
+    km.tilesXMagic = exact ? unsigned(magic) : 0u;
     km.firstTile = 0;
 }
 
@@ -646,10 +650,11 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
         if (m.rowBegin == m.rowEnd)
             continue; // nothing of this mip belongs to this launch
         KernelMip& km = k.mips[used++];
-        const int tileHeight = reference ? kRefTileHeight : kTileHeight;
-        if (reference)
-            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes,
-                p->weightMode == NTCB_WEIGHTS_FP8 ? kRefFootprintLoBytes : kRefInt8FootprintLoBytes, kRefTileHeight);
+        const int tileHeight = reference ? kChainTileHeight : kTileHeight;
+        if (reference && p->weightMode == NTCB_WEIGHTS_FP8)
+            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes, kRefFootprintLoBytes, kChainTileWidth, kChainTileHeight);
+        else if (reference)
+            FillKernelMip(m, p->numFeatures / 4, km, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes, kChainTileWidth, kChainTileHeight);
         else
             FillKernelMip(m, p->numFeatures / 4, km);
         km.firstTile = int(tiles);
@@ -661,11 +666,6 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
             km.storeBytes = !(address & 15) && !(texelBytes & 15) ? 16 : !(address & 7) && !(texelBytes & 7) ? 8 : 4;
         }
         const long long mipTiles = (long long)km.tilesX * ((m.rowEnd - m.rowBegin + tileHeight - 1) / tileHeight);
-        if (mipTiles * km.tilesX >= 0x100000000ll)
-        {
-            SetError("ntcb_decode: mip %d is too large for one launch.", i);
-            return NTCB_ERR_OUT_OF_RANGE;
-        }
         tiles += mipTiles;
         if (tiles > 0x7FFFFFFF)
         {
@@ -740,6 +740,8 @@ int ntcb_sample(const NtcbSampleParams* p, void* stream)
     k.numLayers = p->numFeatures / 4;
     k.channels = p->channels;
     k.interleaved = p->latentLayout == NTCB_LATENTS_INTERLEAVED;
+    const uintptr_t placement = reinterpret_cast<uintptr_t>(p->out) | uintptr_t(p->channels * 2); // address and stride of the answers
+    k.storeBytes = !(placement & 15) ? 16 : !(placement & 7) ? 8 : 4;
     for (int i = 0; i < p->numMips; ++i)
     {
         NtcbMipDesc m = p->mips[i];
