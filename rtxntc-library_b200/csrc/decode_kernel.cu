@@ -257,7 +257,7 @@ __device__ __forceinline__ int IssueLayer(const TileContext& ctx, int failed)
 
 // Second half of a layer: waits for the MMA, then applies the activation and writes the next
 // layer's A operand (layers 0-2) or runs the output epilogue (layer 3).
-template <bool kFp8, int kLayer, bool kConvert, bool kBiasTable, typename Params>
+template <bool kFp8, int kLayer, int kConvert, bool kBiasTable, typename Params>
 __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const SharedStorage& shared,
     const TileContext& ctx, uint32_t& phase, int& failed)
 {
@@ -372,14 +372,10 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Sha
                 }
             }
         }
-        if constexpr (kConvert)
+        if constexpr (kConvert != kConvertNone)
         {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j >= channelPairs)
-                    bits[j] = 0;
             if (ctx.out)
-                StoreConverted(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
+                StoreConverted<kConvert>(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
         }
         else if (ctx.out)
             StoreTexel(ctx.out, ctx.outStepWords, ctx.storeBytes, bits, channelPairs);
@@ -388,7 +384,7 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Sha
 
 // Second half of a layer.  An int8 layer's bias is part of the accumulator already (bias slots of
 // the matrix product) unless the staged network says that it has to come from the table.
-template <bool kFp8, int kLayer, bool kConvert, typename Params>
+template <bool kFp8, int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ void ConsumeLayer(const Params& params, const SharedStorage& shared,
     const TileContext& ctx, uint32_t& phase, int& failed)
 {
@@ -399,7 +395,7 @@ __device__ __forceinline__ void ConsumeLayer(const Params& params, const SharedS
         ConsumeLayerImpl<kFp8, kLayer, kConvert, false>(params, shared, ctx, phase, failed);
 }
 
-template <bool kFp8, int kLayer, bool kConvert, typename Params>
+template <bool kFp8, int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ int RunLayer(const Params& params, const SharedStorage& shared,
     const TileContext& ctx, uint32_t& phase, int& failed)
 {
@@ -460,8 +456,8 @@ __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* ne
     return 0;
 }
 
-template <bool kFp8, bool kConvert>
-__global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConverting : kFp8 ? kCtasPerSmFp8 : kCtasPerSmInt8)
+template <bool kFp8, int kConvert>
+__global__ void __launch_bounds__(kThreadsPerCta, kConvert != kConvertNone ? kCtasPerSmConverting : kFp8 ? kCtasPerSmFp8 : kCtasPerSmInt8)
     DecodeKernel(const __grid_constant__ KernelParams params)
 {
     // more than the 48 KB a kernel may declare statically: passed as dynamic shared memory at launch
@@ -534,7 +530,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConvertin
             const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
                                           : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
             const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
-            if constexpr (kConvert)
+            if constexpr (kConvert != kConvertNone)
             {
                 // pixels of dstChannels components, rows without padding; outOffset counts components
                 const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
@@ -570,11 +566,11 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert ? kCtasPerSmConvertin
             PrepareTile<WideTile, kFp8, false, 0>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, lane, warp, keepsTables && place.mipIndex == tablesMip);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
-        ConsumeLayer<kFp8, 0, false>(params, shared, ctx, phase, failed);
+        ConsumeLayer<kFp8, 0, kConvertNone>(params, shared, ctx, phase, failed);
 
         // ---- 3./4. layers 1-3 (their barriers also order the next tile's tables before its use) ---
-        aborted = RunLayer<kFp8, 1, false>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 2, false>(params, shared, ctx, phase, failed);
+        aborted = RunLayer<kFp8, 1, kConvertNone>(params, shared, ctx, phase, failed);
+        if (!aborted) aborted = RunLayer<kFp8, 2, kConvertNone>(params, shared, ctx, phase, failed);
         if (!aborted) aborted = RunLayer<kFp8, 3, kConvert>(params, shared, ctx, phase, failed);
         if (aborted)
             break;
@@ -690,10 +686,10 @@ __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPe
                 ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);
         }
 
-        aborted = RunLayer<kFp8, 0, false>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 1, false>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 2, false>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 3, false>(params, shared, ctx, phase, failed);
+        aborted = RunLayer<kFp8, 0, kConvertNone>(params, shared, ctx, phase, failed);
+        if (!aborted) aborted = RunLayer<kFp8, 1, kConvertNone>(params, shared, ctx, phase, failed);
+        if (!aborted) aborted = RunLayer<kFp8, 2, kConvertNone>(params, shared, ctx, phase, failed);
+        if (!aborted) aborted = RunLayer<kFp8, 3, kConvertNone>(params, shared, ctx, phase, failed);
         if (aborted)
             break;
     }
@@ -749,12 +745,20 @@ cudaError_t LaunchSample(const SampleParams& params, bool fp8, int ctas, cudaStr
 
 cudaError_t LaunchDecode(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream)
 {
-    static std::atomic<unsigned long long> done[4];
-    if (params.convert)
-        return fp8 ? LaunchWithSharedStorage(DecodeKernel<true, true>, done[3], params, ctas, stream)
-                   : LaunchWithSharedStorage(DecodeKernel<false, true>, done[2], params, ctas, stream);
-    return fp8 ? LaunchWithSharedStorage(DecodeKernel<true, false>, done[1], params, ctas, stream)
-               : LaunchWithSharedStorage(DecodeKernel<false, false>, done[0], params, ctas, stream);
+    static std::atomic<unsigned long long> done[3][2];
+    std::atomic<unsigned long long>& flag = done[params.convert][fp8 ? 1 : 0];
+    switch (params.convert)
+    {
+    case kConvertNone:
+        return fp8 ? LaunchWithSharedStorage(DecodeKernel<true, kConvertNone>, flag, params, ctas, stream)
+                   : LaunchWithSharedStorage(DecodeKernel<false, kConvertNone>, flag, params, ctas, stream);
+    case kConvertUnorm8:
+        return fp8 ? LaunchWithSharedStorage(DecodeKernel<true, kConvertUnorm8>, flag, params, ctas, stream)
+                   : LaunchWithSharedStorage(DecodeKernel<false, kConvertUnorm8>, flag, params, ctas, stream);
+    default:
+        return fp8 ? LaunchWithSharedStorage(DecodeKernel<true, kConvertGeneral>, flag, params, ctas, stream)
+                   : LaunchWithSharedStorage(DecodeKernel<false, kConvertGeneral>, flag, params, ctas, stream);
+    }
 }
 
 } // namespace ntcb

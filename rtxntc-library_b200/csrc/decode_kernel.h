@@ -140,7 +140,7 @@ struct KernelParams
     int outputLayout;
     int totalTiles;
     uint32_t loadWaitPolls; // polls a CTA spends waiting for the network image before it gives up (kSpinLimit by default)
-    // converting epilogue (convert != 0): `out` receives pixels in the client's format instead of fp16 texels
+    // converting epilogue (kConvert* other than kConvertNone): `out` receives pixels in the client's format instead of fp16 texels
     int convert;
     int firstChannel, numChannels; // channels the converted pixel starts with
     OutputConversion conversion;

@@ -43,6 +43,7 @@
 
 #include <atomic>
 #include <cstddef>
+#include <type_traits>
 
 #include "decode_kernel.h"
 #include "kernel_parts.cuh"
@@ -501,7 +502,7 @@ __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
 
 // Second half of a layer: waits for the MMA, then applies the activation and writes the next
 // layer's A operand (layers 0-2) or stores the texel (layer 3).
-template <bool kFp8, int kLayer, bool kConvert, typename Params>
+template <bool kFp8, int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefTileContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
@@ -555,21 +556,17 @@ __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefT
         TmemLoadWait();
         const int channelPairs = params.channels >> 1;
         ScrubSpecials(bits, channelPairs);
-        if constexpr (kConvert)
+        if constexpr (kConvert != kConvertNone)
         {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j >= channelPairs)
-                    bits[j] = 0;
             if (ctx.out)
-                StoreConverted(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
+                StoreConverted<kConvert>(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
         }
         else if (ctx.out)
             StoreTexel(ctx.out, ctx.outStepWords, ctx.storeBytes, bits, channelPairs);
     }
 }
 
-template <bool kFp8, int kLayer, bool kConvert, typename Params>
+template <bool kFp8, int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext& ctx, uint32_t& phase)
 {
     if (IssueLayerRef<kLayer>(ctx))
@@ -645,7 +642,7 @@ __device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const R
 // The kernels
 // ---------------------------------------------------------------------------------------------
 
-template <bool kFp8, bool kConvert, int kLayers>
+template <bool kFp8, int kConvert, int kLayers>
 __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernelRef(const __grid_constant__ KernelParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
@@ -720,10 +717,10 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
             PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, keepsTables && place.mipIndex == tablesMip);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
-        ConsumeLayerRef<kFp8, 0, false>(params, ctx, phase);
+        ConsumeLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
 
-        RunLayerRef<kFp8, 1, false>(params, ctx, phase);
-        RunLayerRef<kFp8, 2, false>(params, ctx, phase);
+        RunLayerRef<kFp8, 1, kConvertNone>(params, ctx, phase);
+        RunLayerRef<kFp8, 2, kConvertNone>(params, ctx, phase);
         {
             // where the texel goes (worked out only now: nothing of it has to stay in registers through the
             // layers); the element index inside a mip fits 32 bits (checked on the host)
@@ -731,7 +728,7 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
             const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
                                           : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
             const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
-            if constexpr (kConvert)
+            if constexpr (kConvert != kConvertNone)
             {
                 // pixels of dstChannels components, rows without padding; outOffset counts components
                 const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
@@ -871,12 +868,12 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
         }
 
         // nothing is shared between the chains of a query tile: each runs at its own pace
-        aborted = RunLayerRef<kFp8, 0, false>(params, ctx, phase);
+        aborted = RunLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
         if (aborted)
             break;
-        RunLayerRef<kFp8, 1, false>(params, ctx, phase);
-        RunLayerRef<kFp8, 2, false>(params, ctx, phase);
-        RunLayerRef<kFp8, 3, false>(params, ctx, phase);
+        RunLayerRef<kFp8, 1, kConvertNone>(params, ctx, phase);
+        RunLayerRef<kFp8, 2, kConvertNone>(params, ctx, phase);
+        RunLayerRef<kFp8, 3, kConvertNone>(params, ctx, phase);
     }
     TeardownCtaRef(shared, ctx, phase, tid, warp);
 }
@@ -1040,7 +1037,7 @@ __device__ __forceinline__ uint32_t ActivateToE4m3(uint32_t bits)
     return uint32_t(__nv_cvt_halfraw2_to_fp8x2(static_cast<__half2_raw>(y), __NV_SATFINITE, __NV_E4M3));
 }
 
-template <int kLayer, bool kConvert, typename Params>
+template <int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const RefTileContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
@@ -1175,14 +1172,10 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
         }
         const int channelPairs = params.channels >> 1;
         ScrubSpecials(bits, channelPairs);
-        if constexpr (kConvert)
+        if constexpr (kConvert != kConvertNone)
         {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j >= channelPairs)
-                    bits[j] = 0;
             if (ctx.out)
-                StoreConverted(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
+                StoreConverted<kConvert>(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
         }
         else if (ctx.out)
         {
@@ -1202,7 +1195,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     }
 }
 
-template <int kLayer, bool kConvert, typename Params>
+template <int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ int RunLayerRefFp8(const Params& params, RefTileContext& ctx, uint32_t& phase)
 {
     if (IssueLayerRefFp8<kLayer>(ctx))
@@ -1264,7 +1257,7 @@ __device__ __forceinline__ void TeardownCtaRefFp8(RefFp8SharedStorage& shared, c
         TmemFree(shared.tmemBase, kTmemColumns);
 }
 
-template <bool kConvert, int kLayers>
+template <int kConvert, int kLayers>
 __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernelRefFp8(const __grid_constant__ KernelParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
@@ -1348,17 +1341,17 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
                     keepsTables && place.mipIndex == tablesMip && !(kAblate & 64));
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
-        ConsumeLayerRefFp8<0, false>(params, ctx, phase);
+        ConsumeLayerRefFp8<0, kConvertNone>(params, ctx, phase);
 
-        RunLayerRefFp8<1, false>(params, ctx, phase);
-        RunLayerRefFp8<2, false>(params, ctx, phase);
+        RunLayerRefFp8<1, kConvertNone>(params, ctx, phase);
+        RunLayerRefFp8<2, kConvertNone>(params, ctx, phase);
         {
             // where the texel goes (worked out only now: nothing of it has to stay in registers through the layers)
             const bool planar = params.outputLayout == kLayoutPlanarPairs;
             const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
                                           : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
             const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
-            if constexpr (kConvert)
+            if constexpr (kConvert != kConvertNone)
             {
                 const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
                 const size_t component = size_t(mip.outOffset) + size_t(pixelIndex) * size_t(params.conversion.dstChannels);
@@ -1467,12 +1460,12 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
         }
 
         // nothing is shared between the chains of a query tile: each runs at its own pace
-        aborted = RunLayerRefFp8<0, false>(params, ctx, phase);
+        aborted = RunLayerRefFp8<0, kConvertNone>(params, ctx, phase);
         if (aborted)
             break;
-        RunLayerRefFp8<1, false>(params, ctx, phase);
-        RunLayerRefFp8<2, false>(params, ctx, phase);
-        RunLayerRefFp8<3, false>(params, ctx, phase);
+        RunLayerRefFp8<1, kConvertNone>(params, ctx, phase);
+        RunLayerRefFp8<2, kConvertNone>(params, ctx, phase);
+        RunLayerRefFp8<3, kConvertNone>(params, ctx, phase);
     }
     TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
 }
@@ -1499,50 +1492,37 @@ cudaError_t LaunchRefKernel(Kernel kernel, std::atomic<unsigned long long>& done
     return LaunchOverlapped(kernel, ctas, threads, sharedBytes, stream, params);
 }
 
+// The kernel of a weight set and epilogue compiled for 2, 3 or 4 latent layers, or the one for any number.
+template <bool kFp8Weights, int kConvert>
+cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStream_t stream)
+{
+    static std::atomic<unsigned long long> done[5];
+    auto launch = [&](auto layers) {
+        constexpr int kLayers = decltype(layers)::value;
+        if constexpr (kFp8Weights) // 8-bit operands
+            return LaunchRefKernel(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], sizeof(RefFp8SharedStorage), kThreadsPerCta, params, ctas, stream);
+        else
+            return LaunchRefKernel(DecodeKernelRef<false, kConvert, kLayers>, done[kLayers], sizeof(RefSharedStorage), kRefThreadsPerCta, params, ctas, stream);
+    };
+    switch (params.numLayers)
+    {
+    case 2: return launch(std::integral_constant<int, 2>());
+    case 3: return launch(std::integral_constant<int, 3>());
+    case 4: return launch(std::integral_constant<int, 4>());
+    default: return launch(std::integral_constant<int, 0>());
+    }
+}
+
 cudaError_t LaunchDecodeRef(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream)
 {
-    // kernels compiled for 2, 3 or 4 latent layers and one for any number, each with and without the
-    // converting epilogue
-    static std::atomic<unsigned long long> done[2][2][5];
-    const int layers = params.numLayers < 2 || params.numLayers > 4 ? 0 : params.numLayers;
-    const int convert = params.convert ? 1 : 0;
-    if (fp8)
+    switch (params.convert)
     {
-        // FP8 networks take the kernel with 8-bit operands (same bits, four CTAs per SM)
-        const size_t bytes = sizeof(RefFp8SharedStorage);
-        std::atomic<unsigned long long>& flag = done[1][convert][layers];
-        if (convert)
-            switch (layers)
-            {
-            case 2: return LaunchRefKernel(DecodeKernelRefFp8<true, 2>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-            case 3: return LaunchRefKernel(DecodeKernelRefFp8<true, 3>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-            case 4: return LaunchRefKernel(DecodeKernelRefFp8<true, 4>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-            default: return LaunchRefKernel(DecodeKernelRefFp8<true, 0>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-            }
-        switch (layers)
-        {
-        case 2: return LaunchRefKernel(DecodeKernelRefFp8<false, 2>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-        case 3: return LaunchRefKernel(DecodeKernelRefFp8<false, 3>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-        case 4: return LaunchRefKernel(DecodeKernelRefFp8<false, 4>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-        default: return LaunchRefKernel(DecodeKernelRefFp8<false, 0>, flag, bytes, kThreadsPerCta, params, ctas, stream);
-        }
-    }
-    const size_t bytes = sizeof(RefSharedStorage);
-    std::atomic<unsigned long long>& flag = done[0][convert][layers];
-    if (convert)
-        switch (layers)
-        {
-        case 2: return LaunchRefKernel(DecodeKernelRef<false, true, 2>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-        case 3: return LaunchRefKernel(DecodeKernelRef<false, true, 3>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-        case 4: return LaunchRefKernel(DecodeKernelRef<false, true, 4>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-        default: return LaunchRefKernel(DecodeKernelRef<false, true, 0>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-        }
-    switch (layers)
-    {
-    case 2: return LaunchRefKernel(DecodeKernelRef<false, false, 2>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-    case 3: return LaunchRefKernel(DecodeKernelRef<false, false, 3>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-    case 4: return LaunchRefKernel(DecodeKernelRef<false, false, 4>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
-    default: return LaunchRefKernel(DecodeKernelRef<false, false, 0>, flag, bytes, kRefThreadsPerCta, params, ctas, stream);
+    case kConvertNone:
+        return fp8 ? LaunchDecodeRefLayers<true, kConvertNone>(params, ctas, stream) : LaunchDecodeRefLayers<false, kConvertNone>(params, ctas, stream);
+    case kConvertUnorm8:
+        return fp8 ? LaunchDecodeRefLayers<true, kConvertUnorm8>(params, ctas, stream) : LaunchDecodeRefLayers<false, kConvertUnorm8>(params, ctas, stream);
+    default:
+        return fp8 ? LaunchDecodeRefLayers<true, kConvertGeneral>(params, ctas, stream) : LaunchDecodeRefLayers<false, kConvertGeneral>(params, ctas, stream);
     }
 }
 

@@ -78,6 +78,30 @@ __device__ __forceinline__ float SrgbEncodeSaturated(float linear)
     return linear <= 0.0031308f ? low : high;
 }
 
+// Two linear channels; codes of 16 bits in the low bits, with anything above.
+template <int kFormat>
+__device__ __forceinline__ void LinearPair(uint32_t pair, uint32_t& lo, uint32_t& hi)
+{
+    if (kFormat == kFormatUnorm16)
+    {
+        // the sums round down: x + 0.5 to a grid that holds the integers, then to the integers
+        const float2 v = __half22float2(__hmul2_sat(AsHalf2(pair), __float2half2_rn(1.f)));
+        lo = __float_as_uint(__fadd_rd(__fadd_rd(MulFtz(v.x, 65535.f), 0.5f), 8388608.f));
+        hi = __float_as_uint(__fadd_rd(__fadd_rd(MulFtz(v.y, 65535.f), 0.5f), 8388608.f));
+    }
+    else if (kFormat == kFormatFloat16)
+    {
+        lo = pair; // finite binary16 values as they are
+        hi = pair >> 16;
+    }
+    else
+    {
+        const float2 v = __half22float2(AsHalf2(pair));
+        lo = QuantizeComponent(kFormat, v.x, 0.f);
+        hi = QuantizeComponent(kFormat, v.y, 0.f);
+    }
+}
+
 // An undithered component that is a channel in colour spaces, or a default (0; component 3: 1).
 template <int kFormat>
 __device__ __forceinline__ uint32_t UnditheredComponent(const OutputConversion& conversion, int numChannels, int c, uint32_t half)
@@ -92,8 +116,6 @@ __device__ __forceinline__ uint32_t UnditheredComponent(const OutputConversion& 
     if (kFormat == kFormatFloat16 && kind == kKindLinear)
         return half; // finite binary16 values as they are
     float value = __half2float(__ushort_as_half((unsigned short)half));
-    if (kFormat == kFormatUnorm8 && kind == kKindSrgbEncode)
-        return __byte_perm(RoundToByte1(MulFtz(SrgbEncodeSaturated(value), 255.f)), 0u, 0x4441);
     if (kind != kKindLinear)
     {
         const int srcSpace = (conversion.srcSpaces >> (2 * c)) & 3, dstSpace = (conversion.dstSpaces >> (2 * c)) & 3;
@@ -115,6 +137,39 @@ __device__ __forceinline__ uint32_t LinearCodes(uint32_t pair)
     return AsU32(__hfma2(clamped, __float2half2_rn(255.f), __float2half2_rn(1024.f)));
 }
 
+// The kConvertUnorm8 epilogue: word by word, four linear channels in six instructions, then the bytes of the channels that are
+// encoded to sRGB.  What a word takes is the same for every pixel.  (With one sRGB texture in a 12-channel set all channels
+// went through the general quantiser: 500 us more on a 4096 x 4096 chain than fp16 texels; now 100.)
+template <typename Context>
+__device__ __forceinline__ void ConvertUnorm8Pixel(const OutputConversion& conversion, const Context& ctx, const uint32_t (&pairs)[8])
+{
+    uint32_t words[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+    {
+        if (4 * w < conversion.dstChannels)
+        {
+            uint32_t word = __byte_perm(LinearCodes(pairs[2 * w]), LinearCodes(pairs[2 * w + 1]), 0x6420);
+            if ((conversion.srgb >> (4 * w)) & 15u)
+            {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    if ((conversion.srgb >> (4 * w + k)) & 1u)
+                    {
+                        const __half2 pair = AsHalf2(pairs[2 * w + (k >> 1)]);
+                        const float value = (k & 1) ? __high2float(pair) : __low2float(pair);
+                        constexpr uint32_t kInsert[4] = {0x3215u, 0x3251u, 0x3521u, 0x5210u}; // byte 1 of the second operand as byte k
+                        word = __byte_perm(word, RoundToByte1(MulFtz(SrgbEncodeSaturated(value), 255.f)), kInsert[k]);
+                    }
+                }
+            }
+            words[w] = (word & conversion.keep[w]) | conversion.ones[w];
+        }
+    }
+    StorePixel<4>(reinterpret_cast<unsigned char*>(ctx.out), words, conversion.dstChannels);
+}
+
 // Converting epilogue for one channel format: pairs[j] holds the requested channels 2j and 2j + 1
 // as (scrubbed) binary16; the pixel goes to ctx.out.  What ITextureSet::ReadChannels would produce
 // from the stored texels (src/TextureSet.cpp:915-985, src/ImageProcessing.cu:220-266).
@@ -131,34 +186,7 @@ __device__ __forceinline__ void ConvertPixel(const OutputConversion& conversion,
     for (int w = 0; w < kMaxWords; ++w)
         words[w] = 0;
 
-    if (!conversion.dither && kFormat == kFormatUnorm8)
-    {
-        // Word by word.  What the four components of a word take is the same for every pixel; four linear channels, the
-        // usual case, cost five instructions.  (With one sRGB texture in a 12-channel set all channels went through the general
-        // quantiser: 500 us more on a 4096 x 4096 chain than fp16 texels; now 165.)
-#pragma unroll
-        for (int w = 0; w < kMaxWords; ++w)
-        {
-            if (4 * w < components)
-            {
-                const uint32_t kinds = (conversion.componentKinds >> (8 * w)) & 0xFFu;
-                if (kinds == kKindLinear * 0x55u)
-                    words[w] = __byte_perm(LinearCodes(pairs[2 * w]), LinearCodes(pairs[2 * w + 1]), 0x6420);
-                else
-                {
-                    uint32_t word = 0;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                    {
-                        const uint32_t half = (k & 1) ? pairs[2 * w + (k >> 1)] >> 16 : pairs[2 * w + (k >> 1)] & 0xFFFFu;
-                        word |= UnditheredComponent<kFormat>(conversion, numChannels, 4 * w + k, half) << (8 * k);
-                    }
-                    words[w] = word;
-                }
-            }
-        }
-    }
-    else if (!conversion.dither)
+    if (!conversion.dither)
     {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -166,20 +194,22 @@ __device__ __forceinline__ void ConvertPixel(const OutputConversion& conversion,
             if (2 * j < components)
             {
                 uint32_t lo, hi;
-                if (kFormat == kFormatFloat16 && ((conversion.componentKinds >> (4 * j)) & 15u) == kKindLinear * 5u)
+                if (((conversion.componentKinds >> (4 * j)) & 15u) == kKindLinear * 5u)
+                    LinearPair<kFormat>(pairs[j], lo, hi);
+                else
                 {
-                    words[j % kMaxWords] = pairs[j];
-                    continue;
+                    lo = UnditheredComponent<kFormat>(conversion, numChannels, 2 * j, pairs[j] & 0xFFFFu);
+                    hi = 2 * j + 1 < components ? UnditheredComponent<kFormat>(conversion, numChannels, 2 * j + 1, pairs[j] >> 16) : 0u;
                 }
-                lo = UnditheredComponent<kFormat>(conversion, numChannels, 2 * j, pairs[j] & 0xFFFFu);
-                hi = 2 * j + 1 < components ? UnditheredComponent<kFormat>(conversion, numChannels, 2 * j + 1, pairs[j] >> 16) : 0u;
                 if (kBytes == 4)
                 {
                     words[(2 * j) % kMaxWords] = lo;
                     words[(2 * j + 1) % kMaxWords] = hi;
                 }
-                else
+                else if (kBytes == 2)
                     words[j % kMaxWords] = __byte_perm(lo, hi, 0x5410);
+                else
+                    words[(j >> 1) % kMaxWords] |= (lo | hi << 8) << (16 * (j & 1));
             }
         }
     }
@@ -191,21 +221,23 @@ __device__ __forceinline__ void ConvertPixel(const OutputConversion& conversion,
         {
             if (c < components)
             {
-                const float dither = DitherDraw(seed, uint32_t(c) + 1u);
                 const __half2 pair = AsHalf2(pairs[c >> 1]);
-                const __half texel = (c & 1) ? __high2half(pair) : __low2half(pair);
+                float value = __half2float((c & 1) ? __high2half(pair) : __low2half(pair));
+                const uint32_t kind = (conversion.componentKinds >> (2 * c)) & 3u;
+                if (kind == kKindSrgbEncode)
+                    value = SrgbEncode(value);
+                else if (kind == kKindOther)
+                    value = EncodeColorSpace((conversion.dstSpaces >> (2 * c)) & 3, DecodeColorSpace((conversion.srcSpaces >> (2 * c)) & 3, value));
+                else if (kind == kKindDefault)
+                    value = c == 3 ? 1.f : 0.f;
+                const float dither = DitherDraw(seed, uint32_t(c) + 1u);
                 uint32_t component;
-                if (c < numChannels)
-                {
-                    float value = __half2float(texel);
-                    const int srcSpace = (conversion.srcSpaces >> (2 * c)) & 3;
-                    const int dstSpace = (conversion.dstSpaces >> (2 * c)) & 3;
-                    if (srcSpace | dstSpace)
-                        value = EncodeColorSpace(dstSpace, DecodeColorSpace(srcSpace, value));
-                    component = QuantizeComponent(kFormat, value, dither);
-                }
+                if (kFormat == kFormatUnorm8)
+                    component = __byte_perm(RoundToByte1(MulFtz(AddFtz(value, ApproxDivide(dither, 255.f)), 255.f)), 0u, 0x4441);
+                else if (kFormat == kFormatUnorm16)
+                    component = RoundTo16Bits(MulFtz(AddFtz(value, ApproxDivide(dither, 65535.f)), 65535.f));
                 else
-                    component = QuantizeComponent(kFormat, c == 3 ? 1.f : 0.f, dither);
+                    component = QuantizeComponent(kFormat, value, dither);
                 words[c / kPerWord] |= component << (8 * kBytes * (c % kPerWord));
             }
         }
@@ -215,7 +247,7 @@ __device__ __forceinline__ void ConvertPixel(const OutputConversion& conversion,
 
 // Converting epilogue: the thread's (scrubbed) fp16 channel pairs -> the pixel in the client's
 // format, stored at ctx.out.
-template <typename Context>
+template <int kConvert, typename Context>
 __device__ __forceinline__ void StoreConverted(const OutputConversion& conversion, int firstChannel, int numChannels,
     const Context& ctx, uint32_t (&bits)[8])
 {
@@ -236,6 +268,11 @@ __device__ __forceinline__ void StoreConverted(const OutputConversion& conversio
             const uint32_t hi = c1 < 16 ? *reinterpret_cast<const uint16_t*>(parked + (c1 >> 3) * 2048 + (c1 & 7) * 2) : 0u;
             bits[j] = lo | (hi << 16);
         }
+    }
+    if (kConvert == kConvertUnorm8)
+    {
+        ConvertUnorm8Pixel(conversion, ctx, bits);
+        return;
     }
     switch (conversion.format)
     {

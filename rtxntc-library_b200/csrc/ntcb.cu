@@ -194,7 +194,11 @@ int MakeOutputConversion(const NtcbOutputConversion& request, int channels, Outp
         const bool toSrgb = request.srcColorSpaces[c] == NTCB_COLOR_SPACE_LINEAR && request.dstColorSpaces[c] == NTCB_COLOR_SPACE_SRGB;
         const bool linear = request.srcColorSpaces[c] == NTCB_COLOR_SPACE_LINEAR && request.dstColorSpaces[c] == NTCB_COLOR_SPACE_LINEAR;
         out.componentKinds |= (linear ? kKindLinear : toSrgb ? kKindSrgbEncode : kKindOther) << (2 * c);
+        out.keep[c / 4] |= 0xFFu << (8 * (c % 4));
+        out.srgb |= (toSrgb ? 1u : 0u) << c;
     }
+    if (request.numChannels <= 3)
+        out.ones[0] = 0xFF000000u; // component 3 without a channel is 1
     return NTCB_OK;
 }
 
@@ -591,12 +595,20 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     }
     const bool reference = p->numerics == NTCB_NUMERICS_REFERENCE;
     KernelParams k{};
+    k.outputLayout = p->outputLayout;
+    bool texels = !p->conversion; // what is stored are interleaved or planar fp16 texels
     if (p->conversion)
     {
         int rc = MakeOutputConversion(*p->conversion, p->channels, k.conversion);
         if (rc != NTCB_OK)
             return rc;
-        k.convert = 1;
+        bool plain = k.conversion.format == kFormatUnorm8 && !k.conversion.dither;
+        for (int c = 0; c < p->conversion->numChannels; ++c)
+            plain = plain && ((k.conversion.componentKinds >> (2 * c)) & 3u) != kKindOther;
+        k.convert = plain ? kConvertUnorm8 : kConvertGeneral;
+        // every channel as FLOAT16, none in another colour space: the pixels are the interleaved texels (which are finite)
+        texels = k.conversion.format == kFormatFloat16 && p->conversion->firstChannel == 0 && p->conversion->numChannels == p->channels &&
+                 k.conversion.dstChannels == p->channels && k.conversion.componentKinds == 0x55555555u >> (32 - 2 * p->channels);
         k.firstChannel = p->conversion->firstChannel;
         k.numChannels = p->conversion->numChannels;
     }
@@ -606,7 +618,6 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     k.status = p->status;
     k.numLayers = p->numFeatures / 4;
     k.channels = p->channels;
-    k.outputLayout = p->outputLayout;
     long long tiles = 0;
     int used = 0;
     for (int i = 0; i < p->numMips; ++i)
@@ -635,12 +646,16 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
                 return NTCB_ERR_INVALID_ARGUMENT;
             }
         }
-        else if (uint64_t(m.width) * uint64_t(m.height) * uint64_t(p->channels) > 0xFFFFFFFFull)
+        if (uint64_t(m.width) * uint64_t(m.height) * uint64_t(p->channels) > 0xFFFFFFFFull)
         {
-            // the kernels index the elements of a mip with 32 bits
-            SetError("ntcb_decode: mip %d has %llu x %d values; a mip may hold at most 2^32 - 1.", i,
-                (unsigned long long)m.width * (unsigned long long)m.height, p->channels);
-            return NTCB_ERR_OUT_OF_RANGE;
+            // the kernels index the elements of a mip of texels with 32 bits
+            texels = false;
+            if (!k.convert)
+            {
+                SetError("ntcb_decode: mip %d has %llu x %d values; a mip may hold at most 2^32 - 1.", i,
+                    (unsigned long long)m.width * (unsigned long long)m.height, p->channels);
+                return NTCB_ERR_OUT_OF_RANGE;
+            }
         }
         if (k.convert && uint64_t(m.width) * uint64_t(m.height) > 0xFFFFFFFFull)
         {
@@ -659,7 +674,7 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
             FillKernelMip(m, p->numFeatures / 4, km);
         km.firstTile = int(tiles);
         km.storeBytes = 4;
-        if (!k.convert && p->outputLayout == NTCB_LAYOUT_INTERLEAVED)
+        if (k.convert || p->outputLayout == NTCB_LAYOUT_INTERLEAVED)
         {
             const uintptr_t address = reinterpret_cast<uintptr_t>(p->out) + size_t(m.outOffset) * 2;
             const size_t texelBytes = size_t(p->channels) * 2;
@@ -678,6 +693,11 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
         return NTCB_OK;
     k.numMips = used;
     k.totalTiles = int(tiles);
+    if (k.convert && texels)
+    {
+        k.convert = kConvertNone;
+        k.outputLayout = NTCB_LAYOUT_INTERLEAVED;
+    }
     k.loadWaitPolls = g_networkWaitPolls.load(std::memory_order_relaxed);
 
     const bool fp8 = p->weightMode == NTCB_WEIGHTS_FP8;

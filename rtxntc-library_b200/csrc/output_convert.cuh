@@ -37,7 +37,15 @@ struct OutputConversion
     int dither;       // nonzero: add a hash-based offset in [-0.5, 0.5) code units before rounding
     uint32_t srcSpaces, dstSpaces;
     uint32_t componentKinds; // kKind* of component c in bits 2 c and 2 c + 1 (MakeOutputConversion)
+    // Undithered UNORM8 whose channels keep their values or are encoded to sRGB: a word of four components is (codes & keep) |
+    // ones, where the codes of the components in `srgb` (bit c) are those of the encoded values.
+    uint32_t keep[4], ones[4], srgb;
 };
+
+// The epilogues the decode kernels are compiled with.
+constexpr int kConvertNone = 0;    // fp16 texels
+constexpr int kConvertUnorm8 = 1;  // undithered UNORM8, channels linear or encoded to sRGB
+constexpr int kConvertGeneral = 2; // everything else
 
 // What an undithered component takes.
 constexpr uint32_t kKindDefault = 0;    // no channel: 0, component 3: 1
