@@ -543,6 +543,12 @@ int ntcb_texture_set_make_and_store_bc7_mode_buffer(NtcbTextureSet* textureSet, 
 int ntcb_texture_set_block_compress_texture(NtcbTextureSet* textureSet, int textureIndex, int mipLevel, float alphaThreshold,
                                             void* deviceBlocks, size_t rowPitch);
 
+/* The same in one call for a caller that hands in a buffer of its own stream's and wants the blocks at once: orders the set's
+   stream after `clientStream` (ntcb_texture_set_wait_for_stream), encodes, and waits for the blocks
+   (ntcb_texture_set_synchronize). */
+int ntcb_texture_set_encode_texture(NtcbTextureSet* textureSet, int textureIndex, int mipLevel, float alphaThreshold,
+    void* deviceBlocks, size_t rowPitch, void* clientStream);
+
 /* ---- Several GPUs of one machine ------------------------------------------------------------ */
 
 /* One texture set of a batch: its container, and the host image that receives the decoded chain. */

@@ -222,6 +222,8 @@ def lib():
                                                                 ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_size_t)]
         handle.ntcb_texture_set_make_and_store_bc7_mode_buffer.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                                                            ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_size_t]
+        handle.ntcb_texture_set_encode_texture.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_float,
+                                                           ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
         handle.ntcb_texture_set_block_compress_texture.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_float,
                                                                    ctypes.c_void_p, ctypes.c_size_t]
         handle.ntcb_bc7_mode_buffer_size.argtypes = [ctypes.c_int, ctypes.c_int]
@@ -676,20 +678,11 @@ class TextureSet:
                                                         ctypes.byref(features), ctypes.byref(self.handle)))
         self.desc = TextureSetDesc()
         check(lib().ntcb_texture_set_get_desc(self.handle, ctypes.byref(self.desc)))
-        self._block_formats: dict = {}  # texture index -> the block format its header names
+        self._block_shapes: dict = {}  # (texture index, mip) -> shape of its blocks in the format the header names
 
-    def _empty_blocks(self, mip: int, block_format: int):
-        """(uninitialised CUDA uint8 tensor for the blocks of one mip, its row pitch).  The set's stream is made to wait for
-        torch's current one, whose queued work may still be using the memory the tensor was given; the encoders write
-        every block, so nothing has to be cleared and the host waits for nothing here."""
-        import torch
-
+    def _blocks_shape(self, mip: int, block_format: int) -> Tuple[int, int, int]:
         width, height = self.mip_size(mip)
-        bw, bh = (width + 3) // 4, (height + 3) // 4
-        block_bytes = 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
-        out = torch.empty((bh, bw, block_bytes), dtype=torch.uint8, device="cuda")
-        check(lib().ntcb_texture_set_wait_for_stream(self.handle, torch._C._cuda_getCurrentRawStream(out.device.index)))
-        return out, bw * block_bytes
+        return (height + 3) // 4, (width + 3) // 4, 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
 
     def mip_size(self, mip: int) -> Tuple[int, int]:
         return max(1, self.desc.width >> mip), max(1, self.desc.height >> mip)
@@ -770,15 +763,20 @@ class TextureSet:
                        alpha_threshold: float = 1.0 / 255.0):
         """One decoded mip as BC1 - BC5 blocks: a CUDA uint8 tensor [blocks_y][blocks_x][8 or 16]
         (waits for the texture set's stream)."""
-        out, row_pitch = self._empty_blocks(mip, block_format)
+        import torch
+
+        shape = self._blocks_shape(mip, block_format)
+        out = torch.empty(shape, dtype=torch.uint8, device="cuda")  # the encoders write every block
+        # the memory may still be in use by work queued on torch's current stream
+        check(lib().ntcb_texture_set_wait_for_stream(self.handle, torch._C._cuda_getCurrentRawStream(out.get_device())))
         check(lib().ntcb_texture_set_block_compress(self.handle, mip, first_channel, num_channels, block_format,
-                                                    alpha_threshold, out.data_ptr(), row_pitch))
+                                                    alpha_threshold, out.data_ptr(), shape[1] * shape[2]))
         self.synchronize()
         return out
 
     def load_from_memory(self, container: bytes) -> None:
         """Another compressed set of the same shape into this one's buffers (ITextureSet::LoadFromMemory)."""
-        self._block_formats = {}
+        self._block_shapes = {}
         check(lib().ntcb_texture_set_load_from_memory(self.handle, container, len(container)))
 
     def bc7_mode_buffer(self, texture_index: int, mip_level: int) -> Optional[np.ndarray]:
@@ -799,13 +797,16 @@ class TextureSet:
     def block_compress_texture(self, texture_index: int, mip_level: int, alpha_threshold: float = 1.0 / 255.0):
         """One mip of one texture in the block format its header names (BC7: from its stored mode bitmap when it
         has one): a CUDA uint8 tensor [blocks_y][blocks_x][8 or 16] (waits for the texture set's stream)."""
-        block_format = self._block_formats.get(texture_index)
-        if block_format is None:
-            block_format = self._block_formats[texture_index] = self.textures()[texture_index]["blockCompressedFormat"]
-        out, row_pitch = self._empty_blocks(mip_level, block_format)
-        check(lib().ntcb_texture_set_block_compress_texture(self.handle, texture_index, mip_level, alpha_threshold,
-                                                            out.data_ptr(), row_pitch))
-        self.synchronize()
+        import torch
+
+        # the shape of the blocks is kept: a small mip is encoded in less time than Python takes to work it out
+        shape = self._block_shapes.get((texture_index, mip_level))
+        if shape is None:
+            shape = self._block_shapes[(texture_index, mip_level)] = self._blocks_shape(
+                mip_level, self.textures()[texture_index]["blockCompressedFormat"])
+        out = torch.empty(shape, dtype=torch.uint8, device="cuda")  # the encoders write every block
+        check(lib().ntcb_texture_set_encode_texture(self.handle, texture_index, mip_level, alpha_threshold, out.data_ptr(),
+                                                    shape[1] * shape[2], torch._C._cuda_getCurrentRawStream(out.get_device())))
         return out
 
     def textures(self) -> list:

@@ -1677,6 +1677,22 @@ int ntcb_texture_set_block_compress_texture(NtcbTextureSet* textureSet, int text
     return ntcb::Guarded(__func__, [&]() { return textureSet->impl->BlockCompressTexture(textureIndex, mipLevel, alphaThreshold, deviceBlocks, rowPitch); });
 }
 
+int ntcb_texture_set_encode_texture(NtcbTextureSet* textureSet, int textureIndex, int mipLevel, float alphaThreshold,
+    void* deviceBlocks, size_t rowPitch, void* clientStream)
+{
+    if (!textureSet)
+    {
+        ntcb::SetError("textureSet is NULL.");
+        return NTCB_ERR_INVALID_ARGUMENT;
+    }
+    return ntcb::Guarded(__func__, [&]() {
+        int status = textureSet->impl->WaitForStream(clientStream);
+        if (status == NTCB_OK)
+            status = textureSet->impl->BlockCompressTexture(textureIndex, mipLevel, alphaThreshold, deviceBlocks, rowPitch);
+        return status == NTCB_OK ? textureSet->impl->Synchronize() : status;
+    });
+}
+
 int ntcb_texture_set_get_texture(NtcbTextureSet* textureSet, int index, NtcbTextureDesc* outTexture, int* outCount)
 {
     if (!textureSet)
