@@ -159,7 +159,7 @@ __device__ __forceinline__ void ConvertUnorm8Pixel(const OutputConversion& conve
                     {
                         const __half2 pair = AsHalf2(pairs[2 * w + (k >> 1)]);
                         const float value = (k & 1) ? __high2float(pair) : __low2float(pair);
-                        constexpr uint32_t kInsert[4] = {0x3215u, 0x3251u, 0x3521u, 0x5210u}; // byte 1 of the second operand as byte k
+                        constexpr uint32_t kInsert[4] = {0x3215u, 0x3250u, 0x3510u, 0x5210u}; // byte 1 of the second operand as byte k
                         word = __byte_perm(word, RoundToByte1(MulFtz(SrgbEncodeSaturated(value), 255.f)), kInsert[k]);
                     }
                 }

@@ -233,6 +233,39 @@ def test_fused_epilogue_on_ragged_shapes_row_ranges_and_fp8(oracle, numerics):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("request_", [
+    # UNORM8: sRGB at every place of a word of four pixels' bytes, alone and in runs, first channels that shift the words
+    (UNORM8, 16, 0, 16, 0x0001), (UNORM8, 16, 0, 16, 0x0022), (UNORM8, 16, 0, 16, 0x0407), (UNORM8, 15, 1, 15, 0x7080),
+    (UNORM8, 12, 0, 12, 0x0007), (UNORM8, 9, 7, 9, 0x01FF), (UNORM8, 6, 2, 8, 0x0036), (UNORM8, 3, 13, 4, 0x0007),
+    (UNORM8, 2, 3, 4, 0x0002), (UNORM8, 1, 15, 1, 0x0001), (UNORM8, 5, 0, 5, 0x0000),
+    # FLOAT16: all channels as they are (plain texels), with a default component, one channel less, one encoded
+    (FLOAT16, 16, 0, 16, 0x0000), (FLOAT16, 15, 0, 16, 0x0000), (FLOAT16, 15, 1, 15, 0x0000), (FLOAT16, 16, 0, 16, 0x8000),
+], ids=lambda r: "-".join("%x" % v for v in r))
+def test_each_epilogue_writes_what_the_conversion_kernel_writes(request_):
+    import torch
+
+    channel_format, count, first, components, srgb = request_
+    spec = synthetic.TextureSetSpec(37, 19, 16, 0, 2, 8, seed=5, network="unit")
+    data = synthetic.make_texture_set(spec)
+    geo = data.geometry
+    conversion = binding.make_conversion(channel_format, count, first, components, None,
+                                         [SRGB if srgb >> c & 1 else LINEAR for c in range(count)], False)
+    for numerics in (binding.NUMERICS_REFERENCE, binding.NUMERICS_EXACT):
+        resident = binding.ResidentTextureSet.from_synthetic(data, numerics=numerics)
+        for use_int8 in (False, True):
+            resident.decode(use_int8)
+            pixels = resident.decode_converted(use_int8, conversion)
+            torch.cuda.synchronize()
+            resident.check_status()
+            for cm in geo.color_mips:
+                texels = resident.out[cm.texel_offset * 16:(cm.texel_offset + cm.width * cm.height) * 16]
+                expected = binding.convert_channels(texels.view(cm.height, cm.width, 16), conversion)
+                start = cm.texel_offset * components
+                got = pixels[start:start + cm.width * cm.height * components].view(cm.height, cm.width, -1)
+                assert torch.equal(got, expected), (numerics, use_int8, cm.width)
+
+
+@pytest.mark.gpu
 def test_read_channels_argument_checks(case):
     index, fixture = case
     with binding.Context(0) as context:
