@@ -85,18 +85,14 @@ constexpr int kRefOperandBytes = 128 * 96;
 // Each walks tiles of its own, 16 x 8 texels, with its own tables and footprints, and meets only its own threads in barriers.
 constexpr int kChainTileWidth = 16;
 constexpr int kChainTileHeight = 8;
-constexpr int kRefChains = 2;
-constexpr int kRefThreadsPerCta = 128 * kRefChains;
-constexpr int kRefTmemColumns = kRefChains * kTmemColumnsPerHalf;
+constexpr int kMaxChains = 8;
+constexpr int kMaxThreadsPerCta = 128 * kMaxChains;
 // Footprints of a chain: what a tile covers at a grid-to-mip ratio of 1 (high-res: 18 x 10 pixels of 24 bytes) and 1/2
 // (low-res: 10 x 6).
 constexpr int kRefFootprintHiBytes = 4352;
 constexpr int kRefFootprintLoBytes = 1536;
 constexpr int kRefInt8FootprintHiBytes = kRefFootprintHiBytes;
 constexpr int kRefInt8FootprintLoBytes = 1440;
-constexpr int kCtasPerSmRef = 4;       // Int8 networks: 56 KB of shared memory and 64 registers, like the FP8 kernels
-constexpr int kCtasPerSmRefFp8 = 4; // FP8 networks: 8-bit operands halve the A buffers
-constexpr int kCtasPerSmRefSample = 4; // inference on sample, Int8 networks (its launches leave the footprints out)
 
 // Dynamic shared memory a CTA may have for `ctas` of them to be resident: an SM has 228 KB, 1 KB per CTA is the system's.
 template <int ctas>

@@ -194,24 +194,108 @@ struct __align__(16) ChainStage
     uint8_t footprintHi[kHiBytes];
     uint8_t footprintLo[kLoBytes];
 };
-using RefStage = ChainStage<RefTileTables, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes>;
+
+// What the threads of a chain keep of their texel's place in a tile while the tables stay the same: with power-of-two sizes that is from the
+// first inner tile of a mip on.  The positional encoding stays in the operand row, whose last chunks only the input stage writes.  (Worked out per
+// tile - eight products and eight conversions - a 4096 x 4096 FP8 set took 867 us instead of 851.)
+struct __align__(16) TexelTables
+{
+    uint4 weights[2][128]; // per grid and texel: w00, w01, w10, w11, each twice
+    uint4 taps[128];       // byte offset of the upper left tap and bytes per footprint row, high-res and low-res grid
+};
+
+struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes>
+{
+    TexelTables texels;
+};
+
+template <typename Stage>
+__device__ __forceinline__ void PrepareTexel(Stage& stage, int texel, int tileColumn, int tileRow)
+{
+    uint32_t offsets[4];
+#pragma unroll
+    for (int grid = 0; grid < 2; ++grid)
+    {
+        const int4 col = stage.tables.taps.colTap[grid][tileColumn];
+        const int4 row = stage.tables.taps.rowTap[grid][tileRow];
+        const float dx = __int_as_float(col.y), dxn = __int_as_float(col.z);
+        const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
+        // src/FeatureGridDevice.h:46-49
+        const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);
+        stage.texels.weights[grid][texel] = make_uint4(AsU32(__floats2half2_rn(f00, f00)), AsU32(__floats2half2_rn(f01, f01)),
+                                                       AsU32(__floats2half2_rn(f10, f10)), AsU32(__floats2half2_rn(f11, f11)));
+        offsets[2 * grid] = uint32_t(col.x + row.x);
+        offsets[2 * grid + 1] = uint32_t(row.w);
+    }
+    stage.texels.taps[texel] = make_uint4(offsets[0], offsets[1], offsets[2], offsets[3]);
+}
+
+// Calls blend(grid, layer, four taps, four weights) for the latents of a texel in the staged footprints.
+template <int kLayers, typename Stage, typename Blend>
+__device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, Blend blend)
+{
+    const uint4 taps = stage.texels.taps[texel];
+    const int stride = StrideBytes<kLayers>(mip);
+#pragma unroll
+    for (int grid = 0; grid < 2; ++grid)
+    {
+        const uint4 w = stage.texels.weights[grid][texel];
+        const uint8_t* tap00 = grid ? stage.footprintLo + taps.z : stage.footprintHi + taps.x;
+        const uint8_t* tap10 = tap00 + (grid ? taps.w : taps.y);
+#pragma unroll
+        for (int layer = 0; layer < 4; ++layer)
+        {
+            if (layer < NumLayers<kLayers>(params))
+                blend(grid, layer, *reinterpret_cast<const uint2*>(tap00 + layer * 8), *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8),
+                    *reinterpret_cast<const uint2*>(tap10 + layer * 8), *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8),
+                    AsHalf2(w.x), AsHalf2(w.y), AsHalf2(w.z), AsHalf2(w.w));
+        }
+    }
+}
 
 struct __align__(128) RefSharedStorage
 {
     uint8_t network[kRefInt8NetworkBytes];                 // binary16 weights and the matrix of biases
-    alignas(128) uint8_t operandA[kRefChains * kRefOperandBytes]; // A operands of layers 0 and 1 (its first half), one per chain
     // Constant A operands of the bias steps: four core matrices (8 rows x 8 halves) whose rows are the unit
     // vectors e_0 .. e_3, and one of zeros (the second 8-wide half of every step).  A stride offset of 0 in
     // the descriptor makes all sixteen 8-row groups of the 128-row operand read the same core matrix.
     alignas(128) uint8_t onesRegion[5 * 128];
-    uint64_t barrier[kRefChains]; // MMA completion, per chain: a chain's threads go on as soon as their accumulators are ready
+    uint64_t barrier[kMaxChains]; // MMA completion, per chain: a chain's threads go on as soon as their accumulators are ready
     uint64_t loadBarrier;  // arrival of the network image
-    alignas(8) uint32_t giveUp[kRefChains][2]; // see LayerBarrier
+    alignas(8) uint32_t giveUp[kMaxChains][2]; // see LayerBarrier
+    uint32_t claims;              // inference on sample: query tiles handed out so far
+    uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    // what inference on sample does not use comes last: its launches ask for the bytes before `stage` only
-    alignas(128) RefStage stage[kRefChains];
+    // A operands of layers 0 and 1 (its first half), one per chain of the CTA; after them a RefStage per chain, which inference on
+    // sample does without (SharedBytes)
+    alignas(128) uint8_t operandA[kMaxChains * kRefOperandBytes];
 };
-static_assert(sizeof(RefSharedStorage) <= kMaxSharedBytes<kCtasPerSmRef>, "resident CTAs must fit into shared memory");
+static_assert(sizeof(RefSharedStorage) + kMaxChains * sizeof(RefStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
+
+// Dynamic shared memory of a CTA of `chains` chains, each with an operand and `perChain` more bytes.
+template <typename Storage>
+constexpr size_t SharedBytes(int chains, size_t perChain)
+{
+    return offsetof(Storage, operandA) + chains * (sizeof(Storage::operandA) / kMaxChains + perChain);
+}
+
+// What `chain` prepares per tile: after the operands of all chains.
+template <typename Stage, typename Storage>
+__device__ __forceinline__ Stage& StageOf(Storage& shared, int chain)
+{
+    return reinterpret_cast<Stage*>(shared.operandA + (blockDim.x >> 7) * (sizeof(Storage::operandA) / kMaxChains))[chain];
+}
+
+// Inference on sample: tiles of 128 queries are claimed, not dealt.  The chains of a CTA draw from a counter in shared memory, two tiles
+// ahead, as the queries are requested one tile ahead; tile k of CTA b is tile b + k * gridDim.x.  The threads of a chain read the claim between
+// the barriers of layers 0 and 1.  (16.7 M queries: 780 us dealt, 768 claimed; the tiles of a decode, whose costs differ less, are dealt: claimed
+// they take 2 % longer.)
+template <typename Storage>
+__device__ __forceinline__ void ClaimTile(Storage& shared, int chain)
+{
+    if ((threadIdx.x & 127) == 0)
+        shared.claimed[chain] = atomicAdd(&shared.claims, 1u);
+}
 
 struct RefTileContext
 {
@@ -288,37 +372,6 @@ __device__ __forceinline__ void BlendLayerRef(uint2 l00, uint2 l01, uint2 l10, u
     words[1] = AsU32(QuantizeInputRef<kFp8>(b));
 }
 
-// Inputs 0..15 or 16..31 of one texel (eight binary16 pairs) from the staged footprint of one grid.
-template <bool kFp8, int kLayers = 0>
-__device__ __forceinline__ void GatherGridRef(const KernelParams& params, const KernelMip& mip, const RefStage& stage,
-    int grid, int tileColumn, int tileRow, uint32_t* words)
-{
-    const int4 col = stage.tables.taps.colTap[grid][tileColumn];
-    const int4 row = stage.tables.taps.rowTap[grid][tileRow];
-    const float dx = __int_as_float(col.y), dxn = __int_as_float(col.z);
-    const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
-    // src/FeatureGridDevice.h:46-49
-    const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);
-    const __half2 w00 = __floats2half2_rn(f00, f00), w01 = __floats2half2_rn(f01, f01);
-    const __half2 w10 = __floats2half2_rn(f10, f10), w11 = __floats2half2_rn(f11, f11);
-
-    const int stride = StrideBytes<kLayers>(mip);
-    const uint8_t* tap00 = (grid ? stage.footprintLo : stage.footprintHi) + (col.x + row.x);
-    const uint8_t* tap10 = tap00 + row.w;
-#pragma unroll
-    for (int layer = 0; layer < 4; ++layer)
-    {
-        if (layer < NumLayers<kLayers>(params))
-        {
-            const uint2 l00 = *reinterpret_cast<const uint2*>(tap00 + layer * 8);
-            const uint2 l01 = *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8);
-            const uint2 l10 = *reinterpret_cast<const uint2*>(tap10 + layer * 8);
-            const uint2 l11 = *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8);
-            BlendLayerRef<kFp8>(l00, l01, l10, l11, w00, w01, w10, w11, words + 2 * layer);
-        }
-    }
-}
-
 // One latent layer of one grid (the low 16 bits of each p are the tap's four features) -> two pairs of inputs.
 template <bool kFp8>
 __device__ __forceinline__ void BlendPixelsRef(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, uint32_t* words)
@@ -353,12 +406,13 @@ __device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plan
     BlendPixelsRef<kFp8>(p00, p01, p10, p11, taps, words);
 }
 
-// The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.
+// The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.  `known`: TexelTables and the
+// row's last two chunks are those of an earlier tile with the same tables.
 template <bool kFp8, int kLayers = 0>
-__device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, const RefStage& stage,
-    const RefTileContext& ctx, int tileColumn, int tileRow)
+__device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
+    const RefTileContext& ctx, int tileColumn, int tileRow, bool known)
 {
-    uint32_t words[24];
+    uint32_t words[16];
     const uint32_t zeroPair = stage.tables.zeroPair;
 #pragma unroll
     for (int i = 0; i < 16; ++i)
@@ -366,8 +420,10 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
 
     if (mip.staged)
     {
-        GatherGridRef<kFp8, kLayers>(params, mip, stage, 0, tileColumn, tileRow, words);
-        GatherGridRef<kFp8, kLayers>(params, mip, stage, 1, tileColumn, tileRow, words + 8);
+        if (!known)
+            PrepareTexel(stage, ctx.tid & 127, tileColumn, tileRow);
+        GatherTexel<kLayers>(params, mip, stage, ctx.tid & 127, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00,
+            __half2 w01, __half2 w10, __half2 w11) { BlendLayerRef<kFp8>(l00, l01, l10, l11, w00, w01, w10, w11, words + 8 * grid + 2 * layer); });
     }
     else
     {
@@ -391,20 +447,17 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
                 SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
     }
 
-    // positional encoding: per wave the inputs (x phase 0, y phase 0, x phase 0.25, y phase 0.25)
-    const uint4 cx = stage.tables.colEnc[tileColumn];
-    const uint4 ry = stage.tables.rowEnc[tileRow];
-    words[16] = __byte_perm(cx.x, ry.x, 0x5410);
-    words[17] = __byte_perm(cx.x, ry.x, 0x7632);
-    words[18] = __byte_perm(cx.y, ry.y, 0x5410);
-    words[19] = __byte_perm(cx.y, ry.y, 0x7632);
-    words[20] = __byte_perm(cx.z, ry.z, 0x5410);
-    words[21] = __byte_perm(cx.z, ry.z, 0x7632);
-    words[22] = stage.tables.lodPair;
-    words[23] = zeroPair;
-
+    if (!known)
+    {
+        // positional encoding: per wave the inputs (x phase 0, y phase 0, x phase 0.25, y phase 0.25)
+        const uint4 cx = stage.tables.colEnc[tileColumn];
+        const uint4 ry = stage.tables.rowEnc[tileRow];
+        ctx.rowChunk[4 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5410), __byte_perm(cx.x, ry.x, 0x7632),
+                                           __byte_perm(cx.y, ry.y, 0x5410), __byte_perm(cx.y, ry.y, 0x7632));
+        ctx.rowChunk[5 * 128] = make_uint4(__byte_perm(cx.z, ry.z, 0x5410), __byte_perm(cx.z, ry.z, 0x7632), stage.tables.lodPair, zeroPair);
+    }
 #pragma unroll
-    for (int chunk = 0; chunk < 6; ++chunk)
+    for (int chunk = 0; chunk < 4; ++chunk)
         ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);
 }
 
@@ -583,7 +636,7 @@ __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint
     GridDependencyLaunch();
     // constant A operands of the bias steps: core matrix l (8 rows of 16 bytes) has 1.0 as half l of every row,
     // core matrix 4 is zero
-    for (int i = tid; i < 5 * 8; i += kRefThreadsPerCta)
+    for (int i = tid; i < 5 * 8; i += int(blockDim.x))
     {
         const int unit = i >> 3;
         reinterpret_cast<uint4*>(shared.onesRegion)[i] =
@@ -592,16 +645,17 @@ __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint
     const uint32_t loadBarrier = SharedAddress(&shared.loadBarrier);
     if (tid == 0)
     {
-        for (int chain = 0; chain < kRefChains; ++chain)
+        for (int chain = 0; chain < kMaxChains; ++chain)
         {
             MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
             shared.giveUp[chain][0] = shared.giveUp[chain][1] = 0;
         }
+        shared.claims = 2 * (blockDim.x >> 7);
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
     }
     if (warp == 0)
-        TmemAlloc(SharedAddress(&shared.tmemBase), kRefTmemColumns);
+        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerHalf);
     GridDependencyWait();
     if (tid == 0)
     {
@@ -626,16 +680,15 @@ __device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const R
 {
     TcgenFenceBeforeSync();
     __syncthreads();
-    const volatile uint32_t* gaveUp = &shared.giveUp[0][0];
-    if (tid == 0 && (gaveUp[0] | gaveUp[1] | gaveUp[2] | gaveUp[3]))
+    const volatile uint32_t* gaveUp = &shared.giveUp[warp >> 2][0];
+    if ((tid & 127) == 0 && (gaveUp[0] | gaveUp[1]))
     {
-        for (int chain = 0; chain < kRefChains; ++chain)
-            (void)MbarrierWaitBounded(SharedAddress(&shared.barrier[chain]), phase ^ 1);
+        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1);
         (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
     }
     __syncthreads();
     if (warp == 0)
-        TmemFree(shared.tmemBase, kRefTmemColumns);
+        TmemFree(shared.tmemBase, (blockDim.x >> 7) * kTmemColumnsPerHalf);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -643,7 +696,7 @@ __device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const R
 // ---------------------------------------------------------------------------------------------
 
 template <bool kFp8, int kConvert, int kLayers>
-__global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernelRef(const __grid_constant__ KernelParams params)
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __grid_constant__ KernelParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
     RefSharedStorage& shared = *reinterpret_cast<RefSharedStorage*>(dynamicShared);
@@ -666,18 +719,18 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
 
-    RefStage& stage = shared.stage[chain];
+    RefStage& stage = StageOf<RefStage>(shared, chain);
     struct TilePlace
     {
         int mipIndex, tileX0, tileY0;
     };
-    auto locate = [&](int tile, int fromMip) {
+    auto locate = [&](uint32_t tile, int fromMip) {
         TilePlace place;
         place.mipIndex = fromMip;
-        while (place.mipIndex + 1 < params.numMips && tile >= params.mips[place.mipIndex + 1].firstTile)
+        while (place.mipIndex + 1 < params.numMips && tile >= uint32_t(params.mips[place.mipIndex + 1].firstTile))
             ++place.mipIndex;
         const KernelMip& mip = params.mips[place.mipIndex];
-        const int local = tile - mip.firstTile;
+        const int local = int(tile) - mip.firstTile;
         const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
         place.tileX0 = (local - tileY * mip.tilesX) * kChainTileWidth;
         place.tileY0 = mip.rowBegin + tileY * kChainTileHeight;
@@ -685,36 +738,39 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
     };
 
     // the first chains of all CTAs take the first tiles, so that a launch of few tiles spreads over the SMs
-    int tile = int(blockIdx.x) + chain * int(gridDim.x);
+    const uint32_t chains = blockDim.x >> 7;
+    uint32_t tile = blockIdx.x + uint32_t(chain) * gridDim.x;
     TilePlace place{0, 0, 0};
+    bool known = false; // the tables, and what the threads keep of them, are already the tile's
     int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
-    if (tile < params.totalTiles)
+    if (tile < uint32_t(params.totalTiles))
     {
         place = locate(tile, 0);
         PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, false);
         tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
         ChainBarrier(chain);
     }
-    while (tile < params.totalTiles)
+    while (tile < uint32_t(params.totalTiles))
     {
         const KernelMip& mip = params.mips[place.mipIndex];
-        ctx.tile = tile;
+        ctx.tile = int(tile);
         ctx.x = place.tileX0 + tileColumn;
         ctx.y = place.tileY0 + tileRow;
-        BuildInputsRef<kFp8, kLayers>(params, mip, stage, ctx, tileColumn, tileRow);
+        BuildInputsRef<kFp8, kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
 
         // layer 0; while the tensor core works on it, prepare the chain's NEXT tile (its tables and
         // footprints replace this tile's, which nobody reads after the barrier inside IssueLayerRef)
         aborted = IssueLayerRef<0>(ctx);
         if (aborted)
             break;
-        const int nextTile = tile + kRefChains * int(gridDim.x);
-        if (nextTile < params.totalTiles)
+        const uint32_t nextTile = tile + chains * gridDim.x;
+        if (nextTile < uint32_t(params.totalTiles))
         {
             place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
             const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
-            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, keepsTables && place.mipIndex == tablesMip);
+            known = keepsTables && place.mipIndex == tablesMip;
+            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, known);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
@@ -755,7 +811,7 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRef) DecodeKernel
 // (mip = clamp(floor(lod)), x = min(floor(u * W), W - 1), y likewise) is evaluated exactly as the
 // decode kernel evaluates it; the taps are read straight from global memory.
 template <bool kFp8>
-__global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) SampleKernelRef(const __grid_constant__ SampleParams params)
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __grid_constant__ SampleParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
     RefSharedStorage& shared = *reinterpret_cast<RefSharedStorage*>(dynamicShared);
@@ -763,7 +819,7 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
-    const int half = warp >> 2;
+    const int chain = warp >> 2;
 
     // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCtaRef)
     if (tid < params.numMips)
@@ -774,33 +830,36 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemLane = shared.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier[half]);
-    ctx.giveUp = SharedAddress(&shared.giveUp[half][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kRefOperandBytes) + (tid & 127);
+    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
     ctx.outStepWords = 1;
     ctx.storeBytes = params.storeBytes;
 
     const uint32_t zeroPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(0.f)));
-    const unsigned long long tiles = (params.numQueries + kRefThreadsPerCta - 1) / kRefThreadsPerCta;
+    const unsigned long long tiles = (params.numQueries + 127) / 128;
+    const int row = tid & 127;
     // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
     float nextU = 0.f, nextV = 0.f, nextLod = 0.f;
     auto requestQuery = [&](unsigned long long ofTile) {
         if (ofTile < tiles)
         {
-            const unsigned long long q = min(ofTile * kRefThreadsPerCta + tid, params.numQueries - 1);
+            const unsigned long long q = min(ofTile * 128 + row, params.numQueries - 1);
             nextU = __ldg(params.queries + 3 * q);
             nextV = __ldg(params.queries + 3 * q + 1);
             nextLod = __ldg(params.queries + 3 * q + 2);
         }
     };
-    requestQuery(blockIdx.x);
-    for (unsigned long long tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+    unsigned long long tile = blockIdx.x + (unsigned long long)chain * gridDim.x, nextTile = tile + (blockDim.x >> 7) * gridDim.x;
+    requestQuery(tile);
+    while (tile < tiles)
     {
-        const unsigned long long query = tile * kRefThreadsPerCta + tid;
+        ClaimTile(shared, chain);
+        const unsigned long long query = tile * 128 + row;
         const bool valid = query < params.numQueries;
         const float u = nextU, v = nextV, lod = nextLod;
-        requestQuery(tile + gridDim.x);
+        requestQuery(nextTile);
         const int mipIndex = max(0, min(params.numMips - 1, int(floorf(lod))));
         const KernelMip& mip = mipTable[mipIndex];
         const int x = max(0, min(mip.width - 1, int(floorf(__fmul_rn(u, float(mip.width))))));
@@ -871,6 +930,8 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
         aborted = RunLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
         if (aborted)
             break;
+        tile = nextTile;
+        nextTile = blockIdx.x + (unsigned long long)shared.claimed[chain] * gridDim.x;
         RunLayerRef<kFp8, 1, kConvertNone>(params, ctx, phase);
         RunLayerRef<kFp8, 2, kConvertNone>(params, ctx, phase);
         RunLayerRef<kFp8, 3, kConvertNone>(params, ctx, phase);
@@ -894,22 +955,52 @@ __global__ void __launch_bounds__(kRefThreadsPerCta, kCtasPerSmRefSample) Sample
 // activations, weights rebuilt from int8) stays on the binary16 path; its 32 inputs fit the same
 // 64-byte rows.
 
-using RefFp8Stage = ChainStage<TileTables<ChainTile>, kRefFootprintHiBytes, kRefFootprintLoBytes>;
+struct __align__(16) RefFp8Stage : ChainStage<TileTables<ChainTile>, kRefFootprintHiBytes, kRefFootprintLoBytes>
+{
+    TexelTables texels;
+};
 
 struct __align__(128) RefFp8SharedStorage
 {
     uint8_t network[kRefNetworkBytes];                  // layers 0-2: split e4m3 weight copies; layer 3 and bias steps: binary16
-    alignas(128) uint8_t operandA[2 * kOperandBytes];   // A operands (top half, bottom half): 128 rows x 64 bytes each
     alignas(128) uint8_t biasRegion[128 * 32];          // constant binary16 A operand of the bias step: rows (1, 0 x 15)
-    uint64_t barrier[kRefChains]; // MMA completion, per chain
+    uint64_t barrier[kMaxChains]; // MMA completion, per chain
     uint64_t loadBarrier;         // arrival of the network image
-    alignas(8) uint32_t giveUp[kRefChains][2]; // see LayerBarrier
+    alignas(8) uint32_t giveUp[kMaxChains][2]; // see LayerBarrier
+    uint32_t claims;              // inference on sample: query tiles handed out so far
+    uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    // what inference on sample does not use comes last: its launches ask for the bytes before `stage` only
-    // (with the whole structure a sample kernel's static table of mips would cost it the fourth CTA per SM)
-    alignas(128) RefFp8Stage stage[kRefChains];
+    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row; then the RefFp8Stages
 };
-static_assert(sizeof(RefFp8SharedStorage) <= kMaxSharedBytes<kCtasPerSmRefFp8>, "resident CTAs must fit into shared memory");
+static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(RefFp8Stage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
+
+// The 64-byte operand row of a texel.  `known`: TexelTables and the row's last two chunks are those of an earlier tile with the same tables.
+template <int kLayers>
+__device__ __forceinline__ void BuildInputsRefFp8(const KernelParams& params, const KernelMip& mip, RefFp8Stage& stage,
+    const RefTileContext& ctx, int tileColumn, int tileRow, bool known)
+{
+    if (!mip.staged)
+    {
+        BuildInputs<true, true, kLayers>(params, mip, stage, ctx, tileColumn, tileRow);
+        return;
+    }
+    const int texel = ctx.tid & 127;
+    if (!known)
+    {
+        PrepareTexel(stage, texel, tileColumn, tileRow);
+        // positional encoding: interleave the column's x bytes with the row's y bytes
+        const uint2 cx = stage.tables.colEnc[tileColumn];
+        const uint2 ry = stage.tables.rowEnc[tileRow];
+        ctx.rowChunk[2 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5140), __byte_perm(cx.x, ry.x, 0x7362),
+                                           __byte_perm(cx.y, ry.y, 0x5140), stage.tables.lodWord);
+        ctx.rowChunk[3 * 128] = make_uint4(0, 0, 0, 0); // K padding
+    }
+    uint32_t words[8] = {0, 0, 0, 0, 0, 0, 0, 0}; // unused feature slots hold zeros (src/Inference.cu:49)
+    GatherTexel<kLayers>(params, mip, stage, texel, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00, __half2 w01,
+        __half2 w10, __half2 w11) { words[4 * grid + layer] = BlendLayer<true>(l00, l01, l10, l11, w00, w01, w10, w11); });
+    ctx.rowChunk[0] = make_uint4(words[0], words[1], words[2], words[3]);
+    ctx.rowChunk[128] = make_uint4(words[4], words[5], words[6], words[7]);
+}
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 e4m3 operands, binary16 accumulators.
 __device__ __forceinline__ void UmmaE4m3F16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
@@ -1208,21 +1299,22 @@ __device__ __forceinline__ int RunLayerRefFp8(const Params& params, RefTileConte
 __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
     GridDependencyLaunch();
-    for (int i = tid; i < 128 * 32 / 16; i += kThreadsPerCta)
+    for (int i = tid; i < 128 * 32 / 16; i += int(blockDim.x))
         reinterpret_cast<uint4*>(shared.biasRegion)[i] = make_uint4(i < 128 ? 0x00003C00u : 0u, 0u, 0u, 0u);
     const uint32_t loadBarrier = SharedAddress(&shared.loadBarrier);
     if (tid == 0)
     {
-        for (int chain = 0; chain < kRefChains; ++chain)
+        for (int chain = 0; chain < kMaxChains; ++chain)
         {
             MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
             shared.giveUp[chain][0] = shared.giveUp[chain][1] = 0;
         }
+        shared.claims = 2 * (blockDim.x >> 7);
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
     }
     if (warp == 0)
-        TmemAlloc(SharedAddress(&shared.tmemBase), kTmemColumns);
+        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerHalf);
     GridDependencyWait();
     if (tid == 0)
     {
@@ -1245,20 +1337,19 @@ __device__ __forceinline__ void TeardownCtaRefFp8(RefFp8SharedStorage& shared, c
 {
     TcgenFenceBeforeSync();
     __syncthreads();
-    const volatile uint32_t* gaveUp = &shared.giveUp[0][0];
-    if (tid == 0 && (gaveUp[0] | gaveUp[1] | gaveUp[2] | gaveUp[3]))
+    const volatile uint32_t* gaveUp = &shared.giveUp[warp >> 2][0];
+    if ((tid & 127) == 0 && (gaveUp[0] | gaveUp[1]))
     {
-        for (int chain = 0; chain < kRefChains; ++chain)
-            (void)MbarrierWaitBounded(SharedAddress(&shared.barrier[chain]), phase ^ 1);
+        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1);
         (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
     }
     __syncthreads();
     if (warp == 0)
-        TmemFree(shared.tmemBase, kTmemColumns);
+        TmemFree(shared.tmemBase, (blockDim.x >> 7) * kTmemColumnsPerHalf);
 }
 
 template <int kConvert, int kLayers>
-__global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernelRefFp8(const __grid_constant__ KernelParams params)
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const __grid_constant__ KernelParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
     RefFp8SharedStorage& shared = *reinterpret_cast<RefFp8SharedStorage*>(dynamicShared);
@@ -1280,18 +1371,18 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kOperandBytes) + (tid & 127);
 
-    RefFp8Stage& stage = shared.stage[chain];
+    RefFp8Stage& stage = StageOf<RefFp8Stage>(shared, chain);
     struct TilePlace
     {
         int mipIndex, tileX0, tileY0;
     };
-    auto locate = [&](int tile, int fromMip) {
+    auto locate = [&](uint32_t tile, int fromMip) {
         TilePlace place;
         place.mipIndex = fromMip;
-        while (place.mipIndex + 1 < params.numMips && tile >= params.mips[place.mipIndex + 1].firstTile)
+        while (place.mipIndex + 1 < params.numMips && tile >= uint32_t(params.mips[place.mipIndex + 1].firstTile))
             ++place.mipIndex;
         const KernelMip& mip = params.mips[place.mipIndex];
-        const int local = tile - mip.firstTile;
+        const int local = int(tile) - mip.firstTile;
         const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
         place.tileX0 = (local - tileY * mip.tilesX) * kChainTileWidth;
         place.tileY0 = mip.rowBegin + tileY * kChainTileHeight;
@@ -1299,20 +1390,22 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
     };
 
     // the first chains of all CTAs take the first tiles, so that a launch of few tiles spreads over the SMs
-    int tile = int(blockIdx.x) + chain * int(gridDim.x);
+    const uint32_t chains = blockDim.x >> 7;
+    uint32_t tile = blockIdx.x + uint32_t(chain) * gridDim.x;
     TilePlace place{0, 0, 0};
+    bool known = false; // the tables, and what the threads keep of them, are already the tile's
     int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
-    if (tile < params.totalTiles)
+    if (tile < uint32_t(params.totalTiles))
     {
         place = locate(tile, 0);
         PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, false);
         tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
         ChainBarrier(chain);
     }
-    while (tile < params.totalTiles)
+    while (tile < uint32_t(params.totalTiles))
     {
         const KernelMip& mip = params.mips[place.mipIndex];
-        ctx.tile = tile;
+        ctx.tile = int(tile);
         ctx.x = place.tileX0 + tileColumn;
         ctx.y = place.tileY0 + tileRow;
         // the e4m3 input stage is the one of the exact-accumulation kernel (64-byte rows of codes)
@@ -1324,21 +1417,21 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
                 ctx.rowChunk[chunk * 128] = make_uint4(filler, filler + chunk, filler, filler);
         }
         else
-            BuildInputs<true, true, kLayers>(params, mip, stage, ctx, tileColumn, tileRow);
+            BuildInputsRefFp8<kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
 
         aborted = IssueLayerRefFp8<0>(ctx);
         if (aborted)
             break;
-        const int nextTile = tile + kRefChains * int(gridDim.x);
-        if (nextTile < params.totalTiles)
+        const uint32_t nextTile = tile + chains * gridDim.x;
+        if (nextTile < uint32_t(params.totalTiles))
         {
             if (!(kAblate & 512))
                 place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
             const bool keepsTables = (kAblate & 512) ? true : TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
+            known = keepsTables && place.mipIndex == tablesMip && !(kAblate & 64);
             if (!(kAblate & 1))
-                PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp,
-                    keepsTables && place.mipIndex == tablesMip && !(kAblate & 64));
+                PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, known);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayerRefFp8<0, kConvertNone>(params, ctx, phase);
@@ -1374,7 +1467,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) DecodeKernel
 
 // Inference on sample for FP8 networks (8-bit operands): one thread per query, taps read straight
 // from global memory.
-__global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernelRefFp8(const __grid_constant__ SampleParams params)
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const __grid_constant__ SampleParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
     RefFp8SharedStorage& shared = *reinterpret_cast<RefFp8SharedStorage*>(dynamicShared);
@@ -1382,7 +1475,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
-    const int half = warp >> 2;
+    const int chain = warp >> 2;
 
     if (tid < params.numMips)
         mipTable[tid] = params.mips[tid];
@@ -1392,32 +1485,35 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemLane = shared.tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier[half]);
-    ctx.giveUp = SharedAddress(&shared.giveUp[half][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kOperandBytes) + (tid & 127);
+    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kOperandBytes) + (tid & 127);
     ctx.outStepWords = 1;
     ctx.storeBytes = params.storeBytes;
 
-    const unsigned long long tiles = (params.numQueries + kThreadsPerCta - 1) / kThreadsPerCta;
+    const unsigned long long tiles = (params.numQueries + 127) / 128;
+    const int row = tid & 127;
     // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
     float nextU = 0.f, nextV = 0.f, nextLod = 0.f;
     auto requestQuery = [&](unsigned long long ofTile) {
         if (ofTile < tiles)
         {
-            const unsigned long long q = min(ofTile * kThreadsPerCta + tid, params.numQueries - 1);
+            const unsigned long long q = min(ofTile * 128 + row, params.numQueries - 1);
             nextU = __ldg(params.queries + 3 * q);
             nextV = __ldg(params.queries + 3 * q + 1);
             nextLod = __ldg(params.queries + 3 * q + 2);
         }
     };
-    requestQuery(blockIdx.x);
-    for (unsigned long long tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+    unsigned long long tile = blockIdx.x + (unsigned long long)chain * gridDim.x, nextTile = tile + (blockDim.x >> 7) * gridDim.x;
+    requestQuery(tile);
+    while (tile < tiles)
     {
-        const unsigned long long query = tile * kThreadsPerCta + tid;
+        ClaimTile(shared, chain);
+        const unsigned long long query = tile * 128 + row;
         const bool valid = query < params.numQueries;
         const float u = nextU, v = nextV, lod = nextLod;
-        requestQuery(tile + gridDim.x);
+        requestQuery(nextTile);
         const int mipIndex = max(0, min(params.numMips - 1, int(floorf(lod))));
         const KernelMip& mip = mipTable[mipIndex];
         const int x = max(0, min(mip.width - 1, int(floorf(__fmul_rn(u, float(mip.width))))));
@@ -1463,6 +1559,8 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
         aborted = RunLayerRefFp8<0, kConvertNone>(params, ctx, phase);
         if (aborted)
             break;
+        tile = nextTile;
+        nextTile = blockIdx.x + (unsigned long long)shared.claimed[chain] * gridDim.x;
         RunLayerRefFp8<1, kConvertNone>(params, ctx, phase);
         RunLayerRefFp8<2, kConvertNone>(params, ctx, phase);
         RunLayerRefFp8<3, kConvertNone>(params, ctx, phase);
@@ -1473,9 +1571,9 @@ __global__ void __launch_bounds__(kThreadsPerCta, kCtasPerSmRefFp8) SampleKernel
 } // namespace
 
 // One kernel, set up for its dynamic shared memory on first use per device (`done`: one bit per device).
-template <typename Kernel>
-cudaError_t LaunchRefKernel(Kernel kernel, std::atomic<unsigned long long>& done, size_t sharedBytes, int threads,
-    const KernelParams& params, int ctas, cudaStream_t stream)
+template <typename Kernel, typename Params>
+cudaError_t LaunchRefKernel(Kernel kernel, std::atomic<unsigned long long>& done, size_t sharedBytes, size_t maxSharedBytes, int chains,
+    const Params& params, int ctas, cudaStream_t stream)
 {
     int device = 0;
     cudaError_t err = cudaGetDevice(&device);
@@ -1484,12 +1582,21 @@ cudaError_t LaunchRefKernel(Kernel kernel, std::atomic<unsigned long long>& done
     const unsigned long long bit = 1ull << (device & 63);
     if (!(done.load(std::memory_order_acquire) & bit))
     {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sharedBytes));
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(maxSharedBytes));
         if (err != cudaSuccess)
             return err;
         done.fetch_or(bit, std::memory_order_release);
     }
-    return LaunchOverlapped(kernel, ctas, threads, sharedBytes, stream, params);
+    return LaunchOverlapped(kernel, ctas, 128 * chains, sharedBytes, stream, params);
+}
+
+// Chains of a CTA: no more than tiles, a power of two as the tensor-memory allocation has to be.
+int ChainsPerCta(unsigned long long tiles, int ctas)
+{
+    int chains = 1;
+    while (chains < kMaxChains && (unsigned long long)chains * (unsigned long long)ctas < tiles)
+        chains *= 2;
+    return chains;
 }
 
 // The kernel of a weight set and epilogue compiled for 2, 3 or 4 latent layers, or the one for any number.
@@ -1499,10 +1606,13 @@ cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStre
     static std::atomic<unsigned long long> done[5];
     auto launch = [&](auto layers) {
         constexpr int kLayers = decltype(layers)::value;
+        const int chains = ChainsPerCta(uint32_t(params.totalTiles), ctas);
         if constexpr (kFp8Weights) // 8-bit operands
-            return LaunchRefKernel(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], sizeof(RefFp8SharedStorage), kThreadsPerCta, params, ctas, stream);
+            return LaunchRefKernel(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, sizeof(RefFp8Stage)),
+                SharedBytes<RefFp8SharedStorage>(kMaxChains, sizeof(RefFp8Stage)), chains, params, ctas, stream);
         else
-            return LaunchRefKernel(DecodeKernelRef<false, kConvert, kLayers>, done[kLayers], sizeof(RefSharedStorage), kRefThreadsPerCta, params, ctas, stream);
+            return LaunchRefKernel(DecodeKernelRef<false, kConvert, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, sizeof(RefStage)),
+                SharedBytes<RefSharedStorage>(kMaxChains, sizeof(RefStage)), chains, params, ctas, stream);
     };
     switch (params.numLayers)
     {
@@ -1529,38 +1639,10 @@ cudaError_t LaunchDecodeRef(const KernelParams& params, bool fp8, int ctas, cuda
 cudaError_t LaunchSampleRef(const SampleParams& params, bool fp8, int ctas, cudaStream_t stream)
 {
     static std::atomic<unsigned long long> done[2];
-    auto launch = [&](auto kernel, std::atomic<unsigned long long>& doneMask) -> cudaError_t {
-        int device = 0;
-        cudaError_t err = cudaGetDevice(&device);
-        if (err != cudaSuccess)
-            return err;
-        const unsigned long long bit = 1ull << (device & 63);
-        if (!(doneMask.load(std::memory_order_acquire) & bit))
-        {
-            err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(offsetof(RefSharedStorage, stage)));
-            if (err != cudaSuccess)
-                return err;
-            doneMask.fetch_or(bit, std::memory_order_release);
-        }
-        return LaunchOverlapped(kernel, ctas, kRefThreadsPerCta, offsetof(RefSharedStorage, stage), stream, params);
-    };
-    if (fp8)
-    {
-        int device = 0;
-        cudaError_t err = cudaGetDevice(&device);
-        if (err != cudaSuccess)
-            return err;
-        const unsigned long long bit = 1ull << (device & 63);
-        if (!(done[1].load(std::memory_order_acquire) & bit))
-        {
-            err = cudaFuncSetAttribute(SampleKernelRefFp8, cudaFuncAttributeMaxDynamicSharedMemorySize, int(offsetof(RefFp8SharedStorage, stage)));
-            if (err != cudaSuccess)
-                return err;
-            done[1].fetch_or(bit, std::memory_order_release);
-        }
-        return LaunchOverlapped(SampleKernelRefFp8, ctas, kThreadsPerCta, offsetof(RefFp8SharedStorage, stage), stream, params);
-    }
-    return launch(SampleKernelRef<false>, done[0]);
+    const int chains = ChainsPerCta((params.numQueries + 127) / 128, ctas);
+    // the tables and footprints are not used
+    return fp8 ? LaunchRefKernel(SampleKernelRefFp8, done[1], SharedBytes<RefFp8SharedStorage>(chains, 0), SharedBytes<RefFp8SharedStorage>(kMaxChains, 0), chains, params, ctas, stream)
+               : LaunchRefKernel(SampleKernelRef<false>, done[0], SharedBytes<RefSharedStorage>(chains, 0), SharedBytes<RefSharedStorage>(kMaxChains, 0), chains, params, ctas, stream);
 }
 
 } // namespace ntcb

@@ -362,10 +362,7 @@ __device__ __forceinline__ uint32_t ElectOne()
 // All 128 threads of a chain.
 __device__ __forceinline__ void ChainBarrier(int chain)
 {
-    if (chain)
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-    else
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+    asm volatile("bar.sync %0, 128;" ::"r"(chain + 1) : "memory");
 }
 
 // The barrier before a layer's matrix products (reference-numerics kernels).  The operand rows, tables and footprints of a

@@ -240,11 +240,9 @@ int ResidentCtas(bool fp8, bool converting, int* outCtas, bool reference = false
     // occupancy query reports one CTA per SM for kernels that allocate tensor memory, so it is not
     // used here.)
     static_assert(kCtasPerSmInt8 * kTmemColumns <= 512 && kCtasPerSmFp8 * kTmemColumns <= 512 &&
-                      kCtasPerSmConverting * kTmemColumns <= 512 && kCtasPerSmRef * kRefTmemColumns <= 512 &&
-                      kCtasPerSmRefSample * kRefTmemColumns <= 512 &&
-                      kCtasPerSmRefFp8 * kTmemColumns <= 512,
+                      kCtasPerSmConverting * kTmemColumns <= 512 && kMaxChains * kTmemColumnsPerHalf <= 512,
         "resident CTAs must fit into tensor memory");
-    const int perSm = reference ? (fp8 ? kCtasPerSmRefFp8 : sample ? kCtasPerSmRefSample : kCtasPerSmRef) : converting ? kCtasPerSmConverting : fp8 ? kCtasPerSmFp8 : kCtasPerSmInt8;
+    const int perSm = reference ? 1 : converting ? kCtasPerSmConverting : fp8 ? kCtasPerSmFp8 : kCtasPerSmInt8;
     *outCtas = sms * perSm;
     if (device >= 0 && device < 64)
         cache[device][variant].store(*outCtas, std::memory_order_relaxed);
@@ -796,7 +794,7 @@ int ntcb_sample(const NtcbSampleParams* p, void* stream)
     int rc = ResidentCtas(fp8, false, &resident, reference, true);
     if (rc != NTCB_OK)
         return rc;
-    const unsigned long long perCta = reference ? kRefThreadsPerCta : kThreadsPerCta;
+    const unsigned long long perCta = reference ? 128 : kThreadsPerCta; // (reference numerics: of a chain)
     const unsigned long long tiles = (p->numQueries + perCta - 1) / perCta;
     const int ctas = tiles < (unsigned long long)resident ? int(tiles) : resident;
     cudaError_t err = reference ? LaunchSampleRef(k, fp8, ctas, static_cast<cudaStream_t>(stream))
