@@ -81,8 +81,9 @@ constexpr int kRefInt8NetworkBytes = 17408; // ... what the Int8 kernels copy to
 // has 48 inputs; of layer 1's 64 the first 32 are here, the other 32 in tensor memory, like all of
 // layers 2 and 3.
 constexpr int kRefOperandBytes = 128 * 96;
-// Reference-numerics kernels: a CTA is two chains of 128 threads that share the network in shared memory and nothing else.
-// Each walks tiles of its own, 16 x 8 texels, with its own tables and footprints, and meets only its own threads in barriers.
+// Reference-numerics kernels: a CTA is up to eight chains of 128 threads - 64 tensor-memory columns and 64 registers a thread each, which
+// fills an SM - that share the network in shared memory and nothing else.  Each walks tiles of its own, 16 x 8 texels, with its
+// own tables and footprints, and meets only its own threads in barriers.
 constexpr int kChainTileWidth = 16;
 constexpr int kChainTileHeight = 8;
 constexpr int kMaxChains = 8;

@@ -4,9 +4,15 @@
 //
 // tcgen05.mma kind::f16 with a binary16 accumulator format (K = 16 per instruction) rounds exactly
 // like the legacy wmma m16n16k16 path the reference is built on, so this kernel reproduces the
-// reference's output bit for bit while keeping the structure of the exact-accumulation kernel in
-// decode_kernel.cu: a 32x8 texel tile per CTA of 256 threads (thread = texel), two 128-row GEMM
-// chains per tile, weights resident in shared memory, accumulators in tensor memory.
+// reference's output bit for bit: thread = texel, 128-row GEMM chains, weights resident in shared memory, accumulators in
+// tensor memory, as in decode_kernel.cu.
+//
+// Work decomposition.  One CTA per SM of up to eight chains of 128 threads.  The chains share the network and nothing else: each
+// walks tiles of 16 x 8 texels of its own, with its own tables and footprints, and meets only its own threads in
+// barriers.  What bounds the kernels is instruction issue (75 % of the slots busy; 8 x 4 warps of 64 registers and 8 x 64
+// tensor-memory columns fill an SM), so the split aims at few instructions and warps that never wait for another chain.  (With four
+// CTAs per SM of two chains each, the four copies of the network left no room for TexelTables, and on average 3.3 of the four were
+// active - the scheduler favours the older, whose share ends early: 4096 x 4096 FP8 897 us, now 832; 8192 x 8192 Int8 4985, now 4523.)
 //
 // What differs from decode_kernel.cu:
 //   * the A operand holds binary16 values (the de-quantised network inputs / activations), up to 128
@@ -15,8 +21,6 @@
 //     it from tensor memory, where the activation step stores it (columns 32.. of the chain's 64,
 //     beside those layers' accumulators); layer 1 reads its first two K steps from shared memory and
 //     its last two from the 16 tensor-memory columns its 48 accumulators leave free;
-//   * between the layers of a tile the two chains do not wait for each other (LayerBarrier,
-//     kernel_parts.cuh);
 //   * each layer starts with a "bias step": an MMA whose A operand has constant rows - a unit vector -
 //     and whose B operand holds the bias in the column the unit vector picks, which sets the
 //     accumulators to the binary16 bias exactly; the K = 16 steps of the layer then accumulate onto it.
@@ -51,7 +55,7 @@
 #include "output_convert.cuh"
 #include "epilogue_convert.cuh"
 
-// Profiling aid: NTCB_ABLATE (a bit mask, 0 in the product build; 512: no tile walk, every tile at the place of the CTA's
+// Profiling aid: NTCB_ABLATE (a bit mask, 0 in the product build; 512: no tile walk, every tile at the place of the chain's
 // first; 1024: no barrier before a layer's products - only together with 16) removes one phase of
 // DecodeKernelRefFp8 at a time so that its share of the kernel's instructions and time can be
 // measured as a difference (`make ablations` builds one library per mask; their output is wrong by
@@ -303,7 +307,7 @@ struct RefTileContext
     uint32_t tmemLane;    // the chain's first tensor-memory column at this thread's lane (its warp's first lane, to be precise)
     uint32_t barrier;     // shared address of the chain's MMA-completion mbarrier
     uint32_t giveUp;      // shared address of the chain's give-up word for the current tile (LayerBarrier)
-    uint4* rowChunk; // this thread's 16-byte slot in chunk 0 of its half's A operand
+    uint4* rowChunk; // this thread's 16-byte slot in chunk 0 of its chain's A operand
     int tile, x, y;
     uint32_t* out;
     uint32_t outStepWords;
@@ -951,7 +955,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
 // which one has columns 16-31 zeroed and the other columns 0-15: each instruction adds 16 real
 // products (and 16 exact zeros) to the accumulator and rounds once - bit for bit what the binary16
 // path does (checked on the GPU against wmma on 1.2 M accumulators before this kernel was written).
-// The A operand shrinks to 64 bytes per row, which lets four CTAs share an SM.  Layer 3 (int8-grid
+// The A operand shrinks to 64 bytes per row.  Layer 3 (int8-grid
 // activations, weights rebuilt from int8) stays on the binary16 path; its 32 inputs fit the same
 // 64-byte rows.
 

@@ -2,7 +2,7 @@
 // pairs) become the pixel in the client's channel format and are stored.  `Context` is the
 // kernel's per-thread tile context: `out` is the address of the thread's pixel, `outStepWords` the
 // pixel's linear index in its mip (the dither seed), `rowChunk` the thread's 16-byte slot in chunk 0
-// of its half's A operand (chunks are 2048 bytes apart).
+// of its chain's A operand (chunks are 2048 bytes apart).
 #pragma once
 
 #include <cuda_fp16.h>

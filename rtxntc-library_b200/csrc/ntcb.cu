@@ -206,10 +206,10 @@ namespace
 {
 
 // Number of CTAs that fill the current device, cached per device.
-int ResidentCtas(bool fp8, bool converting, int* outCtas, bool reference = false, bool sample = false)
+int ResidentCtas(bool fp8, bool converting, int* outCtas, bool reference = false)
 {
-    static std::atomic<int> cache[64][6];
-    const int variant = reference ? (fp8 ? 4 : sample ? 5 : 3) : converting ? 2 : fp8 ? 1 : 0;
+    static std::atomic<int> cache[64][4];
+    const int variant = reference ? 3 : converting ? 2 : fp8 ? 1 : 0;
     int device = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess)
@@ -235,7 +235,8 @@ int ResidentCtas(bool fp8, bool converting, int* outCtas, bool reference = false
             device, major);
         return NTCB_ERR_CUDA;
     }
-    // The kernel is compiled for kCtasPerSmInt8 / kCtasPerSmFp8 resident CTAs (__launch_bounds__), each of which holds
+    // The reference-numerics kernels run one CTA per SM, whose chains fill the tensor memory.  The exact kernels are compiled for
+    // kCtasPerSmInt8 / kCtasPerSmFp8 resident CTAs (__launch_bounds__), each of which holds
     // kTmemColumns of the SM's 512 tensor-memory columns for its whole lifetime.  (The runtime's
     // occupancy query reports one CTA per SM for kernels that allocate tensor memory, so it is not
     // used here.)
@@ -791,7 +792,7 @@ int ntcb_sample(const NtcbSampleParams* p, void* stream)
         return NTCB_OK;
     const bool fp8 = p->weightMode == NTCB_WEIGHTS_FP8;
     int resident = 0;
-    int rc = ResidentCtas(fp8, false, &resident, reference, true);
+    int rc = ResidentCtas(fp8, false, &resident, reference);
     if (rc != NTCB_OK)
         return rc;
     const unsigned long long perCta = reference ? 128 : kThreadsPerCta; // (reference numerics: of a chain)
