@@ -248,20 +248,29 @@ def check(code: int) -> None:
         raise NtcbError(code, lib().ntcb_last_error().decode())
 
 
+_torch_c = None
+
+
 def _queue(device, entry_point, *arguments) -> None:
     """Calls a C entry point whose last argument is a stream with torch's current stream of `device` (a torch.device
     with an index), on that device.  The small launches are bound by what Python does per call, so the stream is looked
     up as a plain handle (torch.cuda.current_stream() builds an object: 3.3 us) and the device is only switched when
     another one is current (the context manager: 1.5 us)."""
-    import torch
+    global _torch_c
+    if _torch_c is None:
+        import torch
 
+        _torch_c = torch._C
     index = device.index
-    stream = torch._C._cuda_getCurrentRawStream(index)
-    if torch.cuda.current_device() == index:
-        check(entry_point(*arguments, stream))
+    if _torch_c._cuda_getDevice() == index:
+        code = entry_point(*arguments, _torch_c._cuda_getCurrentRawStream(index))
     else:
+        import torch
+
         with torch.cuda.device(index):
-            check(entry_point(*arguments, stream))
+            code = entry_point(*arguments, _torch_c._cuda_getCurrentRawStream(index))
+    if code:
+        check(code)
 
 
 def stage_network(blob: bytes, weight_mode: int, numerics: int = NUMERICS_REFERENCE) -> np.ndarray:
@@ -398,7 +407,7 @@ def pack_latents(latents, width: int, height: int, num_layers: int, latent_strid
     needed = (num_layers - 1) * latent_stride * 2 + latent_stride + width * height * 2
     if latents.dtype != torch.float16 or latents.numel() < needed:
         raise ValueError(f"latents must be float16 with at least {needed} elements")
-    out = torch.empty((num_layers, height, width), dtype=torch.int16, device=latents.device)
+    out = latents.new_empty((num_layers, height, width), dtype=torch.int16)  # (0.5 us less than torch.empty on a device)
     _queue(latents.device, lib().ntcb_pack_latents, latents.data_ptr(), width, height, num_layers, latent_stride, out.data_ptr())
     return out
 
@@ -415,19 +424,18 @@ def quantize_network(weights, biases, weight_mode: int, output_scale=None, outpu
     if biases.dtype != torch.float16 or biases.numel() != NETWORK_COLUMN_COUNT:
         raise ValueError("biases must be float16 with NETWORK_COLUMN_COUNT elements")
     blob_bytes = INT8_BLOB_BYTES if weight_mode == WEIGHTS_INT8 else FP8_BLOB_BYTES
-    blob = torch.empty(blob_bytes, dtype=torch.uint8, device=weights.device)  # the sections fill it without gaps
+    blob = weights.new_empty(blob_bytes, dtype=torch.uint8)  # the sections fill it without gaps
     rounded = torch.empty_like(weights) if want_rounded else None
     params = QuantizeNetworkParams()
     params.weights, params.biases = weights.data_ptr(), biases.data_ptr()
-    keep = []
-    for name, values in (("outputScale", output_scale), ("outputBias", output_bias)):
-        if values is not None:
-            array = (ctypes.c_float * 16)(*[float(v) for v in values])
-            keep.append(array)
-            setattr(params, name, array)
+    if output_scale is not None:
+        params.outputScale = (ctypes.c_float * 16)(*[float(v) for v in output_scale])
+    if output_bias is not None:
+        params.outputBias = (ctypes.c_float * 16)(*[float(v) for v in output_bias])
     params.weightMode = weight_mode
     params.blob = blob.data_ptr()
-    params.roundedWeights = rounded.data_ptr() if want_rounded else None
+    if want_rounded:
+        params.roundedWeights = rounded.data_ptr()
     _queue(weights.device, lib().ntcb_quantize_network, ctypes.byref(params))
     return (blob, rounded) if want_rounded else blob
 
