@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert != kConvertNone ? kCt
 // (the reference's NtcSampleTextureSet takes an integer texel and mip and runs the same network,
 // include/libntc/shaders/Inference.hlsli:282-357).  Queries are incoherent, so the taps are read
 // straight from global memory; a tile is 256 consecutive queries, i.e. two 128-row GEMM chains.
-template <bool kFp8>
+template <bool kFp8, bool kInterleaved, int kLayers>
 __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPerSmInt8) SampleKernel(const __grid_constant__ SampleParams params)
 {
     // more than the 48 KB a kernel may declare statically: passed as dynamic shared memory at launch
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPe
             const uint32_t slotFill = kFp8 ? 0u : kBiasSlotValue * 0x01010101u;
             words[12] = words[13] = words[14] = slotFill;
             words[15] = kFp8 ? 0u : ((slotFill & 0x00FFFFFFu) | 0x01000000u);
-            SampleGridsDirect<kFp8, false>(params.latents, params.numLayers, mip, x, y, words, params.interleaved != 0);
+            SampleGridsDirect<kFp8, false>(params.latents, kLayers ? kLayers : params.numLayers, mip, x, y, words, kInterleaved);
             // src/RegressionKernels.h:59-85
             float xf = __fmul_rn(float(x), mip.positionScale);
             float yf = __fmul_rn(float(y), mip.positionScale);
@@ -748,14 +748,30 @@ cudaError_t LaunchDecodeLayers(const KernelParams& params, int ctas, cudaStream_
     }
 }
 
+template <bool kFp8, bool kInterleaved>
+cudaError_t LaunchSampleLayers(const SampleParams& params, int ctas, cudaStream_t stream)
+{
+    static std::atomic<unsigned long long> done[4];
+    const size_t bytes = offsetof(SharedStorage, stage); // the tables and footprints are not used
+    if constexpr (kInterleaved) // as in the reference-numerics kernels: the presets' layer counts
+    {
+        switch (params.numLayers)
+        {
+        case 2: return LaunchWithSharedStorage(SampleKernel<kFp8, true, 2>, done[1], params, ctas, stream, bytes);
+        case 3: return LaunchWithSharedStorage(SampleKernel<kFp8, true, 3>, done[2], params, ctas, stream, bytes);
+        case 4: return LaunchWithSharedStorage(SampleKernel<kFp8, true, 4>, done[3], params, ctas, stream, bytes);
+        }
+    }
+    return LaunchWithSharedStorage(SampleKernel<kFp8, kInterleaved, 0>, done[0], params, ctas, stream, bytes);
+}
+
 } // namespace
 
 cudaError_t LaunchSample(const SampleParams& params, bool fp8, int ctas, cudaStream_t stream)
 {
-    static std::atomic<unsigned long long> done[2];
-    const size_t bytes = offsetof(SharedStorage, stage); // the tables and footprints are not used
-    return fp8 ? LaunchWithSharedStorage(SampleKernel<true>, done[1], params, ctas, stream, bytes)
-               : LaunchWithSharedStorage(SampleKernel<false>, done[0], params, ctas, stream, bytes);
+    if (fp8)
+        return params.interleaved ? LaunchSampleLayers<true, true>(params, ctas, stream) : LaunchSampleLayers<true, false>(params, ctas, stream);
+    return params.interleaved ? LaunchSampleLayers<false, true>(params, ctas, stream) : LaunchSampleLayers<false, false>(params, ctas, stream);
 }
 
 cudaError_t LaunchDecode(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream)
