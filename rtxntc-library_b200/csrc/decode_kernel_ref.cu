@@ -301,10 +301,16 @@ __device__ __forceinline__ void ClaimTile(Storage& shared, int chain)
         shared.claimed[chain] = atomicAdd(&shared.claims, 1u);
 }
 
-// The warp of a chain that hands its products to the tensor core.  All four meet before every layer, so the busiest sets the pace:
-// warps 0 and 1 stage the footprints (warp 2 a share of large ones), so it is the last one.  (Issued by warp 0, which also stages the
-// high-res grid, a 4096 x 4096 FP8 set took 832 us instead of 774, an 8192 x 8192 Int8 one 4527 instead of 4256.)
-constexpr int kIssuingWarp = 3;
+// What a warp of a chain does besides its texels: roles 0 and 1 stage the footprints of the high-res and the low-res grid (2 and 3 the rest of large
+// ones), role 3 hands the products to the tensor core.  All four meet before every layer, so the busiest sets the pace.
+// Warp w of every chain runs on sub-partition w % 4 of the SM, so the roles go round from chain to chain.
+// (Warp 0 staging and issuing in every chain: 4096 x 4096 FP8 832 us, 8192 x 8192 Int8 4530, 16.7 M queries 725.  Issued by warp 3 instead: 775,
+// 4210, 723.  Rotated: 780, 4190, 692, and 8-bit pixels 962 instead of 985.)
+constexpr int kIssuingRole = 3;
+__device__ __forceinline__ int WarpRole(int warpIndex)
+{
+    return (warpIndex + (warpIndex >> 2)) & 3;
+}
 
 struct RefTileContext
 {
@@ -525,7 +531,7 @@ __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
     // The whole issuing warp runs the descriptor arithmetic on values that are visibly the same in every
     // lane; one elected lane hands the work to the tensor core (see IssueLayerRefFp8).
     const int warpIndex = ctx.tid >> 5;
-    if ((warpIndex & 3) == kIssuingWarp)
+    if (WarpRole(warpIndex) == kIssuingRole)
     {
         TcgenFenceAfterSync();
         constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
@@ -713,7 +719,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int chain = warp >> 2, chainWarp = warp & 3;
+    const int chain = warp >> 2, role = WarpRole(warp);
     const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
     SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
@@ -755,7 +761,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
     if (tile < uint32_t(params.totalTiles))
     {
         place = locate(tile, 0);
-        PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, false);
+        PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, false);
         tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
         ChainBarrier(chain);
     }
@@ -779,7 +785,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
             const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
             known = keepsTables && place.mipIndex == tablesMip;
-            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, known);
+            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
@@ -1118,7 +1124,7 @@ __device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
     // from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
     // (Tried: building the descriptors before the barrier - 3 % slower.)
     const int warpIndex = ctx.tid >> 5;
-    if ((warpIndex & 3) == kIssuingWarp && !(kAblate & 16))
+    if (WarpRole(warpIndex) == kIssuingRole && !(kAblate & 16))
     {
         TcgenFenceAfterSync();
         const uint32_t elected = ElectOne();
@@ -1367,7 +1373,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int chain = warp >> 2, chainWarp = warp & 3;
+    const int chain = warp >> 2, role = WarpRole(warp);
     const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
     SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
@@ -1408,7 +1414,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const
     if (tile < uint32_t(params.totalTiles))
     {
         place = locate(tile, 0);
-        PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, false);
+        PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, false);
         tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
         ChainBarrier(chain);
     }
@@ -1441,7 +1447,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const
             const bool keepsTables = (kAblate & 512) ? true : TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
             known = keepsTables && place.mipIndex == tablesMip && !(kAblate & 64);
             if (!(kAblate & 1))
-                PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, chainWarp, known);
+                PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayerRefFp8<0, kConvertNone>(params, ctx, phase);
