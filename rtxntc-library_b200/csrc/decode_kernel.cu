@@ -414,7 +414,6 @@ __device__ __forceinline__ int RunLayer(const Params& params, const SharedStorag
 // bounded wait for the copy done, tensor memory released): the caller returns at once.
 __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
-    GridDependencyLaunch();
     // constant inputs of the bias K step: 31 slots of kBiasSlotValue and a last slot of 1 per row
     for (int i = tid; i < kBiasRegionBytes / 16; i += kThreadsPerCta)
     {
@@ -441,6 +440,7 @@ __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* ne
     TcgenFenceBeforeSync();
     __syncthreads();         // also publishes the barriers' initialisation
     TcgenFenceAfterSync();
+    GridDependencyLaunch();
     int failed = 0;
     if (!MbarrierWaitBounded(loadBarrier, 0, loadWaitPolls))
     {

@@ -648,7 +648,6 @@ __device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext&
 // thread that gave up waiting for the image (status words written).
 __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
-    GridDependencyLaunch();
     // constant A operands of the bias steps: core matrix l (8 rows of 16 bytes) has 1.0 as half l of every row,
     // core matrix 4 is zero
     for (int i = tid; i < 5 * 8; i += int(blockDim.x))
@@ -681,6 +680,7 @@ __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint
     TcgenFenceBeforeSync();
     __syncthreads();
     TcgenFenceAfterSync();
+    GridDependencyLaunch();
     if (!MbarrierWaitBounded(loadBarrier, 0, loadWaitPolls))
     {
         SetGiveUp(SharedAddress(&shared.giveUp[tid >> 7][0]));
@@ -1314,7 +1314,6 @@ __device__ __forceinline__ int RunLayerRefFp8(const Params& params, RefTileConte
 // Setup and teardown as for the binary16 kernel, on the FP8 kernel's shared-memory structure.
 __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
-    GridDependencyLaunch();
     for (int i = tid; i < 128 * 32 / 16; i += int(blockDim.x))
         reinterpret_cast<uint4*>(shared.biasRegion)[i] = make_uint4(i < 128 ? 0x00003C00u : 0u, 0u, 0u, 0u);
     const uint32_t loadBarrier = SharedAddress(&shared.loadBarrier);
@@ -1341,6 +1340,7 @@ __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, cons
     TcgenFenceBeforeSync();
     __syncthreads();
     TcgenFenceAfterSync();
+    GridDependencyLaunch();
     if (!MbarrierWaitBounded(loadBarrier, 0, loadWaitPolls))
     {
         SetGiveUp(SharedAddress(&shared.giveUp[tid >> 7][0]));

@@ -103,9 +103,13 @@ __device__ __noinline__ void ReportTimeout(uint32_t* status, uint32_t tile, uint
 }
 
 // Programmatic dependent launch: the decode kernels are launched so that the next one in the stream may start once all
-// CTAs of this one are running (LaunchOverlapped).  Until GridDependencyWait returns - everything before this
-// kernel in the stream has completed and is visible - a CTA touches nothing in global memory; it sets up barriers, constant tables
-// and tensor memory meanwhile.
+// CTAs of this one are running and hold their tensor memory (LaunchOverlapped).  Until GridDependencyWait returns - everything
+// before this kernel in the stream has completed and is visible - a CTA touches nothing in global memory; it sets up barriers,
+// constant tables and tensor memory meanwhile.
+//
+// GridDependencyLaunch comes after the barrier that follows the CTA's TmemAlloc, never before: a CTA of the next kernel takes its
+// columns and keeps them while it waits for this kernel to end, so a CTA of this kernel that had not allocated by then
+// could wait for those columns for good.
 __device__ __forceinline__ void GridDependencyWait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -359,6 +359,36 @@ def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, 
         texture_set.close()
 
 
+@BOTH_NUMERICS
+def test_kernels_queued_back_to_back_overlap_without_a_trace(numerics):
+    """A decode or sample kernel starts while the one before it in the stream still runs and waits for its end: launches
+    of few and of many CTAs in turn, each of which reads or overwrites what the ones around it use, give the bits
+    that they give one at a time."""
+    import torch
+
+    sets = [binding.ResidentTextureSet.from_synthetic(synthetic.make_texture_set(
+        synthetic.TextureSetSpec(w, h, c, 0, 2, f, seed=w, network="unit")), numerics=numerics) for w, h, c, f in ((40, 24, 4, 8), (512, 700, 8, 12))]
+    queries = torch.rand((3000, 3), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    expected = {}
+    for use_int8 in (False, True):
+        for index, resident in enumerate(sets):
+            resident.decode(use_int8)
+            _sync()
+            expected[index, use_int8] = resident.out.clone(), resident.sample(queries, use_int8)
+            _sync()
+    queued = []
+    for step in range(60):
+        index, use_int8 = (step * 5 // 3) % 2, step % 3 == 0
+        sets[index].decode(use_int8)
+        queued.append((index, use_int8, sets[index].out.clone() if step % 4 == 0 else None, sets[index].sample(queries, use_int8)))
+    _sync()
+    for index, use_int8, texels, answers in queued:
+        assert texels is None or torch.equal(texels.view(torch.int16), expected[index, use_int8][0].view(torch.int16))
+        assert torch.equal(answers.view(torch.int16), expected[index, use_int8][1].view(torch.int16))
+    for resident in sets:
+        resident.check_status()
+
+
 def test_live_reference_comparison(oracle):
     """Runs the unmodified reference decoder (oracle/_ref) on this GPU next to ours on a set the
     fixtures do not contain."""
