@@ -485,7 +485,7 @@ int ntcb_quantize_network(const NtcbQuantizeNetworkParams* params, void* stream)
    before any stream capture).  Queued on `stream`; returns without waiting. */
 typedef struct NtcbBlockCompressParams
 {
-    const void* deviceMip;   /* decoded texels of one mip */
+    const void* deviceMip;   /* decoded texels of one mip, 2-byte aligned (at multiples of 4 the loads are wider) */
     int32_t layout;          /* NtcbOutputLayout of deviceMip */
     int32_t width, height, channels; /* of deviceMip */
     int32_t firstChannel;    /* BC4: the channel; BC5: it and the next; BC1-3, BC7: red, then green, blue, alpha */

@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kBc4Threads) BlockCompressKernel(const Bc4Argu
     const int blocks = min(args.blocksPerCta, args.totalBlocks - firstBlock);
     if (tid < 2)
         shared.next[tid] = 0;
-    const bool pairs = args.channels == 2 && !(args.base.firstChannel & 1) && !(args.base.channels & 1);
+    const bool pairs = args.channels == 2 && args.base.pairs;
     // a column of four texels per thread and turn, neighbouring threads on neighbouring columns
     for (int within = tid; within < 4 * blocks; within += kBc4Threads)
     {
@@ -1103,8 +1103,6 @@ __global__ void __launch_bounds__(kColorThreads, 8) ColorBlockCompressKernel(con
     const int tid = threadIdx.x;
     // The CTA's 64 x 16 texels are loaded with neighbouring threads on neighbouring texels of a row
     // (coalesced) and handed to the threads that own their block through shared memory.
-    // an even first channel of an even channel count: channel pairs are aligned 32-bit words in both layouts
-    const bool pairs = !(args.base.firstChannel & 1) && !(args.base.channels & 1);
 #pragma unroll 4
     for (int k = 0; k < 16 * kColorBlocks / kColorThreads; ++k)
     {
@@ -1117,7 +1115,7 @@ __global__ void __launch_bounds__(kColorThreads, 8) ColorBlockCompressKernel(con
         if (inside)
         {
             const int first = args.base.firstChannel, count = args.numChannels;
-            if (pairs)
+            if (args.base.pairs)
             {
                 redGreen = count >= 2 ? LoadPair(args.base, x, y, first) : uint32_t(__half_as_ushort(LoadHalf(args.base, x, y, first)));
                 blueAlpha = count == 4 ? LoadPair(args.base, x, y, first + 2)
@@ -1298,6 +1296,12 @@ extern "C" int ntcb_block_compress(const NtcbBlockCompressParams* params, void* 
         return NTCB_ERR_INVALID_ARGUMENT;
     }
 
+    if (reinterpret_cast<uintptr_t>(params->deviceMip) & 1)
+    {
+        SetError("ntcb_block_compress: deviceMip must be 2-byte aligned.");
+        return NTCB_ERR_INVALID_ARGUMENT;
+    }
+
     BlockCompressArguments args;
     args.texels = static_cast<const __half*>(params->deviceMip);
     args.layout = params->layout;
@@ -1310,6 +1314,7 @@ extern "C" int ntcb_block_compress(const NtcbBlockCompressParams* params, void* 
     args.widthInBlocks = params->widthInBlocks;
     args.heightInBlocks = params->heightInBlocks;
     args.formatChannels = formatChannels;
+    args.pairs = ChannelPairs(args);
     args.blocks = static_cast<uint8_t*>(params->deviceBlocks);
     args.rowPitch = params->rowPitch;
 

@@ -15,20 +15,16 @@ struct BlockCompressArguments
     const __half* texels;
     int layout, width, height, channels, firstChannel;
     int srcLeft, srcTop, widthInBlocks, heightInBlocks, formatChannels;
+    bool pairs; // see ChannelPairs
     uint8_t* blocks;
     size_t rowPitch;
 };
 
-// A texel outside the mip reads as 0, as an out-of-range texture load does.
-__device__ __forceinline__ float LoadChannel(const BlockCompressArguments& args, int x, int y, int channel)
+// Whether channel firstChannel and those two, four ... after it can be loaded with the next one as an aligned 32-bit word (LoadPair): in
+// both layouts when the mip starts on such a word, the channel is even and so is their count.  `texels` may be any address of halves.
+inline bool ChannelPairs(const BlockCompressArguments& args)
 {
-    if (x >= args.width || y >= args.height)
-        return 0.f;
-    const size_t w = size_t(args.width), c = size_t(args.channels);
-    const size_t index = args.layout == NTCB_LAYOUT_INTERLEAVED
-        ? (size_t(y) * w + size_t(x)) * c + size_t(channel)
-        : size_t(y) * w * c + size_t(channel & ~1) * w + 2 * size_t(x) + size_t(channel & 1);
-    return __half2float(args.texels[index]);
+    return !(reinterpret_cast<uintptr_t>(args.texels) & 3) && !(args.firstChannel & 1) && !(args.channels & 1);
 }
 
 __device__ __forceinline__ __half LoadHalf(const BlockCompressArguments& args, int x, int y, int channel)
@@ -40,7 +36,7 @@ __device__ __forceinline__ __half LoadHalf(const BlockCompressArguments& args, i
     return args.texels[index];
 }
 
-// Channels `channel` (even) and `channel + 1` of one texel as one word; needs an even channel count.
+// Channels `channel` and `channel + 1` of one texel as one word (args.pairs).
 __device__ __forceinline__ uint32_t LoadPair(const BlockCompressArguments& args, int x, int y, int channel)
 {
     const size_t w = size_t(args.width), c = size_t(args.channels);

@@ -848,7 +848,7 @@ __device__ __forceinline__ uint2 LoadTexel(const Bc7Arguments& args, int x, int 
     if (x >= args.base.width || y >= args.base.height)
         return make_uint2(0u, 0u);
     const int first = args.base.firstChannel, count = args.numChannels;
-    if (!(first & 1) && !(args.base.channels & 1)) // channel pairs are aligned words in both layouts
+    if (args.base.pairs)
     {
         const uint32_t redGreen = count >= 2 ? LoadPair(args.base, x, y, first) : uint32_t(__half_as_ushort(LoadHalf(args.base, x, y, first)));
         const uint32_t blueAlpha = count == 4 ? LoadPair(args.base, x, y, first + 2)

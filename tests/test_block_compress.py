@@ -346,6 +346,8 @@ def test_arguments_are_checked():
     assert lib.ntcb_block_compress(params, None) == -1 and b"rowPitch" in lib.ntcb_last_error()
     params.format, params.rowPitch, params.srcLeft = binding.BLOCK_FORMAT_BC4, 16, -4
     assert lib.ntcb_block_compress(params, None) == -9 and b"srcLeft" in lib.ntcb_last_error()
+    params.srcLeft, params.deviceMip = 0, 4097
+    assert lib.ntcb_block_compress(params, None) == -1 and b"deviceMip" in lib.ntcb_last_error()
 
 
 # ---------------------------------------------------------------------------------------------
@@ -542,6 +544,24 @@ def test_colour_kernels_with_odd_channel_offsets_and_the_planar_layout(oracle):
         got = binding.block_compress(torch.from_numpy(planar).cuda(), binding.BLOCK_FORMAT_BC1, first, layout=binding.LAYOUT_PLANAR_PAIRS,
                                      width=w, height=h, channels=c, num_channels=count).cpu().numpy()
         assert np.array_equal(got, oracle.block_compress_color(image, 1, first, count)), (first, count)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [binding.LAYOUT_INTERLEAVED, binding.LAYOUT_PLANAR_PAIRS])
+@pytest.mark.parametrize("block_format", [1, 2, 3, 4, 5, 7])
+def test_texels_may_start_at_any_half(block_format, layout):
+    """A mip that starts at an odd half of a buffer - a view of a larger tensor - is encoded like its aligned copy: the
+    word loads of channel pairs are only taken when the mip starts on a word."""
+    import torch
+
+    generator = torch.Generator(device="cuda").manual_seed(block_format)
+    buffer = torch.rand(1 + 21 * 30 * 4, device="cuda", generator=generator).to(torch.float16)
+    aligned = buffer[1:].clone()
+    assert buffer[1:].data_ptr() % 4 == 2 and aligned.data_ptr() % 4 == 0
+    size = dict(layout=layout, width=30, height=21, channels=4)
+    for first in (0, 2) if block_format in (4, 5) else (0,):
+        got = binding.block_compress(buffer[1:], block_format, first, **size)
+        assert torch.equal(got, binding.block_compress(aligned, block_format, first, **size))
 
 
 @pytest.mark.gpu
