@@ -394,12 +394,19 @@ int ntcb_texture_set_get_texture(NtcbTextureSet* textureSet, int index, NtcbText
 int ntcb_texture_set_sample(NtcbTextureSet* textureSet, const float* deviceQueries, uint64_t numQueries, void* deviceOut,
     int useInt8Weights);
 
+/* The same for queries and a buffer that `clientStream` (a cudaStream_t) may still be writing or reading: orders the set's
+   stream after it first (ntcb_texture_set_wait_for_stream), in one call because a few queries are answered in less time than
+   a client takes for two. */
+int ntcb_texture_set_sample_after(NtcbTextureSet* textureSet, const float* deviceQueries, uint64_t numQueries, void* deviceOut,
+    int useInt8Weights, void* clientStream);
+
 /* Waits for everything queued on the texture set's stream. */
 int ntcb_texture_set_synchronize(NtcbTextureSet* textureSet);
 
 /* Orders the texture set's stream after what is queued on `stream` (a cudaStream_t) at the time of the call: work the
-   set queues from here on - blocks, pixels or answers written into a buffer of the caller's - starts when that has
-   finished.  The host does not wait. */
+   set queues from here on - blocks, pixels or answers written into a buffer of the caller's, queries read from one - starts
+   when that has finished.  The set's stream follows no other by itself, the default stream included: a caller whose device
+   buffers are still being written or read elsewhere makes this call first.  The host does not wait. */
 int ntcb_texture_set_wait_for_stream(NtcbTextureSet* textureSet, void* stream);
 
 /* One decoded mip (fp16, device memory, `layout`, `channels` channels per texel) converted into

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -177,6 +178,8 @@ def lib():
         handle.ntcb_decode.argtypes = [ctypes.POINTER(DecodeParams), ctypes.c_void_p]
         handle.ntcb_sample.argtypes = [ctypes.POINTER(SampleParams), ctypes.c_void_p]
         handle.ntcb_texture_set_sample.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_int]
+        handle.ntcb_texture_set_sample_after.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p, ctypes.c_int,
+                                                         ctypes.c_void_p]
         handle.ntcb_interleave_latents.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(MipDesc), ctypes.c_int,
                                                    ctypes.c_int, ctypes.c_void_p]
         handle.ntcb_decode_resident_ctas.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
@@ -688,6 +691,13 @@ class TextureSet:
         check(lib().ntcb_texture_set_get_desc(self.handle, ctypes.byref(self.desc)))
         self._block_shapes: dict = {}  # (texture index, mip) -> shape of its blocks in the format the header names
 
+    def _after_torch(self) -> None:
+        """Orders the set's stream after what is queued on torch's current stream of its device.  A buffer of torch's
+        that a call reads or fills may still be in use there: the set's stream follows no other by itself."""
+        torch = sys.modules.get("torch")
+        if torch is not None and torch.cuda.is_initialized():
+            check(lib().ntcb_texture_set_wait_for_stream(self.handle, torch._C._cuda_getCurrentRawStream(self.context.device)))
+
     def _blocks_shape(self, mip: int, block_format: int) -> Tuple[int, int, int]:
         width, height = self.mip_size(mip)
         return (height + 3) // 4, (width + 3) // 4, 8 if block_format in (BLOCK_FORMAT_BC1, BLOCK_FORMAT_BC4) else 16
@@ -725,6 +735,8 @@ class TextureSet:
         if dst_color_spaces is not None:
             spaces = (ctypes.c_int32 * len(dst_color_spaces))(*dst_color_spaces)
             params.dstColorSpaces = ctypes.cast(spaces, ctypes.POINTER(ctypes.c_int32))
+        if to_device:
+            self._after_torch()
         check(lib().ntcb_texture_set_read_channels(self.handle, ctypes.byref(params)))
 
     def read_mip(self, mip: int, first_channel: int = 0, num_channels: Optional[int] = None,
@@ -752,6 +764,7 @@ class TextureSet:
         stats = DecompressionStats()
         stats_ref = ctypes.byref(stats) if want_stats else None
         if device_address is not None:
+            self._after_torch()
             check(lib().ntcb_texture_set_decompress_converted(self.handle, stats_ref, 1 if use_int8 else 0,
                                                                ctypes.byref(conversion), ADDRESS_SPACE_DEVICE, device_address,
                                                                total * dtype.itemsize))
@@ -775,8 +788,7 @@ class TextureSet:
 
         shape = self._blocks_shape(mip, block_format)
         out = torch.empty(shape, dtype=torch.uint8, device="cuda")  # the encoders write every block
-        # the memory may still be in use by work queued on torch's current stream
-        check(lib().ntcb_texture_set_wait_for_stream(self.handle, torch._C._cuda_getCurrentRawStream(out.get_device())))
+        self._after_torch()
         check(lib().ntcb_texture_set_block_compress(self.handle, mip, first_channel, num_channels, block_format,
                                                     alpha_threshold, out.data_ptr(), shape[1] * shape[2]))
         self.synchronize()
@@ -835,14 +847,16 @@ class TextureSet:
         return int(pointer.value), int(size.value)
 
     def sample(self, queries, use_int8: bool):
-        """ntcb_texture_set_sample: `queries` is a float32 CUDA tensor [n][3] of (u, v, lod) on the set's device;
+        """ntcb_texture_set_sample_after: `queries` is a float32 CUDA tensor [n][3] of (u, v, lod) on the set's device;
         returns a float16 CUDA tensor [n][channels] with the bits a decompress would write to the selected texels.
         The call waits for the answers."""
         import torch
 
         queries = queries.contiguous()
         out = torch.empty((queries.shape[0], self.desc.channels), dtype=torch.float16, device=queries.device)
-        check(lib().ntcb_texture_set_sample(self.handle, queries.data_ptr(), queries.shape[0], out.data_ptr(), 1 if use_int8 else 0))
+        # after torch's current stream (_after_torch), which may just be computing the queries, or copying them for contiguous()
+        check(lib().ntcb_texture_set_sample_after(self.handle, queries.data_ptr(), queries.shape[0], out.data_ptr(), 1 if use_int8 else 0,
+                                                  torch._C._cuda_getCurrentRawStream(self.context.device)))
         return out
 
     def synchronize(self) -> None:

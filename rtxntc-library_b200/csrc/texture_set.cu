@@ -1717,6 +1717,20 @@ int ntcb_texture_set_sample(NtcbTextureSet* textureSet, const float* deviceQueri
     return ntcb::Guarded(__func__, [&]() { return textureSet->impl->Sample(deviceQueries, numQueries, deviceOut, useInt8Weights != 0); });
 }
 
+int ntcb_texture_set_sample_after(NtcbTextureSet* textureSet, const float* deviceQueries, uint64_t numQueries, void* deviceOut,
+    int useInt8Weights, void* clientStream)
+{
+    if (!textureSet)
+    {
+        ntcb::SetError("textureSet is NULL.");
+        return NTCB_ERR_INVALID_ARGUMENT;
+    }
+    return ntcb::Guarded(__func__, [&]() {
+        const int status = textureSet->impl->WaitForStream(clientStream);
+        return status == NTCB_OK ? textureSet->impl->Sample(deviceQueries, numQueries, deviceOut, useInt8Weights != 0) : status;
+    });
+}
+
 int ntcb_texture_set_synchronize(NtcbTextureSet* textureSet)
 {
     if (!textureSet)

@@ -359,6 +359,60 @@ def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, 
         texture_set.close()
 
 
+@pytest.mark.parametrize("call", ["sample", "answers", "converted", "read_channels", "block_compress", "block_compress_texture"])
+def test_texture_set_calls_follow_torchs_stream(call):
+    """Queries still being computed, and memory that queued work still uses, on torch's current stream: the set's calls, which run
+    on a stream of the set's own, come after that work."""
+    import torch
+
+    width, height = 128, 96
+    textures = [{"name": "Mask", "firstChannel": 1, "numChannels": 1, "bcFormat": "BC4"}]
+    data = synthetic.make_texture_set(synthetic.TextureSetSpec(width, height, 4, 1, 2, 8, seed=9, network="unit"))
+    data = synthetic.SyntheticSet(data.spec, data.geometry, data.latents, data.int8_blob, data.fp8_blob, textures=textures)
+    queries = torch.rand((5000, 3), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    conversion = binding.make_conversion(binding.CHANNEL_FORMAT_UNORM8, 4)
+    pixels = torch.zeros(width * height * 4, dtype=torch.uint8, device="cuda")
+    texels = torch.zeros(width * height * 4, dtype=torch.float16, device="cuda")
+    late = torch.zeros_like(queries)
+
+    def run(texture_set, asked):
+        if call in ("sample", "answers"):
+            return texture_set.sample(asked, True)
+        if call == "converted":
+            texture_set.decompress_converted(conversion, True, device_address=pixels.data_ptr())
+            return pixels
+        if call == "read_channels":
+            texture_set.read_channels_into(0, texels.data_ptr(), True)
+            return texels
+        if call == "block_compress":
+            return texture_set.block_compress(0, binding.BLOCK_FORMAT_BC5, 0)
+        return texture_set.block_compress_texture(0, 0)
+
+    with binding.Context(0) as context:
+        texture_set = context.create_texture_set(data.container)
+        texture_set.decompress(True)
+        texture_set.synchronize()
+        expected = run(texture_set, queries).clone()
+        _sync()
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            reused = torch.empty_like(expected)
+            torch.cuda._sleep(20_000_000)  # 10 ms
+            if call == "sample":
+                late.copy_(queries)
+            elif call == "converted":
+                pixels.fill_(7)
+            elif call == "read_channels":
+                texels.fill_(7)
+            else:
+                reused.fill_(7)
+                del reused  # the allocator hands its memory to the answers
+            got = run(texture_set, late if call == "sample" else queries)
+        _sync()
+        assert torch.equal(got, expected)
+        texture_set.close()
+
+
 @BOTH_NUMERICS
 def test_kernels_queued_back_to_back_overlap_without_a_trace(numerics):
     """A decode or sample kernel starts while the one before it in the stream still runs and waits for its end: launches
