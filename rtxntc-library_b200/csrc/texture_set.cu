@@ -732,6 +732,18 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
     const int firstRows = rowRanges ? 0 : FirstBandRows(forHost ? conversion
         ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat) : size_t(m_geometry.channels) * sizeof(__half) : 0);
     const bool streamed = firstRows > 0 && m_latentBytes >= kStreamedUploadBytes && LatentRows(firstRows) < m_geometry.latentHeight[0] - 1;
+    // Work queued later - another upload, sampling, a refill of the pinned image - relies on m_stream for the end of this upload.
+    // Until m_stream waits for its last part, a return with an error has to wait here.
+    struct UploadInFlight
+    {
+        cudaStream_t stream;
+        ~UploadInFlight()
+        {
+            if (stream)
+                cudaStreamSynchronize(stream);
+        }
+    } inFlight{streamed ? m_uploadStream : nullptr};
+    m_deviceCurrent = false;
     cudaError_t err = streamed ? UploadFirst(firstRows)
                                : cudaMemcpyAsync(m_deviceUpload, m_hostUpload, m_uploadBytes, cudaMemcpyHostToDevice, m_stream);
     if (err != cudaSuccess)
@@ -800,6 +812,7 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
                 err = cudaStreamWaitEvent(m_stream, m_eventUploaded, 0);
                 if (err != cudaSuccess)
                     return CudaFailure("cudaStreamWaitEvent (compressed data)", err);
+                inFlight.stream = nullptr;
             }
             status = ntcb_decode(b == 0 ? &first : &params, m_stream);
             if (status == NTCB_OK && forHost && cudaEventRecord(m_bandEvents[b], m_stream) != cudaSuccess)

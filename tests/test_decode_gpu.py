@@ -359,6 +359,32 @@ def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, 
         texture_set.close()
 
 
+def test_a_refused_decompress_leaves_no_upload_behind():
+    """A set of 2^32 texel values can be sampled but not decompressed; the call is refused when the streamed upload has already
+    begun.  What follows - sampling, loading another set - finds the whole upload, of the right set."""
+    import torch
+
+    first, second, third = (synthetic.make_texture_set(synthetic.TextureSetSpec(16384, 16384, 16, 1, 6, 4, seed=seed, network="unit"))
+                            for seed in (3, 4, 5))
+    assert first.geometry.encoded_latent_bytes >= 4 << 20
+    queries = torch.rand((200000, 3), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    expected = [binding.ResidentTextureSet.from_synthetic(data, allocate_output=False).sample(queries, True) for data in (first, second, third)]
+    _sync()
+    with binding.Context(0) as context:
+        texture_set = context.create_texture_set(first.container)
+        assert torch.equal(texture_set.sample(queries, True), expected[0])
+        texture_set.load_from_memory(second.container)
+        with pytest.raises(binding.NtcbError) as refused:
+            texture_set.decompress(True)
+        assert refused.value.code == -9
+        assert torch.equal(texture_set.sample(queries, True), expected[1])
+        with pytest.raises(binding.NtcbError):
+            texture_set.decompress(True)
+        texture_set.load_from_memory(third.container)
+        assert torch.equal(texture_set.sample(queries, True), expected[2])
+        texture_set.close()
+
+
 @pytest.mark.parametrize("call", ["sample", "answers", "converted", "read_channels", "block_compress", "block_compress_texture"])
 def test_texture_set_calls_follow_torchs_stream(call):
     """Queries still being computed, and memory that queued work still uses, on torch's current stream: the set's calls, which run
