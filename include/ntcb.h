@@ -270,7 +270,8 @@ typedef struct NtcbTextureSetFeatures
    reference image, which a decoder-only texture set never has, so only the timing is kept. */
 typedef struct NtcbDecompressionStats
 {
-    float gpuTimeMilliseconds; /* device time of the decode launch, as the reference times its mip loop */
+    float gpuTimeMilliseconds; /* device time of the decode launches, as the reference times its mip loop (a call that asks for
+                                  it uploads first and decodes then, also where they would otherwise overlap) */
 } NtcbDecompressionStats;
 
 #define NTCB_ADDRESS_SPACE_HOST 0   /* ntc::AddressSpace::Host */

@@ -149,7 +149,7 @@ private:
     static constexpr int kBandMinRows = 512;
     // An upload of this size (73 us) is worth the second launch even when the texels stay on the device.
     static constexpr size_t kStreamedUploadBytes = size_t(4) << 20;
-    int FirstBandRows(size_t hostTexelBytes) const;
+    int FirstBandRows(size_t hostTexelBytes, bool streamed) const;
     int LatentRows(int firstRows) const;
     cudaError_t UploadFirst(int firstRows);
     cudaStream_t m_uploadStream = nullptr;
@@ -655,14 +655,14 @@ Status TextureSet::GrowStaging(size_t bytes)
 // the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips apart took five launches, each with a ramp at both
 // ends: 326 us for a 2048 x 2048 set that decodes in 250.)
 //
-// For a streamed upload: decoding the first band should take as long as the rest of the upload does.
-int TextureSet::FirstBandRows(size_t hostTexelBytes) const
+// `streamed`, an upload beside the decode: decoding the first band should take as long as the rest of the upload does.
+int TextureSet::FirstBandRows(size_t hostTexelBytes, bool streamed) const
 {
     const int height = m_geometry.mipHeight[0];
     if (height < kBandMinRows)
         return 0;
     float share = hostTexelBytes ? 1.f / (1.f + 0.35f * float(hostTexelBytes)) : 0.f;
-    if (m_latentBytes >= kStreamedUploadBytes)
+    if (streamed)
     {
         const float latentBytes = float(m_geometry.latentPixelOffset[1]) * float(m_geometry.numLayers) * 2.f;
         const float upload = latentBytes / 57.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 20.f; // nanoseconds
@@ -728,10 +728,11 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
 
     // Upload the encoded latents and the network weights, as the reference does on every
     // Decompress of a loaded set (src/TextureSet.cpp:1691-1757).  A large upload runs beside the decode: the first rows of mip 0
-    // start when what they read has arrived.
+    // start when what they read has arrived.  (Not when the device time is asked for: it would include waiting for the host link.)
+    const bool mayStream = !pOutStats && m_latentBytes >= kStreamedUploadBytes;
     const int firstRows = rowRanges ? 0 : FirstBandRows(forHost ? conversion
-        ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat) : size_t(m_geometry.channels) * sizeof(__half) : 0);
-    const bool streamed = firstRows > 0 && m_latentBytes >= kStreamedUploadBytes && LatentRows(firstRows) < m_geometry.latentHeight[0] - 1;
+        ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat) : size_t(m_geometry.channels) * sizeof(__half) : 0, mayStream);
+    const bool streamed = firstRows > 0 && mayStream && LatentRows(firstRows) < m_geometry.latentHeight[0] - 1;
     // Work queued later - another upload, sampling, a refill of the pinned image - relies on m_stream for the end of this upload.
     // Until m_stream waits for its last part, a return with an error has to wait here.
     struct UploadInFlight
