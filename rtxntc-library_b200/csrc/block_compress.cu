@@ -1321,7 +1321,6 @@ extern "C" int ntcb_block_compress(const NtcbBlockCompressParams* params, void* 
     const cudaStream_t cudaStream = static_cast<cudaStream_t>(stream);
     if (format == NTCB_BLOCK_FORMAT_BC7)
         return LaunchBlockCompressBc7(*params, args, cudaStream);
-    const dim3 grid(unsigned(params->widthInBlocks + 15) / 16, unsigned(params->heightInBlocks + 3) / 4);
     cudaError_t error = cudaSuccess;
     if (!color)
         error = LaunchBc4(args, formatChannels, cudaStream);
@@ -1331,26 +1330,27 @@ extern "C" int ntcb_block_compress(const NtcbBlockCompressParams* params, void* 
         if (status != NTCB_OK)
             return status;
         ColorCompressArguments colorArgs;
-        colorArgs.base = args;
         colorArgs.numChannels = formatChannels;
         colorArgs.alphaThreshold = params->alphaThreshold;
-        if (format == NTCB_BLOCK_FORMAT_BC1)
-            ColorBlockCompressKernel<NTCB_BLOCK_FORMAT_BC1><<<grid, kColorThreads, 0, cudaStream>>>(colorArgs);
-        else if (format == NTCB_BLOCK_FORMAT_BC2)
-            ColorBlockCompressKernel<NTCB_BLOCK_FORMAT_BC2><<<grid, kColorThreads, 0, cudaStream>>>(colorArgs);
-        else
+        ForEachGrid(args, 16, 4, [&](const BlockCompressArguments& part, int, dim3 grid) {
+            colorArgs.base = part;
+            if (format == NTCB_BLOCK_FORMAT_BC1)
+                ColorBlockCompressKernel<NTCB_BLOCK_FORMAT_BC1><<<grid, kColorThreads, 0, cudaStream>>>(colorArgs);
+            else if (format == NTCB_BLOCK_FORMAT_BC2)
+                ColorBlockCompressKernel<NTCB_BLOCK_FORMAT_BC2><<<grid, kColorThreads, 0, cudaStream>>>(colorArgs);
+            else
+                ColorBlockCompressKernel<NTCB_BLOCK_FORMAT_BC3><<<grid, kColorThreads, 0, cudaStream>>>(colorArgs);
+            CountLaunch();
+        });
+        if (format == NTCB_BLOCK_FORMAT_BC3)
         {
             // colour halves by the colour kernel, alpha halves by the BC4 kernel: two lean kernels instead
             // of one with both encoders inlined (158 registers; 1.56 ms against 1.1 ms on a 4096^2 mip)
-            ColorBlockCompressKernel<NTCB_BLOCK_FORMAT_BC3><<<grid, kColorThreads, 0, cudaStream>>>(colorArgs);
-            CountLaunch();
             BlockCompressArguments alphaArgs = args;
             alphaArgs.firstChannel = formatChannels == 4 ? args.firstChannel + 3 : -1;
             alphaArgs.formatChannels = 2; // 16-byte blocks, the alpha block first
             error = LaunchBc4(alphaArgs, 1, cudaStream);
         }
-        if (format != NTCB_BLOCK_FORMAT_BC3)
-            CountLaunch();
     }
     if (error == cudaSuccess)
         error = cudaGetLastError();

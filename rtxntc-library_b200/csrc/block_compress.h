@@ -64,6 +64,22 @@ __device__ __forceinline__ uint64_t JoinIndices(uint64_t x)
     return (x & kWord) | ((x >> (8 * kGap)) & (kWord << (8 * kBits)));
 }
 
+// Calls launch(part, first row of blocks, grid) for the block rectangle in rows of as many CTAs of `width` x `height` blocks as a grid may have
+// (an image of a million and more texel rows takes several launches).
+template <typename Launch>
+inline void ForEachGrid(const BlockCompressArguments& args, int width, int height, Launch&& launch)
+{
+    for (int top = 0, rows = 0; top < args.heightInBlocks; top += rows)
+    {
+        rows = args.heightInBlocks - top < 65535 * height ? args.heightInBlocks - top : 65535 * height;
+        BlockCompressArguments part = args;
+        part.srcTop = args.srcTop + 4 * top;
+        part.heightInBlocks = rows;
+        part.blocks = args.blocks + size_t(top) * args.rowPitch;
+        launch(part, top, dim3(unsigned(part.widthInBlocks + width - 1) / width, unsigned(part.heightInBlocks + height - 1) / height));
+    }
+}
+
 // The BC7 half of ntcb_block_compress (block_compress_bc7.cu); `params` has passed the checks common to all formats.
 int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCompressArguments& args, cudaStream_t stream);
 

@@ -1865,12 +1865,15 @@ int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCom
     args.groupWidthLog2 = blocks >= 256ll * sms ? 5 : 4;
     args.groupHeight = blocks >= 128ll * sms ? 8 : 4;
     const int groupWidth = search ? kSearchWidth : 1 << args.groupWidthLog2, groupHeight = search ? kSearchHeight : args.groupHeight;
-    const dim3 grid(unsigned(base.widthInBlocks + groupWidth - 1) / groupWidth, unsigned(base.heightInBlocks + groupHeight - 1) / groupHeight);
-    if (search)
-        Bc7SearchKernel<<<grid, kSearchThreads, 0, stream>>>(args);
-    else
-        Bc7ModeKernel<<<grid, kThreads, 0, stream>>>(args);
-    CountLaunch();
+    ForEachGrid(base, groupWidth, groupHeight, [&](const BlockCompressArguments& part, int top, dim3 grid) {
+        args.base = part;
+        args.modeMapOffsetY = params.modeMapOffsetY + top;
+        if (search)
+            Bc7SearchKernel<<<grid, kSearchThreads, 0, stream>>>(args);
+        else
+            Bc7ModeKernel<<<grid, kThreads, 0, stream>>>(args);
+        CountLaunch();
+    });
     error = cudaGetLastError();
     if (error != cudaSuccess)
         return CudaFailure("Bc7 kernel", error);

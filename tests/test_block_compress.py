@@ -565,6 +565,30 @@ def test_texels_may_start_at_any_half(block_format, layout):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("block_format", [1, 2, 3, 4, 5, 7, -7])
+def test_images_of_more_rows_than_a_grid_has(block_format):
+    """Two million texel rows and some: the encoders' grids (65535 rows of 4 or 8 blocks) take several launches.  The rows repeat,
+    so every block of the column is one of 64 known ones; -7: BC7 with a mode buffer."""
+    import torch
+
+    period, blocks = 64, 8 * 65535 + 77
+    generator = torch.Generator(device="cuda").manual_seed(abs(block_format))
+    tile = torch.rand((4 * period, 4, 4), device="cuda", generator=generator).to(torch.float16)
+    image = tile.repeat((blocks + period - 1) // period, 1, 1)[:4 * blocks - 1].contiguous()
+    expected = binding.block_compress(tile, abs(block_format))
+    options = {}
+    if block_format < 0:
+        column = expected.repeat((blocks + period - 1) // period, 1, 1)[:blocks]
+        options["mode_buffer"] = torch.from_numpy(binding.make_bc7_mode_buffer(column.cpu().numpy())).cuda()
+        single = torch.from_numpy(binding.make_bc7_mode_buffer(expected.cpu().numpy())).cuda()
+        expected = binding.block_compress(tile, 7, mode_buffer=single)
+    got = binding.block_compress(image, abs(block_format), **options)
+    assert got.shape[0] == blocks
+    order = torch.arange(blocks - 1, device="cuda") % period  # (the last block is cut off)
+    assert torch.equal(got[:-1], expected[order])
+
+
+@pytest.mark.gpu
 def test_kernel_on_ragged_images_windows_and_the_planar_layout(oracle):
     import torch
 
