@@ -570,13 +570,23 @@ static void mlp_ref(const Network* net, const NtcoOptions* opt, const h16 in[MLP
 /* Drivers                                                                                      */
 /* ------------------------------------------------------------------------------------------ */
 
-static int setup_mip(const NtcoTextureSet* set, const NtcoGeometry* geo, int mip, MipContext* mc)
+/* 1 / extent, moved by `ulps` units in the last place. */
+static float reciprocal(int extent, int ulps)
 {
+    float r = 1.0f / (float)extent;
+    for (; ulps > 0; --ulps) r = nextafterf(r, INFINITY);
+    for (; ulps < 0; ++ulps) r = nextafterf(r, 0.0f);
+    return r;
+}
+
+static int setup_mip(const NtcoTextureSet* set, const NtcoGeometry* geo, const NtcoOptions* opt, int mip, MipContext* mc)
+{
+    const int ref = opt->numerics == NTCO_NUMERICS_REF;
     int lod = geo->neuralLod[mip];
     mc->width = geo->mipWidth[mip];
     mc->height = geo->mipHeight[mip];
-    mc->invWidth = 1.0f / (float)mc->width;
-    mc->invHeight = 1.0f / (float)mc->height;
+    mc->invWidth = reciprocal(mc->width, ref ? opt->refReciprocalUlpsX : 0);
+    mc->invHeight = reciprocal(mc->height, ref ? opt->refReciprocalUlpsY : 0);
     mc->hiW = geo->latentWidth[lod];
     mc->hiH = geo->latentHeight[lod];
     /* src/TextureSet.cpp:1816-1817 */
@@ -674,7 +684,7 @@ int ntco_decode_mip(const NtcoTextureSet* set, const NtcoOptions* opt, int mip, 
     if (!opt || !out || ntco_geometry(set, &geo) != 0 || mip < 0 || mip >= set->numMips)
         return -1;
     MipContext mc;
-    if (setup_mip(set, &geo, mip, &mc) != 0 || y0 < 0 || y1 > mc.height || y0 > y1)
+    if (setup_mip(set, &geo, opt, mip, &mc) != 0 || y0 < 0 || y1 > mc.height || y0 > y1)
         return -1;
     init_tables();
     Network* net = (Network*)malloc(sizeof(Network));
@@ -715,7 +725,7 @@ int ntco_sample(const NtcoTextureSet* set, const NtcoOptions* opt, const float* 
         return -1;
     MipContext mips[NTCO_MAX_MIPS];
     for (int m = 0; m < set->numMips; ++m)
-        if (setup_mip(set, &geo, m, &mips[m]) != 0)
+        if (setup_mip(set, &geo, opt, m, &mips[m]) != 0)
             return -1;
     init_tables();
     Network* net = (Network*)malloc(sizeof(Network));

@@ -86,6 +86,10 @@ typedef struct NtcoOptions
                           >= 16: addends aligned to the largest exponent and truncated below
                           2^(emax - refAccMode), summed exactly, then one rounding */
     int refActFma;     /* reserved */
+    /* The reference normalises texel coordinates with CUDA's approximate division, whose result may lie off the product with the
+       correctly rounded reciprocal of the mip's size: units in the last place that the reciprocals of its width and
+       height are moved by. */
+    int refReciprocalUlpsX, refReciprocalUlpsY;
 } NtcoOptions;
 
 /* Geometry of a texture set: neural mip sizes, colour-mip -> neural-LOD map, positional encoding

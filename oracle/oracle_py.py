@@ -38,7 +38,8 @@ class Geometry(ctypes.Structure):
 class Options(ctypes.Structure):
     _fields_ = [("weights", ctypes.c_int), ("numerics", ctypes.c_int), ("threads", ctypes.c_int),
                 ("refBlendFma", ctypes.c_int), ("refQuantFma", ctypes.c_int), ("refAccChunk", ctypes.c_int),
-                ("refAccMode", ctypes.c_int), ("refActFma", ctypes.c_int)]
+                ("refAccMode", ctypes.c_int), ("refActFma", ctypes.c_int),
+                ("refReciprocalUlpsX", ctypes.c_int), ("refReciprocalUlpsY", ctypes.c_int)]
 
 
 WEIGHTS_INT8, WEIGHTS_FP8 = 0, 1
@@ -241,14 +242,16 @@ class OracleSet:
 
 # Switches of the reference-emulating numerics that reproduce the reference kernel's outputs
 # (see tests/golden/README.md for how they were pinned).
-REF_DEFAULTS = dict(refBlendFma=2, refQuantFma=1, refAccChunk=16, refAccMode=25, refActFma=0)
+REF_DEFAULTS = dict(refBlendFma=2, refQuantFma=1, refAccChunk=16, refAccMode=25, refActFma=0, refReciprocalUlpsX=0,
+                    refReciprocalUlpsY=0)
 
 
 def make_options(use_int8: bool, numerics: int, threads: int = 0, **ref_switches) -> Options:
     switches = dict(REF_DEFAULTS)
     switches.update(ref_switches)
     return Options(WEIGHTS_INT8 if use_int8 else WEIGHTS_FP8, numerics, threads, switches["refBlendFma"],
-                   switches["refQuantFma"], switches["refAccChunk"], switches["refAccMode"], switches["refActFma"])
+                   switches["refQuantFma"], switches["refAccChunk"], switches["refAccMode"], switches["refActFma"], switches["refReciprocalUlpsX"],
+                   switches["refReciprocalUlpsY"])
 
 
 # ---------------------------------------------------------------------------------------------

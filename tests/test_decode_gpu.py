@@ -55,11 +55,28 @@ def _assert_matches_contract(decoded, expected, use_int8, what):
     assert different <= allowed, "%s: %d of %d values differ from the CPU restatement" % (what, different, decoded.size)
 
 
-def _restated(oracle, checker, mip, use_int8, numerics):
-    """The CPU restatement of the kernel that implements `numerics`."""
+def _restated(oracle, checker, mip, use_int8, numerics, decoded):
+    """The CPU restatement of the kernel that implements `numerics`, of `decoded`.
+
+    The reference's numerics divide texel coordinates by the mip's size with div.approx.ftz.f32, which the restatement
+    can only bound: its documented error is 2 ulp, that of the reciprocal approximation (rcp.approx.ftz.f32) 1 ulp.  So where
+    the product with the correctly rounded reciprocal does not explain the kernel's texels, the two neighbours of either
+    reciprocal may: ONE choice has to fit the whole mip, at the same budget.  (Sizes that are powers of two have exact
+    reciprocals and no choice.)"""
     if numerics == EXACT:
         return checker.decode_mip(mip, use_int8, oracle.NUMERICS_SPEC)
-    return checker.decode_mip(mip, use_int8, oracle.NUMERICS_REF, **oracle.REF_DEFAULTS)
+    cm = checker.geometry.color_mips[mip]
+    choices = [(0,) if size & (size - 1) == 0 else (0, -1, 1) for size in (cm.width, cm.height)]
+    closest, fewest = None, None
+    for x in choices[0]:
+        for y in choices[1]:
+            expected = checker.decode_mip(mip, use_int8, oracle.NUMERICS_REF, refReciprocalUlpsX=x, refReciprocalUlpsY=y)
+            different = int((decoded.view(np.uint16) != expected.view(np.uint16)).sum())
+            if closest is None or different < fewest:
+                closest, fewest = expected, different
+            if fewest <= decoded.size * 2e-4:
+                return closest
+    return closest
 
 
 class _Tally:
@@ -162,8 +179,8 @@ def test_kernel_matches_contract_on_ragged_shapes(oracle, shape, network, numeri
                 assert np.array_equal(resident.mip_numpy(mip).reshape(-1).view(np.uint16), theirs.view(np.uint16)), \
                     "%s mip %d differs from the live reference" % (shape, mip)
             else:
-                tally.add(resident.mip_numpy(mip), _restated(oracle, checker, mip, use_int8, numerics), use_int8,
-                          "%s mip %d" % (shape, mip))
+                decoded = resident.mip_numpy(mip)
+                tally.add(decoded, _restated(oracle, checker, mip, use_int8, numerics, decoded), use_int8, "%s mip %d" % (shape, mip))
     tally.check()
 
 
