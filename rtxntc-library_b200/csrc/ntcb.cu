@@ -57,27 +57,27 @@ constexpr int kWeightOffsets[4] = {kWeightOffset0, kWeightOffset1, kWeightOffset
 constexpr int kRefWeightOffsets[4] = {kRefWeightOffset0, kRefWeightOffset1, kRefWeightOffset2, kRefWeightOffset3};
 constexpr int kRefBiasOffsets[4] = {kRefBiasOffset0, kRefBiasOffset1, kRefBiasOffset2, kRefBiasOffset3};
 
-// binary32 -> binary16, round to nearest even (after the branch-free form of F. Giesen's float_to_half_fast3_rtne, public
-// domain, 2016): no branches, so that the compiler converts several weights at once - the library conversion took two thirds of the
-// time of staging a network.  NaN becomes 0x7fff.
+// binary32 -> binary16, round to nearest even, NaN -> 0x7fff, without branches, so that the compiler converts several weights
+// at once (the library conversion took two thirds of the time of staging a network).
+//
+// binary16 numbers are the multiples of 2^(E - 10), where E is the exponent of the value or -14, whichever is larger.  A
+// binary32 sum with 2^(E + 13) has exactly that spacing, so adding it rounds the magnitude to such a multiple, and the low bits of the sum
+// count the multiples.  There are 1024 of them to a binade, so the binades below (E + 14) and the count add up to the code; a
+// count of 2048 carries into the next binade, up to infinity after the last.
 inline uint16_t HalfBits(float value)
 {
-    uint32_t bits;
-    memcpy(&bits, &value, 4);
-    const uint32_t sign = (bits >> 16) & 0x8000u;
-    bits &= 0x7fffffffu;
-    // below the smallest normal: adding 0.5 leaves the rounded subnormal in the low bits
-    float magnitude;
-    memcpy(&magnitude, &bits, 4);
-    magnitude += 0.5f;
-    uint32_t subnormal;
-    memcpy(&subnormal, &magnitude, 4);
-    subnormal -= 0x3f000000u;
-    const uint32_t normal = (bits - 0x38000000u + 0xfffu + ((bits >> 13) & 1u)) >> 13;
-    uint32_t half = bits < 0x38800000u ? subnormal : normal;
-    half = bits >= 0x47800000u ? 0x7c00u : half;
-    half = bits > 0x7f800000u ? 0x7fffu : half;
-    return uint16_t(half | (bits > 0x7f800000u ? 0u : sign));
+    auto bitsOf = [](float v) { uint32_t bits; memcpy(&bits, &v, 4); return bits; };
+    auto floatOf = [](uint32_t bits) { float v; memcpy(&v, &bits, 4); return v; };
+    const uint32_t sign = (bitsOf(value) >> 16) & 0x8000u, magnitude = bitsOf(value) & 0x7fffffffu;
+    constexpr float kLowest = 1.f / 16384.f, kHighest = 32768.f; // first and last binade of normal numbers
+    float binade = floatOf(magnitude & 0x7f800000u); // 2^exponent
+    binade = binade > kLowest ? binade : kLowest;
+    binade = binade < kHighest ? binade : kHighest;
+    const float spacing = binade * 8192.f, sum = floatOf(magnitude) + spacing;
+    uint32_t half = (bitsOf(binade) >> 13) - (113u << 10) + bitsOf(sum) - bitsOf(spacing); // (113: the biased exponent of kLowest)
+    half = magnitude >= 0x47800000u ? 0x7c00u : half; // 2^16 and more
+    half |= sign;
+    return uint16_t(magnitude > 0x7f800000u ? 0x7fffu : half);
 }
 
 // `pairedOutput`: the launch stores fp16 channel pairs as 32-bit words, so a mip must start on one.

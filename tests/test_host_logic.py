@@ -292,6 +292,44 @@ def test_reference_network_staging():
                 assert not step_operand[0, :, 1:].any() and not step_operand[1].any()
 
 
+def test_staged_weights_are_rounded_to_the_nearest_half():
+    """The Int8 weights and first-layer biases as the reference-numerics kernels read them: products in binary32, rounded to
+    binary16 as numpy rounds them (to nearest, ties to even), over the format's whole range and beyond it: subnormal, tiny, huge,
+    infinite and NaN (0x7fff) scales, ties, both signs."""
+    rng = np.random.default_rng(11)
+    inputs, outputs = geometry.MLP_LAYER_INPUTS, geometry.MLP_LAYER_OUTPUTS
+    offsets = (0, 6144, 12288, 15360)
+    seen = set()
+    for draw in range(24):
+        weights = rng.integers(-128, 128, size=8192).astype(np.int8)
+        scales = (2.0 ** rng.uniform(-36, 14, 160) * rng.choice([-1, 1], 160)).astype(np.float32)
+        if draw % 3 == 0:  # few significant bits: products halfway between two halves
+            scales = (scales.view(np.uint32) & np.uint32(0xFFFC0000)).view(np.float32)
+        scales[:4] = (np.inf, np.nan, 0.0, -0.0)
+        biases = rng.integers(-2 ** 20, 2 ** 20, size=160).astype(np.int32)
+        staged = binding.stage_network(weights.tobytes() + scales.tobytes() + biases.tobytes(), binding.WEIGHTS_INT8, binding.NUMERICS_REFERENCE)
+        halves = staged.view(np.uint16)
+        start = column = 0
+        with np.errstate(all="ignore"):
+            for layer in range(4):
+                nin, nout = inputs[layer], outputs[layer]
+                factor = np.float32(127.5) if layer == 0 else np.float32(1) / (np.float32(3.1875) / np.float32(255))
+                layer_scales = scales[column:column + nout] * factor
+                products = weights[start:start + nin * nout].reshape(nout, nin).astype(np.float32) * layer_scales[:, None]
+                # chunks of eight inputs: half (n, k) at (k / 8) * 8 * nout + 8 n + k % 8
+                got = halves[offsets[layer] // 2:offsets[layer] // 2 + nin * nout].reshape(nin // 8, nout, 8).transpose(1, 0, 2).reshape(nout, nin)
+                expected = np.where(np.isnan(products), np.uint16(0x7FFF), products.astype(np.float16).view(np.uint16))
+                assert np.array_equal(got, expected), (draw, layer)
+                seen.update(np.unique(expected >> 10))
+                if layer == 0:
+                    bias = biases[:nout].astype(np.float32) * scales[:nout]
+                    expected = np.where(np.isnan(bias), np.uint16(0x7FFF), bias.astype(np.float16).view(np.uint16))
+                    assert np.array_equal(halves[8192:8192 + 8 * nout:8], expected)
+                start += nin * nout
+                column += nout
+    assert len(seen) == 64  # every sign and exponent
+
+
 def test_stage_network_rejects_wrong_sizes():
     for numerics in (binding.NUMERICS_REFERENCE, binding.NUMERICS_EXACT):
         with pytest.raises(binding.NtcbError) as error:
