@@ -36,9 +36,8 @@
 //
 // Two kernels live here.  DecodeKernelRef (first part of the file) keeps every operand in binary16
 // and serves Int8 networks.  DecodeKernelRefFp8 (second part) serves FP8 networks with 8-bit operands
-// for layers 0-2 (those of layers 1-3 in tensor memory) and produces the same bits; since ntcb_stage_network_reference lays an FP8
-// network out for it, the binary16 kernel's templates are only instantiated with kFp8 = false
-// (their kFp8 = true paths describe what the FP8 kernel replaces: e4m3 round trips in binary16).
+// for layers 0-2 (those of layers 1-3 in tensor memory) and produces the same bits;
+// ntcb_stage_network_reference lays an FP8 network out for it.
 
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -55,34 +54,18 @@
 #include "output_convert.cuh"
 #include "epilogue_convert.cuh"
 
-// Profiling aid: NTCB_ABLATE (a bit mask, 0 in the product build; 512: no tile walk, every tile at the place of the chain's
-// first; 1024: no barrier before a layer's products - only together with 16) removes one phase of
-// DecodeKernelRefFp8 at a time so that its share of the kernel's instructions and time can be
-// measured as a difference (`make ablations` builds one library per mask; their output is wrong by
-// construction).  1: the per-tile tables and footprint staging after the first tile; 2: the latent
-// gather and blend (constants are stored instead); 64: the tap tables are rebuilt for every tile; 4: the activation arithmetic of layers 0-2 (the
-// raw accumulator words are stored); 8: the global stores of the epilogue; 16: the tensor-core work
-// (no MMA issue, no wait for it); 32: the tensor-memory loads; 128: the proxy fence before each layer's
-// barrier.
-#ifndef NTCB_ABLATE
-#define NTCB_ABLATE 0
-#endif
-
 namespace ntcb
 {
 namespace
 {
 
-constexpr int kAblate = NTCB_ABLATE;
 // FP8 networks: the A operand of layers 1-3 lives in tensor memory, not in shared memory.  A layer's 64-byte
 // input row is 16 of the 32-bit columns of its thread's own TMEM lane; layers 1-3 have at most 48 outputs,
 // so their accumulators leave columns 48..63 of the chain's 64 free for it.  (Layer 0 has 64 outputs: its
 // operand, the gathered inputs, stays in shared memory.)  The activations are stored with tcgen05.st, the
 // products read them with the A-in-tensor-memory form of tcgen05.mma: no shared-memory stores, no proxy
 // fence, and no operand reads from shared memory by the tensor core for three of the four layers (3 %).
-constexpr bool kTmemOperand = true;
 constexpr uint32_t kOperandColumn = 48;
-
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 16 binary16 operands, binary16 accumulators.
 __device__ __forceinline__ void UmmaF16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
@@ -134,20 +117,10 @@ __device__ __forceinline__ void TmemLoadPacked8(uint32_t address, uint32_t (&r)[
 // Quantisers (value in, de-quantised value out)
 // ---------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ __half2 RoundTripE4m3(__half2 x)
-{
-    // src/tin/tin_activation.h:44-48: round to nearest even e4m3, saturating, and back to binary16
-    const __nv_fp8x2_storage_t codes = __nv_cvt_halfraw2_to_fp8x2(static_cast<__half2_raw>(x), __NV_SATFINITE, __NV_E4M3);
-    return __half2(__nv_cvt_fp8x2_to_halfraw2(codes, __NV_E4M3));
-}
-
-// A pair of network inputs as the first layer sees them.  Int8: floor(x * 127.5 - 0.5) clamped to
-// +-127, times 1 / 127.5 (src/tin/tin_mlp.h:22-37).  FP8: rounded to e4m3.
-template <bool kFp8>
+// A pair of network inputs as the first layer of an Int8 network sees them: floor(x * 127.5 - 0.5) clamped to
+// +-127, times 1 / 127.5 (src/tin/tin_mlp.h:22-37).
 __device__ __forceinline__ __half2 QuantizeInputRef(__half2 x)
 {
-    if (kFp8)
-        return RoundTripE4m3(x);
     __half2 y = __hfma2(x, __float2half2_rn(127.5f), __float2half2_rn(-0.5f));
     y = h2floor(y);
     y = __hmax2(__hmin2(y, __float2half2_rn(127.f)), __float2half2_rn(-127.f));
@@ -155,8 +128,7 @@ __device__ __forceinline__ __half2 QuantizeInputRef(__half2 x)
 }
 
 // Clamped HGELU in binary16 (src/tin/tin_activation.h:88-92) followed by the quantiser of the next
-// layer's inputs: e4m3, or the int8 grid rint(y * 80) * 0.0125 (src/tin/tin_activation.h:94-99).
-template <bool kToFp8>
+// layer's inputs, the int8 grid rint(y * 80) * 0.0125 (src/tin/tin_activation.h:94-99).
 __device__ __forceinline__ uint32_t ActivateRef(uint32_t bits)
 {
     const __half2 x = AsHalf2(bits);
@@ -164,8 +136,6 @@ __device__ __forceinline__ uint32_t ActivateRef(uint32_t bits)
     const __half2 t = __hfma2_sat(third, x, __float2half2_rn(0.5f));
     const __half2 m = __hmin2(x, __float2half2_rn(3.f));
     const __half2 y = __hmul2_rn(m, t);
-    if (kToFp8)
-        return AsU32(RoundTripE4m3(y));
     const __half2 p = __hmul2_rn(y, __float2half2_rn(80.f));
     // rint(p), p in [-15, 240]: the binary16 spacing is 1 in [1024, 2048)
     __half2 r = __hadd2_rn(p, __float2half2_rn(1536.f));
@@ -331,7 +301,7 @@ struct RefTileContext
 
 // Builds the tile's lookup tables and stages the latent footprint of both grids in shared memory
 // (`tablesValid`: the tables already hold this tile's values, see PrepareTaps).  `warp`: of the chain's four.
-template <bool kFp8, int kLayers = 0>
+template <int kLayers = 0>
 __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
     int tileX0, int tileY0, int lane, int warp, bool tablesValid)
 {
@@ -349,7 +319,7 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
         {
             const float e0 = __fmaf_rn(Frac(f), 2.f, -1.f);
             const float e1 = __fmaf_rn(Frac(__fadd_rn(f, 0.25f)), 2.f, -1.f);
-            q[wave] = AsU32(QuantizeInputRef<kFp8>(__floats2half2_rn(e0, e1)));
+            q[wave] = AsU32(QuantizeInputRef(__floats2half2_rn(e0, e1)));
             f = __fmul_rn(f, 2.f);
         }
         if (!rows && lane < ChainTile::kWidth)
@@ -358,8 +328,8 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
             stage.tables.rowEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
         if (rows && lane == ChainTile::kHeight)
         {
-            stage.tables.lodPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(mip.positionLod)));
-            stage.tables.zeroPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(0.f)));
+            stage.tables.lodPair = AsU32(QuantizeInputRef(__float2half2_rn(mip.positionLod)));
+            stage.tables.zeroPair = AsU32(QuantizeInputRef(__float2half2_rn(0.f)));
         }
     }
     PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, tileX0,
@@ -368,7 +338,6 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
 
 // Four inputs of one latent layer from the four taps, as two binary16 pairs.
 // Blend order as the reference build evaluates it: fma(l11,w3, fma(l10,w2, fma(l00,w0, l01*w1))).
-template <bool kFp8>
 __device__ __forceinline__ void BlendLayerRef(uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00, __half2 w01,
     __half2 w10, __half2 w11, uint32_t* words)
 {
@@ -383,22 +352,20 @@ __device__ __forceinline__ void BlendLayerRef(uint2 l00, uint2 l01, uint2 l10, u
     b = __hfma2(AsHalf2(l11.y), w11, b);
     a = __hfma2(a, two, minusOne);
     b = __hfma2(b, two, minusOne);
-    words[0] = AsU32(QuantizeInputRef<kFp8>(a));
-    words[1] = AsU32(QuantizeInputRef<kFp8>(b));
+    words[0] = AsU32(QuantizeInputRef(a));
+    words[1] = AsU32(QuantizeInputRef(b));
 }
 
 // One latent layer of one grid (the low 16 bits of each p are the tap's four features) -> two pairs of inputs.
-template <bool kFp8>
 __device__ __forceinline__ void BlendPixelsRef(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, uint32_t* words)
 {
     __half2 inputs[2];
     BlendPixels(p00, p01, p10, p11, taps, inputs);
-    words[0] = AsU32(QuantizeInputRef<kFp8>(inputs[0]));
-    words[1] = AsU32(QuantizeInputRef<kFp8>(inputs[1]));
+    words[0] = AsU32(QuantizeInputRef(inputs[0]));
+    words[1] = AsU32(QuantizeInputRef(inputs[1]));
 }
 
 // Two latent layers of one grid (a word of each tap) -> two pairs of inputs each.
-template <bool kFp8>
 __device__ __forceinline__ void BlendLayersRef(uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11, const GridTaps& taps, uint32_t* words)
 {
     __half2 inputs[4];
@@ -406,24 +373,23 @@ __device__ __forceinline__ void BlendLayersRef(uint32_t p00, uint32_t p01, uint3
 #pragma unroll
     for (int j = 0; j < 2; ++j)
     {
-        const uint32_t even = AsU32(QuantizeInputRef<kFp8>(inputs[2 * j])), odd = AsU32(QuantizeInputRef<kFp8>(inputs[2 * j + 1]));
+        const uint32_t even = AsU32(QuantizeInputRef(inputs[2 * j])), odd = AsU32(QuantizeInputRef(inputs[2 * j + 1]));
         words[j] = __byte_perm(even, odd, 0x5410);
         words[2 + j] = __byte_perm(even, odd, 0x7632);
     }
 }
 
 // ... with the taps read straight from the layer's plane in global memory.
-template <bool kFp8>
 __device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plane, const GridTaps& taps, uint32_t* words)
 {
     const uint32_t p00 = __ldg(plane + taps.o00), p01 = __ldg(plane + taps.o01);
     const uint32_t p10 = __ldg(plane + taps.o10), p11 = __ldg(plane + taps.o11);
-    BlendPixelsRef<kFp8>(p00, p01, p10, p11, taps, words);
+    BlendPixelsRef(p00, p01, p10, p11, taps, words);
 }
 
 // The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.  `known`: TexelTables and the
 // row's last two chunks are those of an earlier tile with the same tables.
-template <bool kFp8, int kLayers = 0>
+template <int kLayers = 0>
 __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
     const RefTileContext& ctx, int tileColumn, int tileRow, bool known)
 {
@@ -438,7 +404,7 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
         if (!known)
             PrepareTexel(stage, ctx.tid & 127, tileColumn, tileRow);
         GatherTexel<kLayers>(params, mip, stage, ctx.tid & 127, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00,
-            __half2 w01, __half2 w10, __half2 w11) { BlendLayerRef<kFp8>(l00, l01, l10, l11, w00, w01, w10, w11, words + 8 * grid + 2 * layer); });
+            __half2 w01, __half2 w10, __half2 w11) { BlendLayerRef(l00, l01, l10, l11, w00, w01, w10, w11, words + 8 * grid + 2 * layer); });
     }
     else
     {
@@ -453,13 +419,13 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
             if (layer < NumLayers<kLayers>(params))
-                SampleLayerRef<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
+                SampleLayerRef(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
         SetupTaps(u, v, mip.loWidth, mip.loHeight, taps);
         const uint16_t* lo = params.latents + mip.loOffset;
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
             if (layer < NumLayers<kLayers>(params))
-                SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
+                SampleLayerRef(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
     }
 
     if (!known)
@@ -570,7 +536,7 @@ __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
 
 // Second half of a layer: waits for the MMA, then applies the activation and writes the next
 // layer's A operand (layers 0-2) or stores the texel (layer 3).
-template <bool kFp8, int kLayer, int kConvert, typename Params>
+template <int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefTileContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
@@ -585,7 +551,6 @@ __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefT
 
     if (kLayer < 3)
     {
-        constexpr bool kNextFp8 = kFp8 && kLayer < 2; // layer 2 always re-quantises to the int8 grid
         uint4* rowChunk = ctx.rowChunk;
         // all accumulators of the row are requested before the first wait, so that the round trips to
         // tensor memory overlap: 64 -> two loads of 32, 48 -> 32 + 16, 32 -> one load
@@ -609,12 +574,12 @@ __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefT
         };
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-            storeChunk(c, ActivateRef<kNextFp8>(low[4 * c]), ActivateRef<kNextFp8>(low[4 * c + 1]),
-                       ActivateRef<kNextFp8>(low[4 * c + 2]), ActivateRef<kNextFp8>(low[4 * c + 3]));
+            storeChunk(c, ActivateRef(low[4 * c]), ActivateRef(low[4 * c + 1]),
+                       ActivateRef(low[4 * c + 2]), ActivateRef(low[4 * c + 3]));
 #pragma unroll
         for (int c = 0; c < (kN - 32) / 8; ++c)
-            storeChunk(4 + c, ActivateRef<kNextFp8>(high[4 * c]), ActivateRef<kNextFp8>(high[4 * c + 1]),
-                       ActivateRef<kNextFp8>(high[4 * c + 2]), ActivateRef<kNextFp8>(high[4 * c + 3]));
+            storeChunk(4 + c, ActivateRef(high[4 * c]), ActivateRef(high[4 * c + 1]),
+                       ActivateRef(high[4 * c + 2]), ActivateRef(high[4 * c + 3]));
     }
     else
     {
@@ -634,12 +599,12 @@ __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefT
     }
 }
 
-template <bool kFp8, int kLayer, int kConvert, typename Params>
+template <int kLayer, int kConvert, typename Params>
 __device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext& ctx, uint32_t& phase)
 {
     if (IssueLayerRef<kLayer>(ctx))
         return 1;
-    ConsumeLayerRef<kFp8, kLayer, kConvert>(params, ctx, phase);
+    ConsumeLayerRef<kLayer, kConvert>(params, ctx, phase);
     return 0;
 }
 
@@ -710,7 +675,7 @@ __device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const R
 // The kernels
 // ---------------------------------------------------------------------------------------------
 
-template <bool kFp8, int kConvert, int kLayers>
+template <int kConvert, int kLayers>
 __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __grid_constant__ KernelParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
@@ -761,7 +726,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
     if (tile < uint32_t(params.totalTiles))
     {
         place = locate(tile, 0);
-        PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, false);
+        PrepareTileRef<kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, false);
         tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
         ChainBarrier(chain);
     }
@@ -771,7 +736,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
         ctx.tile = int(tile);
         ctx.x = place.tileX0 + tileColumn;
         ctx.y = place.tileY0 + tileRow;
-        BuildInputsRef<kFp8, kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
+        BuildInputsRef<kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
 
         // layer 0; while the tensor core works on it, prepare the chain's NEXT tile (its tables and
         // footprints replace this tile's, which nobody reads after the barrier inside IssueLayerRef)
@@ -785,13 +750,13 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
             const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
             known = keepsTables && place.mipIndex == tablesMip;
-            PrepareTileRef<kFp8, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
+            PrepareTileRef<kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
-        ConsumeLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
+        ConsumeLayerRef<0, kConvertNone>(params, ctx, phase);
 
-        RunLayerRef<kFp8, 1, kConvertNone>(params, ctx, phase);
-        RunLayerRef<kFp8, 2, kConvertNone>(params, ctx, phase);
+        RunLayerRef<1, kConvertNone>(params, ctx, phase);
+        RunLayerRef<2, kConvertNone>(params, ctx, phase);
         {
             // where the texel goes (worked out only now: nothing of it has to stay in registers through the
             // layers); the element index inside a mip fits 32 bits (checked on the host)
@@ -815,7 +780,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
                 ctx.storeBytes = mip.storeBytes;
             }
         }
-        RunLayerRef<kFp8, 3, kConvert>(params, ctx, phase);
+        RunLayerRef<3, kConvert>(params, ctx, phase);
         tile = nextTile;
     }
 
@@ -825,7 +790,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
 // Inference on sample with the reference's numerics: one thread per query (u, v, lod) -> the texel
 // (mip = clamp(floor(lod)), x = min(floor(u * W), W - 1), y likewise) is evaluated exactly as the
 // decode kernel evaluates it; the taps are read straight from global memory.
-template <bool kFp8, bool kInterleaved, int kLayers>
+template <bool kInterleaved, int kLayers>
 __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __grid_constant__ SampleParams params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
@@ -852,7 +817,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
     ctx.outStepWords = 1;
     ctx.storeBytes = params.storeBytes;
 
-    const uint32_t zeroPair = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(0.f)));
+    const uint32_t zeroPair = AsU32(QuantizeInputRef(__float2half2_rn(0.f)));
     const unsigned long long tiles = (params.numQueries + 127) / 128;
     const int row = tid & 127;
     // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
@@ -903,10 +868,10 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
                 SetupTaps(su, sv, mip.loWidth, mip.loHeight, lowTaps);
                 SampleInterleaved(hi, lo, numLayers, taps, lowTaps,
                     [&](int grid, int layer, uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11) {
-                        BlendLayersRef<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, words + 8 * grid + 2 * layer);
+                        BlendLayersRef(p00, p01, p10, p11, grid ? lowTaps : taps, words + 8 * grid + 2 * layer);
                     },
                     [&](int grid, int layer, uint32_t p00, uint32_t p01, uint32_t p10, uint32_t p11) {
-                        BlendPixelsRef<kFp8>(p00, p01, p10, p11, grid ? lowTaps : taps, words + 8 * grid + 2 * layer);
+                        BlendPixelsRef(p00, p01, p10, p11, grid ? lowTaps : taps, words + 8 * grid + 2 * layer);
                     });
             }
             else
@@ -914,12 +879,12 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
 #pragma unroll
                 for (int layer = 0; layer < 4; ++layer)
                     if (layer < numLayers)
-                        SampleLayerRef<kFp8>(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
+                        SampleLayerRef(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
                 SetupTaps(su, sv, mip.loWidth, mip.loHeight, taps);
 #pragma unroll
                 for (int layer = 0; layer < 4; ++layer)
                     if (layer < numLayers)
-                        SampleLayerRef<kFp8>(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
+                        SampleLayerRef(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
             }
             // src/RegressionKernels.h:59-85: per wave the inputs (x phase 0, y phase 0, x phase 0.25, y phase 0.25)
             float xf = __fmul_rn(float(x), mip.positionScale);
@@ -930,12 +895,12 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
                 const float ex = __fmaf_rn(Frac(xf), 2.f, -1.f), ey = __fmaf_rn(Frac(yf), 2.f, -1.f);
                 const float ez = __fmaf_rn(Frac(__fadd_rn(xf, 0.25f)), 2.f, -1.f);
                 const float ew = __fmaf_rn(Frac(__fadd_rn(yf, 0.25f)), 2.f, -1.f);
-                words[16 + 2 * wave] = AsU32(QuantizeInputRef<kFp8>(__floats2half2_rn(ex, ey)));
-                words[17 + 2 * wave] = AsU32(QuantizeInputRef<kFp8>(__floats2half2_rn(ez, ew)));
+                words[16 + 2 * wave] = AsU32(QuantizeInputRef(__floats2half2_rn(ex, ey)));
+                words[17 + 2 * wave] = AsU32(QuantizeInputRef(__floats2half2_rn(ez, ew)));
                 xf = __fmul_rn(xf, 2.f);
                 yf = __fmul_rn(yf, 2.f);
             }
-            words[22] = AsU32(QuantizeInputRef<kFp8>(__float2half2_rn(mip.positionLod)));
+            words[22] = AsU32(QuantizeInputRef(__float2half2_rn(mip.positionLod)));
             words[23] = zeroPair;
 #pragma unroll
             for (int chunk = 0; chunk < 6; ++chunk)
@@ -943,14 +908,14 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
         }
 
         // nothing is shared between the chains of a query tile: each runs at its own pace
-        aborted = RunLayerRef<kFp8, 0, kConvertNone>(params, ctx, phase);
+        aborted = RunLayerRef<0, kConvertNone>(params, ctx, phase);
         if (aborted)
             break;
         tile = nextTile;
         nextTile = blockIdx.x + (unsigned long long)shared.claimed[chain] * gridDim.x;
-        RunLayerRef<kFp8, 1, kConvertNone>(params, ctx, phase);
-        RunLayerRef<kFp8, 2, kConvertNone>(params, ctx, phase);
-        RunLayerRef<kFp8, 3, kConvertNone>(params, ctx, phase);
+        RunLayerRef<1, kConvertNone>(params, ctx, phase);
+        RunLayerRef<2, kConvertNone>(params, ctx, phase);
+        RunLayerRef<3, kConvertNone>(params, ctx, phase);
     }
     TeardownCtaRef(shared, ctx, phase, tid, warp);
 }
@@ -1079,7 +1044,7 @@ __device__ __forceinline__ void IssueChainRefFp8(int chain, uint32_t accumulator
             // 16 products of the 32-wide chunk step / 2: weight copy `step` has the other 16 columns zeroed
             const uint64_t descA = operandBase + uint64_t(((step / 2) * 2 * 2048) >> 4);
             const uint64_t descB = weightBase + uint64_t((step * kN * 32) >> 4);
-            if (kTmemOperand && kLayer > 0)
+            if (kLayer > 0)
                 UmmaE4m3F16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step / 2) * 8u, descB, instr, 1, enabled);
             else
                 UmmaE4m3F16(accumulators, descA, descB, instr, 1, enabled);
@@ -1087,12 +1052,8 @@ __device__ __forceinline__ void IssueChainRefFp8(int chain, uint32_t accumulator
         else
         {
             // binary16 operands: one K step = two core matrices of 8 halves
-            const uint64_t descA = operandBase + uint64_t((step * 2 * 2048) >> 4);
             const uint64_t descB = weightBase + uint64_t((step * 2 * kN * 16) >> 4);
-            if (kTmemOperand)
-                UmmaF16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step) * 8u, descB, instr, 1, enabled);
-            else
-                UmmaF16(accumulators, descA, descB, instr, 1, enabled);
+            UmmaF16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step) * 8u, descB, instr, 1, enabled);
         }
     }
     // arrives once everything issued so far has completed: this chain's accumulators are ready
@@ -1111,12 +1072,12 @@ __device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
     // documented pattern.  A single fence in the issuing warp after the barrier passed every parity test
     // and was 2 % faster - the fence costs each thread about 200 cycles - but is not what the
     // programming guide shows, so it was not adopted.)
-    if (kTmemOperand && kLayer > 0)
+    if (kLayer > 0)
         TmemStoreWait(); // the operand went to tensor memory: nothing the async proxy reads was written
-    else if (!(kAblate & 128))
+    else
         FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
-    if (!(kAblate & 1024) && LayerBarrier<kLayer>(ctx.tid, ctx.giveUp))
+    if (LayerBarrier<kLayer>(ctx.tid, ctx.giveUp))
         return 1;
     // The whole issuing warp runs the descriptor arithmetic, on values the compiler can see are the same
     // in every lane (hence the shuffles, and addresses counted from the start of dynamic shared memory instead of taken from
@@ -1124,7 +1085,7 @@ __device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
     // from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
     // (Tried: building the descriptors before the barrier - 3 % slower.)
     const int warpIndex = ctx.tid >> 5;
-    if (WarpRole(warpIndex) == kIssuingRole && !(kAblate & 16))
+    if (WarpRole(warpIndex) == kIssuingRole)
     {
         TcgenFenceAfterSync();
         const uint32_t elected = ElectOne();
@@ -1153,7 +1114,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     // three blocked in a named barrier executes 1.5 % fewer instructions but wakes the chain later, 4.5 %
     // slower; an issuing thread per chain instead of one for both, 7 % slower; polls without a suspend-time
     // hint, the same speed.)
-    if (!(kAblate & 16) && !MbarrierWaitBounded(ctx.barrier, phase))
+    if (!MbarrierWaitBounded(ctx.barrier, phase))
     {
         SetGiveUp(ctx.giveUp);
         ReportTimeout(params.status, uint32_t(ctx.tile), uint32_t(kLayer));
@@ -1161,62 +1122,22 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     phase ^= 1;
     TcgenFenceAfterSync();
 
-    if ((kAblate & 4) && kLayer < 3)
-    {
-        // profiling variant: the accumulator words go to the operand as they are
-        uint4* rowChunk = ctx.rowChunk;
-        uint32_t low[16];
-        if (!(kAblate & 32))
-        {
-            TmemLoadPacked16(ctx.tmemLane, low);
-            TmemLoadWait();
-        }
-        else
-        {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                low[i] = uint32_t(ctx.tile + i);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-        {
-            if (kTmemOperand)
-                TmemStore4(ctx.tmemLane + kOperandColumn + 4u * uint32_t(c), low[4 * c], low[4 * c + 1], low[4 * c + 2], low[4 * c + 3]);
-            else
-                rowChunk[c * 128] = make_uint4(low[4 * c], low[4 * c + 1], low[4 * c + 2], low[4 * c + 3]);
-        }
-        return;
-    }
-
     if (kLayer < 2)
     {
         // e4m3 codes for the next layer: 16 per 16-byte chunk
-        uint4* rowChunk = ctx.rowChunk;
         uint32_t low[16], high[16];
-        if (!(kAblate & 32))
-        {
-            TmemLoadPacked16(ctx.tmemLane, low);
-            if (kN == 64)
-                TmemLoadPacked16(ctx.tmemLane + 32, high);
-            else
-            {
-                uint32_t (&tail)[8] = reinterpret_cast<uint32_t (&)[8]>(high);
-                TmemLoadPacked8(ctx.tmemLane + 32, tail);
-            }
-            TmemLoadWait();
-        }
+        TmemLoadPacked16(ctx.tmemLane, low);
+        if (kN == 64)
+            TmemLoadPacked16(ctx.tmemLane + 32, high);
         else
         {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                low[i] = high[i] = uint32_t(ctx.tile * 3 + i) & 0x3FFF3FFFu;
+            uint32_t (&tail)[8] = reinterpret_cast<uint32_t (&)[8]>(high);
+            TmemLoadPacked8(ctx.tmemLane + 32, tail);
         }
-        // chunk c of the next layer's operand row: to shared memory, or to tensor memory columns 48 + 4 c ..
+        TmemLoadWait();
+        // chunk c of the next layer's operand row: tensor-memory columns 48 + 4 c ..
         auto storeChunk = [&](int c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
-            if (kTmemOperand)
-                TmemStore4(ctx.tmemLane + kOperandColumn + 4u * uint32_t(c), w0, w1, w2, w3);
-            else
-                rowChunk[c * 128] = make_uint4(w0, w1, w2, w3);
+            TmemStore4(ctx.tmemLane + kOperandColumn + 4u * uint32_t(c), w0, w1, w2, w3);
         };
 #pragma unroll
         for (int c = 0; c < 2; ++c)
@@ -1238,45 +1159,23 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     else if (kLayer == 2)
     {
         // layer 3 runs on the binary16 path: its inputs are the int8 grid values rint(y * 80) * 0.0125
-        uint4* rowChunk = ctx.rowChunk;
         uint32_t acc[16];
-        if (!(kAblate & 32))
-        {
-            TmemLoadPacked16(ctx.tmemLane, acc);
-            TmemLoadWait();
-        }
-        else
-        {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                acc[i] = uint32_t(ctx.tile * 5 + i) & 0x3FFF3FFFu;
-        }
+        TmemLoadPacked16(ctx.tmemLane, acc);
+        TmemLoadWait();
 #pragma unroll
         for (int c = 0; c < 4; ++c)
         {
-            const uint32_t w0 = ActivateRef<false>(acc[4 * c]), w1 = ActivateRef<false>(acc[4 * c + 1]);
-            const uint32_t w2 = ActivateRef<false>(acc[4 * c + 2]), w3 = ActivateRef<false>(acc[4 * c + 3]);
-            if (kTmemOperand)
-                TmemStore4(ctx.tmemLane + kOperandColumn + 4u * uint32_t(c), w0, w1, w2, w3);
-            else
-                rowChunk[c * 128] = make_uint4(w0, w1, w2, w3);
+            const uint32_t w0 = ActivateRef(acc[4 * c]), w1 = ActivateRef(acc[4 * c + 1]);
+            const uint32_t w2 = ActivateRef(acc[4 * c + 2]), w3 = ActivateRef(acc[4 * c + 3]);
+            TmemStore4(ctx.tmemLane + kOperandColumn + 4u * uint32_t(c), w0, w1, w2, w3);
         }
     }
     else
     {
         // output (src/Inference.cu:121-135): the accumulators are the channels
         uint32_t bits[8];
-        if (!(kAblate & 32))
-        {
-            TmemLoadPacked8(ctx.tmemLane, bits);
-            TmemLoadWait();
-        }
-        else
-        {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                bits[i] = uint32_t(ctx.tile * 7 + i) & 0x3FFF3FFFu;
-        }
+        TmemLoadPacked8(ctx.tmemLane, bits);
+        TmemLoadWait();
         const int channelPairs = params.channels >> 1;
         ScrubSpecials(bits, channelPairs);
         if constexpr (kConvert != kConvertNone)
@@ -1285,20 +1184,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
                 StoreConverted<kConvert>(params.conversion, params.firstChannel, params.numChannels, ctx, bits);
         }
         else if (ctx.out)
-        {
-            if (kAblate & 8)
-            {
-                // profiling variant: keep the values alive without storing them (the condition never holds)
-                uint32_t all = 0;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    all ^= bits[j];
-                if (all == 0x12345679u && ctx.tile < 0)
-                    ctx.out[0] = all;
-            }
-            else
-                StoreTexel(ctx.out, ctx.outStepWords, ctx.storeBytes, bits, channelPairs);
-        }
+            StoreTexel(ctx.out, ctx.outStepWords, ctx.storeBytes, bits, channelPairs);
     }
 }
 
@@ -1425,15 +1311,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const
         ctx.x = place.tileX0 + tileColumn;
         ctx.y = place.tileY0 + tileRow;
         // the e4m3 input stage is the one of the exact-accumulation kernel (64-byte rows of codes)
-        if (kAblate & 2)
-        {
-            const uint32_t filler = uint32_t(tile) & 0x3F3F3F3Fu;
-#pragma unroll
-            for (int chunk = 0; chunk < 4; ++chunk)
-                ctx.rowChunk[chunk * 128] = make_uint4(filler, filler + chunk, filler, filler);
-        }
-        else
-            BuildInputsRefFp8<kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
+        BuildInputsRefFp8<kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
 
         aborted = IssueLayerRefFp8<0>(ctx);
         if (aborted)
@@ -1441,13 +1319,11 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const
         const uint32_t nextTile = tile + chains * gridDim.x;
         if (nextTile < uint32_t(params.totalTiles))
         {
-            if (!(kAblate & 512))
-                place = locate(nextTile, place.mipIndex);
+            place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = (kAblate & 512) ? true : TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
-            known = keepsTables && place.mipIndex == tablesMip && !(kAblate & 64);
-            if (!(kAblate & 1))
-                PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
+            const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
+            known = keepsTables && place.mipIndex == tablesMip;
+            PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayerRefFp8<0, kConvertNone>(params, ctx, phase);
@@ -1628,7 +1504,7 @@ cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStre
             return LaunchRefKernel(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, sizeof(RefFp8Stage)),
                 SharedBytes<RefFp8SharedStorage>(kMaxChains, sizeof(RefFp8Stage)), chains, params, ctas, stream);
         else
-            return LaunchRefKernel(DecodeKernelRef<false, kConvert, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, sizeof(RefStage)),
+            return LaunchRefKernel(DecodeKernelRef<kConvert, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, sizeof(RefStage)),
                 SharedBytes<RefSharedStorage>(kMaxChains, sizeof(RefStage)), chains, params, ctas, stream);
     };
     switch (params.numLayers)
@@ -1665,7 +1541,7 @@ cudaError_t LaunchSampleRefLayers(const SampleParams& params, int ctas, cudaStre
             return LaunchRefKernel(SampleKernelRefFp8<kInterleaved, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, 0),
                 SharedBytes<RefFp8SharedStorage>(kMaxChains, 0), chains, params, ctas, stream);
         else
-            return LaunchRefKernel(SampleKernelRef<false, kInterleaved, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, 0),
+            return LaunchRefKernel(SampleKernelRef<kInterleaved, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, 0),
                 SharedBytes<RefSharedStorage>(kMaxChains, 0), chains, params, ctas, stream);
     };
     if constexpr (kInterleaved)
