@@ -177,6 +177,7 @@ inline size_t ConvertedPixelAlignment(size_t pixelBytes)
 int MakeOutputConversion(const ::NtcbOutputConversion& request, int channels, OutputConversion& out);
 
 cudaError_t LaunchDecode(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream);
+cudaError_t LaunchDecodeConverting(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream); // (LaunchDecode's, for params.convert)
 // The reference-numerics kernel (decode_kernel_ref.cu): params.network is a kRefNetworkBytes image.
 cudaError_t LaunchDecodeRef(const KernelParams& params, bool fp8, int ctas, cudaStream_t stream);
 cudaError_t LaunchSampleRef(const SampleParams& params, bool fp8, int ctas, cudaStream_t stream);
