@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(kThreads) Bc7ModeKernel(const Bc7Arguments arg
 //
 // With one thread per block for everything a 1024 x 1024 image was 2048 warps of 800 k instructions, 14 resident per SM:
 // 1.81 ms.  Eight warps per 64 blocks and packed arithmetic fill the machine from a few thousand blocks up: 0.52 ms, bound by
-// the FMA pipe (61 % of its cycles) and instruction issue (67 %), three CTAs of 80 registers per SM (four of 64 spill in the
+// the FMA pipe and instruction issue (66 % and 65 % busy on a 2048 x 2048 one), three CTAs of 80 registers per SM (four of 64 spill in the
 // tasks: 3 % slower).
 constexpr int kSearchWarps = 8;
 constexpr int kSearchThreads = 32 * kSearchWarps;

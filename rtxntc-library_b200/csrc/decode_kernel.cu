@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert != kConvertNone ? kCt
             ++place.mipIndex;
         const KernelMip& mip = params.mips[place.mipIndex];
         const int local = tile - mip.firstTile;
-        // local / tilesX through a precomputed reciprocal (exact while local * tilesX < 2^32)
+        // local / tilesX through a precomputed reciprocal where that is exact for every tile of the mip (FillKernelMip)
         const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
         place.tileX0 = (local - tileY * mip.tilesX) * kTileWidth;
         place.tileY0 = mip.rowBegin + tileY * kTileHeight;

@@ -9,10 +9,11 @@
 //
 // Work decomposition.  One CTA per SM of up to eight chains of 128 threads.  The chains share the network and nothing else: each
 // walks tiles of 16 x 8 texels of its own, with its own tables and footprints, and meets only its own threads in
-// barriers.  What bounds the kernels is instruction issue (75 % of the slots busy; 8 x 4 warps of 64 registers and 8 x 64
+// barriers.  What bounds the kernels is instruction issue (81 % of the slots busy, Int8 75 %; 8 x 4 warps of 64 registers and 8 x 64
 // tensor-memory columns fill an SM), so the split aims at few instructions and warps that never wait for another chain.  (With four
 // CTAs per SM of two chains each, the four copies of the network left no room for TexelTables, and on average 3.3 of the four were
-// active - the scheduler favours the older, whose share ends early: 4096 x 4096 FP8 897 us, now 832; 8192 x 8192 Int8 4985, now 4523.)
+// active - the scheduler favours the older, whose share ends early: 4096 x 4096 FP8 897 us instead of 832, 8192 x 8192 Int8 4985 instead of
+// 4523.  With the warps' roles as they are now, see WarpRole: 779 and 4190.)
 //
 // What differs from decode_kernel.cu:
 //   * the A operand holds binary16 values (the de-quantised network inputs / activations), up to 128
@@ -473,8 +474,8 @@ __device__ __forceinline__ void UmmaF16FromTmem(uint32_t tmemD, uint32_t tmemA, 
         : "memory");
 }
 
-// First half of a layer for the chain's current tile: the chain's barrier (LayerBarrier), and MMA issue by its first
-// warp.  Returns nonzero (uniformly over the chain) when some thread gave up on a wait.
+// First half of a layer for the chain's current tile: the chain's barrier (LayerBarrier), and MMA issue by the warp of
+// kIssuingRole.  Returns nonzero (uniformly over the chain) when some thread gave up on a wait.
 template <int kLayer>
 __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
 {
@@ -609,8 +610,8 @@ __device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext&
 }
 
 // One-time setup of a CTA: the network image arrives by one TMA bulk copy while the threads fill
-// the constant tables, set up the barriers and allocate tensor memory.  Returns nonzero in every
-// thread that gave up waiting for the image (status words written).
+// the constant tables, set up the barriers and allocate tensor memory.  A thread that gives up waiting for the image
+// sets its chain's give-up word (status words written): the chain leaves at its first tile.
 __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
 {
     // constant A operands of the bias steps: core matrix l (8 rows of 16 bytes) has 1.0 as half l of every row,
@@ -1112,8 +1113,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
 
     // (Every warp polls the barrier itself.  Tried and dropped: one polling warp per chain with the other
     // three blocked in a named barrier executes 1.5 % fewer instructions but wakes the chain later, 4.5 %
-    // slower; an issuing thread per chain instead of one for both, 7 % slower; polls without a suspend-time
-    // hint, the same speed.)
+    // slower; polls without a suspend-time hint, the same speed.)
     if (!MbarrierWaitBounded(ctx.barrier, phase))
     {
         SetGiveUp(ctx.giveUp);

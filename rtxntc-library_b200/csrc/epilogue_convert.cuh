@@ -139,7 +139,7 @@ __device__ __forceinline__ uint32_t LinearCodes(uint32_t pair)
 
 // The kConvertUnorm8 epilogue: word by word, four linear channels in six instructions, then the bytes of the channels that are
 // encoded to sRGB.  What a word takes is the same for every pixel.  (With one sRGB texture in a 12-channel set all channels
-// went through the general quantiser: 500 us more on a 4096 x 4096 chain than fp16 texels; now 100.)
+// went through the general quantiser: 500 us more on a 4096 x 4096 chain than fp16 texels; now about 115.)
 template <typename Context>
 __device__ __forceinline__ void ConvertUnorm8Pixel(const OutputConversion& conversion, const Context& ctx, const uint32_t (&pairs)[8])
 {
