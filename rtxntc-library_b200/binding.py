@@ -566,8 +566,8 @@ class ResidentTextureSet:
         _queue(self.latents.device, lib().ntcb_decode, ctypes.byref(params))
 
     def _pointers(self, mode: int) -> tuple:
-        """What the parameters of a launch depend on besides the geometry: they are filled again when one of these changes."""
-        return (self.latents.data_ptr(), self.networks[mode].data_ptr(), self.status.data_ptr(),
+        """What the parameters of a launch depend on: they are filled again when one of these changes."""
+        return (self.geometry, self.latents.data_ptr(), self.networks[mode].data_ptr(), self.status.data_ptr(),
                 None if self.out is None else self.out.data_ptr(), self.layout, self.numerics)
 
     def decode(self, use_int8: bool, mips=None, row_ranges=None) -> None:

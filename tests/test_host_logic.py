@@ -330,6 +330,32 @@ def test_staged_weights_are_rounded_to_the_nearest_half():
     assert len(seen) == 64  # every sign and exponent
 
 
+def test_kept_launch_parameters_follow_the_set():
+    """ResidentTextureSet keeps the parameters of a whole-set decode: they are filled again when anything they were filled from is
+    replaced, the geometry included."""
+    import torch
+
+    class Recording(binding.ResidentTextureSet):
+        def launch(self, params):
+            launched.append(binding.DecodeParams.from_buffer_copy(params))
+
+    launched = []
+    first, second = (synthetic.make_texture_set(synthetic.TextureSetSpec(w, 32, 4, 1, 2, 8, seed=1)) for w in (64, 48))
+    resident = Recording.from_synthetic(first, device="cpu")
+    resident.decode(True)
+    resident.decode(True)
+    assert [p.mips[0].width for p in launched] == [64, 64] and launched[0].out == launched[1].out
+    resident.geometry = second.geometry
+    resident.decode(True)
+    assert launched[-1].mips[0].width == 48
+    resident.out = torch.empty_like(resident.out)
+    resident.decode(True)
+    assert launched[-1].out == resident.out.data_ptr() != launched[0].out
+    resident.latents = resident.latents.clone()
+    resident.decode(True)
+    assert launched[-1].latents == resident.latents.data_ptr()
+
+
 def test_stage_network_rejects_wrong_sizes():
     for numerics in (binding.NUMERICS_REFERENCE, binding.NUMERICS_EXACT):
         with pytest.raises(binding.NtcbError) as error:
