@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kBc4Threads) BlockCompressKernel(const Bc4Argu
         {
             const int y = args.base.srcTop + blockY * 4 + row;
             float texel[2] = {0.f, 0.f};
-            if (x < args.base.width && y < args.base.height)
+            if (Inside(args.base, x, y))
             {
                 if (args.base.firstChannel < 0)
                     texel[0] = 1.f; // the alpha of texels that carry none
@@ -1109,7 +1109,7 @@ __global__ void __launch_bounds__(kColorThreads, 8) ColorBlockCompressKernel(con
         const int p = k * kColorThreads + tid;
         const int localX = p & 63, localY = p >> 6;
         const int x = args.base.srcLeft + blockIdx.x * 64 + localX, y = args.base.srcTop + blockIdx.y * 16 + localY;
-        const bool inside = x < args.base.width && y < args.base.height;
+        const bool inside = Inside(args.base, x, y);
         // missing channels read 0, alpha 1 (0x3c00)
         uint32_t redGreen = 0u, blueAlpha = 0u;
         if (inside)
@@ -1309,8 +1309,9 @@ extern "C" int ntcb_block_compress(const NtcbBlockCompressParams* params, void* 
     args.height = params->height;
     args.channels = params->channels;
     args.firstChannel = params->firstChannel;
-    args.srcLeft = params->srcLeft;
-    args.srcTop = params->srcTop;
+    // (a window that starts outside the mip holds no texel of it, wherever that is)
+    args.srcLeft = std::min(params->srcLeft, params->width);
+    args.srcTop = std::min(params->srcTop, params->height);
     args.widthInBlocks = params->widthInBlocks;
     args.heightInBlocks = params->heightInBlocks;
     args.formatChannels = formatChannels;

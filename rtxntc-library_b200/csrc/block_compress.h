@@ -27,6 +27,12 @@ inline bool ChannelPairs(const BlockCompressArguments& args)
     return !(reinterpret_cast<uintptr_t>(args.texels) & 3) && !(args.firstChannel & 1) && !(args.channels & 1);
 }
 
+// Whether a texel lies inside the mip.  (Unsigned: a position that has passed 2^31 - a window far outside - counts as outside.)
+__device__ __forceinline__ bool Inside(const BlockCompressArguments& args, int x, int y)
+{
+    return unsigned(x) < unsigned(args.width) && unsigned(y) < unsigned(args.height);
+}
+
 __device__ __forceinline__ __half LoadHalf(const BlockCompressArguments& args, int x, int y, int channel)
 {
     const size_t w = size_t(args.width), c = size_t(args.channels);

@@ -845,7 +845,7 @@ __device__ uint4 EncodeInMode(const uint2* texels, int stride, uint32_t mode, ui
 // every component reads 0.
 __device__ __forceinline__ uint2 LoadTexel(const Bc7Arguments& args, int x, int y)
 {
-    if (x >= args.base.width || y >= args.base.height)
+    if (!Inside(args.base, x, y))
         return make_uint2(0u, 0u);
     const int first = args.base.firstChannel, count = args.numChannels;
     if (args.base.pairs)

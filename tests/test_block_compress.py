@@ -589,6 +589,19 @@ def test_images_of_more_rows_than_a_grid_has(block_format):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("block_format", [1, 2, 3, 4, 5, 7])
+def test_windows_far_outside_the_mip_hold_zeros(block_format):
+    """Every position a window may start at outside the mip, up to the last an int holds: the texels read as 0."""
+    import torch
+
+    image = torch.full((24, 20, 4), 0.75, dtype=torch.float16, device="cuda")
+    window = dict(width_in_blocks=40, height_in_blocks=9, num_channels=0 if block_format in (4, 5) else 4)  # (with alpha, which reads 0 too)
+    expected = binding.block_compress(torch.zeros((36, 160, 4), dtype=torch.float16, device="cuda"), block_format, **window)
+    for left, top in ((20, 0), (0, 24), (2 ** 31 - 1, 0), (2 ** 31 - 64, 2 ** 31 - 4), (4, 2 ** 31 - 1)):
+        assert torch.equal(binding.block_compress(image, block_format, src_left=left, src_top=top, **window), expected), (left, top)
+
+
+@pytest.mark.gpu
 def test_kernel_on_ragged_images_windows_and_the_planar_layout(oracle):
     import torch
 
