@@ -130,29 +130,22 @@ __host__ __device__ constexpr uint32_t MakeInstrDescriptor(bool fp8, int n)
 // Small arithmetic helpers
 // ---------------------------------------------------------------------------------------------
 
-// Clamped HGELU in binary16 (src/tin/tin_activation.h:88-92) followed by re-quantisation:
-// e4m3 when `toFp8`, otherwise the int8 code rint(y * 80) - 113 (src/tin/tin_activation.h:94-99,
+// Clamped HGELU followed by re-quantisation to the int8 code rint(y * 80) - 113 (src/tin/tin_activation.h:94-99,
 // the -113 offset is folded into the next layer's stored bias, src/Quantizer.cu:176-181).
 // y * 80 lies in [-15, 240], so 113 is the only offset that fits int8; being odd, it cannot be
 // merged into the even magic addend without changing how ties round.
-template <bool kToFp8>
-__device__ __forceinline__ uint32_t ActivatePair(__half2 x)
+__device__ __forceinline__ uint32_t ActivateToInt8(__half2 x)
 {
-    const __half2 third = __float2half2_rn(1 / 3.f);
-    __half2 t = __hfma2_sat(third, x, __float2half2_rn(0.5f));
-    __half2 m = __hmin2(x, __float2half2_rn(3.f));
-    __half2 y = __hmul2_rn(m, t);
-    if (kToFp8)
-    {
-        return uint32_t(__nv_cvt_halfraw2_to_fp8x2(static_cast<__half2_raw>(y), __NV_SATFINITE, __NV_E4M3));
-    }
-    else
-    {
-        __half2 p = __hmul2_rn(y, __float2half2_rn(80.f));
-        __half2 r = __hadd2_rn(p, __float2half2_rn(1536.f)); // rint(p): ulp is 1 in [1024, 2048)
-        r = __hadd2_rn(r, __float2half2_rn(-113.f));         // exact
-        return AsU32(r);
-    }
+    const __half2 p = __hmul2_rn(ClampedHgelu(x), __float2half2_rn(80.f));
+    const __half2 r = __hadd2_rn(p, __float2half2_rn(1536.f)); // rint(p): ulp is 1 in [1024, 2048)
+    return AsU32(__hadd2_rn(r, __float2half2_rn(-113.f)));     // exact
+}
+
+// Two pairs of activations (e4m3) or of int8 codes -> the next layer's four operand bytes.
+template <bool kToFp8>
+__device__ __forceinline__ uint32_t PackCodes(uint32_t first, uint32_t second)
+{
+    return kToFp8 ? E4m3Codes(AsHalf2(first), AsHalf2(second)) : __byte_perm(first, second, 0x6420);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -320,7 +313,7 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Sha
                             float f1 = __fmul_rn(float(int32_t(acc[c][2 * j + 1]) + (kBiasTable ? biasI[colIndex + 1] : 0)), scale[colIndex + 1]);
                             xh = __floats2half2_rn(f0, f1);
                         }
-                        pairs[j] = ActivatePair<kNextFp8>(xh);
+                        pairs[j] = kNextFp8 ? AsU32(ClampedHgelu(xh)) : ActivateToInt8(xh);
                     }
                     const uint4 codes =
                         make_uint4(PackCodes<kNextFp8>(pairs[0], pairs[1]), PackCodes<kNextFp8>(pairs[2], pairs[3]),
@@ -658,8 +651,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPe
 
         {
             uint32_t words[16];
-            const uint32_t zeroWord = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(0.f)),
-                                                      QuantizeInputPair<kFp8>(__float2half2_rn(0.f)));
+            const uint32_t zeroWord = QuantizedZeros<kFp8>();
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 words[i] = zeroWord;
@@ -677,13 +669,11 @@ __global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPe
                 const float ex = __fmaf_rn(Frac(xf), 2.f, -1.f), ey = __fmaf_rn(Frac(yf), 2.f, -1.f);
                 const float ez = __fmaf_rn(Frac(__fadd_rn(xf, 0.25f)), 2.f, -1.f);
                 const float ew = __fmaf_rn(Frac(__fadd_rn(yf, 0.25f)), 2.f, -1.f);
-                words[8 + wave] = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__floats2half2_rn(ex, ey)),
-                                                   QuantizeInputPair<kFp8>(__floats2half2_rn(ez, ew)));
+                words[8 + wave] = QuantizeInputs<kFp8>(__floats2half2_rn(ex, ey), __floats2half2_rn(ez, ew));
                 xf = __fmul_rn(xf, 2.f);
                 yf = __fmul_rn(yf, 2.f);
             }
-            words[11] = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(mip.positionLod)),
-                                        QuantizeInputPair<kFp8>(__float2half2_rn(0.f)));
+            words[11] = QuantizeLod<kFp8>(mip.positionLod);
 #pragma unroll
             for (int chunk = 0; chunk < 4; ++chunk)
                 ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);

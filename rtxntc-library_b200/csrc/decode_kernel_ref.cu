@@ -128,16 +128,11 @@ __device__ __forceinline__ __half2 QuantizeInputRef(__half2 x)
     return __hmul2_rn(y, __float2half2_rn(1.f / 127.5f));
 }
 
-// Clamped HGELU in binary16 (src/tin/tin_activation.h:88-92) followed by the quantiser of the next
-// layer's inputs, the int8 grid rint(y * 80) * 0.0125 (src/tin/tin_activation.h:94-99).
+// Clamped HGELU followed by the quantiser of the next layer's inputs, the int8 grid rint(y * 80) * 0.0125
+// (src/tin/tin_activation.h:94-99).
 __device__ __forceinline__ uint32_t ActivateRef(uint32_t bits)
 {
-    const __half2 x = AsHalf2(bits);
-    const __half2 third = __float2half2_rn(1 / 3.f);
-    const __half2 t = __hfma2_sat(third, x, __float2half2_rn(0.5f));
-    const __half2 m = __hmin2(x, __float2half2_rn(3.f));
-    const __half2 y = __hmul2_rn(m, t);
-    const __half2 p = __hmul2_rn(y, __float2half2_rn(80.f));
+    const __half2 p = __hmul2_rn(ClampedHgelu(AsHalf2(bits)), __float2half2_rn(80.f));
     // rint(p), p in [-15, 240]: the binary16 spacing is 1 in [1024, 2048)
     __half2 r = __hadd2_rn(p, __float2half2_rn(1536.f));
     r = __hadd2_rn(r, __float2half2_rn(-1536.f));
@@ -1095,15 +1090,10 @@ __device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
     return 0;
 }
 
-// Clamped HGELU in binary16 and the e4m3 code of the result: two codes in the low 16 bits.
-__device__ __forceinline__ uint32_t ActivateToE4m3(uint32_t bits)
+// Clamped HGELU of two pairs of accumulators and the e4m3 codes of the results.
+__device__ __forceinline__ uint32_t ActivateToE4m3(uint32_t first, uint32_t second)
 {
-    const __half2 x = AsHalf2(bits);
-    const __half2 third = __float2half2_rn(1 / 3.f);
-    const __half2 t = __hfma2_sat(third, x, __float2half2_rn(0.5f));
-    const __half2 m = __hmin2(x, __float2half2_rn(3.f));
-    const __half2 y = __hmul2_rn(m, t);
-    return uint32_t(__nv_cvt_halfraw2_to_fp8x2(static_cast<__half2_raw>(y), __NV_SATFINITE, __NV_E4M3));
+    return E4m3Codes(ClampedHgelu(AsHalf2(first)), ClampedHgelu(AsHalf2(second)));
 }
 
 template <int kLayer, int kConvert, typename Params>
@@ -1142,17 +1132,17 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
 #pragma unroll
         for (int c = 0; c < 2; ++c)
             storeChunk(c,
-                PackCodes<true>(ActivateToE4m3(low[8 * c]), ActivateToE4m3(low[8 * c + 1])),
-                PackCodes<true>(ActivateToE4m3(low[8 * c + 2]), ActivateToE4m3(low[8 * c + 3])),
-                PackCodes<true>(ActivateToE4m3(low[8 * c + 4]), ActivateToE4m3(low[8 * c + 5])),
-                PackCodes<true>(ActivateToE4m3(low[8 * c + 6]), ActivateToE4m3(low[8 * c + 7])));
+                ActivateToE4m3(low[8 * c], low[8 * c + 1]),
+                ActivateToE4m3(low[8 * c + 2], low[8 * c + 3]),
+                ActivateToE4m3(low[8 * c + 4], low[8 * c + 5]),
+                ActivateToE4m3(low[8 * c + 6], low[8 * c + 7]));
 #pragma unroll
         for (int c = 0; c < (kN - 32) / 16; ++c)
             storeChunk(2 + c,
-                PackCodes<true>(ActivateToE4m3(high[8 * c]), ActivateToE4m3(high[8 * c + 1])),
-                PackCodes<true>(ActivateToE4m3(high[8 * c + 2]), ActivateToE4m3(high[8 * c + 3])),
-                PackCodes<true>(ActivateToE4m3(high[8 * c + 4]), ActivateToE4m3(high[8 * c + 5])),
-                PackCodes<true>(ActivateToE4m3(high[8 * c + 6]), ActivateToE4m3(high[8 * c + 7])));
+                ActivateToE4m3(high[8 * c], high[8 * c + 1]),
+                ActivateToE4m3(high[8 * c + 2], high[8 * c + 3]),
+                ActivateToE4m3(high[8 * c + 4], high[8 * c + 5]),
+                ActivateToE4m3(high[8 * c + 6], high[8 * c + 7]));
         if (kLayer == 1)
             storeChunk(3, 0, 0, 0, 0); // layer 2 has 48 inputs: the rest of its second chunk must be zeros
     }
@@ -1418,8 +1408,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const
 
         {
             uint32_t words[16];
-            const uint32_t zeroWord = PackCodes<true>(QuantizeInputPair<true>(__float2half2_rn(0.f)),
-                                                      QuantizeInputPair<true>(__float2half2_rn(0.f)));
+            const uint32_t zeroWord = QuantizedZeros<true>();
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 words[i] = zeroWord; // unused feature slots hold quantised zeros (src/Inference.cu:49)
@@ -1436,13 +1425,11 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const
                 const float ex = __fmaf_rn(Frac(xf), 2.f, -1.f), ey = __fmaf_rn(Frac(yf), 2.f, -1.f);
                 const float ez = __fmaf_rn(Frac(__fadd_rn(xf, 0.25f)), 2.f, -1.f);
                 const float ew = __fmaf_rn(Frac(__fadd_rn(yf, 0.25f)), 2.f, -1.f);
-                words[8 + wave] = PackCodes<true>(QuantizeInputPair<true>(__floats2half2_rn(ex, ey)),
-                                                  QuantizeInputPair<true>(__floats2half2_rn(ez, ew)));
+                words[8 + wave] = QuantizeInputs<true>(__floats2half2_rn(ex, ey), __floats2half2_rn(ez, ew));
                 xf = __fmul_rn(xf, 2.f);
                 yf = __fmul_rn(yf, 2.f);
             }
-            words[11] = PackCodes<true>(QuantizeInputPair<true>(__float2half2_rn(mip.positionLod)),
-                                        QuantizeInputPair<true>(__float2half2_rn(0.f)));
+            words[11] = QuantizeLod<true>(mip.positionLod);
 #pragma unroll
             for (int chunk = 0; chunk < 4; ++chunk)
                 ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);

@@ -53,19 +53,27 @@ __device__ __forceinline__ uint32_t QuantizeInputPair(__half2 x)
     }
 }
 
-// Two quantised pairs -> four operand bytes.
+// Four network inputs -> four operand bytes.  (Not for constants: see E4m3Codes.)
 template <bool kFp8>
-__device__ __forceinline__ uint32_t PackCodes(uint32_t pair0, uint32_t pair1)
+__device__ __forceinline__ uint32_t QuantizeInputs(__half2 first, __half2 second)
 {
     if (kFp8)
-    {
-        // pair0 | pair1 << 16 (both are 16-bit values) as an integer multiply-add: it runs on the FMA
-        // pipe, leaving the busier ALU pipe to the conversions and min/max
-        uint32_t packed;
-        asm("mad.lo.u32 %0, %1, 65536, %2;" : "=r"(packed) : "r"(pair1), "r"(pair0));
-        return packed;
-    }
-    return __byte_perm(pair0, pair1, 0x6420);
+        return E4m3Codes(first, second);
+    return __byte_perm(QuantizeInputPair<kFp8>(first), QuantizeInputPair<kFp8>(second), 0x6420);
+}
+
+// The operand bytes of the inputs (value, value, 0, 0), and of four zeros.  (The e4m3 code of 0 is 0.)
+template <bool kFp8>
+__device__ __forceinline__ uint32_t QuantizeLod(float value)
+{
+    const uint32_t pair = QuantizeInputPair<kFp8>(__float2half2_rn(value));
+    return kFp8 ? pair : __byte_perm(pair, QuantizeInputPair<false>(__float2half2_rn(0.f)), 0x6420);
+}
+
+template <bool kFp8>
+__device__ __forceinline__ uint32_t QuantizedZeros()
+{
+    return kFp8 ? 0u : QuantizeInputs<false>(__float2half2_rn(0.f), __float2half2_rn(0.f));
 }
 
 // The bilinear blend of four taps and its mapping to [-1, 1].
@@ -112,7 +120,7 @@ __device__ __forceinline__ uint32_t BlendLayer(uint32_t p00, uint32_t p01, uint3
 {
     __half2 inputs[2];
     BlendPixels(p00, p01, p10, p11, taps, inputs);
-    return PackCodes<kFp8>(QuantizeInputPair<kFp8>(inputs[0]), QuantizeInputPair<kFp8>(inputs[1]));
+    return QuantizeInputs<kFp8>(inputs[0], inputs[1]);
 }
 
 // Two layers of one grid -> four quantised inputs each.
@@ -225,7 +233,7 @@ template <typename Tile>
 struct __align__(16) TileTables
 {
     TapTables<Tile> taps;
-    // positional-encoding operand bytes: x = {X0 w0, X1 w0, X0 w1, X1 w1}, y = {X0 w2, X1 w2, 0, 0}
+    // positional-encoding operand bytes: x = {X0 w0, X1 w0, X0 w1, X1 w1}, y = {X0 w2, X1 w2, unused}
     uint2 colEnc[Tile::kWidth];
     uint2 rowEnc[Tile::kHeight];
     uint32_t lodWord;  // operand bytes of inputs 44..47: lod, lod, 0, 0
@@ -346,23 +354,23 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
         const int coordinate = rows ? min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1)
                                     : min(tileX0 + (lane & (Tile::kWidth - 1)), mip.width - 1);
         float f = __fmul_rn(float(coordinate), mip.positionScale);
-        uint32_t q[3];
+        __half2 waves[3];
 #pragma unroll
         for (int wave = 0; wave < 3; ++wave)
         {
             const float e0 = __fmaf_rn(Frac(f), 2.f, -1.f);
             const float e1 = __fmaf_rn(Frac(__fadd_rn(f, 0.25f)), 2.f, -1.f);
-            q[wave] = QuantizeInputPair<kFp8>(__floats2half2_rn(e0, e1));
+            waves[wave] = __floats2half2_rn(e0, e1);
             f = __fmul_rn(f, 2.f);
         }
-        const uint2 enc = make_uint2(PackCodes<kFp8>(q[0], q[1]), PackCodes<kFp8>(q[2], 0));
+        const uint2 enc = make_uint2(QuantizeInputs<kFp8>(waves[0], waves[1]),
+                                     kFp8 ? QuantizeInputPair<kFp8>(waves[2]) : QuantizeInputs<kFp8>(waves[2], waves[2]));
         if (!rows && lane < Tile::kWidth)
             stage.tables.colEnc[lane] = enc;
         if (rows && lane < Tile::kHeight)
             stage.tables.rowEnc[lane] = enc;
         if (rows && lane == Tile::kHeight)
-            stage.tables.lodWord = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(mip.positionLod)),
-                                                   QuantizeInputPair<kFp8>(__float2half2_rn(0.f)));
+            stage.tables.lodWord = QuantizeLod<kFp8>(mip.positionLod);
     }
     PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo,
         tileX0, tileY0, lane, warp, tablesValid);
@@ -394,7 +402,7 @@ __device__ __forceinline__ uint32_t BlendLayer(uint2 l00, uint2 l01, uint2 l10, 
     b = __hfma2(AsHalf2(l11.y), w11, b);
     a = __hfma2(a, two, minusOne);
     b = __hfma2(b, two, minusOne);
-    return PackCodes<kFp8>(QuantizeInputPair<kFp8>(a), QuantizeInputPair<kFp8>(b));
+    return QuantizeInputs<kFp8>(a, b);
 }
 
 // Inputs 0..15 or 16..31 of one texel from the staged footprint of one grid.
@@ -472,8 +480,7 @@ __device__ __forceinline__ void BuildInputs(const KernelParams& params, const Ke
     const Context& ctx, int tileColumn, int tileRow)
 {
     uint32_t words[16];
-    const uint32_t zeroWord = PackCodes<kFp8>(QuantizeInputPair<kFp8>(__float2half2_rn(0.f)),
-                                              QuantizeInputPair<kFp8>(__float2half2_rn(0.f)));
+    const uint32_t zeroWord = QuantizedZeros<kFp8>();
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         words[i] = zeroWord; // unused feature slots hold quantised zeros (src/Inference.cu:49)

@@ -195,6 +195,31 @@ __device__ __forceinline__ __half2 AsHalf2(uint32_t v)
     return *reinterpret_cast<__half2*>(&v);
 }
 
+// Clamped HGELU in binary16 (src/tin/tin_activation.h:88-92).
+__device__ __forceinline__ __half2 ClampedHgelu(__half2 x)
+{
+    const __half2 t = __hfma2_sat(__float2half2_rn(1 / 3.f), x, __float2half2_rn(0.5f));
+    return __hmul2_rn(__hmin2(x, __float2half2_rn(3.f)), t);
+}
+
+// Two pairs of values -> four e4m3 codes (round to nearest even, saturating).  The conversions fill the two halves of one register, which
+// leaves nothing to extend or to join (with 16-bit results widened and joined by a multiply-add a texel of an FP8 network took 987
+// instructions instead of 891: 4096 x 4096 779 -> 719 us, 16.7 M queries 692 -> 648).
+// Not for constants: of E4m3Codes(0, 0) nvcc 12.9 left part of the word undefined.
+__device__ __forceinline__ uint32_t E4m3Codes(__half2 first, __half2 second)
+{
+    uint32_t codes;
+    asm("{\n\t"
+        ".reg .b16 low, high;\n\t"
+        "cvt.rn.satfinite.e4m3x2.f16x2 low, %1;\n\t"
+        "cvt.rn.satfinite.e4m3x2.f16x2 high, %2;\n\t"
+        "mov.b32 %0, {low, high};\n\t"
+        "}"
+        : "=r"(codes)
+        : "r"(AsU32(first)), "r"(AsU32(second)));
+    return codes;
+}
+
 // Inf / NaN -> 0 in the channel pairs of one texel (src/Inference.cu:125-126, src/CudaUtils.h:30-35).
 // A binary16 value times zero is a zero unless the value is an infinity or a NaN, so one fused
 // multiply-add per pair into a common sum detects whether anything has to be done at all.
