@@ -82,14 +82,15 @@ constexpr int kRefInt8NetworkBytes = 17408; // ... what the Int8 kernels copy to
 // layers 2 and 3.
 constexpr int kRefOperandBytes = 128 * 96;
 // Reference-numerics kernels: a CTA is up to eight chains of 128 threads - 64 tensor-memory columns and 64 registers a thread each, which
-// fills an SM - that share the network in shared memory and nothing else.  Each walks tiles of its own, 16 x 8 texels, with its
-// own tables and footprints, and meets only its own threads in barriers.
+// fills an SM - that share the network in shared memory and nothing else.  Each walks tiles of its own, 16 x 8 texels, in runs of
+// up to four side by side, with its own tables and footprints, and meets only its own threads in barriers.
 constexpr int kChainTileWidth = 16;
 constexpr int kChainTileHeight = 8;
+constexpr int kMaxRunTiles = 4; // ... tiles of a run, see KernelMip::runTiles
 constexpr int kMaxChains = 8;
 constexpr int kMaxThreadsPerCta = 128 * kMaxChains;
 // Footprints of a chain: what a tile covers at a grid-to-mip ratio of 1 (high-res: 18 x 10 pixels of 24 bytes) and 1/2
-// (low-res: 10 x 6).
+// (low-res: 10 x 6), or a run of tiles at a smaller one.
 constexpr int kRefFootprintHiBytes = 4352;
 constexpr int kRefFootprintLoBytes = 1536;
 constexpr int kRefInt8FootprintHiBytes = kRefFootprintHiBytes;
@@ -113,8 +114,11 @@ struct KernelMip
     unsigned long long outOffset;
     float invWidth, invHeight;
     float positionScale, positionLod;
+    // Where the mip stands in the launch's list of work, and how much of it a row of tiles has: counted in tiles (exact accumulation)
+    // or in runs of tiles (reference numerics).
     int firstTile, tilesX;
     unsigned tilesXMagic; // ceil(2^32 / tilesX): local / tilesX == umulhi(local, magic) for every tile of the mip; 0: divide
+    int runTiles;         // tiles side by side whose tables and footprints are prepared together (1, 2 or 4)
     int staged;      // the tile footprints of both grids fit into shared memory
     int strideBytes; // bytes per staged latent pixel: 8 per layer, padded to an odd multiple of 8 (8, 24, 24, 40) so that
                      // the 8-byte reads of neighbouring pixels fall into different shared-memory banks

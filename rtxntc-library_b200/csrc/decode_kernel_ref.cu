@@ -143,20 +143,20 @@ __device__ __forceinline__ uint32_t ActivateRef(uint32_t bits)
 // Shared memory
 // ---------------------------------------------------------------------------------------------
 
-// Per-tile lookup tables: the taps (shared with the other kernels) and the positional encoding as
+// Lookup tables of a run of tiles: the taps (shared with the other kernels) and the positional encoding as
 // quantised binary16 pairs.
 struct __align__(16) RefTileTables
 {
     TapTables<ChainTile> taps;
     // positional encoding: word w = (wave w phase 0, wave w phase 0.25)
-    uint4 colEnc[ChainTile::kWidth];
+    uint32_t colEnc[3][ChainTile::kColumns];
     uint4 rowEnc[ChainTile::kHeight];
     uint32_t lodPair;   // (lod, lod)
     uint32_t zeroPair;  // (quantised 0, quantised 0)
     uint32_t pad[2];
 };
 
-// What a chain prepares per tile.
+// What a chain prepares per run of tiles.
 template <typename Tables, int kHiBytes, int kLoBytes>
 struct __align__(16) ChainStage
 {
@@ -166,7 +166,7 @@ struct __align__(16) ChainStage
 };
 
 // What the threads of a chain keep of their texel's place in a tile while the tables stay the same: with power-of-two sizes that is from the
-// first inner tile of a mip on.  The positional encoding stays in the operand row, whose last chunks only the input stage writes.  (Worked out per
+// first inner run of a mip on, and the tiles of a run differ by whole latent pixels (`shift` in DecodeRuns).  The positional encoding stays in the operand row, whose last chunks only the input stage writes.  (Worked out per
 // tile - eight products and eight conversions - a 4096 x 4096 FP8 set took 867 us instead of 851.)
 struct __align__(16) TexelTables
 {
@@ -180,15 +180,15 @@ struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8FootprintHiByt
 };
 
 template <typename Stage>
-__device__ __forceinline__ void PrepareTexel(Stage& stage, int texel, int tileColumn, int tileRow)
+__device__ __forceinline__ void PrepareTexel(Stage& stage, int texel, int column, int tileRow)
 {
     uint32_t offsets[4];
 #pragma unroll
     for (int grid = 0; grid < 2; ++grid)
     {
-        const int4 col = stage.tables.taps.colTap[grid][tileColumn];
+        const int2 col = stage.tables.taps.colTap[grid][column];
         const int4 row = stage.tables.taps.rowTap[grid][tileRow];
-        const float dx = __int_as_float(col.y), dxn = __int_as_float(col.z);
+        const float dx = __int_as_float(col.y), dxn = __fsub_rn(1.f, dx);
         const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
         // src/FeatureGridDevice.h:46-49
         const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);
@@ -200,9 +200,10 @@ __device__ __forceinline__ void PrepareTexel(Stage& stage, int texel, int tileCo
     stage.texels.taps[texel] = make_uint4(offsets[0], offsets[1], offsets[2], offsets[3]);
 }
 
-// Calls blend(grid, layer, four taps, four weights) for the latents of a texel in the staged footprints.
+// Calls blend(grid, layer, four taps, four weights) for the latents of a texel in the staged footprints.  `shift`: bytes the taps of a
+// grid lie past those in TexelTables.
 template <int kLayers, typename Stage, typename Blend>
-__device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, Blend blend)
+__device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, int2 shift, Blend blend)
 {
     const uint4 taps = stage.texels.taps[texel];
     const int stride = StrideBytes<kLayers>(mip);
@@ -210,7 +211,7 @@ __device__ __forceinline__ void GatherTexel(const KernelParams& params, const Ke
     for (int grid = 0; grid < 2; ++grid)
     {
         const uint4 w = stage.texels.weights[grid][texel];
-        const uint8_t* tap00 = grid ? stage.footprintLo + taps.z : stage.footprintHi + taps.x;
+        const uint8_t* tap00 = grid ? stage.footprintLo + (taps.z + shift.y) : stage.footprintHi + (taps.x + shift.x);
         const uint8_t* tap10 = tap00 + (grid ? taps.w : taps.y);
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
@@ -295,41 +296,33 @@ struct RefTileContext
 // Inputs
 // ---------------------------------------------------------------------------------------------
 
-// Builds the tile's lookup tables and stages the latent footprint of both grids in shared memory
-// (`tablesValid`: the tables already hold this tile's values, see PrepareTaps).  `warp`: of the chain's four.
+// Builds the lookup tables of a run of tiles, `columns` wide, and stages the latent footprint of both grids in shared memory
+// (`tablesValid`: the tables already hold this run's values, see PrepareTaps).  `warp`: of the chain's four.
 template <int kLayers = 0>
 __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
-    int tileX0, int tileY0, int lane, int warp, bool tablesValid)
+    int tileX0, int tileY0, int columns, int lane, int warp, bool tablesValid)
 {
     if (!tablesValid && warp >= 2 && warp < 4)
     {
-        // positional encoding (src/RegressionKernels.h:59-85): warp 2 the x part per column, warp 3
-        // the y part per row, quantised exactly as the per-texel inputs would be
-        const bool rows = warp == 3;
-        const int coordinate = rows ? min(tileY0 + (lane & (ChainTile::kHeight - 1)), mip.rowEnd - 1)
-                                    : min(tileX0 + (lane & (ChainTile::kWidth - 1)), mip.width - 1);
-        float f = __fmul_rn(float(coordinate), mip.positionScale);
-        uint32_t q[3];
+        EncodePositions<ChainTile>(mip, tileX0, tileY0, columns, lane, warp, [&](const __half2 (&waves)[3], bool rows, int index) {
+            const uint32_t q[3] = {AsU32(QuantizeInputRef(waves[0])), AsU32(QuantizeInputRef(waves[1])), AsU32(QuantizeInputRef(waves[2]))};
+            if (!rows)
+            {
 #pragma unroll
-        for (int wave = 0; wave < 3; ++wave)
-        {
-            const float e0 = __fmaf_rn(Frac(f), 2.f, -1.f);
-            const float e1 = __fmaf_rn(Frac(__fadd_rn(f, 0.25f)), 2.f, -1.f);
-            q[wave] = AsU32(QuantizeInputRef(__floats2half2_rn(e0, e1)));
-            f = __fmul_rn(f, 2.f);
-        }
-        if (!rows && lane < ChainTile::kWidth)
-            stage.tables.colEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
-        if (rows && lane < ChainTile::kHeight)
-            stage.tables.rowEnc[lane] = make_uint4(q[0], q[1], q[2], 0);
-        if (rows && lane == ChainTile::kHeight)
-        {
-            stage.tables.lodPair = AsU32(QuantizeInputRef(__float2half2_rn(mip.positionLod)));
-            stage.tables.zeroPair = AsU32(QuantizeInputRef(__float2half2_rn(0.f)));
-        }
+                for (int wave = 0; wave < 3; ++wave)
+                    stage.tables.colEnc[wave][index] = q[wave];
+            }
+            else if (index < ChainTile::kHeight)
+                stage.tables.rowEnc[index] = make_uint4(q[0], q[1], q[2], 0);
+            else if (index == ChainTile::kHeight)
+            {
+                stage.tables.lodPair = AsU32(QuantizeInputRef(__float2half2_rn(mip.positionLod)));
+                stage.tables.zeroPair = AsU32(QuantizeInputRef(__float2half2_rn(0.f)));
+            }
+        });
     }
     PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, tileX0,
-        tileY0, lane, warp, tablesValid);
+        tileY0, columns, lane, warp, tablesValid);
 }
 
 // Four inputs of one latent layer from the four taps, as two binary16 pairs.
@@ -383,11 +376,11 @@ __device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plan
     BlendPixelsRef(p00, p01, p10, p11, taps, words);
 }
 
-// The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.  `known`: TexelTables and the
-// row's last two chunks are those of an earlier tile with the same tables.
+// The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.  `column`: in the run.  `known`: TexelTables
+// and the row's last two chunks are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
 template <int kLayers = 0>
 __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
-    const RefTileContext& ctx, int tileColumn, int tileRow, bool known)
+    const RefTileContext& ctx, int column, int tileRow, bool known, int2 shift)
 {
     uint32_t words[16];
     const uint32_t zeroPair = stage.tables.zeroPair;
@@ -398,8 +391,8 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
     if (mip.staged)
     {
         if (!known)
-            PrepareTexel(stage, ctx.tid & 127, tileColumn, tileRow);
-        GatherTexel<kLayers>(params, mip, stage, ctx.tid & 127, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00,
+            PrepareTexel(stage, ctx.tid & 127, column, tileRow);
+        GatherTexel<kLayers>(params, mip, stage, ctx.tid & 127, shift, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00,
             __half2 w01, __half2 w10, __half2 w11) { BlendLayerRef(l00, l01, l10, l11, w00, w01, w10, w11, words + 8 * grid + 2 * layer); });
     }
     else
@@ -427,7 +420,7 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
     if (!known)
     {
         // positional encoding: per wave the inputs (x phase 0, y phase 0, x phase 0.25, y phase 0.25)
-        const uint4 cx = stage.tables.colEnc[tileColumn];
+        const uint3 cx = make_uint3(stage.tables.colEnc[0][column], stage.tables.colEnc[1][column], stage.tables.colEnc[2][column]);
         const uint4 ry = stage.tables.rowEnc[tileRow];
         ctx.rowChunk[4 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5410), __byte_perm(cx.x, ry.x, 0x7632),
                                            __byte_perm(cx.y, ry.y, 0x5410), __byte_perm(cx.y, ry.y, 0x7632));
@@ -671,11 +664,19 @@ __device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const R
 // The kernels
 // ---------------------------------------------------------------------------------------------
 
-template <int kConvert, int kLayers>
-__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __grid_constant__ KernelParams params)
+// A chain's share of a launch.  `Chain` says how its tiles are prepared, fed and consumed.
+//
+// The unit of work is a run of up to kMaxRunTiles tiles side by side (KernelMip::runTiles).  Tables and footprints are made once per run, by all
+// four warps, under the products of the run before: the footprints of neighbouring tiles overlap (with a grid at a quarter of the mip's resolution
+// four tiles have 72 + 30 latent pixels, one has 24 + 12), the latents' way from the L2 is waited for once, and finding the place of the
+// work is paid for once.
+template <typename Chain, int kConvert, int kLayers>
+__device__ __forceinline__ void DecodeRuns(const KernelParams& params)
 {
     extern __shared__ __align__(128) unsigned char dynamicShared[];
-    RefSharedStorage& shared = *reinterpret_cast<RefSharedStorage*>(dynamicShared);
+    using Storage = typename Chain::Storage;
+    using Stage = typename Chain::Stage;
+    Storage& shared = *reinterpret_cast<Storage*>(dynamicShared);
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -683,9 +684,8 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
     const int chain = warp >> 2, role = WarpRole(warp);
     const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
-    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    Chain::Setup(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
     uint32_t phase = 0;
-    int aborted = 0;  // some thread of the chain gave up (uniform over the chain)
 
     RefTileContext ctx;
     ctx.tid = tid;
@@ -693,66 +693,73 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
     ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
     ctx.barrier = SharedAddress(&shared.barrier[chain]);
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * (sizeof(Storage::operandA) / kMaxChains)) + (tid & 127);
 
-    RefStage& stage = StageOf<RefStage>(shared, chain);
-    struct TilePlace
-    {
-        int mipIndex, tileX0, tileY0;
+    Stage& stage = StageOf<Stage>(shared, chain);
+    // the first chains of all CTAs take the first runs, so that a launch of few spreads over the SMs
+    const uint32_t runStep = (blockDim.x >> 7) * gridDim.x;
+    uint32_t run = blockIdx.x + uint32_t(chain) * gridDim.x;
+    int mipIndex = 0, x0 = 0, y0 = 0; // the next tile's mip and place
+    int tilesLeft = 0;                // of the run
+    int column = 0;                   // of the next tile's first texel in the run
+    int2 shift = make_int2(0, 0);     // bytes the next tile's taps lie past those in TexelTables
+    bool keeps = false;               // the run's tables serve others of its mip, and its later tiles what the threads keep of the first
+    bool known = false;               // the tables, and what the threads keep of them, are already the next tile's
+    int tablesMip = -1;               // mip whose tables are in shared memory and valid for every inner run of it
+    auto prepareRun = [&]() {
+        while (mipIndex + 1 < params.numMips && run >= uint32_t(params.mips[mipIndex + 1].firstTile))
+            ++mipIndex; // runs are visited in increasing order, so the search resumes at the current mip
+        const KernelMip& mip = params.mips[mipIndex];
+        const int local = int(run) - mip.firstTile;
+        const int row = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
+        const int columns = mip.runTiles * kChainTileWidth;
+        x0 = (local - row * mip.tilesX) * columns;
+        y0 = mip.rowBegin + row * kChainTileHeight;
+        tilesLeft = min(mip.runTiles, (mip.width - x0 + kChainTileWidth - 1) / kChainTileWidth);
+        column = 0;
+        shift = make_int2(0, 0);
+        keeps = TileKeepsTables<ChainTile>(mip, x0, y0, columns);
+        // the tables of the previous run serve this one too when both lie inside the same mip with invariant tables
+        known = keeps && mipIndex == tablesMip;
+        Chain::template Prepare<kLayers>(params, mip, stage, x0, y0, columns, lane, role, known);
+        tablesMip = keeps ? mipIndex : -1;
     };
-    auto locate = [&](uint32_t tile, int fromMip) {
-        TilePlace place;
-        place.mipIndex = fromMip;
-        while (place.mipIndex + 1 < params.numMips && tile >= uint32_t(params.mips[place.mipIndex + 1].firstTile))
-            ++place.mipIndex;
-        const KernelMip& mip = params.mips[place.mipIndex];
-        const int local = int(tile) - mip.firstTile;
-        const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
-        place.tileX0 = (local - tileY * mip.tilesX) * kChainTileWidth;
-        place.tileY0 = mip.rowBegin + tileY * kChainTileHeight;
-        return place;
-    };
-
-    // the first chains of all CTAs take the first tiles, so that a launch of few tiles spreads over the SMs
-    const uint32_t chains = blockDim.x >> 7;
-    uint32_t tile = blockIdx.x + uint32_t(chain) * gridDim.x;
-    TilePlace place{0, 0, 0};
-    bool known = false; // the tables, and what the threads keep of them, are already the tile's
-    int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
-    if (tile < uint32_t(params.totalTiles))
+    if (run < uint32_t(params.totalTiles))
     {
-        place = locate(tile, 0);
-        PrepareTileRef<kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, false);
-        tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
+        prepareRun();
         ChainBarrier(chain);
     }
-    while (tile < uint32_t(params.totalTiles))
+    while (tilesLeft)
     {
-        const KernelMip& mip = params.mips[place.mipIndex];
-        ctx.tile = int(tile);
-        ctx.x = place.tileX0 + tileColumn;
-        ctx.y = place.tileY0 + tileRow;
-        BuildInputsRef<kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
+        const KernelMip& mip = params.mips[mipIndex];
+        ctx.tile = int(run);
+        ctx.x = x0 + tileColumn;
+        ctx.y = y0 + tileRow;
+        Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known, shift);
 
-        // layer 0; while the tensor core works on it, prepare the chain's NEXT tile (its tables and
-        // footprints replace this tile's, which nobody reads after the barrier inside IssueLayerRef)
-        aborted = IssueLayerRef<0>(ctx);
-        if (aborted)
-            break;
-        const uint32_t nextTile = tile + chains * gridDim.x;
-        if (nextTile < uint32_t(params.totalTiles))
+        // layer 0; while the tensor core works on it, prepare the chain's NEXT run (its tables and
+        // footprints replace this run's, which nobody reads after the barrier inside Issue)
+        if (Chain::template Issue<0>(ctx))
+            break; // some thread of the chain gave up on a wait
+        if (--tilesLeft)
         {
-            place = locate(nextTile, place.mipIndex);
-            // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
-            known = keepsTables && place.mipIndex == tablesMip;
-            PrepareTileRef<kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
-            tablesMip = keepsTables ? place.mipIndex : -1;
+            x0 += kChainTileWidth;
+            column += kChainTileWidth;
+            known = keeps;
+            if (keeps)
+            {
+                shift.x += mip.hiStepX * StrideBytes<kLayers>(mip);
+                shift.y += mip.loStepX * StrideBytes<kLayers>(mip);
+            }
         }
-        ConsumeLayerRef<0, kConvertNone>(params, ctx, phase);
+        else if ((run += runStep) < uint32_t(params.totalTiles))
+            prepareRun();
+        Chain::template Consume<0, kConvertNone>(params, ctx, phase);
 
-        RunLayerRef<1, kConvertNone>(params, ctx, phase);
-        RunLayerRef<2, kConvertNone>(params, ctx, phase);
+        Chain::template Issue<1>(ctx);
+        Chain::template Consume<1, kConvertNone>(params, ctx, phase);
+        Chain::template Issue<2>(ctx);
+        Chain::template Consume<2, kConvertNone>(params, ctx, phase);
         {
             // where the texel goes (worked out only now: nothing of it has to stay in registers through the
             // layers); the element index inside a mip fits 32 bits (checked on the host)
@@ -776,11 +783,53 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __
                 ctx.storeBytes = mip.storeBytes;
             }
         }
-        RunLayerRef<3, kConvert>(params, ctx, phase);
-        tile = nextTile;
+        Chain::template Issue<3>(ctx);
+        Chain::template Consume<3, kConvert>(params, ctx, phase);
     }
+    Chain::Teardown(shared, ctx, phase, tid, warp);
+}
 
-    TeardownCtaRef(shared, ctx, phase, tid, warp);
+// A chain of an Int8 network: binary16 operands.
+struct Int8Chain
+{
+    using Storage = RefSharedStorage;
+    using Stage = RefStage;
+    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp)
+    {
+        SetupCtaRef(shared, network, status, polls, tid, warp);
+    }
+    static __device__ __forceinline__ void Teardown(Storage& shared, const RefTileContext& ctx, uint32_t phase, int tid, int warp)
+    {
+        TeardownCtaRef(shared, ctx, phase, tid, warp);
+    }
+    template <int kLayers>
+    static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
+        int lane, int role, bool tablesValid)
+    {
+        PrepareTileRef<kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid);
+    }
+    template <int kLayers>
+    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const RefTileContext& ctx,
+        int column, int tileRow, bool known, int2 shift)
+    {
+        BuildInputsRef<kLayers>(params, mip, stage, ctx, column, tileRow, known, shift);
+    }
+    template <int kLayer>
+    static __device__ __forceinline__ int Issue(RefTileContext& ctx)
+    {
+        return IssueLayerRef<kLayer>(ctx);
+    }
+    template <int kLayer, int kConvert>
+    static __device__ __forceinline__ void Consume(const KernelParams& params, const RefTileContext& ctx, uint32_t& phase)
+    {
+        ConsumeLayerRef<kLayer, kConvert>(params, ctx, phase);
+    }
+};
+
+template <int kConvert, int kLayers>
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRef(const __grid_constant__ KernelParams params)
+{
+    DecodeRuns<Int8Chain, kConvert, kLayers>(params);
 }
 
 // Inference on sample with the reference's numerics: one thread per query (u, v, lod) -> the texel
@@ -951,29 +1000,29 @@ struct __align__(128) RefFp8SharedStorage
 };
 static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(RefFp8Stage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
-// The 64-byte operand row of a texel.  `known`: TexelTables and the row's last two chunks are those of an earlier tile with the same tables.
+// The 64-byte operand row of a texel, as BuildInputsRef.
 template <int kLayers>
 __device__ __forceinline__ void BuildInputsRefFp8(const KernelParams& params, const KernelMip& mip, RefFp8Stage& stage,
-    const RefTileContext& ctx, int tileColumn, int tileRow, bool known)
+    const RefTileContext& ctx, int column, int tileRow, bool known, int2 shift)
 {
     if (!mip.staged)
     {
-        BuildInputs<true, true, kLayers>(params, mip, stage, ctx, tileColumn, tileRow);
+        BuildInputs<true, true, kLayers>(params, mip, stage, ctx, column, tileRow);
         return;
     }
     const int texel = ctx.tid & 127;
     if (!known)
     {
-        PrepareTexel(stage, texel, tileColumn, tileRow);
+        PrepareTexel(stage, texel, column, tileRow);
         // positional encoding: interleave the column's x bytes with the row's y bytes
-        const uint2 cx = stage.tables.colEnc[tileColumn];
+        const uint2 cx = stage.tables.colEnc[column];
         const uint2 ry = stage.tables.rowEnc[tileRow];
         ctx.rowChunk[2 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5140), __byte_perm(cx.x, ry.x, 0x7362),
                                            __byte_perm(cx.y, ry.y, 0x5140), stage.tables.lodWord);
         ctx.rowChunk[3 * 128] = make_uint4(0, 0, 0, 0); // K padding
     }
     uint32_t words[8] = {0, 0, 0, 0, 0, 0, 0, 0}; // unused feature slots hold zeros (src/Inference.cu:49)
-    GatherTexel<kLayers>(params, mip, stage, texel, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00, __half2 w01,
+    GatherTexel<kLayers>(params, mip, stage, texel, shift, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00, __half2 w01,
         __half2 w10, __half2 w11) { words[4 * grid + layer] = BlendLayer<true>(l00, l01, l10, l11, w00, w01, w10, w11); });
     ctx.rowChunk[0] = make_uint4(words[0], words[1], words[2], words[3]);
     ctx.rowChunk[128] = make_uint4(words[4], words[5], words[6], words[7]);
@@ -1240,111 +1289,47 @@ __device__ __forceinline__ void TeardownCtaRefFp8(RefFp8SharedStorage& shared, c
         TmemFree(shared.tmemBase, (blockDim.x >> 7) * kTmemColumnsPerHalf);
 }
 
+// A chain of an FP8 network: 8-bit operands, the input stage of the exact-accumulation kernel's 64-byte rows of codes.
+struct Fp8Chain
+{
+    using Storage = RefFp8SharedStorage;
+    using Stage = RefFp8Stage;
+    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp)
+    {
+        SetupCtaRefFp8(shared, network, status, polls, tid, warp);
+    }
+    static __device__ __forceinline__ void Teardown(Storage& shared, const RefTileContext& ctx, uint32_t phase, int tid, int warp)
+    {
+        TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
+    }
+    template <int kLayers>
+    static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
+        int lane, int role, bool tablesValid)
+    {
+        PrepareTile<ChainTile, true, true, kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid);
+    }
+    template <int kLayers>
+    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const RefTileContext& ctx,
+        int column, int tileRow, bool known, int2 shift)
+    {
+        BuildInputsRefFp8<kLayers>(params, mip, stage, ctx, column, tileRow, known, shift);
+    }
+    template <int kLayer>
+    static __device__ __forceinline__ int Issue(RefTileContext& ctx)
+    {
+        return IssueLayerRefFp8<kLayer>(ctx);
+    }
+    template <int kLayer, int kConvert>
+    static __device__ __forceinline__ void Consume(const KernelParams& params, const RefTileContext& ctx, uint32_t& phase)
+    {
+        ConsumeLayerRefFp8<kLayer, kConvert>(params, ctx, phase);
+    }
+};
+
 template <int kConvert, int kLayers>
 __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const __grid_constant__ KernelParams params)
 {
-    extern __shared__ __align__(128) unsigned char dynamicShared[];
-    RefFp8SharedStorage& shared = *reinterpret_cast<RefFp8SharedStorage*>(dynamicShared);
-
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = tid >> 5;
-    const int chain = warp >> 2, role = WarpRole(warp);
-    const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
-
-    SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
-    uint32_t phase = 0;
-    int aborted = 0;
-
-    RefTileContext ctx;
-    ctx.tid = tid;
-    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier[chain]);
-    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kOperandBytes) + (tid & 127);
-
-    RefFp8Stage& stage = StageOf<RefFp8Stage>(shared, chain);
-    struct TilePlace
-    {
-        int mipIndex, tileX0, tileY0;
-    };
-    auto locate = [&](uint32_t tile, int fromMip) {
-        TilePlace place;
-        place.mipIndex = fromMip;
-        while (place.mipIndex + 1 < params.numMips && tile >= uint32_t(params.mips[place.mipIndex + 1].firstTile))
-            ++place.mipIndex;
-        const KernelMip& mip = params.mips[place.mipIndex];
-        const int local = int(tile) - mip.firstTile;
-        const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
-        place.tileX0 = (local - tileY * mip.tilesX) * kChainTileWidth;
-        place.tileY0 = mip.rowBegin + tileY * kChainTileHeight;
-        return place;
-    };
-
-    // the first chains of all CTAs take the first tiles, so that a launch of few tiles spreads over the SMs
-    const uint32_t chains = blockDim.x >> 7;
-    uint32_t tile = blockIdx.x + uint32_t(chain) * gridDim.x;
-    TilePlace place{0, 0, 0};
-    bool known = false; // the tables, and what the threads keep of them, are already the tile's
-    int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
-    if (tile < uint32_t(params.totalTiles))
-    {
-        place = locate(tile, 0);
-        PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, false);
-        tablesMip = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0) ? place.mipIndex : -1;
-        ChainBarrier(chain);
-    }
-    while (tile < uint32_t(params.totalTiles))
-    {
-        const KernelMip& mip = params.mips[place.mipIndex];
-        ctx.tile = int(tile);
-        ctx.x = place.tileX0 + tileColumn;
-        ctx.y = place.tileY0 + tileRow;
-        // the e4m3 input stage is the one of the exact-accumulation kernel (64-byte rows of codes)
-        BuildInputsRefFp8<kLayers>(params, mip, stage, ctx, tileColumn, tileRow, known);
-
-        aborted = IssueLayerRefFp8<0>(ctx);
-        if (aborted)
-            break;
-        const uint32_t nextTile = tile + chains * gridDim.x;
-        if (nextTile < uint32_t(params.totalTiles))
-        {
-            place = locate(nextTile, place.mipIndex);
-            // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = TileKeepsTables<ChainTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0);
-            known = keepsTables && place.mipIndex == tablesMip;
-            PrepareTile<ChainTile, true, true, kLayers>(params, params.mips[place.mipIndex], stage, place.tileX0, place.tileY0, lane, role, known);
-            tablesMip = keepsTables ? place.mipIndex : -1;
-        }
-        ConsumeLayerRefFp8<0, kConvertNone>(params, ctx, phase);
-
-        RunLayerRefFp8<1, kConvertNone>(params, ctx, phase);
-        RunLayerRefFp8<2, kConvertNone>(params, ctx, phase);
-        {
-            // where the texel goes (worked out only now: nothing of it has to stay in registers through the layers)
-            const bool planar = params.outputLayout == kLayoutPlanarPairs;
-            const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
-                                          : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
-            const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
-            if constexpr (kConvert != kConvertNone)
-            {
-                const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
-                const size_t component = size_t(mip.outOffset) + size_t(pixelIndex) * size_t(params.conversion.dstChannels);
-                unsigned char* bytes = reinterpret_cast<unsigned char*>(params.out) + component * BytesPerComponent(params.conversion.format);
-                ctx.out = inside ? reinterpret_cast<uint32_t*>(bytes) : nullptr;
-                ctx.outStepWords = pixelIndex;
-            }
-            else
-            {
-                ctx.out = inside ? reinterpret_cast<uint32_t*>(params.out + mip.outOffset + first) : nullptr;
-                ctx.outStepWords = planar ? uint32_t(mip.width) : 1u;
-                ctx.storeBytes = mip.storeBytes;
-            }
-        }
-        RunLayerRefFp8<3, kConvert>(params, ctx, phase);
-        tile = nextTile;
-    }
-    TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
+    DecodeRuns<Fp8Chain, kConvert, kLayers>(params);
 }
 
 // Inference on sample for FP8 networks (8-bit operands): one thread per query, taps read straight

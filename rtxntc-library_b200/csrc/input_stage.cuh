@@ -196,35 +196,40 @@ __device__ __forceinline__ void SampleInterleaved(const uint16_t* __restrict__ h
     }
 }
 
-// The unit of texels whose tables and footprints are prepared together, and the warps that do it: all eight of a CTA on a
-// 32 x 8 tile (exact accumulation), or the four of a chain on a 16 x 8 tile of its own (reference numerics).
+// The unit of texels that a group of threads works on, thread = texel, the warps of the group, and the most columns whose tables and
+// footprints they prepare together: all eight warps of a CTA on a 32 x 8 tile (exact accumulation), or the four of a chain on 16 x 8 tiles
+// of its own, prepared in runs of up to four side by side (reference numerics).
 struct WideTile
 {
-    static constexpr int kWidth = kTileWidth, kHeight = kTileHeight, kWarps = 8, kWidthLog2 = 5, kHeightLog2 = 3;
+    using ColumnTap = int4;
+    static constexpr int kWidth = kTileWidth, kHeight = kTileHeight, kWarps = 8, kWidthLog2 = 5, kHeightLog2 = 3, kColumns = kWidth;
 };
 struct ChainTile
 {
-    static constexpr int kWidth = kChainTileWidth, kHeight = kChainTileHeight, kWarps = 4, kWidthLog2 = 4, kHeightLog2 = 3;
+    using ColumnTap = int2;
+    static constexpr int kWidth = kChainTileWidth, kHeight = kChainTileHeight, kWarps = 4, kWidthLog2 = 4, kHeightLog2 = 3,
+                         kColumns = kWidth * kMaxRunTiles;
 };
 static_assert(WideTile::kWidth == 1 << WideTile::kWidthLog2 && WideTile::kHeight == 1 << WideTile::kHeightLog2 &&
                   ChainTile::kWidth == 1 << ChainTile::kWidthLog2 && ChainTile::kHeight == 1 << ChainTile::kHeightLog2 &&
+                  WideTile::kColumns <= 16 * WideTile::kWarps && ChainTile::kColumns <= 16 * ChainTile::kWarps &&
                   WideTile::kWidth * WideTile::kHeight == 32 * WideTile::kWarps && ChainTile::kWidth * ChainTile::kHeight == 32 * ChainTile::kWarps,
     "one thread per texel");
 
-// Per-tile lookup tables of the bilinear taps: tap position and weights are separable in x and y, so
-// they are computed once per tile column / row instead of once per texel.  Shared by every decode
+// Lookup tables of the bilinear taps of a run of tiles: tap position and weights are separable in x and y, so
+// they are computed once per column / row instead of once per texel.  Shared by every decode
 // kernel.
 template <typename Tile>
 struct __align__(16) TapTables
 {
-    // per grid (0 = high-res, 1 = low-res) and tile column: byte offset of the left tap inside a footprint row, dx, 1 - dx
-    int4 colTap[2][Tile::kWidth];
+    // per grid (0 = high-res, 1 = low-res) and column: byte offset of the left tap inside a footprint row, dx (, 1 - dx)
+    typename Tile::ColumnTap colTap[2][Tile::kColumns];
     // per grid and tile row: byte offset of the upper tap's footprint row, dy, 1 - dy, bytes per footprint row
     int4 rowTap[2][Tile::kHeight];
     // per grid: footprint width and height in latent pixels, pixel count, and the multiplier that divides a
     // pixel index by the width (p / width == (p * magic) >> 20 for p < 2048)
     int4 footprint[2];
-    // per grid: the footprint origin (tap of the first column / row) of the tile the tables were built for, and that tile's origin
+    // per grid: the footprint origin (tap of the first column / row) of the run the tables were built for, and that run's origin
     int4 origin[2];
 };
 
@@ -234,26 +239,26 @@ struct __align__(16) TileTables
 {
     TapTables<Tile> taps;
     // positional-encoding operand bytes: x = {X0 w0, X1 w0, X0 w1, X1 w1}, y = {X0 w2, X1 w2, unused}
-    uint2 colEnc[Tile::kWidth];
+    uint2 colEnc[Tile::kColumns];
     uint2 rowEnc[Tile::kHeight];
     uint32_t lodWord;  // operand bytes of inputs 44..47: lod, lod, 0, 0
     uint32_t pad[3];
 };
 
-// Builds the tile's tap tables and stages the latent footprint of both grids in shared memory
+// Builds the tap tables of a run of tiles, `columns` wide, and stages its latent footprint of both grids in shared memory
 // (nibbles unpacked to binary16 once per latent pixel instead of once per texel and tap).
 // Even warps work on the high-res grid, odd warps on the low-res grid; the threads of a grid share its footprint pixels.
 // (Tried and dropped, both slower although they execute fewer instructions: two warps staging the
 // footprints while the others go on - the tile then waits for those two; and requesting the latents
 // before the wait for layer 0 and unpacking them after it.)
 //
-// `tablesValid`: the tables already hold this tile's values.  In a mip whose sizes and grid sizes
-// are powers of two (KernelMip::invariant) every tile that lies wholly inside the mip has the same
+// `tablesValid`: the tables already hold this run's values.  In a mip whose sizes and grid sizes
+// are powers of two (KernelMip::invariant) every run that lies wholly inside the mip has the same
 // tap offsets and fractions relative to its own footprint - all the arithmetic is exact - so the
-// tables are built for the first such tile and only the footprint is staged for the others.
+// tables are built for the first such run and only the footprint is staged for the others.
 template <typename Tile, bool kReferenceDivision, int kLayers>
 __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const KernelMip& mip, TapTables<Tile>& taps,
-    uint8_t* footprintHi, uint8_t* footprintLo, int tileX0, int tileY0, int lane, int warp,
+    uint8_t* footprintHi, uint8_t* footprintLo, int tileX0, int tileY0, int columns, int lane, int warp,
     bool tablesValid)
 {
     const int grid = warp & 1;
@@ -280,24 +285,43 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
     }
     else
     {
-        int xb, yb;
+        // each warp of a grid has 32 of the columns
+        const int column = lane + (Tile::kColumns > 32 ? 32 * (warp >> 1) : 0);
+        int xb, tap; // of a column, of a row
         float dx, dy;
-        AxisTap<kReferenceDivision>(min(tileX0 + (lane & (Tile::kWidth - 1)), mip.width - 1), mip.width, mip.invWidth, gw, xb, dx);
-        AxisTap<kReferenceDivision>(min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1), mip.height, mip.invHeight, gh, yb, dy);
-        fx0 = __shfl_sync(0xFFFFFFFFu, xb, 0);
-        fy0 = __shfl_sync(0xFFFFFFFFu, yb, 0);
-        footW = __shfl_sync(0xFFFFFFFFu, xb, Tile::kWidth - 1) - fx0 + 2;
-        const int footH = __shfl_sync(0xFFFFFFFFu, yb, Tile::kHeight - 1) - fy0 + 2;
+        AxisTap<kReferenceDivision>(min(tileX0 + column, mip.width - 1), mip.width, mip.invWidth, gw, xb, dx);
+        if constexpr (Tile::kColumns > 32)
+        {
+            // the rows in the first lanes; the first and the last column in the two after them
+            const bool row = lane < Tile::kHeight;
+            const int texel = row ? min(tileY0 + lane, mip.rowEnd - 1) : lane == Tile::kHeight ? tileX0 : min(tileX0 + columns - 1, mip.width - 1);
+            AxisTap<kReferenceDivision>(texel, row ? mip.height : mip.width, row ? mip.invHeight : mip.invWidth, row ? gh : gw, tap, dy);
+            fx0 = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight);
+            footW = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight + 1) - fx0 + 2;
+        }
+        else
+        {
+            AxisTap<kReferenceDivision>(min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1), mip.height, mip.invHeight, gh, tap, dy);
+            fx0 = __shfl_sync(0xFFFFFFFFu, xb, 0);
+            footW = __shfl_sync(0xFFFFFFFFu, xb, Tile::kWidth - 1) - fx0 + 2;
+        }
+        fy0 = __shfl_sync(0xFFFFFFFFu, tap, 0);
+        const int footH = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight - 1) - fy0 + 2;
         count = footW * footH;
         // the IEEE quotient of 2^20 / footW floors exactly
         magic = uint32_t(__float2int_rd(__fdiv_rn(1048576.f, float(footW)))) + 1;
+        if constexpr (Tile::kColumns > 32)
+        {
+            if (column < columns)
+                taps.colTap[grid][column] = make_int2((xb - fx0) * stride, __float_as_int(dx));
+        }
         if (warp < 2)
         {
-            if (lane < Tile::kWidth)
+            if constexpr (Tile::kColumns <= 32)
                 taps.colTap[grid][lane] = make_int4((xb - fx0) * stride, __float_as_int(dx), __float_as_int(__fsub_rn(1.f, dx)), 0);
             if (lane < Tile::kHeight)
                 taps.rowTap[grid][lane] =
-                    make_int4((yb - fy0) * footW * stride, __float_as_int(dy), __float_as_int(__fsub_rn(1.f, dy)), footW * stride);
+                    make_int4((tap - fy0) * footW * stride, __float_as_int(dy), __float_as_int(__fsub_rn(1.f, dy)), footW * stride);
             if (lane == 0)
             {
                 taps.footprint[grid] = make_int4(footW, footH, count, int(magic));
@@ -341,48 +365,64 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
     }
 }
 
-// The tile's tables (taps and positional encoding as operand bytes) and its staged footprints.
+// Positional encoding of one coordinate (src/RegressionKernels.h:59-85): per wave the values at phase 0 and 0.25.
+__device__ __forceinline__ void EncodePosition(int coordinate, float scale, __half2 (&waves)[3])
+{
+    float f = __fmul_rn(float(coordinate), scale);
+#pragma unroll
+    for (int wave = 0; wave < 3; ++wave)
+    {
+        const float e0 = __fmaf_rn(Frac(f), 2.f, -1.f);
+        const float e1 = __fmaf_rn(Frac(__fadd_rn(f, 0.25f)), 2.f, -1.f);
+        waves[wave] = __floats2half2_rn(e0, e1);
+        f = __fmul_rn(f, 2.f);
+    }
+}
+
+// Calls encode(waves, rows, index) for the positional encoding of the run's columns (warp 2) and rows (warp 3), and for the
+// lane past the rows.  Quantised, the values are exactly the per-texel inputs.
+template <typename Tile, typename Encode>
+__device__ __forceinline__ void EncodePositions(const KernelMip& mip, int tileX0, int tileY0, int columns, int lane, int warp, Encode encode)
+{
+    const bool rows = warp == 3;
+#pragma unroll 1
+    for (int index = lane; index < (rows ? 32 : columns); index += 32)
+    {
+        __half2 waves[3];
+        EncodePosition(rows ? min(tileY0 + index, mip.rowEnd - 1) : min(tileX0 + index, mip.width - 1), mip.positionScale, waves);
+        encode(waves, rows, index);
+    }
+}
+
+// The tables of a run of tiles (taps and positional encoding as operand bytes) and its staged footprints.
 template <typename Tile, bool kFp8, bool kReferenceDivision, int kLayers, typename Stage>
 __device__ __forceinline__ void PrepareTile(const KernelParams& params, const KernelMip& mip, Stage& stage,
-    int tileX0, int tileY0, int lane, int warp, bool tablesValid)
+    int tileX0, int tileY0, int columns, int lane, int warp, bool tablesValid)
 {
     if (!tablesValid && warp >= 2 && warp < 4)
     {
-        // positional encoding (src/RegressionKernels.h:59-85): warp 2 the x part per column, warp 3
-        // the y part per row, quantised exactly as the per-texel inputs would be
-        const bool rows = warp == 3;
-        const int coordinate = rows ? min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1)
-                                    : min(tileX0 + (lane & (Tile::kWidth - 1)), mip.width - 1);
-        float f = __fmul_rn(float(coordinate), mip.positionScale);
-        __half2 waves[3];
-#pragma unroll
-        for (int wave = 0; wave < 3; ++wave)
-        {
-            const float e0 = __fmaf_rn(Frac(f), 2.f, -1.f);
-            const float e1 = __fmaf_rn(Frac(__fadd_rn(f, 0.25f)), 2.f, -1.f);
-            waves[wave] = __floats2half2_rn(e0, e1);
-            f = __fmul_rn(f, 2.f);
-        }
-        const uint2 enc = make_uint2(QuantizeInputs<kFp8>(waves[0], waves[1]),
-                                     kFp8 ? QuantizeInputPair<kFp8>(waves[2]) : QuantizeInputs<kFp8>(waves[2], waves[2]));
-        if (!rows && lane < Tile::kWidth)
-            stage.tables.colEnc[lane] = enc;
-        if (rows && lane < Tile::kHeight)
-            stage.tables.rowEnc[lane] = enc;
-        if (rows && lane == Tile::kHeight)
-            stage.tables.lodWord = QuantizeLod<kFp8>(mip.positionLod);
+        EncodePositions<Tile>(mip, tileX0, tileY0, columns, lane, warp, [&](const __half2 (&waves)[3], bool rows, int index) {
+            const uint2 enc = make_uint2(QuantizeInputs<kFp8>(waves[0], waves[1]),
+                                         kFp8 ? QuantizeInputPair<kFp8>(waves[2]) : QuantizeInputs<kFp8>(waves[2], waves[2]));
+            if (!rows)
+                stage.tables.colEnc[index] = enc;
+            else if (index < Tile::kHeight)
+                stage.tables.rowEnc[index] = enc;
+            else if (index == Tile::kHeight)
+                stage.tables.lodWord = QuantizeLod<kFp8>(mip.positionLod);
+        });
     }
     PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo,
-        tileX0, tileY0, lane, warp, tablesValid);
+        tileX0, tileY0, columns, lane, warp, tablesValid);
 }
 
-// Whether the tables built for one tile of `mip` serve the tile at (tileX0, tileY0) too, and whether
-// tables built for that tile may be kept for later ones: the tile lies wholly inside the decoded rows
+// Whether the tables built for one run of `mip` serve the run at (tileX0, tileY0) too, and whether
+// tables built for that run may be kept for later ones: it lies wholly inside the decoded rows
 // of a mip with invariant tables.
 template <typename Tile>
-__device__ __forceinline__ bool TileKeepsTables(const KernelMip& mip, int tileX0, int tileY0)
+__device__ __forceinline__ bool TileKeepsTables(const KernelMip& mip, int tileX0, int tileY0, int columns)
 {
-    return mip.invariant && tileX0 + Tile::kWidth <= mip.width && tileY0 + Tile::kHeight <= mip.rowEnd;
+    return mip.invariant && tileX0 + columns <= mip.width && tileY0 + Tile::kHeight <= mip.rowEnd;
 }
 
 // Four quantised inputs of one latent layer from the four staged taps.
@@ -410,9 +450,14 @@ template <bool kFp8, int kLayers = 0, typename Stage>
 __device__ __forceinline__ void GatherGrid(const KernelParams& params, const KernelMip& mip, const Stage& stage,
     int grid, int tileColumn, int tileRow, uint32_t* words)
 {
-    const int4 col = stage.tables.taps.colTap[grid][tileColumn];
+    const auto col = stage.tables.taps.colTap[grid][tileColumn];
     const int4 row = stage.tables.taps.rowTap[grid][tileRow];
-    const float dx = __int_as_float(col.y), dxn = __int_as_float(col.z);
+    const float dx = __int_as_float(col.y);
+    float dxn;
+    if constexpr (sizeof(col) == sizeof(int4))
+        dxn = __int_as_float(col.z);
+    else
+        dxn = __fsub_rn(1.f, dx);
     const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
     // src/FeatureGridDevice.h:46-49
     const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);

@@ -90,9 +90,9 @@ bool ValidMip(const NtcbMipDesc& m, bool pairedOutput)
              m.hiPlane > 0x3FFFFFFFull || m.loPlane > 0x3FFFFFFFull);
 }
 
-// The kernel's view of one mip (everything but its place in the tile list).
+// The kernel's view of one mip (everything but its place in the tile list).  `maxRunTiles`: the longest run of tiles.
 void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprintHiBytes = kFootprintHiBytes,
-    int footprintLoBytes = kFootprintLoBytes, int tileWidth = kTileWidth, int tileHeight = kTileHeight)
+    int footprintLoBytes = kFootprintLoBytes, int tileWidth = kTileWidth, int tileHeight = kTileHeight, int maxRunTiles = 1)
 {
     km.width = m.width;
     km.height = m.height;
@@ -111,14 +111,20 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprin
     km.invHeight = 1.0f / float(m.height);
     km.positionScale = m.positionScale;
     km.positionLod = m.positionLod;
-    // Largest footprint a tile can have in each grid: the tap index of the last column (row) minus
-    // that of the first is at most floor((size - 1) * grid / mip) + 1, plus the second tap.
+    // Largest footprint a run of tiles can have in each grid: the tap index of the last column (row) minus
+    // that of the first is at most floor((size - 1) * grid / mip) + 1, plus the second tap.  The run is as long as allowed, as the mip is
+    // wide, and as its footprint fits.
     km.strideBytes = layers == 1 ? 8 : layers <= 3 ? 24 : 40;
     const long long hiCapacity = footprintHiBytes / km.strideBytes, loCapacity = footprintLoBytes / km.strideBytes;
     auto footprint = [](int grid, int mip, int span) { return (long long)((long long)span * grid / mip) + 3; };
-    const long long hiPixels = footprint(m.hiWidth, m.width, tileWidth - 1) * footprint(m.hiHeight, m.height, tileHeight - 1);
-    const long long loPixels = footprint(m.loWidth, m.width, tileWidth - 1) * footprint(m.loHeight, m.height, tileHeight - 1);
-    km.staged = (hiPixels <= hiCapacity && loPixels <= loCapacity) ? 1 : 0;
+    auto fits = [&](int columns) {
+        return footprint(m.hiWidth, m.width, columns - 1) * footprint(m.hiHeight, m.height, tileHeight - 1) <= hiCapacity &&
+               footprint(m.loWidth, m.width, columns - 1) * footprint(m.loHeight, m.height, tileHeight - 1) <= loCapacity;
+    };
+    km.staged = fits(tileWidth) ? 1 : 0;
+    km.runTiles = 1;
+    while (km.runTiles < maxRunTiles && km.runTiles * tileWidth < m.width && fits(2 * km.runTiles * tileWidth))
+        km.runTiles *= 2;
     // Tables that do not depend on the tile: with power-of-two sizes all the tap arithmetic is exact in
     // binary32, and when a tile's width and height map to whole latent pixels of both grids (and to whole
     // periods of the positional encoding) moving from tile to tile shifts every tap by an integer.
@@ -141,13 +147,22 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprin
         km.hiStepY = int((long long)tileHeight * m.hiHeight / m.height);
         km.loStepY = int((long long)tileHeight * m.loHeight / m.height);
     }
-    km.tilesX = (m.width + tileWidth - 1) / tileWidth;
+    km.tilesX = (m.width + km.runTiles * tileWidth - 1) / (km.runTiles * tileWidth);
     // ceil(2^32 / tilesX) divides every local < n when local * (magic * tilesX - 2^32) stays below 2^32
     const unsigned long long tilesX = (unsigned long long)km.tilesX, magic = (0x100000000ull + tilesX - 1) / tilesX;
     const unsigned long long tilesY = (unsigned long long)((m.rowEnd - m.rowBegin + tileHeight - 1) / tileHeight);
     const bool exact = tilesX > 1 && (tilesX * tilesY) * (magic * tilesX - 0x100000000ull) < 0x100000000ull;
     km.tilesXMagic = exact ? unsigned(magic) : 0u;
     km.firstTile = 0;
+}
+
+// Longest run of tiles for a launch of `tiles` tiles on `chains` chains.  A run of r tiles costs a chain 0.36 / r of a tile for tables and
+// footprints (FP8 weights; 0.2 with Int8), and the launch about r tiles at its end, when chains run out of work: four pay from 32 tiles a chain,
+// two from 8.  (4096 x 4096 FP8, 148 tiles a chain, runs of 1, 2 and 4: 717, 673 and 655 us; 1500 x 1100, 15 tiles: 86.9, 80.2 and 83.1;
+// 1024 x 512, 5 tiles: 30.1, 30.9 and 33.0.)
+int LongestRun(long long tiles, long long chains)
+{
+    return tiles >= 32 * chains ? kMaxRunTiles : tiles >= 8 * chains ? 2 : 1;
 }
 
 } // namespace
@@ -617,6 +632,20 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     k.status = p->status;
     k.numLayers = p->numFeatures / 4;
     k.channels = p->channels;
+    const bool fp8 = p->weightMode == NTCB_WEIGHTS_FP8;
+    int resident = 0, longestRun = 1;
+    if (reference)
+    {
+        long long tiles = 0;
+        for (int i = 0; i < p->numMips; ++i)
+        {
+            const NtcbMipDesc& m = p->mips[i];
+            if (m.width > 0 && m.rowEnd > m.rowBegin)
+                tiles += ((long long)m.width + kChainTileWidth - 1) / kChainTileWidth *
+                         (((long long)m.rowEnd - m.rowBegin + kChainTileHeight - 1) / kChainTileHeight);
+        }
+        longestRun = LongestRun(tiles, kMaxChains * 148); // a B200's 148 SMs
+    }
     long long tiles = 0;
     int used = 0;
     for (int i = 0; i < p->numMips; ++i)
@@ -666,9 +695,9 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
         KernelMip& km = k.mips[used++];
         const int tileHeight = reference ? kChainTileHeight : kTileHeight;
         if (reference && p->weightMode == NTCB_WEIGHTS_FP8)
-            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes, kRefFootprintLoBytes, kChainTileWidth, kChainTileHeight);
+            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes, kRefFootprintLoBytes, kChainTileWidth, kChainTileHeight, longestRun);
         else if (reference)
-            FillKernelMip(m, p->numFeatures / 4, km, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes, kChainTileWidth, kChainTileHeight);
+            FillKernelMip(m, p->numFeatures / 4, km, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes, kChainTileWidth, kChainTileHeight, longestRun);
         else
             FillKernelMip(m, p->numFeatures / 4, km);
         km.firstTile = int(tiles);
@@ -699,8 +728,6 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     }
     k.loadWaitPolls = g_networkWaitPolls.load(std::memory_order_relaxed);
 
-    const bool fp8 = p->weightMode == NTCB_WEIGHTS_FP8;
-    int resident = 0;
     int rc = ResidentCtas(fp8, k.convert != 0, &resident, reference);
     if (rc != NTCB_OK)
         return rc;

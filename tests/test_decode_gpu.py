@@ -255,6 +255,34 @@ def test_row_ranges_tile_rows_and_guard_bands(oracle, numerics):
         assert (got[~rows] == -7.0).all()
 
 
+# Launches of enough tiles (16 x 8 texels) for 1184 chains to walk them in runs of two (8 tiles a chain) or of four (32 a chain): mip sizes that
+# are no multiples of a tile or a run, grids at 1/2 to 1/6 of the mip (the longest runs do not fit all of them), and powers of two.
+@pytest.mark.parametrize("numerics,shape", [
+    (REFERENCE, (1500, 1100, 10, 0, 4, 12)), (REFERENCE, (2510, 2012, 6, 0, 3, 8)), (REFERENCE, (2048, 3001, 4, 2, 6, 16)),
+    (REFERENCE, (2600, 2048, 4, 1, 2, 4)), (REFERENCE, (2048, 2048, 8, 0, 4, 12)), (REFERENCE, (4096, 2048, 4, 2, 2, 16)),
+    (REFERENCE, (40, 130000, 4, 1, 4, 8))])
+def test_runs_of_tiles_give_the_texels_of_single_tiles(numerics, shape):
+    """The tables and footprints of neighbouring tiles are prepared together in large launches, and one tile at a time in small ones:
+    a whole decode has the bits of one in bands of a few rows."""
+    import torch
+
+    data = synthetic.make_texture_set(synthetic.TextureSetSpec(*shape, seed=17, network="unit"))
+    geo = data.geometry
+    resident = binding.ResidentTextureSet.from_synthetic(data, numerics=numerics)
+    for use_int8 in (True, False):
+        resident.out.fill_(-7.0)
+        resident.decode(use_int8)
+        whole = resident.out.clone()
+        resident.out.fill_(-7.0)
+        for mip, cm in enumerate(geo.color_mips):
+            rows = max(8, 8 * (8000 // ((cm.width + 15) // 16)))  # fewer than eight tiles a chain
+            for begin in range(0, cm.height, rows):
+                resident.decode(use_int8, mips=[mip], row_ranges={mip: (begin, min(begin + rows, cm.height))})
+        _sync()
+        resident.check_status()
+        assert torch.equal(whole.view(torch.int16), resident.out.view(torch.int16)), use_int8
+
+
 def test_texture_set_api_decompress_and_read_channels(oracle):
     """The texture-set level of the C ABI: load from a container in host memory, Decompress,
     ReadChannels with full, subset and padded requests, to host and to device memory, for both
