@@ -163,6 +163,22 @@ __device__ __forceinline__ void TmemStore4(uint32_t address, uint32_t a, uint32_
                  : "memory");
 }
 
+// Eight, sixteen.
+__device__ __forceinline__ void TmemStore8(uint32_t address, const uint32_t* w)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(address), "r"(w[0]), "r"(w[1]),
+                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
+__device__ __forceinline__ void TmemStore16(uint32_t address, const uint32_t* w)
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(address), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+                 "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+                 : "memory");
+}
+
 __device__ __forceinline__ void TmemStoreWait()
 {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

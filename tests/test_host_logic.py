@@ -510,3 +510,22 @@ def test_reference_loader_accepts_the_texture_headers(oracle):
     probed = oracle.reference_probe(_set_with_textures().container)
     assert probed[:6] == [64, 64, 6, 7, 2, 8]
     assert probed[7] == 0b111111  # the reference's valid-channel mask: the channels the textures cover
+
+
+def test_rounding_to_the_activation_grid_as_a_subnormal_number():
+    """The reference-numerics kernels round p = y * 80 to an integer as a multiple of 2^-24, the subnormal binary16 numbers: for every
+    activation input the product with the grid's step is the number that rint and a product give."""
+    def half(values):
+        return values.astype(np.float16)  # (round to nearest even; a binary64 holds every sum and product here exactly)
+
+    x = np.arange(65536, dtype=np.uint16).view(np.float16)
+    x = x[np.isfinite(x)].astype(np.float64)
+    third, step = float(np.float16(1 / 3)), float(np.float16(np.float32(3.1875) / np.float32(255)))
+    t = half(np.clip(x * third + 0.5, 0, 1)).astype(np.float64)
+    y = half(np.minimum(x, 3) * t).astype(np.float64)
+    p = half(y * 80).astype(np.float64)
+    code = half(p * 2.0 ** -24 + 2.0 ** -20).view(np.uint16)
+    assert code.min() >= 1 and code.max() <= 256
+    assert float(np.float16(step * 2 ** 22)) == step * 2 ** 22 and float(np.float16(16 * step)) == 16 * step
+    scaled = (code << 2).view(np.float16).astype(np.float64)
+    assert np.array_equal(half(scaled * (step * 2 ** 22) - 16 * step), half(np.rint(p) * step))
