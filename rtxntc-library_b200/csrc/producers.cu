@@ -122,18 +122,33 @@ __device__ __forceinline__ float RoundAway(float x)
     return roundf(x);
 }
 
+// A column has at most 64 weights: two per lane, rows r = lane and lane + 32.
+constexpr int kRowsPerLane = 2;
+
 // One output column quantised to int8 with a per-column scale and an integer bias
-// (QuantizeColumnInt8, src/Quantizer.cu:90-208).
-__device__ void QuantizeColumnInt8(int layer, int column, const __half* weights, float bias, int8_t* codes, __half* rounded,
-    float* scaleOut, int32_t* biasOut, float outputScale, float outputBias)
+// (QuantizeColumnInt8, src/Quantizer.cu:90-208), by a warp.
+__device__ __forceinline__ void QuantizeColumnInt8(int layer, int rows, int lane, const __half* weights, float bias, int8_t* codes,
+    __half* rounded, float* scaleOut, int32_t* biasOut, float outputScale, float outputBias)
 {
-    const int rows = LayerInputs(layer);
+    float w[kRowsPerLane];
     float low = 3.402823466e+38f, high = 1.175494351e-38f; // the reference's starting values
-    for (int r = 0; r < rows; ++r)
+#pragma unroll
+    for (int i = 0; i < kRowsPerLane; ++i)
     {
-        const float w = __half2float(weights[r]);
-        low = fminf(low, w);
-        high = fmaxf(high, w);
+        const int r = lane + 32 * i;
+        if (r < rows)
+        {
+            w[i] = __half2float(weights[r]);
+            low = fminf(low, w[i]);
+            high = fmaxf(high, w[i]);
+        }
+    }
+    // (a minimum and a maximum do not depend on the order, and a NaN never is one)
+#pragma unroll
+    for (int distance = 16; distance > 0; distance >>= 1)
+    {
+        low = fminf(low, __shfl_xor_sync(0xFFFFFFFFu, low, distance));
+        high = fmaxf(high, __shfl_xor_sync(0xFFFFFFFFu, high, distance));
     }
     const float limit = fmaxf(fabsf(high), fabsf(low));
     float inverseLimit;
@@ -141,17 +156,19 @@ __device__ void QuantizeColumnInt8(int layer, int column, const __half* weights,
 
     const float scale = 127.5f, inverseScale = 1.f / 127.5f;
     const float ratio = ApproxDivide(scale, limit); // the odd rows use scale / limit, the even ones scale * (1 / limit)
+    float q[kRowsPerLane];
     int sum = 0;
-    for (int r = 0; r < rows; ++r)
+#pragma unroll
+    for (int i = 0; i < kRowsPerLane; ++i)
     {
-        const float w = __half2float(weights[r]);
-        float q = (r & 1) ? RoundAway(MulFtz(w, ratio)) : RoundAway(MulFtz(MulFtz(w, scale), inverseLimit));
-        q = fmaxf(fminf(q, 127.f), -127.f);
-        codes[r] = int8_t(q);
-        sum += int(q);
-        if (rounded)
-            rounded[r] = __float2half_rn(MulFtz(MulFtz(q, limit), inverseScale));
+        if (lane + 32 * i < rows)
+        {
+            q[i] = (lane & 1) ? RoundAway(MulFtz(w[i], ratio)) : RoundAway(MulFtz(MulFtz(w[i], scale), inverseLimit));
+            q[i] = fmaxf(fminf(q[i], 127.f), -127.f);
+            sum += int(q[i]);
+        }
     }
+    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
 
     float layerScale = MulFtz(limit, inverseScale);
     float layerBias = bias;
@@ -172,42 +189,53 @@ __device__ void QuantizeColumnInt8(int layer, int column, const __half* weights,
 
     // (output * scale + bias) becomes ((output + integer bias) * scale); a zero scale (a constant
     // image channel) is replaced by 2^-16 with zero weights.
-    int integerBias;
-    if (layerScale == 0.f)
-    {
+    const bool constant = layerScale == 0.f;
+    if (constant)
         layerScale = 1.f / 65536.f;
-        integerBias = int(RoundAway(MulFtz(layerBias, 65536.f)));
-        for (int r = 0; r < rows; ++r)
-            codes[r] = 0;
+#pragma unroll
+    for (int i = 0; i < kRowsPerLane; ++i)
+    {
+        const int r = lane + 32 * i;
+        if (r < rows)
+        {
+            codes[r] = constant ? int8_t(0) : int8_t(q[i]);
+            if (rounded)
+                rounded[r] = __float2half_rn(MulFtz(MulFtz(q[i], limit), inverseScale));
+        }
     }
-    else
-        integerBias = int(RoundAway(ApproxDivide(layerBias, layerScale)));
-    *scaleOut = layerScale;
-    *biasOut = integerBias;
+    if (lane == 0)
+    {
+        *scaleOut = layerScale;
+        *biasOut = constant ? int(RoundAway(MulFtz(layerBias, 65536.f))) : int(RoundAway(ApproxDivide(layerBias, layerScale)));
+    }
 }
 
 // One output column rounded to e4m3; the bias stays fp16 (QuantizeColumnFP8, src/Quantizer.cu:210-252).
-__device__ void QuantizeColumnFp8(int rows, const __half* weights, uint8_t* codes, __half* rounded)
+__device__ __forceinline__ void QuantizeColumnFp8(int rows, int lane, const __half* weights, uint8_t* codes, __half* rounded)
 {
-    for (int r = 0; r < rows; r += 2)
+#pragma unroll
+    for (int i = 0; i < kRowsPerLane; ++i)
     {
-        const __half2 pair = __halves2half2(weights[r], weights[r + 1]);
-        const __nv_fp8x2_e4m3 q(pair);
-        codes[r] = uint8_t(q.__x & 0xff);
-        codes[r + 1] = uint8_t(q.__x >> 8);
-        if (rounded)
+        const int r = lane + 32 * i;
+        if (r < rows)
         {
-            const __half2 back = __half2(q);
-            rounded[r] = __low2half(back);
-            rounded[r + 1] = __high2half(back);
+            const __nv_fp8_e4m3 q(weights[r]);
+            codes[r] = q.__x;
+            if (rounded)
+                rounded[r] = __half(q);
         }
     }
 }
 
-// One thread per output column, the columns of all layers one after another: a single CTA.
-__global__ void __launch_bounds__(kColumns) QuantizeNetworkKernel(const QuantizeArguments args)
+// One warp per output column, the columns of all layers one after another.  A latency-bound step: launch, one load, a reduction, two
+// divisions.  (With a thread per column, which walked its weights twice, a call took 23 us.)
+constexpr int kQuantizeThreads = 128;
+static_assert(kColumns % (kQuantizeThreads / 32) == 0, "every warp has a column");
+
+__global__ void __launch_bounds__(kQuantizeThreads) QuantizeNetworkKernel(const __grid_constant__ QuantizeArguments args)
 {
-    int column = threadIdx.x, layer = 0, weightOffset = 0, columnOffset = 0;
+    const int lane = threadIdx.x & 31;
+    int column = int(blockIdx.x * (kQuantizeThreads / 32) + (threadIdx.x >> 5)), layer = 0, weightOffset = 0, columnOffset = 0;
     while (column >= LayerOutputs(layer))
     {
         column -= LayerOutputs(layer);
@@ -226,19 +254,20 @@ __global__ void __launch_bounds__(kColumns) QuantizeNetworkKernel(const Quantize
         // weights, then the scales of all layers, then the integer biases (src/WeightLayout.cpp:184-255)
         float* scales = reinterpret_cast<float*>(args.blob + kWeights) + columnOffset + column;
         int32_t* biases = reinterpret_cast<int32_t*>(args.blob + kWeights + 4 * kColumns) + columnOffset + column;
-        QuantizeColumnInt8(layer, column, weights, __half2float(bias), reinterpret_cast<int8_t*>(codes), rounded, scales, biases,
+        QuantizeColumnInt8(layer, rows, lane, weights, __half2float(bias), reinterpret_cast<int8_t*>(codes), rounded, scales, biases,
             args.outputScale[column & 15], args.outputBias[column & 15]);
     }
     else if (layer < kLayers - 1)
     {
         // weights, then the fp16 biases of layers 0-2, then the output layer's scales and integer biases
-        QuantizeColumnFp8(rows, weights, codes, rounded);
-        reinterpret_cast<__half*>(args.blob + kWeights)[columnOffset + column] = bias;
+        QuantizeColumnFp8(rows, lane, weights, codes, rounded);
+        if (lane == 0)
+            reinterpret_cast<__half*>(args.blob + kWeights)[columnOffset + column] = bias;
     }
     else
     {
         uint8_t* tail = args.blob + kWeights + 2 * (kColumns - 16);
-        QuantizeColumnInt8(layer, column, weights, __half2float(bias), reinterpret_cast<int8_t*>(codes), rounded,
+        QuantizeColumnInt8(layer, rows, lane, weights, __half2float(bias), reinterpret_cast<int8_t*>(codes), rounded,
             reinterpret_cast<float*>(tail) + column, reinterpret_cast<int32_t*>(tail + 64) + column,
             args.outputScale[column], args.outputBias[column]);
     }
@@ -432,7 +461,7 @@ extern "C" int ntcb_quantize_network(const NtcbQuantizeNetworkParams* params, vo
         args.outputScale[c] = params->outputScale ? params->outputScale[c] : 1.f;
         args.outputBias[c] = params->outputBias ? params->outputBias[c] : 0.f;
     }
-    QuantizeNetworkKernel<<<1, kColumns, 0, static_cast<cudaStream_t>(stream)>>>(args);
+    QuantizeNetworkKernel<<<kColumns / (kQuantizeThreads / 32), kQuantizeThreads, 0, static_cast<cudaStream_t>(stream)>>>(args);
     CountLaunch();
     const cudaError_t error = cudaGetLastError();
     if (error != cudaSuccess)
