@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert != kConvertNone ? kCt
     {
         // ---- tables and latent footprints of the first tile -----------------------------------
         place = locate(tile, 0);
-        PrepareTile<WideTile, kFp8, false, kLayers>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, kTileWidth, lane, warp, false);
+        PrepareTile<WideTile, kFp8, false, kLayers>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, kTileWidth, lane, warp, false, []() {});
         tablesMip = TileKeepsTables<WideTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0, kTileWidth) ? place.mipIndex : -1;
         __syncthreads();
     }
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kThreadsPerCta, kConvert != kConvertNone ? kCt
             place = locate(nextTile, place.mipIndex);
             // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
             const bool keepsTables = TileKeepsTables<WideTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0, kTileWidth);
-            PrepareTile<WideTile, kFp8, false, kLayers>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, kTileWidth, lane, warp, keepsTables && place.mipIndex == tablesMip);
+            PrepareTile<WideTile, kFp8, false, kLayers>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, kTileWidth, lane, warp, keepsTables && place.mipIndex == tablesMip, []() {});
             tablesMip = keepsTables ? place.mipIndex : -1;
         }
         ConsumeLayer<kFp8, 0, kConvertNone>(params, shared, ctx, phase, failed);

@@ -302,9 +302,9 @@ struct RefTileContext
 
 // Builds the lookup tables of a run of tiles, `columns` wide, and stages the latent footprint of both grids in shared memory
 // (`tablesValid`: the tables already hold this run's values, see PrepareTaps).  `warp`: of the chain's four.
-template <int kLayers = 0>
+template <int kLayers, typename Between>
 __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
-    int tileX0, int tileY0, int columns, int lane, int warp, bool tablesValid)
+    int tileX0, int tileY0, int columns, int lane, int warp, bool tablesValid, Between between)
 {
     if (!tablesValid && warp >= 2 && warp < 4)
     {
@@ -326,7 +326,7 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
         });
     }
     PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, tileX0,
-        tileY0, columns, lane, warp, tablesValid);
+        tileY0, columns, lane, warp, tablesValid, between);
 }
 
 // Four inputs of one latent layer from the four taps, as two binary16 pairs.
@@ -607,9 +607,13 @@ __device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext&
 }
 
 // One-time setup of a CTA: the network image arrives by one TMA bulk copy while the threads fill
-// the constant tables, set up the barriers and allocate tensor memory.  A thread that gives up waiting for the image
-// sets its chain's give-up word (status words written): the chain leaves at its first tile.
-__device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
+// the constant tables, set up the barriers and allocate tensor memory.  `first(dependency)` does what the first tile needs: what it can
+// without global memory, then dependency() - the end of the kernel before this one, and the request for the network - and then the rest, under the
+// network's way from the L2.  A thread that gives up waiting for the image sets its chain's give-up word (status words written): the chain
+// leaves at its first tile.
+template <typename First>
+__device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp,
+    First first)
 {
     // constant A operands of the bias steps: core matrix l (8 rows of 16 bytes) has 1.0 as half l of every row,
     // core matrix 4 is zero
@@ -633,12 +637,14 @@ __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint
     }
     if (warp == 0)
         TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerHalf);
-    GridDependencyWait();
-    if (tid == 0)
-    {
-        MbarrierArriveExpectTx(loadBarrier, kRefInt8NetworkBytes);
-        BulkCopyToShared(SharedAddress(shared.network), network, kRefInt8NetworkBytes, loadBarrier);
-    }
+    first([&]() {
+        GridDependencyWait();
+        if (tid == 0)
+        {
+            MbarrierArriveExpectTx(loadBarrier, kRefInt8NetworkBytes);
+            BulkCopyToShared(SharedAddress(shared.network), network, kRefInt8NetworkBytes, loadBarrier);
+        }
+    });
     FenceProxyAsyncShared(); // the bias region is read by the tensor core (async proxy)
     TcgenFenceBeforeSync();
     __syncthreads();
@@ -693,7 +699,34 @@ __device__ __forceinline__ void DecodeRuns(const KernelParams& params)
     const int chain = warp >> 2, role = WarpRole(warp);
     const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
-    Chain::Setup(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    Stage& stage = StageOf<Stage>(shared, chain);
+    // the first chains of all CTAs take the first runs, so that a launch of few spreads over the SMs
+    uint32_t run = blockIdx.x + uint32_t(chain) * gridDim.x;
+    // (What can be worked out from these is, tile by tile: the registers are worth more than the instructions.)
+    int mipIndex = 0, x0 = 0, y0 = 0; // the next tile's mip and place
+    bool known = false;               // the tables, and what the threads keep of them, are already the next tile's
+    int tablesMip = -1;               // mip whose tables are in shared memory and valid for every inner run of it
+    auto prepareRun = [&](auto between) {
+        while (mipIndex + 1 < params.numMips && run >= uint32_t(params.mips[mipIndex + 1].firstTile))
+            ++mipIndex; // runs are visited in increasing order, so the search resumes at the current mip
+        const KernelMip& mip = params.mips[mipIndex];
+        const int local = int(run) - mip.firstTile;
+        const int row = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
+        const int columns = mip.runTiles * kChainTileWidth;
+        x0 = (local - row * mip.tilesX) * columns;
+        y0 = mip.rowBegin + row * kChainTileHeight;
+        const bool keeps = TileKeepsTables<ChainTile>(mip, x0, y0, columns);
+        // the tables of the previous run serve this one too when both lie inside the same mip with invariant tables
+        known = keeps && mipIndex == tablesMip;
+        Chain::template Prepare<kLayers>(params, mip, stage, x0, y0, columns, lane, role, known, between);
+        tablesMip = keeps ? mipIndex : -1;
+    };
+    Chain::Setup(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [&](auto dependency) {
+        if (run < uint32_t(params.totalTiles))
+            prepareRun(dependency);
+        else
+            dependency();
+    });
     uint32_t phase = 0;
 
     RefTileContext ctx;
@@ -704,65 +737,27 @@ __device__ __forceinline__ void DecodeRuns(const KernelParams& params)
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * (sizeof(Storage::operandA) / kMaxChains)) + (tid & 127);
 
-    Stage& stage = StageOf<Stage>(shared, chain);
-    // the first chains of all CTAs take the first runs, so that a launch of few spreads over the SMs
-    const uint32_t runStep = (blockDim.x >> 7) * gridDim.x;
-    uint32_t run = blockIdx.x + uint32_t(chain) * gridDim.x;
-    int mipIndex = 0, x0 = 0, y0 = 0; // the next tile's mip and place
-    int tilesLeft = 0;                // of the run
-    int column = 0;                   // of the next tile's first texel in the run
-    int2 shift = make_int2(0, 0);     // bytes the next tile's taps lie past those in TexelTables
-    bool keeps = false;               // the run's tables serve others of its mip, and its later tiles what the threads keep of the first
-    bool known = false;               // the tables, and what the threads keep of them, are already the next tile's
-    int tablesMip = -1;               // mip whose tables are in shared memory and valid for every inner run of it
-    auto prepareRun = [&]() {
-        while (mipIndex + 1 < params.numMips && run >= uint32_t(params.mips[mipIndex + 1].firstTile))
-            ++mipIndex; // runs are visited in increasing order, so the search resumes at the current mip
-        const KernelMip& mip = params.mips[mipIndex];
-        const int local = int(run) - mip.firstTile;
-        const int row = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
-        const int columns = mip.runTiles * kChainTileWidth;
-        x0 = (local - row * mip.tilesX) * columns;
-        y0 = mip.rowBegin + row * kChainTileHeight;
-        tilesLeft = min(mip.runTiles, (mip.width - x0 + kChainTileWidth - 1) / kChainTileWidth);
-        column = 0;
-        shift = make_int2(0, 0);
-        keeps = TileKeepsTables<ChainTile>(mip, x0, y0, columns);
-        // the tables of the previous run serve this one too when both lie inside the same mip with invariant tables
-        known = keeps && mipIndex == tablesMip;
-        Chain::template Prepare<kLayers>(params, mip, stage, x0, y0, columns, lane, role, known);
-        tablesMip = keeps ? mipIndex : -1;
-    };
-    if (run < uint32_t(params.totalTiles))
-    {
-        prepareRun();
-        ChainBarrier(chain);
-    }
-    while (tilesLeft)
+    while (run < uint32_t(params.totalTiles))
     {
         const KernelMip& mip = params.mips[mipIndex];
         ctx.tile = int(run);
         ctx.x = x0 + tileColumn;
         ctx.y = y0 + tileRow;
-        Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known, shift);
+        // runs start at multiples of their width
+        const int column = x0 & (mip.runTiles * kChainTileWidth - 1);
+        const int steps = known ? column / kChainTileWidth * StrideBytes<kLayers>(mip) : 0;
+        Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known,
+            make_int2(steps * mip.hiStepX, steps * mip.loStepX));
 
         // layer 0; while the tensor core works on it, prepare the chain's NEXT run (its tables and
         // footprints replace this run's, which nobody reads after the barrier inside Issue)
         if (Chain::template Issue<0>(ctx))
             break; // some thread of the chain gave up on a wait
-        if (--tilesLeft)
-        {
-            x0 += kChainTileWidth;
-            column += kChainTileWidth;
-            known = keeps;
-            if (keeps)
-            {
-                shift.x += mip.hiStepX * StrideBytes<kLayers>(mip);
-                shift.y += mip.loStepX * StrideBytes<kLayers>(mip);
-            }
-        }
-        else if ((run += runStep) < uint32_t(params.totalTiles))
-            prepareRun();
+        x0 += kChainTileWidth;
+        if (x0 < mip.width && (x0 & (mip.runTiles * kChainTileWidth - 1)))
+            known = tablesMip == mipIndex; // a run whose tables serve others: so does what the threads keep of its first tile
+        else if ((run += (blockDim.x >> 7) * gridDim.x) < uint32_t(params.totalTiles))
+            prepareRun([]() {});
         Chain::template Consume<0, kConvertNone>(params, ctx, phase);
 
         Chain::template Issue<1>(ctx);
@@ -803,19 +798,21 @@ struct Int8Chain
 {
     using Storage = RefSharedStorage;
     using Stage = RefStage;
-    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp)
+    template <typename First>
+    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp,
+        First first)
     {
-        SetupCtaRef(shared, network, status, polls, tid, warp);
+        SetupCtaRef(shared, network, status, polls, tid, warp, first);
     }
     static __device__ __forceinline__ void Teardown(Storage& shared, const RefTileContext& ctx, uint32_t phase, int tid, int warp)
     {
         TeardownCtaRef(shared, ctx, phase, tid, warp);
     }
-    template <int kLayers>
+    template <int kLayers, typename Between>
     static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
-        int lane, int role, bool tablesValid)
+        int lane, int role, bool tablesValid, Between between)
     {
-        PrepareTileRef<kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid);
+        PrepareTileRef<kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid, between);
     }
     template <int kLayers>
     static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const RefTileContext& ctx,
@@ -858,7 +855,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
     // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCtaRef)
     if (tid < params.numMips)
         mipTable[tid] = params.mips[tid];
-    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [](auto dependency) { dependency(); });
     int aborted = 0;
     uint32_t phase = 0;
 
@@ -1246,7 +1243,9 @@ __device__ __forceinline__ int RunLayerRefFp8(const Params& params, RefTileConte
 }
 
 // Setup and teardown as for the binary16 kernel, on the FP8 kernel's shared-memory structure.
-__device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
+template <typename First>
+__device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp,
+    First first)
 {
     for (int i = tid; i < 128 * 32 / 16; i += int(blockDim.x))
         reinterpret_cast<uint4*>(shared.biasRegion)[i] = make_uint4(i < 128 ? 0x00003C00u : 0u, 0u, 0u, 0u);
@@ -1264,12 +1263,14 @@ __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, cons
     }
     if (warp == 0)
         TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerHalf);
-    GridDependencyWait();
-    if (tid == 0)
-    {
-        MbarrierArriveExpectTx(loadBarrier, kRefNetworkBytes);
-        BulkCopyToShared(SharedAddress(shared.network), network, kRefNetworkBytes, loadBarrier);
-    }
+    first([&]() {
+        GridDependencyWait();
+        if (tid == 0)
+        {
+            MbarrierArriveExpectTx(loadBarrier, kRefNetworkBytes);
+            BulkCopyToShared(SharedAddress(shared.network), network, kRefNetworkBytes, loadBarrier);
+        }
+    });
     FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
     __syncthreads();
@@ -1303,19 +1304,21 @@ struct Fp8Chain
 {
     using Storage = RefFp8SharedStorage;
     using Stage = RefFp8Stage;
-    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp)
+    template <typename First>
+    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp,
+        First first)
     {
-        SetupCtaRefFp8(shared, network, status, polls, tid, warp);
+        SetupCtaRefFp8(shared, network, status, polls, tid, warp, first);
     }
     static __device__ __forceinline__ void Teardown(Storage& shared, const RefTileContext& ctx, uint32_t phase, int tid, int warp)
     {
         TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
     }
-    template <int kLayers>
+    template <int kLayers, typename Between>
     static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
-        int lane, int role, bool tablesValid)
+        int lane, int role, bool tablesValid, Between between)
     {
-        PrepareTile<ChainTile, true, true, kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid);
+        PrepareTile<ChainTile, true, true, kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid, between);
     }
     template <int kLayers>
     static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const RefTileContext& ctx,
@@ -1356,7 +1359,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const
 
     if (tid < params.numMips)
         mipTable[tid] = params.mips[tid];
-    SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp);
+    SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [](auto dependency) { dependency(); });
     int aborted = 0;
     uint32_t phase = 0;
 

@@ -256,10 +256,12 @@ struct __align__(16) TileTables
 // are powers of two (KernelMip::invariant) every run that lies wholly inside the mip has the same
 // tap offsets and fractions relative to its own footprint - all the arithmetic is exact - so the
 // tables are built for the first such run and only the footprint is staged for the others.
-template <typename Tile, bool kReferenceDivision, int kLayers>
+//
+// `between()` is called between building the tables, which needs nothing from global memory, and staging (not with valid tables).
+template <typename Tile, bool kReferenceDivision, int kLayers, typename Between>
 __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const KernelMip& mip, TapTables<Tile>& taps,
     uint8_t* footprintHi, uint8_t* footprintLo, int tileX0, int tileY0, int columns, int lane, int warp,
-    bool tablesValid)
+    bool tablesValid, Between between)
 {
     const int grid = warp & 1;
     const int gw = grid ? mip.loWidth : mip.hiWidth;
@@ -328,6 +330,7 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
                 taps.origin[grid] = make_int4(fx0, fy0, tileX0, tileY0);
             }
         }
+        between();
     }
 
     if (mip.staged)
@@ -395,9 +398,9 @@ __device__ __forceinline__ void EncodePositions(const KernelMip& mip, int tileX0
 }
 
 // The tables of a run of tiles (taps and positional encoding as operand bytes) and its staged footprints.
-template <typename Tile, bool kFp8, bool kReferenceDivision, int kLayers, typename Stage>
+template <typename Tile, bool kFp8, bool kReferenceDivision, int kLayers, typename Stage, typename Between>
 __device__ __forceinline__ void PrepareTile(const KernelParams& params, const KernelMip& mip, Stage& stage,
-    int tileX0, int tileY0, int columns, int lane, int warp, bool tablesValid)
+    int tileX0, int tileY0, int columns, int lane, int warp, bool tablesValid, Between between)
 {
     if (!tablesValid && warp >= 2 && warp < 4)
     {
@@ -413,7 +416,7 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
         });
     }
     PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo,
-        tileX0, tileY0, columns, lane, warp, tablesValid);
+        tileX0, tileY0, columns, lane, warp, tablesValid, between);
 }
 
 // Whether the tables built for one run of `mip` serve the run at (tileX0, tileY0) too, and whether
