@@ -286,6 +286,12 @@ __device__ __forceinline__ int WarpRole(int warpIndex)
 struct RefTileContext
 {
     int tid;
+    // The same in all lanes of a warp (Uniform): the thread's warp, and its chain's first tensor-memory column at lane 0.  What follows from
+    // them - roles, barriers, the place of a tile and its mip's constants - lives in uniform registers.  (Taken from the thread's
+    // index, all of that took vector registers, and branches on it reconverged: 8192 x 8192 Int8 3803 -> 3640 us, 4096 x 4096 FP8 664 -> 649,
+    // its 8-bit pixels 874 -> 828, 16.7 M queries 658 -> 641.)
+    int warp;
+    uint32_t accumulators;
     uint32_t tmemLane;    // the chain's first tensor-memory column at this thread's lane (its warp's first lane, to be precise)
     uint32_t barrier;     // shared address of the chain's MMA-completion mbarrier
     uint32_t giveUp;      // shared address of the chain's give-up word for the current tile (LayerBarrier)
@@ -484,13 +490,12 @@ __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
     if (kRefOperandInShared<kLayer>)
         FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
-    if (LayerBarrier<kLayer>(ctx.tid, ctx.giveUp))
+    if (LayerBarrier<kLayer>(ctx.warp >> 2, ctx.giveUp))
         return 1;
 
     // The whole issuing warp runs the descriptor arithmetic on values that are visibly the same in every
     // lane; one elected lane hands the work to the tensor core (see IssueLayerRefFp8).
-    const int warpIndex = ctx.tid >> 5;
-    if (WarpRole(warpIndex) == kIssuingRole)
+    if (WarpRole(ctx.warp) == kIssuingRole)
     {
         TcgenFenceAfterSync();
         constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
@@ -504,8 +509,8 @@ __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
         // the matrix of biases, read twice (leading offset 0): its second copy meets the zeros
         const uint64_t biasBase = MakeSmemDescriptor(networkBase + kRefInt8BiasOffset, 0, 128);
         const uint32_t elected = ElectOne();
-        const int chain = __shfl_sync(0xFFFFFFFFu, warpIndex >> 2, 0);
-        const uint32_t accumulators = __shfl_sync(0xFFFFFFFFu, ctx.tmemLane & 0xFFFFu, 0); // the columns, at lane 0
+        const int chain = ctx.warp >> 2;
+        const uint32_t accumulators = ctx.accumulators;
         const uint64_t chainOperand = operandBase + uint64_t(uint32_t(chain) * uint32_t(kRefOperandBytes >> 4));
         // accumulators := bias (rows e_l times the matrix whose column l is the layer's bias: exact)
         UmmaF16(accumulators, onesBase, biasBase, instr, 0, elected);
@@ -695,7 +700,7 @@ __device__ __forceinline__ void DecodeRuns(const KernelParams& params)
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int warp = tid >> 5;
+    const int warp = int(Uniform(uint32_t(tid) >> 5));
     const int chain = warp >> 2, role = WarpRole(warp);
     const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
 
@@ -731,8 +736,10 @@ __device__ __forceinline__ void DecodeRuns(const KernelParams& params)
 
     RefTileContext ctx;
     ctx.tid = tid;
+    ctx.warp = warp;
+    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerHalf;
     // a warp may only touch the TMEM lanes 32 * (warp % 4) .. + 31
-    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
     ctx.barrier = SharedAddress(&shared.barrier[chain]);
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * (sizeof(Storage::operandA) / kMaxChains)) + (tid & 127);
@@ -849,7 +856,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
     __shared__ KernelMip mipTable[16];
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = int(Uniform(uint32_t(tid) >> 5));
     const int chain = warp >> 2;
 
     // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCtaRef)
@@ -861,7 +868,9 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.warp = warp;
+    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerHalf;
+    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
     ctx.barrier = SharedAddress(&shared.barrier[chain]);
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
@@ -1128,19 +1137,17 @@ __device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
     else
         FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
-    if (LayerBarrier<kLayer>(ctx.tid, ctx.giveUp))
+    if (LayerBarrier<kLayer>(ctx.warp >> 2, ctx.giveUp))
         return 1;
     // The whole issuing warp runs the descriptor arithmetic, on values the compiler can see are the same
-    // in every lane (hence the shuffles, and addresses counted from the start of dynamic shared memory instead of taken from
-    // the context: five shuffles per layer less were 2 %), and one elected lane hands the work to the tensor core: issued
-    // from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
+    // in every lane (RefTileContext; addresses counted from the start of dynamic shared memory), and one elected lane hands the work to
+    // the tensor core: issued from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
     // (Tried: building the descriptors before the barrier - 3 % slower.)
-    const int warpIndex = ctx.tid >> 5;
-    if (WarpRole(warpIndex) == kIssuingRole)
+    if (WarpRole(ctx.warp) == kIssuingRole)
     {
         TcgenFenceAfterSync();
         const uint32_t elected = ElectOne();
-        IssueChainRefFp8<kLayer>(__shfl_sync(0xFFFFFFFFu, warpIndex >> 2, 0), __shfl_sync(0xFFFFFFFFu, ctx.tmemLane & 0xFFFFu, 0), elected);
+        IssueChainRefFp8<kLayer>(ctx.warp >> 2, ctx.accumulators, elected);
     }
     return 0;
 }
@@ -1354,7 +1361,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const
     __shared__ KernelMip mipTable[16];
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = int(Uniform(uint32_t(tid) >> 5));
     const int chain = warp >> 2;
 
     if (tid < params.numMips)
@@ -1365,7 +1372,9 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const
 
     RefTileContext ctx;
     ctx.tid = tid;
-    ctx.tmemLane = shared.tmemBase + chain * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
+    ctx.warp = warp;
+    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerHalf;
+    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
     ctx.barrier = SharedAddress(&shared.barrier[chain]);
     ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
     ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kOperandBytes) + (tid & 127);

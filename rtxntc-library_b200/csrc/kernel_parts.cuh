@@ -400,6 +400,13 @@ __device__ __forceinline__ uint32_t ElectOne()
     return elected;
 }
 
+// The same value of a warp's first lane in all of its lanes, visibly so: what is computed from it stays in uniform registers, and branches on it
+// need no reconvergence.
+__device__ __forceinline__ uint32_t Uniform(uint32_t value)
+{
+    return __shfl_sync(0xFFFFFFFFu, value, 0);
+}
+
 // All 128 threads of a chain.
 __device__ __forceinline__ void ChainBarrier(int chain)
 {
@@ -421,9 +428,9 @@ __device__ __forceinline__ void SetGiveUp(uint32_t word)
 }
 
 template <int kLayer>
-__device__ __forceinline__ uint32_t LayerBarrier(int tid, uint32_t& giveUp)
+__device__ __forceinline__ uint32_t LayerBarrier(int chain, uint32_t& giveUp)
 {
-    ChainBarrier(tid >> 7);
+    ChainBarrier(chain);
     if (kLayer != 0)
         return 0;
     uint32_t word;
