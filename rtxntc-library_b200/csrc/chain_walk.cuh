@@ -1,0 +1,458 @@
+// What the decode kernels share around their layers: a CTA per SM of up to eight chains of 128 threads, which share the network and nothing
+// else.  A chain walks runs of tiles (DecodeRuns) or tiles of queries (SampleTiles); how a layer is issued and consumed is its kernel's (`Chain`).
+#pragma once
+
+#include <cuda_fp16.h>
+#include <stdint.h>
+
+#include <atomic>
+#include <cstddef>
+
+#include "decode_kernel.h"
+#include "kernel_parts.cuh"
+#include "input_stage.cuh"
+#include "output_convert.cuh"
+
+namespace ntcb
+{
+namespace
+{
+
+// What a chain prepares per run of tiles.
+template <typename Tables, int kHiBytes, int kLoBytes>
+struct __align__(16) ChainStage
+{
+    Tables tables;
+    uint8_t footprintHi[kHiBytes];
+    uint8_t footprintLo[kLoBytes];
+};
+
+// What the threads of a chain keep of their texel's place in a tile while the tables stay the same: with power-of-two sizes that is from the
+// first inner run of a mip on, and the tiles of a run differ by whole latent pixels (`shift` in DecodeRuns).  The positional encoding stays in the operand row, whose last chunks only the input stage writes.  (Worked out per
+// tile - eight products and eight conversions - a 4096 x 4096 FP8 set took 867 us instead of 851.)
+struct __align__(16) TexelTables
+{
+    uint4 weights[2][128]; // per grid and texel: w00, w01, w10, w11, each twice
+    uint4 taps[128];       // byte offset of the upper left tap and bytes per footprint row, high-res and low-res grid
+};
+
+// ... of the kernels whose layer-0 operand is 64-byte rows of codes.
+struct __align__(16) CodesStage : ChainStage<TileTables<ChainTile>, kRefFootprintHiBytes, kRefFootprintLoBytes>
+{
+    TexelTables texels;
+};
+
+
+template <typename Stage>
+__device__ __forceinline__ void PrepareTexel(Stage& stage, int texel, int column, int tileRow)
+{
+    uint32_t offsets[4];
+#pragma unroll
+    for (int grid = 0; grid < 2; ++grid)
+    {
+        const int2 col = stage.tables.taps.colTap[grid][column];
+        const int4 row = stage.tables.taps.rowTap[grid][tileRow];
+        const float dx = __int_as_float(col.y), dxn = __fsub_rn(1.f, dx);
+        const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
+        // src/FeatureGridDevice.h:46-49
+        const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);
+        stage.texels.weights[grid][texel] = make_uint4(AsU32(__floats2half2_rn(f00, f00)), AsU32(__floats2half2_rn(f01, f01)),
+                                                       AsU32(__floats2half2_rn(f10, f10)), AsU32(__floats2half2_rn(f11, f11)));
+        offsets[2 * grid] = uint32_t(col.x + row.x);
+        offsets[2 * grid + 1] = uint32_t(row.w);
+    }
+    stage.texels.taps[texel] = make_uint4(offsets[0], offsets[1], offsets[2], offsets[3]);
+}
+
+// Calls blend(grid, layer, four taps, four weights) for the latents of a texel in the staged footprints.  `shift`: bytes the taps of a
+// grid lie past those in TexelTables.
+template <int kLayers, typename Stage, typename Blend>
+__device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, int2 shift, Blend blend)
+{
+    const uint4 taps = stage.texels.taps[texel];
+    const int stride = StrideBytes<kLayers>(mip);
+#pragma unroll
+    for (int grid = 0; grid < 2; ++grid)
+    {
+        const uint4 w = stage.texels.weights[grid][texel];
+        const uint8_t* tap00 = grid ? stage.footprintLo + (taps.z + shift.y) : stage.footprintHi + (taps.x + shift.x);
+        const uint8_t* tap10 = tap00 + (grid ? taps.w : taps.y);
+#pragma unroll
+        for (int layer = 0; layer < 4; ++layer)
+        {
+            if (layer < NumLayers<kLayers>(params))
+                blend(grid, layer, *reinterpret_cast<const uint2*>(tap00 + layer * 8), *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8),
+                    *reinterpret_cast<const uint2*>(tap10 + layer * 8), *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8),
+                    AsHalf2(w.x), AsHalf2(w.y), AsHalf2(w.z), AsHalf2(w.w));
+        }
+    }
+}
+
+// Dynamic shared memory of a CTA of `chains` chains, each with an operand and `perChain` more bytes.
+template <typename Storage>
+constexpr size_t SharedBytes(int chains, size_t perChain)
+{
+    return offsetof(Storage, operandA) + chains * (sizeof(Storage::operandA) / kMaxChains + perChain);
+}
+
+// What `chain` prepares per tile: after the operands of all chains.
+template <typename Stage, typename Storage>
+__device__ __forceinline__ Stage& StageOf(Storage& shared, int chain)
+{
+    return reinterpret_cast<Stage*>(shared.operandA + (blockDim.x >> 7) * (sizeof(Storage::operandA) / kMaxChains))[chain];
+}
+
+// Inference on sample: tiles of 128 queries are claimed, not dealt.  The chains of a CTA draw from a counter in shared memory, two tiles
+// ahead, as the queries are requested one tile ahead; tile k of CTA b is tile b + k * gridDim.x.  The threads of a chain read the claim between
+// the barriers of layers 0 and 1.  (16.7 M queries: 780 us dealt, 768 claimed; the tiles of a decode, whose costs differ less, are dealt: claimed
+// they take 2 % longer.)
+template <typename Storage>
+__device__ __forceinline__ void ClaimTile(Storage& shared, int chain)
+{
+    if ((threadIdx.x & 127) == 0)
+        shared.claimed[chain] = atomicAdd(&shared.claims, 1u);
+}
+
+// What a warp of a chain does besides its texels: roles 0 and 1 stage the footprints of the high-res and the low-res grid (2 and 3 the rest of large
+// ones), role 3 hands the products to the tensor core.  All four meet before every layer, so the busiest sets the pace.
+// Warp w of every chain runs on sub-partition w % 4 of the SM, so the roles go round from chain to chain.
+// (Warp 0 staging and issuing in every chain: 4096 x 4096 FP8 832 us, 8192 x 8192 Int8 4530, 16.7 M queries 725.  Issued by warp 3 instead: 775,
+// 4210, 723.  Rotated: 780, 4190, 692, and 8-bit pixels 962 instead of 985.)
+constexpr int kIssuingRole = 3;
+__device__ __forceinline__ int WarpRole(int warpIndex)
+{
+    return (warpIndex + (warpIndex >> 2)) & 3;
+}
+
+struct ChainContext
+{
+    int tid;
+    // The same in all lanes of a warp (Uniform): the thread's warp, and its chain's first tensor-memory column at lane 0.  What follows from
+    // them - roles, barriers, the place of a tile and its mip's constants - lives in uniform registers.  (Taken from the thread's
+    // index, all of that took vector registers, and branches on it reconverged: 8192 x 8192 Int8 3803 -> 3640 us, 4096 x 4096 FP8 664 -> 649,
+    // its 8-bit pixels 874 -> 828, 16.7 M queries 658 -> 641.)
+    int warp;
+    uint32_t accumulators;
+    uint32_t tmemLane;    // the chain's first tensor-memory column at this thread's lane (its warp's first lane, to be precise)
+    uint32_t barrier;     // shared address of the chain's MMA-completion mbarrier
+    uint32_t giveUp;      // shared address of the chain's give-up word for the current tile (LayerBarrier)
+    uint4* rowChunk; // this thread's 16-byte slot in chunk 0 of its chain's A operand
+    int tile, x, y;
+    uint32_t* out;
+    uint32_t outStepWords;
+    int storeBytes; // widest store the texel may go out with (KernelMip::storeBytes)
+};
+
+// The 64-byte operand row of a texel: 48 inputs as codes, then K padding - zeros (e4m3) or the constant inputs of the bias slots (int8).
+// `column`: in the run.  `known`: TexelTables, and the row's last two chunks where the layers after the first leave them alone (FP8: their operands are
+// in tensor memory), are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
+template <bool kFp8, bool kReferenceDivision, int kLayers>
+__device__ __forceinline__ void BuildCodes(const KernelParams& params, const KernelMip& mip, CodesStage& stage, const ChainContext& ctx,
+    int column, int tileRow, bool known, int2 shift)
+{
+    if (!mip.staged)
+    {
+        BuildInputs<kFp8, kReferenceDivision, kLayers>(params, mip, stage, ctx, column, tileRow);
+        return;
+    }
+    const int texel = ctx.tid & 127;
+    if (!known)
+        PrepareTexel(stage, texel, column, tileRow);
+    if (!known || !kFp8)
+    {
+        // positional encoding: interleave the column's x bytes with the row's y bytes
+        const uint2 cx = stage.tables.colEnc[column];
+        const uint2 ry = stage.tables.rowEnc[tileRow];
+        ctx.rowChunk[2 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5140), __byte_perm(cx.x, ry.x, 0x7362),
+                                           __byte_perm(cx.y, ry.y, 0x5140), stage.tables.lodWord);
+        ctx.rowChunk[3 * 128] = PaddingCodes<kFp8>();
+    }
+    uint32_t words[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        words[i] = QuantizedZeros<kFp8>(); // unused feature slots hold quantised zeros (src/Inference.cu:49)
+    GatherTexel<kLayers>(params, mip, stage, texel, shift, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00, __half2 w01,
+        __half2 w10, __half2 w11) { words[4 * grid + layer] = BlendLayer<kFp8>(l00, l01, l10, l11, w00, w01, w10, w11); });
+    ctx.rowChunk[0] = make_uint4(words[0], words[1], words[2], words[3]);
+    ctx.rowChunk[128] = make_uint4(words[4], words[5], words[6], words[7]);
+}
+
+// End of a CTA: agrees on whether anything went wrong, gives work in flight one more bounded chance
+// to drain, and releases the tensor memory.
+template <typename Storage>
+__device__ __forceinline__ void TeardownCta(Storage& shared, const ChainContext& ctx, uint32_t phase,
+    int tid, int warp)
+{
+    TcgenFenceBeforeSync();
+    __syncthreads();
+    const volatile uint32_t* gaveUp = &shared.giveUp[warp >> 2][0];
+    if ((tid & 127) == 0 && (gaveUp[0] | gaveUp[1]))
+    {
+        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1);
+        (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
+    }
+    __syncthreads();
+    if (warp == 0)
+        TmemFree(shared.tmemBase, (blockDim.x >> 7) * kTmemColumnsPerChain);
+}
+
+// A chain's share of a launch.  `Chain` says how its tiles are prepared, fed and consumed.
+//
+// The unit of work is a run of up to kMaxRunTiles tiles side by side (KernelMip::runTiles).  Tables and footprints are made once per run, by all
+// four warps, under the products of the run before: the footprints of neighbouring tiles overlap (with a grid at a quarter of the mip's resolution
+// four tiles have 72 + 30 latent pixels, one has 24 + 12), the latents' way from the L2 is waited for once, and finding the place of the
+// work is paid for once.
+template <typename Chain, int kConvert, int kLayers>
+__device__ __forceinline__ void DecodeRuns(const KernelParams& params)
+{
+    extern __shared__ __align__(128) unsigned char dynamicShared[];
+    using Storage = typename Chain::Storage;
+    using Stage = typename Chain::Stage;
+    Storage& shared = *reinterpret_cast<Storage*>(dynamicShared);
+
+    const int tid = threadIdx.x;
+    const int lane = tid & 31;
+    const int warp = int(Uniform(uint32_t(tid) >> 5));
+    const int chain = warp >> 2, role = WarpRole(warp);
+    const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
+
+    Stage& stage = StageOf<Stage>(shared, chain);
+    // the first chains of all CTAs take the first runs, so that a launch of few spreads over the SMs
+    uint32_t run = blockIdx.x + uint32_t(chain) * gridDim.x;
+    // (What can be worked out from these is, tile by tile: the registers are worth more than the instructions.)
+    int mipIndex = 0, x0 = 0, y0 = 0; // the next tile's mip and place
+    bool known = false;               // the tables, and what the threads keep of them, are already the next tile's
+    int tablesMip = -1;               // mip whose tables are in shared memory and valid for every inner run of it
+    auto prepareRun = [&](auto between) {
+        while (mipIndex + 1 < params.numMips && run >= uint32_t(params.mips[mipIndex + 1].firstTile))
+            ++mipIndex; // runs are visited in increasing order, so the search resumes at the current mip
+        const KernelMip& mip = params.mips[mipIndex];
+        const int local = int(run) - mip.firstTile;
+        const int row = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
+        const int columns = mip.runTiles * kChainTileWidth;
+        x0 = (local - row * mip.tilesX) * columns;
+        y0 = mip.rowBegin + row * kChainTileHeight;
+        const bool keeps = TileKeepsTables<ChainTile>(mip, x0, y0, columns);
+        // the tables of the previous run serve this one too when both lie inside the same mip with invariant tables
+        known = keeps && mipIndex == tablesMip;
+        Chain::template Prepare<kLayers>(params, mip, stage, x0, y0, columns, lane, role, known, between);
+        tablesMip = keeps ? mipIndex : -1;
+    };
+    Chain::Setup(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [&](auto dependency) {
+        if (run < uint32_t(params.totalTiles))
+            prepareRun(dependency);
+        else
+            dependency();
+    });
+    uint32_t phase = 0;
+
+    ChainContext ctx;
+    ctx.tid = tid;
+    ctx.warp = warp;
+    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerChain;
+    // a warp may only touch the TMEM lanes 32 * (warp % 4) .. + 31
+    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * (sizeof(Storage::operandA) / kMaxChains)) + (tid & 127);
+
+    while (run < uint32_t(params.totalTiles))
+    {
+        const KernelMip& mip = params.mips[mipIndex];
+        ctx.tile = int(run);
+        ctx.x = x0 + tileColumn;
+        ctx.y = y0 + tileRow;
+        // runs start at multiples of their width
+        const int column = x0 & (mip.runTiles * kChainTileWidth - 1);
+        const int steps = known ? column / kChainTileWidth * StrideBytes<kLayers>(mip) : 0;
+        Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known,
+            make_int2(steps * mip.hiStepX, steps * mip.loStepX));
+
+        // layer 0; while the tensor core works on it, prepare the chain's NEXT run (its tables and
+        // footprints replace this run's, which nobody reads after the barrier inside Issue)
+        if (Chain::template Issue<0>(ctx))
+            break; // some thread of the chain gave up on a wait
+        x0 += kChainTileWidth;
+        if (x0 < mip.width && (x0 & (mip.runTiles * kChainTileWidth - 1)))
+            known = tablesMip == mipIndex; // a run whose tables serve others: so does what the threads keep of its first tile
+        else if ((run += (blockDim.x >> 7) * gridDim.x) < uint32_t(params.totalTiles))
+            prepareRun([]() {});
+        Chain::template Consume<0, kConvertNone>(params, ctx, phase);
+
+        Chain::template Issue<1>(ctx);
+        Chain::template Consume<1, kConvertNone>(params, ctx, phase);
+        Chain::template Issue<2>(ctx);
+        Chain::template Consume<2, kConvertNone>(params, ctx, phase);
+        {
+            // where the texel goes (worked out only now: nothing of it has to stay in registers through the
+            // layers); the element index inside a mip fits 32 bits (checked on the host)
+            const bool planar = params.outputLayout == kLayoutPlanarPairs;
+            const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
+                                          : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
+            const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
+            if constexpr (kConvert != kConvertNone)
+            {
+                // pixels of dstChannels components, rows without padding; outOffset counts components
+                const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
+                const size_t component = size_t(mip.outOffset) + size_t(pixelIndex) * size_t(params.conversion.dstChannels);
+                unsigned char* bytes = reinterpret_cast<unsigned char*>(params.out) + component * BytesPerComponent(params.conversion.format);
+                ctx.out = inside ? reinterpret_cast<uint32_t*>(bytes) : nullptr;
+                ctx.outStepWords = pixelIndex;
+            }
+            else
+            {
+                ctx.out = inside ? reinterpret_cast<uint32_t*>(params.out + mip.outOffset + first) : nullptr;
+                ctx.outStepWords = planar ? uint32_t(mip.width) : 1u;
+                ctx.storeBytes = mip.storeBytes;
+            }
+        }
+        Chain::template Issue<3>(ctx);
+        Chain::template Consume<3, kConvert>(params, ctx, phase);
+    }
+    TeardownCta(shared, ctx, phase, tid, warp);
+}
+
+// Inference on sample with an operand of 8-bit codes: one thread per query (u, v, lod) -> the texel (mip = clamp(floor(lod)),
+// x = min(floor(u * W), W - 1), y likewise) is evaluated exactly as the decode kernel evaluates it (the reference's NtcSampleTextureSet takes
+// an integer texel and mip and runs the same network, include/libntc/shaders/Inference.hlsli:282-357).  Queries are incoherent, so the
+// taps are read straight from global memory.
+template <typename Chain, bool kFp8, bool kReferenceDivision, bool kInterleaved, int kLayers>
+__device__ __forceinline__ void SampleTiles(const SampleParams& params)
+{
+    extern __shared__ __align__(128) unsigned char dynamicShared[];
+    using Storage = typename Chain::Storage;
+    Storage& shared = *reinterpret_cast<Storage*>(dynamicShared);
+    __shared__ KernelMip mipTable[16];
+
+    const int tid = threadIdx.x;
+    const int warp = int(Uniform(uint32_t(tid) >> 5));
+    const int chain = warp >> 2;
+
+    if (tid < params.numMips)
+        mipTable[tid] = params.mips[tid];
+    const unsigned long long tiles = (params.numQueries + 127) / 128;
+    const int row = tid & 127;
+    // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
+    float nextU = 0.f, nextV = 0.f, nextLod = 0.f;
+    auto requestQuery = [&](unsigned long long ofTile) {
+        if (ofTile < tiles)
+        {
+            const unsigned long long q = min(ofTile * 128 + row, params.numQueries - 1);
+            nextU = __ldg(params.queries + 3 * q);
+            nextV = __ldg(params.queries + 3 * q + 1);
+            nextLod = __ldg(params.queries + 3 * q + 2);
+        }
+    };
+    unsigned long long tile = blockIdx.x + (unsigned long long)chain * gridDim.x, nextTile = tile + (blockDim.x >> 7) * gridDim.x;
+    // (the first ones under the network's way from the L2)
+    Chain::Setup(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [&](auto dependency) {
+        dependency();
+        requestQuery(tile);
+    });
+    uint32_t phase = 0;
+
+    ChainContext ctx;
+    ctx.tid = tid;
+    ctx.warp = warp;
+    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerChain;
+    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * (sizeof(Storage::operandA) / kMaxChains)) + (tid & 127);
+    ctx.outStepWords = 1;
+    ctx.storeBytes = params.storeBytes;
+
+    while (tile < tiles)
+    {
+        ClaimTile(shared, chain);
+        const unsigned long long query = tile * 128 + row;
+        const bool valid = query < params.numQueries;
+        const float u = nextU, v = nextV, lod = nextLod;
+        requestQuery(nextTile);
+        const int mipIndex = max(0, min(params.numMips - 1, int(floorf(lod))));
+        const KernelMip& mip = mipTable[mipIndex];
+        const int x = max(0, min(mip.width - 1, int(floorf(__fmul_rn(u, float(mip.width))))));
+        const int y = max(0, min(mip.height - 1, int(floorf(__fmul_rn(v, float(mip.height))))));
+        ctx.tile = int(tile);
+        ctx.x = x;
+        ctx.y = y;
+        ctx.out = valid ? reinterpret_cast<uint32_t*>(params.out + query * params.channels) : nullptr;
+
+        {
+            uint32_t words[16];
+            const uint32_t zeroWord = QuantizedZeros<kFp8>();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                words[i] = zeroWord; // unused feature slots hold quantised zeros (src/Inference.cu:49)
+            const uint4 padding = PaddingCodes<kFp8>();
+            words[12] = padding.x;
+            words[13] = padding.y;
+            words[14] = padding.z;
+            words[15] = padding.w;
+            SampleGridsDirect<kFp8, kReferenceDivision>(params.latents, kLayers ? kLayers : params.numLayers, mip, x, y, words, kInterleaved);
+            // src/RegressionKernels.h:59-85
+            float xf = __fmul_rn(float(x), mip.positionScale);
+            float yf = __fmul_rn(float(y), mip.positionScale);
+#pragma unroll
+            for (int wave = 0; wave < 3; ++wave)
+            {
+                const float ex = __fmaf_rn(Frac(xf), 2.f, -1.f), ey = __fmaf_rn(Frac(yf), 2.f, -1.f);
+                const float ez = __fmaf_rn(Frac(__fadd_rn(xf, 0.25f)), 2.f, -1.f);
+                const float ew = __fmaf_rn(Frac(__fadd_rn(yf, 0.25f)), 2.f, -1.f);
+                words[8 + wave] = QuantizeInputs<kFp8>(__floats2half2_rn(ex, ey), __floats2half2_rn(ez, ew));
+                xf = __fmul_rn(xf, 2.f);
+                yf = __fmul_rn(yf, 2.f);
+            }
+            words[11] = QuantizeLod<kFp8>(mip.positionLod);
+#pragma unroll
+            for (int chunk = 0; chunk < 4; ++chunk)
+                ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);
+        }
+
+        // nothing is shared between the chains of a query tile: each runs at its own pace
+        if (Chain::template Issue<0>(ctx))
+            break;
+        Chain::template Consume<0, kConvertNone>(params, ctx, phase);
+        tile = nextTile;
+        nextTile = blockIdx.x + (unsigned long long)shared.claimed[chain] * gridDim.x;
+        Chain::template Issue<1>(ctx);
+        Chain::template Consume<1, kConvertNone>(params, ctx, phase);
+        Chain::template Issue<2>(ctx);
+        Chain::template Consume<2, kConvertNone>(params, ctx, phase);
+        Chain::template Issue<3>(ctx);
+        Chain::template Consume<3, kConvertNone>(params, ctx, phase);
+    }
+    TeardownCta(shared, ctx, phase, tid, warp);
+}
+
+// One kernel, set up for its dynamic shared memory on first use per device (`done`: one bit per device).
+template <typename Kernel, typename Params>
+cudaError_t LaunchChains(Kernel kernel, std::atomic<unsigned long long>& done, size_t sharedBytes, size_t maxSharedBytes, int chains,
+    const Params& params, int ctas, cudaStream_t stream)
+{
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess)
+        return err;
+    const unsigned long long bit = 1ull << (device & 63);
+    if (!(done.load(std::memory_order_acquire) & bit))
+    {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(maxSharedBytes));
+        if (err != cudaSuccess)
+            return err;
+        done.fetch_or(bit, std::memory_order_release);
+    }
+    return LaunchOverlapped(kernel, ctas, 128 * chains, sharedBytes, stream, params);
+}
+
+// Chains of a CTA: no more than tiles, a power of two as the tensor-memory allocation has to be.
+int ChainsPerCta(unsigned long long tiles, int ctas)
+{
+    int chains = 1;
+    while (chains < kMaxChains && (unsigned long long)chains * (unsigned long long)ctas < tiles)
+        chains *= 2;
+    return chains;
+}
+
+} // namespace
+} // namespace ntcb

@@ -1,19 +1,18 @@
-// NTC decode kernel for sm_100a: one launch decodes every listed colour mip of a texture set.
+// NTC decode kernel for sm_100a with EXACT accumulation: one launch decodes every listed colour mip of a texture set.
 //
-// Work decomposition.  A tile is 32x8 texels; one CTA of 256 threads owns one tile at a time
-// (thread = texel) and walks the tile list of the whole mip chain with a grid stride.  The tile is
-// two 128-row GEMM chains (rows 0-3 and rows 4-7 of the tile; a thread's texel is one row of its
-// half's 128x{64,48,32,16} chain and one TMEM lane), issued together.  Several CTAs are resident
-// per SM, so the SIMT phases of one tile overlap the tensor-core phases of the others.
+// Work decomposition: chains of 128 threads on tiles of 16 x 8 texels (thread = texel = row of the 128 x {64,48,32,16} products = TMEM lane),
+// up to eight in the one CTA of an SM, walking runs of tiles of their own (chain_walk.cuh).  (As CTAs of 256 threads on tiles of 32 x 8, four to
+// an SM, with tables per tile, a CTA-wide reducing barrier before every layer and the products issued inside a divergent branch: 1920 x 1080
+// Int8 172 us, 2048 x 2048 Int8 347, 1536 x 1100 FP8 107, 300 x 200 FP8 9.4.  As chains 158, 305, 88 and 6.7.)
 //
 // Per tile:
-//   1. every thread samples the two latent grids for its texel (packed BGRA4 pixels, nibble ->
-//      binary16, bilinear blend in binary16), appends the positional encoding and quantises the 48 inputs to int8 codes or e4m3, and writes its 64-byte
+//   1. every thread samples the two latent grids for its texel (staged footprints of binary16 latents, bilinear blend in
+//      binary16), appends the positional encoding and quantises the 48 inputs to int8 codes or e4m3, and writes its 64-byte
 //      row of the A operand straight into the tensor core's K-major core-matrix order (a 16-byte
 //      chunk per store, consecutive threads hit consecutive chunks: conflict-free);
 //   2. one thread issues tcgen05.mma (kind::i8 or kind::f8f6f4, M=128, N=64/48/32/16, K=32 per
 //      instruction) against the weights resident in shared memory; accumulators live in TMEM;
-//   3. after the commit arrives on the mbarrier every thread pulls its row of accumulators with
+//   3. after the commit arrives on the chain's mbarrier every thread pulls its row of accumulators with
 //      tcgen05.ld, applies bias/scale and the clamped HGELU in packed binary16, re-quantises and
 //      writes the next layer's A operand over the previous one - with FP8 weights into tensor memory
 //      (tcgen05.st; the next product takes A from there), with Int8 weights into shared memory;
@@ -24,8 +23,8 @@
 // src/RegressionKernels.h:59-85, src/tin/tin_mlp.h:22-37, src/tin/tin_activation.h:88-104); the
 // matrix products accumulate exactly (int32, or fp32 for e4m3 operands) instead of in binary16.
 //
-// Every wait on the mbarrier is bounded; on expiry the CTA records an error in the status words,
-// skips the remaining tiles, releases its TMEM columns and exits.
+// Every wait on an mbarrier is bounded; on expiry the thread records an error in the status words, its chain
+// skips the remaining tiles, and the CTA releases its TMEM columns and exits.
 
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -34,10 +33,12 @@
 
 #include <atomic>
 #include <cstddef>
+#include <type_traits>
 
 #include "decode_kernel.h"
 #include "kernel_parts.cuh"
 #include "input_stage.cuh"
+#include "chain_walk.cuh"
 #include "output_convert.cuh"
 #include "epilogue_convert.cuh"
 
@@ -52,56 +53,60 @@ namespace
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 bytes of 8-bit operands.
 template <bool kFp8>
-__device__ __forceinline__ void Umma(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate)
+__device__ __forceinline__ void Umma(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate, uint32_t enabled)
 {
     if (kFp8)
     {
         asm volatile(
             "{\n\t"
-            ".reg .pred p;\n\t"
+            ".reg .pred p, q;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "l"(descA), "l"(descB), "r"(instr), "r"(accumulate)
+            "l"(descA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
             : "memory");
     }
     else
     {
         asm volatile(
             "{\n\t"
-            ".reg .pred p;\n\t"
+            ".reg .pred p, q;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "l"(descA), "l"(descB), "r"(instr), "r"(accumulate)
+            "l"(descA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
             : "memory");
     }
 }
 
 // The same with the A operand in tensor memory: 8 columns (32 bytes per lane) starting at `tmemA`.
 template <bool kFp8>
-__device__ __forceinline__ void UmmaFromTmem(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t instr, uint32_t accumulate)
+__device__ __forceinline__ void UmmaFromTmem(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t instr, uint32_t accumulate, uint32_t enabled)
 {
     if (kFp8)
     {
         asm volatile(
             "{\n\t"
-            ".reg .pred p;\n\t"
+            ".reg .pred p, q;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate)
+            "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
             : "memory");
     }
     else
     {
         asm volatile(
             "{\n\t"
-            ".reg .pred p;\n\t"
+            ".reg .pred p, q;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate)
+            "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
             : "memory");
     }
 }
@@ -152,52 +157,24 @@ __device__ __forceinline__ uint32_t PackCodes(uint32_t first, uint32_t second)
 // The kernel
 // ---------------------------------------------------------------------------------------------
 
-struct __align__(128) SharedStorage
+struct __align__(128) ExactStorage
 {
     uint8_t network[kStagedNetworkBytes]; // weights in core-matrix order, scales, biases
-    // the tensor core reads operands as 128-byte core matrices: keep them on 128-byte lines
-    alignas(128) uint8_t operandA[2 * kOperandBytes];  // A operands of the current layer (top half, bottom half), core-matrix order
     alignas(128) uint8_t biasRegion[kBiasRegionBytes]; // constant A operand of the bias K step of the int8 layers
-    uint64_t barrier;                     // MMA completion
-    uint64_t loadBarrier;                 // arrival of the network image (bulk copy)
+    uint64_t barrier[kMaxChains]; // MMA completion, per chain
+    uint64_t loadBarrier;         // arrival of the network image (bulk copy)
+    alignas(8) uint32_t giveUp[kMaxChains][2]; // see LayerBarrier
+    uint32_t claims;              // inference on sample: query tiles handed out so far
+    uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    // What inference on sample does not use comes last: its launches ask for the bytes before `stage` only.
-    // (With the whole structure, a sample kernel's own static shared memory - its table of mips - puts four CTAs
-    // above an SM's 228 KB: three were resident and the fourth quarter of the grid ran alone afterwards.)
-    struct alignas(128)
-    {
-        TileTables<WideTile> tables;
-        uint8_t footprintHi[kFootprintHiBytes]; // unpacked latents of the tile's footprint in the high-res grid
-        uint8_t footprintLo[kFootprintLoBytes]; // ... and in the low-res grid
-    } stage;
+    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands, 64 bytes a row, in core-matrix order; then the CodesStages
 };
+static_assert(sizeof(ExactStorage) + kMaxChains * sizeof(CodesStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
-
-struct TileContext
-{
-    int tid;
-    uint32_t tmemBase; // TMEM address of the CTA's accumulators: columns [0,64) top half, [64,128) bottom half
-    uint32_t tmemLane; // ... of this thread's half at this thread's lane
-    uint32_t barrier;  // shared address of the MMA-completion mbarrier
-    uint32_t operandA; // shared address of the A operands (top half, then bottom half)
-    uint4* rowChunk;   // this thread's 16-byte slot in chunk 0 of its half's A operand
-    uint32_t networkBase;
-    uint32_t biasRegion; // shared address of the constant A operand of the bias K step
-    int tile, x, y;
-    uint32_t* out;          // where this thread's first channel pair goes (nullptr: store nothing); with a
-                            // converting epilogue: the address of the thread's pixel in the client's format
-    uint32_t outStepWords;  // 32-bit words between consecutive channel pairs; with a converting epilogue:
-                            // the pixel's linear index in its mip (the dither seed)
-    int storeBytes;         // widest store the texel may go out with (KernelMip::storeBytes)
-};
-
-// First half of a layer of the MLP for the CTA's current tile: barrier and MMA issue (both halves
-// of the tile).  Returns nonzero (uniformly over the CTA) when some thread gave up on a wait.
-// (The default kernels' issue path - descriptors built warp-uniformly, an elected lane, one completion
-// barrier per chain, chain-local barriers between layers - was tried here too: no gain with FP8 weights,
-// 3.5 % slower with Int8 weights, where it spills under the 64-register cap.)
+// First half of a layer: hands the A operand written before this call to the tensor core, an elected lane of the warp of kIssuingRole.  Returns
+// nonzero (uniformly over the chain) when some thread gave up on a wait.
 template <bool kFp8, int kLayer>
-__device__ __forceinline__ int IssueLayer(const TileContext& ctx, int failed)
+__device__ __forceinline__ int IssueLayer(ChainContext& ctx)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
     constexpr int kK = kLayer == 3 ? 32 : 64;
@@ -214,39 +191,35 @@ __device__ __forceinline__ int IssueLayer(const TileContext& ctx, int failed)
     else
         FenceProxyAsyncShared();
     TcgenFenceBeforeSync();
-    if (__syncthreads_or(failed))
+    if (LayerBarrier<kLayer>(ctx.warp >> 2, ctx.giveUp))
         return 1;
 
-    // (A thread of the last warp: the first ones also stage footprints, and all wait for the busiest before the next layer.  2048 x 2048
-    // Int8 346.6 -> 343.9 us, FP8 273.4 -> 270.6.  Issued by that warp through an elected lane, as the reference-numerics kernels
-    // do, Int8 sets took 12 % longer.)
-    if (ctx.tid == kThreadsPerCta - 32)
+    if (WarpRole(ctx.warp) == kIssuingRole)
     {
         TcgenFenceAfterSync();
         constexpr uint32_t instr = MakeInstrDescriptor(kLayerFp8, kN);
+        const uint32_t elected = ElectOne();
+        const uint32_t base = DynamicSharedBase();
+        const int chain = ctx.warp >> 2;
+        const uint32_t accumulators = ctx.accumulators + kAccumulatorColumn<kFp8, kLayer>;
+        const uint64_t operandBase =
+            MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, operandA)) + uint32_t(chain) * uint32_t(kOperandBytes), 2048, 128);
+        const uint64_t weightBase = MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, network)) + kWeightOffset, kN * 16, 128);
 #pragma unroll
-        for (int half = 0; half < 2; ++half)
+        for (int kStep = 0; kStep < kK / 32; ++kStep)
         {
-#pragma unroll
-            for (int kStep = 0; kStep < kK / 32; ++kStep)
-            {
-                // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
-                uint64_t descA = MakeSmemDescriptor(ctx.operandA + half * kOperandBytes + kStep * 2 * 2048, 2048, 128);
-                uint64_t descB = MakeSmemDescriptor(ctx.networkBase + kWeightOffset + kStep * 2 * kN * 16, kN * 16, 128);
-                if (kOperandInTmem<kFp8, kLayer>)
-                    UmmaFromTmem<kLayerFp8>(ctx.tmemBase + half * kTmemColumnsPerHalf + kAccumulatorColumn<kFp8, kLayer>,
-                        ctx.tmemBase + half * kTmemColumnsPerHalf + kStep * 8, descB, instr, kStep != 0);
-                else
-                    Umma<kLayerFp8>(ctx.tmemBase + half * kTmemColumnsPerHalf, descA, descB, instr, kStep != 0);
-            }
-            if (kBiasStep)
-            {
-                uint64_t descA = MakeSmemDescriptor(ctx.biasRegion, 2048, 128);
-                uint64_t descB = MakeSmemDescriptor(ctx.networkBase + kWeightOffset + (kK / 32) * 2 * kN * 16, kN * 16, 128);
-                Umma<kLayerFp8>(ctx.tmemBase + half * kTmemColumnsPerHalf, descA, descB, instr, 1);
-            }
+            // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
+            const uint64_t descB = weightBase + uint64_t((kStep * 2 * kN * 16) >> 4);
+            if (kOperandInTmem<kFp8, kLayer>)
+                UmmaFromTmem<kLayerFp8>(accumulators, ctx.accumulators + kStep * 8, descB, instr, kStep != 0, elected);
+            else
+                Umma<kLayerFp8>(accumulators, operandBase + uint64_t((kStep * 2 * 2048) >> 4), descB, instr, kStep != 0, elected);
         }
-        UmmaCommit(ctx.barrier);
+        if (kBiasStep)
+            Umma<kLayerFp8>(accumulators, MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, biasRegion)), 2048, 128),
+                weightBase + uint64_t(((kK / 32) * 2 * kN * 16) >> 4), instr, 1, elected);
+        if (elected)
+            UmmaCommit(base + uint32_t(offsetof(ExactStorage, barrier)) + chain * 8);
     }
     return 0;
 }
@@ -254,18 +227,16 @@ __device__ __forceinline__ int IssueLayer(const TileContext& ctx, int failed)
 // Second half of a layer: waits for the MMA, then applies the activation and writes the next
 // layer's A operand (layers 0-2) or runs the output epilogue (layer 3).
 template <bool kFp8, int kLayer, int kConvert, bool kBiasTable, typename Params>
-__device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const SharedStorage& shared,
-    const TileContext& ctx, uint32_t& phase, int& failed)
+__device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const ExactStorage& shared, const ChainContext& ctx, uint32_t& phase)
 {
-    uint32_t* const status = params.status;
     const int channels = params.channels;
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
     constexpr bool kLayerFp8 = kFp8 && kLayer < 3;
 
     if (!MbarrierWaitBounded(ctx.barrier, phase))
     {
-        failed = 1;
-        ReportTimeout(status, uint32_t(ctx.tile), uint32_t(kLayer));
+        SetGiveUp(ctx.giveUp);
+        ReportTimeout(params.status, uint32_t(ctx.tile), uint32_t(kLayer));
     }
     phase ^= 1;
     TcgenFenceAfterSync();
@@ -381,34 +352,22 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Sha
 // Second half of a layer.  An int8 layer's bias is part of the accumulator already (bias slots of
 // the matrix product) unless the staged network says that it has to come from the table.
 template <bool kFp8, int kLayer, int kConvert, typename Params>
-__device__ __forceinline__ void ConsumeLayer(const Params& params, const SharedStorage& shared,
-    const TileContext& ctx, uint32_t& phase, int& failed)
+__device__ __forceinline__ void ConsumeLayer(const Params& params, const ExactStorage& shared, const ChainContext& ctx, uint32_t& phase)
 {
     // (FP8 mode has a single int8 layer of 16 outputs: it keeps the table)
     if (kFp8 || (*reinterpret_cast<const uint32_t*>(shared.network + kFlagsOffset) & kFlagBiasTable))
-        ConsumeLayerImpl<kFp8, kLayer, kConvert, true>(params, shared, ctx, phase, failed);
+        ConsumeLayerImpl<kFp8, kLayer, kConvert, true>(params, shared, ctx, phase);
     else
-        ConsumeLayerImpl<kFp8, kLayer, kConvert, false>(params, shared, ctx, phase, failed);
+        ConsumeLayerImpl<kFp8, kLayer, kConvert, false>(params, shared, ctx, phase);
 }
 
-template <bool kFp8, int kLayer, int kConvert, typename Params>
-__device__ __forceinline__ int RunLayer(const Params& params, const SharedStorage& shared,
-    const TileContext& ctx, uint32_t& phase, int& failed)
-{
-    if (IssueLayer<kFp8, kLayer>(ctx, failed))
-        return 1;
-    ConsumeLayer<kFp8, kLayer, kConvert>(params, shared, ctx, phase, failed);
-    return 0;
-}
-
-// One-time setup of a CTA: the network image arrives by one TMA bulk copy while the threads fill
-// the constant tables, set up the barriers and allocate tensor memory.  Returns nonzero, uniformly
-// over the CTA, when some thread gave up waiting for the image (status words written, one more
-// bounded wait for the copy done, tensor memory released): the caller returns at once.
-__device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp)
+// One-time setup of a CTA, as in the reference-numerics kernels (SetupCtaRef).
+template <typename First>
+__device__ __forceinline__ void SetupCta(ExactStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp,
+    First first)
 {
     // constant inputs of the bias K step: 31 slots of kBiasSlotValue and a last slot of 1 per row
-    for (int i = tid; i < kBiasRegionBytes / 16; i += kThreadsPerCta)
+    for (int i = tid; i < kBiasRegionBytes / 16; i += int(blockDim.x))
     {
         const uint32_t fill = kBiasSlotValue * 0x01010101u;
         reinterpret_cast<uint4*>(shared.biasRegion)[i] =
@@ -417,345 +376,129 @@ __device__ __forceinline__ int SetupCta(SharedStorage& shared, const uint8_t* ne
     const uint32_t loadBarrier = SharedAddress(&shared.loadBarrier);
     if (tid == 0)
     {
-        MbarrierInit(SharedAddress(&shared.barrier), 1);
+        for (int chain = 0; chain < kMaxChains; ++chain)
+        {
+            MbarrierInit(SharedAddress(&shared.barrier[chain]), 1);
+            shared.giveUp[chain][0] = shared.giveUp[chain][1] = 0;
+        }
+        shared.claims = 2 * (blockDim.x >> 7);
         MbarrierInit(loadBarrier, 1);
         FenceBarrierInit();
     }
     if (warp == 0)
-        TmemAlloc(SharedAddress(&shared.tmemBase), kTmemColumns);
-    GridDependencyWait();
-    if (tid == 0)
-    {
-        MbarrierArriveExpectTx(loadBarrier, kStagedNetworkBytes);
-        BulkCopyToShared(SharedAddress(shared.network), network, kStagedNetworkBytes, loadBarrier);
-    }
+        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerChain);
+    first([&]() {
+        GridDependencyWait();
+        if (tid == 0)
+        {
+            MbarrierArriveExpectTx(loadBarrier, kStagedNetworkBytes);
+            BulkCopyToShared(SharedAddress(shared.network), network, kStagedNetworkBytes, loadBarrier);
+        }
+    });
     FenceProxyAsyncShared(); // the bias region is read by the tensor core (async proxy)
     TcgenFenceBeforeSync();
     __syncthreads();         // also publishes the barriers' initialisation
     TcgenFenceAfterSync();
     GridDependencyLaunch();
-    int failed = 0;
     if (!MbarrierWaitBounded(loadBarrier, 0, loadWaitPolls))
     {
-        failed = 1;
+        SetGiveUp(SharedAddress(&shared.giveUp[tid >> 7][0]));
         ReportTimeout(status, 0xFFFFFFFFu, 0xFFFFFFFFu); // no tile: the network image did not arrive
     }
-    if (__syncthreads_or(failed))
-    {
-        if (tid == 0)
-            (void)MbarrierWaitBounded(loadBarrier, 0);
-        __syncthreads();
-        if (warp == 0)
-            TmemFree(shared.tmemBase, kTmemColumns);
-        return 1;
-    }
-    return 0;
 }
+
+// A chain with exact accumulation.
+template <bool kFp8>
+struct ExactChain
+{
+    using Storage = ExactStorage;
+    using Stage = CodesStage;
+    template <typename First>
+    static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp,
+        First first)
+    {
+        SetupCta(shared, network, status, polls, tid, warp, first);
+    }
+    template <int kLayers, typename Between>
+    static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
+        int lane, int role, bool tablesValid, Between between)
+    {
+        PrepareTile<ChainTile, kFp8, false, kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid, between);
+    }
+    template <int kLayers>
+    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const ChainContext& ctx,
+        int column, int tileRow, bool known, int2 shift)
+    {
+        BuildCodes<kFp8, false, kLayers>(params, mip, stage, ctx, column, tileRow, known, shift);
+    }
+    template <int kLayer>
+    static __device__ __forceinline__ int Issue(ChainContext& ctx)
+    {
+        return IssueLayer<kFp8, kLayer>(ctx);
+    }
+    template <int kLayer, int kConvert, typename Params>
+    static __device__ __forceinline__ void Consume(const Params& params, const ChainContext& ctx, uint32_t& phase)
+    {
+        extern __shared__ __align__(128) unsigned char dynamicShared[];
+        ConsumeLayer<kFp8, kLayer, kConvert>(params, *reinterpret_cast<const Storage*>(dynamicShared), ctx, phase);
+    }
+};
 
 template <bool kFp8, int kConvert, int kLayers>
-__global__ void __launch_bounds__(kThreadsPerCta, kConvert != kConvertNone ? kCtasPerSmConverting : kFp8 ? kCtasPerSmFp8 : kCtasPerSmInt8)
-    DecodeKernel(const __grid_constant__ KernelParams params)
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernel(const __grid_constant__ KernelParams params)
 {
-    // more than the 48 KB a kernel may declare statically: passed as dynamic shared memory at launch
-    extern __shared__ __align__(128) unsigned char dynamicShared[];
-    SharedStorage& shared = *reinterpret_cast<SharedStorage*>(dynamicShared);
-
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = tid >> 5;      // = the thread's row of the tile
-    const int half = warp >> 2;     // 0: rows 0-3 of the tile, 1: rows 4-7
-
-    if (SetupCta(shared, params.network, params.status, params.loadWaitPolls, tid, warp))
-        return;
-    int failed = 0;   // this thread gave up on a wait
-    const uint32_t tmemBase = shared.tmemBase;
-    uint32_t phase = 0;
-    int aborted = 0;  // some thread of the CTA did (uniform: comes out of a barrier)
-
-    TileContext ctx;
-    ctx.tid = tid;
-    ctx.tmemBase = tmemBase;
-    // a warp may only touch the TMEM lanes 32 * (warp % 4) .. + 31
-    ctx.tmemLane = tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier);
-    ctx.operandA = SharedAddress(shared.operandA);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kOperandBytes) + (tid & 127);
-    ctx.networkBase = SharedAddress(shared.network);
-    ctx.biasRegion = SharedAddress(shared.biasRegion);
-
-    // Position of a tile in its mip.
-    struct TilePlace
-    {
-        int mipIndex, tileX0, tileY0;
-    };
-    auto locate = [&](int tile, int fromMip) {
-        // tiles are visited in increasing order, so the search resumes at the current mip
-        TilePlace place;
-        place.mipIndex = fromMip;
-        while (place.mipIndex + 1 < params.numMips && tile >= params.mips[place.mipIndex + 1].firstTile)
-            ++place.mipIndex;
-        const KernelMip& mip = params.mips[place.mipIndex];
-        const int local = tile - mip.firstTile;
-        // local / tilesX through a precomputed reciprocal where that is exact for every tile of the mip (FillKernelMip)
-        const int tileY = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
-        place.tileX0 = (local - tileY * mip.tilesX) * kTileWidth;
-        place.tileY0 = mip.rowBegin + tileY * kTileHeight;
-        return place;
-    };
-
-    int tile = blockIdx.x;
-    TilePlace place{0, 0, 0};
-    int tablesMip = -1; // mip whose tap / encoding tables are in shared memory and valid for every inner tile of it
-    if (tile < params.totalTiles)
-    {
-        // ---- tables and latent footprints of the first tile -----------------------------------
-        place = locate(tile, 0);
-        PrepareTile<WideTile, kFp8, false, kLayers>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, kTileWidth, lane, warp, false, []() {});
-        tablesMip = TileKeepsTables<WideTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0, kTileWidth) ? place.mipIndex : -1;
-        __syncthreads();
-    }
-    while (tile < params.totalTiles)
-    {
-        const KernelMip& mip = params.mips[place.mipIndex];
-        ctx.tile = tile;
-        ctx.x = place.tileX0 + lane;
-        ctx.y = place.tileY0 + warp;
-        {
-            // element index inside the mip fits 32 bits (8192^2 texels x 16 channels is 2^30)
-            const bool planar = params.outputLayout == kLayoutPlanarPairs;
-            const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
-                                          : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
-            const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
-            if constexpr (kConvert != kConvertNone)
-            {
-                // pixels of dstChannels components, rows without padding; outOffset counts components
-                const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
-                const size_t component = size_t(mip.outOffset) + size_t(pixelIndex) * size_t(params.conversion.dstChannels);
-                unsigned char* bytes = reinterpret_cast<unsigned char*>(params.out) + component * BytesPerComponent(params.conversion.format);
-                ctx.out = inside ? reinterpret_cast<uint32_t*>(bytes) : nullptr;
-                ctx.outStepWords = pixelIndex;
-            }
-            else
-            {
-                ctx.out = inside ? reinterpret_cast<uint32_t*>(params.out + mip.outOffset + first) : nullptr;
-                ctx.outStepWords = planar ? uint32_t(mip.width) : 1u; // channel pairs are 2 * width or 2 elements apart
-                ctx.storeBytes = mip.storeBytes;
-            }
-        }
-
-        // ---- 1. this tile's network inputs -> A operand (the last MMA that read the A operand has
-        //         completed: every thread waited for it) -------------------------------------------
-        BuildInputs<kFp8, false, kLayers>(params, mip, shared.stage, ctx, lane, warp);
-
-        // ---- 2. layer 0; while the tensor core works on it, prepare the NEXT tile: its tables and
-        //         footprints replace this tile's, which nobody reads after the barrier inside
-        //         IssueLayer, and the global-memory latency of the footprint hides behind the MMA ----
-        aborted = IssueLayer<kFp8, 0>(ctx, failed);
-        if (aborted)
-            break;
-        const int nextTile = tile + int(gridDim.x);
-        if (nextTile < params.totalTiles)
-        {
-            place = locate(nextTile, place.mipIndex);
-            // the tables of the previous tile serve this one too when both lie inside the same mip with invariant tables
-            const bool keepsTables = TileKeepsTables<WideTile>(params.mips[place.mipIndex], place.tileX0, place.tileY0, kTileWidth);
-            PrepareTile<WideTile, kFp8, false, kLayers>(params, params.mips[place.mipIndex], shared.stage, place.tileX0, place.tileY0, kTileWidth, lane, warp, keepsTables && place.mipIndex == tablesMip, []() {});
-            tablesMip = keepsTables ? place.mipIndex : -1;
-        }
-        ConsumeLayer<kFp8, 0, kConvertNone>(params, shared, ctx, phase, failed);
-
-        // ---- 3./4. layers 1-3 (their barriers also order the next tile's tables before its use) ---
-        aborted = RunLayer<kFp8, 1, kConvertNone>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 2, kConvertNone>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 3, kConvert>(params, shared, ctx, phase, failed);
-        if (aborted)
-            break;
-        tile = nextTile;
-    }
-
-    // ---- teardown -------------------------------------------------------------------------
-    TcgenFenceBeforeSync();
-    aborted = __syncthreads_or(failed);
-    if (aborted && tid == 0)
-        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1); // one more bounded chance for work in flight to drain
-    __syncthreads();
-    if (warp == 0)
-        TmemFree(tmemBase, kTmemColumns);
+    DecodeRuns<ExactChain<kFp8>, kConvert, kLayers>(params);
 }
 
-// Inference on sample: one thread per query (u, v, lod) -> the texel (mip = clamp(floor(lod)),
-// x = min(floor(u * W), W - 1), y likewise) is evaluated exactly as the decode kernel evaluates it
-// (the reference's NtcSampleTextureSet takes an integer texel and mip and runs the same network,
-// include/libntc/shaders/Inference.hlsli:282-357).  Queries are incoherent, so the taps are read
-// straight from global memory; a tile is 256 consecutive queries, i.e. two 128-row GEMM chains.
 template <bool kFp8, bool kInterleaved, int kLayers>
-__global__ void __launch_bounds__(kThreadsPerCta, kFp8 ? kCtasPerSmFp8 : kCtasPerSmInt8) SampleKernel(const __grid_constant__ SampleParams params)
+__global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernel(const __grid_constant__ SampleParams params)
 {
-    // more than the 48 KB a kernel may declare statically: passed as dynamic shared memory at launch
-    extern __shared__ __align__(128) unsigned char dynamicShared[];
-    SharedStorage& shared = *reinterpret_cast<SharedStorage*>(dynamicShared);
-    __shared__ KernelMip mipTable[16];
-
-    const int tid = threadIdx.x;
-    const int warp = tid >> 5;
-    const int half = warp >> 2;
-
-    // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCta)
-    if (tid < params.numMips)
-        mipTable[tid] = params.mips[tid];
-    if (SetupCta(shared, params.network, params.status, params.loadWaitPolls, tid, warp))
-        return;
-    int failed = 0, aborted = 0;
-    const uint32_t tmemBase = shared.tmemBase;
-    uint32_t phase = 0;
-
-    TileContext ctx;
-    ctx.tid = tid;
-    ctx.tmemBase = tmemBase;
-    ctx.tmemLane = tmemBase + half * kTmemColumnsPerHalf + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier);
-    ctx.operandA = SharedAddress(shared.operandA);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + half * kOperandBytes) + (tid & 127);
-    ctx.networkBase = SharedAddress(shared.network);
-    ctx.biasRegion = SharedAddress(shared.biasRegion);
-    ctx.outStepWords = 1;
-    ctx.storeBytes = params.storeBytes;
-
-    const unsigned long long tiles = (params.numQueries + kThreadsPerCta - 1) / kThreadsPerCta;
-    // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
-    float nextU = 0.f, nextV = 0.f, nextLod = 0.f;
-    auto requestQuery = [&](unsigned long long ofTile) {
-        if (ofTile < tiles)
-        {
-            const unsigned long long q = min(ofTile * kThreadsPerCta + tid, params.numQueries - 1);
-            nextU = __ldg(params.queries + 3 * q);
-            nextV = __ldg(params.queries + 3 * q + 1);
-            nextLod = __ldg(params.queries + 3 * q + 2);
-        }
-    };
-    requestQuery(blockIdx.x);
-    for (unsigned long long tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-    {
-        const unsigned long long query = tile * kThreadsPerCta + tid;
-        const bool valid = query < params.numQueries;
-        const float u = nextU, v = nextV, lod = nextLod;
-        requestQuery(tile + gridDim.x);
-        const int mipIndex = max(0, min(params.numMips - 1, int(floorf(lod))));
-        const KernelMip& mip = mipTable[mipIndex];
-        const int x = max(0, min(mip.width - 1, int(floorf(__fmul_rn(u, float(mip.width))))));
-        const int y = max(0, min(mip.height - 1, int(floorf(__fmul_rn(v, float(mip.height))))));
-        ctx.tile = int(tile);
-        ctx.x = x;
-        ctx.y = y;
-        ctx.out = valid ? reinterpret_cast<uint32_t*>(params.out + query * params.channels) : nullptr;
-
-        {
-            uint32_t words[16];
-            const uint32_t zeroWord = QuantizedZeros<kFp8>();
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                words[i] = zeroWord;
-            // K padding: zeros (e4m3) or the constant inputs of the bias slots (int8)
-            const uint32_t slotFill = kFp8 ? 0u : kBiasSlotValue * 0x01010101u;
-            words[12] = words[13] = words[14] = slotFill;
-            words[15] = kFp8 ? 0u : ((slotFill & 0x00FFFFFFu) | 0x01000000u);
-            SampleGridsDirect<kFp8, false>(params.latents, kLayers ? kLayers : params.numLayers, mip, x, y, words, kInterleaved);
-            // src/RegressionKernels.h:59-85
-            float xf = __fmul_rn(float(x), mip.positionScale);
-            float yf = __fmul_rn(float(y), mip.positionScale);
-#pragma unroll
-            for (int wave = 0; wave < 3; ++wave)
-            {
-                const float ex = __fmaf_rn(Frac(xf), 2.f, -1.f), ey = __fmaf_rn(Frac(yf), 2.f, -1.f);
-                const float ez = __fmaf_rn(Frac(__fadd_rn(xf, 0.25f)), 2.f, -1.f);
-                const float ew = __fmaf_rn(Frac(__fadd_rn(yf, 0.25f)), 2.f, -1.f);
-                words[8 + wave] = QuantizeInputs<kFp8>(__floats2half2_rn(ex, ey), __floats2half2_rn(ez, ew));
-                xf = __fmul_rn(xf, 2.f);
-                yf = __fmul_rn(yf, 2.f);
-            }
-            words[11] = QuantizeLod<kFp8>(mip.positionLod);
-#pragma unroll
-            for (int chunk = 0; chunk < 4; ++chunk)
-                ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);
-        }
-
-        aborted = RunLayer<kFp8, 0, kConvertNone>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 1, kConvertNone>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 2, kConvertNone>(params, shared, ctx, phase, failed);
-        if (!aborted) aborted = RunLayer<kFp8, 3, kConvertNone>(params, shared, ctx, phase, failed);
-        if (aborted)
-            break;
-    }
-
-    TcgenFenceBeforeSync();
-    aborted = __syncthreads_or(failed);
-    if (aborted && tid == 0)
-        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1);
-    __syncthreads();
-    if (warp == 0)
-        TmemFree(tmemBase, kTmemColumns);
-}
-
-
-
-// Lets `kernel` use sizeof(SharedStorage) bytes of dynamic shared memory on the current device
-// (needed once per device and kernel; remembered per device).
-template <typename Kernel>
-cudaError_t AllowSharedStorage(Kernel kernel, std::atomic<unsigned long long>& doneMask)
-{
-    int device = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess)
-        return err;
-    const unsigned long long bit = 1ull << (device & 63);
-    if (doneMask.load(std::memory_order_acquire) & bit)
-        return cudaSuccess;
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SharedStorage)));
-    if (err == cudaSuccess)
-        doneMask.fetch_or(bit, std::memory_order_release);
-    return err;
-}
-
-template <typename Kernel, typename Params>
-cudaError_t LaunchWithSharedStorage(Kernel kernel, std::atomic<unsigned long long>& doneMask, const Params& params, int ctas,
-    cudaStream_t stream, size_t bytes = sizeof(SharedStorage))
-{
-    cudaError_t err = AllowSharedStorage(kernel, doneMask);
-    if (err != cudaSuccess)
-        return err;
-    return LaunchOverlapped(kernel, ctas, kThreadsPerCta, bytes, stream, params);
+    SampleTiles<ExactChain<kFp8>, kFp8, false, kInterleaved, kLayers>(params);
 }
 
 // The layer counts of the presets are compiled in: the loops over layers of staging and gathering unroll, and strides and
-// lane masks become constants (1920 x 1080 with full mips, Int8, 2 layers: 188 -> 176 us; 2048 x 2048, FP8, 3 layers: 302 -> 279).
+// lane masks become constants (1920 x 1080 with full mips, Int8, 2 layers, as measured when it came: 188 -> 176 us; 2048 x 2048, FP8, 3 layers:
+// 302 -> 279).
 template <bool kFp8, int kConvert>
 cudaError_t LaunchDecodeLayers(const KernelParams& params, int ctas, cudaStream_t stream)
 {
-    static std::atomic<unsigned long long> done[4];
+    static std::atomic<unsigned long long> done[5];
+    auto launch = [&](auto layers) {
+        constexpr int kLayers = decltype(layers)::value;
+        const int chains = ChainsPerCta(uint32_t(params.totalTiles), ctas);
+        return LaunchChains(DecodeKernel<kFp8, kConvert, kLayers>, done[kLayers], SharedBytes<ExactStorage>(chains, sizeof(CodesStage)),
+            SharedBytes<ExactStorage>(kMaxChains, sizeof(CodesStage)), chains, params, ctas, stream);
+    };
     switch (params.numLayers)
     {
-    case 2: return LaunchWithSharedStorage(DecodeKernel<kFp8, kConvert, 2>, done[1], params, ctas, stream);
-    case 3: return LaunchWithSharedStorage(DecodeKernel<kFp8, kConvert, 3>, done[2], params, ctas, stream);
-    case 4: return LaunchWithSharedStorage(DecodeKernel<kFp8, kConvert, 4>, done[3], params, ctas, stream);
-    default: return LaunchWithSharedStorage(DecodeKernel<kFp8, kConvert, 0>, done[0], params, ctas, stream);
+    case 2: return launch(std::integral_constant<int, 2>());
+    case 3: return launch(std::integral_constant<int, 3>());
+    case 4: return launch(std::integral_constant<int, 4>());
+    default: return launch(std::integral_constant<int, 0>());
     }
 }
 
 template <bool kFp8, bool kInterleaved>
 cudaError_t LaunchSampleLayers(const SampleParams& params, int ctas, cudaStream_t stream)
 {
-    static std::atomic<unsigned long long> done[4];
-    const size_t bytes = offsetof(SharedStorage, stage); // the tables and footprints are not used
+    static std::atomic<unsigned long long> done[5];
+    auto launch = [&](auto layers) {
+        constexpr int kLayers = decltype(layers)::value;
+        const int chains = ChainsPerCta((params.numQueries + 127) / 128, ctas);
+        // the tables and footprints are not used
+        return LaunchChains(SampleKernel<kFp8, kInterleaved, kLayers>, done[kLayers], SharedBytes<ExactStorage>(chains, 0),
+            SharedBytes<ExactStorage>(kMaxChains, 0), chains, params, ctas, stream);
+    };
     if constexpr (kInterleaved) // as in the reference-numerics kernels: the presets' layer counts
     {
         switch (params.numLayers)
         {
-        case 2: return LaunchWithSharedStorage(SampleKernel<kFp8, true, 2>, done[1], params, ctas, stream, bytes);
-        case 3: return LaunchWithSharedStorage(SampleKernel<kFp8, true, 3>, done[2], params, ctas, stream, bytes);
-        case 4: return LaunchWithSharedStorage(SampleKernel<kFp8, true, 4>, done[3], params, ctas, stream, bytes);
+        case 2: return launch(std::integral_constant<int, 2>());
+        case 3: return launch(std::integral_constant<int, 3>());
+        case 4: return launch(std::integral_constant<int, 4>());
         }
     }
-    return LaunchWithSharedStorage(SampleKernel<kFp8, kInterleaved, 0>, done[0], params, ctas, stream, bytes);
+    return launch(std::integral_constant<int, 0>());
 }
 
 } // namespace

@@ -12,19 +12,10 @@ struct NtcbOutputConversion; // include/ntcb.h
 namespace ntcb
 {
 
-constexpr int kTileWidth = 32;
-constexpr int kTileHeight = 8;      // a tile is two 32x4 halves, each a 128-row GEMM chain
-constexpr int kThreadsPerCta = kTileWidth * kTileHeight; // one thread per texel of a tile
-constexpr int kOperandBytes = 128 * 64; // A operand of one half: 128 rows x 64 bytes
-constexpr int kCtasPerSmInt8 = 4;  // resident CTAs per SM the two kernel variants are compiled for
-constexpr int kCtasPerSmFp8 = 4;
-constexpr int kCtasPerSmConverting = 4; // ... and the variants with a converting epilogue (either weight mode)
-constexpr int kTmemColumnsPerHalf = 64;    // widest accumulator (layer 0: 64 outputs)
-constexpr int kTmemColumns = 2 * kTmemColumnsPerHalf;
+constexpr int kOperandBytes = 128 * 64; // A operand of codes: 128 rows x 64 bytes
+constexpr int kTmemColumnsPerChain = 64;    // widest accumulator (layer 0: 64 outputs)
 constexpr uint32_t kSpinLimit = 1u << 20;  // mbarrier polls before a wait is declared expired (about two seconds)
 constexpr uint32_t kWaitHintNanoseconds = 2000; // how long one poll may suspend the thread
-constexpr int kFootprintHiBytes = 11264;   // shared memory for a tile's unpacked footprint in the high-res grid
-constexpr int kFootprintLoBytes = 4096;    // ... and in the low-res grid (half the resolution)
 
 // Image of the network in shared memory (produced on the host by ntcb_stage_network).
 // Weight matrix of layer l: N_l rows (outputs) x K_l bytes (inputs, padded to a multiple of 32) in
@@ -81,7 +72,7 @@ constexpr int kRefInt8NetworkBytes = 17408; // ... what the Int8 kernels copy to
 // has 48 inputs; of layer 1's 64 the first 32 are here, the other 32 in tensor memory, like all of
 // layers 2 and 3.
 constexpr int kRefOperandBytes = 128 * 96;
-// Reference-numerics kernels: a CTA is up to eight chains of 128 threads - 64 tensor-memory columns and 64 registers a thread each, which
+// A CTA is up to eight chains of 128 threads - 64 tensor-memory columns and 64 registers a thread each, which
 // fills an SM - that share the network in shared memory and nothing else.  Each walks tiles of its own, 16 x 8 texels, in runs of
 // up to four side by side, with its own tables and footprints, and meets only its own threads in barriers.
 constexpr int kChainTileWidth = 16;
@@ -114,8 +105,7 @@ struct KernelMip
     unsigned long long outOffset;
     float invWidth, invHeight;
     float positionScale, positionLod;
-    // Where the mip stands in the launch's list of work, and how much of it a row of tiles has: counted in tiles (exact accumulation)
-    // or in runs of tiles (reference numerics).
+    // Where the mip stands in the launch's list of work, and how much of it a row of tiles has: counted in runs of tiles.
     int firstTile, tilesX;
     unsigned tilesXMagic; // ceil(2^32 / tilesX): local / tilesX == umulhi(local, magic) for every tile of the mip; 0: divide
     int runTiles;         // tiles side by side whose tables and footprints are prepared together (1, 2 or 4)

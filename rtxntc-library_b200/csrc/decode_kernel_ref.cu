@@ -52,6 +52,7 @@
 #include "decode_kernel.h"
 #include "kernel_parts.cuh"
 #include "input_stage.cuh"
+#include "chain_walk.cuh"
 #include "output_convert.cuh"
 #include "epilogue_convert.cuh"
 
@@ -160,73 +161,10 @@ struct __align__(16) RefTileTables
     uint32_t pad[2];
 };
 
-// What a chain prepares per run of tiles.
-template <typename Tables, int kHiBytes, int kLoBytes>
-struct __align__(16) ChainStage
-{
-    Tables tables;
-    uint8_t footprintHi[kHiBytes];
-    uint8_t footprintLo[kLoBytes];
-};
-
-// What the threads of a chain keep of their texel's place in a tile while the tables stay the same: with power-of-two sizes that is from the
-// first inner run of a mip on, and the tiles of a run differ by whole latent pixels (`shift` in DecodeRuns).  The positional encoding stays in the operand row, whose last chunks only the input stage writes.  (Worked out per
-// tile - eight products and eight conversions - a 4096 x 4096 FP8 set took 867 us instead of 851.)
-struct __align__(16) TexelTables
-{
-    uint4 weights[2][128]; // per grid and texel: w00, w01, w10, w11, each twice
-    uint4 taps[128];       // byte offset of the upper left tap and bytes per footprint row, high-res and low-res grid
-};
-
 struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes>
 {
     TexelTables texels;
 };
-
-template <typename Stage>
-__device__ __forceinline__ void PrepareTexel(Stage& stage, int texel, int column, int tileRow)
-{
-    uint32_t offsets[4];
-#pragma unroll
-    for (int grid = 0; grid < 2; ++grid)
-    {
-        const int2 col = stage.tables.taps.colTap[grid][column];
-        const int4 row = stage.tables.taps.rowTap[grid][tileRow];
-        const float dx = __int_as_float(col.y), dxn = __fsub_rn(1.f, dx);
-        const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
-        // src/FeatureGridDevice.h:46-49
-        const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);
-        stage.texels.weights[grid][texel] = make_uint4(AsU32(__floats2half2_rn(f00, f00)), AsU32(__floats2half2_rn(f01, f01)),
-                                                       AsU32(__floats2half2_rn(f10, f10)), AsU32(__floats2half2_rn(f11, f11)));
-        offsets[2 * grid] = uint32_t(col.x + row.x);
-        offsets[2 * grid + 1] = uint32_t(row.w);
-    }
-    stage.texels.taps[texel] = make_uint4(offsets[0], offsets[1], offsets[2], offsets[3]);
-}
-
-// Calls blend(grid, layer, four taps, four weights) for the latents of a texel in the staged footprints.  `shift`: bytes the taps of a
-// grid lie past those in TexelTables.
-template <int kLayers, typename Stage, typename Blend>
-__device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, int2 shift, Blend blend)
-{
-    const uint4 taps = stage.texels.taps[texel];
-    const int stride = StrideBytes<kLayers>(mip);
-#pragma unroll
-    for (int grid = 0; grid < 2; ++grid)
-    {
-        const uint4 w = stage.texels.weights[grid][texel];
-        const uint8_t* tap00 = grid ? stage.footprintLo + (taps.z + shift.y) : stage.footprintHi + (taps.x + shift.x);
-        const uint8_t* tap10 = tap00 + (grid ? taps.w : taps.y);
-#pragma unroll
-        for (int layer = 0; layer < 4; ++layer)
-        {
-            if (layer < NumLayers<kLayers>(params))
-                blend(grid, layer, *reinterpret_cast<const uint2*>(tap00 + layer * 8), *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8),
-                    *reinterpret_cast<const uint2*>(tap10 + layer * 8), *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8),
-                    AsHalf2(w.x), AsHalf2(w.y), AsHalf2(w.z), AsHalf2(w.w));
-        }
-    }
-}
 
 struct __align__(128) RefSharedStorage
 {
@@ -246,61 +184,6 @@ struct __align__(128) RefSharedStorage
     alignas(128) uint8_t operandA[kMaxChains * kRefOperandBytes];
 };
 static_assert(sizeof(RefSharedStorage) + kMaxChains * sizeof(RefStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
-
-// Dynamic shared memory of a CTA of `chains` chains, each with an operand and `perChain` more bytes.
-template <typename Storage>
-constexpr size_t SharedBytes(int chains, size_t perChain)
-{
-    return offsetof(Storage, operandA) + chains * (sizeof(Storage::operandA) / kMaxChains + perChain);
-}
-
-// What `chain` prepares per tile: after the operands of all chains.
-template <typename Stage, typename Storage>
-__device__ __forceinline__ Stage& StageOf(Storage& shared, int chain)
-{
-    return reinterpret_cast<Stage*>(shared.operandA + (blockDim.x >> 7) * (sizeof(Storage::operandA) / kMaxChains))[chain];
-}
-
-// Inference on sample: tiles of 128 queries are claimed, not dealt.  The chains of a CTA draw from a counter in shared memory, two tiles
-// ahead, as the queries are requested one tile ahead; tile k of CTA b is tile b + k * gridDim.x.  The threads of a chain read the claim between
-// the barriers of layers 0 and 1.  (16.7 M queries: 780 us dealt, 768 claimed; the tiles of a decode, whose costs differ less, are dealt: claimed
-// they take 2 % longer.)
-template <typename Storage>
-__device__ __forceinline__ void ClaimTile(Storage& shared, int chain)
-{
-    if ((threadIdx.x & 127) == 0)
-        shared.claimed[chain] = atomicAdd(&shared.claims, 1u);
-}
-
-// What a warp of a chain does besides its texels: roles 0 and 1 stage the footprints of the high-res and the low-res grid (2 and 3 the rest of large
-// ones), role 3 hands the products to the tensor core.  All four meet before every layer, so the busiest sets the pace.
-// Warp w of every chain runs on sub-partition w % 4 of the SM, so the roles go round from chain to chain.
-// (Warp 0 staging and issuing in every chain: 4096 x 4096 FP8 832 us, 8192 x 8192 Int8 4530, 16.7 M queries 725.  Issued by warp 3 instead: 775,
-// 4210, 723.  Rotated: 780, 4190, 692, and 8-bit pixels 962 instead of 985.)
-constexpr int kIssuingRole = 3;
-__device__ __forceinline__ int WarpRole(int warpIndex)
-{
-    return (warpIndex + (warpIndex >> 2)) & 3;
-}
-
-struct RefTileContext
-{
-    int tid;
-    // The same in all lanes of a warp (Uniform): the thread's warp, and its chain's first tensor-memory column at lane 0.  What follows from
-    // them - roles, barriers, the place of a tile and its mip's constants - lives in uniform registers.  (Taken from the thread's
-    // index, all of that took vector registers, and branches on it reconverged: 8192 x 8192 Int8 3803 -> 3640 us, 4096 x 4096 FP8 664 -> 649,
-    // its 8-bit pixels 874 -> 828, 16.7 M queries 658 -> 641.)
-    int warp;
-    uint32_t accumulators;
-    uint32_t tmemLane;    // the chain's first tensor-memory column at this thread's lane (its warp's first lane, to be precise)
-    uint32_t barrier;     // shared address of the chain's MMA-completion mbarrier
-    uint32_t giveUp;      // shared address of the chain's give-up word for the current tile (LayerBarrier)
-    uint4* rowChunk; // this thread's 16-byte slot in chunk 0 of its chain's A operand
-    int tile, x, y;
-    uint32_t* out;
-    uint32_t outStepWords;
-    int storeBytes; // widest store the texel may go out with (KernelMip::storeBytes)
-};
 
 // ---------------------------------------------------------------------------------------------
 // Inputs
@@ -390,7 +273,7 @@ __device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plan
 // and the row's last two chunks are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
 template <int kLayers = 0>
 __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
-    const RefTileContext& ctx, int column, int tileRow, bool known, int2 shift)
+    const ChainContext& ctx, int column, int tileRow, bool known, int2 shift)
 {
     uint32_t words[16];
     const uint32_t zeroPair = stage.tables.zeroPair;
@@ -475,7 +358,7 @@ __device__ __forceinline__ void UmmaF16FromTmem(uint32_t tmemD, uint32_t tmemA, 
 // First half of a layer for the chain's current tile: the chain's barrier (LayerBarrier), and MMA issue by the warp of
 // kIssuingRole.  Returns nonzero (uniformly over the chain) when some thread gave up on a wait.
 template <int kLayer>
-__device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
+__device__ __forceinline__ int IssueLayerRef(ChainContext& ctx)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
     constexpr int kK = kLayer == 0 ? 48 : kLayer == 1 ? 64 : kLayer == 2 ? 48 : 32;
@@ -535,7 +418,7 @@ __device__ __forceinline__ int IssueLayerRef(RefTileContext& ctx)
 // Second half of a layer: waits for the MMA, then applies the activation and writes the next
 // layer's A operand (layers 0-2) or stores the texel (layer 3).
 template <int kLayer, int kConvert, typename Params>
-__device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefTileContext& ctx, uint32_t& phase)
+__device__ __forceinline__ void ConsumeLayerRef(const Params& params, const ChainContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
 
@@ -603,7 +486,7 @@ __device__ __forceinline__ void ConsumeLayerRef(const Params& params, const RefT
 }
 
 template <int kLayer, int kConvert, typename Params>
-__device__ __forceinline__ int RunLayerRef(const Params& params, RefTileContext& ctx, uint32_t& phase)
+__device__ __forceinline__ int RunLayerRef(const Params& params, ChainContext& ctx, uint32_t& phase)
 {
     if (IssueLayerRef<kLayer>(ctx))
         return 1;
@@ -641,7 +524,7 @@ __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint
         FenceBarrierInit();
     }
     if (warp == 0)
-        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerHalf);
+        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerChain);
     first([&]() {
         GridDependencyWait();
         if (tid == 0)
@@ -662,143 +545,9 @@ __device__ __forceinline__ void SetupCtaRef(RefSharedStorage& shared, const uint
     }
 }
 
-// End of a CTA: agrees on whether anything went wrong, gives work in flight one more bounded chance
-// to drain, and releases the tensor memory.
-__device__ __forceinline__ void TeardownCtaRef(RefSharedStorage& shared, const RefTileContext& ctx, uint32_t phase,
-    int tid, int warp)
-{
-    TcgenFenceBeforeSync();
-    __syncthreads();
-    const volatile uint32_t* gaveUp = &shared.giveUp[warp >> 2][0];
-    if ((tid & 127) == 0 && (gaveUp[0] | gaveUp[1]))
-    {
-        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1);
-        (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
-    }
-    __syncthreads();
-    if (warp == 0)
-        TmemFree(shared.tmemBase, (blockDim.x >> 7) * kTmemColumnsPerHalf);
-}
-
 // ---------------------------------------------------------------------------------------------
 // The kernels
 // ---------------------------------------------------------------------------------------------
-
-// A chain's share of a launch.  `Chain` says how its tiles are prepared, fed and consumed.
-//
-// The unit of work is a run of up to kMaxRunTiles tiles side by side (KernelMip::runTiles).  Tables and footprints are made once per run, by all
-// four warps, under the products of the run before: the footprints of neighbouring tiles overlap (with a grid at a quarter of the mip's resolution
-// four tiles have 72 + 30 latent pixels, one has 24 + 12), the latents' way from the L2 is waited for once, and finding the place of the
-// work is paid for once.
-template <typename Chain, int kConvert, int kLayers>
-__device__ __forceinline__ void DecodeRuns(const KernelParams& params)
-{
-    extern __shared__ __align__(128) unsigned char dynamicShared[];
-    using Storage = typename Chain::Storage;
-    using Stage = typename Chain::Stage;
-    Storage& shared = *reinterpret_cast<Storage*>(dynamicShared);
-
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = int(Uniform(uint32_t(tid) >> 5));
-    const int chain = warp >> 2, role = WarpRole(warp);
-    const int tileColumn = tid & (kChainTileWidth - 1), tileRow = (tid & 127) / kChainTileWidth; // this thread's texel of a tile
-
-    Stage& stage = StageOf<Stage>(shared, chain);
-    // the first chains of all CTAs take the first runs, so that a launch of few spreads over the SMs
-    uint32_t run = blockIdx.x + uint32_t(chain) * gridDim.x;
-    // (What can be worked out from these is, tile by tile: the registers are worth more than the instructions.)
-    int mipIndex = 0, x0 = 0, y0 = 0; // the next tile's mip and place
-    bool known = false;               // the tables, and what the threads keep of them, are already the next tile's
-    int tablesMip = -1;               // mip whose tables are in shared memory and valid for every inner run of it
-    auto prepareRun = [&](auto between) {
-        while (mipIndex + 1 < params.numMips && run >= uint32_t(params.mips[mipIndex + 1].firstTile))
-            ++mipIndex; // runs are visited in increasing order, so the search resumes at the current mip
-        const KernelMip& mip = params.mips[mipIndex];
-        const int local = int(run) - mip.firstTile;
-        const int row = mip.tilesXMagic ? int(__umulhi(uint32_t(local), mip.tilesXMagic)) : local / mip.tilesX;
-        const int columns = mip.runTiles * kChainTileWidth;
-        x0 = (local - row * mip.tilesX) * columns;
-        y0 = mip.rowBegin + row * kChainTileHeight;
-        const bool keeps = TileKeepsTables<ChainTile>(mip, x0, y0, columns);
-        // the tables of the previous run serve this one too when both lie inside the same mip with invariant tables
-        known = keeps && mipIndex == tablesMip;
-        Chain::template Prepare<kLayers>(params, mip, stage, x0, y0, columns, lane, role, known, between);
-        tablesMip = keeps ? mipIndex : -1;
-    };
-    Chain::Setup(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [&](auto dependency) {
-        if (run < uint32_t(params.totalTiles))
-            prepareRun(dependency);
-        else
-            dependency();
-    });
-    uint32_t phase = 0;
-
-    RefTileContext ctx;
-    ctx.tid = tid;
-    ctx.warp = warp;
-    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerHalf;
-    // a warp may only touch the TMEM lanes 32 * (warp % 4) .. + 31
-    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier[chain]);
-    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * (sizeof(Storage::operandA) / kMaxChains)) + (tid & 127);
-
-    while (run < uint32_t(params.totalTiles))
-    {
-        const KernelMip& mip = params.mips[mipIndex];
-        ctx.tile = int(run);
-        ctx.x = x0 + tileColumn;
-        ctx.y = y0 + tileRow;
-        // runs start at multiples of their width
-        const int column = x0 & (mip.runTiles * kChainTileWidth - 1);
-        const int steps = known ? column / kChainTileWidth * StrideBytes<kLayers>(mip) : 0;
-        Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known,
-            make_int2(steps * mip.hiStepX, steps * mip.loStepX));
-
-        // layer 0; while the tensor core works on it, prepare the chain's NEXT run (its tables and
-        // footprints replace this run's, which nobody reads after the barrier inside Issue)
-        if (Chain::template Issue<0>(ctx))
-            break; // some thread of the chain gave up on a wait
-        x0 += kChainTileWidth;
-        if (x0 < mip.width && (x0 & (mip.runTiles * kChainTileWidth - 1)))
-            known = tablesMip == mipIndex; // a run whose tables serve others: so does what the threads keep of its first tile
-        else if ((run += (blockDim.x >> 7) * gridDim.x) < uint32_t(params.totalTiles))
-            prepareRun([]() {});
-        Chain::template Consume<0, kConvertNone>(params, ctx, phase);
-
-        Chain::template Issue<1>(ctx);
-        Chain::template Consume<1, kConvertNone>(params, ctx, phase);
-        Chain::template Issue<2>(ctx);
-        Chain::template Consume<2, kConvertNone>(params, ctx, phase);
-        {
-            // where the texel goes (worked out only now: nothing of it has to stay in registers through the
-            // layers); the element index inside a mip fits 32 bits (checked on the host)
-            const bool planar = params.outputLayout == kLayoutPlanarPairs;
-            const uint32_t first = planar ? uint32_t(ctx.y) * uint32_t(mip.width) * uint32_t(params.channels) + 2u * uint32_t(ctx.x)
-                                          : (uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x)) * uint32_t(params.channels);
-            const bool inside = ctx.x < mip.width && ctx.y < mip.rowEnd;
-            if constexpr (kConvert != kConvertNone)
-            {
-                // pixels of dstChannels components, rows without padding; outOffset counts components
-                const uint32_t pixelIndex = uint32_t(ctx.y) * uint32_t(mip.width) + uint32_t(ctx.x);
-                const size_t component = size_t(mip.outOffset) + size_t(pixelIndex) * size_t(params.conversion.dstChannels);
-                unsigned char* bytes = reinterpret_cast<unsigned char*>(params.out) + component * BytesPerComponent(params.conversion.format);
-                ctx.out = inside ? reinterpret_cast<uint32_t*>(bytes) : nullptr;
-                ctx.outStepWords = pixelIndex;
-            }
-            else
-            {
-                ctx.out = inside ? reinterpret_cast<uint32_t*>(params.out + mip.outOffset + first) : nullptr;
-                ctx.outStepWords = planar ? uint32_t(mip.width) : 1u;
-                ctx.storeBytes = mip.storeBytes;
-            }
-        }
-        Chain::template Issue<3>(ctx);
-        Chain::template Consume<3, kConvert>(params, ctx, phase);
-    }
-    Chain::Teardown(shared, ctx, phase, tid, warp);
-}
 
 // A chain of an Int8 network: binary16 operands.
 struct Int8Chain
@@ -811,10 +560,6 @@ struct Int8Chain
     {
         SetupCtaRef(shared, network, status, polls, tid, warp, first);
     }
-    static __device__ __forceinline__ void Teardown(Storage& shared, const RefTileContext& ctx, uint32_t phase, int tid, int warp)
-    {
-        TeardownCtaRef(shared, ctx, phase, tid, warp);
-    }
     template <int kLayers, typename Between>
     static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
         int lane, int role, bool tablesValid, Between between)
@@ -822,18 +567,18 @@ struct Int8Chain
         PrepareTileRef<kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid, between);
     }
     template <int kLayers>
-    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const RefTileContext& ctx,
+    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const ChainContext& ctx,
         int column, int tileRow, bool known, int2 shift)
     {
         BuildInputsRef<kLayers>(params, mip, stage, ctx, column, tileRow, known, shift);
     }
     template <int kLayer>
-    static __device__ __forceinline__ int Issue(RefTileContext& ctx)
+    static __device__ __forceinline__ int Issue(ChainContext& ctx)
     {
         return IssueLayerRef<kLayer>(ctx);
     }
-    template <int kLayer, int kConvert>
-    static __device__ __forceinline__ void Consume(const KernelParams& params, const RefTileContext& ctx, uint32_t& phase)
+    template <int kLayer, int kConvert, typename Params>
+    static __device__ __forceinline__ void Consume(const Params& params, const ChainContext& ctx, uint32_t& phase)
     {
         ConsumeLayerRef<kLayer, kConvert>(params, ctx, phase);
     }
@@ -862,21 +607,6 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
     // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCtaRef)
     if (tid < params.numMips)
         mipTable[tid] = params.mips[tid];
-    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [](auto dependency) { dependency(); });
-    int aborted = 0;
-    uint32_t phase = 0;
-
-    RefTileContext ctx;
-    ctx.tid = tid;
-    ctx.warp = warp;
-    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerHalf;
-    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier[chain]);
-    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
-    ctx.outStepWords = 1;
-    ctx.storeBytes = params.storeBytes;
-
     const uint32_t zeroPair = AsU32(QuantizeInputRef(__float2half2_rn(0.f)));
     const unsigned long long tiles = (params.numQueries + 127) / 128;
     const int row = tid & 127;
@@ -892,7 +622,25 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
         }
     };
     unsigned long long tile = blockIdx.x + (unsigned long long)chain * gridDim.x, nextTile = tile + (blockDim.x >> 7) * gridDim.x;
-    requestQuery(tile);
+    // (the first ones under the network's way from the L2)
+    SetupCtaRef(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [&](auto dependency) {
+        dependency();
+        requestQuery(tile);
+    });
+    int aborted = 0;
+    uint32_t phase = 0;
+
+    ChainContext ctx;
+    ctx.tid = tid;
+    ctx.warp = warp;
+    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerChain;
+    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
+    ctx.barrier = SharedAddress(&shared.barrier[chain]);
+    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
+    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kRefOperandBytes) + (tid & 127);
+    ctx.outStepWords = 1;
+    ctx.storeBytes = params.storeBytes;
+
     while (tile < tiles)
     {
         ClaimTile(shared, chain);
@@ -977,7 +725,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
         RunLayerRef<2, kConvertNone>(params, ctx, phase);
         RunLayerRef<3, kConvertNone>(params, ctx, phase);
     }
-    TeardownCtaRef(shared, ctx, phase, tid, warp);
+    TeardownCta(shared, ctx, phase, tid, warp);
 }
 
 // =============================================================================================
@@ -996,11 +744,6 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
 // activations, weights rebuilt from int8) stays on the binary16 path; its 32 inputs fit the same
 // 64-byte rows.
 
-struct __align__(16) RefFp8Stage : ChainStage<TileTables<ChainTile>, kRefFootprintHiBytes, kRefFootprintLoBytes>
-{
-    TexelTables texels;
-};
-
 struct __align__(128) RefFp8SharedStorage
 {
     uint8_t network[kRefNetworkBytes];                  // layers 0-2: split e4m3 weight copies; layer 3 and bias steps: binary16
@@ -1011,37 +754,9 @@ struct __align__(128) RefFp8SharedStorage
     uint32_t claims;              // inference on sample: query tiles handed out so far
     uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row; then the RefFp8Stages
+    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row; then the CodesStages
 };
-static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(RefFp8Stage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
-
-// The 64-byte operand row of a texel, as BuildInputsRef.
-template <int kLayers>
-__device__ __forceinline__ void BuildInputsRefFp8(const KernelParams& params, const KernelMip& mip, RefFp8Stage& stage,
-    const RefTileContext& ctx, int column, int tileRow, bool known, int2 shift)
-{
-    if (!mip.staged)
-    {
-        BuildInputs<true, true, kLayers>(params, mip, stage, ctx, column, tileRow);
-        return;
-    }
-    const int texel = ctx.tid & 127;
-    if (!known)
-    {
-        PrepareTexel(stage, texel, column, tileRow);
-        // positional encoding: interleave the column's x bytes with the row's y bytes
-        const uint2 cx = stage.tables.colEnc[column];
-        const uint2 ry = stage.tables.rowEnc[tileRow];
-        ctx.rowChunk[2 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5140), __byte_perm(cx.x, ry.x, 0x7362),
-                                           __byte_perm(cx.y, ry.y, 0x5140), stage.tables.lodWord);
-        ctx.rowChunk[3 * 128] = make_uint4(0, 0, 0, 0); // K padding
-    }
-    uint32_t words[8] = {0, 0, 0, 0, 0, 0, 0, 0}; // unused feature slots hold zeros (src/Inference.cu:49)
-    GatherTexel<kLayers>(params, mip, stage, texel, shift, [&](int grid, int layer, uint2 l00, uint2 l01, uint2 l10, uint2 l11, __half2 w00, __half2 w01,
-        __half2 w10, __half2 w11) { words[4 * grid + layer] = BlendLayer<true>(l00, l01, l10, l11, w00, w01, w10, w11); });
-    ctx.rowChunk[0] = make_uint4(words[0], words[1], words[2], words[3]);
-    ctx.rowChunk[128] = make_uint4(words[4], words[5], words[6], words[7]);
-}
+static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(CodesStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 e4m3 operands, binary16 accumulators.
 __device__ __forceinline__ void UmmaE4m3F16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
@@ -1124,7 +839,7 @@ __device__ __forceinline__ void IssueChainRefFp8(int chain, uint32_t accumulator
 // First half of a layer: hands the A operand written before this call to the tensor core.  Returns
 // nonzero (uniformly over the chain) when some thread gave up on a wait.
 template <int kLayer>
-__device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
+__device__ __forceinline__ int IssueLayerRefFp8(ChainContext& ctx)
 {
     // Makes the A operand visible to the tensor core (async proxy), orders this thread's reads of the
     // previous layer's accumulators before they are overwritten, and agrees on giving up.
@@ -1140,7 +855,7 @@ __device__ __forceinline__ int IssueLayerRefFp8(RefTileContext& ctx)
     if (LayerBarrier<kLayer>(ctx.warp >> 2, ctx.giveUp))
         return 1;
     // The whole issuing warp runs the descriptor arithmetic, on values the compiler can see are the same
-    // in every lane (RefTileContext; addresses counted from the start of dynamic shared memory), and one elected lane hands the work to
+    // in every lane (ChainContext; addresses counted from the start of dynamic shared memory), and one elected lane hands the work to
     // the tensor core: issued from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
     // (Tried: building the descriptors before the barrier - 3 % slower.)
     if (WarpRole(ctx.warp) == kIssuingRole)
@@ -1159,7 +874,7 @@ __device__ __forceinline__ uint32_t ActivateToE4m3(uint32_t first, uint32_t seco
 }
 
 template <int kLayer, int kConvert, typename Params>
-__device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const RefTileContext& ctx, uint32_t& phase)
+__device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const ChainContext& ctx, uint32_t& phase)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
 
@@ -1240,16 +955,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const R
     }
 }
 
-template <int kLayer, int kConvert, typename Params>
-__device__ __forceinline__ int RunLayerRefFp8(const Params& params, RefTileContext& ctx, uint32_t& phase)
-{
-    if (IssueLayerRefFp8<kLayer>(ctx))
-        return 1;
-    ConsumeLayerRefFp8<kLayer, kConvert>(params, ctx, phase);
-    return 0;
-}
-
-// Setup and teardown as for the binary16 kernel, on the FP8 kernel's shared-memory structure.
+// Set-up as for the binary16 kernel, on the FP8 kernel's shared-memory structure.
 template <typename First>
 __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, const uint8_t* network, uint32_t* status, uint32_t loadWaitPolls, int tid, int warp,
     First first)
@@ -1269,7 +975,7 @@ __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, cons
         FenceBarrierInit();
     }
     if (warp == 0)
-        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerHalf);
+        TmemAlloc(SharedAddress(&shared.tmemBase), (blockDim.x >> 7) * kTmemColumnsPerChain);
     first([&]() {
         GridDependencyWait();
         if (tid == 0)
@@ -1290,36 +996,16 @@ __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, cons
     }
 }
 
-__device__ __forceinline__ void TeardownCtaRefFp8(RefFp8SharedStorage& shared, const RefTileContext& ctx, uint32_t phase,
-    int tid, int warp)
-{
-    TcgenFenceBeforeSync();
-    __syncthreads();
-    const volatile uint32_t* gaveUp = &shared.giveUp[warp >> 2][0];
-    if ((tid & 127) == 0 && (gaveUp[0] | gaveUp[1]))
-    {
-        (void)MbarrierWaitBounded(ctx.barrier, phase ^ 1);
-        (void)MbarrierWaitBounded(SharedAddress(&shared.loadBarrier), 0);
-    }
-    __syncthreads();
-    if (warp == 0)
-        TmemFree(shared.tmemBase, (blockDim.x >> 7) * kTmemColumnsPerHalf);
-}
-
 // A chain of an FP8 network: 8-bit operands, the input stage of the exact-accumulation kernel's 64-byte rows of codes.
 struct Fp8Chain
 {
     using Storage = RefFp8SharedStorage;
-    using Stage = RefFp8Stage;
+    using Stage = CodesStage;
     template <typename First>
     static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp,
         First first)
     {
         SetupCtaRefFp8(shared, network, status, polls, tid, warp, first);
-    }
-    static __device__ __forceinline__ void Teardown(Storage& shared, const RefTileContext& ctx, uint32_t phase, int tid, int warp)
-    {
-        TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
     }
     template <int kLayers, typename Between>
     static __device__ __forceinline__ void Prepare(const KernelParams& params, const KernelMip& mip, Stage& stage, int x0, int y0, int columns,
@@ -1328,18 +1014,18 @@ struct Fp8Chain
         PrepareTile<ChainTile, true, true, kLayers>(params, mip, stage, x0, y0, columns, lane, role, tablesValid, between);
     }
     template <int kLayers>
-    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const RefTileContext& ctx,
+    static __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, Stage& stage, const ChainContext& ctx,
         int column, int tileRow, bool known, int2 shift)
     {
-        BuildInputsRefFp8<kLayers>(params, mip, stage, ctx, column, tileRow, known, shift);
+        BuildCodes<true, true, kLayers>(params, mip, stage, ctx, column, tileRow, known, shift);
     }
     template <int kLayer>
-    static __device__ __forceinline__ int Issue(RefTileContext& ctx)
+    static __device__ __forceinline__ int Issue(ChainContext& ctx)
     {
         return IssueLayerRefFp8<kLayer>(ctx);
     }
-    template <int kLayer, int kConvert>
-    static __device__ __forceinline__ void Consume(const KernelParams& params, const RefTileContext& ctx, uint32_t& phase)
+    template <int kLayer, int kConvert, typename Params>
+    static __device__ __forceinline__ void Consume(const Params& params, const ChainContext& ctx, uint32_t& phase)
     {
         ConsumeLayerRefFp8<kLayer, kConvert>(params, ctx, phase);
     }
@@ -1351,139 +1037,13 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) DecodeKernelRefFp8(const
     DecodeRuns<Fp8Chain, kConvert, kLayers>(params);
 }
 
-// Inference on sample for FP8 networks (8-bit operands): one thread per query, taps read straight
-// from global memory.
 template <bool kInterleaved, int kLayers>
 __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const __grid_constant__ SampleParams params)
 {
-    extern __shared__ __align__(128) unsigned char dynamicShared[];
-    RefFp8SharedStorage& shared = *reinterpret_cast<RefFp8SharedStorage*>(dynamicShared);
-    __shared__ KernelMip mipTable[16];
-
-    const int tid = threadIdx.x;
-    const int warp = int(Uniform(uint32_t(tid) >> 5));
-    const int chain = warp >> 2;
-
-    if (tid < params.numMips)
-        mipTable[tid] = params.mips[tid];
-    SetupCtaRefFp8(shared, params.network, params.status, params.loadWaitPolls, tid, warp, [](auto dependency) { dependency(); });
-    int aborted = 0;
-    uint32_t phase = 0;
-
-    RefTileContext ctx;
-    ctx.tid = tid;
-    ctx.warp = warp;
-    ctx.accumulators = Uniform(shared.tmemBase) + chain * kTmemColumnsPerHalf;
-    ctx.tmemLane = ctx.accumulators + (uint32_t((warp & 3) * 32) << 16);
-    ctx.barrier = SharedAddress(&shared.barrier[chain]);
-    ctx.giveUp = SharedAddress(&shared.giveUp[chain][0]);
-    ctx.rowChunk = reinterpret_cast<uint4*>(shared.operandA + chain * kOperandBytes) + (tid & 127);
-    ctx.outStepWords = 1;
-    ctx.storeBytes = params.storeBytes;
-
-    const unsigned long long tiles = (params.numQueries + 127) / 128;
-    const int row = tid & 127;
-    // a tile's queries are requested one tile ahead: their latency passes under the previous tile's layers
-    float nextU = 0.f, nextV = 0.f, nextLod = 0.f;
-    auto requestQuery = [&](unsigned long long ofTile) {
-        if (ofTile < tiles)
-        {
-            const unsigned long long q = min(ofTile * 128 + row, params.numQueries - 1);
-            nextU = __ldg(params.queries + 3 * q);
-            nextV = __ldg(params.queries + 3 * q + 1);
-            nextLod = __ldg(params.queries + 3 * q + 2);
-        }
-    };
-    unsigned long long tile = blockIdx.x + (unsigned long long)chain * gridDim.x, nextTile = tile + (blockDim.x >> 7) * gridDim.x;
-    requestQuery(tile);
-    while (tile < tiles)
-    {
-        ClaimTile(shared, chain);
-        const unsigned long long query = tile * 128 + row;
-        const bool valid = query < params.numQueries;
-        const float u = nextU, v = nextV, lod = nextLod;
-        requestQuery(nextTile);
-        const int mipIndex = max(0, min(params.numMips - 1, int(floorf(lod))));
-        const KernelMip& mip = mipTable[mipIndex];
-        const int x = max(0, min(mip.width - 1, int(floorf(__fmul_rn(u, float(mip.width))))));
-        const int y = max(0, min(mip.height - 1, int(floorf(__fmul_rn(v, float(mip.height))))));
-        ctx.tile = int(tile);
-        ctx.x = x;
-        ctx.y = y;
-        ctx.out = valid ? reinterpret_cast<uint32_t*>(params.out + query * params.channels) : nullptr;
-
-        {
-            uint32_t words[16];
-            const uint32_t zeroWord = QuantizedZeros<true>();
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                words[i] = zeroWord; // unused feature slots hold quantised zeros (src/Inference.cu:49)
-#pragma unroll
-            for (int i = 12; i < 16; ++i)
-                words[i] = 0;        // K padding
-            SampleGridsDirect<true, true>(params.latents, kLayers ? kLayers : params.numLayers, mip, x, y, words, kInterleaved);
-            // src/RegressionKernels.h:59-85
-            float xf = __fmul_rn(float(x), mip.positionScale);
-            float yf = __fmul_rn(float(y), mip.positionScale);
-#pragma unroll
-            for (int wave = 0; wave < 3; ++wave)
-            {
-                const float ex = __fmaf_rn(Frac(xf), 2.f, -1.f), ey = __fmaf_rn(Frac(yf), 2.f, -1.f);
-                const float ez = __fmaf_rn(Frac(__fadd_rn(xf, 0.25f)), 2.f, -1.f);
-                const float ew = __fmaf_rn(Frac(__fadd_rn(yf, 0.25f)), 2.f, -1.f);
-                words[8 + wave] = QuantizeInputs<true>(__floats2half2_rn(ex, ey), __floats2half2_rn(ez, ew));
-                xf = __fmul_rn(xf, 2.f);
-                yf = __fmul_rn(yf, 2.f);
-            }
-            words[11] = QuantizeLod<true>(mip.positionLod);
-#pragma unroll
-            for (int chunk = 0; chunk < 4; ++chunk)
-                ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);
-        }
-
-        // nothing is shared between the chains of a query tile: each runs at its own pace
-        aborted = RunLayerRefFp8<0, kConvertNone>(params, ctx, phase);
-        if (aborted)
-            break;
-        tile = nextTile;
-        nextTile = blockIdx.x + (unsigned long long)shared.claimed[chain] * gridDim.x;
-        RunLayerRefFp8<1, kConvertNone>(params, ctx, phase);
-        RunLayerRefFp8<2, kConvertNone>(params, ctx, phase);
-        RunLayerRefFp8<3, kConvertNone>(params, ctx, phase);
-    }
-    TeardownCtaRefFp8(shared, ctx, phase, tid, warp);
+    SampleTiles<Fp8Chain, true, true, kInterleaved, kLayers>(params);
 }
 
 } // namespace
-
-// One kernel, set up for its dynamic shared memory on first use per device (`done`: one bit per device).
-template <typename Kernel, typename Params>
-cudaError_t LaunchRefKernel(Kernel kernel, std::atomic<unsigned long long>& done, size_t sharedBytes, size_t maxSharedBytes, int chains,
-    const Params& params, int ctas, cudaStream_t stream)
-{
-    int device = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess)
-        return err;
-    const unsigned long long bit = 1ull << (device & 63);
-    if (!(done.load(std::memory_order_acquire) & bit))
-    {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(maxSharedBytes));
-        if (err != cudaSuccess)
-            return err;
-        done.fetch_or(bit, std::memory_order_release);
-    }
-    return LaunchOverlapped(kernel, ctas, 128 * chains, sharedBytes, stream, params);
-}
-
-// Chains of a CTA: no more than tiles, a power of two as the tensor-memory allocation has to be.
-int ChainsPerCta(unsigned long long tiles, int ctas)
-{
-    int chains = 1;
-    while (chains < kMaxChains && (unsigned long long)chains * (unsigned long long)ctas < tiles)
-        chains *= 2;
-    return chains;
-}
 
 // The kernel of a weight set and epilogue compiled for 2, 3 or 4 latent layers, or the one for any number.
 template <bool kFp8Weights, int kConvert>
@@ -1494,10 +1054,10 @@ cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStre
         constexpr int kLayers = decltype(layers)::value;
         const int chains = ChainsPerCta(uint32_t(params.totalTiles), ctas);
         if constexpr (kFp8Weights) // 8-bit operands
-            return LaunchRefKernel(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, sizeof(RefFp8Stage)),
-                SharedBytes<RefFp8SharedStorage>(kMaxChains, sizeof(RefFp8Stage)), chains, params, ctas, stream);
+            return LaunchChains(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, sizeof(CodesStage)),
+                SharedBytes<RefFp8SharedStorage>(kMaxChains, sizeof(CodesStage)), chains, params, ctas, stream);
         else
-            return LaunchRefKernel(DecodeKernelRef<kConvert, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, sizeof(RefStage)),
+            return LaunchChains(DecodeKernelRef<kConvert, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, sizeof(RefStage)),
                 SharedBytes<RefSharedStorage>(kMaxChains, sizeof(RefStage)), chains, params, ctas, stream);
     };
     switch (params.numLayers)
@@ -1531,10 +1091,10 @@ cudaError_t LaunchSampleRefLayers(const SampleParams& params, int ctas, cudaStre
         const int chains = ChainsPerCta((params.numQueries + 127) / 128, ctas);
         // the tables and footprints are not used
         if constexpr (kFp8Weights)
-            return LaunchRefKernel(SampleKernelRefFp8<kInterleaved, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, 0),
+            return LaunchChains(SampleKernelRefFp8<kInterleaved, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, 0),
                 SharedBytes<RefFp8SharedStorage>(kMaxChains, 0), chains, params, ctas, stream);
         else
-            return LaunchRefKernel(SampleKernelRef<kInterleaved, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, 0),
+            return LaunchChains(SampleKernelRef<kInterleaved, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, 0),
                 SharedBytes<RefSharedStorage>(kMaxChains, 0), chains, params, ctas, stream);
     };
     if constexpr (kInterleaved)

@@ -70,6 +70,14 @@ __device__ __forceinline__ uint32_t QuantizeLod(float value)
     return kFp8 ? pair : __byte_perm(pair, QuantizeInputPair<false>(__float2half2_rn(0.f)), 0x6420);
 }
 
+// The last 16 operand bytes of layer 0, past its 48 inputs: zeros (e4m3), or the constant inputs of the bias slots (int8).
+template <bool kFp8>
+__device__ __forceinline__ uint4 PaddingCodes()
+{
+    const uint32_t fill = kFp8 ? 0u : kBiasSlotValue * 0x01010101u;
+    return make_uint4(fill, fill, fill, kFp8 ? 0u : (fill & 0x00FFFFFFu) | 0x01000000u);
+}
+
 template <bool kFp8>
 __device__ __forceinline__ uint32_t QuantizedZeros()
 {
@@ -196,24 +204,15 @@ __device__ __forceinline__ void SampleInterleaved(const uint16_t* __restrict__ h
     }
 }
 
-// The unit of texels that a group of threads works on, thread = texel, the warps of the group, and the most columns whose tables and
-// footprints they prepare together: all eight warps of a CTA on a 32 x 8 tile (exact accumulation), or the four of a chain on 16 x 8 tiles
-// of its own, prepared in runs of up to four side by side (reference numerics).
-struct WideTile
-{
-    using ColumnTap = int4;
-    static constexpr int kWidth = kTileWidth, kHeight = kTileHeight, kWarps = 8, kWidthLog2 = 5, kHeightLog2 = 3, kColumns = kWidth;
-};
+// The unit of texels that the four warps of a chain work on, thread = texel, and the most columns whose tables and footprints they prepare
+// together: tiles of 16 x 8, in runs of up to four side by side.
 struct ChainTile
 {
-    using ColumnTap = int2;
     static constexpr int kWidth = kChainTileWidth, kHeight = kChainTileHeight, kWarps = 4, kWidthLog2 = 4, kHeightLog2 = 3,
                          kColumns = kWidth * kMaxRunTiles;
 };
-static_assert(WideTile::kWidth == 1 << WideTile::kWidthLog2 && WideTile::kHeight == 1 << WideTile::kHeightLog2 &&
-                  ChainTile::kWidth == 1 << ChainTile::kWidthLog2 && ChainTile::kHeight == 1 << ChainTile::kHeightLog2 &&
-                  WideTile::kColumns <= 16 * WideTile::kWarps && ChainTile::kColumns <= 16 * ChainTile::kWarps &&
-                  WideTile::kWidth * WideTile::kHeight == 32 * WideTile::kWarps && ChainTile::kWidth * ChainTile::kHeight == 32 * ChainTile::kWarps,
+static_assert(ChainTile::kWidth == 1 << ChainTile::kWidthLog2 && ChainTile::kHeight == 1 << ChainTile::kHeightLog2 &&
+                  ChainTile::kColumns <= 16 * ChainTile::kWarps && ChainTile::kWidth * ChainTile::kHeight == 32 * ChainTile::kWarps,
     "one thread per texel");
 
 // Lookup tables of the bilinear taps of a run of tiles: tap position and weights are separable in x and y, so
@@ -222,8 +221,8 @@ static_assert(WideTile::kWidth == 1 << WideTile::kWidthLog2 && WideTile::kHeight
 template <typename Tile>
 struct __align__(16) TapTables
 {
-    // per grid (0 = high-res, 1 = low-res) and column: byte offset of the left tap inside a footprint row, dx (, 1 - dx)
-    typename Tile::ColumnTap colTap[2][Tile::kColumns];
+    // per grid (0 = high-res, 1 = low-res) and column: byte offset of the left tap inside a footprint row, dx
+    int2 colTap[2][Tile::kColumns];
     // per grid and tile row: byte offset of the upper tap's footprint row, dy, 1 - dy, bytes per footprint row
     int4 rowTap[2][Tile::kHeight];
     // per grid: footprint width and height in latent pixels, pixel count, and the multiplier that divides a
@@ -288,40 +287,26 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
     else
     {
         // each warp of a grid has 32 of the columns
-        const int column = lane + (Tile::kColumns > 32 ? 32 * (warp >> 1) : 0);
+        const int column = lane + 32 * (warp >> 1);
         int xb, tap; // of a column, of a row
         float dx, dy;
         AxisTap<kReferenceDivision>(min(tileX0 + column, mip.width - 1), mip.width, mip.invWidth, gw, xb, dx);
-        if constexpr (Tile::kColumns > 32)
-        {
-            // the rows in the first lanes; the first and the last column in the two after them
-            const bool row = lane < Tile::kHeight;
-            const int texel = row ? min(tileY0 + lane, mip.rowEnd - 1) : lane == Tile::kHeight ? tileX0 : min(tileX0 + columns - 1, mip.width - 1);
-            AxisTap<kReferenceDivision>(texel, row ? mip.height : mip.width, row ? mip.invHeight : mip.invWidth, row ? gh : gw, tap, dy);
-            fx0 = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight);
-            footW = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight + 1) - fx0 + 2;
-        }
-        else
-        {
-            AxisTap<kReferenceDivision>(min(tileY0 + (lane & (Tile::kHeight - 1)), mip.rowEnd - 1), mip.height, mip.invHeight, gh, tap, dy);
-            fx0 = __shfl_sync(0xFFFFFFFFu, xb, 0);
-            footW = __shfl_sync(0xFFFFFFFFu, xb, Tile::kWidth - 1) - fx0 + 2;
-        }
+        // the rows in the first lanes; the first and the last column in the two after them
+        const bool row = lane < Tile::kHeight;
+        const int texel = row ? min(tileY0 + lane, mip.rowEnd - 1) : lane == Tile::kHeight ? tileX0 : min(tileX0 + columns - 1, mip.width - 1);
+        AxisTap<kReferenceDivision>(texel, row ? mip.height : mip.width, row ? mip.invHeight : mip.invWidth, row ? gh : gw, tap, dy);
+        fx0 = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight);
+        footW = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight + 1) - fx0 + 2;
         fy0 = __shfl_sync(0xFFFFFFFFu, tap, 0);
         const int footH = __shfl_sync(0xFFFFFFFFu, tap, Tile::kHeight - 1) - fy0 + 2;
         count = footW * footH;
         // the IEEE quotient of 2^20 / footW floors exactly
         magic = uint32_t(__float2int_rd(__fdiv_rn(1048576.f, float(footW)))) + 1;
-        if constexpr (Tile::kColumns > 32)
-        {
-            if (column < columns)
-                taps.colTap[grid][column] = make_int2((xb - fx0) * stride, __float_as_int(dx));
-        }
+        if (column < columns)
+            taps.colTap[grid][column] = make_int2((xb - fx0) * stride, __float_as_int(dx));
         if (warp < 2)
         {
-            if constexpr (Tile::kColumns <= 32)
-                taps.colTap[grid][lane] = make_int4((xb - fx0) * stride, __float_as_int(dx), __float_as_int(__fsub_rn(1.f, dx)), 0);
-            if (lane < Tile::kHeight)
+            if (row)
                 taps.rowTap[grid][lane] =
                     make_int4((tap - fy0) * footW * stride, __float_as_int(dy), __float_as_int(__fsub_rn(1.f, dy)), footW * stride);
             if (lane == 0)
@@ -448,42 +433,6 @@ __device__ __forceinline__ uint32_t BlendLayer(uint2 l00, uint2 l01, uint2 l10, 
     return QuantizeInputs<kFp8>(a, b);
 }
 
-// Inputs 0..15 or 16..31 of one texel from the staged footprint of one grid.
-template <bool kFp8, int kLayers = 0, typename Stage>
-__device__ __forceinline__ void GatherGrid(const KernelParams& params, const KernelMip& mip, const Stage& stage,
-    int grid, int tileColumn, int tileRow, uint32_t* words)
-{
-    const auto col = stage.tables.taps.colTap[grid][tileColumn];
-    const int4 row = stage.tables.taps.rowTap[grid][tileRow];
-    const float dx = __int_as_float(col.y);
-    float dxn;
-    if constexpr (sizeof(col) == sizeof(int4))
-        dxn = __int_as_float(col.z);
-    else
-        dxn = __fsub_rn(1.f, dx);
-    const float dy = __int_as_float(row.y), dyn = __int_as_float(row.z);
-    // src/FeatureGridDevice.h:46-49
-    const float f00 = __fmul_rn(dxn, dyn), f01 = __fmul_rn(dx, dyn), f10 = __fmul_rn(dxn, dy), f11 = __fmul_rn(dx, dy);
-    const __half2 w00 = __floats2half2_rn(f00, f00), w01 = __floats2half2_rn(f01, f01);
-    const __half2 w10 = __floats2half2_rn(f10, f10), w11 = __floats2half2_rn(f11, f11);
-
-    const int stride = StrideBytes<kLayers>(mip);
-    const uint8_t* tap00 = (grid ? stage.footprintLo : stage.footprintHi) + (col.x + row.x);
-    const uint8_t* tap10 = tap00 + row.w;
-#pragma unroll
-    for (int layer = 0; layer < 4; ++layer)
-    {
-        if (layer < NumLayers<kLayers>(params))
-        {
-            const uint2 l00 = *reinterpret_cast<const uint2*>(tap00 + layer * 8);
-            const uint2 l01 = *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8);
-            const uint2 l10 = *reinterpret_cast<const uint2*>(tap10 + layer * 8);
-            const uint2 l11 = *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8);
-            words[layer] = BlendLayer<kFp8>(l00, l01, l10, l11, w00, w01, w10, w11);
-        }
-    }
-}
-
 // Inputs 0..31 of one texel with the taps read straight from global memory (`interleaved`: from the pixel-major
 // copy ntcb_interleave_latents makes instead of the file's planes; the mip's offsets then refer to that copy).
 template <bool kFp8, bool kReferenceDivision>
@@ -521,46 +470,27 @@ __device__ __forceinline__ void SampleGridsDirect(const uint16_t* __restrict__ l
             words[4 + layer] = SampleLayer<kFp8>(lo + size_t(layer) * mip.loPlane, taps);
 }
 
-// The 48 network inputs of one texel -> its 64-byte row of the A operand (K-major core matrices:
-// 16-byte chunk j of row r lives at j * 2048 + r * 16).
+// The 48 network inputs of one texel of a mip whose footprints are too large to stage (strong minification) -> its 64-byte row of the A operand
+// (K-major core matrices: 16-byte chunk j of row r lives at j * 2048 + r * 16).
 template <bool kFp8, bool kReferenceDivision, int kLayers = 0, typename Stage, typename Context>
 __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, const Stage& stage,
     const Context& ctx, int tileColumn, int tileRow)
 {
-    uint32_t words[16];
-    const uint32_t zeroWord = QuantizedZeros<kFp8>();
+    uint32_t words[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-        words[i] = zeroWord; // unused feature slots hold quantised zeros (src/Inference.cu:49)
-    // K padding: zeros for e4m3 operands; for int8 operands the constant inputs of the bias slots
-    const uint32_t slotFill = kFp8 ? 0u : kBiasSlotValue * 0x01010101u;
-    words[12] = words[13] = words[14] = slotFill;
-    words[15] = kFp8 ? 0u : ((slotFill & 0x00FFFFFFu) | 0x01000000u);
-
-    if (mip.staged)
-    {
-        GatherGrid<kFp8, kLayers>(params, mip, stage, 0, tileColumn, tileRow, words);
-        GatherGrid<kFp8, kLayers>(params, mip, stage, 1, tileColumn, tileRow, words + 4);
-    }
-    else
-    {
-        // footprint too large to stage (strong minification): read the taps from global memory;
-        // threads past the right / bottom edge compute a clamped texel and store nothing
-        SampleGridsDirect<kFp8, kReferenceDivision>(params.latents, NumLayers<kLayers>(params), mip, min(ctx.x, mip.width - 1), min(ctx.y, mip.rowEnd - 1),
-            words);
-    }
-
+        words[i] = QuantizedZeros<kFp8>(); // unused feature slots hold quantised zeros (src/Inference.cu:49)
+    // the taps are read from global memory; threads past the right / bottom edge compute a clamped texel and store nothing
+    SampleGridsDirect<kFp8, kReferenceDivision>(params.latents, NumLayers<kLayers>(params), mip, min(ctx.x, mip.width - 1), min(ctx.y, mip.rowEnd - 1),
+        words);
     // positional encoding: interleave the column's x bytes with the row's y bytes
     const uint2 cx = stage.tables.colEnc[tileColumn];
     const uint2 ry = stage.tables.rowEnc[tileRow];
-    words[8] = __byte_perm(cx.x, ry.x, 0x5140);
-    words[9] = __byte_perm(cx.x, ry.x, 0x7362);
-    words[10] = __byte_perm(cx.y, ry.y, 0x5140);
-    words[11] = stage.tables.lodWord;
-
-#pragma unroll
-    for (int chunk = 0; chunk < 4; ++chunk)
-        ctx.rowChunk[chunk * 128] = make_uint4(words[4 * chunk], words[4 * chunk + 1], words[4 * chunk + 2], words[4 * chunk + 3]);
+    ctx.rowChunk[0] = make_uint4(words[0], words[1], words[2], words[3]);
+    ctx.rowChunk[128] = make_uint4(words[4], words[5], words[6], words[7]);
+    ctx.rowChunk[2 * 128] = make_uint4(__byte_perm(cx.x, ry.x, 0x5140), __byte_perm(cx.x, ry.x, 0x7362),
+                                       __byte_perm(cx.y, ry.y, 0x5140), stage.tables.lodWord);
+    ctx.rowChunk[3 * 128] = PaddingCodes<kFp8>();
 }
 
 } // namespace

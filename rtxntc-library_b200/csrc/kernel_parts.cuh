@@ -413,7 +413,7 @@ __device__ __forceinline__ void ChainBarrier(int chain)
     asm volatile("bar.sync %0, 128;" ::"r"(chain + 1) : "memory");
 }
 
-// The barrier before a layer's matrix products (reference-numerics kernels).  The operand rows, tables and footprints of a
+// The barrier before a layer's matrix products.  The operand rows, tables and footprints of a
 // chain are written by the chain's own 128 threads, and only they read its accumulators, so a chain meets in a named barrier of
 // its own and the chains of a CTA, up to eight, drift apart instead of waiting for each other.
 //

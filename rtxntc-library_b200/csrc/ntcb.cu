@@ -91,9 +91,10 @@ bool ValidMip(const NtcbMipDesc& m, bool pairedOutput)
 }
 
 // The kernel's view of one mip (everything but its place in the tile list).  `maxRunTiles`: the longest run of tiles.
-void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprintHiBytes = kFootprintHiBytes,
-    int footprintLoBytes = kFootprintLoBytes, int tileWidth = kTileWidth, int tileHeight = kTileHeight, int maxRunTiles = 1)
+void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprintHiBytes = kRefFootprintHiBytes,
+    int footprintLoBytes = kRefFootprintLoBytes, int maxRunTiles = 1)
 {
+    constexpr int tileWidth = kChainTileWidth, tileHeight = kChainTileHeight;
     km.width = m.width;
     km.height = m.height;
     km.rowBegin = m.rowBegin;
@@ -221,17 +222,16 @@ namespace
 {
 
 // Number of CTAs that fill the current device, cached per device.
-int ResidentCtas(bool fp8, bool converting, int* outCtas, bool reference = false)
+int ResidentCtas(int* outCtas)
 {
-    static std::atomic<int> cache[64][4];
-    const int variant = reference ? 3 : converting ? 2 : fp8 ? 1 : 0;
+    static std::atomic<int> cache[64];
     int device = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess)
         return CudaFailure("cudaGetDevice", err);
     if (device >= 0 && device < 64)
     {
-        int cached = cache[device][variant].load(std::memory_order_relaxed);
+        int cached = cache[device].load(std::memory_order_relaxed);
         if (cached > 0)
         {
             *outCtas = cached;
@@ -250,18 +250,11 @@ int ResidentCtas(bool fp8, bool converting, int* outCtas, bool reference = false
             device, major);
         return NTCB_ERR_CUDA;
     }
-    // The reference-numerics kernels run one CTA per SM, whose chains fill the tensor memory.  The exact kernels are compiled for
-    // kCtasPerSmInt8 / kCtasPerSmFp8 resident CTAs (__launch_bounds__), each of which holds
-    // kTmemColumns of the SM's 512 tensor-memory columns for its whole lifetime.  (The runtime's
-    // occupancy query reports one CTA per SM for kernels that allocate tensor memory, so it is not
-    // used here.)
-    static_assert(kCtasPerSmInt8 * kTmemColumns <= 512 && kCtasPerSmFp8 * kTmemColumns <= 512 &&
-                      kCtasPerSmConverting * kTmemColumns <= 512 && kMaxChains * kTmemColumnsPerHalf <= 512,
-        "resident CTAs must fit into tensor memory");
-    const int perSm = reference ? 1 : converting ? kCtasPerSmConverting : fp8 ? kCtasPerSmFp8 : kCtasPerSmInt8;
-    *outCtas = sms * perSm;
+    // One CTA per SM, whose chains fill the tensor memory.
+    static_assert(kMaxChains * kTmemColumnsPerChain <= 512, "a CTA's chains must fit into tensor memory");
+    *outCtas = sms;
     if (device >= 0 && device < 64)
-        cache[device][variant].store(*outCtas, std::memory_order_relaxed);
+        cache[device].store(*outCtas, std::memory_order_relaxed);
     return NTCB_OK;
 }
 
@@ -308,7 +301,7 @@ int ntcb_decode_resident_ctas(int weightMode, int* outCtas)
         SetError("ntcb_decode_resident_ctas: invalid arguments.");
         return NTCB_ERR_INVALID_ARGUMENT;
     }
-    return ResidentCtas(weightMode == NTCB_WEIGHTS_FP8, false, outCtas);
+    return ResidentCtas(outCtas);
 }
 
 int ntcb_stage_network(const void* blob, size_t blobBytes, int weightMode, void* staged)
@@ -633,19 +626,15 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     k.numLayers = p->numFeatures / 4;
     k.channels = p->channels;
     const bool fp8 = p->weightMode == NTCB_WEIGHTS_FP8;
-    int resident = 0, longestRun = 1;
-    if (reference)
+    long long allTiles = 0;
+    for (int i = 0; i < p->numMips; ++i)
     {
-        long long tiles = 0;
-        for (int i = 0; i < p->numMips; ++i)
-        {
-            const NtcbMipDesc& m = p->mips[i];
-            if (m.width > 0 && m.rowEnd > m.rowBegin)
-                tiles += ((long long)m.width + kChainTileWidth - 1) / kChainTileWidth *
-                         (((long long)m.rowEnd - m.rowBegin + kChainTileHeight - 1) / kChainTileHeight);
-        }
-        longestRun = LongestRun(tiles, kMaxChains * 148); // a B200's 148 SMs
+        const NtcbMipDesc& m = p->mips[i];
+        if (m.width > 0 && m.rowEnd > m.rowBegin)
+            allTiles += ((long long)m.width + kChainTileWidth - 1) / kChainTileWidth *
+                        (((long long)m.rowEnd - m.rowBegin + kChainTileHeight - 1) / kChainTileHeight);
     }
+    const int longestRun = LongestRun(allTiles, kMaxChains * 148); // a B200's 148 SMs
     long long tiles = 0;
     int used = 0;
     for (int i = 0; i < p->numMips; ++i)
@@ -693,13 +682,10 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
         if (m.rowBegin == m.rowEnd)
             continue; // nothing of this mip belongs to this launch
         KernelMip& km = k.mips[used++];
-        const int tileHeight = reference ? kChainTileHeight : kTileHeight;
-        if (reference && p->weightMode == NTCB_WEIGHTS_FP8)
-            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes, kRefFootprintLoBytes, kChainTileWidth, kChainTileHeight, longestRun);
-        else if (reference)
-            FillKernelMip(m, p->numFeatures / 4, km, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes, kChainTileWidth, kChainTileHeight, longestRun);
+        if (reference && !fp8)
+            FillKernelMip(m, p->numFeatures / 4, km, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes, longestRun);
         else
-            FillKernelMip(m, p->numFeatures / 4, km);
+            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes, kRefFootprintLoBytes, longestRun);
         km.firstTile = int(tiles);
         km.storeBytes = 4;
         if (k.convert || p->outputLayout == NTCB_LAYOUT_INTERLEAVED)
@@ -708,7 +694,7 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
             const size_t texelBytes = size_t(p->channels) * 2;
             km.storeBytes = !(address & 15) && !(texelBytes & 15) ? 16 : !(address & 7) && !(texelBytes & 7) ? 8 : 4;
         }
-        const long long mipTiles = (long long)km.tilesX * ((m.rowEnd - m.rowBegin + tileHeight - 1) / tileHeight);
+        const long long mipTiles = (long long)km.tilesX * ((m.rowEnd - m.rowBegin + kChainTileHeight - 1) / kChainTileHeight);
         tiles += mipTiles;
         if (tiles > 0x7FFFFFFF)
         {
@@ -728,7 +714,8 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     }
     k.loadWaitPolls = g_networkWaitPolls.load(std::memory_order_relaxed);
 
-    int rc = ResidentCtas(fp8, k.convert != 0, &resident, reference);
+    int resident = 0;
+    int rc = ResidentCtas(&resident);
     if (rc != NTCB_OK)
         return rc;
     const int ctas = k.totalTiles < resident ? k.totalTiles : resident;
@@ -819,11 +806,10 @@ int ntcb_sample(const NtcbSampleParams* p, void* stream)
         return NTCB_OK;
     const bool fp8 = p->weightMode == NTCB_WEIGHTS_FP8;
     int resident = 0;
-    int rc = ResidentCtas(fp8, false, &resident, reference);
+    int rc = ResidentCtas(&resident);
     if (rc != NTCB_OK)
         return rc;
-    const unsigned long long perCta = reference ? 128 : kThreadsPerCta; // (reference numerics: of a chain)
-    const unsigned long long tiles = (p->numQueries + perCta - 1) / perCta;
+    const unsigned long long tiles = (p->numQueries + 127) / 128;
     const int ctas = tiles < (unsigned long long)resident ? int(tiles) : resident;
     cudaError_t err = reference ? LaunchSampleRef(k, fp8, ctas, static_cast<cudaStream_t>(stream))
                                 : LaunchSample(k, fp8, ctas, static_cast<cudaStream_t>(stream));

@@ -260,7 +260,7 @@ def test_row_ranges_tile_rows_and_guard_bands(oracle, numerics):
 @pytest.mark.parametrize("numerics,shape", [
     (REFERENCE, (1500, 1100, 10, 0, 4, 12)), (REFERENCE, (2510, 2012, 6, 0, 3, 8)), (REFERENCE, (2048, 3001, 4, 2, 6, 16)),
     (REFERENCE, (2600, 2048, 4, 1, 2, 4)), (REFERENCE, (2048, 2048, 8, 0, 4, 12)), (REFERENCE, (4096, 2048, 4, 2, 2, 16)),
-    (REFERENCE, (40, 130000, 4, 1, 4, 8))])
+    (REFERENCE, (40, 130000, 4, 1, 4, 8)), (EXACT, (1500, 1100, 10, 0, 4, 12)), (EXACT, (2510, 2012, 6, 0, 3, 8)), (EXACT, (2048, 2048, 8, 0, 4, 16))])
 def test_runs_of_tiles_give_the_texels_of_single_tiles(numerics, shape):
     """The tables and footprints of neighbouring tiles are prepared together in large launches, and one tile at a time in small ones:
     a whole decode has the bits of one in bands of a few rows."""
