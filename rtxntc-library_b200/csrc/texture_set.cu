@@ -665,7 +665,7 @@ int TextureSet::FirstBandRows(size_t hostTexelBytes, bool streamed) const
     if (streamed)
     {
         const float latentBytes = float(m_geometry.latentPixelOffset[1]) * float(m_geometry.numLayers) * 2.f;
-        const float upload = latentBytes / 57.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 20.f; // nanoseconds
+        const float upload = latentBytes / 57.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 27.f; // nanoseconds
         share = std::max(share, upload / (upload + decode));
     }
     return std::min(height, (int(float(height) * share) + 15) & ~15);
