@@ -605,8 +605,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRef(const __
     const int chain = warp >> 2;
 
     // the mip descriptions are indexed per thread: a copy in shared memory (visible after the barrier inside SetupCtaRef)
-    if (tid < params.numMips)
-        mipTable[tid] = params.mips[tid];
+    CopyMips(params, mipTable, tid);
     const uint32_t zeroPair = AsU32(QuantizeInputRef(__float2half2_rn(0.f)));
     const unsigned long long tiles = (params.numQueries + 127) / 128;
     const int row = tid & 127;
