@@ -822,3 +822,44 @@ def test_flat_and_binary_blocks_decode_exactly_at_full_size():
     for channel in range(2):
         expected = torch.round(texels[..., channel].to(torch.float32).clamp(0, 1) * 255.0).double()
         assert torch.equal(decode(blocks[..., 8 * channel:8 * channel + 8]), expected), channel
+
+
+def _search_images(height, width):
+    """[height][width][3] texels: smooth, noisy, outside [0, 1], of tiny extents (whose squares vanish), and with infinities and NaN."""
+    rng = np.random.default_rng(5)
+    y, x = np.mgrid[0:height, 0:width]
+    smooth = np.stack([0.5 + 0.4 * np.sin(x / 9 + c) * np.cos(y / 7 - c) for c in range(3)], axis=-1)
+    noise = rng.random((height, width, 3))
+    special = noise.copy()
+    special[rng.random(special.shape) < 0.02] = np.inf
+    special[rng.random(special.shape) < 0.02] = -np.inf
+    special[rng.random(special.shape) < 0.02] = np.nan
+    return {"smooth": smooth, "noise": noise, "outside": 4 * noise - 1.5, "tiny": 0.25 + 6e-5 * rng.integers(0, 3, noise.shape),
+            "denormal": 6e-8 * rng.integers(0, 4, noise.shape), "special": special}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [(64, 16), (61, 35), (128, 48)])
+def test_bc7_search_leaves_constant_components_out_without_a_trace(size):
+    """The partition searches of a texture of one channel leave out green, blue and, in groups (16 x 4 blocks) inside the mip, alpha: the blocks are
+    those of the texels as three channels; and of those with an alpha of 1, whatever the other blocks of a group hold in theirs."""
+    import torch
+
+    width, height = size
+    for name, image in _search_images(height, width).items():
+        four = np.concatenate([image, np.ones((height, width, 1))], axis=-1).astype(np.float16)
+        mixed = four.copy()
+        group = np.zeros(((height + 3) // 4, (width + 3) // 4), dtype=bool)
+        group[::4, ::16] = True  # one block of every group
+        rows, columns = np.nonzero(np.kron(group, np.ones((4, 4), dtype=bool))[:height, :width])
+        mixed[rows, columns, 3] = ((rows + columns) % 3) / 2
+        flat_blocks, mixed_blocks, three_blocks = (
+            binding.block_compress(torch.from_numpy(texels).cuda(), binding.BLOCK_FORMAT_BC7, 0, num_channels=channels).cpu().numpy()
+            for texels, channels in ((four, 4), (mixed, 4), (four, 3)))
+        assert np.array_equal(flat_blocks, three_blocks), name
+        assert np.array_equal(flat_blocks[~group], mixed_blocks[~group]), name
+        red = four.copy()
+        red[..., 1:3] = 0
+        red_blocks, one_blocks = (binding.block_compress(torch.from_numpy(red).cuda(), binding.BLOCK_FORMAT_BC7, 0, num_channels=channels).cpu().numpy()
+                                  for channels in (3, 1))
+        assert np.array_equal(red_blocks, one_blocks), name
