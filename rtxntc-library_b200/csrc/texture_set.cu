@@ -655,7 +655,8 @@ Status TextureSet::GrowStaging(size_t bytes)
 // the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips apart took five launches, each with a ramp at both
 // ends: 326 us for a 2048 x 2048 set that decodes in 250.)
 //
-// `streamed`, an upload beside the decode: decoding the first band should take as long as the rest of the upload does.
+// `streamed`, an upload beside the decode: decoding the first band should take as long as the rest of the upload does (at the present 27
+// Gtexel/s; with 20 the band ended early, and 4096 x 4096 8-bit pixels took 835 us instead of 812).
 int TextureSet::FirstBandRows(size_t hostTexelBytes, bool streamed) const
 {
     const int height = m_geometry.mipHeight[0];
