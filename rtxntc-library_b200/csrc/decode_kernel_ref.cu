@@ -7,13 +7,13 @@
 // reference's output bit for bit: thread = texel, 128-row GEMM chains, weights resident in shared memory, accumulators in
 // tensor memory, as in decode_kernel.cu.
 //
-// Work decomposition.  One CTA per SM of up to eight chains of 128 threads.  The chains share the network and nothing else: each
-// walks tiles of 16 x 8 texels of its own, with its own tables and footprints, and meets only its own threads in
-// barriers.  What bounds the kernels is instruction issue (81 % of the slots busy, Int8 75 %; 8 x 4 warps of 64 registers and 8 x 64
-// tensor-memory columns fill an SM), so the split aims at few instructions and warps that never wait for another chain.  (With four
-// CTAs per SM of two chains each, the four copies of the network left no room for TexelTables, and on average 3.3 of the four were
+// Work decomposition.  One CTA per SM of up to eight chains of 128 threads (chain_walk.cuh).  The chains share the network and nothing else: each
+// walks runs of tiles of 16 x 8 texels of its own, with its own tables and footprints, and meets only its own threads in
+// barriers.  What bounds the kernels is instruction issue (75 % of the slots busy, Int8 77 % and the packed-fp16 pipe 68 %; 8 x 4 warps of 64
+// registers and 8 x 64 tensor-memory columns fill an SM), so the split aims at few instructions and warps that never wait for another chain.
+// (With four CTAs per SM of two chains each, the four copies of the network left no room for TexelTables, and on average 3.3 of the four were
 // active - the scheduler favours the older, whose share ends early: 4096 x 4096 FP8 897 us instead of 832, 8192 x 8192 Int8 4985 instead of
-// 4523.  With the warps' roles as they are now, see WarpRole: 779 and 4190.)
+// 4523, when that was changed.  Now 653 and 3653.)
 //
 // What differs from decode_kernel.cu:
 //   * the A operand holds binary16 values (the de-quantised network inputs / activations), up to 128
