@@ -150,7 +150,7 @@ private:
     // An upload of this size (73 us) is worth the second launch even when the texels stay on the device.
     static constexpr size_t kStreamedUploadBytes = size_t(4) << 20;
     int FirstBandRows(size_t hostTexelBytes, bool streamed) const;
-    int LatentRows(int firstRows) const;
+    int LatentRows(int firstRows, int neuralMip) const;
     cudaError_t UploadFirst(int firstRows);
     cudaStream_t m_uploadStream = nullptr;
     cudaEvent_t m_eventUploaded = nullptr;
@@ -655,8 +655,8 @@ Status TextureSet::GrowStaging(size_t bytes)
 // the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips apart took five launches, each with a ramp at both
 // ends: 326 us for a 2048 x 2048 set that decodes in 250.)
 //
-// `streamed`, an upload beside the decode: decoding the first band should take as long as the rest of the upload does (at the present 27
-// Gtexel/s; with 20 the band ended early, and 4096 x 4096 8-bit pixels took 835 us instead of 812).
+// `streamed`, an upload beside the decode: decoding the first band should take as long as the rest of the upload does, at the 27 Gtexel/s
+// of the present kernels and what many copies get of the host link.
 int TextureSet::FirstBandRows(size_t hostTexelBytes, bool streamed) const
 {
     const int height = m_geometry.mipHeight[0];
@@ -665,45 +665,54 @@ int TextureSet::FirstBandRows(size_t hostTexelBytes, bool streamed) const
     float share = hostTexelBytes ? 1.f / (1.f + 0.35f * float(hostTexelBytes)) : 0.f;
     if (streamed)
     {
-        const float latentBytes = float(m_geometry.latentPixelOffset[1]) * float(m_geometry.numLayers) * 2.f;
-        const float upload = latentBytes / 57.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 27.f; // nanoseconds
+        const float upload = float(m_latentBytes) / 50.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 27.f; // nanoseconds
         share = std::max(share, upload / (upload + decode));
     }
     return std::min(height, (int(float(height) * share) + 15) & ~15);
 }
 
-// Rows of neural mip 0 that texel rows [0, firstRows) of mip 0 read, apart from the last one (row -1 wraps around to it).
-int TextureSet::LatentRows(int firstRows) const
+// Rows of a neural mip that texel rows [0, firstRows) of mip 0 read, apart from the last one (row -1 wraps around to it).
+int TextureSet::LatentRows(int firstRows, int neuralMip) const
 {
-    return int((int64_t(firstRows) * m_geometry.latentHeight[0] + m_geometry.mipHeight[0] - 1) / m_geometry.mipHeight[0]) + 2;
+    return int((int64_t(firstRows) * m_geometry.latentHeight[neuralMip] + m_geometry.mipHeight[0] - 1) / m_geometry.mipHeight[0]) + 2;
 }
 
-// The compressed data to the device on the upload stream, what the first rows of mip 0 read before the rest; m_stream waits
-// for the former here, the caller makes it wait for m_eventUploaded before it reads the rest.
+// The compressed data to the device on the upload stream, what the first rows of mip 0 read before the rest: rows of neural mips 0 and 1, and the
+// networks.  m_stream waits for those here, the caller makes it wait for m_eventUploaded before it reads the rest.  (With all of the other neural
+// mips among the first, a quarter of the upload, 4096 x 4096 8-bit pixels took 812 us instead of 791.)
 cudaError_t TextureSet::UploadFirst(int firstRows)
 {
-    const size_t rowBytes = size_t(m_geometry.latentWidth[0]) * 2, planeBytes = rowBytes * m_geometry.latentHeight[0];
-    const size_t otherMips = planeBytes * m_geometry.numLayers; // the networks follow the latents
-    const int needed = LatentRows(firstRows), last = m_geometry.latentHeight[0] - 1;
-    auto copyRows = [&](int begin, int end) { // rows of every layer of neural mip 0
-        return cudaMemcpy2DAsync(m_deviceUpload + begin * rowBytes, planeBytes, m_hostUpload + begin * rowBytes, planeBytes,
-            (end - begin) * rowBytes, m_geometry.numLayers, cudaMemcpyHostToDevice, m_uploadStream);
-    };
+    const int layers = m_geometry.numLayers;
     cudaError_t err = cudaEventRecord(m_eventUploaded, m_stream); // what is queued reads the data of an earlier upload
     if (err == cudaSuccess)
         err = cudaStreamWaitEvent(m_uploadStream, m_eventUploaded, 0);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(m_deviceUpload + otherMips, m_hostUpload + otherMips, m_uploadBytes - otherMips, cudaMemcpyHostToDevice, m_uploadStream);
-    if (err == cudaSuccess)
-        err = copyRows(0, needed);
-    if (err == cudaSuccess)
-        err = copyRows(last, last + 1);
+    auto copy = [&](size_t begin, size_t end) {
+        if (err == cudaSuccess && begin < end)
+            err = cudaMemcpyAsync(m_deviceUpload + begin, m_hostUpload + begin, end - begin, cudaMemcpyHostToDevice, m_uploadStream);
+    };
+    auto copyRows = [&](int neuralMip, int begin, int end) { // rows of every layer
+        if (err != cudaSuccess || begin >= end)
+            return;
+        const size_t rowBytes = size_t(m_geometry.latentWidth[neuralMip]) * 2, planeBytes = rowBytes * m_geometry.latentHeight[neuralMip];
+        const size_t offset = m_geometry.latentPixelOffset[neuralMip] * layers * 2 + begin * rowBytes;
+        err = cudaMemcpy2DAsync(m_deviceUpload + offset, planeBytes, m_hostUpload + offset, planeBytes, (end - begin) * rowBytes, layers,
+            cudaMemcpyHostToDevice, m_uploadStream);
+    };
+    copy(m_latentBytes, m_uploadBytes); // the networks follow the latents
+    for (int neuralMip = 0; neuralMip < 2; ++neuralMip)
+    {
+        const int last = m_geometry.latentHeight[neuralMip] - 1;
+        copyRows(neuralMip, 0, std::min(LatentRows(firstRows, neuralMip), last));
+        copyRows(neuralMip, last, last + 1);
+    }
     if (err == cudaSuccess)
         err = cudaEventRecord(m_eventUploaded, m_uploadStream);
     if (err == cudaSuccess)
         err = cudaStreamWaitEvent(m_stream, m_eventUploaded, 0);
-    if (err == cudaSuccess)
-        err = copyRows(needed, last);
+    for (int neuralMip = 0; neuralMip < 2; ++neuralMip)
+        copyRows(neuralMip, LatentRows(firstRows, neuralMip), m_geometry.latentHeight[neuralMip] - 1);
+    const size_t planes = size_t(m_geometry.latentWidth[1]) * m_geometry.latentHeight[1];
+    copy((m_geometry.latentPixelOffset[1] + planes) * layers * 2, m_latentBytes);
     if (err == cudaSuccess)
         err = cudaEventRecord(m_eventUploaded, m_uploadStream);
     return err;
@@ -733,7 +742,7 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
     const bool mayStream = !pOutStats && m_latentBytes >= kStreamedUploadBytes;
     const int firstRows = rowRanges ? 0 : FirstBandRows(forHost ? conversion
         ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat) : size_t(m_geometry.channels) * sizeof(__half) : 0, mayStream);
-    const bool streamed = firstRows > 0 && mayStream && LatentRows(firstRows) < m_geometry.latentHeight[0] - 1;
+    const bool streamed = firstRows > 0 && mayStream && LatentRows(firstRows, 0) < m_geometry.latentHeight[0] - 1;
     // Work queued later - another upload, sampling, a refill of the pinned image - relies on m_stream for the end of this upload.
     // Until m_stream waits for its last part, a return with an error has to wait here.
     struct UploadInFlight
