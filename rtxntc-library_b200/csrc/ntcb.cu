@@ -15,6 +15,7 @@
 
 #include "decode_kernel.h"
 #include "error.h"
+#include "footprint.h"
 #include "network_shape.h"
 
 namespace ntcb
@@ -112,15 +113,12 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprin
     km.invHeight = 1.0f / float(m.height);
     km.positionScale = m.positionScale;
     km.positionLod = m.positionLod;
-    // Largest footprint a run of tiles can have in each grid: the tap index of the last column (row) minus
-    // that of the first is at most floor((size - 1) * grid / mip) + 1, plus the second tap.  The run is as long as allowed, as the mip is
-    // wide, and as its footprint fits.
+    // The run is as long as allowed, as the mip is wide, and as the largest footprint it can have in each grid fits.
     km.strideBytes = layers == 1 ? 8 : layers <= 3 ? 24 : 40;
     const long long hiCapacity = footprintHiBytes / km.strideBytes, loCapacity = footprintLoBytes / km.strideBytes;
-    auto footprint = [](int grid, int mip, int span) { return (long long)((long long)span * grid / mip) + 3; };
     auto fits = [&](int columns) {
-        return footprint(m.hiWidth, m.width, columns - 1) * footprint(m.hiHeight, m.height, tileHeight - 1) <= hiCapacity &&
-               footprint(m.loWidth, m.width, columns - 1) * footprint(m.loHeight, m.height, tileHeight - 1) <= loCapacity;
+        return FootprintPixels(m.hiWidth, m.width, columns - 1) * FootprintPixels(m.hiHeight, m.height, tileHeight - 1) <= hiCapacity &&
+               FootprintPixels(m.loWidth, m.width, columns - 1) * FootprintPixels(m.loHeight, m.height, tileHeight - 1) <= loCapacity;
     };
     km.staged = fits(tileWidth) ? 1 : 0;
     km.runTiles = 1;

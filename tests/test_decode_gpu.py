@@ -255,6 +255,25 @@ def test_row_ranges_tile_rows_and_guard_bands(oracle, numerics):
         assert (got[~rows] == -7.0).all()
 
 
+# Wide mips (23953 and 65513 texels) over a coarse grid of a third of their size, of which some tiles read 8 columns, by rounding, where 7 are the
+# real extent: 8 x 5 pixels of 40 bytes are more than the smallest staging buffers hold.
+@BOTH_NUMERICS
+@pytest.mark.parametrize("width", [47906, 131027])
+def test_wide_mips_whose_footprints_rounding_makes_wider(oracle, width, numerics):
+    data = synthetic.make_texture_set(synthetic.TextureSetSpec(width, 24, 4, 2, 3, 16, seed=29, network="unit"))
+    checker = oracle.OracleSet.from_synthetic(data)
+    resident = binding.ResidentTextureSet.from_synthetic(data, numerics=numerics)
+    tally = _Tally(numerics)
+    for use_int8 in (True, False):
+        resident.out.fill_(float("nan"))
+        resident.decode(use_int8, mips=[1])
+        _sync()
+        resident.check_status()
+        decoded = resident.mip_numpy(1)
+        tally.add(decoded, _restated(oracle, checker, 1, use_int8, numerics, decoded), use_int8, width)
+    tally.check()
+
+
 # Launches of enough tiles (16 x 8 texels) for 1184 chains to walk them in runs of two (8 tiles a chain) or of four (32 a chain): mip sizes that
 # are no multiples of a tile or a run, grids at 1/2 to 1/6 of the mip (the longest runs do not fit all of them), and powers of two.
 @pytest.mark.parametrize("numerics,shape", [

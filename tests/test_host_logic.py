@@ -529,3 +529,26 @@ def test_rounding_to_the_activation_grid_as_a_subnormal_number():
     assert float(np.float16(step * 2 ** 22)) == step * 2 ** 22 and float(np.float16(16 * step)) == 16 * step
     scaled = (code << 2).view(np.float16).astype(np.float64)
     assert np.array_equal(half(scaled * (step * 2 ** 22) - 16 * step), half(np.rint(p) * step))
+
+
+def test_no_run_of_tiles_reads_more_latent_pixels_than_its_buffer_is_checked_for(tmp_path):
+    """The footprint bound that decides whether a mip's latents are staged in shared memory, against the kernels' binary32 taps, at every run of mips
+    of texture sets up to 131072 wide: among them widths where rounding makes a footprint a column wider than its real extent."""
+    import os
+    import subprocess
+
+    from conftest import ROOT
+
+    binary = str(tmp_path / "footprint_bound")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-march=x86-64-v3", "-ffp-contract=off", os.path.join(ROOT, "tests", "cpp", "footprint_bound.cpp"),
+                    "-o", binary], check=True)
+    rng = np.random.default_rng(11)
+    widths = {47906, 109460, 109889, 131027, 131068, 131072, 8192, 4097} | {int(2.0 ** x) for x in rng.uniform(0, 17, 400)}
+    pairs = {(4, 4 << 17), (1 << 23, 1 << 22), ((1 << 23) + 12345, (1 << 22) - 77)}  # a grid finer than its mip; sizes that binary32 rounds
+    for width in widths:
+        for scale in range(1, 7):
+            geo = synthetic.TextureSetSpec(width, 48, 4, min(4, int(width).bit_length()), scale, 4, seed=0).geometry()
+            for mip in geo.color_mips:
+                pairs |= {(mip.width, geo.latent_width[mip.neural_lod + grid]) for grid in (0, 1)}
+    wider = subprocess.run([binary], input="".join("%d %d\n" % pair for pair in sorted(pairs)), stdout=subprocess.PIPE, text=True, check=True).stdout
+    assert wider == ""
