@@ -37,7 +37,8 @@ struct __align__(16) TexelTables
 };
 
 // ... of the kernels whose layer-0 operand is 64-byte rows of codes.
-struct __align__(16) CodesStage : ChainStage<TileTables<ChainTile>, kRefFootprintHiBytes, kRefFootprintLoBytes>
+template <int kHiBytes, int kLoBytes>
+struct __align__(16) CodesStage : ChainStage<TileTables<ChainTile>, kHiBytes, kLoBytes>
 {
     TexelTables texels;
 };
@@ -146,8 +147,8 @@ struct ChainContext
 // The 64-byte operand row of a texel: 48 inputs as codes, then K padding - zeros (e4m3) or the constant inputs of the bias slots (int8).
 // `column`: in the run.  `known`: TexelTables, and the row's last two chunks where the layers after the first leave them alone (FP8: their operands are
 // in tensor memory), are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
-template <bool kFp8, bool kReferenceDivision, int kLayers>
-__device__ __forceinline__ void BuildCodes(const KernelParams& params, const KernelMip& mip, CodesStage& stage, const ChainContext& ctx,
+template <bool kFp8, bool kReferenceDivision, int kLayers, typename Stage>
+__device__ __forceinline__ void BuildCodes(const KernelParams& params, const KernelMip& mip, Stage& stage, const ChainContext& ctx,
     int column, int tileRow, bool known, int2 shift)
 {
     if (!mip.staged)

@@ -167,9 +167,10 @@ struct __align__(128) ExactStorage
     uint32_t claims;              // inference on sample: query tiles handed out so far
     uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands, 64 bytes a row, in core-matrix order; then the CodesStages
+    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands, 64 bytes a row, in core-matrix order; then the ExactStages
 };
-static_assert(sizeof(ExactStorage) + kMaxChains * sizeof(CodesStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
+using ExactStage = CodesStage<kExactFootprint.hiBytes, kExactFootprint.loBytes>;
+static_assert(sizeof(ExactStorage) + kMaxChains * sizeof(ExactStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
 // First half of a layer: hands the A operand written before this call to the tensor core, an elected lane of the warp of kIssuingRole.  Returns
 // nonzero (uniformly over the chain) when some thread gave up on a wait.
@@ -412,7 +413,7 @@ template <bool kFp8>
 struct ExactChain
 {
     using Storage = ExactStorage;
-    using Stage = CodesStage;
+    using Stage = ExactStage;
     template <typename First>
     static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp,
         First first)
@@ -466,8 +467,8 @@ cudaError_t LaunchDecodeLayers(const KernelParams& params, int ctas, cudaStream_
     auto launch = [&](auto layers) {
         constexpr int kLayers = decltype(layers)::value;
         const int chains = ChainsPerCta(uint32_t(params.totalTiles), ctas);
-        return LaunchChains(DecodeKernel<kFp8, kConvert, kLayers>, done[kLayers], SharedBytes<ExactStorage>(chains, sizeof(CodesStage)),
-            SharedBytes<ExactStorage>(kMaxChains, sizeof(CodesStage)), chains, params, ctas, stream);
+        return LaunchChains(DecodeKernel<kFp8, kConvert, kLayers>, done[kLayers], SharedBytes<ExactStorage>(chains, sizeof(ExactStage)),
+            SharedBytes<ExactStorage>(kMaxChains, sizeof(ExactStage)), chains, params, ctas, stream);
     };
     switch (params.numLayers)
     {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "footprint.h"
 #include "output_convert.cuh"
 
 struct NtcbOutputConversion; // include/ntcb.h
@@ -75,17 +76,8 @@ constexpr int kRefOperandBytes = 128 * 96;
 // A CTA is up to eight chains of 128 threads - 64 tensor-memory columns and 64 registers a thread each, which
 // fills an SM - that share the network in shared memory and nothing else.  Each walks tiles of its own, 16 x 8 texels, in runs of
 // up to four side by side, with its own tables and footprints, and meets only its own threads in barriers.
-constexpr int kChainTileWidth = 16;
-constexpr int kChainTileHeight = 8;
-constexpr int kMaxRunTiles = 4; // ... tiles of a run, see KernelMip::runTiles
 constexpr int kMaxChains = 8;
 constexpr int kMaxThreadsPerCta = 128 * kMaxChains;
-// Footprints of a chain: what a tile covers at a grid-to-mip ratio of 1 (high-res: 18 x 10 pixels of 24 bytes) and 1/2
-// (low-res: 10 x 6), or a run of tiles at a smaller one.
-constexpr int kRefFootprintHiBytes = 4352;
-constexpr int kRefFootprintLoBytes = 1536;
-constexpr int kRefInt8FootprintHiBytes = kRefFootprintHiBytes;
-constexpr int kRefInt8FootprintLoBytes = 1440;
 
 // Dynamic shared memory a CTA may have for `ctas` of them to be resident: an SM has 228 KB, 1 KB per CTA is the system's.
 template <int ctas>

@@ -161,7 +161,7 @@ struct __align__(16) RefTileTables
     uint32_t pad[2];
 };
 
-struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes>
+struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8Footprint.hiBytes, kRefInt8Footprint.loBytes>
 {
     TexelTables texels;
 };
@@ -753,9 +753,10 @@ struct __align__(128) RefFp8SharedStorage
     uint32_t claims;              // inference on sample: query tiles handed out so far
     uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row; then the CodesStages
+    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row; then the RefFp8Stages
 };
-static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(CodesStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
+using RefFp8Stage = CodesStage<kRefFp8Footprint.hiBytes, kRefFp8Footprint.loBytes>;
+static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(RefFp8Stage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 e4m3 operands, binary16 accumulators.
 __device__ __forceinline__ void UmmaE4m3F16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
@@ -999,7 +1000,7 @@ __device__ __forceinline__ void SetupCtaRefFp8(RefFp8SharedStorage& shared, cons
 struct Fp8Chain
 {
     using Storage = RefFp8SharedStorage;
-    using Stage = CodesStage;
+    using Stage = RefFp8Stage;
     template <typename First>
     static __device__ __forceinline__ void Setup(Storage& shared, const uint8_t* network, uint32_t* status, uint32_t polls, int tid, int warp,
         First first)
@@ -1053,8 +1054,8 @@ cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStre
         constexpr int kLayers = decltype(layers)::value;
         const int chains = ChainsPerCta(uint32_t(params.totalTiles), ctas);
         if constexpr (kFp8Weights) // 8-bit operands
-            return LaunchChains(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, sizeof(CodesStage)),
-                SharedBytes<RefFp8SharedStorage>(kMaxChains, sizeof(CodesStage)), chains, params, ctas, stream);
+            return LaunchChains(DecodeKernelRefFp8<kConvert, kLayers>, done[kLayers], SharedBytes<RefFp8SharedStorage>(chains, sizeof(RefFp8Stage)),
+                SharedBytes<RefFp8SharedStorage>(kMaxChains, sizeof(RefFp8Stage)), chains, params, ctas, stream);
         else
             return LaunchChains(DecodeKernelRef<kConvert, kLayers>, done[kLayers], SharedBytes<RefSharedStorage>(chains, sizeof(RefStage)),
                 SharedBytes<RefSharedStorage>(kMaxChains, sizeof(RefStage)), chains, params, ctas, stream);

@@ -1,10 +1,29 @@
-// How many latent pixels a run of texels can touch: what decides whether its footprint fits a staging buffer.
+// Runs of tiles and their footprints: how many latent pixels one can touch, and whether its buffers in shared memory hold them.
 #pragma once
 
 #include <stdint.h>
 
 namespace ntcb
 {
+
+constexpr int kChainTileWidth = 16;
+constexpr int kChainTileHeight = 8;
+constexpr int kMaxRunTiles = 4; // tiles of a run, see KernelMip::runTiles
+
+// Shared memory of a chain for the latents of a run of tiles, in the high-res and the low-res grid.
+struct FootprintBuffers
+{
+    int hiBytes, loBytes;
+};
+// What a tile covers at a grid-to-mip ratio of 1 (high-res: 18 x 10 pixels of 24 bytes) and 1/2 (low-res: 10 x 6), or a run of tiles at a smaller
+// one.
+constexpr FootprintBuffers kRefFp8Footprint{4352, 1536};
+constexpr FootprintBuffers kRefInt8Footprint{4352, 1440}; // (all that the CTA has left)
+// The exact-accumulation kernels have room for a tile at a ratio of 4/5 with four latent layers (15 x 8 pixels of 40 bytes, 9 x 5).  (With the FP8
+// kernels' buffers mips at 4/5 and 2/3 were read tap by tap: mip 1 of a 3000 x 4000 Int8 set of 16 features at scale 3 took 224 us, now
+// 196, FP8 162 and 135; mip 2 of 4096 x 4096 at scale 5 79.5 and 72.6.  With 6144 and 2432 bytes more runs would be longer, some for the worse:
+// 3000 x 2000 Int8, 12 features, 445 and 455 us.)
+constexpr FootprintBuffers kExactFootprint{4800, 1808};
 
 // Most latent pixels, of a grid of `grid` pixels, that texels x .. x + span of an axis of `extent` texels read: the last tap's index minus
 // the first's, plus the second tap of each end.
@@ -20,6 +39,26 @@ constexpr long long FootprintPixels(int grid, int extent, int span)
     // (span + extent * units / 2^24) * grid / extent
     const long long slack = (long long)extent * units;
     return (long long)((__int128)grid * (((long long)span << 24) + slack) / ((long long)extent << 24)) + 3;
+}
+
+// Tiles side by side, a power of two up to `most`, whose footprints in both grids fit the buffers; 0: not even those of one do, and texels read their
+// taps from global memory, as they do where a footprint has more pixels than its texels have taps.  (Mip 1 of a 4096 x 4096 set of 4 features at
+// scale 1, 33 x 17 pixels for 128 texels, exact accumulation: staged 301 us Int8 and 233 FP8, read directly 237 and 167.)  A run is no longer than its
+// mip is wide.
+constexpr int StagedTiles(int hiWidth, int hiHeight, int loWidth, int loHeight, int width, int height, int pixelBytes, FootprintBuffers buffers,
+    int most)
+{
+    int tiles = 0;
+    for (int next = 1; next <= most && (next == 1 || (next / 2) * kChainTileWidth < width); next *= 2)
+    {
+        const int columns = next * kChainTileWidth - 1, rows = kChainTileHeight - 1;
+        const long long hiPixels = FootprintPixels(hiWidth, width, columns) * FootprintPixels(hiHeight, height, rows);
+        if (hiPixels > 4 * next * kChainTileWidth * kChainTileHeight || hiPixels > buffers.hiBytes / pixelBytes ||
+            FootprintPixels(loWidth, width, columns) * FootprintPixels(loHeight, height, rows) > buffers.loBytes / pixelBytes)
+            break;
+        tiles = next;
+    }
+    return tiles;
 }
 
 } // namespace ntcb

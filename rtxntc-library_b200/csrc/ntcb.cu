@@ -15,7 +15,6 @@
 
 #include "decode_kernel.h"
 #include "error.h"
-#include "footprint.h"
 #include "network_shape.h"
 
 namespace ntcb
@@ -92,8 +91,7 @@ bool ValidMip(const NtcbMipDesc& m, bool pairedOutput)
 }
 
 // The kernel's view of one mip (everything but its place in the tile list).  `maxRunTiles`: the longest run of tiles.
-void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprintHiBytes = kRefFootprintHiBytes,
-    int footprintLoBytes = kRefFootprintLoBytes, int maxRunTiles = 1)
+void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, FootprintBuffers buffers, int maxRunTiles)
 {
     constexpr int tileWidth = kChainTileWidth, tileHeight = kChainTileHeight;
     km.width = m.width;
@@ -113,17 +111,10 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, int footprin
     km.invHeight = 1.0f / float(m.height);
     km.positionScale = m.positionScale;
     km.positionLod = m.positionLod;
-    // The run is as long as allowed, as the mip is wide, and as the largest footprint it can have in each grid fits.
     km.strideBytes = layers == 1 ? 8 : layers <= 3 ? 24 : 40;
-    const long long hiCapacity = footprintHiBytes / km.strideBytes, loCapacity = footprintLoBytes / km.strideBytes;
-    auto fits = [&](int columns) {
-        return FootprintPixels(m.hiWidth, m.width, columns - 1) * FootprintPixels(m.hiHeight, m.height, tileHeight - 1) <= hiCapacity &&
-               FootprintPixels(m.loWidth, m.width, columns - 1) * FootprintPixels(m.loHeight, m.height, tileHeight - 1) <= loCapacity;
-    };
-    km.staged = fits(tileWidth) ? 1 : 0;
-    km.runTiles = 1;
-    while (km.runTiles < maxRunTiles && km.runTiles * tileWidth < m.width && fits(2 * km.runTiles * tileWidth))
-        km.runTiles *= 2;
+    const int staged = StagedTiles(m.hiWidth, m.hiHeight, m.loWidth, m.loHeight, m.width, m.height, km.strideBytes, buffers, maxRunTiles);
+    km.staged = staged > 0;
+    km.runTiles = staged > 0 ? staged : 1;
     // Tables that do not depend on the tile: with power-of-two sizes all the tap arithmetic is exact in
     // binary32, and when a tile's width and height map to whole latent pixels of both grids (and to whole
     // periods of the positional encoding) moving from tile to tile shifts every tap by an integer.
@@ -680,10 +671,7 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
         if (m.rowBegin == m.rowEnd)
             continue; // nothing of this mip belongs to this launch
         KernelMip& km = k.mips[used++];
-        if (reference && !fp8)
-            FillKernelMip(m, p->numFeatures / 4, km, kRefInt8FootprintHiBytes, kRefInt8FootprintLoBytes, longestRun);
-        else
-            FillKernelMip(m, p->numFeatures / 4, km, kRefFootprintHiBytes, kRefFootprintLoBytes, longestRun);
+        FillKernelMip(m, p->numFeatures / 4, km, !reference ? kExactFootprint : fp8 ? kRefFp8Footprint : kRefInt8Footprint, longestRun);
         km.firstTile = int(tiles);
         km.storeBytes = 4;
         if (k.convert || p->outputLayout == NTCB_LAYOUT_INTERLEAVED)
@@ -784,7 +772,7 @@ int ntcb_sample(const NtcbSampleParams* p, void* stream)
             SetError("ntcb_sample: mip %d has invalid dimensions or offsets.", i);
             return NTCB_ERR_INVALID_ARGUMENT;
         }
-        FillKernelMip(m, k.numLayers, k.mips[i]);
+        FillKernelMip(m, k.numLayers, k.mips[i], kRefFp8Footprint, 1); // (nothing is staged)
         if (k.interleaved)
         {
             // the grid's place in the pixel-major copy: slots of 1, 2 or 4 elements per pixel
