@@ -17,6 +17,7 @@
 #include "container.h"
 #include "decode_kernel.h"
 #include "error.h"
+#include "first_band.h"
 #include "ntcb.h"
 #include "ntcb_host.h"
 #include "output_convert.cuh"
@@ -146,10 +147,8 @@ private:
     // read may follow, so that it can start copying the first band while the rest is still being decoded (the
     // read-back, not the decode, bounds Decompress + ReadChannels), or when the upload is large.  See FirstBandRows.
     static constexpr int kBands = 2;
-    static constexpr int kBandMinRows = 512;
     // An upload of this size (73 us) is worth the second launch even when the texels stay on the device.
     static constexpr size_t kStreamedUploadBytes = size_t(4) << 20;
-    int FirstBandRows(size_t hostTexelBytes, bool streamed) const;
     int LatentRows(int firstRows, int neuralMip) const;
     cudaError_t UploadFirst(int firstRows);
     cudaStream_t m_uploadStream = nullptr;
@@ -647,30 +646,6 @@ Status TextureSet::GrowStaging(size_t bytes)
     return NTCB_OK;
 }
 
-// Rows of mip 0 that are decoded in a launch of their own, 0: none.
-//
-// For a host read of texels of `hostTexelBytes` bytes (0: the texels stay on the device): copying the first band should take
-// as long as decoding everything else does, so that the copies never wait again.  The kernels decode about 20 Gtexel/s, the
-// host link takes about 57 GB/s: copying a texel of n bytes takes 0.35 n times as long as decoding it, and the band's share of
-// the work is 1 / (1 + 0.35 n).  (Four equal bands and the other mips apart took five launches, each with a ramp at both
-// ends: 326 us for a 2048 x 2048 set that decodes in 250.)
-//
-// `streamed`, an upload beside the decode: decoding the first band should take as long as the rest of the upload does, at the 27 Gtexel/s
-// of the present kernels and what many copies get of the host link.
-int TextureSet::FirstBandRows(size_t hostTexelBytes, bool streamed) const
-{
-    const int height = m_geometry.mipHeight[0];
-    if (height < kBandMinRows)
-        return 0;
-    float share = hostTexelBytes ? 1.f / (1.f + 0.35f * float(hostTexelBytes)) : 0.f;
-    if (streamed)
-    {
-        const float upload = float(m_latentBytes) / 50.f, decode = float(m_geometry.mipWidth[0]) * float(height) / 27.f; // nanoseconds
-        share = std::max(share, upload / (upload + decode));
-    }
-    return std::min(height, (int(float(height) * share) + 15) & ~15);
-}
-
 // Rows of a neural mip that texel rows [0, firstRows) of mip 0 read, apart from the last one (row -1 wraps around to it).
 int TextureSet::LatentRows(int firstRows, int neuralMip) const
 {
@@ -740,8 +715,10 @@ Status TextureSet::DecodeInto(const int32_t* rowRanges, DecompressionStats* pOut
     // Decompress of a loaded set (src/TextureSet.cpp:1691-1757).  A large upload runs beside the decode: the first rows of mip 0
     // start when what they read has arrived.  (Not when the device time is asked for: it would include waiting for the host link.)
     const bool mayStream = !pOutStats && m_latentBytes >= kStreamedUploadBytes;
-    const int firstRows = rowRanges ? 0 : FirstBandRows(forHost ? conversion
-        ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat) : size_t(m_geometry.channels) * sizeof(__half) : 0, mayStream);
+    const size_t hostTexelBytes = !forHost ? 0 : conversion ? size_t(conversion->components) * BytesPerComponent(conversion->channelFormat)
+                                                            : size_t(m_geometry.channels) * sizeof(__half);
+    const int firstRows = rowRanges ? 0 : FirstBandRows(m_geometry.mipWidth[0], m_geometry.mipHeight[0], hostTexelBytes, mayStream ? m_latentBytes : 0,
+                                              DecodeRate(m_numerics == NTCB_NUMERICS_EXACT, useInt8Weights));
     const bool streamed = firstRows > 0 && mayStream && LatentRows(firstRows, 0) < m_geometry.latentHeight[0] - 1;
     // Work queued later - another upload, sampling, a refill of the pinned image - relies on m_stream for the end of this upload.
     // Until m_stream waits for its last part, a return with an error has to wait here.

@@ -839,3 +839,21 @@ def test_which_mips_have_their_latents_staged(tmp_path):
                 assert int(tiles) >= 1, (kernel, case)
             elif case[-1] >= 1.9:  # more latent pixels than taps
                 assert int(tiles) == 0, (kernel, case)
+
+
+def test_first_band_of_a_streamed_upload_by_the_kernels_rate(tmp_path):
+    """The first rows of a decompress, decoded while the rest of the upload is under way, take as long as that does by the rate of the set's own
+    kernels: the slowest, exact accumulation with Int8 weights (17.7 to 19 texels a nanosecond), get fewer."""
+    mips = [(2048, 2048, 0, 22 << 20), (4096, 4096, 0, 45 << 20), (4000, 3000, 20, 11 << 20), (4096, 4096, 24, 0), (2048, 511, 16, 22 << 20)]
+    answers = _build_cpp(tmp_path, "first_band")("%d %d %d %d %d %d" % (*mip, exact, int8) for mip in mips for exact in (0, 1) for int8 in (0, 1))
+    rows = np.array(answers.split(), dtype=int).reshape(len(mips), 2, 2)  # [mip][exact][int8]
+    for (width, height, texel_bytes, streamed), answer in zip(mips, rows):
+        assert answer[0, 0] == answer[0, 1] == answer[1, 0] and (answer <= height).all() and (answer % 16 == 0).all()
+        assert (answer > 0).all() == (height >= 512)
+        if not streamed:
+            assert (answer == answer[0, 0]).all()
+        elif height >= 512:
+            # rounded down to a row and up to 16: from a row before to 15 after where the two times meet, which differ by `row` more with every row
+            decode, rest = answer[1, 1] * width / 18, streamed / 50 * (1 - answer[1, 1] / height)  # nanoseconds
+            row = width / 18 + streamed / 50 / height
+            assert answer[1, 1] < answer[0, 0] and -row <= decode - rest <= 16 * row
