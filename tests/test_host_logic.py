@@ -547,264 +547,6 @@ def test_no_run_of_tiles_reads_more_latent_pixels_than_its_buffer_is_checked_for
     """The footprint bound that decides whether a mip's latents are staged in shared memory, against the kernels' binary32 taps, at every run of mips
     of texture sets up to 131072 wide: among them widths where rounding makes a footprint a column wider than its real extent."""
     rng = np.random.default_rng(11)
-    inputs, outputs = geometry.MLP_LAYER_INPUTS, geometry.MLP_LAYER_OUTPUTS
-    offsets = (0, 6144, 12288, 15360)
-    seen = set()
-    for draw in range(24):
-        weights = rng.integers(-128, 128, size=8192).astype(np.int8)
-        scales = (2.0 ** rng.uniform(-36, 14, 160) * rng.choice([-1, 1], 160)).astype(np.float32)
-        if draw % 3 == 0:  # few significant bits: products halfway between two halves
-            scales = (scales.view(np.uint32) & np.uint32(0xFFFC0000)).view(np.float32)
-        scales[:4] = (np.inf, np.nan, 0.0, -0.0)
-        biases = rng.integers(-2 ** 20, 2 ** 20, size=160).astype(np.int32)
-        staged = binding.stage_network(weights.tobytes() + scales.tobytes() + biases.tobytes(), binding.WEIGHTS_INT8, binding.NUMERICS_REFERENCE)
-        halves = staged.view(np.uint16)
-        start = column = 0
-        with np.errstate(all="ignore"):
-            for layer in range(4):
-                nin, nout = inputs[layer], outputs[layer]
-                factor = np.float32(127.5) if layer == 0 else np.float32(1) / (np.float32(3.1875) / np.float32(255))
-                layer_scales = scales[column:column + nout] * factor
-                products = weights[start:start + nin * nout].reshape(nout, nin).astype(np.float32) * layer_scales[:, None]
-                # chunks of eight inputs: half (n, k) at (k / 8) * 8 * nout + 8 n + k % 8
-                got = halves[offsets[layer] // 2:offsets[layer] // 2 + nin * nout].reshape(nin // 8, nout, 8).transpose(1, 0, 2).reshape(nout, nin)
-                expected = np.where(np.isnan(products), np.uint16(0x7FFF), products.astype(np.float16).view(np.uint16))
-                assert np.array_equal(got, expected), (draw, layer)
-                seen.update(np.unique(expected >> 10))
-                if layer == 0:
-                    bias = biases[:nout].astype(np.float32) * scales[:nout]
-                    expected = np.where(np.isnan(bias), np.uint16(0x7FFF), bias.astype(np.float16).view(np.uint16))
-                    assert np.array_equal(halves[8192:8192 + 8 * nout:8], expected)
-                start += nin * nout
-                column += nout
-    assert len(seen) == 64  # every sign and exponent
-
-
-def test_kept_launch_parameters_follow_the_set():
-    """ResidentTextureSet keeps the parameters of a whole-set decode: they are filled again when anything they were filled from is
-    replaced, the geometry included."""
-    import torch
-
-    class Recording(binding.ResidentTextureSet):
-        def launch(self, params):
-            launched.append(binding.DecodeParams.from_buffer_copy(params))
-
-    launched = []
-    first, second = (synthetic.make_texture_set(synthetic.TextureSetSpec(w, 32, 4, 1, 2, 8, seed=1)) for w in (64, 48))
-    resident = Recording.from_synthetic(first, device="cpu")
-    resident.decode(True)
-    resident.decode(True)
-    assert [p.mips[0].width for p in launched] == [64, 64] and launched[0].out == launched[1].out
-    resident.geometry = second.geometry
-    resident.decode(True)
-    assert launched[-1].mips[0].width == 48
-    resident.out = torch.empty_like(resident.out)
-    resident.decode(True)
-    assert launched[-1].out == resident.out.data_ptr() != launched[0].out
-    resident.latents = resident.latents.clone()
-    resident.decode(True)
-    assert launched[-1].latents == resident.latents.data_ptr()
-
-
-def test_stage_network_rejects_wrong_sizes():
-    for numerics in (binding.NUMERICS_REFERENCE, binding.NUMERICS_EXACT):
-        with pytest.raises(binding.NtcbError) as error:
-            binding.stage_network(bytes(100), binding.WEIGHTS_INT8, numerics)
-        assert error.value.code == -1
-
-
-def test_decode_validates_arguments_before_touching_the_gpu():
-    lib = binding.lib()
-    params = binding.DecodeParams()
-    assert lib.ntcb_decode(ctypes.byref(params), None) == -1
-    assert b"NULL" in lib.ntcb_last_error()
-    geo = synthetic.TextureSetSpec(64, 64, 4, 1, 2, 8, seed=0).geometry()
-    good = binding.fill_params(geo, 0x1000, 0x2000, 0x3000, 0x4000, binding.WEIGHTS_INT8)
-    good.channels = 5
-    assert lib.ntcb_decode(ctypes.byref(good), None) == -1
-    good.channels = 4
-    good.mips[0].rowEnd = 100
-    assert lib.ntcb_decode(ctypes.byref(good), None) == -1
-
-
-def test_sample_and_interleave_validate_arguments_before_touching_the_gpu():
-    lib = binding.lib()
-    geo = synthetic.TextureSetSpec(64, 64, 4, 1, 2, 8, seed=0).geometry()
-    decode = binding.fill_params(geo, 0x1000, 0x2000, 0x3000, 0x4000, binding.WEIGHTS_INT8)
-    params = binding.SampleParams()
-    params.latents, params.network, params.queries, params.out, params.status = 0x1000, 0x2000, 0x5000, 0x3000, 0x4000
-    params.numQueries, params.numMips, params.numFeatures, params.channels = 16, decode.numMips, 8, 4
-    params.weightMode, params.numerics = binding.WEIGHTS_INT8, binding.NUMERICS_REFERENCE
-    for i in range(decode.numMips):
-        params.mips[i] = decode.mips[i]
-    params.latentLayout = 2
-    assert lib.ntcb_sample(ctypes.byref(params), None) == -1
-    assert b"latent layout" in lib.ntcb_last_error()
-    params.latentLayout = binding.LATENTS_INTERLEAVED
-    params.latents = 0x1004
-    assert lib.ntcb_sample(ctypes.byref(params), None) == -1
-    assert b"8-byte aligned" in lib.ntcb_last_error()
-    # ntcb_interleave_latents: NULL, aliased or misaligned buffers, bad counts, a grid larger than its plane,
-    # an offset that is not a multiple of the layer count
-    mips = decode.mips
-    assert lib.ntcb_interleave_latents(None, ctypes.c_void_p(0x1000), mips, 1, 8, None) == -1
-    assert lib.ntcb_interleave_latents(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x1000), mips, 1, 8, None) == -1
-    assert lib.ntcb_interleave_latents(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x9004), mips, 1, 8, None) == -1
-    assert lib.ntcb_interleave_latents(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x9000), mips, 0, 8, None) == -1
-    assert lib.ntcb_interleave_latents(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x9000), mips, 1, 6, None) == -1
-    broken = (binding.MipDesc * 1)(decode.mips[0])
-    broken[0].hiPlane = 1
-    assert lib.ntcb_interleave_latents(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x9000), broken, 1, 8, None) == -1
-    assert b"between its layers" in lib.ntcb_last_error()
-    broken = (binding.MipDesc * 1)(decode.mips[0])
-    broken[0].loOffset = decode.mips[0].loOffset + 1
-    assert lib.ntcb_interleave_latents(ctypes.c_void_p(0x1000), ctypes.c_void_p(0x9000), broken, 1, 8, None) == -1
-    assert b"multiple of the layer count" in lib.ntcb_last_error()
-
-
-def test_misaligned_and_oversized_requests_are_refused_on_the_host():
-    """Requests that would make a kernel issue a misaligned vector access, or overflow its 32-bit
-    element index, are refused before anything is launched (the addresses here are never touched)."""
-    import torch
-
-    gpu_present = torch.cuda.is_available()
-    lib = binding.lib()
-    geo = synthetic.TextureSetSpec(64, 64, 4, 1, 2, 8, seed=0).geometry()
-    # converting epilogue: a pixel of 16 (8) bytes is stored as one 16-byte (8-byte) vector
-    for channel_format, components, misaligned, aligned in (
-            (binding.CHANNEL_FORMAT_FLOAT32, 4, 0x3004, 0x3010), (binding.CHANNEL_FORMAT_FLOAT16, 8, 0x3008, 0x3020),
-            (binding.CHANNEL_FORMAT_FLOAT16, 4, 0x3004, 0x3008), (binding.CHANNEL_FORMAT_UNORM8, 16, 0x3004, 0x3030)):
-        conversion = binding.make_conversion(channel_format, 4, components=components)
-        params = binding.fill_params(geo, 0x1000, 0x2000, misaligned, 0x4000, binding.WEIGHTS_INT8, conversion=conversion)
-        assert lib.ntcb_decode(ctypes.byref(params), None) == -1
-        assert b"multiple of" in lib.ntcb_last_error()
-        if not gpu_present:
-            # the aligned request passes the argument checks and fails only for want of a GPU (never tried
-            # where a GPU is present: the addresses are made up)
-            params = binding.fill_params(geo, 0x1000, 0x2000, aligned, 0x4000, binding.WEIGHTS_INT8, conversion=conversion)
-            assert lib.ntcb_decode(ctypes.byref(params), None) == -2
-    # a mip of 2^32 values or more
-    params = binding.fill_params(geo, 0x1000, 0x2000, 0x3000, 0x4000, binding.WEIGHTS_INT8)
-    params.mips[0].width, params.mips[0].height, params.mips[0].rowEnd = 65536, 16384, 16384
-    assert lib.ntcb_decode(ctypes.byref(params), None) == -9
-    # ntcb_convert_channels and the allocation-free read take channel pairs as 32-bit words
-    convert = binding.ConvertParams()
-    convert.deviceMip, convert.layout, convert.width, convert.height, convert.channels = 0x5002, binding.LAYOUT_INTERLEAVED, 8, 8, 4
-    convert.deviceDestination, convert.pixelStride, convert.rowPitch = 0x6000, 8, 64
-    convert.conversion = binding.make_conversion(binding.CHANNEL_FORMAT_FLOAT16, 4)
-    assert lib.ntcb_convert_channels(ctypes.byref(convert), None) == -1
-    host = np.zeros(8 * 8 * 4, dtype=np.float16)
-    assert lib.ntcb_read_channels_to_host_noalloc(0x5002, binding.LAYOUT_INTERLEAVED, 8, 8, 4, 0, 4, host.ctypes.data, 8, 64, None) == -1
-
-
-def test_no_cpu_fallback():
-    """Without a usable GPU the compute entry points fail with a CUDA error instead of computing
-    on the host."""
-    import torch
-
-    if torch.cuda.is_available():
-        pytest.skip("a GPU is present")
-    lib = binding.lib()
-    handle = ctypes.c_void_p()
-    assert lib.ntcb_context_create(0, ctypes.byref(handle)) == -2
-    geo = synthetic.TextureSetSpec(64, 64, 4, 1, 2, 8, seed=0).geometry()
-    params = binding.fill_params(geo, 0x1000, 0x2000, 0x3000, 0x4000, binding.WEIGHTS_INT8)
-    assert lib.ntcb_decode(ctypes.byref(params), None) == -2
-
-
-TEXTURES = [
-    {"name": "Albedo", "firstChannel": 0, "numChannels": 3, "channelFormat": "UNORM8", "rgbColorSpace": "sRGB", "bcFormat": "BC1"},
-    {"name": "Normal", "firstChannel": 3, "numChannels": 2, "bcFormat": "BC5"},
-    {"name": "Emissive HDR with a rather long name " + "x" * 120, "firstChannel": 5, "numChannels": 1,
-     "channelFormat": "FLOAT16", "rgbColorSpace": "HLG", "alphaColorSpace": "Linear", "bcFormat": "BC6"},
-]
-
-
-def _set_with_textures(textures=TEXTURES):
-    data = synthetic.make_texture_set(synthetic.TextureSetSpec(64, 64, 6, 0, 2, 8, seed=3))
-    data.textures = textures
-    return data
-
-
-def test_texture_headers_are_read_with_the_reference_defaults():
-    """ITextureSetMetadata::GetTexture: name, channel range and intended formats; a field the file
-    leaves out takes the default the reference's loader gives it (UNORM8, Linear, no block format)."""
-    textures = binding.probe_textures(_set_with_textures().container)
-    assert [t["name"] for t in textures[:2]] == ["Albedo", "Normal"]
-    assert textures[2]["name"] == TEXTURES[2]["name"][:127]  # the C structure holds 127 characters
-    assert [(t["firstChannel"], t["numChannels"]) for t in textures] == [(0, 3), (3, 2), (5, 1)]
-    assert [t["channelFormat"] for t in textures] == [1, 1, 3]
-    assert [t["blockCompressedFormat"] for t in textures] == [1, 5, 6]
-    assert [(t["rgbColorSpace"], t["alphaColorSpace"]) for t in textures] == [(1, 0), (0, 0), (2, 0)]
-    assert binding.probe_textures(synthetic.make_texture_set(synthetic.TextureSetSpec(64, 64, 4, 0, 2, 8, seed=3)).container) == []
-
-
-def test_texture_header_errors():
-    lib = binding.lib()
-    for bad in ([{"name": "A", "firstChannel": 0, "numChannels": 3, "bcFormat": "BC9"}],
-                [{"firstChannel": 0, "numChannels": 3}],
-                [{"name": "A", "numChannels": 3}],
-                ["Albedo"]):
-        container = _set_with_textures(bad).container
-        buffer = np.frombuffer(container, dtype=np.uint8)
-        assert lib.ntcb_probe_container_texture(buffer.ctypes.data, len(container), 0, None, None) == -3, bad
-    container = _set_with_textures().container
-    buffer = np.frombuffer(container, dtype=np.uint8)
-    desc = binding.TextureDesc()
-    assert lib.ntcb_probe_container_texture(buffer.ctypes.data, len(container), 3, ctypes.byref(desc), None) == -9
-
-
-def test_reference_loader_accepts_the_texture_headers(oracle):
-    if not oracle.reference_available():
-        pytest.skip("oracle/_ref/libntc_ref.so is not built")
-    probed = oracle.reference_probe(_set_with_textures().container)
-    assert probed[:6] == [64, 64, 6, 7, 2, 8]
-    assert probed[7] == 0b111111  # the reference's valid-channel mask: the channels the textures cover
-
-
-def test_rounding_to_the_activation_grid_as_a_subnormal_number():
-    """The reference-numerics kernels round p = y * 80 to an integer as a multiple of 2^-24, the subnormal binary16 numbers: for every
-    activation input the product with the grid's step is the number that rint and a product give."""
-    def half(values):
-        return values.astype(np.float16)  # (round to nearest even; a binary64 holds every sum and product here exactly)
-
-    x = np.arange(65536, dtype=np.uint16).view(np.float16)
-    x = x[np.isfinite(x)].astype(np.float64)
-    third, step = float(np.float16(1 / 3)), float(np.float16(np.float32(3.1875) / np.float32(255)))
-    t = half(np.clip(x * third + 0.5, 0, 1)).astype(np.float64)
-    y = half(np.minimum(x, 3) * t).astype(np.float64)
-    p = half(y * 80).astype(np.float64)
-    code = half(p * 2.0 ** -24 + 2.0 ** -20).view(np.uint16)
-    assert code.min() >= 1 and code.max() <= 256
-    assert float(np.float16(step * 2 ** 22)) == step * 2 ** 22 and float(np.float16(16 * step)) == 16 * step
-    scaled = (code << 2).view(np.float16).astype(np.float64)
-    assert np.array_equal(half(scaled * (step * 2 ** 22) - 16 * step), half(np.rint(p) * step))
-
-
-def _build_cpp(tmp_path, name):
-    import os
-    import subprocess
-
-    from conftest import ROOT
-
-    binary = str(tmp_path / name)
-    subprocess.run(["g++", "-std=c++17", "-O2", "-march=x86-64-v3", "-ffp-contract=off", os.path.join(ROOT, "tests", "cpp", name + ".cpp"),
-                    "-o", binary], check=True)
-    return lambda lines: subprocess.run([binary], input="".join(line + "\n" for line in lines), stdout=subprocess.PIPE, text=True, check=True).stdout
-
-
-def test_no_run_of_tiles_reads_more_latent_pixels_than_its_buffer_is_checked_for(tmp_path):
-    """The footprint bound that decides whether a mip's latents are staged in shared memory, against the kernels' binary32 taps, at every run of mips
-    of texture sets up to 131072 wide: among them widths where rounding makes a footprint a column wider than its real extent."""
-    import os
-    import subprocess
-
-    from conftest import ROOT
-
-    binary = str(tmp_path / "footprint_bound")
-    subprocess.run(["g++", "-std=c++17", "-O2", "-march=x86-64-v3", "-ffp-contract=off", os.path.join(ROOT, "tests", "cpp", "footprint_bound.cpp"),
-                    "-o", binary], check=True)
-    rng = np.random.default_rng(11)
     widths = {47906, 109460, 109889, 131027, 131068, 131072, 8192, 4097} | {int(2.0 ** x) for x in rng.uniform(0, 17, 400)}
     pairs = {(4, 4 << 17), (1 << 23, 1 << 22), ((1 << 23) + 12345, (1 << 22) - 77)}  # a grid finer than its mip; sizes that binary32 rounds
     for width in widths:
