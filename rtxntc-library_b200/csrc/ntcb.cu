@@ -149,7 +149,8 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, FootprintBuf
 // Longest run of tiles for a launch of `tiles` tiles on `chains` chains.  A run of r tiles costs a chain 0.36 / r of a tile for tables and
 // footprints (FP8 weights; 0.2 with Int8), and the launch about r tiles at its end, when chains run out of work: four pay from 32 tiles a chain,
 // two from 8.  (4096 x 4096 FP8, 148 tiles a chain, runs of 1, 2 and 4: 717, 673 and 655 us; 1500 x 1100, 15 tiles: 86.9, 80.2 and 83.1;
-// 1024 x 512, 5 tiles: 30.1, 30.9 and 33.0.)
+// 1024 x 512, 5 tiles: 30.1, 30.9 and 33.0.  Exact accumulation, Int8 and 12 features, alike: 4096 x 4096 1223, 1192 and 1164, 1500 x 1100 136, 130
+// and 139, 1024 x 512 44.8, 46.3 and 51.0.)
 int LongestRun(long long tiles, long long chains)
 {
     return tiles >= 32 * chains ? kMaxRunTiles : tiles >= 8 * chains ? 2 : 1;
@@ -623,7 +624,9 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
             allTiles += ((long long)m.width + kChainTileWidth - 1) / kChainTileWidth *
                         (((long long)m.rowEnd - m.rowBegin + kChainTileHeight - 1) / kChainTileHeight);
     }
-    const int longestRun = LongestRun(allTiles, kMaxChains * 148); // a B200's 148 SMs
+    int resident = 1;
+    const bool deviceKnown = ResidentCtas(&resident) == NTCB_OK; // (its error is reported once the arguments are known to be valid)
+    const int longestRun = LongestRun(allTiles, (long long)kMaxChains * resident);
     long long tiles = 0;
     int used = 0;
     for (int i = 0; i < p->numMips; ++i)
@@ -700,10 +703,12 @@ int ntcb_decode(const NtcbDecodeParams* p, void* stream)
     }
     k.loadWaitPolls = g_networkWaitPolls.load(std::memory_order_relaxed);
 
-    int resident = 0;
-    int rc = ResidentCtas(&resident);
-    if (rc != NTCB_OK)
-        return rc;
+    if (!deviceKnown)
+    {
+        const int rc = ResidentCtas(&resident);
+        if (rc != NTCB_OK)
+            return rc;
+    }
     const int ctas = k.totalTiles < resident ? k.totalTiles : resident;
     cudaError_t err = reference ? LaunchDecodeRef(k, fp8, ctas, static_cast<cudaStream_t>(stream)) : LaunchDecode(k, fp8, ctas, static_cast<cudaStream_t>(stream));
     if (err != cudaSuccess)
