@@ -53,7 +53,7 @@ __device__ __forceinline__ uint32_t QuantizeInputPair(__half2 x)
     }
 }
 
-// Four network inputs -> four operand bytes.  (Not for constants: see E4m3Codes.)
+// Four network inputs -> four operand bytes.  (Not the same pair twice: see E4m3Codes.)
 template <bool kFp8>
 __device__ __forceinline__ uint32_t QuantizeInputs(__half2 first, __half2 second)
 {
@@ -391,7 +391,7 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
     {
         EncodePositions<Tile>(mip, tileX0, tileY0, columns, lane, warp, [&](const __half2 (&waves)[3], bool rows, int index) {
             const uint2 enc = make_uint2(QuantizeInputs<kFp8>(waves[0], waves[1]),
-                                         kFp8 ? QuantizeInputPair<kFp8>(waves[2]) : QuantizeInputs<kFp8>(waves[2], waves[2]));
+                                         kFp8 ? QuantizeInputPair<true>(waves[2]) : QuantizeInputs<false>(waves[2], waves[2]));
             if (!rows)
                 stage.tables.colEnc[index] = enc;
             else if (index < Tile::kHeight)

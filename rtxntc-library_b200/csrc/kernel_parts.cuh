@@ -221,7 +221,10 @@ __device__ __forceinline__ __half2 ClampedHgelu(__half2 x)
 // Two pairs of values -> four e4m3 codes (round to nearest even, saturating).  The conversions fill the two halves of one register, which
 // leaves nothing to extend or to join (with 16-bit results widened and joined by a multiply-add a texel of an FP8 network took 987
 // instructions instead of 891: 4096 x 4096 779 -> 719 us, 16.7 M queries 692 -> 648).
-// Not for constants: of E4m3Codes(0, 0) nvcc 12.9 left part of the word undefined.
+// No value may be converted twice where the compiler can see that it is the same, in the other half or in another word: ptxas 12.9 then shares one
+// conversion between them and leaves bytes undefined - for E4m3Codes(x, x), also of constants, and E4m3Codes(x, y) beside E4m3Codes(y, x); without
+// optimisation all are right.  (Joining 16-bit results by a shift, a permutation or a multiply-add has no such fault.)  The callers convert
+// accumulators, blended features and encoded positions, once each.
 __device__ __forceinline__ uint32_t E4m3Codes(__half2 first, __half2 second)
 {
     uint32_t codes;

@@ -1,6 +1,7 @@
 """Rules of the kernel sources that no run can show (a violation would hang a GPU, or show only under a rare schedule)."""
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -34,3 +35,41 @@ def test_dependent_launches_are_released_after_the_tensor_memory_is_held(kernels
 def test_every_set_up_of_a_decode_kernel_releases_its_dependents():
     assert sorted(file for file, _ in _functions_calling("GridDependencyLaunch")) == \
         ["decode_kernel.cu", "decode_kernel_ref.cu", "decode_kernel_ref.cu"]
+
+
+def test_no_value_is_converted_to_e4m3_twice():
+    """E4m3Codes is wrong where both operands are visibly the same value (kernel_parts.cuh): its callers pass two different expressions, no literals."""
+    calls = 0
+    for file in sorted(os.listdir(CSRC)):
+        if not file.endswith((".cu", ".cuh")):
+            continue
+        with open(os.path.join(CSRC, file)) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for call in re.finditer(r"\b(?:E4m3Codes|ActivateToE4m3|PackCodes<\w+>|QuantizeInputs<(?!false)\w+>)\(", text):
+            arguments, depth, end = [""], 1, call.end()
+            while depth:
+                character = text[end]
+                depth += {"(": 1, "[": 1, ")": -1, "]": -1}.get(character, 0)
+                if character == "," and depth == 1:
+                    arguments.append("")
+                elif depth:
+                    arguments[-1] += character
+                end += 1
+            first, second = (argument.strip() for argument in arguments)
+            if re.match(r"(?:__half2|uint32_t) \w+$", first):
+                continue  # its definition
+            calls += 1
+            assert first != second, (file, first)
+            for argument in (first, second):
+                assert not re.match(r"(?:__float2half2_rn\(|AsHalf2\()?[-\d]", argument), (file, argument)
+    assert calls >= 15
+
+
+@pytest.mark.gpu
+def test_e4m3_codes_of_every_binary16_number(tmp_path):
+    """tests/cpp/e4m3_codes.cu: every number in each of the four places of a word, against single conversions."""
+    binary = str(tmp_path / "e4m3_codes")
+    subprocess.run([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-I", CSRC,
+                    "-I", os.path.join(ROOT, "include"), os.path.join(ROOT, "tests", "cpp", "e4m3_codes.cu"), "-o", binary], check=True)
+    result = subprocess.run([binary], stdout=subprocess.PIPE, text=True)
+    assert result.returncode == 0, result.stdout
