@@ -393,11 +393,14 @@ def test_large_sets_decode_in_row_bands_with_pipelined_readback():
             texture_set.close()
 
 
-@pytest.mark.parametrize("width,height,mips,scale,features", [(1024, 1024, 0, 1, 8), (1000, 1531, 1, 1, 12), (2048, 512, 3, 1, 16)])
-def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, mips, scale, features):
+@pytest.mark.parametrize("width,height,mips,scale,features,numerics", [
+    (1024, 1024, 0, 1, 8, REFERENCE), (1000, 1531, 1, 1, 12, REFERENCE), (2048, 512, 3, 1, 16, REFERENCE), (1999, 2013, 2, 3, 16, REFERENCE),
+    (2003, 3601, 1, 4, 16, REFERENCE), (1999, 2013, 0, 3, 16, EXACT), (1200, 6007, 1, 4, 16, EXACT)])
+def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, mips, scale, features, numerics):
     """Latents of 4 MiB and more are uploaded in parts while the first rows of mip 0 are already being decoded: the same bits
     as a decode of resident latents, for texels read by the host, converted pixels on the device, and again after another
-    set of the same shape was loaded."""
+    set of the same shape was loaded.  Grids at a third and a quarter of the mip and heights that no tile divides among them: what the first rows
+    read of two neural mips differs with both."""
     import torch
 
     first, second = (synthetic.make_texture_set(synthetic.TextureSetSpec(width, height, 4, mips, scale, features, seed=seed, network="unit"))
@@ -405,10 +408,10 @@ def test_uploads_streamed_beside_the_decode_give_the_same_texels(width, height, 
     assert first.geometry.encoded_latent_bytes >= 4 << 20
     conversion = binding.make_conversion(binding.CHANNEL_FORMAT_UNORM8, 4)
     with binding.Context(0) as context:
-        texture_set = context.create_texture_set(first.container)
+        texture_set = context.create_texture_set(first.container, numerics=numerics)
         for data in (first, second, first):
             texture_set.load_from_memory(data.container)
-            resident = binding.ResidentTextureSet.from_synthetic(data)
+            resident = binding.ResidentTextureSet.from_synthetic(data, numerics=numerics)
             resident.decode(True)
             expected_pixels = resident.decode_converted(True, conversion)
             _sync()
