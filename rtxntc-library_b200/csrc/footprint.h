@@ -35,10 +35,10 @@ constexpr FootprintBuffers kExactFootprint{4800, 1808};
 // 23953-wide mip over a grid of 7984 was 7 columns where some tiles have 8: their last pixels were staged past the buffer.)
 constexpr long long FootprintPixels(int grid, int extent, int span)
 {
-    const long long units = grid > (1 << 22) || extent > (1 << 22) ? 20 : 10; // both positions, in 2^-24 of the grid
-    // (span + extent * units / 2^24) * grid / extent
-    const long long slack = (long long)extent * units;
-    return (long long)((__int128)grid * (((long long)span << 24) + slack) / ((long long)extent << 24)) + 3;
+    // (span + extent * units / 2^24) * grid / extent, where `units` is what both positions may be off, in 2^-24 of the grid
+    if (grid <= (1 << 22) && extent <= (1 << 22))
+        return (long long)grid * (((long long)span << 24) + (long long)extent * 10) / ((long long)extent << 24) + 3; // (below 2^53)
+    return (long long)((__int128)grid * (((long long)span << 24) + (long long)extent * 20) / ((long long)extent << 24)) + 3;
 }
 
 // Tiles side by side, a power of two up to `most`, whose footprints in both grids fit the buffers; 0: not even those of one do, and texels read their
