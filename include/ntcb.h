@@ -662,14 +662,15 @@ void ntcb_batch_decoder_destroy(NtcbBatchDecoder* decoder);
 int ntcb_read_channels_to_host_noalloc(const void* deviceMip, int layout, int width, int height, int channels,
     int firstChannel, int numChannels, void* hostDestination, size_t pixelStride, size_t rowPitch, void* stream);
 
-/* Number of CTAs the decode kernel keeps resident on the current device for a weight mode (the
-   grid size of large launches): SM count x resident CTAs per SM, the latter bounded by registers,
-   shared memory and tensor-memory columns.  For benchmarks and tests. */
+/* Number of CTAs the decode kernels keep resident on the current device (the grid size of large
+   launches): one per SM, whose chains fill its tensor memory and registers, with either weights (weightMode
+   only has to be a valid one).  For benchmarks and tests. */
 int ntcb_decode_resident_ctas(int weightMode, int* outCtas);
 
 /* Test hook for the kernels' timeout path (no counterpart in the reference).  Every wait inside the
    kernels is bounded; a CTA whose wait runs out records it in the status words (word 0 =
-   1, word 1 = tile, word 2 = layer; 0xFFFFFFFF in both for the wait described here), lets the work it has in
+   1, word 1 = the number of the run of tiles within a decode launch, or of the 128 queries within a sample
+   launch, word 2 = layer; 0xFFFFFFFF in both for the wait described here), lets the work it has in
    flight finish, releases its tensor memory and exits, and the host reports NTCB_ERR_DEVICE_TIMEOUT.
    This call sets, for every later launch of the process, how many polls a CTA spends on its FIRST
    wait - for the network image its bulk copy brings into shared memory, before any tile is touched

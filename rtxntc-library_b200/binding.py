@@ -631,7 +631,7 @@ class ResidentTextureSet:
     def check_status(self) -> None:
         words = self.status.cpu().numpy()
         if words[0] != 0:
-            raise NtcbError(-7, "a bounded wait in the decode kernel expired (tile %d, layer %d)" % (words[1], words[2]))
+            raise NtcbError(-7, "a bounded wait in a kernel expired (run of tiles or 128 queries number %d, layer %d)" % (words[1], words[2]))
 
     def mip_view(self, mip: int):
         """The decoded fp16 texels of one mip as a tensor: [H][W][C] (interleaved layout) or

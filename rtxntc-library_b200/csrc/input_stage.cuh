@@ -1,8 +1,6 @@
-// Input stage of the decode kernels whose A operand holds 8-bit codes (int8 or e4m3): per-tile
-// lookup tables, staging of the latent footprint, the bilinear gather, and the thread's 64-byte row
-// of the A operand.  `Shared` is the kernel's shared-memory structure (members tables,
-// footprintHi, footprintLo), `Context` its per-thread tile context (members x, y,
-// rowChunk).
+// Input stage of the decode kernels: lookup tables of a run of tiles, staging of its latent footprint, and, for the
+// kernels whose A operand holds 8-bit codes (int8 or e4m3), the bilinear gather and the thread's 64-byte row of it.  `Stage` is what a chain
+// prepares per run (ChainStage: members tables, footprintHi, footprintLo), `Context` what a thread knows of its texel (members x, y, rowChunk).
 #pragma once
 
 #include <cuda_fp16.h>

@@ -366,8 +366,8 @@ def test_texture_set_api_decompress_and_read_channels(oracle):
 
 
 def test_large_sets_decode_in_row_bands_with_pipelined_readback():
-    """A set whose mip 0 has 512 rows or more is decoded by the texture-set API in four row-band
-    launches plus one for the other mips, and a host read of mip 0 copies band by band: same bits
+    """A set whose mip 0 has 512 rows or more is decoded by the texture-set API in two launches, the first rows of mip 0
+    and everything else, and a host read of mip 0 copies band by band: same bits
     as the single launch, for fp16 and for converted pixels, in both numerics."""
     data = synthetic.make_texture_set(synthetic.TextureSetSpec(200, 530, 6, 0, 2, 8, seed=12, network="unit"))
     geo = data.geometry
