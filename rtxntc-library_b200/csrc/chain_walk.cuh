@@ -145,8 +145,8 @@ struct ChainContext
 };
 
 // The 64-byte operand row of a texel: 48 inputs as codes, then K padding - zeros (e4m3) or the constant inputs of the bias slots (int8).
-// `column`: in the run.  `known`: TexelTables, and the row's last two chunks where the layers after the first leave them alone (FP8: their operands are
-// in tensor memory), are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
+// `column`: in the run.  `known`: TexelTables and the row's last two chunks, which the layers after the first leave alone (their operands are in tensor
+// memory), are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
 template <bool kFp8, bool kReferenceDivision, int kLayers, typename Stage>
 __device__ __forceinline__ void BuildCodes(const KernelParams& params, const KernelMip& mip, Stage& stage, const ChainContext& ctx,
     int column, int tileRow, bool known, int2 shift)
@@ -159,7 +159,7 @@ __device__ __forceinline__ void BuildCodes(const KernelParams& params, const Ker
     const int texel = ctx.tid & 127;
     if (!known)
         PrepareTexel(stage, texel, column, tileRow);
-    if (!known || !kFp8)
+    if (!known)
     {
         // positional encoding: interleave the column's x bytes with the row's y bytes
         const uint2 cx = stage.tables.colEnc[column];

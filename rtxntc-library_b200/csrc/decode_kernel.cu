@@ -14,8 +14,7 @@
 //      instruction) against the weights resident in shared memory; accumulators live in TMEM;
 //   3. after the commit arrives on the chain's mbarrier every thread pulls its row of accumulators with
 //      tcgen05.ld, applies bias/scale and the clamped HGELU in packed binary16, re-quantises and
-//      writes the next layer's A operand over the previous one - with FP8 weights into tensor memory
-//      (tcgen05.st; the next product takes A from there), with Int8 weights into shared memory;
+//      writes the next layer's A operand into tensor memory (tcgen05.st; the next product takes A from there);
 //   4. after the fourth layer the epilogue scales, converts to fp16 and stores.
 //
 // Arithmetic contract (what the CPU checker restates): everything outside the matrix products is
@@ -111,16 +110,17 @@ __device__ __forceinline__ void UmmaFromTmem(uint32_t tmemD, uint32_t tmemA, uin
     }
 }
 
-// FP8 networks keep the A operands of layers 1-3 in tensor memory: the activation codes of a row (at most
+// The A operands of layers 1-3 are in tensor memory: the activation codes of a row (at most
 // 64 bytes) go to columns [0,16) of the row's lane, and the accumulators of those layers start at column
 // 16 (48 + 16 = 64 columns per chain).  Layer 0 reads its operand from shared memory and accumulates into
 // columns [0,64); its consumer has loaded columns [0,32) before it stores the first codes to [0,8), and
-// [32,64) before it stores to [8,16).  Int8 networks have the bias K step's operand in shared memory
-// and 65 - 80 operand bytes per row: they keep every operand there.
-template <bool kFp8, int kLayer>
-constexpr bool kOperandInTmem = kFp8 && kLayer >= 1;
-template <bool kFp8, int kLayer>
-constexpr uint32_t kAccumulatorColumn = kOperandInTmem<kFp8, kLayer> ? 16u : 0u;
+// [32,64) before it stores to [8,16).  Of an Int8 network's operands only that of the bias K step, the same for every row, is in shared memory.
+// (With all of an Int8 network's operands there, every layer had its stores and proxy fence, the tensor core its reads, and the last chunks of the input rows had to
+// be written again for every tile: 1920 x 1080, 8 features, 158 us instead of 146; 2048 x 2048, 12 features, 308 instead of 274.)
+template <int kLayer>
+constexpr bool kOperandInTmem = kLayer >= 1;
+template <int kLayer>
+constexpr uint32_t kAccumulatorColumn = kOperandInTmem<kLayer> ? 16u : 0u;
 
 // Instruction descriptor: dense, K-major A and B, M = 128.
 __host__ __device__ constexpr uint32_t MakeInstrDescriptor(bool fp8, int n)
@@ -167,7 +167,7 @@ struct __align__(128) ExactStorage
     uint32_t claims;              // inference on sample: query tiles handed out so far
     uint32_t claimed[kMaxChains]; // ... per chain the number of the tile it takes after the next (ClaimTile)
     uint32_t tmemBase;
-    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands, 64 bytes a row, in core-matrix order; then the ExactStages
+    alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row, in core-matrix order; then the ExactStages
 };
 using ExactStage = CodesStage<kExactFootprint.hiBytes, kExactFootprint.loBytes>;
 static_assert(sizeof(ExactStorage) + kMaxChains * sizeof(ExactStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
@@ -187,7 +187,7 @@ __device__ __forceinline__ int IssueLayer(ChainContext& ctx)
     // Makes the A operand written before this call visible to the tensor core, orders every
     // thread's TMEM reads of the previous layer before the accumulators are overwritten, and agrees
     // on whether any thread gave up waiting.
-    if (kOperandInTmem<kFp8, kLayer>)
+    if (kOperandInTmem<kLayer>)
         TmemStoreWait();
     else
         FenceProxyAsyncShared();
@@ -202,7 +202,7 @@ __device__ __forceinline__ int IssueLayer(ChainContext& ctx)
         const uint32_t elected = ElectOne();
         const uint32_t base = DynamicSharedBase();
         const int chain = ctx.warp >> 2;
-        const uint32_t accumulators = ctx.accumulators + kAccumulatorColumn<kFp8, kLayer>;
+        const uint32_t accumulators = ctx.accumulators + kAccumulatorColumn<kLayer>;
         const uint64_t operandBase =
             MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, operandA)) + uint32_t(chain) * uint32_t(kOperandBytes), 2048, 128);
         const uint64_t weightBase = MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, network)) + kWeightOffset, kN * 16, 128);
@@ -211,7 +211,7 @@ __device__ __forceinline__ int IssueLayer(ChainContext& ctx)
         {
             // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
             const uint64_t descB = weightBase + uint64_t((kStep * 2 * kN * 16) >> 4);
-            if (kOperandInTmem<kFp8, kLayer>)
+            if (kOperandInTmem<kLayer>)
                 UmmaFromTmem<kLayerFp8>(accumulators, ctx.accumulators + kStep * 8, descB, instr, kStep != 0, elected);
             else
                 Umma<kLayerFp8>(accumulators, operandBase + uint64_t((kStep * 2 * 2048) >> 4), descB, instr, kStep != 0, elected);
@@ -249,7 +249,6 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Exa
     if (kLayer < 3)
     {
         constexpr bool kNextFp8 = kFp8 && kLayer < 2; // layer 2 always re-quantises to int8
-        uint4* rowChunk = ctx.rowChunk;
         // 32 accumulator columns at a time keeps the register footprint small
 #pragma unroll
         for (int part = 0; part < (kN + 31) / 32; ++part)
@@ -260,7 +259,7 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Exa
 #pragma unroll
             for (int c = 0; c < 2; ++c)
                 if (firstChunk + c < kChunksTotal)
-                    TmemLoad16(ctx.tmemLane + kAccumulatorColumn<kFp8, kLayer> + (firstChunk + c) * 16, acc[c]);
+                    TmemLoad16(ctx.tmemLane + kAccumulatorColumn<kLayer> + (firstChunk + c) * 16, acc[c]);
             TmemLoadWait();
 #pragma unroll
             for (int c = 0; c < 2; ++c)
@@ -290,28 +289,22 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Exa
                     const uint4 codes =
                         make_uint4(PackCodes<kNextFp8>(pairs[0], pairs[1]), PackCodes<kNextFp8>(pairs[2], pairs[3]),
                                    PackCodes<kNextFp8>(pairs[4], pairs[5]), PackCodes<kNextFp8>(pairs[6], pairs[7]));
-                    if (kFp8)
-                        TmemStore4(ctx.tmemLane + (firstChunk + c) * 4, codes.x, codes.y, codes.z, codes.w);
-                    else
-                        rowChunk[(firstChunk + c) * 128] = codes;
+                    TmemStore4(ctx.tmemLane + (firstChunk + c) * 4, codes.x, codes.y, codes.z, codes.w);
                 }
             }
         }
         if (kLayer == 1)
         {
             // layer 2 has 48 inputs, K is padded to 64: zeros (e4m3) or the bias slots' inputs (int8)
-            const uint32_t fill = kFp8 ? 0u : kBiasSlotValue * 0x01010101u;
-            if (kFp8)
-                TmemStore4(ctx.tmemLane + 12, 0u, 0u, 0u, 0u);
-            else
-                rowChunk[3 * 128] = make_uint4(fill, fill, fill, (fill & 0x00FFFFFFu) | 0x01000000u);
+            const uint4 padding = PaddingCodes<kFp8>();
+            TmemStore4(ctx.tmemLane + 12, padding.x, padding.y, padding.z, padding.w);
         }
     }
     else
     {
         // output epilogue (src/Inference.cu:121-135)
         uint32_t acc[16];
-        TmemLoad16(ctx.tmemLane + kAccumulatorColumn<kFp8, kLayer>, acc);
+        TmemLoad16(ctx.tmemLane + kAccumulatorColumn<kLayer>, acc);
         TmemLoadWait();
         const int channelPairs = channels >> 1;
         uint32_t bits[8];
