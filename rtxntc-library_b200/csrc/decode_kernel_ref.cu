@@ -129,6 +129,15 @@ __device__ __forceinline__ __half2 QuantizeInputRef(__half2 x)
     return __hmul2_rn(y, __float2half2_rn(1.f / 127.5f));
 }
 
+// The same for a pair of blended features (TwiceFeatureCodes): the product with the step as one multiply-add on code + 128 in the subnormal numbers.
+// The step has 9 significant bits, so 2^22 of them and 128 of them are binary16 numbers.
+__device__ __forceinline__ __half2 QuantizeFeatureRef(__half2 x)
+{
+    constexpr float kStep = 257.f / 32768.f; // 1 / 127.5 in binary16
+    const uint32_t code = ((TwiceFeatureCodes(x) & 0xFFFEFFFEu) << 1) + 0x00040004u; // 4 (code + 128)
+    return __hfma2(AsHalf2(code), __float2half2_rn(kStep * 4194304.f), __float2half2_rn(-128.f * kStep));
+}
+
 // Clamped HGELU followed by the quantiser of the next layer's inputs, the int8 grid rint(y * 80) * 0.0125
 // (src/tin/tin_activation.h:94-99).
 __device__ __forceinline__ uint32_t ActivateRef(uint32_t bits)
@@ -234,8 +243,8 @@ __device__ __forceinline__ void BlendLayerRef(uint2 l00, uint2 l01, uint2 l10, u
     b = __hfma2(AsHalf2(l11.y), w11, b);
     a = __hfma2(a, two, minusOne);
     b = __hfma2(b, two, minusOne);
-    words[0] = AsU32(QuantizeInputRef(a));
-    words[1] = AsU32(QuantizeInputRef(b));
+    words[0] = AsU32(QuantizeFeatureRef(a));
+    words[1] = AsU32(QuantizeFeatureRef(b));
 }
 
 // One latent layer of one grid (the low 16 bits of each p are the tap's four features) -> two pairs of inputs.
@@ -243,8 +252,8 @@ __device__ __forceinline__ void BlendPixelsRef(uint32_t p00, uint32_t p01, uint3
 {
     __half2 inputs[2];
     BlendPixels(p00, p01, p10, p11, taps, inputs);
-    words[0] = AsU32(QuantizeInputRef(inputs[0]));
-    words[1] = AsU32(QuantizeInputRef(inputs[1]));
+    words[0] = AsU32(QuantizeFeatureRef(inputs[0]));
+    words[1] = AsU32(QuantizeFeatureRef(inputs[1]));
 }
 
 // Two latent layers of one grid (a word of each tap) -> two pairs of inputs each.
@@ -255,7 +264,7 @@ __device__ __forceinline__ void BlendLayersRef(uint32_t p00, uint32_t p01, uint3
 #pragma unroll
     for (int j = 0; j < 2; ++j)
     {
-        const uint32_t even = AsU32(QuantizeInputRef(inputs[2 * j])), odd = AsU32(QuantizeInputRef(inputs[2 * j + 1]));
+        const uint32_t even = AsU32(QuantizeFeatureRef(inputs[2 * j])), odd = AsU32(QuantizeFeatureRef(inputs[2 * j + 1]));
         words[j] = __byte_perm(even, odd, 0x5410);
         words[2 + j] = __byte_perm(even, odd, 0x7632);
     }

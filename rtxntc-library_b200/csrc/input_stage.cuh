@@ -51,6 +51,35 @@ __device__ __forceinline__ uint32_t QuantizeInputPair(__half2 x)
     }
 }
 
+// The same int8 codes for a pair of blended features: 2 (code + 127), or 1 more, as an integer in either half.
+//
+// Taps lie in [0, 1], weights add up to 1 but for their rounding, so a blend is at most (1 + 2^-11)^5 and x lies in [-1, 1.005].  There
+// floor(x * 127.5 - 0.5), rounded to binary16 before the floor as the reference has it, is half of the integer nearest to 2 w + 254, w = x * 127.5 - 0.75
+// rounded to binary16: w is a quarter less, on the same grid of binary16 numbers, so twice the integer boundary is a tie, and ties go to the even
+// number above it.  The clamp to -127 is the clamp to 0 of the second operation, whose results are subnormal numbers, multiples of 2^-24; nothing gets to 128.
+// (All x a blend can have compared: tests/test_host_logic.py.)  Two packed operations instead of a multiply-add, two conversions on the quarter-rate
+// pipe and a clamp of two.
+__device__ __forceinline__ uint32_t TwiceFeatureCodes(__half2 x)
+{
+    const __half2 w = __hfma2(x, __float2half2_rn(127.5f), __float2half2_rn(-0.75f));
+    return AsU32(__hfma2_relu(w, __float2half2_rn(0x1p-23f), __float2half2_rn(254.f * 0x1p-24f)));
+}
+
+// Four bytes code + 127, 0 .. 254, to two's complement.
+__device__ __forceinline__ uint32_t FromExcess127(uint32_t codes)
+{
+    return (codes + 0x01010101u) ^ 0x80808080u;
+}
+
+// Two pairs of blended features -> four operand bytes.
+template <bool kFp8>
+__device__ __forceinline__ uint32_t QuantizeFeatures(__half2 first, __half2 second)
+{
+    if (kFp8)
+        return E4m3Codes(first, second);
+    return FromExcess127(__byte_perm(TwiceFeatureCodes(first) >> 1, TwiceFeatureCodes(second) >> 1, 0x6420));
+}
+
 // Four network inputs -> four operand bytes.  (Not the same pair twice: see E4m3Codes.)
 template <bool kFp8>
 __device__ __forceinline__ uint32_t QuantizeInputs(__half2 first, __half2 second)
@@ -126,7 +155,7 @@ __device__ __forceinline__ uint32_t BlendLayer(uint32_t p00, uint32_t p01, uint3
 {
     __half2 inputs[2];
     BlendPixels(p00, p01, p10, p11, taps, inputs);
-    return QuantizeInputs<kFp8>(inputs[0], inputs[1]);
+    return QuantizeFeatures<kFp8>(inputs[0], inputs[1]);
 }
 
 // Two layers of one grid -> four quantised inputs each.
@@ -138,12 +167,17 @@ __device__ __forceinline__ void BlendLayers(uint32_t p00, uint32_t p01, uint32_t
     uint32_t codes[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f)
-        codes[f] = QuantizeInputPair<kFp8>(inputs[f]);
+        codes[f] = kFp8 ? QuantizeInputPair<true>(inputs[f]) : TwiceFeatureCodes(inputs[f]) >> 1;
     // the first layer's codes of two features, then the second layer's (e4m3: bytes 0 and 1; int8: bytes 0 and 2)
     constexpr uint32_t kInterleave = kFp8 ? 0x5140u : 0x6240u;
     const uint32_t low = __byte_perm(codes[0], codes[1], kInterleave), high = __byte_perm(codes[2], codes[3], kInterleave);
     words[0] = __byte_perm(low, high, 0x5410);
     words[1] = __byte_perm(low, high, 0x7632);
+    if (!kFp8)
+    {
+        words[0] = FromExcess127(words[0]);
+        words[1] = FromExcess127(words[1]);
+    }
 }
 
 // ... with the taps read from one layer's plane in global memory.
@@ -428,7 +462,7 @@ __device__ __forceinline__ uint32_t BlendLayer(uint2 l00, uint2 l01, uint2 l10, 
     b = __hfma2(AsHalf2(l11.y), w11, b);
     a = __hfma2(a, two, minusOne);
     b = __hfma2(b, two, minusOne);
-    return QuantizeInputs<kFp8>(a, b);
+    return QuantizeFeatures<kFp8>(a, b);
 }
 
 // Inputs 0..31 of one texel with the taps read straight from global memory (`interleaved`: from the pixel-major

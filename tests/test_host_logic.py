@@ -531,6 +531,29 @@ def test_rounding_to_the_activation_grid_as_a_subnormal_number():
     assert np.array_equal(half(scaled * (step * 2 ** 22) - 16 * step), half(np.rint(p) * step))
 
 
+def test_int8_codes_of_blended_features():
+    """The int8 code of a blended feature, floor(x * 127.5 - 0.5) clamped to +-127, as half of an integer that one multiply-add rounds to, for every x
+    = 2 d - 1 that a blend d can give: weights that add up to 1, rounded, times taps of at most 1, through four rounded operations."""
+    def half(values):
+        return values.astype(np.float16)  # (round to nearest even; a binary64 holds every sum and product here exactly)
+
+    d = np.arange(65536, dtype=np.uint16).view(np.float16)
+    d = d[np.isfinite(d)].astype(np.float64)
+    d = d[(d >= 0) & (d <= (1 + 2.0 ** -11) ** 5)]
+    x = half(2 * d - 1).astype(np.float64)
+    code = np.clip(np.floor(half(x * 127.5 - 0.5)).astype(np.float64), -127, 127)
+    w = half(x * 127.5 - 0.75).astype(np.float64)
+    twice = np.maximum(half(w * 2.0 ** -23 + 254 * 2.0 ** -24), np.float16(0)).view(np.uint16)
+    assert np.array_equal((twice >> 1).astype(np.float64) - 127, code)
+    # the reference-numerics kernels: the product with the step, from 4 (code + 128) as a subnormal number
+    step = float(np.float16(1 / 127.5))
+    assert float(np.float16(step * 2 ** 22)) == step * 2 ** 22 and float(np.float16(128 * step)) == 128 * step
+    scaled = (((twice & 0xFFFE) << 1) + 4).astype(np.uint16).view(np.float16).astype(np.float64)
+    assert np.array_equal(half(scaled * (step * 2 ** 22) - 128 * step), half(code * step))
+    # the exact-accumulation kernels: the byte in two's complement
+    assert np.array_equal(((((twice >> 1) + 1) & 0xFF) ^ 0x80).astype(np.uint8).view(np.int8), code.astype(np.int8))
+
+
 def _build_cpp(tmp_path, name):
     import os
     import subprocess
