@@ -15,8 +15,7 @@ namespace ntcb
 
 constexpr int kOperandBytes = 128 * 64; // A operand of codes: 128 rows x 64 bytes
 constexpr int kTmemColumnsPerChain = 64;    // widest accumulator (layer 0: 64 outputs)
-constexpr uint32_t kSpinLimit = 1u << 20;  // mbarrier polls before a wait is declared expired (about two seconds)
-constexpr uint32_t kWaitHintNanoseconds = 2000; // how long one poll may suspend the thread
+constexpr uint32_t kSpinLimit = 1u << 20;  // mbarrier polls before a wait is declared expired (about one and a half seconds)
 
 // Image of the network in shared memory (produced on the host by ntcb_stage_network).
 // Weight matrix of layer l: N_l rows (outputs) x K_l bytes (inputs, padded to a multiple of 32) in

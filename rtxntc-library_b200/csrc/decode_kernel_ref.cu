@@ -888,8 +888,7 @@ __device__ __forceinline__ void ConsumeLayerRefFp8(const Params& params, const C
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
 
     // (Every warp polls the barrier itself.  Tried and dropped: one polling warp per chain with the other
-    // three blocked in a named barrier executes 1.5 % fewer instructions but wakes the chain later, 4.5 %
-    // slower; polls without a suspend-time hint, the same speed.)
+    // three blocked in a named barrier executes 1.5 % fewer instructions but wakes the chain later, 4.5 % slower.)
     if (!MbarrierWaitBounded(ctx.barrier, phase))
     {
         SetGiveUp(ctx.giveUp);

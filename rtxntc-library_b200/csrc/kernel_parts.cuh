@@ -36,20 +36,20 @@ __device__ __forceinline__ void FenceBarrierInit()
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// One poll of a barrier phase.  The instruction may suspend the thread until the phase completes
-// or `kWaitHintNanoseconds` have passed, whichever comes first (measured: the same speed as polls
-// without the hint).
+// One poll of a barrier phase.  The instruction may suspend the thread until the phase completes, and gives up by itself after 1.4 us.
+// (With a suspend-time hint a poll is three instructions, one of them a sleep: 4096 x 4096 FP8 647 us instead of 640, 2048 x 2048 of 8 features 163
+// instead of 153, 8192 x 8192 Int8 3612 instead of 3572, 16.7 M queries 643 instead of 634.)
 __device__ __forceinline__ bool MbarrierTryWait(uint32_t bar, uint32_t parity)
 {
     uint32_t done;
     asm volatile(
         "{\n\t"
         ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t"
         "}"
         : "=r"(done)
-        : "r"(bar), "r"(parity), "r"(kWaitHintNanoseconds)
+        : "r"(bar), "r"(parity)
         : "memory");
     return done != 0;
 }
