@@ -134,7 +134,7 @@ __device__ __forceinline__ __half2 QuantizeInputRef(__half2 x)
 __device__ __forceinline__ __half2 QuantizeFeatureRef(__half2 x)
 {
     constexpr float kStep = 257.f / 32768.f; // 1 / 127.5 in binary16
-    const uint32_t code = ((TwiceFeatureCodes(x) & 0xFFFEFFFEu) << 1) + 0x00040004u; // 4 (code + 128)
+    const uint32_t code = ((TwiceFeatureCodes(x) & 0x7FFE7FFEu) << 1) + 0x00040004u; // 4 (code + 128); a clamped zero may keep its sign
     return __hfma2(AsHalf2(code), __float2half2_rn(kStep * 4194304.f), __float2half2_rn(-128.f * kStep));
 }
 
