@@ -50,20 +50,24 @@ namespace
 // PTX wrappers
 // ---------------------------------------------------------------------------------------------
 
-// D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 bytes of 8-bit operands.
+// D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 bytes of 8-bit operands.  `lowA`, `lowB`: low words of the operands' descriptors, whose groups
+// of eight rows are 128 bytes apart.  Called by a converged warp, of which elect.sync picks the lane that issues, always the same.
 template <bool kFp8>
-__device__ __forceinline__ void Umma(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate, uint32_t enabled)
+__device__ __forceinline__ void Umma(uint32_t tmemD, uint32_t lowA, uint32_t lowB, uint32_t instr, uint32_t accumulate)
 {
     if (kFp8)
     {
         asm volatile(
             "{\n\t"
             ".reg .pred p, q;\n\t"
+            ".reg .b64 a, b;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "setp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+            "mov.b64 a, {%1, %5};\n\t"
+            "mov.b64 b, {%2, %6};\n\t"
+            "elect.sync _|q, 0xFFFFFFFF;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "l"(descA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+            "r"(lowA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(128)), "n"(DescriptorHigh(128))
             : "memory");
     }
     else
@@ -71,29 +75,34 @@ __device__ __forceinline__ void Umma(uint32_t tmemD, uint64_t descA, uint64_t de
         asm volatile(
             "{\n\t"
             ".reg .pred p, q;\n\t"
+            ".reg .b64 a, b;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "setp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
+            "mov.b64 a, {%1, %5};\n\t"
+            "mov.b64 b, {%2, %6};\n\t"
+            "elect.sync _|q, 0xFFFFFFFF;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "l"(descA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+            "r"(lowA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(128)), "n"(DescriptorHigh(128))
             : "memory");
     }
 }
 
 // The same with the A operand in tensor memory: 8 columns (32 bytes per lane) starting at `tmemA`.
 template <bool kFp8>
-__device__ __forceinline__ void UmmaFromTmem(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t instr, uint32_t accumulate, uint32_t enabled)
+__device__ __forceinline__ void UmmaFromTmem(uint32_t tmemD, uint32_t tmemA, uint32_t lowB, uint32_t instr, uint32_t accumulate)
 {
     if (kFp8)
     {
         asm volatile(
             "{\n\t"
             ".reg .pred p, q;\n\t"
+            ".reg .b64 b;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "setp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
+            "mov.b64 b, {%2, %5};\n\t"
+            "elect.sync _|q, 0xFFFFFFFF;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], b, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+            "r"(tmemA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(128))
             : "memory");
     }
     else
@@ -101,11 +110,13 @@ __device__ __forceinline__ void UmmaFromTmem(uint32_t tmemD, uint32_t tmemA, uin
         asm volatile(
             "{\n\t"
             ".reg .pred p, q;\n\t"
+            ".reg .b64 b;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "setp.ne.b32 q, %5, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t"
+            "mov.b64 b, {%2, %5};\n\t"
+            "elect.sync _|q, 0xFFFFFFFF;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], b, %3, p;\n\t"
             "}" ::"r"(tmemD),
-            "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+            "r"(tmemA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(128))
             : "memory");
     }
 }
@@ -198,29 +209,28 @@ __device__ __forceinline__ int IssueLayer(ChainContext& ctx)
     if (WarpRole(ctx.warp) == kIssuingRole)
     {
         TcgenFenceAfterSync();
+        // (In one branch on elect.sync, as the reference-numerics kernels have it, the Int8 kernels of 12 and 16 features spill more: 2048 x 2048, 12
+        // features, 270 us instead of 267, 16 features 285 instead of 279; FP8 is 0.5 % faster.  With a predicate made from one election: 275, 288.)
         constexpr uint32_t instr = MakeInstrDescriptor(kLayerFp8, kN);
-        const uint32_t elected = ElectOne();
-        const uint32_t base = DynamicSharedBase();
+        const uint32_t base = DescriptorAddress(DynamicSharedBase());
         const int chain = ctx.warp >> 2;
         const uint32_t accumulators = ctx.accumulators + kAccumulatorColumn<kLayer>;
-        const uint64_t operandBase =
-            MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, operandA)) + uint32_t(chain) * uint32_t(kOperandBytes), 2048, 128);
-        const uint64_t weightBase = MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, network)) + kWeightOffset, kN * 16, 128);
+        const uint32_t operand = base + uint32_t(chain) * uint32_t(kOperandBytes >> 4) + uint32_t(offsetof(ExactStorage, operandA) >> 4) + DescriptorLow(2048);
+        const uint32_t weights = base + uint32_t((offsetof(ExactStorage, network) + kWeightOffset) >> 4) + DescriptorLow(kN * 16);
 #pragma unroll
         for (int kStep = 0; kStep < kK / 32; ++kStep)
         {
             // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
-            const uint64_t descB = weightBase + uint64_t((kStep * 2 * kN * 16) >> 4);
+            const uint32_t stepWeights = weights + uint32_t((kStep * 2 * kN * 16) >> 4);
             if (kOperandInTmem<kLayer>)
-                UmmaFromTmem<kLayerFp8>(accumulators, ctx.accumulators + kStep * 8, descB, instr, kStep != 0, elected);
+                UmmaFromTmem<kLayerFp8>(accumulators, ctx.accumulators + kStep * 8, stepWeights, instr, kStep != 0);
             else
-                Umma<kLayerFp8>(accumulators, operandBase + uint64_t((kStep * 2 * 2048) >> 4), descB, instr, kStep != 0, elected);
+                Umma<kLayerFp8>(accumulators, operand + uint32_t((kStep * 2 * 2048) >> 4), stepWeights, instr, kStep != 0);
         }
         if (kBiasStep)
-            Umma<kLayerFp8>(accumulators, MakeSmemDescriptor(base + uint32_t(offsetof(ExactStorage, biasRegion)), 2048, 128),
-                weightBase + uint64_t(((kK / 32) * 2 * kN * 16) >> 4), instr, 1, elected);
-        if (elected)
-            UmmaCommit(base + uint32_t(offsetof(ExactStorage, barrier)) + chain * 8);
+            Umma<kLayerFp8>(accumulators, base + uint32_t(offsetof(ExactStorage, biasRegion) >> 4) + DescriptorLow(2048),
+                weights + uint32_t(((kK / 32) * 2 * kN * 16) >> 4), instr, 1);
+        UmmaCommitElected(ctx.barrier);
     }
     return 0;
 }

@@ -69,18 +69,21 @@ namespace
 // fence, and no operand reads from shared memory by the tensor core for three of the four layers (3 %).
 constexpr uint32_t kOperandColumn = 48;
 
-// D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 16 binary16 operands, binary16 accumulators.
-__device__ __forceinline__ void UmmaF16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
-    uint32_t enabled = 1)
+// D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 16 binary16 operands, binary16 accumulators.  `lowA`, `lowB`: low words of the operands'
+// descriptors; B's groups of eight rows are 128 bytes apart.  To be called by one elected thread.
+template <uint32_t kStrideA = 128>
+__device__ __forceinline__ void UmmaF16(uint32_t tmemD, uint32_t lowA, uint32_t lowB, uint32_t instr, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t"
-        ".reg .pred p, q;\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 a, b;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "mov.b64 a, {%1, %5};\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
         "}" ::"r"(tmemD),
-        "l"(descA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+        "r"(lowA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(kStrideA)), "n"(DescriptorHigh(128))
         : "memory");
 }
 
@@ -350,17 +353,17 @@ constexpr bool kRefOperandInTmem = kRefFirstTmemStep<kLayer> == 0;      // nothi
 template <int kLayer>
 constexpr bool kRefOperandInShared = kRefFirstTmemStep<kLayer> != 0;    // some of it in shared memory
 
-__device__ __forceinline__ void UmmaF16FromTmem(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t instr, uint32_t accumulate,
-    uint32_t enabled)
+__device__ __forceinline__ void UmmaF16FromTmem(uint32_t tmemD, uint32_t tmemA, uint32_t lowB, uint32_t instr, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t"
-        ".reg .pred p, q;\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 b;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+        "mov.b64 b, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t"
         "}" ::"r"(tmemD),
-        "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+        "r"(tmemA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(128))
         : "memory");
 }
 
@@ -385,41 +388,37 @@ __device__ __forceinline__ int IssueLayerRef(ChainContext& ctx)
     if (LayerBarrier<kLayer>(ctx.warp >> 2, ctx.giveUp))
         return 1;
 
-    // The whole issuing warp runs the descriptor arithmetic on values that are visibly the same in every
-    // lane; one elected lane hands the work to the tensor core (see IssueLayerRefFp8).
+    // One elected lane hands the work to the tensor core (see IssueLayerRefFp8).
     if (WarpRole(ctx.warp) == kIssuingRole)
     {
         TcgenFenceAfterSync();
-        constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
-        const uint32_t base = DynamicSharedBase(), networkBase = base + uint32_t(offsetof(RefSharedStorage, network));
-        // the four base descriptors are built once, every operand is then a constant offset (in 16-byte
-        // units) added to the address field
-        const uint64_t operandBase = MakeSmemDescriptor(base + uint32_t(offsetof(RefSharedStorage, operandA)), 2048, 128);
-        // rows e_kLayer (every 8-row group reads the same core matrix: stride 0), then the core matrix of zeros
-        const uint64_t onesBase = MakeSmemDescriptor(base + uint32_t(offsetof(RefSharedStorage, onesRegion)) + kLayer * 128, (4 - kLayer) * 128, 0);
-        const uint64_t weightBase = MakeSmemDescriptor(networkBase + kWeightOffset, kN * 16, 128);
-        // the matrix of biases, read twice (leading offset 0): its second copy meets the zeros
-        const uint64_t biasBase = MakeSmemDescriptor(networkBase + kRefInt8BiasOffset, 0, 128);
-        const uint32_t elected = ElectOne();
-        const int chain = ctx.warp >> 2;
-        const uint32_t accumulators = ctx.accumulators;
-        const uint64_t chainOperand = operandBase + uint64_t(uint32_t(chain) * uint32_t(kRefOperandBytes >> 4));
-        // accumulators := bias (rows e_l times the matrix whose column l is the layer's bias: exact)
-        UmmaF16(accumulators, onesBase, biasBase, instr, 0, elected);
-#pragma unroll
-        for (int kStep = 0; kStep < kK / 16; ++kStep)
+        if (ElectOne())
         {
-            // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
-            const uint64_t descA = chainOperand + uint64_t((kStep * 2 * 2048) >> 4);
-            const uint64_t descB = weightBase + uint64_t((kStep * 2 * kN * 16) >> 4);
-            if (kStep >= kRefFirstTmemStep<kLayer>)
-                UmmaF16FromTmem(accumulators, accumulators + kRefOperandColumn + uint32_t(kStep) * 8u, descB, instr, 1, elected);
-            else
-                UmmaF16(accumulators, descA, descB, instr, 1, elected);
+            constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
+            const uint32_t base = DescriptorAddress(DynamicSharedBase());
+            const int chain = ctx.warp >> 2;
+            const uint32_t accumulators = ctx.accumulators;
+            const uint32_t operand = base + uint32_t(chain) * uint32_t(kRefOperandBytes >> 4) + uint32_t(offsetof(RefSharedStorage, operandA) >> 4) + DescriptorLow(2048);
+            const uint32_t weights = base + uint32_t((offsetof(RefSharedStorage, network) + kWeightOffset) >> 4) + DescriptorLow(kN * 16);
+            // rows e_kLayer (every 8-row group reads the same core matrix: stride 0), then the core matrix of zeros
+            const uint32_t ones = base + uint32_t((offsetof(RefSharedStorage, onesRegion) + kLayer * 128) >> 4) + DescriptorLow((4 - kLayer) * 128);
+            // the matrix of biases, read twice (leading offset 0): its second copy meets the zeros
+            const uint32_t biases = base + uint32_t((offsetof(RefSharedStorage, network) + kRefInt8BiasOffset) >> 4) + DescriptorLow(0);
+            // accumulators := bias (rows e_l times the matrix whose column l is the layer's bias: exact)
+            UmmaF16<0>(accumulators, ones, biases, instr, 0);
+#pragma unroll
+            for (int kStep = 0; kStep < kK / 16; ++kStep)
+            {
+                // one K step = two 16-byte core matrices; A: 2048 bytes apart, B: kN*16 bytes apart
+                const uint32_t stepWeights = weights + uint32_t((kStep * 2 * kN * 16) >> 4);
+                if (kStep >= kRefFirstTmemStep<kLayer>)
+                    UmmaF16FromTmem(accumulators, accumulators + kRefOperandColumn + uint32_t(kStep) * 8u, stepWeights, instr, 1);
+                else
+                    UmmaF16(accumulators, operand + uint32_t((kStep * 2 * 2048) >> 4), stepWeights, instr, 1);
+            }
+            // arrives once everything issued so far has completed: the chain's accumulators are ready
+            UmmaCommit(ctx.barrier);
         }
-        // arrives once everything issued so far has completed: the chain's accumulators are ready
-        if (elected)
-            UmmaCommit(base + uint32_t(offsetof(RefSharedStorage, barrier)) + chain * 8);
     }
     return 0;
 }
@@ -768,39 +767,40 @@ using RefFp8Stage = CodesStage<kRefFp8Footprint.hiBytes, kRefFp8Footprint.loByte
 static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(RefFp8Stage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 e4m3 operands, binary16 accumulators.
-__device__ __forceinline__ void UmmaE4m3F16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t instr, uint32_t accumulate,
-    uint32_t enabled = 1)
+template <uint32_t kStrideA = 128>
+__device__ __forceinline__ void UmmaE4m3F16(uint32_t tmemD, uint32_t lowA, uint32_t lowB, uint32_t instr, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t"
-        ".reg .pred p, q;\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 a, b;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+        "mov.b64 a, {%1, %5};\n\t"
+        "mov.b64 b, {%2, %6};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n\t"
         "}" ::"r"(tmemD),
-        "l"(descA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+        "r"(lowA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(kStrideA)), "n"(DescriptorHigh(128))
         : "memory");
 }
 
 // The same two products with the A operand in tensor memory (lane = row, four 8-bit or two 16-bit K values per column).
-__device__ __forceinline__ void UmmaE4m3F16FromTmem(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t instr, uint32_t accumulate,
-    uint32_t enabled)
+__device__ __forceinline__ void UmmaE4m3F16FromTmem(uint32_t tmemD, uint32_t tmemA, uint32_t lowB, uint32_t instr, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t"
-        ".reg .pred p, q;\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b64 b;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
+        "mov.b64 b, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], b, %3, p;\n\t"
         "}" ::"r"(tmemD),
-        "r"(tmemA), "l"(descB), "r"(instr), "r"(accumulate), "r"(enabled)
+        "r"(tmemA), "r"(lowB), "r"(instr), "r"(accumulate), "n"(DescriptorHigh(128))
         : "memory");
 }
 
-// The matrix products of one layer of a chain's tile, issued by the thread with `enabled` set.  `accumulators`: the chain's
-// first tensor-memory column.
+// The matrix products of one layer of a chain's tile, issued by one elected thread.
 template <int kLayer>
-__device__ __forceinline__ void IssueChainRefFp8(int chain, uint32_t accumulators, uint32_t enabled)
+__device__ __forceinline__ void IssueChainRefFp8(const ChainContext& ctx)
 {
     constexpr int kN = kLayer == 0 ? 64 : kLayer == 1 ? 48 : kLayer == 2 ? 32 : 16;
     constexpr int kK = kLayer == 0 ? 48 : kLayer == 1 ? 64 : kLayer == 2 ? 48 : 32;
@@ -810,39 +810,35 @@ __device__ __forceinline__ void IssueChainRefFp8(int chain, uint32_t accumulator
         kLayer == 0 ? kRefBiasOffset0 : kLayer == 1 ? kRefBiasOffset1 : kLayer == 2 ? kRefBiasOffset2 : kRefBiasOffset3;
     // both descriptors: binary16 accumulators, operand formats 0 (binary16 for kind::f16, e4m3 for kind::f8f6f4)
     constexpr uint32_t instr = MakeInstrDescriptorF16(kN);
-    // The issuing thread is the critical path of the layer: the four base descriptors are built
-    // once, every operand is then a constant offset (in 16-byte units) added to the address field.
-    const uint32_t base = DynamicSharedBase(), networkBase = base + uint32_t(offsetof(RefFp8SharedStorage, network));
-    const uint64_t operandBase =
-        MakeSmemDescriptor(base + uint32_t(offsetof(RefFp8SharedStorage, operandA)) + uint32_t(chain) * uint32_t(kOperandBytes), 2048, 128);
-    const uint64_t onesBase = MakeSmemDescriptor(base + uint32_t(offsetof(RefFp8SharedStorage, biasRegion)), 2048, 128);
-    const uint64_t weightBase = MakeSmemDescriptor(networkBase + kWeightOffset, kN * 16, 128);
-    const uint64_t biasBase = MakeSmemDescriptor(networkBase + kBiasOffset, kN * 16, 128);
+    // The issuing thread is the critical path of the layer: every operand is a constant distance from one of two addresses.
+    const uint32_t base = DescriptorAddress(DynamicSharedBase());
+    const uint32_t accumulators = ctx.accumulators;
+    const uint32_t operand = base + uint32_t(ctx.warp >> 2) * uint32_t(kOperandBytes >> 4) + uint32_t(offsetof(RefFp8SharedStorage, operandA) >> 4) + DescriptorLow(2048);
+    const uint32_t ones = base + uint32_t(offsetof(RefFp8SharedStorage, biasRegion) >> 4) + DescriptorLow(2048);
+    const uint32_t weights = base + uint32_t((offsetof(RefFp8SharedStorage, network) + kWeightOffset) >> 4) + DescriptorLow(kN * 16);
+    const uint32_t biases = base + uint32_t((offsetof(RefFp8SharedStorage, network) + kBiasOffset) >> 4) + DescriptorLow(kN * 16);
     // accumulators := bias (binary16 step: rows (1, 0, ...) times the bias column: exact)
-    UmmaF16(accumulators, onesBase, biasBase, instr, 0, enabled);
+    UmmaF16(accumulators, ones, biases, instr, 0);
 #pragma unroll
     for (int step = 0; step < kK / 16; ++step)
     {
         if (kLayer < 3)
         {
             // 16 products of the 32-wide chunk step / 2: weight copy `step` has the other 16 columns zeroed
-            const uint64_t descA = operandBase + uint64_t(((step / 2) * 2 * 2048) >> 4);
-            const uint64_t descB = weightBase + uint64_t((step * kN * 32) >> 4);
+            const uint32_t stepWeights = weights + uint32_t((step * kN * 32) >> 4);
             if (kLayer > 0)
-                UmmaE4m3F16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step / 2) * 8u, descB, instr, 1, enabled);
+                UmmaE4m3F16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step / 2) * 8u, stepWeights, instr, 1);
             else
-                UmmaE4m3F16(accumulators, descA, descB, instr, 1, enabled);
+                UmmaE4m3F16(accumulators, operand + uint32_t(((step / 2) * 2 * 2048) >> 4), stepWeights, instr, 1);
         }
         else
         {
             // binary16 operands: one K step = two core matrices of 8 halves
-            const uint64_t descB = weightBase + uint64_t((step * 2 * kN * 16) >> 4);
-            UmmaF16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step) * 8u, descB, instr, 1, enabled);
+            UmmaF16FromTmem(accumulators, accumulators + kOperandColumn + uint32_t(step) * 8u, weights + uint32_t((step * 2 * kN * 16) >> 4), instr, 1);
         }
     }
     // arrives once everything issued so far has completed: this chain's accumulators are ready
-    if (enabled)
-        UmmaCommit(base + uint32_t(offsetof(RefFp8SharedStorage, barrier)) + chain * 8);
+    UmmaCommit(ctx.barrier);
 }
 
 // First half of a layer: hands the A operand written before this call to the tensor core.  Returns
@@ -863,15 +859,16 @@ __device__ __forceinline__ int IssueLayerRefFp8(ChainContext& ctx)
     TcgenFenceBeforeSync();
     if (LayerBarrier<kLayer>(ctx.warp >> 2, ctx.giveUp))
         return 1;
-    // The whole issuing warp runs the descriptor arithmetic, on values the compiler can see are the same
-    // in every lane (ChainContext; addresses counted from the start of dynamic shared memory), and one elected lane hands the work to
-    // the tensor core: issued from a single thread inside a divergent branch the same code cost 85 instructions per texel more.
-    // (Tried: building the descriptors before the barrier - 3 % slower.)
+    // One elected lane hands the work to the tensor core, in one branch on elect.sync, which the compiler knows to be taken by a single lane: what
+    // the operands' descriptors are made of is the same in the whole warp (ChainContext; addresses counted from the start of dynamic shared
+    // memory) and stays in uniform registers.  (Every instruction with a predicate of its own, which the compiler turned into a branch around each:
+    // 4096 x 4096 FP8 641 us instead of 595, 2048 x 2048 of 8 features 153 instead of 145, 8192 x 8192 Int8 3579 instead of 3567, 16.7 M queries 635
+    // instead of 622.  Issued from a thread picked by its index: 85 instructions per texel more.)
     if (WarpRole(ctx.warp) == kIssuingRole)
     {
         TcgenFenceAfterSync();
-        const uint32_t elected = ElectOne();
-        IssueChainRefFp8<kLayer>(ctx.warp >> 2, ctx.accumulators, elected);
+        if (ElectOne())
+            IssueChainRefFp8<kLayer>(ctx);
     }
     return 0;
 }

@@ -144,6 +144,18 @@ __device__ __forceinline__ void UmmaCommit(uint32_t bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// ... by a converged warp, from the lane that elect.sync picks.
+__device__ __forceinline__ void UmmaCommitElected(uint32_t bar)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred q;\n\t"
+        "elect.sync _|q, 0xFFFFFFFF;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "}" ::"r"(bar)
+        : "memory");
+}
+
 // 16 consecutive 32-bit columns of this thread's TMEM lane.
 __device__ __forceinline__ void TmemLoad16(uint32_t address, uint32_t (&r)[16])
 {
@@ -190,15 +202,19 @@ __device__ __forceinline__ void TmemLoadWait()
 }
 
 // Shared-memory matrix descriptor, K-major, no swizzle: 8x16-byte core matrices; `leadingBytes`
-// separates core matrices along K, `strideBytes` separates 8-row groups along M/N.
-__device__ __forceinline__ uint64_t MakeSmemDescriptor(uint32_t sharedAddress, uint32_t leadingBytes, uint32_t strideBytes)
+// separates core matrices along K, `strideBytes` separates 8-row groups along M/N.  As its two words: the high one is a constant, the low one
+// holds the address in units of 16 bytes (DescriptorAddress), so operands at constant distances are one 32-bit addition apart.
+__host__ __device__ constexpr uint32_t DescriptorLow(uint32_t leadingBytes)
 {
-    uint64_t desc = 0;
-    desc |= uint64_t((sharedAddress & 0x3FFFF) >> 4);
-    desc |= uint64_t((leadingBytes >> 4) & 0x3FFF) << 16;
-    desc |= uint64_t((strideBytes >> 4) & 0x3FFF) << 32;
-    desc |= uint64_t(1) << 46; // descriptor version of this architecture
-    return desc;               // base offset 0, layout type 0 (no swizzle)
+    return (leadingBytes >> 4) << 16;
+}
+__host__ __device__ constexpr uint32_t DescriptorHigh(uint32_t strideBytes)
+{
+    return (strideBytes >> 4) | 1u << 14; // bit 46: descriptor version of this architecture; base offset 0, layout type 0 (no swizzle)
+}
+__device__ __forceinline__ uint32_t DescriptorAddress(uint32_t sharedAddress)
+{
+    return (sharedAddress & 0x3FFFF) >> 4;
 }
 
 __device__ __forceinline__ uint32_t AsU32(__half2 v)
