@@ -147,21 +147,22 @@ __host__ __device__ constexpr uint32_t MakeInstrDescriptor(bool fp8, int n)
 // ---------------------------------------------------------------------------------------------
 
 // Clamped HGELU followed by re-quantisation to the int8 code rint(y * 80) - 113 (src/tin/tin_activation.h:94-99,
-// the -113 offset is folded into the next layer's stored bias, src/Quantizer.cu:176-181).
-// y * 80 lies in [-15, 240], so 113 is the only offset that fits int8; being odd, it cannot be
-// merged into the even magic addend without changing how ties round.
-__device__ __forceinline__ uint32_t ActivateToInt8(__half2 x)
+// the -113 offset is folded into the next layer's stored bias, src/Quantizer.cu:176-181): 368 - rint(y * 80), whose low byte in either half is the
+// code's complement.  y * 80 lies in [-15.01, 240]; the subnormal binary16 numbers are the multiples of 2^-24, so one multiply-add rounds to an
+// integer, ties as rint does because 368 is even.  (By adding 1536 and then -113 it was one packed operation more for two codes, and no complement for
+// four: 2048 x 2048 of 8 features 259 us instead of 249, 12 features 283 instead of 267, 16 features 291
+// instead of 279.)
+__device__ __forceinline__ uint32_t ActivateToComplement(__half2 x)
 {
     const __half2 p = __hmul2_rn(ClampedHgelu(x), __float2half2_rn(80.f));
-    const __half2 r = __hadd2_rn(p, __float2half2_rn(1536.f)); // rint(p): ulp is 1 in [1024, 2048)
-    return AsU32(__hadd2_rn(r, __float2half2_rn(-113.f)));     // exact
+    return AsU32(__hfma2(p, __float2half2_rn(-0x1p-24f), __float2half2_rn(368.f * 0x1p-24f)));
 }
 
-// Two pairs of activations (e4m3) or of int8 codes -> the next layer's four operand bytes.
+// Two pairs of activations (e4m3) or of complements of int8 codes -> the next layer's four operand bytes.
 template <bool kToFp8>
 __device__ __forceinline__ uint32_t PackCodes(uint32_t first, uint32_t second)
 {
-    return kToFp8 ? E4m3Codes(AsHalf2(first), AsHalf2(second)) : __byte_perm(first, second, 0x6420);
+    return kToFp8 ? E4m3Codes(AsHalf2(first), AsHalf2(second)) : ~__byte_perm(first, second, 0x6420);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -294,7 +295,7 @@ __device__ __forceinline__ void ConsumeLayerImpl(const Params& params, const Exa
                             float f1 = __fmul_rn(float(int32_t(acc[c][2 * j + 1]) + (kBiasTable ? biasI[colIndex + 1] : 0)), scale[colIndex + 1]);
                             xh = __floats2half2_rn(f0, f1);
                         }
-                        pairs[j] = kNextFp8 ? AsU32(ClampedHgelu(xh)) : ActivateToInt8(xh);
+                        pairs[j] = kNextFp8 ? AsU32(ClampedHgelu(xh)) : ActivateToComplement(xh);
                     }
                     const uint4 codes =
                         make_uint4(PackCodes<kNextFp8>(pairs[0], pairs[1]), PackCodes<kNextFp8>(pairs[2], pairs[3]),

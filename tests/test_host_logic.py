@@ -531,6 +531,20 @@ def test_rounding_to_the_activation_grid_as_a_subnormal_number():
     assert np.array_equal(half(scaled * (step * 2 ** 22) - 16 * step), half(np.rint(p) * step))
 
 
+def test_int8_codes_of_activations_as_complements():
+    """The exact-accumulation kernels' code rint(y * 80) - 113 of an activation: the complement of the low byte of 368 - rint(y * 80), which one
+    multiply-add gives as a subnormal binary16 number, for every activation input but -infinity (whose activation is no number)."""
+    def half(values):
+        return values.astype(np.float16)  # (round to nearest even; a binary64 holds every sum and product here exactly)
+
+    x = np.arange(65536, dtype=np.uint16).view(np.float16)
+    x = x[~np.isnan(x) & (x != -np.inf)].astype(np.float64)
+    t = half(np.clip(x * float(np.float16(1 / 3)) + 0.5, 0, 1)).astype(np.float64)
+    p = half(half(np.minimum(x, 3) * t).astype(np.float64) * 80).astype(np.float64)
+    bits = half(p * -2.0 ** -24 + 368 * 2.0 ** -24).view(np.uint16)
+    assert np.array_equal((~bits & 0xFF).astype(np.uint8).view(np.int8), (np.rint(p) - 113).astype(np.int8))
+
+
 def test_int8_codes_of_blended_features():
     """The int8 code of a blended feature, floor(x * 127.5 - 0.5) clamped to +-127, as half of an integer that one multiply-add rounds to, for every x
     = 2 d - 1 that a blend d can give: weights that add up to 1, rounded, times taps of at most 1, through four rounded operations."""
