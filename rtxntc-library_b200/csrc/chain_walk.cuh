@@ -19,12 +19,14 @@ namespace
 {
 
 // What a chain prepares per run of tiles.
-template <typename Tables, int kHiBytes, int kLoBytes>
+template <typename Tables, const FootprintBuffers& kBuffers>
 struct __align__(16) ChainStage
 {
+    template <int kLayers>
+    static constexpr int kPixelBytes = kBuffers.pixelBytes[kLayers];
     Tables tables;
-    uint8_t footprintHi[kHiBytes];
-    uint8_t footprintLo[kLoBytes];
+    uint8_t footprintHi[kBuffers.hiBytes];
+    uint8_t footprintLo[kBuffers.loBytes];
 };
 
 // What the threads of a chain keep of their texel's place in a tile while the tables stay the same: with power-of-two sizes that is from the
@@ -37,8 +39,8 @@ struct __align__(16) TexelTables
 };
 
 // ... of the kernels whose layer-0 operand is 64-byte rows of codes.
-template <int kHiBytes, int kLoBytes>
-struct __align__(16) CodesStage : ChainStage<TileTables<ChainTile>, kHiBytes, kLoBytes>
+template <const FootprintBuffers& kBuffers>
+struct __align__(16) CodesStage : ChainStage<TileTables<ChainTile>, kBuffers>
 {
     TexelTables texels;
 };
@@ -71,20 +73,34 @@ template <int kLayers, typename Stage, typename Blend>
 __device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, int2 shift, Blend blend)
 {
     const uint4 taps = stage.texels.taps[texel];
-    const int stride = StrideBytes<kLayers>(mip);
+    const int stride = StrideBytes<Stage, kLayers>(mip);
 #pragma unroll
     for (int grid = 0; grid < 2; ++grid)
     {
         const uint4 w = stage.texels.weights[grid][texel];
         const uint8_t* tap00 = grid ? stage.footprintLo + (taps.z + shift.y) : stage.footprintHi + (taps.x + shift.x);
         const uint8_t* tap10 = tap00 + (grid ? taps.w : taps.y);
-#pragma unroll
-        for (int layer = 0; layer < 4; ++layer)
+        const __half2 w00 = AsHalf2(w.x), w01 = AsHalf2(w.y), w10 = AsHalf2(w.z), w11 = AsHalf2(w.w);
+        if constexpr (kLayers % 2 == 0 && kLayers != 0 && Stage::template kPixelBytes<kLayers> % 16 == 0)
         {
-            if (layer < NumLayers<kLayers>(params))
-                blend(grid, layer, *reinterpret_cast<const uint2*>(tap00 + layer * 8), *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8),
-                    *reinterpret_cast<const uint2*>(tap10 + layer * 8), *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8),
-                    AsHalf2(w.x), AsHalf2(w.y), AsHalf2(w.z), AsHalf2(w.w));
+            // two layers of a tap at once
+#pragma unroll
+            for (int layer = 0; layer < kLayers; layer += 2)
+            {
+                const uint4 l00 = *reinterpret_cast<const uint4*>(tap00 + layer * 8), l01 = *reinterpret_cast<const uint4*>(tap00 + stride + layer * 8);
+                const uint4 l10 = *reinterpret_cast<const uint4*>(tap10 + layer * 8), l11 = *reinterpret_cast<const uint4*>(tap10 + stride + layer * 8);
+                blend(grid, layer, make_uint2(l00.x, l00.y), make_uint2(l01.x, l01.y), make_uint2(l10.x, l10.y), make_uint2(l11.x, l11.y), w00, w01, w10, w11);
+                blend(grid, layer + 1, make_uint2(l00.z, l00.w), make_uint2(l01.z, l01.w), make_uint2(l10.z, l10.w), make_uint2(l11.z, l11.w), w00, w01, w10,
+                    w11);
+            }
+        }
+        else
+        {
+#pragma unroll
+            for (int layer = 0; layer < 4; ++layer)
+                if (layer < NumLayers<kLayers>(params))
+                    blend(grid, layer, *reinterpret_cast<const uint2*>(tap00 + layer * 8), *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8),
+                        *reinterpret_cast<const uint2*>(tap10 + layer * 8), *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8), w00, w01, w10, w11);
         }
     }
 }
@@ -265,7 +281,7 @@ __device__ __forceinline__ void DecodeRuns(const KernelParams& params)
         ctx.y = y0 + tileRow;
         // runs start at multiples of their width
         const int column = x0 & (mip.runTiles * kChainTileWidth - 1);
-        const int steps = known ? column / kChainTileWidth * StrideBytes<kLayers>(mip) : 0;
+        const int steps = known ? column / kChainTileWidth * StrideBytes<Stage, kLayers>(mip) : 0;
         Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known,
             make_int2(steps * mip.hiStepX, steps * mip.loStepX));
 

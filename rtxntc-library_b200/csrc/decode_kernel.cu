@@ -181,7 +181,7 @@ struct __align__(128) ExactStorage
     uint32_t tmemBase;
     alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row, in core-matrix order; then the ExactStages
 };
-using ExactStage = CodesStage<kExactFootprint.hiBytes, kExactFootprint.loBytes>;
+using ExactStage = CodesStage<kExactFootprint>;
 static_assert(sizeof(ExactStorage) + kMaxChains * sizeof(ExactStage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
 // First half of a layer: hands the A operand written before this call to the tensor core, an elected lane of the warp of kIssuingRole.  Returns

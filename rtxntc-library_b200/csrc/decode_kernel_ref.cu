@@ -177,7 +177,7 @@ struct __align__(16) RefTileTables
     uint32_t pad[2];
 };
 
-struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8Footprint.hiBytes, kRefInt8Footprint.loBytes>
+struct __align__(16) RefStage : ChainStage<RefTileTables, kRefInt8Footprint>
 {
     TexelTables texels;
 };
@@ -230,7 +230,7 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
             }
         });
     }
-    PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, tileX0,
+    PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, StrideBytes<RefStage, kLayers>(mip), tileX0,
         tileY0, columns, lane, warp, tablesValid, between);
 }
 
@@ -767,7 +767,7 @@ struct __align__(128) RefFp8SharedStorage
     uint32_t tmemBase;
     alignas(128) uint8_t operandA[kMaxChains * kOperandBytes]; // A operands of layer 0, 64 bytes a row; then the RefFp8Stages
 };
-using RefFp8Stage = CodesStage<kRefFp8Footprint.hiBytes, kRefFp8Footprint.loBytes>;
+using RefFp8Stage = CodesStage<kRefFp8Footprint>;
 static_assert(sizeof(RefFp8SharedStorage) + kMaxChains * sizeof(RefFp8Stage) <= kMaxSharedBytes<1>, "a CTA must fit into shared memory");
 
 // D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 32 e4m3 operands, binary16 accumulators.

@@ -10,20 +10,26 @@ constexpr int kChainTileWidth = 16;
 constexpr int kChainTileHeight = 8;
 constexpr int kMaxRunTiles = 4; // tiles of a run, see KernelMip::runTiles
 
-// Shared memory of a chain for the latents of a run of tiles, in the high-res and the low-res grid.
+// Shared memory of a chain for the latents of a run of tiles, in the high-res and the low-res grid, and what a latent pixel takes of it: eight bytes per
+// layer, either side by side without gaps, where two layers of a tap are one load of 16 bytes (GatherTexel), or padded to an odd multiple of eight, so
+// that 8-byte loads of neighbouring pixels fall into different banks.
+// Wide loads are taken where they pay: 16 features, Int8, 2048 x 2048, 228.5 us instead of 231.1, 1920 x 1080 at a grid of a half 139.6 instead of
+// 142.7; 8 features, FP8, 143.5 instead of 145.1, at a half 153.7 instead of 157.6.  With 16 features and FP8 weights (166.9 instead of 161.7) or with exact
+// accumulation (8 features 256 instead of 249, 16 features 288 instead of 279) the kernels run out of registers.
 struct FootprintBuffers
 {
     int hiBytes, loBytes;
+    int pixelBytes[5]; // by layers
 };
 // What a tile covers at a grid-to-mip ratio of 1 (high-res: 18 x 10 pixels of 24 bytes) and 1/2 (low-res: 10 x 6), or a run of tiles at a smaller
 // one.
-constexpr FootprintBuffers kRefFp8Footprint{4352, 1536};
-constexpr FootprintBuffers kRefInt8Footprint{4352, 1440}; // (all that the CTA has left)
+inline constexpr FootprintBuffers kRefFp8Footprint{4352, 1536, {0, 8, 16, 24, 40}};
+inline constexpr FootprintBuffers kRefInt8Footprint{4352, 1440, {0, 8, 16, 24, 32}}; // (all that the CTA has left)
 // The exact-accumulation kernels have room for a tile at a ratio of 4/5 with four latent layers (15 x 8 pixels of 40 bytes, 9 x 5).  (With the FP8
 // kernels' buffers mips at 4/5 and 2/3 were read tap by tap: mip 1 of a 3000 x 4000 Int8 set of 16 features at scale 3 took 224 us, now
 // 196, FP8 162 and 135; mip 2 of 4096 x 4096 at scale 5 79.5 and 72.6.  With 6144 and 2432 bytes more runs would be longer, some for the worse:
 // 3000 x 2000 Int8, 12 features, 445 and 455 us.)
-constexpr FootprintBuffers kExactFootprint{4800, 1808};
+inline constexpr FootprintBuffers kExactFootprint{4800, 1808, {0, 8, 24, 24, 40}};
 
 // Most latent pixels, of a grid of `grid` pixels, that texels x .. x + span of an axis of `extent` texels read: the last tap's index minus
 // the first's, plus the second tap of each end.

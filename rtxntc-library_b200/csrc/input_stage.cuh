@@ -25,10 +25,11 @@ __device__ __forceinline__ int NumLayers(const KernelParams& params)
     return kLayers ? kLayers : params.numLayers;
 }
 
-template <int kLayers>
+template <typename Stage, int kLayers>
 __device__ __forceinline__ int StrideBytes(const KernelMip& mip)
 {
-    return kLayers ? (kLayers == 1 ? 8 : kLayers <= 3 ? 24 : 40) : mip.strideBytes;
+    constexpr int kBytes = Stage::template kPixelBytes<kLayers>;
+    return kLayers ? kBytes : mip.strideBytes;
 }
 
 // Quantises a pair of network inputs.  Int8: floor(x * 127.5 - 0.5) clamped to +-127
@@ -291,13 +292,12 @@ struct __align__(16) TileTables
 // `between()` is called between building the tables, which needs nothing from global memory, and staging (not with valid tables).
 template <typename Tile, bool kReferenceDivision, int kLayers, typename Between>
 __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const KernelMip& mip, TapTables<Tile>& taps,
-    uint8_t* footprintHi, uint8_t* footprintLo, int tileX0, int tileY0, int columns, int lane, int warp,
+    uint8_t* footprintHi, uint8_t* footprintLo, int stride, int tileX0, int tileY0, int columns, int lane, int warp,
     bool tablesValid, Between between)
 {
     const int grid = warp & 1;
     const int gw = grid ? mip.loWidth : mip.hiWidth;
     const int gh = grid ? mip.loHeight : mip.hiHeight;
-    const int stride = StrideBytes<kLayers>(mip);
 
     int fx0, fy0, footW, count;
     uint32_t magic;
@@ -432,7 +432,7 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
                 stage.tables.lodWord = QuantizeLod<kFp8>(mip.positionLod);
         });
     }
-    PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo,
+    PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, StrideBytes<Stage, kLayers>(mip),
         tileX0, tileY0, columns, lane, warp, tablesValid, between);
 }
 

@@ -111,7 +111,7 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, FootprintBuf
     km.invHeight = 1.0f / float(m.height);
     km.positionScale = m.positionScale;
     km.positionLod = m.positionLod;
-    km.strideBytes = layers == 1 ? 8 : layers <= 3 ? 24 : 40;
+    km.strideBytes = buffers.pixelBytes[layers];
     const int staged = StagedTiles(m.hiWidth, m.hiHeight, m.loWidth, m.loHeight, m.width, m.height, km.strideBytes, buffers, maxRunTiles);
     km.staged = staged > 0;
     km.runTiles = staged > 0 ? staged : 1;
