@@ -256,15 +256,15 @@ __device__ __forceinline__ uint32_t E4m3Codes(__half2 first, __half2 second)
 }
 
 // Inf / NaN -> 0 in the channel pairs of one texel (src/Inference.cu:125-126, src/CudaUtils.h:30-35).
-// A binary16 value times zero is a zero unless the value is an infinity or a NaN, so one fused
-// multiply-add per pair into a common sum detects whether anything has to be done at all.
+// The largest magnitude of all pairs, a NaN counting as largest, shows whether anything has to be done at all.  (Sums of products with zero show it
+// in as many instructions, but on the packed-fp16 pipe, the busiest: 8192 x 8192 Int8 3468 us instead of 3448, 4096 x 4096 FP8 592.7 instead of 589.5.)
 __device__ __forceinline__ void ScrubSpecials(uint32_t (&bits)[8], int channelPairs)
 {
-    __half2 sum = __float2half2_rn(0.f);
+    uint32_t largest = bits[0];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) // (all pairs: a special value in a pair beyond the channels only leads to the check of each)
-        sum = __hfma2(AsHalf2(bits[j]), __float2half2_rn(0.f), sum);
-    if (AsU32(sum) & 0x7FFF7FFFu)
+    for (int j = 1; j < 8; ++j) // (all pairs: a special value in a pair beyond the channels only leads to the check of each)
+        asm("max.NaN.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(largest) : "r"(largest), "r"(bits[j]));
+    if (((largest & 0x7C007C00u) + 0x04000400u) & 0x80008000u)
     {
         // rare, so kept off the common path
 #pragma unroll
