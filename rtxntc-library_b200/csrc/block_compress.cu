@@ -88,20 +88,23 @@ constexpr float kMagic = 8388608.f; // 2^23: a sum with it holds an integer in i
 // Pixels go through the search two at a time in packed instructions, through the sums - whose order is part of the
 // result - one by one.  kNear: d <= h.  All of 0 .. d are palette values then, the smallest rank at t < d is 2 t, and rank N
 // has the value d together with others, of which its index is the lowest.
-template <bool kSix, bool kNear>
-__device__ __forceinline__ void AssignPalette(const Pair (&values)[8], float a0, float a1, uint64_t& indices, float& squaredError, RefitSums& sums)
+// kPairs: the eight pairs of a block, or one; `weights`, if any, receives the weights of endpoint 0, and what `sums` has is of no use then.
+template <bool kSix, bool kNear, int kPairs>
+__device__ __forceinline__ void AssignPalette(const Pair (&values)[kPairs], float a0, float a1, uint64_t& indices, float& squaredError, RefitSums& sums,
+    float* weights = nullptr)
 {
     constexpr float kSteps = kSix ? 5.f : 7.f, kHalf = kSix ? 2.f : 3.f, kPerStep = 1.f / kSteps;
     const float distance = kSix ? a1 - a0 : a0 - a1;
     const Pair inverse = Both(__fdividef(1.f, distance)), length = Both(distance), start = Both(a0);
     const float lastRank = distance > 0.f ? kMagic + kSteps : kMagic; // (kNear)
     // Eight ranks each, four bits per pixel.  The sum of the magic numbers' own bits is taken out beforehand.
-    uint32_t ranks[2] = {0u - 0x4b000000u * 0x11111111u, 0u - 0x4b000000u * 0x11111111u};
+    constexpr uint32_t kRanks = kPairs == 1 ? 0x11u : 0x11111111u;
+    uint32_t ranks[2] = {0u - 0x4b000000u * kRanks, 0u - 0x4b000000u * kRanks};
     uint32_t constants[2] = {0u, 0u}; // (kSix) pixels nearest to 0 or 255
     Pair errors = Both(0.f);
     sums.Clear();
 #pragma unroll
-    for (int two = 0; two < 8; ++two)
+    for (int two = 0; two < kPairs; ++two)
     {
         const Pair value = values[two];
         const Pair offset = kSix ? MultiplyAdd(start, Both(-1.f), value) : MultiplyAdd(value, Both(-1.f), start);
@@ -179,6 +182,11 @@ __device__ __forceinline__ void AssignPalette(const Pair (&values)[8], float a0,
             beta1 = __fsub_rn(1.f, alpha1);
         }
         errors = MultiplyAdd(miss, miss, errors); // integers below 2^20: exact in any order
+        if (weights)
+        {
+            weights[2 * two] = alpha0;
+            weights[2 * two + 1] = alpha1;
+        }
         sums.Add(alpha0, beta0, value0);
         sums.Add(alpha1, beta1, value1);
     }
@@ -197,7 +205,7 @@ __device__ __forceinline__ void AssignPalette(const Pair (&values)[8], float a0,
         // entry 6 is 0, entry 7 is 255: whichever half of the range the pixel lies in
         uint64_t upper = 0;
 #pragma unroll
-        for (int two = 0; two < 8; ++two)
+        for (int two = 0; two < kPairs; ++two)
         {
             float value0, value1;
             Split(values[two], value0, value1);
@@ -277,8 +285,79 @@ __device__ __forceinline__ float ByteToFloat(uint32_t word, int byte)
     return __uint_as_float(__byte_perm(word, 0x4b000000u, 0x7650 | byte)) - kMagic;
 }
 
+// The sixteen values of a block in pairs, and the endpoints its search starts from.
+struct StartOfSearch
+{
+    float a0, a1;
+    bool zeroAlpha1, oneAlpha0; // (eight interpolants) pinned to 0 / 255
+};
+
+template <bool kSix>
+__device__ __forceinline__ StartOfSearch StartingEndpoints(uint4 packed, Pair (&values)[8])
+{
+    StartOfSearch start{};
+    const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
+    float low = 255.f, high = 0.f; // six: of the values that are not 0 or 255
+#pragma unroll
+    for (int two = 0; two < 8; ++two)
+    {
+        const float pixels[2] = {ByteToFloat(words[two >> 1], 2 * (two & 1)), ByteToFloat(words[two >> 1], 2 * (two & 1) + 1)};
+        values[two] = MakePair(pixels[0], pixels[1]);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+        {
+            low = kSix && pixels[k] == 0.f ? low : fminf(low, pixels[k]);
+            high = kSix && pixels[k] == 255.f ? high : fmaxf(high, pixels[k]);
+        }
+    }
+    const uint32_t lowest = uint32_t(low), highest = uint32_t(high);
+    // (six: unsigned wrap-around when the block holds nothing but 0 and 255, as in the shader)
+    const uint32_t inset = (highest - lowest) / 34u;
+    if (kSix)
+    {
+        start.a0 = float((lowest + inset) & 0xffu);
+        start.a1 = float((highest - inset) & 0xffu);
+    }
+    else
+    {
+        start.zeroAlpha1 = lowest == 0u;
+        start.oneAlpha0 = highest == 255u;
+        start.a0 = start.oneAlpha0 ? 255.f : float(highest - inset);
+        start.a1 = start.zeroAlpha1 ? 0.f : float(lowest + inset);
+    }
+    return start;
+}
+
+// Least-squares endpoints for the indices of the last pass.
+template <bool kSix>
+__device__ __forceinline__ void Refit(const RefitSums& sums, const StartOfSearch& start, float& a0, float& a1)
+{
+    float determinant, numeratorA, numeratorB;
+    sums.Solve(determinant, numeratorA, numeratorB);
+    if (kSix)
+    {
+        if (determinant != 0.f)
+        {
+            a0 = RoundToByte(__fdiv_rn(numeratorA, determinant));
+            a1 = RoundToByte(__fdiv_rn(numeratorB, determinant));
+        }
+    }
+    else
+    {
+        const float factor = __fdiv_rn(1.f, determinant);
+        const float high = start.oneAlpha0 ? 255.f : RoundToByte(__fmul_rn(numeratorA, factor));
+        const float low = start.zeroAlpha1 ? 0.f : RoundToByte(__fmul_rn(numeratorB, factor));
+        a0 = fmaxf(high, low);
+        a1 = fminf(high, low);
+    }
+}
+
 constexpr int kBc4Threads = 128;
 constexpr int kBc4Batch = 256;       // values for one block's channel that a CTA holds at most
+// Searches per SM up to which eight lanes share one (SearchTogether).  A search alone takes a lane 6 to 13 us, eight lanes 3 to 5, but the eight execute three times
+// as much: 16 x 16 to 128 x 128 texels as BC4 10.5 to 11.2 us against 8.4, 256 x 256 11.5 and 10.5, 384 x 384 12.7 and 14.6, 512 x 512 15.1 and 19.9; as
+// BC5, twice the searches, 256 x 256 14.5 and 12.6, 384 x 384 15.1 and 20.8 (calls of 8 us and more back to back).
+constexpr int kBc4Together = 56;
 constexpr int kBc4RefillLanes = 8;   // lanes that must be free before a warp stops to fetch blocks
 
 struct Bc4Storage
@@ -301,7 +380,7 @@ __device__ __forceinline__ void SearchBatch(Bc4Storage& shared, int count, int l
     for (int two = 0; two < 8; ++two)
         values[two] = Both(0.f);
     float a0 = 0.f, a1 = 0.f, best0 = 0.f, best1 = 0.f, bestError = 0.f;
-    bool zeroAlpha1 = false, oneAlpha0 = false;
+    StartOfSearch start{};
     uint64_t bestIndices = 0;
     RefitSums sums;
     sums.Clear();
@@ -315,25 +394,7 @@ __device__ __forceinline__ void SearchBatch(Bc4Storage& shared, int count, int l
     {
         if (busy)
         {
-            // least-squares endpoints for the indices of the last pass
-            float determinant, numeratorA, numeratorB;
-            sums.Solve(determinant, numeratorA, numeratorB);
-            if (kSix)
-            {
-                if (determinant != 0.f)
-                {
-                    a0 = RoundToByte(__fdiv_rn(numeratorA, determinant));
-                    a1 = RoundToByte(__fdiv_rn(numeratorB, determinant));
-                }
-            }
-            else
-            {
-                const float factor = __fdiv_rn(1.f, determinant);
-                const float high = oneAlpha0 ? 255.f : RoundToByte(__fmul_rn(numeratorA, factor));
-                const float low = zeroAlpha1 ? 0.f : RoundToByte(__fmul_rn(numeratorB, factor));
-                a0 = fmaxf(high, low);
-                a1 = fminf(high, low);
-            }
+            Refit<kSix>(sums, start, a0, a1);
             // the endpoints the best indices came from again: the pass would find the same indices and stop there
             if (a0 == best0 && a1 == best1)
                 finish();
@@ -353,36 +414,9 @@ __device__ __forceinline__ void SearchBatch(Bc4Storage& shared, int count, int l
                 busy = fresh = true;
                 pass = 0;
                 const uint4 packed = shared.values[item];
-                const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
-                float low = 255.f, high = 0.f; // six: of the values that are not 0 or 255
-#pragma unroll
-                for (int two = 0; two < 8; ++two)
-                {
-                    const float pixels[2] = {ByteToFloat(words[two >> 1], 2 * (two & 1)), ByteToFloat(words[two >> 1], 2 * (two & 1) + 1)};
-                    values[two] = MakePair(pixels[0], pixels[1]);
-#pragma unroll
-                    for (int k = 0; k < 2; ++k)
-                    {
-                        low = kSix && pixels[k] == 0.f ? low : fminf(low, pixels[k]);
-                        high = kSix && pixels[k] == 255.f ? high : fmaxf(high, pixels[k]);
-                    }
-                }
-                const uint32_t lowest = uint32_t(low), highest = uint32_t(high);
-                if (kSix)
-                {
-                    // unsigned wrap-around when the block holds nothing but 0 and 255, as in the shader
-                    const uint32_t inset = (highest - lowest) / 34u;
-                    a0 = float((lowest + inset) & 0xffu);
-                    a1 = float((highest - inset) & 0xffu);
-                }
-                else
-                {
-                    zeroAlpha1 = lowest == 0u;
-                    oneAlpha0 = highest == 255u;
-                    const uint32_t inset = (highest - lowest) / 34u;
-                    a0 = oneAlpha0 ? 255.f : float(highest - inset);
-                    a1 = zeroAlpha1 ? 0.f : float(lowest + inset);
-                }
+                start = StartingEndpoints<kSix>(packed, values);
+                a0 = start.a0;
+                a1 = start.a1;
             }
         }
         if (!__any_sync(0xFFFFFFFFu, busy))
@@ -419,6 +453,96 @@ __device__ __forceinline__ void SearchBatch(Bc4Storage& shared, int count, int l
     }
 }
 
+// The same search of one block by eight lanes, a pair of pixels each, for images too small to give every lane a block: what bounds those is the length of
+// one search.  The weights go round by shuffles, and every lane adds all sixteen in the shader's order; the rest of a pass is a pair's instead of
+// eight pairs'.  `item`: the same for the eight lanes; `active`: whether there is one.
+template <bool kSix>
+__device__ __forceinline__ void SearchTogether(Bc4Storage& shared, int item, bool active, int lane)
+{
+    const int two = lane & 7;
+    const uint32_t group = 0xffu << (lane & 24);
+    const uint4 packed = shared.values[active ? item : 0];
+    const uint32_t bytes = reinterpret_cast<const uint16_t*>(shared.values + (active ? item : 0))[two];
+    Pair values[8];
+    const StartOfSearch start = StartingEndpoints<kSix>(packed, values);
+    const Pair mine[1] = {MakePair(ByteToFloat(bytes, 0), ByteToFloat(bytes, 1))};
+    float a0 = start.a0, a1 = start.a1, best0 = 0.f, best1 = 0.f, bestError = 0.f;
+    uint32_t bestIndices = 0; // of this lane's two pixels
+    bool busy = active, fresh = true;
+    RefitSums sums;
+    sums.Clear();
+    for (int pass = 0; __any_sync(0xFFFFFFFFu, busy); ++pass)
+    {
+        if (!fresh)
+        {
+            Refit<kSix>(sums, start, a0, a1);
+            // the endpoints the best indices came from again: the pass would find the same indices and stop there
+            busy = busy && !(a0 == best0 && a1 == best1);
+        }
+        const float distance = kSix ? a1 - a0 : a0 - a1;
+        const bool near = distance <= (kSix ? 2.f : 3.f), other = !(distance >= (kSix ? 0.f : 1.f));
+        uint64_t mineOnly;
+        float error, weights[2];
+        if (near)
+            AssignPalette<kSix, true, 1>(mine, a0, a1, mineOnly, error, sums, weights);
+        else
+            AssignPalette<kSix, false, 1>(mine, a0, a1, mineOnly, error, sums, weights);
+        uint32_t indices = uint32_t(mineOnly) & 0xffu;
+        // (six interpolants) pixels nearest to 0 or 255, which have no part in the refit
+        const uint32_t constants0 = __ballot_sync(0xFFFFFFFFu, (indices & 0x6u) == 0x6u) >> (lane & 24);
+        const uint32_t constants1 = __ballot_sync(0xFFFFFFFFu, (indices & 0x60u) == 0x60u) >> (lane & 24);
+#pragma unroll
+        for (int step = 1; step < 8; step *= 2)
+            error += __shfl_xor_sync(0xFFFFFFFFu, error, step); // integers below 2^20: exact in any order
+        sums.Clear();
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+        {
+            const float alpha0 = __shfl_sync(0xFFFFFFFFu, weights[0], k, 8), alpha1 = __shfl_sync(0xFFFFFFFFu, weights[1], k, 8);
+            float pixel0, pixel1;
+            Split(values[k], pixel0, pixel1);
+            sums.Add(alpha0, __fsub_rn(kSix && (constants0 >> k & 1u) ? 0.f : 1.f, alpha0), pixel0);
+            sums.Add(alpha1, __fsub_rn(kSix && (constants1 >> k & 1u) ? 0.f : 1.f, alpha1), pixel1);
+        }
+        if (other && busy)
+        {
+            uint64_t all;
+            AssignOtherPalette<kSix>(packed, a0, a1, all, error, sums);
+            indices = uint32_t(all >> (8 * two)) & 0xffu;
+        }
+        const bool same = (__ballot_sync(0xFFFFFFFFu, indices == bestIndices) & group) == group;
+        if (busy)
+        {
+            if (fresh || error < bestError)
+            {
+                const bool settled = !fresh && same;
+                best0 = a0;
+                best1 = a1;
+                bestIndices = indices;
+                if (!settled) // (a settled search keeps the error it had, as in the shader)
+                    bestError = error;
+                busy = !(settled || pass == 8);
+            }
+            else
+                busy = false;
+        }
+        fresh = false;
+    }
+    uint32_t low = two < 4 ? bestIndices << (8 * two) : 0u, high = two < 4 ? 0u : bestIndices << (8 * (two - 4));
+#pragma unroll
+    for (int step = 1; step < 8; step *= 2)
+    {
+        low |= __shfl_xor_sync(0xFFFFFFFFu, low, step);
+        high |= __shfl_xor_sync(0xFFFFFFFFu, high, step);
+    }
+    if (active && two == 0)
+    {
+        const uint64_t bits = uint64_t(uint32_t(best0)) | (uint64_t(uint32_t(best1)) << 8) | (JoinIndices<3>(uint64_t(high) << 32 | low) << 16);
+        shared.block[kSix][item] = make_uint2(uint32_t(bits), uint32_t(bits >> 32));
+        shared.error[kSix][item] = bestError;
+    }
+}
+
 struct Bc4Arguments
 {
     BlockCompressArguments base;
@@ -432,6 +556,7 @@ struct Bc4Arguments
 // 2048 x 2048, 12 interleaved channels, decoded texels: BC4 133 -> 80 us, BC5 182 -> 146 us (82 instead of 108 million warp
 // instructions than with the pixels one by one); a third of the time is the loads, which touch every sector of the
 // interleaved texels.  A 16 x 16 mip: 25 -> 10 us.
+template <bool kTogether>
 __global__ void __launch_bounds__(kBc4Threads) BlockCompressKernel(const Bc4Arguments args)
 {
     __shared__ Bc4Storage shared;
@@ -479,7 +604,15 @@ __global__ void __launch_bounds__(kBc4Threads) BlockCompressKernel(const Bc4Argu
     }
     __syncthreads();
     const int count = blocks * args.channels;
-    if (tid < kBc4Threads / 2)
+    if constexpr (kTogether)
+    {
+        const int item = (tid & (kBc4Threads / 2 - 1)) >> 3;
+        if (tid < kBc4Threads / 2)
+            SearchTogether<false>(shared, item, item < count, tid & 31);
+        else
+            SearchTogether<true>(shared, item, item < count, tid & 31);
+    }
+    else if (tid < kBc4Threads / 2)
         SearchBatch<false>(shared, count, tid & 31);
     else
         SearchBatch<true>(shared, count, tid & 31);
@@ -516,10 +649,14 @@ cudaError_t LaunchBc4(const BlockCompressArguments& base, int channels, cudaStre
         // Batches that keep about eight CTAs on every SM: small images are spread over the machine with one block per lane
         // and search, large ones give a lane up to four blocks in turn.
         const long long wanted = (long long)args.totalBlocks * channels / ((long long)sms * 8) / 32;
-        const int batch = int(wanted < 1 ? 32 : wanted > kBc4Batch / 32 ? kBc4Batch : wanted * 32);
+        const bool together = (long long)args.totalBlocks * channels <= kBc4Together * (long long)sms;
+        const int batch = together ? kBc4Threads / 16 : int(wanted < 1 ? 32 : wanted > kBc4Batch / 32 ? kBc4Batch : wanted * 32);
         args.blocksPerCta = batch / channels;
         const int grid = (args.totalBlocks + args.blocksPerCta - 1) / args.blocksPerCta;
-        BlockCompressKernel<<<grid, kBc4Threads, 0, stream>>>(args);
+        if (together)
+            BlockCompressKernel<true><<<grid, kBc4Threads, 0, stream>>>(args);
+        else
+            BlockCompressKernel<false><<<grid, kBc4Threads, 0, stream>>>(args);
         CountLaunch();
     }
     return cudaSuccess;
