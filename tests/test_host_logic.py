@@ -545,6 +545,15 @@ def test_int8_codes_of_activations_as_complements():
     assert np.array_equal((~bits & 0xFF).astype(np.uint8).view(np.int8), (np.rint(p) - 113).astype(np.int8))
 
 
+def test_latent_codes_as_one_multiply_add():
+    """A latent code n, in bits 5-8 of a binary16 the subnormal number z = n * 2^-19, is the reference's fp16(float(n) * (1.f / 15.f)) as z * 34944 + z."""
+    codes = np.arange(16, dtype=np.uint16)
+    z = (codes << 5).view(np.float16).astype(np.float64)
+    expected = (codes.astype(np.float32) * np.float32(1.0 / 15.0)).astype(np.float16)
+    assert float(np.float16(34944)) == 34944
+    assert np.array_equal((z * 34944 + z).astype(np.float16).view(np.uint16), expected.view(np.uint16))
+
+
 def test_int8_codes_of_blended_features():
     """The int8 code of a blended feature, floor(x * 127.5 - 0.5) clamped to +-127, as half of an integer that one multiply-add rounds to, for every x
     = 2 d - 1 that a blend d can give: weights that add up to 1, rounded, times taps of at most 1, through four rounded operations."""
