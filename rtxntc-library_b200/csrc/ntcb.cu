@@ -147,13 +147,14 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, FootprintBuf
 }
 
 // Longest run of tiles for a launch of `tiles` tiles on `chains` chains.  A run of r tiles costs a chain 0.36 / r of a tile for tables and
-// footprints (FP8 weights; 0.2 with Int8), and the launch about r tiles at its end, when chains run out of work: four pay from 32 tiles a chain,
-// two from 8.  (4096 x 4096 FP8, 148 tiles a chain, runs of 1, 2 and 4: 717, 673 and 655 us; 1500 x 1100, 15 tiles: 86.9, 80.2 and 83.1;
+// footprints (FP8 weights; 0.2 with Int8), and the launch about r tiles at its end, when chains run out of work: four pay from 24 tiles a chain,
+// two from 8.  (2048 x 1500 FP8, 27 tiles a chain, runs of 2 and 4: 127.9 and 122.5 us, Int8 169.3 and 168.8; 1920 x 1080, 18 tiles: 87.1 and 90.4; 1024 x 1024
+// mip 0, 7 tiles, Int8, runs of 1 and 2: 42.4 and 42.9.  Before the kernels last became faster: 4096 x 4096 FP8, 148 tiles a chain, runs of 1, 2 and 4: 717, 673 and 655 us; 1500 x 1100, 15 tiles: 86.9, 80.2 and 83.1;
 // 1024 x 512, 5 tiles: 30.1, 30.9 and 33.0.  Exact accumulation, Int8 and 12 features, alike: 4096 x 4096 1223, 1192 and 1164, 1500 x 1100 136, 130
 // and 139, 1024 x 512 44.8, 46.3 and 51.0.)
 int LongestRun(long long tiles, long long chains)
 {
-    return tiles >= 32 * chains ? kMaxRunTiles : tiles >= 8 * chains ? 2 : 1;
+    return tiles >= 24 * chains ? kMaxRunTiles : tiles >= 8 * chains ? 2 : 1;
 }
 
 } // namespace
