@@ -555,7 +555,7 @@ struct Bc4Arguments
 // arithmetic of the passes.
 // 2048 x 2048, 12 interleaved channels, decoded texels: BC4 133 -> 80 us, BC5 182 -> 146 us (82 instead of 108 million warp
 // instructions than with the pixels one by one); a third of the time is the loads, which touch every sector of the
-// interleaved texels.  A 16 x 16 mip: 25 -> 10 us.
+// interleaved texels.  A 16 x 16 mip: 25 -> 10 us, 8 and the call's own time with eight lanes per search (kTogether).
 template <bool kTogether>
 __global__ void __launch_bounds__(kBc4Threads) BlockCompressKernel(const Bc4Arguments args)
 {
@@ -646,8 +646,8 @@ cudaError_t LaunchBc4(const BlockCompressArguments& base, int channels, cudaStre
         args.base.srcTop = base.srcTop + 4 * top;
         args.base.blocks = base.blocks + size_t(top) * base.rowPitch;
         args.totalBlocks = base.widthInBlocks * std::min(rowsPerLaunch, base.heightInBlocks - top);
-        // Batches that keep about eight CTAs on every SM: small images are spread over the machine with one block per lane
-        // and search, large ones give a lane up to four blocks in turn.
+        // Batches that keep about eight CTAs on every SM: the smallest images have eight lanes per search, small ones are spread over the
+        // machine with one block per lane and search, large ones give a lane up to four blocks in turn.
         const long long wanted = (long long)args.totalBlocks * channels / ((long long)sms * 8) / 32;
         const bool together = (long long)args.totalBlocks * channels <= kBc4Together * (long long)sms;
         const int batch = together ? kBc4Threads / 16 : int(wanted < 1 ? 32 : wanted > kBc4Batch / 32 ? kBc4Batch : wanted * 32);
