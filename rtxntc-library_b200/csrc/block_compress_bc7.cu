@@ -29,10 +29,23 @@
 
 namespace ntcb
 {
+
+struct Bc7Arguments
+{
+    BlockCompressArguments base;
+    int numChannels;            // channels that feed the block: red, green, blue, alpha; missing ones read 0, alpha 1
+    const uint32_t* modeBuffer; // null: full search
+    uint32_t modeBufferByteOffset, modeMapWidthInBlocks, modeMapHeightInBlocks;
+    int modeMapOffsetX, modeMapOffsetY;
+    int groupWidthLog2, groupHeight; // mode-buffer kernel: blocks per CTA, at most 256
+};
+
+// The full search of few CTAs (the module of NTCB_BC7_FEW_BLOCKS).
+void LaunchBc7SearchOfFew(const Bc7Arguments& args, dim3 grid, cudaStream_t stream);
+
 namespace
 {
 
-constexpr int kThreads = 256; // of the mode-buffer kernel
 constexpr uint32_t kAllPixels = 0xffffu;
 
 // The partition tables of the BC7 format (Khronos data format specification, BPTC: tables P2, P3 and
@@ -732,15 +745,8 @@ __device__ uint4 EncodeDualPlane(const Pixels& pixels)
 }
 
 // ---- the kernel -----------------------------------------------------------------------------------------
-struct Bc7Arguments
-{
-    BlockCompressArguments base;
-    int numChannels;            // channels that feed the block: red, green, blue, alpha; missing ones read 0, alpha 1
-    const uint32_t* modeBuffer; // null: full search
-    uint32_t modeBufferByteOffset, modeMapWidthInBlocks, modeMapHeightInBlocks;
-    int modeMapOffsetX, modeMapOffsetY;
-    int groupWidthLog2, groupHeight; // mode-buffer kernel: blocks per CTA, at most 256
-};
+#ifndef NTCB_BC7_FEW_BLOCKS // (the mode-buffer kernel's)
+constexpr int kThreads = 256;
 
 // The block a wrong or missing mode-buffer entry produces: four 2x2 squares, black, red, green, blue
 // (CompressBC7.hlsl:1537-1545).
@@ -840,6 +846,7 @@ __device__ uint4 EncodeInMode(const uint2* texels, int stride, uint32_t mode, ui
     }
     return block;
 }
+#endif
 
 // One texel as two words of halves, red-green and blue-alpha; missing channels read 0, alpha 1, and outside the mip
 // every component reads 0.
@@ -863,6 +870,7 @@ __device__ __forceinline__ uint2 LoadTexel(const Bc7Arguments& args, int x, int 
     return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
 }
 
+#ifndef NTCB_BC7_FEW_BLOCKS
 // With a mode buffer.  A CTA takes a rectangle of up to 256 blocks, sorts them by what the mode buffer names - encoder
 // first (eight modes, mode 4 with either index selector), partition second - and its warps work through the encoders' runs
 // of blocks, 32 at a time: a warp runs one encoder, its lanes loop over the same or similar subsets, and different encoders
@@ -980,6 +988,7 @@ __global__ void __launch_bounds__(kThreads) Bc7ModeKernel(const Bc7Arguments arg
         __syncwarp();
     }
 }
+#endif
 
 // ---- full search ------------------------------------------------------------------------------------------
 //
@@ -1000,6 +1009,11 @@ constexpr int kSearchThreads = 32 * kSearchWarps;
 constexpr int kSearchWidth = 16, kSearchHeight = 4; // blocks per CTA
 constexpr int kSearchBlocks = kSearchWidth * kSearchHeight;
 constexpr int kSearchTasks = 8;
+#ifdef NTCB_BC7_FEW_BLOCKS
+constexpr int kPixelsAtOnce = 4;
+#else
+constexpr int kPixelsAtOnce = 1;
+#endif
 
 __device__ __forceinline__ Pair RoundSmall(Pair x) { return PlainAdd(x + Both(12582912.f), Both(-12582912.f)); }
 
@@ -1479,7 +1493,7 @@ __device__ __forceinline__ Pair EstimateSubset(const SearchStorage& shared, int 
         sum[c] = Both(0.f);
     {
         uint64_t rest = list;
-#pragma unroll 1
+#pragma unroll kPixelsAtOnce
         for (int k = 0; k < count; ++k, rest >>= 4)
         {
             const uint4 raw = shared.halves[(uint32_t(rest) & 15u) * 32 + lane];
@@ -1512,7 +1526,7 @@ __device__ __forceinline__ Pair EstimateSubset(const SearchStorage& shared, int 
             center[c] = Negate(DivideByCount(sum[c], countValue, reciprocal));
         Pair redGreen = Both(0.f), redBlue = Both(0.f), greenBlue = Both(0.f);
         uint64_t rest = list;
-#pragma unroll 1
+#pragma unroll kPixelsAtOnce
         for (int k = 0; k < count; ++k, rest >>= 4)
         {
             PairVec<3> p = PairPixel<3>(pixels, int(uint32_t(rest) & 15u));
@@ -1562,7 +1576,7 @@ __device__ __forceinline__ Pair EstimateSubset(const SearchStorage& shared, int 
     const Pair mul = MakePair(mul0, mul1), indexMax = Both(maxIndex), indexScale = Both(1.f / maxIndex);
     Pair error = Both(0.f);
     uint64_t rest = list;
-#pragma unroll 1
+#pragma unroll kPixelsAtOnce
     for (int k = 0; k < count; ++k, rest >>= 4)
     {
         const PairVec<C> texel = PairPixel<C>(pixels, int(uint32_t(rest) & 15u));
@@ -1597,7 +1611,7 @@ __device__ __forceinline__ Pair EstimateRedSubset(const SearchStorage& shared, i
     __half2 low = __halves2half2(__ushort_as_half(0x7c00), __ushort_as_half(0x7c00));
     __half2 high = __halves2half2(__ushort_as_half(0xfc00), __ushort_as_half(0xfc00));
     uint64_t rest = list;
-#pragma unroll 1
+#pragma unroll kPixelsAtOnce
     for (int k = 0; k < count; ++k, rest >>= 4)
     {
         const uint32_t raw = shared.halves[(uint32_t(rest) & 15u) * 32 + lane].x;
@@ -1615,7 +1629,7 @@ __device__ __forceinline__ Pair EstimateRedSubset(const SearchStorage& shared, i
     const Pair mul = MakePair(mul0, mul1), indexMax = Both(maxIndex), indexScale = Both(1.f / maxIndex);
     Pair error = Both(0.f);
     rest = list;
-#pragma unroll 1
+#pragma unroll kPixelsAtOnce
     for (int k = 0; k < count; ++k, rest >>= 4)
     {
         const float2 texel = shared.planes[0][(uint32_t(rest) & 15u) * 32 + lane];
@@ -1774,6 +1788,9 @@ __device__ void RunWholeBlockTask(SearchStorage& shared, int task, int lane)
 // kSingle: a texture of one channel, which has no green, no blue and - in groups of blocks inside the mip - no alpha but 1: the partition searches
 // take red alone.  1024 x 1024 texels: 513 -> 356 us.  (Three channels without alpha in mode 7's partitions gained nothing: 516.4 -> 515.2, and
 // 701 x 503 took 242.1 instead of 238.4, as the groups at the mip's edge need the search with alpha.)
+// kPixelsAtOnce: pixels that the partition searches take at a time.  Up to two CTAs an SM, where a search's own length bounds the time, four: 16 x 16
+// to 384 x 384 texels 113 - 121 -> 101 - 109 us, 512 x 512 170 -> 165.  Above, where warps fill the SM, one: 768 x 768 314 us against 351, 1024 x 1024 518 against 642.  (The kernels for
+// few CTAs are a module of their own, which leaves the others' code as it is without them: beside them 1024 x 1024 took 521.)
 template <bool kSingle>
 __global__ void __launch_bounds__(kSearchThreads, 3) Bc7SearchKernel(const Bc7Arguments args)
 {
@@ -1893,6 +1910,20 @@ __global__ void __launch_bounds__(kSearchThreads, 3) Bc7SearchKernel(const Bc7Ar
 
 } // namespace
 
+#ifdef NTCB_BC7_FEW_BLOCKS
+
+void LaunchBc7SearchOfFew(const Bc7Arguments& args, dim3 grid, cudaStream_t stream)
+{
+    if (args.numChannels == 1)
+        Bc7SearchKernel<true><<<grid, kSearchThreads, 0, stream>>>(args);
+    else
+        Bc7SearchKernel<false><<<grid, kSearchThreads, 0, stream>>>(args);
+}
+
+} // namespace ntcb
+
+#else
+
 int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCompressArguments& base, cudaStream_t stream)
 {
     Bc7Arguments args;
@@ -1933,7 +1964,9 @@ int LaunchBlockCompressBc7(const NtcbBlockCompressParams& params, const BlockCom
     ForEachGrid(base, groupWidth, groupHeight, [&](const BlockCompressArguments& part, int top, dim3 grid) {
         args.base = part;
         args.modeMapOffsetY = params.modeMapOffsetY + top;
-        if (search && args.numChannels == 1)
+        if (search && (long long)grid.x * grid.y <= 2ll * sms)
+            LaunchBc7SearchOfFew(args, grid, stream);
+        else if (search && args.numChannels == 1)
             Bc7SearchKernel<true><<<grid, kSearchThreads, 0, stream>>>(args);
         else if (search)
             Bc7SearchKernel<false><<<grid, kSearchThreads, 0, stream>>>(args);
@@ -2026,3 +2059,5 @@ extern "C" int ntcb_make_bc7_mode_buffer(int widthInBlocks, int heightInBlocks, 
     ClearError();
     return NTCB_OK;
 }
+
+#endif

@@ -589,16 +589,19 @@ def test_images_of_more_rows_than_a_grid_has(block_format):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("block_format", [4, 5])
-def test_blocks_of_small_images_are_those_of_large_ones(block_format):
-    """Up to some number of searches per SM eight lanes share the search of a BC4 block, above it a lane has one: the same bytes, at sizes around that
-    line and at the edges of a CTA's eight searches, for smooth and noisy values, 0 and 1 with and without others between, and NaN."""
+@pytest.mark.parametrize("block_format,channels", [(4, 1), (5, 2), (7, 1), (7, 3), (7, 4)])
+def test_blocks_of_small_images_are_those_of_large_ones(block_format, channels):
+    """Up to some number of searches per SM eight lanes share the search of a BC4 block, above it a lane has one; BC7's full search of few CTAs is unrolled
+    further: the same bytes, at sizes around those lines and at the edges of a CTA's blocks, for smooth and noisy values, 0 and 1 with and without others
+    between, and NaN."""
     import torch
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    columns, rows = 2 * sms, 64  # more than the 56 searches per SM
+    columns, rows = 2 * sms, 68  # more than the 56 searches per SM, and than two of BC7's CTAs of 64 blocks
+    if block_format == 7:
+        rows = 80
     generator = torch.Generator(device="cuda").manual_seed(block_format)
-    shape = (rows * 4, columns * 4, 2)
+    shape = (rows * 4, columns * 4, 4)
     texels = torch.rand(shape, device="cuda", generator=generator)
     band = rows * 4 // 8
     ramp = torch.linspace(0, 1, columns * 4, device="cuda")[None, :, None]
@@ -609,12 +612,13 @@ def test_blocks_of_small_images_are_those_of_large_ones(block_format):
     texels[5 * band:6 * band] = torch.where(texels[5 * band:6 * band] > 0.8, float("nan"), texels[5 * band:6 * band])
     texels[6 * band:7 * band] = ((texels[6 * band:7 * band] * 6).floor() / 5).clamp(0, 1)
     texels = texels.to(torch.float16).contiguous()
-    whole = binding.block_compress(texels, block_format, 0)
-    channels = block_format - 3
-    line = 56 * sms // channels
-    for left, top, width, height in ((0, 0, 1, 1), (3, 9, 7, 1), (5, 17, 1, 8), (9, 25, 9, 1), (1, 33, 33, 3), (0, 0, columns, line // columns), (0, 36, columns, 28 // channels),
-                                     (0, 1, columns, line // columns + 1), (7, 30, columns - 7, 10)):
-        part = binding.block_compress(texels, block_format, 0, src_left=4 * left, src_top=4 * top, width_in_blocks=width, height_in_blocks=height)
+    options = {"num_channels": channels} if block_format == 7 else {}
+    whole = binding.block_compress(texels, block_format, 0, **options)
+    line = (2 * sms // ((columns + 15) // 16) * 4 if block_format == 7 else 56 * sms // channels // columns)  # the tallest window below the line
+    assert line + 1 < rows
+    for left, top, width, height in ((0, 0, 1, 1), (3, 9, 7, 1), (5, 17, 1, 8), (9, 25, 9, 1), (1, 33, 33, 3), (0, 0, columns, line), (0, rows - line, columns, line),
+                                     (0, 1, columns, line + 1), (7, 30, columns - 7, 10)):
+        part = binding.block_compress(texels, block_format, 0, src_left=4 * left, src_top=4 * top, width_in_blocks=width, height_in_blocks=height, **options)
         assert torch.equal(part, whole[top:top + height, left:left + width]), (left, top, width, height)
 
 
