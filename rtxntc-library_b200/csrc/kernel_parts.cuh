@@ -461,7 +461,7 @@ __device__ __forceinline__ uint32_t LayerBarrier(int chain, uint32_t& giveUp)
 
 // Launches a kernel that calls GridDependencyWait before it touches global memory, so that its start overlaps the end of
 // the kernel before it in the stream: when it came, a 96 x 40 set decoded back to back in 6.3 us instead
-// of 8.2, mip 0 of a 1024 x 1024 one in 58.8 instead of 61.6 (now 4.5 and 44.5).
+// of 8.2, mip 0 of a 1024 x 1024 one in 58.8 instead of 61.6 (now 4.3 and 40.9).
 template <typename Kernel, typename Params>
 cudaError_t LaunchOverlapped(Kernel kernel, int ctas, int threads, size_t sharedBytes, cudaStream_t stream, const Params& params)
 {
