@@ -22,8 +22,13 @@ namespace
 template <typename Tables, const FootprintBuffers& kBuffers>
 struct __align__(16) ChainStage
 {
+    // Bytes of a staged latent pixel.
     template <int kLayers>
-    static constexpr int kPixelBytes = kBuffers.pixelBytes[kLayers];
+    static __device__ __forceinline__ constexpr int PixelBytes()
+    {
+        constexpr int kBytes = kBuffers.pixelBytes[kLayers];
+        return kBytes;
+    }
     Tables tables;
     uint8_t footprintHi[kBuffers.hiBytes];
     uint8_t footprintLo[kBuffers.loBytes];
@@ -73,7 +78,7 @@ template <int kLayers, typename Stage, typename Blend>
 __device__ __forceinline__ void GatherTexel(const KernelParams& params, const KernelMip& mip, const Stage& stage, int texel, int2 shift, Blend blend)
 {
     const uint4 taps = stage.texels.taps[texel];
-    const int stride = StrideBytes<Stage, kLayers>(mip);
+    const int stride = Stage::template PixelBytes<kLayers>();
 #pragma unroll
     for (int grid = 0; grid < 2; ++grid)
     {
@@ -81,7 +86,7 @@ __device__ __forceinline__ void GatherTexel(const KernelParams& params, const Ke
         const uint8_t* tap00 = grid ? stage.footprintLo + (taps.z + shift.y) : stage.footprintHi + (taps.x + shift.x);
         const uint8_t* tap10 = tap00 + (grid ? taps.w : taps.y);
         const __half2 w00 = AsHalf2(w.x), w01 = AsHalf2(w.y), w10 = AsHalf2(w.z), w11 = AsHalf2(w.w);
-        if constexpr (kLayers % 2 == 0 && kLayers != 0 && Stage::template kPixelBytes<kLayers> % 16 == 0)
+        if constexpr (kLayers % 2 == 0 && Stage::template PixelBytes<kLayers>() % 16 == 0)
         {
             // two layers of a tap at once
 #pragma unroll
@@ -98,7 +103,7 @@ __device__ __forceinline__ void GatherTexel(const KernelParams& params, const Ke
         {
 #pragma unroll
             for (int layer = 0; layer < 4; ++layer)
-                if (layer < NumLayers<kLayers>(params))
+                if (layer < kLayers)
                     blend(grid, layer, *reinterpret_cast<const uint2*>(tap00 + layer * 8), *reinterpret_cast<const uint2*>(tap00 + stride + layer * 8),
                         *reinterpret_cast<const uint2*>(tap10 + layer * 8), *reinterpret_cast<const uint2*>(tap10 + stride + layer * 8), w00, w01, w10, w11);
         }
@@ -281,7 +286,7 @@ __device__ __forceinline__ void DecodeRuns(const KernelParams& params)
         ctx.y = y0 + tileRow;
         // runs start at multiples of their width
         const int column = x0 & (mip.runTiles * kChainTileWidth - 1);
-        const int steps = known ? column / kChainTileWidth * StrideBytes<Stage, kLayers>(mip) : 0;
+        const int steps = known ? column / kChainTileWidth * Stage::template PixelBytes<kLayers>() : 0;
         Chain::template BuildInputs<kLayers>(params, mip, stage, ctx, column + tileColumn, tileRow, known,
             make_int2(steps * mip.hiStepX, steps * mip.loStepX));
 

@@ -479,7 +479,7 @@ cudaError_t LaunchDecodeLayers(const KernelParams& params, int ctas, cudaStream_
     case 2: return launch(std::integral_constant<int, 2>());
     case 3: return launch(std::integral_constant<int, 3>());
     case 4: return launch(std::integral_constant<int, 4>());
-    default: return launch(std::integral_constant<int, 0>());
+    default: return launch(std::integral_constant<int, 1>());
     }
 }
 

@@ -101,8 +101,6 @@ struct KernelMip
     unsigned tilesXMagic; // ceil(2^32 / tilesX): local / tilesX == umulhi(local, magic) for every tile of the mip; 0: divide
     int runTiles;         // tiles side by side whose tables and footprints are prepared together (1, 2 or 4)
     int staged;      // the tile footprints of both grids fit into shared memory
-    int strideBytes; // bytes per staged latent pixel: 8 per layer, padded to an odd multiple of 8 (8, 24, 24, 40) so that
-                     // the 8-byte reads of neighbouring pixels fall into different shared-memory banks
     int storeBytes;  // widest store (4, 8 or 16 bytes) the fp16 texels of this mip may go out with: the interleaved
                      // layout with a texel size and a mip address that are multiples of it; 4 otherwise
     int invariant;   // every size involved is a power of two: the tap and positional-encoding tables of a tile do not

@@ -231,7 +231,7 @@ __device__ __forceinline__ void PrepareTileRef(const KernelParams& params, const
             }
         });
     }
-    PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, StrideBytes<RefStage, kLayers>(mip), tileX0,
+    PrepareTaps<ChainTile, true, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, RefStage::PixelBytes<kLayers>(), tileX0,
         tileY0, columns, lane, warp, tablesValid, between);
 }
 
@@ -288,7 +288,7 @@ __device__ __forceinline__ void SampleLayerRef(const uint16_t* __restrict__ plan
 
 // The 48 network inputs of one texel as 24 binary16 pairs -> its 96-byte row of the A operand.  `column`: in the run.  `known`: TexelTables
 // and the row's last two chunks are those of an earlier tile with the same tables, whose taps lie `shift` bytes before.
-template <int kLayers = 0>
+template <int kLayers>
 __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const KernelMip& mip, RefStage& stage,
     const ChainContext& ctx, int column, int tileRow, bool known, int2 shift)
 {
@@ -317,13 +317,13 @@ __device__ __forceinline__ void BuildInputsRef(const KernelParams& params, const
         const uint16_t* hi = params.latents + mip.hiOffset;
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
-            if (layer < NumLayers<kLayers>(params))
+            if (layer < kLayers)
                 SampleLayerRef(hi + size_t(layer) * mip.hiPlane, taps, words + 2 * layer);
         SetupTaps(u, v, mip.loWidth, mip.loHeight, taps);
         const uint16_t* lo = params.latents + mip.loOffset;
 #pragma unroll
         for (int layer = 0; layer < 4; ++layer)
-            if (layer < NumLayers<kLayers>(params))
+            if (layer < kLayers)
                 SampleLayerRef(lo + size_t(layer) * mip.loPlane, taps, words + 8 + 2 * layer);
     }
 
@@ -1063,7 +1063,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1) SampleKernelRefFp8(const
 
 } // namespace
 
-// The kernel of a weight set and epilogue compiled for 2, 3 or 4 latent layers, or the one for any number.
+// The kernel of a weight set and epilogue compiled for the number of latent layers, 1 to 4.
 template <bool kFp8Weights, int kConvert>
 cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStream_t stream)
 {
@@ -1083,7 +1083,7 @@ cudaError_t LaunchDecodeRefLayers(const KernelParams& params, int ctas, cudaStre
     case 2: return launch(std::integral_constant<int, 2>());
     case 3: return launch(std::integral_constant<int, 3>());
     case 4: return launch(std::integral_constant<int, 4>());
-    default: return launch(std::integral_constant<int, 0>());
+    default: return launch(std::integral_constant<int, 1>());
     }
 }
 

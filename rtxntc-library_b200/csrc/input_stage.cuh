@@ -15,22 +15,10 @@ namespace ntcb
 namespace
 {
 
-// The decode kernels are compiled for a fixed number of latent layers (kLayers = 2, 3 or 4: 8, 12 or
-// 16 features, the shapes the reference's presets use) and once for any number (kLayers = 0): with
-// the count known the layer loops unroll without predicated-off iterations and the footprint
-// stride is a constant - 5 % fewer instructions on the benchmark set.
-template <int kLayers>
-__device__ __forceinline__ int NumLayers(const KernelParams& params)
-{
-    return kLayers ? kLayers : params.numLayers;
-}
-
-template <typename Stage, int kLayers>
-__device__ __forceinline__ int StrideBytes(const KernelMip& mip)
-{
-    constexpr int kBytes = Stage::template kPixelBytes<kLayers>;
-    return kLayers ? kBytes : mip.strideBytes;
-}
+// The decode kernels are compiled per number of latent layers, 1 to 4 (4 to 16 features): the loops over layers unroll without predicated-off
+// iterations and the footprint stride is a constant - 5 % fewer instructions on the benchmark set than with one kernel for any number, which sets of one
+// layer kept longest (2048 x 2048 of 4 features at scale 4: FP8 154 -> 136 us, Int8 191 -> 183, exact accumulation 177 -> 168 and 253 -> 237; at scale 1
+// FP8 181 -> 150, Int8 222 -> 200).
 
 // Quantises a pair of network inputs.  Int8: floor(x * 127.5 - 0.5) clamped to +-127
 // (src/tin/tin_mlp.h:25-31), returned as the low bytes of the two 16-bit lanes.  FP8: round to
@@ -373,7 +361,7 @@ __device__ __forceinline__ void PrepareTaps(const KernelParams& params, const Ke
 #pragma unroll
             for (int layer = 0; layer < 4; ++layer)
             {
-                if (layer < NumLayers<kLayers>(params))
+                if (layer < kLayers)
                 {
                     const uint32_t pixel = __ldg(plane0 + (first + uint32_t(layer) * planePixels));
                     __half2 first, second;
@@ -432,7 +420,7 @@ __device__ __forceinline__ void PrepareTile(const KernelParams& params, const Ke
                 stage.tables.lodWord = QuantizeLod<kFp8>(mip.positionLod);
         });
     }
-    PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, StrideBytes<Stage, kLayers>(mip),
+    PrepareTaps<Tile, kReferenceDivision, kLayers>(params, mip, stage.tables.taps, stage.footprintHi, stage.footprintLo, Stage::template PixelBytes<kLayers>(),
         tileX0, tileY0, columns, lane, warp, tablesValid, between);
 }
 
@@ -504,7 +492,7 @@ __device__ __forceinline__ void SampleGridsDirect(const uint16_t* __restrict__ l
 
 // The 48 network inputs of one texel of a mip whose footprints are too large to stage (strong minification) -> its 64-byte row of the A operand
 // (K-major core matrices: 16-byte chunk j of row r lives at j * 2048 + r * 16).
-template <bool kFp8, bool kReferenceDivision, int kLayers = 0, typename Stage, typename Context>
+template <bool kFp8, bool kReferenceDivision, int kLayers, typename Stage, typename Context>
 __device__ __forceinline__ void BuildInputs(const KernelParams& params, const KernelMip& mip, const Stage& stage,
     const Context& ctx, int tileColumn, int tileRow)
 {
@@ -513,7 +501,7 @@ __device__ __forceinline__ void BuildInputs(const KernelParams& params, const Ke
     for (int i = 0; i < 8; ++i)
         words[i] = QuantizedZeros<kFp8>(); // unused feature slots hold quantised zeros (src/Inference.cu:49)
     // the taps are read from global memory; threads past the right / bottom edge compute a clamped texel and store nothing
-    SampleGridsDirect<kFp8, kReferenceDivision>(params.latents, NumLayers<kLayers>(params), mip, min(ctx.x, mip.width - 1), min(ctx.y, mip.rowEnd - 1),
+    SampleGridsDirect<kFp8, kReferenceDivision>(params.latents, kLayers, mip, min(ctx.x, mip.width - 1), min(ctx.y, mip.rowEnd - 1),
         words);
     // positional encoding: interleave the column's x bytes with the row's y bytes
     const uint2 cx = stage.tables.colEnc[tileColumn];

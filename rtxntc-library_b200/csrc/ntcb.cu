@@ -111,8 +111,7 @@ void FillKernelMip(const NtcbMipDesc& m, int layers, KernelMip& km, FootprintBuf
     km.invHeight = 1.0f / float(m.height);
     km.positionScale = m.positionScale;
     km.positionLod = m.positionLod;
-    km.strideBytes = buffers.pixelBytes[layers];
-    const int staged = StagedTiles(m.hiWidth, m.hiHeight, m.loWidth, m.loHeight, m.width, m.height, km.strideBytes, buffers, maxRunTiles);
+    const int staged = StagedTiles(m.hiWidth, m.hiHeight, m.loWidth, m.loHeight, m.width, m.height, buffers.pixelBytes[layers], buffers, maxRunTiles);
     km.staged = staged > 0;
     km.runTiles = staged > 0 ? staged : 1;
     // Tables that do not depend on the tile: with power-of-two sizes all the tap arithmetic is exact in
