@@ -494,16 +494,18 @@ cudaError_t LaunchSampleLayers(const SampleParams& params, int ctas, cudaStream_
         return LaunchChains(SampleKernel<kFp8, kInterleaved, kLayers>, done[kLayers], SharedBytes<ExactStorage>(chains, 0),
             SharedBytes<ExactStorage>(kMaxChains, 0), chains, params, ctas, stream);
     };
-    if constexpr (kInterleaved) // as in the reference-numerics kernels: the presets' layer counts
+    if constexpr (kInterleaved) // as in the reference-numerics kernels: the layer counts
     {
         switch (params.numLayers)
         {
         case 2: return launch(std::integral_constant<int, 2>());
         case 3: return launch(std::integral_constant<int, 3>());
         case 4: return launch(std::integral_constant<int, 4>());
+        default: return launch(std::integral_constant<int, 1>());
         }
     }
-    return launch(std::integral_constant<int, 0>());
+    else
+        return launch(std::integral_constant<int, 0>());
 }
 
 } // namespace
